@@ -689,6 +689,29 @@ int rlm_slot_mix_residual(const float* slot_context, const uint8_t* anchor_activ
 int rlm_selftest_bounded_wait(int32_t* status, int64_t cycle_limit, int64_t* waited_cycles,
                               void* stream);
 
+/*
+ * The relation MLP of a whole-sequence pass in one launch (extension): rlm_relation_hidden_cached (rows
+ * form) -> second relation-MLP layer -> rlm_relation_norm_reduce (rows form) -> residual, and with
+ * slot_weight / anchor_active (both or neither) rlm_slot_mix_residual as well.  Neither the hidden states
+ * nor the second layer's rows reach device memory.
+ *   out[n, :] = residual[n, :] + scale * sum_s sum_k u[n, s, k] * LayerNorm(raw[n, s, k, :])
+ * Query row n is position n % rows_per_seq of sequence n / rows_per_seq (of caches [B, T, .]); it has `slots`
+ * anchors anchor_index [N, S] with k_out partners each: partner_index, partner_scores [N, S, K].  u is the
+ * softmax over a slot's partners with finite scores — with limit_by_position also k < clamp(ceil(log2(t + 2)), 1, K) —
+ * times the slot's weight, renormalised over the row's active slots.  scale: one fp32 element, NULL = 1;
+ * residual: NULL = 0, and may be `out` itself.  Caches and weights share bf16 or fp16; second_bias, LayerNorm
+ * parameters, residual and out are fp32.  _supported: k_out and slots powers of two with 2 <= k_out, k_out * slots <= 32,
+ * relation_dim 64 or 128, d_model a multiple of 64 up to 384 or of 128 up to 768.
+ */
+int rlm_relation_mlp_rows_supported(int k_out, int slots, int relation_dim, int hidden_dim, int d_model, int dtype);
+int rlm_relation_mlp_rows(
+    const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index, const int32_t* partner_index,
+    const float* partner_scores, const uint8_t* anchor_active, const float* slot_weight, const float* scale,
+    const void* product_weight, const void* second_weight, const float* second_bias, const float* norm_weight,
+    const float* norm_bias, float norm_eps, const float* residual, float* out, int n_rows, int slots, int n_seq,
+    int rows_per_seq, int max_t, int relation_dim, int hidden_dim, int d_model, int k_out, int limit_by_position, int dtype,
+    int32_t* status, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

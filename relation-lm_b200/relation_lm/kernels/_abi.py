@@ -1,4 +1,5 @@
-"""ctypes binding of ``librelation_lm_b200.so`` (declared in include/relation_lm_b200.h)."""
+"""ctypes binding of ``librelation_lm_b200.so`` (declared in include/relation_lm_b200.h); importing this
+module also loads ``librelation_lm_torch.so``, which registers the ``torch.library`` operators."""
 from __future__ import annotations
 
 import ctypes
@@ -8,6 +9,7 @@ import torch
 
 ABI_VERSION = 2          # RLM_ABI_VERSION of include/relation_lm_b200.h this binding was written against
 _LIB_PATH = Path(__file__).resolve().parents[2] / "lib" / "librelation_lm_b200.so"
+_OPS_PATH = _LIB_PATH.with_name("librelation_lm_torch.so")
 
 DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
 
@@ -47,6 +49,8 @@ PROTOTYPES = {
     "rlm_decode_front": [_P] * 6 + [_F] + [_P] * 4 + [_F] + [_P] * 6 + [_I] * 8 + [_P, _P],
     "rlm_relation_layer_tail_supported": [_I] * 7,
     "rlm_relation_layer_tail": [_P] * 11 + [_F, _P, _P, _P, _P, _F, _P, _P, _P] + [_I] * 8 + [_P, _P],
+    "rlm_relation_mlp_rows_supported": [_I] * 6,
+    "rlm_relation_mlp_rows": [_P] * 13 + [_F, _P, _P] + [_I] * 11 + [_P, _P],
     "rlm_relation_layer_supported": [_I] * 12,
     "rlm_relation_layer": [_P] * 19 + [_L] * 3 + [_I] * 6 + [_P] * 7 + [_F, _P, _P, _P, _P, _F, _P, _P, _P]
                           + [_I] * 8 + [_P, _P],
@@ -54,10 +58,11 @@ PROTOTYPES = {
 
 
 def _load() -> ctypes.CDLL:
-    if not _LIB_PATH.exists():
-        raise ImportError(
-            f"{_LIB_PATH} is missing: build it with `make -C {_LIB_PATH.parents[1] / 'csrc'}` "
-            "(nvcc, sm_100a).  relation_lm has no fallback implementation.")
+    for path in (_LIB_PATH, _OPS_PATH):
+        if not path.exists():
+            raise ImportError(
+                f"{path} is missing: build it with `make -C {_LIB_PATH.parents[1] / 'csrc'}` "
+                "(nvcc, sm_100a).  relation_lm has no fallback implementation.")
     lib = ctypes.CDLL(str(_LIB_PATH))
     for name, argtypes in PROTOTYPES.items():
         fn = getattr(lib, name)
@@ -76,6 +81,7 @@ def _load() -> ctypes.CDLL:
 
 
 LIB = _load()
+torch.ops.load_library(str(_OPS_PATH))
 
 _STATUS: dict[int, torch.Tensor] = {}
 
@@ -85,7 +91,7 @@ def status_tensor(device: torch.device) -> torch.Tensor:
     index = device.index if device.index is not None else torch.cuda.current_device()
     word = _STATUS.get(index)
     if word is None:
-        word = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", index))
+        word = torch.ops.relation_lm._status_word(index)        # the word the native operators pass as well
         _STATUS[index] = word
     return word
 

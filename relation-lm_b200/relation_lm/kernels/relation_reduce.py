@@ -15,6 +15,23 @@ from torch import Tensor
 
 from relation_lm.kernels import _abi
 
+# The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
+_relation_hidden_cached = torch.ops.relation_lm.relation_hidden_cached.default
+_relation_hidden_cached_out = torch.ops.relation_lm.relation_hidden_cached_out.default
+_expanded_cache_append = torch.ops.relation_lm.expanded_cache_append.default
+_expanded_cache_append_packed = torch.ops.relation_lm.expanded_cache_append_packed.default
+_relation_hidden_cache_update = torch.ops.relation_lm.relation_hidden_cache_update.default
+_relation_norm_reduce = torch.ops.relation_lm.relation_norm_reduce.default
+_relation_hidden_cache_update_out = torch.ops.relation_lm.relation_hidden_cache_update_out.default
+_relation_norm_reduce_residual = torch.ops.relation_lm.relation_norm_reduce_residual.default
+_relation_norm_reduce_residual_norm_project = torch.ops.relation_lm.relation_norm_reduce_residual_norm_project.default
+_relation_norm_reduce_residual_norm = torch.ops.relation_lm.relation_norm_reduce_residual_norm.default
+_relation_hidden_cached_rows = torch.ops.relation_lm.relation_hidden_cached_rows.default
+_relation_hidden_cached_rows_out = torch.ops.relation_lm.relation_hidden_cached_rows_out.default
+_relation_norm_reduce_rows = torch.ops.relation_lm.relation_norm_reduce_rows.default
+_relation_mlp_rows = torch.ops.relation_lm.relation_mlp_rows.default
+_relation_layer_tail = torch.ops.relation_lm.relation_layer_tail.default
+
 
 @dataclass(frozen=True)
 class FactorizedRelationWeights:
@@ -61,15 +78,6 @@ def recommended_relation_cache_mode(batch_size: int) -> str:
     return "fused_update" if batch_size == 1 else "separate_update"
 
 
-def _check_indices(anchor_index: Tensor, partner_index: Tensor, rows: int) -> None:
-    if anchor_index.dtype != torch.int32 or partner_index.dtype != torch.int32:
-        raise ValueError("anchor_index and partner_index must be int32")
-    if anchor_index.numel() != rows or partner_index.dim() != 2 or partner_index.size(0) != rows:
-        raise ValueError("anchor_index must be [B] and partner_index [B, K]")
-
-
-@torch.library.custom_op("relation_lm::relation_hidden_cached", mutates_args=(),
-                         device_types="cuda")
 def relation_hidden_cached(
     expanded_cache: Tensor,
     operand_cache: Tensor,
@@ -78,33 +86,15 @@ def relation_hidden_cached(
     product_weight: Tensor,
 ) -> Tensor:
     """``gelu((o[p] * o[a]) W_m^T + E[a, :H] + E[p, H:])`` for every partner slot, ``[B, K, H]`` fp32."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, product_weight=product_weight)
-    batch, max_t, rdim = operand_cache.shape
-    hdim, k_out = product_weight.size(0), partner_index.size(1)
-    _check_indices(anchor_index, partner_index, batch)
-    if expanded_cache.shape != (batch, max_t, 2 * hdim) or product_weight.size(1) != rdim:
-        raise ValueError("expanded_cache must be [B, T, 2H] and product_weight [H, R]")
-    out = torch.empty((batch, k_out, hdim), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cached(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(product_weight), None, _abi.ptr(out), batch, batch,
-            max_t, rdim, hdim, k_out, _abi.same_dtype("cache", expanded_cache, operand_cache),
-            _abi.code(product_weight), _abi.code(out), _abi.ptr(_abi.status_tensor(device)),
-            _abi.stream_ptr(device)))
-    return out
+    return _relation_hidden_cached(expanded_cache, operand_cache, anchor_index, partner_index, product_weight)
 
 
-@relation_hidden_cached.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cached")
 def _(expanded_cache, operand_cache, anchor_index, partner_index, product_weight):
     return operand_cache.new_empty(
         (operand_cache.size(0), partner_index.size(1), product_weight.size(0)), dtype=torch.float32)
 
 
-@torch.library.custom_op("relation_lm::relation_hidden_cached_out", mutates_args=("out",),
-                         device_types="cuda")
 def relation_hidden_cached_out(
     out: Tensor,
     expanded_cache: Tensor,
@@ -115,31 +105,14 @@ def relation_hidden_cached_out(
 ) -> None:
     """``relation_hidden_cached`` writing into a caller-owned ``out [B, K, H]`` of any float dtype
     (extension: a 16-bit ``out`` feeds the second MLP layer without a cast)."""
-    device = _abi.require_cuda_contiguous(
-        out=out, expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, product_weight=product_weight)
-    batch, max_t, rdim = operand_cache.shape
-    hdim, k_out = product_weight.size(0), partner_index.size(1)
-    _check_indices(anchor_index, partner_index, batch)
-    if expanded_cache.shape != (batch, max_t, 2 * hdim) or product_weight.size(1) != rdim \
-            or out.shape != (batch, k_out, hdim):
-        raise ValueError("expected expanded_cache [B, T, 2H], product_weight [H, R] and out [B, K, H]")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cached(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(product_weight), None, _abi.ptr(out), batch, batch,
-            max_t, rdim, hdim, k_out, _abi.same_dtype("cache", expanded_cache, operand_cache),
-            _abi.code(product_weight), _abi.code(out), _abi.ptr(_abi.status_tensor(device)),
-            _abi.stream_ptr(device)))
+    _relation_hidden_cached_out(out, expanded_cache, operand_cache, anchor_index, partner_index, product_weight)
 
 
-@relation_hidden_cached_out.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cached_out")
 def _(out, expanded_cache, operand_cache, anchor_index, partner_index, product_weight):
     return None
 
 
-@torch.library.custom_op("relation_lm::expanded_cache_append", mutates_args=("expanded_cache",),
-                         device_types="cuda")
 def expanded_cache_append(
     expanded_cache: Tensor,
     operand_cache: Tensor,
@@ -152,34 +125,14 @@ def expanded_cache_append(
     (extension, tensor cores): ``expanded[l, :, t] = [W_a[l] o + b_1[l], W_p[l] o]`` with
     ``o = operand_cache[l, :, t]``.  Stacked 16-bit tensors: caches ``[L, B, T, .]``, weights
     ``[L, H, R]``, bias ``[L, H]``.  The per-layer kernels then use ``relation_hidden_cached``."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_weight=anchor_weight,
-        partner_weight=partner_weight, first_bias=first_bias)
-    _abi.require_position(position, device)
-    if operand_cache.dim() != 4 or expanded_cache.dim() != 4 or anchor_weight.dim() != 3:
-        raise ValueError("expected stacked tensors: caches [L, B, T, .], weights [L, H, R], bias [L, H]")
-    layers, batch, max_t, rdim = operand_cache.shape
-    hdim = anchor_weight.size(1)
-    if expanded_cache.shape != (layers, batch, max_t, 2 * hdim) or anchor_weight.shape != (layers, hdim, rdim) \
-            or partner_weight.shape != anchor_weight.shape or first_bias.shape != (layers, hdim):
-        raise ValueError("expected expanded_cache [L, B, T, 2H], weights [L, H, R] and first_bias [L, H]")
-    dtype = _abi.same_dtype("cache", expanded_cache, operand_cache)
-    if len({anchor_weight.dtype, partner_weight.dtype, first_bias.dtype, expanded_cache.dtype}) != 1:
-        raise ValueError("caches, weights and bias must share one 16-bit dtype")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_expanded_cache_append(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_weight),
-            _abi.ptr(partner_weight), _abi.ptr(first_bias), _abi.ptr(position), layers, batch, max_t,
-            rdim, hdim, dtype, _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _expanded_cache_append(expanded_cache, operand_cache, anchor_weight, partner_weight, first_bias, position)
 
 
-@expanded_cache_append.register_fake
+@torch.library.register_fake("relation_lm::expanded_cache_append")
 def _(expanded_cache, operand_cache, anchor_weight, partner_weight, first_bias, position):
     return None
 
 
-@torch.library.custom_op("relation_lm::expanded_cache_append_packed", mutates_args=("expanded_cache",),
-                         device_types="cuda")
 def expanded_cache_append_packed(
     expanded_cache: Tensor,
     packed: Tensor,
@@ -192,35 +145,14 @@ def expanded_cache_append_packed(
     rows ``packed [B, L * (384 + R)]`` (layout of ``sparse_cache_append``) instead of the operand cache:
     same results, no dependence on the state append, which it overlaps under programmatic launch.
     ``packed`` must not come from the launch right before this one on the stream."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, anchor_weight=anchor_weight, partner_weight=partner_weight,
-        first_bias=first_bias)
-    _abi.require_cuda_rows(packed=packed)
-    _abi.require_position(position, device)
-    if expanded_cache.dim() != 4 or anchor_weight.dim() != 3 or packed.dim() != 2:
-        raise ValueError("expected expanded_cache [L, B, T, 2H], packed [B, L * (384 + R)], weights [L, H, R]")
-    layers, batch, max_t, _ = expanded_cache.shape
-    hdim, rdim = anchor_weight.size(1), anchor_weight.size(2)
-    if expanded_cache.size(3) != 2 * hdim or anchor_weight.shape != (layers, hdim, rdim) \
-            or partner_weight.shape != anchor_weight.shape or first_bias.shape != (layers, hdim) \
-            or packed.shape != (batch, layers * (384 + rdim)):
-        raise ValueError("expected expanded_cache [L, B, T, 2H], packed [B, L * (384 + R)], weights [L, H, R], bias [L, H]")
-    if len({anchor_weight.dtype, partner_weight.dtype, first_bias.dtype, expanded_cache.dtype, packed.dtype}) != 1:
-        raise ValueError("cache, packed rows, weights and bias must share one 16-bit dtype")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_expanded_cache_append_packed(
-            _abi.ptr(expanded_cache), _abi.ptr(packed), packed.stride(0), 384 + rdim, 128, _abi.ptr(anchor_weight),
-            _abi.ptr(partner_weight), _abi.ptr(first_bias), _abi.ptr(position), layers, batch, max_t, rdim, hdim,
-            _abi.code(expanded_cache), _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _expanded_cache_append_packed(expanded_cache, packed, anchor_weight, partner_weight, first_bias, position)
 
 
-@expanded_cache_append_packed.register_fake
+@torch.library.register_fake("relation_lm::expanded_cache_append_packed")
 def _(expanded_cache, packed, anchor_weight, partner_weight, first_bias, position):
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_hidden_cache_update",
-                         mutates_args=("expanded_cache",), device_types="cuda")
 def relation_hidden_cache_update(
     expanded_cache: Tensor,
     operand_cache: Tensor,
@@ -233,40 +165,17 @@ def relation_hidden_cache_update(
     position: Tensor,
 ) -> Tensor:
     """As ``relation_hidden_cached``, after computing and storing ``expanded_cache[:, position]``."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, anchor_weight=anchor_weight, partner_weight=partner_weight,
-        product_weight=product_weight, first_bias=first_bias)
-    _abi.require_position(position, device)
-    batch, max_t, rdim = operand_cache.shape
-    hdim, k_out = product_weight.size(0), partner_index.size(1)
-    _check_indices(anchor_index, partner_index, batch)
-    if expanded_cache.shape != (batch, max_t, 2 * hdim) or product_weight.size(1) != rdim \
-            or anchor_weight.shape != product_weight.shape or partner_weight.shape != product_weight.shape \
-            or first_bias.numel() != hdim:
-        raise ValueError("expected expanded_cache [B, T, 2H], weights [H, R] and first_bias [H]")
-    out = torch.empty((batch, k_out, hdim), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cache_update(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(anchor_weight), _abi.ptr(partner_weight),
-            _abi.ptr(product_weight), _abi.ptr(first_bias), _abi.ptr(position), _abi.ptr(out),
-            batch, max_t, rdim, hdim, k_out,
-            _abi.same_dtype("cache", expanded_cache, operand_cache),
-            _abi.same_dtype("weight", anchor_weight, partner_weight, product_weight, first_bias),
-            _abi.code(out), _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-    return out
+    return _relation_hidden_cache_update(expanded_cache, operand_cache, anchor_index, partner_index, anchor_weight,
+                                         partner_weight, product_weight, first_bias, position)
 
 
-@relation_hidden_cache_update.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cache_update")
 def _(expanded_cache, operand_cache, anchor_index, partner_index, anchor_weight, partner_weight,
       product_weight, first_bias, position):
     return operand_cache.new_empty(
         (operand_cache.size(0), partner_index.size(1), product_weight.size(0)), dtype=torch.float32)
 
 
-@torch.library.custom_op("relation_lm::relation_norm_reduce", mutates_args=(),
-                         device_types="cuda")
 def relation_norm_reduce(
     raw: Tensor,
     partner_scores: Tensor,
@@ -277,53 +186,14 @@ def relation_norm_reduce(
 ) -> Tensor:
     """LayerNorm of each partner's relation vector, softmax over the active partner slots
     (``k < clamp(ceil(log2(position + 2)), 1, K)`` and a finite score) and their weighted sum."""
-    device = _abi.require_cuda_contiguous(raw=raw, partner_scores=partner_scores,
-                                          norm_weight=norm_weight, norm_bias=norm_bias)
-    _abi.require_position(position, device)
-    batch, k_out, dim = raw.shape
-    if partner_scores.shape != (batch, k_out) or partner_scores.dtype != torch.float32:
-        raise ValueError("partner_scores must be float32 [B, K]")
-    out = torch.empty((batch, dim), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_norm_reduce(
-            _abi.ptr(raw), _abi.ptr(partner_scores), _abi.ptr(norm_weight), _abi.ptr(norm_bias),
-            _abi.ptr(position), None, float(norm_eps), _abi.ptr(out), None, None, None, None, 0.0, None, 0, 1, 0, None,
-            batch, k_out, dim,
-            _abi.code(raw), _abi.same_dtype("norm parameter", norm_weight, norm_bias),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-    return out
+    return _relation_norm_reduce(raw, partner_scores, norm_weight, norm_bias, position, norm_eps)
 
 
-@relation_norm_reduce.register_fake
+@torch.library.register_fake("relation_lm::relation_norm_reduce")
 def _(raw, partner_scores, norm_weight, norm_bias, position, norm_eps):
     return raw.new_empty((raw.size(0), raw.size(2)), dtype=torch.float32)
 
 
-def _hidden_update_into(out, expanded_cache, operand_cache, anchor_index, partner_index,
-                        anchor_weight, partner_weight, product_weight, first_bias, position):
-    device = _abi.require_cuda_contiguous(
-        out=out, expanded_cache=expanded_cache, operand_cache=operand_cache,
-        anchor_index=anchor_index, partner_index=partner_index, anchor_weight=anchor_weight,
-        partner_weight=partner_weight, product_weight=product_weight, first_bias=first_bias)
-    _abi.require_position(position, device)
-    batch, max_t, rdim = operand_cache.shape
-    hdim, k_out = product_weight.size(0), partner_index.size(1)
-    _check_indices(anchor_index, partner_index, batch)
-    if out.shape != (batch, k_out, hdim) or expanded_cache.shape != (batch, max_t, 2 * hdim):
-        raise ValueError("expected out [B, K, H] and expanded_cache [B, T, 2H]")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cache_update(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(anchor_weight), _abi.ptr(partner_weight),
-            _abi.ptr(product_weight), _abi.ptr(first_bias), _abi.ptr(position), _abi.ptr(out),
-            batch, max_t, rdim, hdim, k_out,
-            _abi.same_dtype("cache", expanded_cache, operand_cache),
-            _abi.same_dtype("weight", anchor_weight, partner_weight, product_weight, first_bias),
-            _abi.code(out), _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-
-
-@torch.library.custom_op("relation_lm::relation_hidden_cache_update_out",
-                         mutates_args=("out", "expanded_cache"), device_types="cuda")
 def relation_hidden_cache_update_out(
     out: Tensor,
     expanded_cache: Tensor,
@@ -338,18 +208,16 @@ def relation_hidden_cache_update_out(
 ) -> None:
     """``relation_hidden_cache_update`` writing into a caller-owned ``out [B, K, H]`` of any
     float dtype (extension: a 16-bit ``out`` feeds the second MLP layer without a cast)."""
-    _hidden_update_into(out, expanded_cache, operand_cache, anchor_index, partner_index,
-                        anchor_weight, partner_weight, product_weight, first_bias, position)
+    _relation_hidden_cache_update_out(out, expanded_cache, operand_cache, anchor_index, partner_index, anchor_weight,
+                                      partner_weight, product_weight, first_bias, position)
 
 
-@relation_hidden_cache_update_out.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cache_update_out")
 def _(out, expanded_cache, operand_cache, anchor_index, partner_index, anchor_weight,
       partner_weight, product_weight, first_bias, position):
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_norm_reduce_residual", mutates_args=("hidden",),
-                         device_types="cuda")
 def relation_norm_reduce_residual(
     raw: Tensor,
     partner_scores: Tensor,
@@ -363,32 +231,14 @@ def relation_norm_reduce_residual(
     """``relation_norm_reduce`` fused with the layer's residual update (extension):
     ``hidden += mix * context`` in place, ``hidden [B, D]`` fp32, ``mix`` a 0-d fp32 tensor
     holding ``sigmoid(mix_logit)``."""
-    device = _abi.require_cuda_contiguous(raw=raw, partner_scores=partner_scores,
-                                          norm_weight=norm_weight, norm_bias=norm_bias,
-                                          hidden=hidden, mix=mix)
-    _abi.require_position(position, device)
-    batch, k_out, dim = raw.shape
-    if partner_scores.shape != (batch, k_out) or partner_scores.dtype != torch.float32:
-        raise ValueError("partner_scores must be float32 [B, K]")
-    if hidden.shape != (batch, dim) or hidden.dtype != torch.float32 or mix.dtype != torch.float32 \
-            or mix.numel() != 1:
-        raise ValueError("hidden must be float32 [B, D] and mix a one-element float32 tensor")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_norm_reduce(
-            _abi.ptr(raw), _abi.ptr(partner_scores), _abi.ptr(norm_weight), _abi.ptr(norm_bias),
-            _abi.ptr(position), None, float(norm_eps), None, _abi.ptr(hidden), _abi.ptr(mix),
-            None, None, 0.0, None, 0, 1, 0, None, batch, k_out, dim, _abi.code(raw),
-            _abi.same_dtype("norm parameter", norm_weight, norm_bias),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _relation_norm_reduce_residual(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix)
 
 
-@relation_norm_reduce_residual.register_fake
+@torch.library.register_fake("relation_lm::relation_norm_reduce_residual")
 def _(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix):
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_norm_reduce_residual_norm_project",
-                         mutates_args=("hidden", "normalized", "projected"), device_types="cuda")
 def relation_norm_reduce_residual_norm_project(
     raw: Tensor,
     partner_scores: Tensor,
@@ -409,44 +259,17 @@ def relation_norm_reduce_residual_norm_project(
     (extension, decode batches of a few rows): ``projected = normalized @ projection_weight.T`` with
     ``projection_weight [N, D]`` and ``projected [B, N]`` in the dtype of ``normalized``,
     ``N`` = 32, 64, ... 256 and ``D`` a multiple of 64.  One launch; a cluster of ``N / 32`` CTAs per row."""
-    device = _abi.require_cuda_contiguous(raw=raw, partner_scores=partner_scores,
-                                          norm_weight=norm_weight, norm_bias=norm_bias,
-                                          hidden=hidden, mix=mix, next_norm_weight=next_norm_weight,
-                                          next_norm_bias=next_norm_bias, normalized=normalized,
-                                          projection_weight=projection_weight, projected=projected)
-    _abi.require_position(position, device)
-    batch, k_out, dim = raw.shape
-    if partner_scores.shape != (batch, k_out) or partner_scores.dtype != torch.float32:
-        raise ValueError("partner_scores must be float32 [B, K]")
-    if hidden.shape != (batch, dim) or hidden.dtype != torch.float32 or mix.dtype != torch.float32 \
-            or mix.numel() != 1:
-        raise ValueError("hidden must be float32 [B, D] and mix a one-element float32 tensor")
-    if normalized.shape != (batch, dim) or next_norm_weight.dtype != torch.float32 \
-            or next_norm_bias.dtype != torch.float32 or next_norm_weight.numel() != dim:
-        raise ValueError("normalized must be [B, D] and the next LayerNorm parameters float32 [D]")
-    n_out = projection_weight.shape[0]
-    if projection_weight.shape != (n_out, dim) or projected.shape != (batch, n_out) \
-            or projection_weight.dtype != normalized.dtype or projected.dtype != normalized.dtype:
-        raise ValueError("projection_weight must be [N, D] and projected [B, N] in the dtype of normalized")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_norm_reduce_project(
-            _abi.ptr(raw), _abi.ptr(partner_scores), _abi.ptr(norm_weight), _abi.ptr(norm_bias),
-            _abi.ptr(position), float(norm_eps), _abi.ptr(hidden), _abi.ptr(mix),
-            _abi.ptr(next_norm_weight), _abi.ptr(next_norm_bias), float(next_norm_eps),
-            _abi.ptr(normalized), _abi.ptr(projection_weight), _abi.ptr(projected), n_out,
-            _abi.code(normalized), None, batch, k_out, dim, _abi.code(raw),
-            _abi.same_dtype("norm parameter", norm_weight, norm_bias),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _relation_norm_reduce_residual_norm_project(raw, partner_scores, norm_weight, norm_bias, position, norm_eps,
+                                                hidden, mix, next_norm_weight, next_norm_bias, next_norm_eps,
+                                                normalized, projection_weight, projected)
 
 
-@relation_norm_reduce_residual_norm_project.register_fake
+@torch.library.register_fake("relation_lm::relation_norm_reduce_residual_norm_project")
 def _(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix, next_norm_weight,
       next_norm_bias, next_norm_eps, normalized, projection_weight, projected):
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_norm_reduce_residual_norm",
-                         mutates_args=("hidden", "normalized"), device_types="cuda")
 def relation_norm_reduce_residual_norm(
     raw: Tensor,
     partner_scores: Tensor,
@@ -464,31 +287,11 @@ def relation_norm_reduce_residual_norm(
     """``relation_norm_reduce_residual`` that also writes ``normalized = layer_norm(hidden)`` of
     the updated rows (extension): ``normalized [B, D]`` bfloat16 / float16 with the next layer's
     (or the output head's) fp32 LayerNorm parameters, ready for the next projection."""
-    device = _abi.require_cuda_contiguous(raw=raw, partner_scores=partner_scores,
-                                          norm_weight=norm_weight, norm_bias=norm_bias,
-                                          hidden=hidden, mix=mix, next_norm_weight=next_norm_weight,
-                                          next_norm_bias=next_norm_bias, normalized=normalized)
-    _abi.require_position(position, device)
-    batch, k_out, dim = raw.shape
-    if partner_scores.shape != (batch, k_out) or partner_scores.dtype != torch.float32:
-        raise ValueError("partner_scores must be float32 [B, K]")
-    if hidden.shape != (batch, dim) or hidden.dtype != torch.float32 or mix.dtype != torch.float32 \
-            or mix.numel() != 1:
-        raise ValueError("hidden must be float32 [B, D] and mix a one-element float32 tensor")
-    if normalized.shape != (batch, dim) or next_norm_weight.dtype != torch.float32 \
-            or next_norm_bias.dtype != torch.float32 or next_norm_weight.numel() != dim:
-        raise ValueError("normalized must be [B, D] and the next LayerNorm parameters float32 [D]")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_norm_reduce(
-            _abi.ptr(raw), _abi.ptr(partner_scores), _abi.ptr(norm_weight), _abi.ptr(norm_bias),
-            _abi.ptr(position), None, float(norm_eps), None, _abi.ptr(hidden), _abi.ptr(mix),
-            _abi.ptr(next_norm_weight), _abi.ptr(next_norm_bias), float(next_norm_eps),
-            _abi.ptr(normalized), _abi.code(normalized), 1, 0, None, batch, k_out, dim, _abi.code(raw),
-            _abi.same_dtype("norm parameter", norm_weight, norm_bias),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _relation_norm_reduce_residual_norm(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix,
+                                        next_norm_weight, next_norm_bias, next_norm_eps, normalized)
 
 
-@relation_norm_reduce_residual_norm.register_fake
+@torch.library.register_fake("relation_lm::relation_norm_reduce_residual_norm")
 def _(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix, next_norm_weight,
       next_norm_bias, next_norm_eps, normalized):
     return None
@@ -617,8 +420,6 @@ def _(relation_hidden, second_weight, second_bias, partner_scores, norm_weight, 
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_hidden_cached_rows", mutates_args=(),
-                         device_types="cuda")
 def relation_hidden_cached_rows(
     expanded_cache: Tensor,
     operand_cache: Tensor,
@@ -630,36 +431,16 @@ def relation_hidden_cached_rows(
     """Per-row form of ``relation_hidden_cached`` (extension, prefill): query row ``i`` gathers
     from sequence ``row_batch[i]`` of caches ``[B, T, ...]``; ``anchor_index [N]``,
     ``partner_index [N, K]``; returns ``[N, K, H]`` fp32."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, product_weight=product_weight, row_batch=row_batch)
-    n_seq, max_t, rdim = operand_cache.shape
-    rows, k_out = partner_index.shape
-    hdim = product_weight.size(0)
-    _check_indices(anchor_index, partner_index, rows)
-    if row_batch.dtype != torch.int32 or row_batch.numel() != rows:
-        raise ValueError("row_batch must be int32 with one entry per query row")
-    if expanded_cache.shape != (n_seq, max_t, 2 * hdim) or product_weight.size(1) != rdim:
-        raise ValueError("expanded_cache must be [B, T, 2H] and product_weight [H, R]")
-    out = torch.empty((rows, k_out, hdim), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cached(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(product_weight), _abi.ptr(row_batch), _abi.ptr(out),
-            rows, n_seq, max_t, rdim, hdim, k_out,
-            _abi.same_dtype("cache", expanded_cache, operand_cache), _abi.code(product_weight),
-            _abi.code(out), _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-    return out
+    return _relation_hidden_cached_rows(expanded_cache, operand_cache, anchor_index, partner_index, product_weight,
+                                        row_batch)
 
 
-@relation_hidden_cached_rows.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cached_rows")
 def _(expanded_cache, operand_cache, anchor_index, partner_index, product_weight, row_batch):
     return operand_cache.new_empty(
         (partner_index.size(0), partner_index.size(1), product_weight.size(0)), dtype=torch.float32)
 
 
-@torch.library.custom_op("relation_lm::relation_hidden_cached_rows_out", mutates_args=("out",),
-                         device_types="cuda")
 def relation_hidden_cached_rows_out(
     out: Tensor,
     expanded_cache: Tensor,
@@ -672,34 +453,15 @@ def relation_hidden_cached_rows_out(
     """``relation_hidden_cached_rows`` into a caller-owned ``out [N, K, H]`` of any float dtype: a
     prefill pass over thousands of rows keeps the hidden states in 16 bits (half the bytes of the
     fp32 form, and the dtype the second relation-MLP layer's tensor-core GEMM reads)."""
-    device = _abi.require_cuda_contiguous(
-        out=out, expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, product_weight=product_weight, row_batch=row_batch)
-    n_seq, max_t, rdim = operand_cache.shape
-    rows, k_out = partner_index.shape
-    hdim = product_weight.size(0)
-    _check_indices(anchor_index, partner_index, rows)
-    if row_batch.dtype != torch.int32 or row_batch.numel() != rows:
-        raise ValueError("row_batch must be int32 with one entry per query row")
-    if expanded_cache.shape != (n_seq, max_t, 2 * hdim) or product_weight.size(1) != rdim \
-            or out.shape != (rows, k_out, hdim):
-        raise ValueError("expanded_cache must be [B, T, 2H], product_weight [H, R] and out [N, K, H]")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_hidden_cached(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index),
-            _abi.ptr(partner_index), _abi.ptr(product_weight), _abi.ptr(row_batch), _abi.ptr(out),
-            rows, n_seq, max_t, rdim, hdim, k_out,
-            _abi.same_dtype("cache", expanded_cache, operand_cache), _abi.code(product_weight),
-            _abi.code(out), _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _relation_hidden_cached_rows_out(out, expanded_cache, operand_cache, anchor_index, partner_index, product_weight,
+                                     row_batch)
 
 
-@relation_hidden_cached_rows_out.register_fake
+@torch.library.register_fake("relation_lm::relation_hidden_cached_rows_out")
 def _(out, expanded_cache, operand_cache, anchor_index, partner_index, product_weight, row_batch):
     return None
 
 
-@torch.library.custom_op("relation_lm::relation_norm_reduce_rows", mutates_args=(),
-                         device_types="cuda")
 def relation_norm_reduce_rows(
     raw: Tensor,
     partner_scores: Tensor,
@@ -710,28 +472,58 @@ def relation_norm_reduce_rows(
 ) -> Tensor:
     """Per-row form of ``relation_norm_reduce`` (extension, prefill): row ``i`` uses the active-K
     limit of position ``row_position[i]``."""
-    device = _abi.require_cuda_contiguous(raw=raw, partner_scores=partner_scores,
-                                          norm_weight=norm_weight, norm_bias=norm_bias,
-                                          row_position=row_position)
-    rows, k_out, dim = raw.shape
-    if partner_scores.shape != (rows, k_out) or partner_scores.dtype != torch.float32:
-        raise ValueError("partner_scores must be float32 [N, K]")
-    if row_position.dtype != torch.int32 or row_position.numel() != rows:
-        raise ValueError("row_position must be int32 with one entry per row")
-    out = torch.empty((rows, dim), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_norm_reduce(
-            _abi.ptr(raw), _abi.ptr(partner_scores), _abi.ptr(norm_weight), _abi.ptr(norm_bias),
-            None, _abi.ptr(row_position), float(norm_eps), _abi.ptr(out), None, None, None, None, 0.0,
-            None, 0, 1, 0, None, rows, k_out,
-            dim, _abi.code(raw), _abi.same_dtype("norm parameter", norm_weight, norm_bias),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-    return out
+    return _relation_norm_reduce_rows(raw, partner_scores, norm_weight, norm_bias, row_position, norm_eps)
 
 
-@relation_norm_reduce_rows.register_fake
+@torch.library.register_fake("relation_lm::relation_norm_reduce_rows")
 def _(raw, partner_scores, norm_weight, norm_bias, row_position, norm_eps):
     return raw.new_empty((raw.size(0), raw.size(2)), dtype=torch.float32)
+
+
+def relation_mlp_rows_supported(k_out: int, slots: int, relation_dim: int, hidden_dim: int, d_model: int,
+                                dtype: torch.dtype) -> bool:
+    """Whether ``relation_mlp_rows`` serves these sizes."""
+    return dtype in (torch.bfloat16, torch.float16) and bool(_abi.LIB.rlm_relation_mlp_rows_supported(
+        int(k_out), int(slots), int(relation_dim), int(hidden_dim), int(d_model), _abi.DTYPE_CODE[dtype]))
+
+
+def relation_mlp_rows(
+    out: Tensor,
+    expanded_cache: Tensor,
+    operand_cache: Tensor,
+    anchor_index: Tensor,
+    partner_index: Tensor,
+    partner_scores: Tensor,
+    anchor_active: Tensor | None,
+    slot_weight: Tensor | None,
+    scale: Tensor | None,
+    product_weight: Tensor,
+    second_weight: Tensor,
+    second_bias: Tensor,
+    norm_weight: Tensor,
+    norm_bias: Tensor,
+    norm_eps: float,
+    residual: Tensor | None,
+    slots: int,
+    rows_per_seq: int,
+    limit_by_position: bool,
+) -> None:
+    """One launch for the relation MLP of whole sequences (extension): ``relation_hidden_cached_rows`` ->
+    second relation-MLP layer -> ``relation_norm_reduce_rows`` -> ``out = residual + scale * context``, and
+    with ``slot_weight [S]`` / ``anchor_active [N, S]`` the slot mixing of ``slot_mix_residual``.  Query row ``n``
+    is position ``n % rows_per_seq`` of sequence ``n // rows_per_seq``; ``anchor_index [N, S]``,
+    ``partner_index`` / ``partner_scores [N, S, K]`` (``S = slots``), ``out`` / ``residual [N, d]`` fp32 (they may be
+    one tensor).  The hidden states never reach device memory."""
+    _relation_mlp_rows(out, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, anchor_active,
+                       slot_weight, scale, product_weight, second_weight, second_bias, norm_weight, norm_bias, norm_eps,
+                       residual, slots, rows_per_seq, limit_by_position)
+
+
+@torch.library.register_fake("relation_lm::relation_mlp_rows")
+def _(out, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, anchor_active, slot_weight,
+      scale, product_weight, second_weight, second_bias, norm_weight, norm_bias, norm_eps, residual, slots,
+      rows_per_seq, limit_by_position):
+    return None
 
 
 def relation_layer_tail_supported(n_seq: int, k_out: int, relation_dim: int, hidden_dim: int, d_model: int,
@@ -744,8 +536,6 @@ def relation_layer_tail_supported(n_seq: int, k_out: int, relation_dim: int, hid
                                                            _abi.DTYPE_CODE[dtype]))
 
 
-@torch.library.custom_op("relation_lm::relation_layer_tail", mutates_args=("hidden", "normalized", "query"),
-                         device_types="cuda")
 def relation_layer_tail(
     expanded_cache: Tensor,
     operand_cache: Tensor,
@@ -774,50 +564,12 @@ def relation_layer_tail(
     ``query_weight [NQ, d]`` is given, ``query = normalized @ query_weight.T``.  The relation hidden
     states never reach device memory and no library GEMM is called.  Caches and weights share
     bfloat16 or float16; ``hidden [B, d]`` and all LayerNorm parameters are fp32."""
-    device = _abi.require_cuda_contiguous(
-        expanded_cache=expanded_cache, operand_cache=operand_cache, anchor_index=anchor_index,
-        partner_index=partner_index, partner_scores=partner_scores, product_weight=product_weight,
-        second_weight=second_weight, second_bias=second_bias, norm_weight=norm_weight, norm_bias=norm_bias,
-        hidden=hidden, mix=mix, next_norm_weight=next_norm_weight, next_norm_bias=next_norm_bias,
-        normalized=normalized, query_weight=query_weight, query=query)
-    _abi.require_position(position, device)
-    batch, max_t, rdim = operand_cache.shape
-    hdim, dim = product_weight.size(0), second_weight.size(0)
-    k_out = partner_index.size(1)
-    if expanded_cache.shape != (batch, max_t, 2 * hdim) or product_weight.shape != (hdim, rdim) \
-            or second_weight.shape != (dim, hdim) or second_bias.numel() != dim \
-            or anchor_index.shape != (batch,) or partner_index.shape != (batch, k_out) \
-            or partner_scores.shape != (batch, k_out) or hidden.shape != (batch, dim) \
-            or normalized.shape != (batch, dim):
-        raise ValueError("relation_layer_tail: inconsistent shapes")
-    if anchor_index.dtype != torch.int32 or partner_index.dtype != torch.int32:
-        raise ValueError("index tensors must be int32")
-    for name, t in (("partner_scores", partner_scores), ("hidden", hidden), ("mix", mix),
-                    ("norm_weight", norm_weight), ("norm_bias", norm_bias),
-                    ("next_norm_weight", next_norm_weight), ("next_norm_bias", next_norm_bias)):
-        if t.dtype != torch.float32:
-            raise ValueError(f"{name} must be float32")
-    n_query = 0
-    if query_weight is not None:
-        if query is None or query_weight.dim() != 2 or query_weight.size(1) != dim \
-                or query.shape != (batch, query_weight.size(0)):
-            raise ValueError("query_weight [NQ, d] needs an output query [B, NQ]")
-        n_query = query_weight.size(0)
-    sixteen = [expanded_cache, operand_cache, product_weight, second_weight, second_bias, normalized]
-    if query_weight is not None:
-        sixteen += [query_weight, query]
-    dtype = _abi.same_dtype("16-bit operand", *sixteen)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_relation_layer_tail(
-            _abi.ptr(expanded_cache), _abi.ptr(operand_cache), _abi.ptr(anchor_index), _abi.ptr(partner_index),
-            _abi.ptr(partner_scores), _abi.ptr(product_weight), _abi.ptr(second_weight), _abi.ptr(second_bias),
-            _abi.ptr(norm_weight), _abi.ptr(norm_bias), _abi.ptr(position), float(norm_eps), _abi.ptr(hidden),
-            _abi.ptr(mix), _abi.ptr(next_norm_weight), _abi.ptr(next_norm_bias), float(next_norm_eps),
-            _abi.ptr(normalized), _abi.ptr(query_weight), _abi.ptr(query), batch, k_out, max_t, rdim, hdim,
-            dim, n_query, dtype, _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _relation_layer_tail(expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight,
+                         second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, hidden, mix,
+                         next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query)
 
 
-@relation_layer_tail.register_fake
+@torch.library.register_fake("relation_lm::relation_layer_tail")
 def _(expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight,
       second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, hidden, mix,
       next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query):

@@ -11,12 +11,15 @@ from torch import Tensor
 
 from relation_lm.kernels import _abi
 
+# The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
+_router_cache_update = torch.ops.relation_lm.router_cache_update.default
+_sparse_cache_append = torch.ops.relation_lm.sparse_cache_append.default
+_router_cache_prefill = torch.ops.relation_lm.router_cache_prefill.default
+
 _MUTATED = ("anchor_raw_cache", "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache",
             "anchor_mean", "anchor_std", "partner_mean", "partner_std")
 
 
-@torch.library.custom_op("relation_lm::router_cache_update", mutates_args=_MUTATED,
-                         device_types="cuda")
 def router_cache_update(
     anchor_raw: Tensor,
     partner_raw: Tensor,
@@ -37,38 +40,12 @@ def router_cache_update(
     mean / biased std for both streams.  ``anchor_raw`` / ``partner_raw`` may be column slices
     of a wider packed projection (row stride is honoured, inner stride must be 1).
     Returns the convolved keys ``[B, 2, 64]`` in fp32."""
-    device = _abi.require_cuda_contiguous(
-        anchor_raw_cache=anchor_raw_cache, partner_raw_cache=partner_raw_cache,
-        anchor_conv_cache=anchor_conv_cache, partner_conv_cache=partner_conv_cache,
-        anchor_mean=anchor_mean, anchor_std=anchor_std, partner_mean=partner_mean,
-        partner_std=partner_std, anchor_conv_weight=anchor_conv_weight,
-        partner_conv_weight=partner_conv_weight)
-    for name, raw in (("anchor_raw", anchor_raw), ("partner_raw", partner_raw)):
-        if raw.device != device or raw.dim() != 2 or raw.size(1) != 64 or raw.stride(1) != 1:
-            raise ValueError(f"{name} must be a [B, 64] CUDA tensor with unit inner stride")
-    _abi.require_position(position, device)
-    batch = anchor_raw.size(0)
-    if anchor_raw_cache.size(2) != 64 or anchor_mean[0, 0].numel() != 64:
-        raise ValueError("this build supports router width 64")
-    out = torch.empty((batch, 2, 64), device=device, dtype=torch.float32)
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_router_cache_update(
-            _abi.ptr(anchor_raw), anchor_raw.stride(0), _abi.ptr(partner_raw), partner_raw.stride(0),
-            _abi.ptr(anchor_raw_cache), _abi.ptr(partner_raw_cache), _abi.ptr(anchor_conv_cache),
-            _abi.ptr(partner_conv_cache), _abi.ptr(anchor_mean), _abi.ptr(anchor_std),
-            _abi.ptr(partner_mean), _abi.ptr(partner_std), _abi.ptr(anchor_conv_weight),
-            _abi.ptr(partner_conv_weight), _abi.ptr(position), _abi.ptr(out), batch,
-            anchor_raw_cache.size(1), anchor_mean.size(1), int(block_size),
-            _abi.same_dtype("raw key", anchor_raw, partner_raw),
-            _abi.same_dtype("router cache", anchor_raw_cache, partner_raw_cache,
-                            anchor_conv_cache, partner_conv_cache),
-            _abi.same_dtype("block statistics", anchor_mean, anchor_std, partner_mean, partner_std),
-            _abi.same_dtype("conv weight", anchor_conv_weight, partner_conv_weight),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
-    return out
+    return _router_cache_update(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_cache,
+                                partner_conv_cache, anchor_mean, anchor_std, partner_mean, partner_std,
+                                anchor_conv_weight, partner_conv_weight, position, block_size)
 
 
-@router_cache_update.register_fake
+@torch.library.register_fake("relation_lm::router_cache_update")
 def _(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_cache,
       partner_conv_cache, anchor_mean, anchor_std, partner_mean, partner_std,
       anchor_conv_weight, partner_conv_weight, position, block_size):
@@ -78,8 +55,6 @@ def _(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_
 _APPEND_MUTATED = ("anchor_keys", "partner_keys", "operand_cache", "partner_anchor_cache") + _MUTATED
 
 
-@torch.library.custom_op("relation_lm::sparse_cache_append", mutates_args=_APPEND_MUTATED,
-                         device_types="cuda")
 def sparse_cache_append(
     packed: Tensor,
     anchor_keys: Tensor,
@@ -103,44 +78,18 @@ def sparse_cache_append(
     ``position`` of their caches and update both router streams (extension of
     ``router_cache_update``; every cache carries a leading layer dimension and ``packed`` is
     ``[B, layers * (384 + R)]`` in the packed column order)."""
-    device = _abi.require_cuda_contiguous(
-        anchor_keys=anchor_keys, partner_keys=partner_keys, operand_cache=operand_cache,
-        partner_anchor_cache=partner_anchor_cache, anchor_raw_cache=anchor_raw_cache,
-        partner_raw_cache=partner_raw_cache, anchor_conv_cache=anchor_conv_cache,
-        partner_conv_cache=partner_conv_cache, anchor_mean=anchor_mean, anchor_std=anchor_std,
-        partner_mean=partner_mean, partner_std=partner_std, anchor_conv_weight=anchor_conv_weight,
-        partner_conv_weight=partner_conv_weight)
-    _abi.require_cuda_rows(packed=packed)
-    _abi.require_position(position, device)
-    layers, batch, max_t, rdim = operand_cache.shape
-    if packed.shape != (batch, layers * (384 + rdim)) or anchor_keys.shape != (layers, batch, max_t, 64) \
-            or partner_anchor_cache.shape != (layers, batch, max_t, 128) \
-            or anchor_raw_cache.shape != (layers, batch, max_t, 64) or anchor_mean.size(0) != layers:
-        raise ValueError("caches must be [layers, B, T, width] and packed [B, layers * (384 + R)]")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_sparse_cache_append(
-            _abi.ptr(packed), packed.stride(0), rdim, _abi.ptr(anchor_keys), _abi.ptr(partner_keys),
-            _abi.ptr(operand_cache), _abi.ptr(partner_anchor_cache), _abi.ptr(anchor_raw_cache),
-            _abi.ptr(partner_raw_cache), _abi.ptr(anchor_conv_cache), _abi.ptr(partner_conv_cache),
-            _abi.ptr(anchor_mean), _abi.ptr(anchor_std), _abi.ptr(partner_mean), _abi.ptr(partner_std),
-            _abi.ptr(anchor_conv_weight), _abi.ptr(partner_conv_weight), _abi.ptr(position), None,
-            layers, batch, max_t, anchor_mean.size(2), int(block_size), _abi.code(packed),
-            _abi.same_dtype("cache", anchor_keys, partner_keys, operand_cache, partner_anchor_cache,
-                            anchor_raw_cache, partner_raw_cache, anchor_conv_cache, partner_conv_cache),
-            _abi.same_dtype("block statistics", anchor_mean, anchor_std, partner_mean, partner_std),
-            _abi.same_dtype("conv weight", anchor_conv_weight, partner_conv_weight),
-            _abi.ptr(_abi.status_tensor(device)), _abi.stream_ptr(device)))
+    _sparse_cache_append(packed, anchor_keys, partner_keys, operand_cache, partner_anchor_cache, anchor_raw_cache,
+                         partner_raw_cache, anchor_conv_cache, partner_conv_cache, anchor_mean, anchor_std,
+                         partner_mean, partner_std, anchor_conv_weight, partner_conv_weight, position, block_size)
 
 
-@sparse_cache_append.register_fake
+@torch.library.register_fake("relation_lm::sparse_cache_append")
 def _(packed, anchor_keys, partner_keys, operand_cache, partner_anchor_cache, anchor_raw_cache,
       partner_raw_cache, anchor_conv_cache, partner_conv_cache, anchor_mean, anchor_std,
       partner_mean, partner_std, anchor_conv_weight, partner_conv_weight, position, block_size):
     return None
 
 
-@torch.library.custom_op("relation_lm::router_cache_prefill", mutates_args=_MUTATED,
-                         device_types="cuda")
 def router_cache_prefill(
     anchor_raw: Tensor,
     partner_raw: Tensor,
@@ -159,35 +108,12 @@ def router_cache_prefill(
     """Fill zero-initialised router caches and block statistics for a whole prefix
     ``anchor_raw, partner_raw [B, length, 64]`` in one launch (extension); the state equals that
     of ``length`` successive ``router_cache_update`` calls."""
-    device = _abi.require_cuda_contiguous(
-        anchor_raw_cache=anchor_raw_cache, partner_raw_cache=partner_raw_cache,
-        anchor_conv_cache=anchor_conv_cache, partner_conv_cache=partner_conv_cache,
-        anchor_mean=anchor_mean, anchor_std=anchor_std, partner_mean=partner_mean,
-        partner_std=partner_std, anchor_conv_weight=anchor_conv_weight,
-        partner_conv_weight=partner_conv_weight)
-    for name, raw in (("anchor_raw", anchor_raw), ("partner_raw", partner_raw)):
-        if raw.device != device or raw.dim() != 3 or raw.size(2) != 64 or raw.stride(2) != 1:
-            raise ValueError(f"{name} must be a [B, length, 64] CUDA tensor with unit inner stride")
-    batch, length = anchor_raw.size(0), anchor_raw.size(1)
-    if partner_raw.shape != anchor_raw.shape:
-        raise ValueError("anchor_raw and partner_raw must have the same shape")
-    with _abi.device_guard(device):
-        _abi.check(_abi.LIB.rlm_router_cache_prefill(
-            _abi.ptr(anchor_raw), anchor_raw.stride(1), anchor_raw.stride(0), _abi.ptr(partner_raw),
-            partner_raw.stride(1), partner_raw.stride(0), _abi.ptr(anchor_raw_cache),
-            _abi.ptr(partner_raw_cache), _abi.ptr(anchor_conv_cache), _abi.ptr(partner_conv_cache),
-            _abi.ptr(anchor_mean), _abi.ptr(anchor_std), _abi.ptr(partner_mean), _abi.ptr(partner_std),
-            _abi.ptr(anchor_conv_weight), _abi.ptr(partner_conv_weight), length, batch,
-            anchor_raw_cache.size(1), anchor_mean.size(1), int(block_size),
-            _abi.same_dtype("raw key", anchor_raw, partner_raw),
-            _abi.same_dtype("router cache", anchor_raw_cache, partner_raw_cache,
-                            anchor_conv_cache, partner_conv_cache),
-            _abi.same_dtype("block statistics", anchor_mean, anchor_std, partner_mean, partner_std),
-            _abi.same_dtype("conv weight", anchor_conv_weight, partner_conv_weight),
-            _abi.stream_ptr(device)))
+    _router_cache_prefill(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_cache,
+                          partner_conv_cache, anchor_mean, anchor_std, partner_mean, partner_std, anchor_conv_weight,
+                          partner_conv_weight, block_size)
 
 
-@router_cache_prefill.register_fake
+@torch.library.register_fake("relation_lm::router_cache_prefill")
 def _(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_cache,
       partner_conv_cache, anchor_mean, anchor_std, partner_mean, partner_std,
       anchor_conv_weight, partner_conv_weight, block_size):
