@@ -29,6 +29,8 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor, nn
 
+from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
+
 
 @dataclass
 class MultiAnchorConfig:
@@ -187,6 +189,11 @@ class MultiAnchorPrefill:
             raise ValueError("the routed pass runs its projections on the tensor cores: bfloat16 or float16")
         self.config, self.device, self.dtype = stack.config, torch.device(device), dtype
         self.tiled_select = bool(tiled_select)           # whole-sequence selector (bfloat16) instead of the per-row one
+        cfg = stack.config
+        # one launch for the relation MLP, norm-reduce and (slot counts that are powers of two) the slot mixing
+        sizes = (cfg.relation_dim, cfg.hidden_dim, cfg.d_model, dtype)
+        self.fused_mix = relation_mlp_rows_supported(cfg.partners_per_anchor, cfg.anchors_per_block, *sizes)
+        self.fused_mlp = self.fused_mix or relation_mlp_rows_supported(cfg.partners_per_anchor, 1, *sizes)
         self.layers = [stack.layer_weights(l, self.device, dtype) for l in range(stack.config.depth)]
         self.final_norm_w = stack.final_norm.weight.detach().to(self.device, torch.float32)
         self.final_norm_b = stack.final_norm.bias.detach().to(self.device, torch.float32)
@@ -238,7 +245,6 @@ class MultiAnchorPrefill:
         cfg, w = self.config, self.layers[layer]
         B, T, d = hidden.shape
         N, S, K, H = B * T, cfg.anchors_per_block, cfg.partners_per_anchor, cfg.hidden_dim
-        rb, rp = self.rows(B, T)
         normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
         layer_norm_cast(hidden.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
         q = packed_projection(normalized, w["w_query"])                          # [N, S * 256]
@@ -261,10 +267,25 @@ class MultiAnchorPrefill:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
+        fused = self.fused_mlp and keep is None
+        if selected is None or not fused:
+            rb, rp = self.rows(B, T)
         if selected is None:
             selected = relation_select_multi_rows(*select_args, rb, rp, cfg.local_window, cfg.top_blocks, K,
                                                   cfg.strict_valid)
         anchor, anchor_score, anchor_active, partner, partner_score, partner_active = selected
+        if fused:
+            mlp = (state["expanded_cache"], state["operand_cache"], anchor, partner, partner_score)
+            weights = (w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"], cfg.norm_eps)
+            # softmax over the finite partner scores of a slot, no active-K limit
+            if self.fused_mix:
+                relation_mlp_rows(hidden.view(N, d), *mlp, anchor_active, w["slot_weight"], w["gate"], *weights,
+                                  hidden.view(N, d), S, T, False)
+            else:
+                slot_context = torch.empty(N * S, d, device=self.device, dtype=torch.float32)
+                relation_mlp_rows(slot_context, *mlp, None, None, None, *weights, None, 1, T * S, False)
+                slot_mix_residual(slot_context.view(N, S, d), anchor_active, w["slot_weight"], w["gate"], hidden.view(N, d))
+            return hidden
         pair_rows = rb.repeat_interleave(S)
         hidden_rel = torch.empty(N * S, K, H, device=self.device, dtype=self.dtype)
         relation_hidden_cached_rows_out(hidden_rel, state["expanded_cache"], state["operand_cache"],

@@ -27,7 +27,8 @@ from torch import Tensor
 
 from relation_lm.inference.routed_model import RoutedRelationLM
 from relation_lm.kernels.packed_projection import layer_norm_cast, packed_projection
-from relation_lm.kernels.relation_reduce import relation_hidden_cached_rows_out, relation_norm_reduce_rows
+from relation_lm.kernels.relation_reduce import (relation_hidden_cached_rows_out, relation_mlp_rows,
+                                                 relation_mlp_rows_supported, relation_norm_reduce_rows)
 from relation_lm.kernels.relation_select import relation_select_packed_prefill, relation_select_packed_rows
 from relation_lm.kernels.router_cache import router_cache_prefill
 
@@ -43,6 +44,9 @@ class RoutedPrefillLayer:
         self.config, self.layer, self.device, self.dtype = model.config, int(layer), torch.device(device), dtype
         w = model.decode_weights(self.device, dtype)
         cfg, l = self.config, self.layer
+        # the relation MLP, norm-reduce and residual as one launch where its tiles fit (never more than the three
+        # launches it replaces cost, from a few hundred rows up)
+        self.fused_mlp = relation_mlp_rows_supported(cfg.k_max, 1, cfg.relation_dim, cfg.hidden_dim, cfg.d_model, dtype)
         width = cfg.packed_width
         self.w = {
             "memory_norm_w": w["memory_norm_w"], "memory_norm_b": w["memory_norm_b"],
@@ -102,7 +106,6 @@ class RoutedPrefillLayer:
         cfg, w = self.config, self.w
         B, T, d = x.shape
         N, K, H = B * T, cfg.k_max, cfg.hidden_dim
-        rb, rp = self.rows(B, T)
         normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
         layer_norm_cast(x.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
         q = packed_projection(normalized, w["w_query"])
@@ -120,10 +123,19 @@ class RoutedPrefillLayer:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
+        fused = self.fused_mlp and keep is None
+        if selected is None or not fused:
+            rb, rp = self.rows(B, T)
         if selected is None:
             selected = relation_select_packed_rows(*select_args, rb, rp, cfg.local_window, cfg.top_blocks, K,
                                                    cfg.strict_valid)
         anchor, anchor_score, partner, partner_score = selected
+        if fused:
+            out = torch.empty(N, d, device=self.device, dtype=torch.float32)
+            relation_mlp_rows(out, state["expanded_cache"], state["operand_cache"], anchor, partner, partner_score, None, None,
+                              w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"],
+                              cfg.norm_eps, x.view(N, d), 1, T, True)
+            return out.view(B, T, d)
         hidden_rel = torch.empty(N, K, H, device=self.device, dtype=self.dtype)
         relation_hidden_cached_rows_out(hidden_rel, state["expanded_cache"], state["operand_cache"], anchor,
                                         partner, w["product_weight"], rb)

@@ -1,0 +1,117 @@
+"""The one-launch relation MLP of a whole-sequence pass against a plain fp32 PyTorch evaluation of the
+same formulas (operands rounded where the kernel rounds: the products and the hidden states)."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from gpu_util import assert_status_clear
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(dtype, batch, length, slots, k, rdim, d, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s, scale=1.0: torch.randn(*s, generator=g, device="cuda") * scale  # noqa: E731
+    H, N = 4 * d, batch * length
+    x = {
+        "expanded": rn(batch, length, 2 * H, scale=0.5).to(dtype), "operand": rn(batch, length, rdim).to(dtype),
+        "anchor": torch.randint(-1, length, (N, slots), generator=g, device="cuda", dtype=torch.int32),
+        "partner": torch.randint(-3, length, (N, slots, k), generator=g, device="cuda", dtype=torch.int32),
+        "score": rn(N, slots, k, scale=2.0), "active": torch.rand(N, slots, generator=g, device="cuda") < 0.8,
+        "slot_weight": torch.softmax(rn(slots), 0), "scale": rn(1).abs(), "wm": rn(H, rdim, scale=rdim ** -0.5).to(dtype),
+        "w2": rn(d, H, scale=H ** -0.5).to(dtype), "b2": rn(d, scale=0.1), "nw": 1 + rn(d, scale=0.1), "nb": rn(d, scale=0.1),
+        "residual": rn(N, d),
+    }
+    x["score"][torch.rand(N, slots, k, generator=g, device="cuda") < 0.15] = -torch.inf
+    return x
+
+
+def _expected(x, length, limited, mixed):
+    dtype = x["operand"].dtype
+    N, S, K = x["score"].shape
+    d = x["w2"].size(0)
+    n = torch.arange(N, device="cuda")
+    seq, t = n // length, n % length
+    a = x["anchor"].long().clamp(0, length - 1)
+    p = x["partner"].long().clamp(0, length - 1)
+    out = torch.empty(N, d, device="cuda")
+    wm, w2 = x["wm"].float(), x["w2"].float()
+    H = wm.size(0)
+    for lo in range(0, N, 256):
+        r = slice(lo, min(N, lo + 256))
+        op, ex = x["operand"][seq[r]].float(), x["expanded"][seq[r]].float()          # [n, T, .]
+        rows = torch.arange(op.size(0), device="cuda")
+        oa, ea = op[rows[:, None], a[r]], ex[rows[:, None], a[r]][..., :H]            # [n, S, .]
+        pp = p[r].reshape(op.size(0), -1)
+        opp = op[rows[:, None], pp].view(-1, S, K, op.size(-1))
+        epp = ex[rows[:, None], pp][..., H:].reshape(-1, S, K, H)
+        prod = (oa[:, :, None] * opp).to(dtype).float()
+        hid = torch.nn.functional.gelu(prod @ wm.T + ea[:, :, None] + epp).to(dtype).float()
+        raw = torch.nn.functional.layer_norm(hid @ w2.T + x["b2"], (d,), x["nw"], x["nb"], 1e-5)
+        s = x["score"][r]
+        live = torch.isfinite(s)
+        if limited:
+            limit = torch.ceil(torch.log2(t[r].double() + 2)).clamp(1, K)
+            live &= torch.arange(K, device="cuda")[None, None] < limit[:, None, None]
+        e = torch.where(live, torch.exp(s - torch.where(live, s, -1e4).amax(-1, keepdim=True)), 0.0)
+        u = e / e.sum(-1, keepdim=True).clamp_min(1e-9)
+        if mixed:
+            w = torch.where(x["active"][r], x["slot_weight"], 0.0)
+            u = u * (w / w.sum(-1, keepdim=True).clamp_min(1e-9))[..., None]
+        out[r] = x["residual"][r] + x["scale"] * (u[..., None] * raw).sum((1, 2))
+    return out
+
+
+# d on both sides of one output part per cluster, tiles of one / several rows, ragged last tiles, every group size
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("batch,length,slots,k,rdim,d,limited", [
+    (1, 3, 1, 8, 128, 512, True), (2, 37, 1, 8, 128, 512, True), (3, 50, 4, 4, 128, 512, False), (1, 129, 1, 4, 64, 256, True),
+    (2, 33, 2, 8, 128, 256, False), (1, 70, 1, 8, 128, 768, True), (1, 21, 4, 8, 128, 768, False), (1, 40, 1, 2, 128, 64, True),
+    (1, 19, 1, 16, 64, 384, True), (2, 45, 8, 2, 128, 128, False), (5, 700, 1, 8, 128, 512, True), (4, 900, 1, 8, 128, 256, True),
+    (3, 600, 4, 4, 128, 512, False), (3, 800, 1, 8, 128, 768, True),
+])
+def test_matches_the_composition(dtype, batch, length, slots, k, rdim, d, limited):
+    from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
+
+    assert relation_mlp_rows_supported(k, slots, rdim, 4 * d, d, dtype)
+    x = _case(dtype, batch, length, slots, k, rdim, d, seed=d + 7 * k + length)
+    mixed = slots > 1
+    out = x["residual"].clone()
+    relation_mlp_rows(out, x["expanded"], x["operand"], x["anchor"], x["partner"], x["score"], x["active"] if mixed else None,
+                      x["slot_weight"] if mixed else None, x["scale"], x["wm"], x["w2"], x["b2"], x["nw"], x["nb"], 1e-5,
+                      out, slots, length, limited)
+    assert_status_clear()
+    want = _expected(x, length, limited, mixed)
+    # fp32 accumulation on both sides; what differs is GELU's last bits, which move a hidden state by one
+    # rounding step (2^-8 in bf16, 2^-11 in fp16) now and then: far below one step once LayerNorm has averaged
+    bound = 4e-3 if dtype == torch.bfloat16 else 1e-3
+    context, expected = (out - x["residual"]) / x["scale"], (want - x["residual"]) / x["scale"]
+    assert float((context - expected).abs().max()) <= bound * float(expected.abs().max().clamp_min(1.0))
+
+
+def test_new_output_without_residual_or_scale():
+    from relation_lm.kernels.relation_reduce import relation_mlp_rows
+
+    x = _case(torch.bfloat16, 2, 40, 1, 8, 128, 512, seed=9)
+    out = torch.full_like(x["residual"], float("nan"))
+    relation_mlp_rows(out, x["expanded"], x["operand"], x["anchor"], x["partner"], x["score"], None, None, None, x["wm"],
+                      x["w2"], x["b2"], x["nw"], x["nb"], 1e-5, None, 1, 40, True)
+    x["residual"].zero_()
+    x["scale"].fill_(1.0)
+    want = _expected(x, 40, True, False)
+    assert float((out - want).abs().max()) <= 4e-3 * float(want.abs().max())
+    assert_status_clear()
+
+
+def test_sizes_outside_the_range_are_refused():
+    from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
+
+    assert not relation_mlp_rows_supported(6, 1, 128, 2048, 512, torch.bfloat16)
+    assert not relation_mlp_rows_supported(8, 8, 128, 2048, 512, torch.bfloat16)
+    assert not relation_mlp_rows_supported(8, 1, 128, 4096, 1024, torch.bfloat16)
+    assert not relation_mlp_rows_supported(8, 1, 128, 2048, 512, torch.float32)
+    x = _case(torch.bfloat16, 1, 8, 1, 6, 128, 128, seed=3)
+    with pytest.raises(ValueError):
+        relation_mlp_rows(x["residual"], x["expanded"], x["operand"], x["anchor"], x["partner"], x["score"], None, None, None,
+                          x["wm"], x["w2"], x["b2"], x["nw"], x["nb"], 1e-5, None, 1, 8, True)
