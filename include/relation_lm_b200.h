@@ -700,7 +700,7 @@ int rlm_selftest_bounded_wait(int32_t* status, int64_t cycle_limit, int64_t* wai
  * softmax over a slot's partners with finite scores — with limit_by_position also k < clamp(ceil(log2(t + 2)), 1, K) —
  * times the slot's weight, renormalised over the row's active slots.  scale: one fp32 element, NULL = 1;
  * residual: NULL = 0, and may be `out` itself.  Caches and weights share bf16 or fp16; second_bias, LayerNorm
- * parameters, residual and out are fp32.  _supported: k_out and slots powers of two with 2 <= k_out, k_out * slots <= 32,
+ * parameters, residual and out are fp32.  _supported: k_out and slots powers of two with 4 <= k_out <= 16, k_out * slots <= 32,
  * relation_dim 64 or 128, d_model a multiple of 64 up to 384 or of 128 up to 768.
  */
 int rlm_relation_mlp_rows_supported(int k_out, int slots, int relation_dim, int hidden_dim, int d_model, int dtype);

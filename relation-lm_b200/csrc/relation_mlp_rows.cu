@@ -19,22 +19,29 @@
 // computes every C-th block of 64 hidden columns, which it passes on to the other through distributed
 // shared memory (one bulk copy per 32 rows, completing on the receiver's mbarrier).
 //
-// kG = 2 pairs the tiles of two neighbouring CTAs on tcgen05.mma.cta_group::2 (256 pair rows, each CTA
-// holding half of the weight rows): what bounds the kernel with kG = 1 is the stream of W_2 out of L2 —
-// 2.5 MB of weights per 128 pairs — and pairing halves it.
+// The tiles of two neighbouring CTAs are paired on tcgen05.mma.cta_group::2 (256 pair rows, each CTA holding
+// half of the weight rows): every 128 pairs otherwise stream 2.5 MB of weights out of L2, more than its
+// bandwidth allows at the tensor cores' rate; pairing halves it.
 //
-// One CTA (24 warps), a persistent loop over tiles:
-//   warps 0-15   epilogue: thread = pair row x 16 hidden columns per block; then the LayerNorm and
-//                the weighted sum of the finished tile (thread = pair row x a quarter of the columns)
-//   warps 16, 19 TMA producers of W_2 and of W_m tiles (apart: a full W_2 ring must not hold up W_m)
-//   warps 17, 18 tcgen05.mma issue of the first and of the second layer (the first CTA of a pair; in the
+// The expanded-cache terms join the first layer's accumulator as matrix products, so that the epilogue is GELU
+// and nothing else: the partners' segments, gathered as a 128 x 64 block in operand layout, times the identity,
+// and the anchors' segments selected by a one-hot matrix.  Both are exact in the fp32 accumulator.  (Added
+// in the epilogue instead they cost a third of its instructions, and the epilogue was the bound.)
+//
+// One CTA (32 warps, registers shifted to the epilogue by setmaxnreg), a persistent loop over tiles:
+//   warps 0-15   epilogue: thread = pair row x 32 columns of a hidden block; then the LayerNorm and the
+//                weighted sum of the finished tile (thread = pair row x a quarter of the columns)
+//   warps 16, 17 TMA producers of W_2 and of W_m tiles (apart: a full W_2 ring must not hold up W_m)
+//   warps 18, 19 tcgen05.mma issue of the first and of the second layer (the first CTA of a pair; in the
 //                second they forward its barriers to the first)
-//   warps 20-23  gathers: operand products into the A tile of the next tile, and for every block the
-//                expanded-cache segments of its pairs
-// Pipelines: two hidden blocks per part in flight (one per epilogue group), two accumulators for the first
-// layer, rings of gathered segments, W_m and W_2 tiles.  (Gathering into the hidden block that the epilogue
-// then overwrites saved 16 KB per block, but put a gather's latency behind the second layer's last use of
-// that block: 2 450 cycles per block of 64 hidden columns at three blocks in flight.)  Every wait is bounded; on expiry the kernel sets RLM_DEV_TIMEOUT, drains and returns.
+//   warps 20-23  gathers of the expanded-cache segments (cp.async; as TMA row gathers, tile::gather4, a block of
+//                128 + 32 rows took 3 500 cycles instead of 1 000)
+//   warps 24-31  indices, weights u, and the operand products of the next tile (the A tile): in registers
+//                while the current tile runs, into shared memory the moment its last product is done
+// Hidden columns go in units of 128 (two blocks of 64, one per epilogue group): up to 256 output columns per
+// CTA leave tensor memory for two units of the first layer's accumulator, more for one, which is then
+// handed over block by block.  Every wait is bounded; on expiry the kernel sets RLM_DEV_TIMEOUT, drains
+// and returns.
 
 #include <map>
 #include <mutex>
@@ -47,10 +54,13 @@ namespace {
 
 constexpr int kMlpEpiWarps = 16;
 constexpr int kMlpGatherWarps = 4;
-constexpr int kMlpThreads = 32 * (kMlpEpiWarps + 4 + kMlpGatherWarps);
+constexpr int kMlpOperandWarps = 8;
+constexpr int kMlpThreads = 32 * (kMlpEpiWarps + 4 + kMlpGatherWarps + kMlpOperandWarps);
+// Registers per thread by warpgroup after start-up; launched with 64 each, 8 warpgroups: 4 * 80 + 2 * 40 + 2 * 56 = 8 * 64.
+constexpr int kMlpEpiRegs = 80, kMlpIssueRegs = 40, kMlpOperandRegs = 56;
+constexpr int kG = 2;                            // CTAs whose MMAs are paired
 constexpr int kMlpHC = 64;                       // hidden columns per block: one 128-byte swizzle atom of K
 constexpr uint32_t kMlpBlock = kBM * 128u;       // a 128 x 64 16-bit block
-constexpr uint32_t kMlpAncStride = 144;          // padded anchor-term row: conflict-free for rows of different anchors
 constexpr int kMlpMaxStages = 4;
 constexpr int kMlpHidden = 2;                    // hidden blocks in flight per part
 constexpr int kMlpMaxTerms = 4;                  // gathered blocks in flight
@@ -75,40 +85,48 @@ struct MlpArgs {
     int n_pairs, n_tiles;            // tiles of 128 pairs
     int cols;                        // output columns per CTA (NC)
     int term_stages, w2_stages, wm_stages;
-    uint32_t idesc1, idesc2;
+    int wide;                        // the first layer in units of 128 columns (else blocks of 64)
+    float inv_d;
+    uint32_t idesc_block, idesc_unit, idesc2;
 };
 
 // Shared-memory plan (byte offsets from the 1024-aligned dynamic base).
 struct MlpPlan {
-    uint32_t a, wm, w2, hid, term, anc, bias, gamma, beta, stats, u, prow, arow, total;
+    uint32_t a, wm, w2, hid, term, anc, onehot, ident, bias, gamma, beta, stats, u, prow, arow, total;
 };
 
-__host__ __device__ inline MlpPlan mlp_plan(int rdim, int cols, int outs, int group_ctas, int term_stages, int wm_stages,
+// Anchor segments of one block: the anchors of both of the pair's tiles, this CTA's half of the columns.
+__host__ __device__ inline uint32_t mlp_anchor_bytes(int k_shift) { return 2u * (kBM >> k_shift) * (kMlpHC / 2) * 2u; }
+
+__host__ __device__ inline MlpPlan mlp_plan(int rdim, int cols, int outs, int wide, int term_stages, int wm_stages,
                                             int w2_stages, int k_shift) {
     MlpPlan p;
     uint32_t off = 0;
     p.a = off;      off += static_cast<uint32_t>(rdim / kBK) * kMlpBlock;
-    p.wm = off;     off += static_cast<uint32_t>(wm_stages * (rdim / kBK)) * (kMlpHC / group_ctas) * 128u;
-    p.w2 = off;     off += static_cast<uint32_t>(w2_stages) * ((cols > 256 ? cols / 2 : cols) / group_ctas) * 128u;
+    p.wm = off;     off += static_cast<uint32_t>(wm_stages * (rdim / kBK)) * ((wide ? 2 : 1) * kMlpHC / kG) * 128u;
+    p.w2 = off;     off += static_cast<uint32_t>(w2_stages) * ((cols > 256 ? cols / 2 : cols) / kG) * 128u;
     p.hid = off;    off += static_cast<uint32_t>(kMlpHidden * outs) * kMlpBlock;
     p.term = off;   off += static_cast<uint32_t>(term_stages) * kMlpBlock;
-    p.anc = off;    off += static_cast<uint32_t>(term_stages) * (kBM >> k_shift) * kMlpAncStride;
+    p.anc = off;    off += static_cast<uint32_t>(term_stages) * mlp_anchor_bytes(k_shift);
+    off = (off + 1023u) & ~1023u;
+    p.onehot = off; off += kBM * (2u * (kBM >> k_shift)) * 2u;
+    off = (off + 1023u) & ~1023u;
+    p.ident = off;  off += (kMlpHC / 2) * 128u;
     p.bias = off;   off += static_cast<uint32_t>(cols) * 4u;
     p.gamma = off;  off += static_cast<uint32_t>(cols) * 4u;
     p.beta = off;   off += static_cast<uint32_t>(cols) * 4u;
     p.stats = off;  off += static_cast<uint32_t>(4 * outs) * kBM * 8u;
     p.u = off;      off += 3u * kBM * 4u;
     p.prow = off;   off += 2u * kBM * 4u;
-    p.arow = off;   off += 2u * (kBM >> k_shift) * 4u;
+    p.arow = off;   off += 4u * (kBM >> k_shift) * 4u;
     p.total = off;
     return p;
 }
 
 struct MlpBars {
-    unsigned long long a_full, a_empty, d2_full, d2_empty, stats_full;
-    unsigned long long u_full[3], d1_full[2], d1_empty[2];
-    unsigned long long wm_full[2], wm_empty[2], peer_wm[2];
-    unsigned long long w2_full[kMlpMaxStages], w2_empty[kMlpMaxStages], peer_w2[kMlpMaxStages];
+    unsigned long long a_full, a_empty, d2_full, d2_empty, stats_full, rows_full[2], u_full[3];
+    unsigned long long d1_full[2], d1_empty[2], wm_full[2], wm_empty[2];
+    unsigned long long w2_full[kMlpMaxStages], w2_empty[kMlpMaxStages];
     unsigned long long hid_full[kMlpHidden][2], hid_empty[kMlpHidden];
     unsigned long long term_full[kMlpMaxTerms], term_empty[kMlpMaxTerms];
 };
@@ -142,10 +160,10 @@ __device__ __forceinline__ void mlp_expect_remote(uint32_t remote_bar, uint32_t 
     asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(remote_bar), "r"(bytes) : "memory");
 }
 // Arrives at the pair leader's barrier at the same offset.
-template <int kG>
-__device__ __forceinline__ void mlp_arrive_leader(uint32_t bar, uint32_t leader) {
-    if (kG == 1) mlp_arrive(bar);
-    else mlp_arrive_remote(mlp_peer(bar, leader));
+__device__ __forceinline__ void mlp_arrive_leader(uint32_t bar, uint32_t leader) { mlp_arrive_remote(mlp_peer(bar, leader)); }
+// Completes `bar` once this thread's cp.async copies so far have landed (one of its expected arrivals).
+__device__ __forceinline__ void mlp_cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mlp_copy_cluster(uint32_t remote_dst, uint32_t src, uint32_t bytes, uint32_t remote_bar) {
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -155,10 +173,6 @@ __device__ __forceinline__ void mlp_copy_cluster(uint32_t remote_dst, uint32_t s
 __device__ __forceinline__ void mlp_store_remote(uint32_t remote_dst, float x, float y, uint32_t remote_bar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
                  ::"r"(remote_dst), "f"(x), "f"(y), "r"(remote_bar) : "memory");
-}
-// Completes `bar` once this thread's cp.async copies so far have landed (one of its expected arrivals).
-__device__ __forceinline__ void mlp_cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 template <bool kCluster>
 __device__ __forceinline__ bool mlp_try_wait(uint32_t bar, uint32_t parity) {
@@ -188,15 +202,19 @@ __device__ __forceinline__ bool mlp_wait(uint32_t bar, uint32_t parity, volatile
     }
     return false;
 }
+template <int kRegs>
+__device__ __forceinline__ void mlp_more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs)); }
+template <int kRegs>
+__device__ __forceinline__ void mlp_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs)); }
 __device__ __forceinline__ void mlp_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// ---- tcgen05 in either CTA group (a kernel uses one of them throughout)
+// ---- tcgen05 on CTA pairs
 //
 // The issuing warps run their loops and waits with all lanes and predicate each tcgen05 instruction on one
 // elected lane.  Inside an `if (lane == 0)` the compiler has to move every descriptor from vector to
-// uniform registers one instruction at a time: 140 cycles per MMA, longer than a 128 x 64 x 16 MMA takes.
+// uniform registers one instruction at a time: 140 cycles per MMA, longer than most of them take.
 
 __device__ __forceinline__ bool mlp_elect() {
     uint32_t p;
@@ -210,56 +228,32 @@ __device__ __forceinline__ bool mlp_elect() {
     return p != 0;
 }
 
-template <int kG>
+// Shared-memory matrix descriptor with explicit leading / stride byte offsets and layout type.
+__device__ __forceinline__ uint64_t mlp_desc(uint32_t addr, uint32_t leading, uint32_t stride, uint32_t layout) {
+    return static_cast<uint64_t>((addr >> 4) & 0x3fffu) | static_cast<uint64_t>(leading >> 4) << 16 |
+           static_cast<uint64_t>(stride >> 4) << 32 | static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(layout) << 61;
+}
+
 __device__ __forceinline__ void mlp_umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
                                          bool issue) {
-    if (kG == 1)
-        asm volatile(
-            "{\n"
-            ".reg .pred p, q;\n"
-            "setp.ne.b32 p, %4, 0;\n"
-            "setp.ne.b32 q, %5, 0;\n"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n"
-            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
-    else
-        asm volatile(
-            "{\n"
-            ".reg .pred p, q;\n"
-            "setp.ne.b32 p, %4, 0;\n"
-            "setp.ne.b32 q, %5, 0;\n"
-            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-            "}\n"
-            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
 }
 // Arrives on the barrier at this offset in every CTA of `mask` when the MMAs issued so far are complete.
-template <int kG>
-__device__ __forceinline__ void mlp_commit(uint32_t bar, uint32_t mask, uint32_t self, bool issue) {
-    const uint16_t m = static_cast<uint16_t>(mask);
-    if (kG == 1 && mask == self)
-        asm volatile(
-            "{\n"
-            ".reg .pred q;\n"
-            "setp.ne.b32 q, %1, 0;\n"
-            "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-            "}\n"
-            ::"r"(bar), "r"(static_cast<uint32_t>(issue)) : "memory");
-    else if (kG == 1)
-        asm volatile(
-            "{\n"
-            ".reg .pred q;\n"
-            "setp.ne.b32 q, %2, 0;\n"
-            "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-            "}\n"
-            ::"r"(bar), "h"(m), "r"(static_cast<uint32_t>(issue)) : "memory");
-    else
-        asm volatile(
-            "{\n"
-            ".reg .pred q;\n"
-            "setp.ne.b32 q, %2, 0;\n"
-            "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-            "}\n"
-            ::"r"(bar), "h"(m), "r"(static_cast<uint32_t>(issue)) : "memory");
+__device__ __forceinline__ void mlp_commit(uint32_t bar, uint32_t mask, bool issue) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "setp.ne.b32 q, %2, 0;\n"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+        "}\n"
+        ::"r"(bar), "h"(static_cast<uint16_t>(mask)), "r"(static_cast<uint32_t>(issue)) : "memory");
 }
 
 // Sums y[0 .. 16) over the 2^kLG lanes of a group, scattered: lane g of the group ends up with columns
@@ -283,14 +277,33 @@ __device__ __forceinline__ void mlp_group_sum(float (&y)[16], int lane) {
     }
 }
 
+// The second layer's values are rounded to 16 bits before the LayerNorm, as where they pass through memory.
+template <int kDt>
+__device__ __forceinline__ float2 mlp_round(float2 x) {
+    const uint32_t w = pack2(x.x, x.y, kDt);
+    if (kDt == RLM_BF16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+
+// Sixteen columns of the second layer's rows: accumulator + bias, rounded.
+template <int kDt>
+__device__ __forceinline__ void mlp_raw(const uint32_t (&v)[16], const float* bias, float2 (&x)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + 4 * i);
+        x[2 * i] = mlp_round<kDt>(__fadd2_rn(make_float2(b.x, b.y), make_float2(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]))));
+        x[2 * i + 1] = mlp_round<kDt>(__fadd2_rn(make_float2(b.z, b.w), make_float2(__uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]))));
+    }
+}
+
 // This warp's columns of a finished tile: the group's weighted sum of its rows, residual and store.
-// `ur` = weight * rstd of this lane's row (0: the row contributes nothing, whatever it holds), `u_sum`, `ur_sum`,
-// `urm_sum` = sums over the group of the weight, of ur and of ur * mean:
-//   sum u LayerNorm(x + b) = gamma (sum ur x + b ur_sum - urm_sum) + beta u_sum.
+// `ur` = weight * rstd of this lane's row (0: the row contributes nothing, whatever it holds), `u_sum` and `urm_sum` =
+// sums over the group of the weight and of ur * mean:
+//   sum u LayerNorm(x) = gamma (sum ur x - urm_sum) + beta u_sum.
 // The next chunk's residual and tensor-memory columns are requested before a chunk is summed.
-template <int kLG>
-__device__ __forceinline__ void mlp_store_rows(uint32_t tmem, int cols, int lane, bool live, float ur, float u_sum, float ur_sum,
-                                               float urm_sum, const float* bias, const float* gamma, const float* beta,
+template <int kLG, int kDt>
+__device__ __forceinline__ void mlp_store_rows(uint32_t tmem, int cols, int lane, bool live, float ur, float u_sum, float urm_sum,
+                                               const float* bias, const float* gamma, const float* beta,
                                                const float* residual, float* out, uint32_t drained_bar, bool drained) {
     constexpr int kSteps = kLG > 4 ? 4 : kLG;
     constexpr int kCols = 16 >> kSteps;
@@ -316,29 +329,37 @@ __device__ __forceinline__ void mlp_store_rows(uint32_t tmem, int cols, int lane
         }
     };
     fetch(0);
+    uint32_t v[16];
+    tmem_ld16(tmem, v);
 #pragma unroll 1
     for (int c = 0; c < cols; c += 16) {
-        uint32_t v[16];
-        tmem_ld16(tmem + static_cast<uint32_t>(c), v);
         float res[kCols];
 #pragma unroll
         for (int k = 0; k < kCols; ++k) res[k] = next[k];
-        if (c + 16 < cols) fetch(c + 16);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c + 16 >= cols) {                            // the accumulator may be overwritten
+        float2 x[8];
+        mlp_raw<kDt>(v, bias + c, x);
+        float y[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 p = __fmul2_rn(x[i], make_float2(ur, ur));
+            y[2 * i] = ur == 0.0f ? 0.0f : p.x;
+            y[2 * i + 1] = ur == 0.0f ? 0.0f : p.y;
+        }
+        if (c + 16 < cols) {
+            tmem_ld16(tmem + static_cast<uint32_t>(c + 16), v);
+            fetch(c + 16);
+        } else {                                         // the accumulator may be overwritten
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (drained) mlp_arrive_remote(drained_bar);
         }
-        float y[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = ur == 0.0f ? 0.0f : __uint_as_float(v[i]) * ur;
         mlp_group_sum<kLG>(y, lane);
         if (!store) continue;
 #pragma unroll
         for (int k = 0; k < kCols; ++k) {
             const int col = c + c0 + k;
-            res[k] += fmaf(gamma[col], fmaf(bias[col], ur_sum, y[k] - urm_sum), beta[col] * u_sum);
+            res[k] += fmaf(gamma[col], y[k] - urm_sum, beta[col] * u_sum);
         }
 #pragma unroll
         for (int k = 0; k < kCols; k += kVec) {
@@ -352,9 +373,10 @@ __device__ __forceinline__ void mlp_store_rows(uint32_t tmem, int cols, int lane
     }
 }
 
-template <int kDt, int kG>
+template <int kDt>
 __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
-    const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2, const MlpArgs a, const int outs) {
+    const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2,
+    const MlpArgs a, const int outs) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) MlpBars bars;
     __shared__ uint32_t tmem_slot;
@@ -362,156 +384,170 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
     volatile int* failed = &failed_s;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // warp-uniform
-    const int C = outs, R = a.rdim, H = a.hdim, NC = a.cols;
+    const int C = outs, R = a.rdim, H = a.hdim, NC = a.cols, wide = a.wide;
     const uint32_t rank = mlp_rank();
     const int o = static_cast<int>(rank) / kG, g = static_cast<int>(rank) % kG;      // output part, row group
     const uint32_t leader = static_cast<uint32_t>(o * kG);                           // issues the pair's MMAs
     const uint32_t pair_mask = ((1u << kG) - 1u) << leader;
-    const int kblocks = R / kBK, J = H / (kMlpHC * C);
+    const int kblocks = R / kBK, U = H / (2 * kMlpHC * C);                           // units of 128 hidden columns per CTA
     const int cluster = static_cast<int>(blockIdx.x) / (C * kG), n_clusters = static_cast<int>(gridDim.x) / (C * kG);
     const int n_super = (a.n_tiles + kG - 1) / kG;
+    const int anchors = kBM >> a.k_shift, sel_k = kG * anchors;                      // anchors of a tile, of the pair
 
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    const MlpPlan plan = mlp_plan(R, NC, C, kG, a.term_stages, a.wm_stages, a.w2_stages, a.k_shift);
+    const MlpPlan plan = mlp_plan(R, NC, C, wide, a.term_stages, a.wm_stages, a.w2_stages, a.k_shift);
     const uint32_t s_a = smem_u32(base + plan.a), s_wm = smem_u32(base + plan.wm), s_w2 = smem_u32(base + plan.w2);
-    const uint32_t s_hid = smem_u32(base + plan.hid);
-    const uint32_t wm_kblock = (kMlpHC / kG) * 128u, wm_stage = static_cast<uint32_t>(kblocks) * wm_kblock;
+    const uint32_t s_hid = smem_u32(base + plan.hid), s_term = smem_u32(base + plan.term), s_anc = smem_u32(base + plan.anc);
+    const uint32_t anc_stage = mlp_anchor_bytes(a.k_shift);
+    const int wm_rows = (wide ? 2 : 1) * kMlpHC / kG;                                // weight rows of a stage in this CTA
+    const uint32_t wm_kblock = static_cast<uint32_t>(wm_rows) * 128u, wm_stage = static_cast<uint32_t>(kblocks) * wm_kblock;
     const int n_inst = NC > 256 ? 2 : 1, NI = NC / n_inst;
-    const uint32_t w2_stage = static_cast<uint32_t>(NI / kG) * 128u;        // one instruction's weight rows
+    const uint32_t w2_stage = static_cast<uint32_t>(NI / kG) * 128u;                 // one instruction's weight rows
     float* bias_s = reinterpret_cast<float*>(base + plan.bias);
     float* gamma_s = reinterpret_cast<float*>(base + plan.gamma);
     float* beta_s = reinterpret_cast<float*>(base + plan.beta);
     float2* stats_s = reinterpret_cast<float2*>(base + plan.stats);
     float* u_s = reinterpret_cast<float*>(base + plan.u);
+    int* prow_s = reinterpret_cast<int*>(base + plan.prow);
+    int* arow_s = reinterpret_cast<int*>(base + plan.arow);
 
     if (tid == 0) {
         failed_s = 0;
         const auto init = [](unsigned long long* b, int count) { mbar_init(smem_u32(b), static_cast<uint32_t>(count)); };
-        init(&bars.a_full, kMlpGatherWarps * kG);
+        // what the leader waits for from both CTAs: its own arrival and the one that the other CTA forwards
+        const int both = g == 0 ? 2 : 1;
+        init(&bars.a_full, kMlpOperandWarps * kG);
         init(&bars.a_empty, 1);
         init(&bars.d2_full, 1);
         init(&bars.d2_empty, kMlpEpiWarps * kG);
         init(&bars.stats_full, C == 1 ? kMlpEpiWarps : 1);
-        for (int i = 0; i < 3; ++i) init(&bars.u_full[i], kMlpGatherWarps);
+        for (int i = 0; i < 3; ++i) init(&bars.u_full[i], kBM / 32);
         for (int i = 0; i < 2; ++i) {
+            init(&bars.rows_full[i], kBM / 32);
             init(&bars.d1_full[i], 1);
-            init(&bars.d1_empty[i], kMlpEpiWarps / 2 * kG);
-            init(&bars.wm_full[i], 1);
+            init(&bars.d1_empty[i], (wide ? kMlpEpiWarps : kMlpEpiWarps / 2) * kG);
+            init(&bars.wm_full[i], both);
             init(&bars.wm_empty[i], 1);
-            init(&bars.peer_wm[i], 1);
         }
         for (int i = 0; i < kMlpMaxStages; ++i) {
-            init(&bars.w2_full[i], 1);
+            init(&bars.w2_full[i], both);
             init(&bars.w2_empty[i], 1);
-            init(&bars.peer_w2[i], 1);
         }
         for (int i = 0; i < kMlpHidden; ++i) {
             for (int b = 0; b < 2; ++b) init(&bars.hid_full[i][b], C == 1 ? kMlpEpiWarps / 2 : 4);
             init(&bars.hid_empty[i], C);
         }
         for (int i = 0; i < kMlpMaxTerms; ++i) {
-            init(&bars.term_full[i], 32 * kMlpGatherWarps);
-            init(&bars.term_empty[i], kMlpEpiWarps / 2);
+            init(&bars.term_full[i], 32 * kMlpGatherWarps + both - 1);
+            init(&bars.term_empty[i], 1);
         }
         fence_barrier_init();
     }
-    if (warp == kMlpEpiWarps + 1) {
-        if (kG == 1) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        }
+    if (warp == kMlpEpiWarps + 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i < NC; i += kMlpThreads) {       // parameters of this CTA's output columns
         bias_s[i] = a.second_bias[o * NC + i];
         gamma_s[i] = a.norm_w[o * NC + i];
         beta_s[i] = a.norm_b[o * NC + i];
     }
+    const uint16_t one = kDt == RLM_BF16 ? 0x3f80 : 0x3c00;
+    for (int i = tid; i < kBM * sel_k / 8; i += kMlpThreads) {          // one-hot rows: K-chunk major core matrices, no swizzle
+        const int c = i / kBM, r = i - c * kBM;
+        const int hot = g * anchors + (r >> a.k_shift) - 8 * c;
+        uint32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = hot >> 1 == e && hot >= 0 ? static_cast<uint32_t>(one) << (16 * (hot & 1)) : 0u;
+        *reinterpret_cast<uint4*>(base + plan.onehot + c * (kBM * 16) + r * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    for (int i = tid; i < (kMlpHC / kG) * 8; i += kMlpThreads) {        // this CTA's half of the 64 x 64 identity
+        const int r = i >> 3, c = i & 7, hot = g * (kMlpHC / kG) + r - 8 * c;
+        uint32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = hot >> 1 == e && hot >= 0 ? static_cast<uint32_t>(one) << (16 * (hot & 1)) : 0u;
+        *reinterpret_cast<uint4*>(base + plan.ident + swizzled(r, c, kMlpBlock)) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    fence_proxy_async();
     griddep_sync();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     mlp_cluster_sync();                                  // every CTA's barriers are initialised
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d2 = __shfl_sync(0xffffffffu, tmem_slot, 0), tmem_d1 = tmem_d2 + static_cast<uint32_t>(NC);
+    // hidden column of block n (64 columns, counted within a tile) of part b
+    const auto column = [&](int n, int b) { return ((n >> 1) * C + b) * (2 * kMlpHC) + (n & 1) * kMlpHC; };
 
     if (warp < kMlpEpiWarps) {
+        mlp_more_registers<kMlpEpiRegs>();
         // ------------------------------------------------------------ epilogue
-        // Two groups of eight warps take the hidden blocks in turn, so that one group's waits and loads fall into
-        // the other's arithmetic; thread = pair row x 32 of a block's 64 columns.
+        // Two groups of eight warps take the two blocks of a unit; thread = pair row x 32 of a block's 64 columns.
         const int row = 32 * (warp & 3) + lane, turn = warp >> 3, half = (warp >> 2) & 1;
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        const uint32_t row_at = static_cast<uint32_t>((row >> 3) * 1024 + (row & 7) * 128);
-        const unsigned char* anc = base + plan.anc + static_cast<uint32_t>(row >> a.k_shift) * kMlpAncStride + 64 * half;
-        const uint32_t anc_stage = static_cast<uint32_t>(kBM >> a.k_shift) * kMlpAncStride;
+        unsigned char* block = base + plan.hid + static_cast<uint32_t>(turn * C + o) * kMlpBlock;
+        uint4* cell[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            cell[c] = reinterpret_cast<uint4*>(block + (row >> 3) * 1024 + (row & 7) * 128 + (((4 * half + c) ^ (row & 7)) << 4));
+        const uint32_t full = smem_u32(&bars.hid_full[turn][o]), part = smem_u32(block) + static_cast<uint32_t>(warp & 3) * 4096u;
         const int q = warp >> 2, quarter = NC / 4;                   // output columns of this warp in the last stage
         const int group = 1 << a.group_shift;
         const uint32_t d2_drained = mlp_peer(smem_u32(&bars.d2_empty), leader);
-        int n = 0, ts = 0, tphase = 0, tix = 0, tix3 = 0, u_phase = 0;
+        const uint32_t d1_at = tmem_d1 + lane_base + static_cast<uint32_t>(turn * kMlpHC + 32 * half);
+        int unit = 0, tix = 0, tix3 = 0, u_phase = 0;
         bool ok = true;
-        for (int super = cluster; super < n_super; super += n_clusters, ++tix) {
-            for (int j = 0; j < J; ++j, ++n) {
-                const int slot = ts, phase = tphase, use = (n >> 1) & 1;
-                if (++ts == a.term_stages) { ts = 0; tphase ^= 1; }
-                if ((n & 1) != turn) continue;
-                const unsigned char* term = base + plan.term + static_cast<uint32_t>(slot) * kMlpBlock + row_at;
-                unsigned char* block = base + plan.hid + static_cast<uint32_t>(turn * C + o) * kMlpBlock;
-                ok = ok && mlp_wait(smem_u32(&bars.d1_full[turn]), use, failed);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t v[2][16];
-                tmem_ld16(tmem_d1 + lane_base + static_cast<uint32_t>(turn * kMlpHC + 32 * half), v[0]);
-                tmem_ld16(tmem_d1 + lane_base + static_cast<uint32_t>(turn * kMlpHC + 32 * half + 16), v[1]);
-                ok = ok && mlp_wait(smem_u32(&bars.term_full[slot]), phase, failed);
+        const auto hidden_block = [&]() {
+            const int buffer = wide ? unit & 1 : turn, phase = wide ? (unit >> 1) & 1 : unit & 1;
+            ok = ok && mlp_wait(smem_u32(&bars.d1_full[buffer]), phase, failed);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t from = d1_at + (wide ? static_cast<uint32_t>(buffer * 2 * kMlpHC) : 0u);
+            uint4 w[4];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                uint32_t v[16];
+                tmem_ld16(from + 16 * hh, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (ok && lane == 0) mlp_arrive_leader<kG>(smem_u32(&bars.d1_empty[turn]), leader);
-                uint4 w[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float2 fa[4], fp[4];
-                    unpack8_pairs(*reinterpret_cast<const uint4*>(anc + slot * anc_stage + 16 * c), kDt, fa);
-                    unpack8_pairs(*reinterpret_cast<const uint4*>(term + ((static_cast<uint32_t>(4 * half + c) ^ (row & 7)) << 4)), kDt, fp);
-                    uint32_t y[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float2 acc = make_float2(__uint_as_float(v[c >> 1][8 * (c & 1) + 2 * i]),
-                                                       __uint_as_float(v[c >> 1][8 * (c & 1) + 2 * i + 1]));
-                        const float2 h = gelu_pair(__fadd2_rn(acc, __fadd2_rn(fa[i], fp[i])));
-                        y[i] = pack2(h.x, h.y, kDt);
-                    }
-                    w[c] = make_uint4(y[0], y[1], y[2], y[3]);
-                }
-                __syncwarp();
-                if (ok && lane == 0) mlp_arrive(smem_u32(&bars.term_empty[slot]));
-                // the block's previous content has been consumed, here and where it was copied to
-                ok = ok && mlp_wait(smem_u32(&bars.hid_empty[turn]), use ^ 1, failed);
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(block + row_at + ((static_cast<uint32_t>(4 * half + c) ^ (row & 7)) << 4)) = w[c];
-                fence_proxy_async();                                  // the block -> tensor core, bulk copy
-                const uint32_t full = smem_u32(&bars.hid_full[turn][o]);
-                if (C == 1) {
+                if (hh == 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (ok && lane == 0) mlp_arrive(full);
-                } else {
-                    // both warps of these 32 rows have written their columns: 4 KB that are contiguous in the block
-                    mlp_bar_sync(1 + 4 * turn + (warp & 3), 64);
-                    if (ok && half == 0 && lane == 0) {
-                        mlp_arrive(full);
-                        const uint32_t part = smem_u32(block) + static_cast<uint32_t>(warp & 3) * 4096u;
-                        for (int other = 0; other < C; ++other) {
-                            if (other == o) continue;
-                            const uint32_t to = static_cast<uint32_t>(other * kG + g);
-                            const uint32_t bar = mlp_peer(full, to);
-                            mlp_expect_remote(bar, 4096u);
-                            mlp_copy_cluster(mlp_peer(part, to), part, 4096u, bar);
-                        }
-                    }
+                    if (ok && lane == 0) mlp_arrive_leader(smem_u32(&bars.d1_empty[buffer]), leader);
+                }
+                uint32_t y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 h = gelu_pair(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+                    y[i] = pack2(h.x, h.y, kDt);
+                }
+                w[2 * hh] = make_uint4(y[0], y[1], y[2], y[3]);
+                w[2 * hh + 1] = make_uint4(y[4], y[5], y[6], y[7]);
+            }
+            // the block's previous content has been consumed, here and where it was copied to
+            ok = ok && mlp_wait(smem_u32(&bars.hid_empty[turn]), (unit & 1) ^ 1, failed);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) *cell[c] = w[c];
+            fence_proxy_async();                                  // the block -> tensor core, bulk copy
+            if (C == 1) {
+                __syncwarp();
+                if (ok && lane == 0) mlp_arrive(full);
+            } else {
+                // both warps of these 32 rows have written their columns: 4 KB that are contiguous in the block
+                mlp_bar_sync(1 + 4 * turn + (warp & 3), 64);
+                if (ok && half == 0 && lane == 0) {
+                    mlp_arrive(full);
+                    const uint32_t to = static_cast<uint32_t>((1 - o) * kG + g), bar = mlp_peer(full, to);
+                    mlp_expect_remote(bar, 4096u);
+                    mlp_copy_cluster(mlp_peer(part, to), part, 4096u, bar);
                 }
             }
+            ++unit;
+        };
+        // The next tile's first unit comes before a tile's last stage: its arithmetic falls into the second layer's
+        // tail, and the second layer finds it ready.
+        if (cluster < n_super) hidden_block();
+        for (int super = cluster; super < n_super; super += n_clusters, ++tix) {
+            for (int j = 1; j < U; ++j) hidden_block();
+            if (super + n_clusters < n_super) hidden_block();
             // ---- the tile's second layer is complete: LayerNorm over d, weighted sum over the group
             const int tile = super * kG + g;
             const uint32_t tmem_row = tmem_d2 + lane_base + static_cast<uint32_t>(q * quarter);
@@ -521,32 +557,31 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             if (C > 1 && ok && tid == 0) mbar_expect_tx(smem_u32(&bars.stats_full), static_cast<uint32_t>(4 * C * kBM * 8));
             // statistics of this thread's columns about the mean of the first sixteen: one pass over the accumulator
             float shift = 0.0f, s1 = 0.0f, s2 = 0.0f;
-#pragma unroll 1
-            for (int c = 0; c < quarter; c += 16) {
+            {
                 uint32_t v[16];
-                tmem_ld16(tmem_row + static_cast<uint32_t>(c), v);
-                float x[16];
+                tmem_ld16(tmem_row, v);
+#pragma unroll 1
+                for (int c = 0; c < quarter; c += 16) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float2 x[8];
+                    mlp_raw<kDt>(v, bias + c, x);
+                    if (c + 16 < quarter) tmem_ld16(tmem_row + static_cast<uint32_t>(c + 16), v);
+                    if (c == 0) {
+                        float2 sum = x[0];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 b = *reinterpret_cast<const float4*>(bias + c + 4 * i);
-                    x[4 * i] = b.x; x[4 * i + 1] = b.y; x[4 * i + 2] = b.z; x[4 * i + 3] = b.w;
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c == 0) {
-                    float sum = 0.0f;
+                        for (int i = 1; i < 8; ++i) sum = __fadd2_rn(sum, x[i]);
+                        shift = (sum.x + sum.y) * 0.0625f;
+                    }
+                    float2 t1 = make_float2(0.0f, 0.0f), t2 = t1;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) sum += __uint_as_float(v[i]) + x[i];
-                    shift = sum * 0.0625f;
+                    for (int i = 0; i < 8; ++i) {
+                        const float2 y = __fadd2_rn(x[i], make_float2(-shift, -shift));
+                        t1 = __fadd2_rn(t1, y);
+                        t2 = __ffma2_rn(y, y, t2);
+                    }
+                    s1 += t1.x + t1.y;
+                    s2 += t2.x + t2.y;
                 }
-                float t1 = 0.0f, t2 = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float y = (__uint_as_float(v[i]) + x[i]) - shift;
-                    t1 += y;
-                    t2 = fmaf(y, y, t2);
-                }
-                s1 += t1;
-                s2 += t2;
             }
             const float inv_quarter = 1.0f / static_cast<float>(quarter);
             const float mean_q = fmaf(s1, inv_quarter, shift), m2 = fmaf(-s1 * inv_quarter, s1, s2);
@@ -558,28 +593,32 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                 if (ok && lane == 0) mlp_arrive(smem_u32(&bars.stats_full));
                 ok = ok && mlp_wait(smem_u32(&bars.stats_full), tix & 1, failed);
             } else {
-                for (int other = 0; ok && other < C; ++other) {
+#pragma unroll
+                for (int other = 0; other < 2; ++other) {
                     const uint32_t to = static_cast<uint32_t>(other * kG + g);
-                    mlp_store_remote(mlp_peer(smem_u32(mine), to), mean_q, m2, mlp_peer(smem_u32(&bars.stats_full), to));
+                    if (ok) mlp_store_remote(mlp_peer(smem_u32(mine), to), mean_q, m2, mlp_peer(smem_u32(&bars.stats_full), to));
                 }
                 ok = ok && mlp_wait<true>(smem_u32(&bars.stats_full), tix & 1, failed);
             }
+            float2 st[8];
             float mean = 0.0f, total = 0.0f;
-            for (int i = 0; i < 4 * C; ++i) mean += stats_s[i * kBM + row].x;
-            mean *= C == 1 ? 0.25f : 0.125f;
-            for (int i = 0; i < 4 * C; ++i) {
-                const float2 s = stats_s[i * kBM + row];
-                total += fmaf(static_cast<float>(quarter) * (s.x - mean), s.x - mean, s.y);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                st[i] = i < 4 * C ? stats_s[i * kBM + row] : make_float2(0.0f, 0.0f);
+                mean += st[i].x;
             }
-            const float rstd = rsqrtf(total / static_cast<float>(a.d) + a.eps);
+            mean *= C == 1 ? 0.25f : 0.125f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < 4 * C) total += fmaf(static_cast<float>(quarter) * (st[i].x - mean), st[i].x - mean, st[i].y);
+            const float rstd = rsqrtf(fmaf(total, a.inv_d, a.eps));
             ok = ok && mlp_wait(smem_u32(&bars.u_full[tix3]), u_phase, failed);
             const float u = u_s[tix3 * kBM + row];
             if (++tix3 == 3) { tix3 = 0; u_phase ^= 1; }
             const float ur = u == 0.0f ? 0.0f : u * rstd;
-            float u_sum = u, ur_sum = ur, urm_sum = u == 0.0f ? 0.0f : ur * mean;
+            float u_sum = u, urm_sum = u == 0.0f ? 0.0f : ur * mean;
             for (int s = 1; s < group; s <<= 1) {
                 u_sum += __shfl_xor_sync(0xffffffffu, u_sum, s);
-                ur_sum += __shfl_xor_sync(0xffffffffu, ur_sum, s);
                 urm_sum += __shfl_xor_sync(0xffffffffu, urm_sum, s);
             }
             const int pair = tile * kBM + row;
@@ -589,9 +628,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             const float *gm = gamma_s + q * quarter, *bt = beta_s + q * quarter;
             float* out = a.out + at;
             const bool drained = ok && lane == 0;
-#define MLP_STORE(kLG) mlp_store_rows<kLG>(tmem_row, quarter, lane, live, ur, u_sum, ur_sum, urm_sum, bias, gm, bt, res, out, d2_drained, drained)
+#define MLP_STORE(kLG) mlp_store_rows<kLG, kDt>(tmem_row, quarter, lane, live, ur, u_sum, urm_sum, bias, gm, bt, res, out, d2_drained, drained)
             switch (a.group_shift) {
-                case 1: MLP_STORE(1); break;
                 case 2: MLP_STORE(2); break;
                 case 3: MLP_STORE(3); break;
                 case 4: MLP_STORE(4); break;
@@ -600,139 +638,213 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
 #undef MLP_STORE
         }
     } else if (warp == kMlpEpiWarps) {
+        mlp_fewer_registers<kMlpIssueRegs>();
         // ------------------------------------------------------------ W_2 tiles
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
             int ws = 0, wphase = 0;
             bool ok = true;
             for (int super = cluster; ok && super < n_super; super += n_clusters)
-                for (int j = 0; ok && j < J; ++j)
-                    for (int part = 0; part < C; ++part)
+                for (int n = 0; ok && n < 2 * U; ++n)
+                    for (int p = 0; p < C; ++p)
                         for (int i = 0; i < n_inst; ++i) {
-                            const int b = part == 0 ? o : 1 - o;
                             const uint32_t bar = smem_u32(&bars.w2_full[ws]);
                             ok = ok && mlp_wait(smem_u32(&bars.w2_empty[ws]), wphase ^ 1, failed);
                             if (!ok) break;
                             mbar_expect_tx(bar, w2_stage);
-                            tma_load_2d(s_w2 + ws * w2_stage, &map_w2, (j * C + b) * kMlpHC, o * NC + i * NI + g * (NI / kG), bar);
+                            tma_load_2d(s_w2 + ws * w2_stage, &map_w2, column(n, p == 0 ? o : 1 - o),
+                                        o * NC + i * NI + g * (NI / kG), bar);
                             if (++ws == a.w2_stages) { ws = 0; wphase ^= 1; }
                         }
         }
         __syncwarp();
-    } else if (warp == kMlpEpiWarps + 3) {
-        // ------------------------------------------------------------ W_m tiles
+    } else if (warp == kMlpEpiWarps + 1) {
+        mlp_fewer_registers<kMlpIssueRegs>();
+        // ------------------------------------------------------------ W_m tiles: a unit's or a block's rows
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_wm) : "memory");
             int ms = 0, mphase = 0;
             bool ok = true;
             for (int super = cluster; ok && super < n_super; super += n_clusters)
-                for (int j = 0; j < J; ++j) {
+                for (int n = 0; n < 2 * U; n += 1 + wide) {
                     const uint32_t bar = smem_u32(&bars.wm_full[ms]);
                     ok = ok && mlp_wait(smem_u32(&bars.wm_empty[ms]), mphase ^ 1, failed);
                     if (!ok) break;
                     mbar_expect_tx(bar, wm_stage);
                     for (int kb = 0; kb < kblocks; ++kb)
-                        tma_load_2d(s_wm + ms * wm_stage + kb * wm_kblock, &map_wm, kb * kBK,
-                                    (j * C + o) * kMlpHC + g * (kMlpHC / kG), bar);
+                        tma_load_2d(s_wm + ms * wm_stage + kb * wm_kblock, &map_wm, kb * kBK, column(n, o) + g * wm_rows, bar);
                     if (++ms == a.wm_stages) { ms = 0; mphase ^= 1; }
                 }
         }
         __syncwarp();
-    } else if (warp == kMlpEpiWarps + 1) {
-        // ------------------------------------------------------------ first layer: D1[n & 1] = products x W_m block
+    } else if (warp == kMlpEpiWarps + 2) {
+        mlp_fewer_registers<kMlpIssueRegs>();
+        // ------------------------------------------------------------ first layer: D1 = segments + products x W_m rows
         const bool elected = mlp_elect(), issue = g == 0;
         const uint64_t a_desc = smem_desc_sw128(s_a), w_desc = smem_desc_sw128(s_wm);
-        int ms = 0, mphase = 0, p = 0, tix = 0;
+        const uint64_t t_desc = smem_desc_sw128(s_term), i_desc = smem_desc_sw128(smem_u32(base + plan.ident));
+        // one-hot rows: 128-byte core matrices, K chunks 16 * 128 bytes apart, 8-row groups 128 bytes apart, no swizzle
+        const uint64_t s_desc = mlp_desc(smem_u32(base + plan.onehot), kBM * 16, 128, 0);
+        // anchor segments [anchor][32 columns]: N-major, 64-byte swizzle, 8-anchor groups 512 bytes apart
+        const uint64_t n_desc = mlp_desc(s_anc, 16, 512, 4);
+        const int sel_steps = sel_k / 16;
+        int ms = 0, mphase = 0, ts = 0, tphase = 0, unit = 0, tix = 0;
         bool ok = true;
+        const auto products = [&](uint32_t d_at, uint32_t idesc, int buffer) {
+            ok = ok && mlp_wait(smem_u32(&bars.wm_full[ms]), mphase, failed);
+            if (issue) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const bool go = elected && ok;
+                const uint64_t wd = w_desc + (static_cast<uint32_t>(ms) * wm_stage >> 4);
+#pragma unroll
+                for (int kk = 0; kk < kBK / 16; ++kk) mlp_umma(d_at, a_desc + 2 * kk, wd + 2 * kk, idesc, 1u, go);
+                if (kblocks > 1)
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        mlp_umma(d_at, a_desc + (kMlpBlock >> 4) + 2 * kk, wd + (wm_kblock >> 4) + 2 * kk, idesc, 1u, go);
+                mlp_commit(smem_u32(&bars.d1_full[buffer]), pair_mask, go);
+                mlp_commit(smem_u32(&bars.wm_empty[ms]), pair_mask, go);
+            } else if (ok && elected) {
+                mlp_arrive_leader(smem_u32(&bars.wm_full[ms]), leader);
+            }
+            if (++ms == a.wm_stages) { ms = 0; mphase ^= 1; }
+        };
         for (int super = cluster; ok && super < n_super; super += n_clusters, ++tix) {
-            if (issue) ok = ok && mlp_wait(smem_u32(&bars.a_full), tix & 1, failed);
-            for (int j = 0; ok && j < J; ++j, ++p) {
-                ok = ok && mlp_wait(smem_u32(&bars.wm_full[ms]), mphase, failed);
-                if (issue) {
-                    if (kG == 2) ok = ok && mlp_wait(smem_u32(&bars.peer_wm[ms]), mphase, failed);
-                    ok = ok && mlp_wait(smem_u32(&bars.d1_empty[p & 1]), ((p >> 1) & 1) ^ 1, failed);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const bool go = elected && ok;
-                    const uint32_t d_at = tmem_d1 + static_cast<uint32_t>((p & 1) * kMlpHC);
-                    const uint64_t wd = w_desc + (static_cast<uint32_t>(ms) * wm_stage >> 4);
-#pragma unroll 2
-                    for (int kb = 0; kb < kblocks; ++kb)
+            for (int j = 0; ok && j < U; ++j, ++unit) {
+                const uint32_t unit_at = tmem_d1 + (wide ? static_cast<uint32_t>((unit & 1) * 2 * kMlpHC) : 0u);
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const uint32_t d_at = unit_at + static_cast<uint32_t>(s * kMlpHC);
+                    if (issue && (s == 0 || !wide))
+                        ok = ok && mlp_wait(smem_u32(&bars.d1_empty[wide ? unit & 1 : s]), (wide ? (unit >> 1) & 1 : unit & 1) ^ 1, failed);
+                    ok = ok && mlp_wait(smem_u32(&bars.term_full[ts]), tphase, failed);
+                    fence_proxy_async();              // the segments came by ordinary (cp.async) writes
+                    if (issue) {
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const bool go = elected && ok;
+                        const uint64_t td = t_desc + (static_cast<uint32_t>(ts) * kMlpBlock >> 4);
+                        const uint64_t nd = n_desc + (static_cast<uint32_t>(ts) * anc_stage >> 4);
 #pragma unroll
                         for (int kk = 0; kk < kBK / 16; ++kk)
-                            mlp_umma<kG>(d_at, a_desc + kb * (kMlpBlock >> 4) + 2 * kk, wd + kb * (wm_kblock >> 4) + 2 * kk, a.idesc1,
-                                         (kb > 0 || kk > 0) ? 1u : 0u, go);
-                    mlp_commit<kG>(smem_u32(&bars.d1_full[p & 1]), pair_mask, pair_mask, go);
-                    mlp_commit<kG>(smem_u32(&bars.wm_empty[ms]), pair_mask, pair_mask, go);
-                    if (j + 1 == J) mlp_commit<kG>(smem_u32(&bars.a_empty), pair_mask, pair_mask, go);
-                } else if (ok && elected) {
-                    mlp_arrive_remote(mlp_peer(smem_u32(&bars.peer_wm[ms]), leader));
+                            mlp_umma(d_at, td + 2 * kk, i_desc + 2 * kk, a.idesc_block, kk > 0 ? 1u : 0u, go);
+                        for (int kk = 0; kk < sel_steps; ++kk)
+                            mlp_umma(d_at, s_desc + kk * (2 * kBM * 16 >> 4), nd + kk * (1024 >> 4), a.idesc_block | (1u << 16), 1u, go);
+                        mlp_commit(smem_u32(&bars.term_empty[ts]), pair_mask, go);
+                    } else if (ok && elected) {
+                        mlp_arrive_leader(smem_u32(&bars.term_full[ts]), leader);
+                    }
+                    if (++ts == a.term_stages) { ts = 0; tphase ^= 1; }
+                    if (s == 0 && j == 0 && issue) ok = ok && mlp_wait(smem_u32(&bars.a_full), tix & 1, failed);
+                    if (!wide) products(d_at, a.idesc_block, s);
                 }
-                if (++ms == a.wm_stages) { ms = 0; mphase ^= 1; }
+                if (wide) products(unit_at, a.idesc_unit, unit & 1);
+                if (issue && j + 1 == U) mlp_commit(smem_u32(&bars.a_empty), pair_mask, elected && ok);
             }
         }
         __syncwarp();
-    } else if (warp == kMlpEpiWarps + 2) {
+    } else if (warp == kMlpEpiWarps + 3) {
+        mlp_fewer_registers<kMlpIssueRegs>();
         // ------------------------------------------------------------ second layer: D2 += hidden blocks x W_2 columns
         const bool elected = mlp_elect(), issue = g == 0;
         const uint64_t h_desc = smem_desc_sw128(s_hid), w_desc = smem_desc_sw128(s_w2);
-        int ws = 0, wphase = 0, n = 0, tix = 0;
+        int ws = 0, wphase = 0, unit = 0, tix = 0;
         bool ok = true;
         for (int super = cluster; ok && super < n_super; super += n_clusters, ++tix) {
             if (issue) ok = ok && mlp_wait(smem_u32(&bars.d2_empty), (tix & 1) ^ 1, failed);
-            for (int j = 0; ok && j < J; ++j, ++n) {
-                const int d = n & 1;
-                for (int part = 0; part < C; ++part) {
-                    const int b = part == 0 ? o : 1 - o;          // this CTA's own block first: the other one is still on its way
-                    ok = ok && mlp_wait(smem_u32(&bars.hid_full[d][b]), (n >> 1) & 1, failed);
+            for (int n = 0; ok && n < 2 * U; ++n) {
+                const int d = n & 1, phase = (unit + (n >> 1)) & 1;
+                for (int p = 0; p < C; ++p) {
+                    const int b = p == 0 ? o : 1 - o;          // this CTA's own block first: the other one is still on its way
+                    ok = ok && mlp_wait(smem_u32(&bars.hid_full[d][b]), phase, failed);
                     const uint64_t hd = h_desc + (static_cast<uint32_t>(d * C + b) * kMlpBlock >> 4);
                     for (int i = 0; i < n_inst; ++i) {
                         ok = ok && mlp_wait(smem_u32(&bars.w2_full[ws]), wphase, failed);
                         if (issue) {
-                            if (kG == 2) ok = ok && mlp_wait(smem_u32(&bars.peer_w2[ws]), wphase, failed);
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             const bool go = elected && ok;
                             const uint64_t wd = w_desc + (static_cast<uint32_t>(ws) * w2_stage >> 4);
 #pragma unroll
                             for (int kk = 0; kk < kBK / 16; ++kk)
-                                mlp_umma<kG>(tmem_d2 + static_cast<uint32_t>(i * NI), hd + 2 * kk, wd + 2 * kk, a.idesc2,
-                                             (j > 0 || part > 0 || kk > 0) ? 1u : 0u, go);
-                            mlp_commit<kG>(smem_u32(&bars.w2_empty[ws]), pair_mask, pair_mask, go);
-                            if (i + 1 == n_inst)
-                                mlp_commit<kG>(smem_u32(&bars.hid_empty[d]), ((1u << kG) - 1u) << (b * kG), pair_mask, go);
+                                mlp_umma(tmem_d2 + static_cast<uint32_t>(i * NI), hd + 2 * kk, wd + 2 * kk, a.idesc2,
+                                         (n > 0 || p > 0 || kk > 0) ? 1u : 0u, go);
+                            mlp_commit(smem_u32(&bars.w2_empty[ws]), pair_mask, go);
+                            if (i + 1 == n_inst) mlp_commit(smem_u32(&bars.hid_empty[d]), ((1u << kG) - 1u) << (b * kG), go);
                         } else if (ok && elected) {
-                            // this CTA's hidden block and weight rows are there
-                            mlp_arrive_remote(mlp_peer(smem_u32(&bars.peer_w2[ws]), leader));
+                            mlp_arrive_leader(smem_u32(&bars.w2_full[ws]), leader);      // this CTA's block and weight rows are there
                         }
                         if (++ws == a.w2_stages) { ws = 0; wphase ^= 1; }
                     }
                 }
-                if (issue && j + 1 == J) mlp_commit<kG>(smem_u32(&bars.d2_full), pair_mask, pair_mask, elected && ok);
             }
+            unit += U;
+            if (issue) mlp_commit(smem_u32(&bars.d2_full), pair_mask, elected && ok);
         }
         __syncwarp();
-    } else {
-        // ------------------------------------------------------------ gathers
-        const int gt = tid - 32 * (kMlpEpiWarps + 4), gw = gt >> 5;
-        int* prow_s = reinterpret_cast<int*>(base + plan.prow);
-        int* arow_s = reinterpret_cast<int*>(base + plan.arow);
-        const int K = 1 << a.k_shift, anchors = kBM >> a.k_shift, chunks = R / 8, rows_per_warp = 32 / chunks;
-        const size_t op_row = static_cast<size_t>(R) * 2, ex_row = static_cast<size_t>(H) * 4;
-        const char* operand = static_cast<const char*>(a.operand_cache);
+    } else if (warp < kMlpEpiWarps + 4 + kMlpGatherWarps) {
+        mlp_fewer_registers<kMlpIssueRegs>();
+        // ------------------------------------------------------------ expanded-cache segments of every block
+        // 64 columns of the tile's 128 partner rows (128-byte swizzle), this CTA's 32 of the 64 columns of the pair's
+        // anchor rows (64-byte swizzle), a thread per 16-byte chunk.
+        const int gt = tid - 32 * (kMlpEpiWarps + 4), c = gt & 7, ac = gt & 3;
+        const size_t ex_row = static_cast<size_t>(H) * 4;
         const char* expanded = static_cast<const char*>(a.expanded_cache);
-        const int cc = lane % chunks, r_first = gw * rows_per_warp + lane / chunks, r_step = kMlpGatherWarps * rows_per_warp;
-        int ts = 0, tphase = 0, tix = 0, u_at = 0;
+        const uint32_t to = swizzled(gt >> 3, c, kMlpBlock);               // rows 16 apart: 2048 bytes apart
+        int ts = 0, tphase = 0, tix = 0;
         bool ok = true;
-        // This thread's pair of tile `super`: cache rows of its partner and anchor into buffer `b`, its weight into u.
+        for (int super = cluster; super < n_super; super += n_clusters, ++tix) {
+            ok = ok && mlp_wait(smem_u32(&bars.rows_full[tix & 1]), (tix >> 1) & 1, failed);
+            const int* arow_t = arow_s + (tix & 1) * sel_k;
+            const char* from[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int row = prow_s[(tix & 1) * kBM + (gt >> 3) + 16 * i];
+                from[i] = row < 0 ? nullptr : expanded + row * ex_row + static_cast<size_t>(H) * 2 + 16 * c;
+            }
+            for (int n = 0; n < 2 * U; ++n) {
+                const size_t h_bytes = static_cast<size_t>(column(n, o)) * 2;
+                const uint32_t block = s_term + static_cast<uint32_t>(ts) * kMlpBlock + to;
+                ok = ok && mlp_wait(smem_u32(&bars.term_empty[ts]), tphase ^ 1, failed);
+                if (ok) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (from[i]) cp_async16(block + 2048u * i, from[i] + h_bytes);
+                    for (int r = gt >> 2; r < sel_k; r += 8 * kMlpGatherWarps) {
+                        const int arow = arow_t[r];
+                        const uint32_t at = plan.anc + static_cast<uint32_t>(ts) * anc_stage +
+                                            static_cast<uint32_t>(r * 64 + ((ac ^ ((r >> 1) & 3)) << 4));
+                        if (arow >= 0)
+                            cp_async16(smem_u32(base + at), expanded + arow * ex_row + h_bytes + g * (kMlpHC / kG) * 2 + 16 * ac);
+                        else      // beyond the last row: every row's product reads it (times zero)
+                            *reinterpret_cast<uint4*>(base + at) = make_uint4(0, 0, 0, 0);
+                    }
+                    mlp_cp_async_arrive(smem_u32(&bars.term_full[ts]));
+                }
+                if (++ts == a.term_stages) { ts = 0; tphase ^= 1; }
+            }
+        }
+        cp_async_wait_all();
+    } else {
+        mlp_fewer_registers<kMlpOperandRegs>();
+        // ------------------------------------------------------------ indices, weights and operand products
+        const int gt = tid - 32 * (kMlpEpiWarps + 4 + kMlpGatherWarps), gw = gt >> 5;
+        const int K = 1 << a.k_shift, chunks = R / 8, rows_per_warp = 32 / chunks;
+        const size_t op_row = static_cast<size_t>(R) * 2;
+        const char* operand = static_cast<const char*>(a.operand_cache);
+        const int cc = lane % chunks, r_first = gw * rows_per_warp + lane / chunks, r_step = kMlpOperandWarps * rows_per_warp;
+        int tix = 0, u_at = 0;
+        bool ok = true;
+        // Tile `super`'s cache rows (its partners; the anchors of both of the pair's tiles) into buffer `b` and this
+        // thread's pair's weight into u.
         const auto indices = [&](int super, int b) {
+            if (gt >= kBM) return;                           // the first four warps, a pair each
             const int pair = (super * kG + g) * kBM + gt;
-            int prow = -1, arow = -1;
+            int prow = -1;
             float u = 0.0f;
             if (pair < a.n_pairs) {
                 const int srow = pair >> a.k_shift, k = pair & (K - 1);
                 const int query = srow / a.slots, slot = srow - query * a.slots;
                 const int seq = query / a.rows_per_seq, t = query - seq * a.rows_per_seq;
                 prow = seq * a.max_t + min(max(a.partner_index[pair], 0), a.max_t - 1);
-                arow = seq * a.max_t + min(max(a.anchor_index[srow], 0), a.max_t - 1);
                 int k_limit = K;
                 if (a.limited) k_limit = min(max(32 - __clz(t + 1), 1), K);          // ceil(log2(t + 2))
                 const float* sc = a.scores + (static_cast<size_t>(srow) << a.k_shift);
@@ -757,24 +869,34 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                 if (a.scale) u *= *a.scale;
             }
             prow_s[b * kBM + gt] = prow;
-            if ((gt & (K - 1)) == 0) arow_s[b * anchors + (gt >> a.k_shift)] = arow;
+            if (gt < sel_k) {
+                const int srow = super * sel_k + gt;
+                int arow = -1;
+                if (srow < a.n_pairs >> a.k_shift)
+                    arow = srow / a.slots / a.rows_per_seq * a.max_t + min(max(a.anchor_index[srow], 0), a.max_t - 1);
+                arow_s[b * sel_k + gt] = arow;
+            }
             u_s[u_at * kBM + gt] = u;
             __syncwarp();
-            if (ok && lane == 0) mlp_arrive(smem_u32(&bars.u_full[u_at]));
+            if (ok && lane == 0) {
+                mlp_arrive(smem_u32(&bars.rows_full[b]));
+                mlp_arrive(smem_u32(&bars.u_full[u_at]));
+            }
             if (++u_at == 3) u_at = 0;
         };
-        indices(cluster, 0);
+        if (cluster < n_super) indices(cluster, 0);
         for (int super = cluster; super < n_super; super += n_clusters, ++tix) {
             const int* prow_t = prow_s + (tix & 1) * kBM;
-            const int* arow_t = arow_s + (tix & 1) * anchors;
-            mlp_bar_sync(9, 32 * kMlpGatherWarps);           // this tile's rows are written, the other buffer is no longer read
-            // A tile: products of the operand rows, a lane per 16-byte chunk, eight rows' loads in flight
-            ok = ok && mlp_wait(smem_u32(&bars.a_empty), (tix & 1) ^ 1, failed);
-            for (int r0 = r_first; r0 < kBM; r0 += 8 * r_step) {
-                uint4 pv[8], av[8];
+            const int* arow_t = arow_s + (tix & 1) * sel_k + g * anchors;
+            mlp_bar_sync(9, 32 * kMlpOperandWarps);          // this tile's rows are written, the other buffer is no longer read
+            // a lane per 16-byte chunk; the products wait in registers until the A tile is free
+            uint4 product[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = r0 + i * r_step, prow = r < kBM ? prow_t[r] : -1;
+            for (int i0 = 0; i0 < 8; i0 += 2) {
+                uint4 pv[2], av[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int r = r_first + (i0 + i) * r_step, prow = r < kBM ? prow_t[r] : -1;
                     pv[i] = av[i] = make_uint4(0, 0, 0, 0);
                     if (prow >= 0) {
                         pv[i] = *reinterpret_cast<const uint4*>(operand + prow * op_row + 16 * cc);
@@ -782,65 +904,38 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = r0 + i * r_step;
-                    if (r >= kBM) break;
+                for (int i = 0; i < 2; ++i) {
                     float fp[8], fa[8];
                     unpack8(pv[i], kDt, fp);
                     unpack8(av[i], kDt, fa);
-                    *reinterpret_cast<uint4*>(base + plan.a + swizzled(r, cc, kMlpBlock)) =
-                        make_uint4(pack2(fp[0] * fa[0], fp[1] * fa[1], kDt), pack2(fp[2] * fa[2], fp[3] * fa[3], kDt),
-                                   pack2(fp[4] * fa[4], fp[5] * fa[5], kDt), pack2(fp[6] * fa[6], fp[7] * fa[7], kDt));
+                    product[i0 + i] = make_uint4(pack2(fp[0] * fa[0], fp[1] * fa[1], kDt), pack2(fp[2] * fa[2], fp[3] * fa[3], kDt),
+                                                 pack2(fp[4] * fa[4], fp[5] * fa[5], kDt), pack2(fp[6] * fa[6], fp[7] * fa[7], kDt));
                 }
+            }
+            ok = ok && mlp_wait(smem_u32(&bars.a_empty), (tix & 1) ^ 1, failed);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = r_first + i * r_step;
+                if (r < kBM) *reinterpret_cast<uint4*>(base + plan.a + swizzled(r, cc, kMlpBlock)) = product[i];
             }
             fence_proxy_async();
             __syncwarp();
-            if (ok && lane == 0) mlp_arrive_leader<kG>(smem_u32(&bars.a_full), leader);
-            // the expanded-cache segments of every block of this CTA
-            const int c = gt & 7;
-            int rows[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) rows[i] = prow_t[(gt >> 3) + 16 * i];
-            for (int j = 0; j < J; ++j) {
-                const size_t h_bytes = static_cast<size_t>((j * C + o) * kMlpHC) * 2 + 16 * c;
-                const uint32_t block = smem_u32(base + plan.term) + static_cast<uint32_t>(ts) * kMlpBlock;
-                ok = ok && mlp_wait(smem_u32(&bars.term_empty[ts]), tphase ^ 1, failed);
-                if (ok) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (rows[i] >= 0)
-                            cp_async16(block + swizzled((gt >> 3) + 16 * i, c, kMlpBlock),
-                                       expanded + rows[i] * ex_row + static_cast<size_t>(H) * 2 + h_bytes);
-                    for (int r = gt >> 3; r < anchors; r += 16) {
-                        const int arow = arow_t[r];
-                        if (arow >= 0)
-                            cp_async16(smem_u32(base + plan.anc) + static_cast<uint32_t>(ts * anchors + r) * kMlpAncStride + 16 * c,
-                                       expanded + arow * ex_row + h_bytes);
-                    }
-                    mlp_cp_async_arrive(smem_u32(&bars.term_full[ts]));
-                }
-                if (++ts == a.term_stages) { ts = 0; tphase ^= 1; }
-                if (j == 0 && super + n_clusters < n_super) indices(super + n_clusters, (tix & 1) ^ 1);
-            }
+            if (ok && lane == 0) mlp_arrive_leader(smem_u32(&bars.a_full), leader);
+            if (super + n_clusters < n_super) indices(super + n_clusters, (tix & 1) ^ 1);
         }
-        cp_async_wait_all();
     }
     // ---- leave together: no CTA may go while another still reads or signals its shared memory
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     mlp_cluster_sync();
     if (tid == 0 && failed_s && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
-    if (warp == kMlpEpiWarps + 1) {
-        if (kG == 1)
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_d2) : "memory");
-        else
-            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d2) : "memory");
-    }
+    if (warp == kMlpEpiWarps + 2)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_d2) : "memory");
 }
 
 // ------------------------------------------------------------------ host
 
-struct MlpShape { int outs, cols, term_stages, wm_stages, w2_stages; uint32_t smem; bool ok; };
+struct MlpShape { int outs, cols, wide, term_stages, wm_stages, w2_stages; uint32_t smem; bool ok; };
 
 bool power_of_two(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
@@ -850,31 +945,28 @@ int log2_of(int v) {
     return s;
 }
 
-// Output columns per CTA (tensor memory: cols of the second layer + 128 of the first), and the deepest
-// pipelines that fit the shared memory: three gathered blocks first (a gather is an L2 or DRAM round trip),
-// then W_2 stages.
-MlpShape mlp_shape(int rdim, int hdim, int d, int k_shift, int group_ctas) {
+// Output columns per CTA (tensor memory: cols of the second layer + one or two units of the first) and the
+// first of a list of pipeline depths that fits the shared memory.  At d = 512, K = 8, where two fit, two gathered
+// blocks with three W_2 stages measured 745 us for 262 144 pairs, three with two 786 us.
+MlpShape mlp_shape(int rdim, int hdim, int d, int k_shift) {
+    static constexpr int kDepths[][3] = {{4, 4, 2}, {3, 4, 2}, {3, 3, 2}, {3, 3, 1}, {2, 4, 1}, {2, 3, 1}, {2, 2, 1}};
     MlpShape s{};
     s.outs = d <= 384 ? 1 : 2;
     s.cols = d / s.outs;
-    if (d % s.outs != 0 || s.cols % 64 != 0 || s.cols > 384 || hdim % (kMlpHC * s.outs) != 0) return s;
-    for (int terms = 3; terms >= 2; --terms)
-        for (int wm = 2; wm >= 1; --wm)
-            for (int w2 = kMlpMaxStages; w2 >= 3 - (terms == 2); --w2) {
-                const MlpPlan p = mlp_plan(rdim, s.cols, s.outs, group_ctas, terms, wm, w2, k_shift);
-                if (p.total + 1024 <= static_cast<uint32_t>(kSmemDynamicLimit)) {
-                    s.term_stages = terms;
-                    s.w2_stages = w2;
-                    s.wm_stages = wm;
-                    s.smem = p.total + 1024;
-                    s.ok = true;
-                    return s;
-                }
-            }
+    if (d % s.outs != 0 || s.cols % 64 != 0 || s.cols > 384 || hdim % (2 * kMlpHC * s.outs) != 0 || hdim < 4 * kMlpHC * s.outs) return s;
+    s.wide = s.cols <= 256;
+    for (const auto& depth : kDepths) {
+        const MlpPlan p = mlp_plan(rdim, s.cols, s.outs, s.wide, depth[0], depth[2], depth[1], k_shift);
+        if (p.total + 1024 > static_cast<uint32_t>(kSmemDynamicLimit)) continue;
+        s.term_stages = depth[0];
+        s.w2_stages = depth[1];
+        s.wm_stages = depth[2];
+        s.smem = p.total + 1024;
+        s.ok = true;
+        break;
+    }
     return s;
 }
-
-constexpr int kGroupCtas = 2;
 
 // Clusters of this kernel that the device runs at a time (asked once per kernel, size and device): the grid
 // is persistent, a cluster beyond that number would only start when another has finished all its tiles.
@@ -905,17 +997,17 @@ int mlp_clusters(const void* kernel, int cluster, uint32_t smem) {
     return n;
 }
 
-template <int kDt, int kG>
+template <int kDt>
 int launch_mlp(const MlpArgs& a0, const MlpShape& s, const void* product_weight, const void* second_weight, void* stream) {
     MlpArgs a = a0;
     CUtensorMap map_wm, map_w2;
     const int n_inst = s.cols > 256 ? 2 : 1;
-    if (!make_map(&map_wm, product_weight, a.hdim, a.rdim, a.rdim, kMlpHC / kG, kDt) ||
+    if (!make_map(&map_wm, product_weight, a.hdim, a.rdim, a.rdim, (s.wide ? 2 : 1) * kMlpHC / kG, kDt) ||
         !make_map(&map_w2, second_weight, a.d, a.hdim, a.hdim, s.cols / n_inst / kG, kDt)) {
         set_error("relation_mlp_rows: tensor map encoding failed");
         return RLM_ERR_LAUNCH;
     }
-    auto* kernel = relation_mlp_rows_kernel<kDt, kG>;
+    auto* kernel = relation_mlp_rows_kernel<kDt>;
     if (int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta)) return rc;
     const int cluster = s.outs * kG, n_super = (a.n_tiles + kG - 1) / kG;
     const int most = mlp_clusters(reinterpret_cast<const void*>(kernel), cluster, s.smem);
@@ -931,10 +1023,10 @@ int launch_mlp(const MlpArgs& a0, const MlpShape& s, const void* product_weight,
 extern "C" int rlm_relation_mlp_rows_supported(int k_out, int slots, int relation_dim, int hidden_dim, int d_model, int dtype) {
     using namespace rlm;
     if (dtype != RLM_BF16 && dtype != RLM_F16) return 0;
-    if (!power_of_two(k_out) || !power_of_two(slots) || k_out * slots > 32 || k_out < 2 || slots > 8) return 0;
+    if (!power_of_two(k_out) || !power_of_two(slots) || k_out * slots > 32 || k_out < 4 || k_out > 16 || slots > 8) return 0;
     if (relation_dim != 64 && relation_dim != 128) return 0;
     if (d_model < 64 || hidden_dim < kMlpHC) return 0;
-    return mlp_shape(relation_dim, hidden_dim, d_model, log2_of(k_out), kGroupCtas).ok ? 1 : 0;
+    return mlp_shape(relation_dim, hidden_dim, d_model, log2_of(k_out)).ok ? 1 : 0;
 }
 
 extern "C" int rlm_relation_mlp_rows(
@@ -967,12 +1059,12 @@ extern "C" int rlm_relation_mlp_rows(
                           static_cast<const void*>(residual)})
         if (!aligned16(q)) { set_error("relation_mlp_rows: tensors must be 16-byte aligned"); return RLM_ERR_ALIGN; }
     const int k_shift = log2_of(k_out);
-    const MlpShape s = mlp_shape(relation_dim, hidden_dim, d_model, k_shift, kGroupCtas);
+    const MlpShape s = mlp_shape(relation_dim, hidden_dim, d_model, k_shift);
     const int n_inst = s.cols > 256 ? 2 : 1;
     const uint32_t fmt = dtype == RLM_BF16 ? 1u : 0u;
     const auto idesc = [&](int n) {
         return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-               (static_cast<uint32_t>((kBM * kGroupCtas) >> 4) << 24);
+               (static_cast<uint32_t>((kBM * kG) >> 4) << 24);
     };
     MlpArgs a{};
     a.expanded_cache = expanded_cache;
@@ -1006,8 +1098,11 @@ extern "C" int rlm_relation_mlp_rows(
     a.term_stages = s.term_stages;
     a.w2_stages = s.w2_stages;
     a.wm_stages = s.wm_stages;
-    a.idesc1 = idesc(kMlpHC);
+    a.wide = s.wide;
+    a.inv_d = 1.0f / static_cast<float>(d_model);
+    a.idesc_block = idesc(kMlpHC);
+    a.idesc_unit = idesc(2 * kMlpHC);
     a.idesc2 = idesc(s.cols / n_inst);
-    return dtype == RLM_BF16 ? launch_mlp<RLM_BF16, kGroupCtas>(a, s, product_weight, second_weight, stream)
-                             : launch_mlp<RLM_F16, kGroupCtas>(a, s, product_weight, second_weight, stream);
+    return dtype == RLM_BF16 ? launch_mlp<RLM_BF16>(a, s, product_weight, second_weight, stream)
+                             : launch_mlp<RLM_F16>(a, s, product_weight, second_weight, stream);
 }

@@ -29,7 +29,7 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor, nn
 
-from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
+from relation_lm.kernels.relation_reduce import MLP_ROWS_MIN_PAIRS, relation_mlp_rows, relation_mlp_rows_supported
 
 
 @dataclass
@@ -267,7 +267,7 @@ class MultiAnchorPrefill:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
-        fused = self.fused_mlp and keep is None
+        fused = self.fused_mlp and keep is None and N * S * K >= MLP_ROWS_MIN_PAIRS
         if selected is None or not fused:
             rb, rp = self.rows(B, T)
         if selected is None:

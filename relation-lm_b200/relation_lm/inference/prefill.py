@@ -27,7 +27,7 @@ from torch import Tensor
 
 from relation_lm.inference.routed_model import RoutedRelationLM
 from relation_lm.kernels.packed_projection import layer_norm_cast, packed_projection
-from relation_lm.kernels.relation_reduce import (relation_hidden_cached_rows_out, relation_mlp_rows,
+from relation_lm.kernels.relation_reduce import (MLP_ROWS_MIN_PAIRS, relation_hidden_cached_rows_out, relation_mlp_rows,
                                                  relation_mlp_rows_supported, relation_norm_reduce_rows)
 from relation_lm.kernels.relation_select import relation_select_packed_prefill, relation_select_packed_rows
 from relation_lm.kernels.router_cache import router_cache_prefill
@@ -44,8 +44,7 @@ class RoutedPrefillLayer:
         self.config, self.layer, self.device, self.dtype = model.config, int(layer), torch.device(device), dtype
         w = model.decode_weights(self.device, dtype)
         cfg, l = self.config, self.layer
-        # the relation MLP, norm-reduce and residual as one launch where its tiles fit (never more than the three
-        # launches it replaces cost, from a few hundred rows up)
+        # the relation MLP, norm-reduce and residual as one launch
         self.fused_mlp = relation_mlp_rows_supported(cfg.k_max, 1, cfg.relation_dim, cfg.hidden_dim, cfg.d_model, dtype)
         width = cfg.packed_width
         self.w = {
@@ -123,7 +122,7 @@ class RoutedPrefillLayer:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
-        fused = self.fused_mlp and keep is None
+        fused = self.fused_mlp and keep is None and N * K >= MLP_ROWS_MIN_PAIRS
         if selected is None or not fused:
             rb, rp = self.rows(B, T)
         if selected is None:

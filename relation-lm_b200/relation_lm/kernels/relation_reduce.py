@@ -480,9 +480,15 @@ def _(raw, partner_scores, norm_weight, norm_bias, row_position, norm_eps):
     return raw.new_empty((raw.size(0), raw.size(2)), dtype=torch.float32)
 
 
+# Half a tile of 128 pairs for each of a B200's 148 SMs.  The one-launch form walks a tile's hidden columns one
+# after another (37 us for a tile of 256 pairs at d 256); below this the three launches, which spread the
+# hidden columns over the SMs, take less (27 us for 4096 pairs at d 256).
+MLP_ROWS_MIN_PAIRS = 9472
+
+
 def relation_mlp_rows_supported(k_out: int, slots: int, relation_dim: int, hidden_dim: int, d_model: int,
                                 dtype: torch.dtype) -> bool:
-    """Whether ``relation_mlp_rows`` serves these sizes."""
+    """Whether ``relation_mlp_rows`` serves these sizes.  Worth it from ``MLP_ROWS_MIN_PAIRS`` pairs up."""
     return dtype in (torch.bfloat16, torch.float16) and bool(_abi.LIB.rlm_relation_mlp_rows_supported(
         int(k_out), int(slots), int(relation_dim), int(hidden_dim), int(d_model), _abi.DTYPE_CODE[dtype]))
 
