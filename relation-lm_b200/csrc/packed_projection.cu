@@ -634,9 +634,11 @@ __global__ void __launch_bounds__(kGemmThreads) norm_projection_kernel(
 
 // ------------------------------------------------------------------ LayerNorm -> 16-bit rows
 //
-// For batches beyond one row tile the normalisation is done once (one warp per row) into a
-// 16-bit matrix that packed_projection_kernel then streams with TMA, instead of once per
-// output-column tile.  Arithmetic identical to the fused kernel above.
+// For batches beyond one row tile the normalisation is done once (a warp per row) into a 16-bit matrix that
+// packed_projection_kernel then streams with TMA, instead of once per output-column tile.  Arithmetic
+// identical to the fused kernel above.  A stream of 6 bytes per element: bound by DRAM as long as nothing
+// else is loaded per row, so a warp keeps its lanes' affine parameters in registers and walks rows.  (With
+// one row per warp and the parameters read element by element: 41 us for 32 768 x 512, 2.4 TB/s.)
 constexpr int kCastThreads = 256;
 
 struct NormCastArgs {
@@ -646,63 +648,79 @@ struct NormCastArgs {
     void* out;
     int64_t x_stride;
     float eps;
-    int m, k, out_dtype;
+    int m, k;
 };
 
+template <int kChunks, bool kBf16>
 __global__ void __launch_bounds__(kCastThreads) layer_norm_cast_kernel(const NormCastArgs a) {
-    griddep_sync();
-    const int lane = threadIdx.x & 31;
-    const int r = blockIdx.x * (kCastThreads / 32) + (threadIdx.x >> 5);
-    if (r >= a.m) return;
-    const int chunks = a.k / 8;
-    const float* row = a.x + r * a.x_stride;
-    float v[kNormMaxPerLane][8];
-    float sum = 0.0f;
+    const int lane = threadIdx.x & 31, chunks = a.k / 8;
+    float4 g[kChunks][2], b[kChunks][2];
 #pragma unroll
-    for (int i = 0; i < kNormMaxPerLane; ++i) {
+    for (int i = 0; i < kChunks; ++i) {
         const int c = lane + 32 * i;
-        if (c < chunks) {
-            const float4 lo = *reinterpret_cast<const float4*>(row + 8 * c);
-            const float4 hi = *reinterpret_cast<const float4*>(row + 8 * c + 4);
+        const bool live = a.gamma && c < chunks;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            g[i][h] = live ? *reinterpret_cast<const float4*>(a.gamma + 8 * c + 4 * h) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+            b[i][h] = live ? *reinterpret_cast<const float4*>(a.beta + 8 * c + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+    griddep_sync();
+    const int warps = gridDim.x * (kCastThreads / 32);
+    for (int r = blockIdx.x * (kCastThreads / 32) + (threadIdx.x >> 5); r < a.m; r += warps) {
+        const float* row = a.x + r * a.x_stride;
+        float v[kChunks][8];
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+            const int c = lane + 32 * i;
+            const bool live = c < chunks;
+            const float4 lo = live ? *reinterpret_cast<const float4*>(row + 8 * c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 hi = live ? *reinterpret_cast<const float4*>(row + 8 * c + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             v[i][0] = lo.x; v[i][1] = lo.y; v[i][2] = lo.z; v[i][3] = lo.w;
             v[i][4] = hi.x; v[i][5] = hi.y; v[i][6] = hi.z; v[i][7] = hi.w;
+        }
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i)
 #pragma unroll
             for (int e = 0; e < 8; ++e) sum += v[i][e];
+        float mean = 0.0f, inv = 1.0f;
+        if (a.gamma) {
+            mean = warp_sum(sum) / static_cast<float>(a.k);
+            float sq = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i)
+                if (lane + 32 * i < chunks)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) { const float d = v[i][e] - mean; sq = fmaf(d, d, sq); }
+            inv = rsqrtf(warp_sum(sq) / static_cast<float>(a.k) + a.eps);
+        }
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+            const int c = lane + 32 * i;
+            if (c >= chunks) continue;
+            const float ge[8] = {g[i][0].x, g[i][0].y, g[i][0].z, g[i][0].w, g[i][1].x, g[i][1].y, g[i][1].z, g[i][1].w};
+            const float be[8] = {b[i][0].x, b[i][0].y, b[i][0].z, b[i][0].w, b[i][1].x, b[i][1].y, b[i][1].z, b[i][1].w};
+            uint32_t packed[4];
+#pragma unroll
+            for (int e = 0; e < 8; e += 2)
+                packed[e / 2] = pack2(fmaf((v[i][e] - mean) * inv, ge[e], be[e]), fmaf((v[i][e + 1] - mean) * inv, ge[e + 1], be[e + 1]),
+                                      kBf16 ? RLM_BF16 : RLM_F16);
+            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + static_cast<size_t>(r) * a.k + 8 * c) =
+                make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
     }
-    float mean = 0.0f, inv = 1.0f;
-    if (a.gamma) {
-        mean = warp_sum(sum) / static_cast<float>(a.k);
-        float sq = 0.0f;
-#pragma unroll
-        for (int i = 0; i < kNormMaxPerLane; ++i)
-            if (lane + 32 * i < chunks)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) { float d = v[i][e] - mean; sq = fmaf(d, d, sq); }
-        inv = rsqrtf(warp_sum(sq) / static_cast<float>(a.k) + a.eps);
-    }
-#pragma unroll
-    for (int i = 0; i < kNormMaxPerLane; ++i) {
-        const int c = lane + 32 * i;
-        if (c >= chunks) continue;
-        uint32_t packed[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-            float y0 = (v[i][e] - mean) * inv, y1 = (v[i][e + 1] - mean) * inv;
-            if (a.gamma) {
-                y0 = fmaf(y0, a.gamma[8 * c + e], a.beta[8 * c + e]);
-                y1 = fmaf(y1, a.gamma[8 * c + e + 1], a.beta[8 * c + e + 1]);
-            }
-            if (a.out_dtype == RLM_BF16) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
-                packed[e / 2] = *reinterpret_cast<uint32_t*>(&h);
-            } else {
-                __half2 h = __floats2half2_rn(y0, y1);
-                packed[e / 2] = *reinterpret_cast<uint32_t*>(&h);
-            }
-        }
-        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + static_cast<size_t>(r) * a.k + 8 * c) =
-            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
+
+template <bool kBf16>
+void launch_norm_cast(const NormCastArgs& a, void* stream) {
+    const int per_cta = kCastThreads / 32, most = 8 * sm_count(), need = (a.m + per_cta - 1) / per_cta;
+    const dim3 grid(need < most ? need : most), block(kCastThreads);
+    switch ((a.k + 255) / 256) {
+        case 1: launch_kernel(layer_norm_cast_kernel<1, kBf16>, grid, block, 0, stream, a); break;
+        case 2: launch_kernel(layer_norm_cast_kernel<2, kBf16>, grid, block, 0, stream, a); break;
+        case 3: launch_kernel(layer_norm_cast_kernel<3, kBf16>, grid, block, 0, stream, a); break;
+        default: launch_kernel(layer_norm_cast_kernel<4, kBf16>, grid, block, 0, stream, a); break;
     }
 }
 
@@ -813,9 +831,9 @@ extern "C" int rlm_layer_norm_cast(const float* x, int64_t x_row_stride, const f
     }
     NormCastArgs a{};
     a.x = x; a.gamma = gamma; a.beta = beta; a.out = out; a.x_stride = x_row_stride; a.eps = eps;
-    a.m = rows; a.k = d_in; a.out_dtype = out_dtype;
-    const int per_cta = kCastThreads / 32;
-    launch_kernel(layer_norm_cast_kernel, dim3((rows + per_cta - 1) / per_cta), dim3(kCastThreads), 0, stream, a);
+    a.m = rows; a.k = d_in;
+    if (out_dtype == RLM_BF16) launch_norm_cast<true>(a, stream);
+    else launch_norm_cast<false>(a, stream);
     count_launch();
     return check_launch("layer_norm_cast_kernel");
 }
