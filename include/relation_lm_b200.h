@@ -712,6 +712,22 @@ int rlm_relation_mlp_rows(
     int rows_per_seq, int max_t, int relation_dim, int hidden_dim, int d_model, int k_out, int limit_by_position, int dtype,
     int32_t* status, void* stream);
 
+/*
+ * The memory-side state of whole sequences from their packed projection rows in one launch (extension): token
+ * caches, raw and convolved router keys, block statistics — equal to column copies and
+ * rlm_router_cache_prefill over zeroed caches, bit for bit.  `packed` rows (batch * max_t of them, row stride in
+ * elements) hold, with slots = 0, anchor key 64 | partner key 64 | operand R | partner-anchor 128 | two router
+ * keys 64; with slots = S >= 1, S times (anchor key | partner key | partner-anchor | two router keys), then the
+ * operand.  Caches: keys and router caches [S, B, T, 64], partner-anchor [S, B, T, 128], operand [B, T, R],
+ * statistics [S, B, T / block_size, 4, 16], conv weights [S, 64, 3].  Rows and caches share bf16 or fp16.
+ */
+int rlm_sequence_state(
+    const void* packed, int64_t row_stride, int slots, int relation_dim, void* anchor_keys, void* partner_keys,
+    void* operand_cache, void* partner_anchor_cache, void* anchor_raw_cache, void* partner_raw_cache,
+    void* anchor_conv_cache, void* partner_conv_cache, void* anchor_mean, void* anchor_std, void* partner_mean,
+    void* partner_std, const void* anchor_conv_weight, const void* partner_conv_weight, int batch, int max_t,
+    int block_size, int dtype, int weight_dtype, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

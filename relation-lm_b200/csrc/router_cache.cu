@@ -224,6 +224,118 @@ __global__ void __launch_bounds__(kThreads) router_cache_prefill_kernel(const Pr
     store_scalar(a.stdv[s], stat, a.stats_dtype, sd);
 }
 
+// The whole memory-side state of sequences from their packed projection rows, in one launch: the token
+// caches (copies of packed columns), the raw router keys, their causal convolution and the block statistics —
+// what column copies followed by router_cache_prefill on zeroed caches leave, bit for bit.  One CTA per block
+// of positions, sequence and slot.  Bound by DRAM: every packed column is read once and written once, in
+// 16-byte pieces; the convolution runs on a tile in shared memory, a thread per eight channels, and only the
+// statistics, whose sums are ordered by position, walk the block's rows, a thread per channel.  (As four
+// strided copies, eight fills and a kernel that walked the rows in global memory: 91 us for 8 sequences of
+// 4096 positions; per anchor slot 30 us more for each.)
+constexpr int kSeqThreads = 256;
+
+struct SequenceArgs {
+    const uint16_t* packed;                  // [B, T, row_stride]
+    int64_t row_stride;
+    int slot_stride, router_at[2], key_at[2], partner_anchor_at, operand_at, rdim;
+    void* key[2];                            // [S, B, T, 64]
+    void* partner_anchor;                    // [S, B, T, 128]
+    void* operand;                           // [B, T, R]
+    void* raw[2];                            // [S, B, T, 64]
+    void* conv[2];
+    void* mean[2];                           // [S, B, NB, 64]
+    void* stdv[2];
+    const void* weight[2];                   // [S, 64, 3]
+    int batch, max_t, n_blocks, block_size, weight_dtype;
+};
+
+template <int kDt>
+__global__ void __launch_bounds__(kSeqThreads) sequence_state_kernel(const SequenceArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ float last[kThreads];                            // the block's last row before rounding
+    const int tid = threadIdx.x, blk = blockIdx.x, b = blockIdx.y, slot = blockIdx.z, bs = a.block_size, start = blk * bs;
+    uint16_t* raw_s = reinterpret_cast<uint16_t*>(smem);        // [bs + 2][128]: two rows of history first
+    uint16_t* conv_s = raw_s + (bs + 2) * kThreads;             // [bs][128]
+    // this thread's eight channels of the convolution
+    const int chunk = tid & 15, stream = chunk >> 3, ch = 8 * (chunk & 7);
+    float w[3][8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            w[k][e] = load_scalar(a.weight[stream], (static_cast<int64_t>(slot) * kD + ch + e) * 3 + k, a.weight_dtype);
+    griddep_sync();
+    const int64_t seq = static_cast<int64_t>(slot) * a.batch + b;
+    const uint16_t* rows = a.packed + (static_cast<int64_t>(b) * a.max_t + start) * a.row_stride + slot * a.slot_stride;
+    // router keys into shared memory and the raw caches
+    for (int i = tid; i < (bs + 2) * 16; i += kSeqThreads) {
+        const int r = (i >> 4) - 2;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (start + r >= 0) v = *reinterpret_cast<const uint4*>(rows + r * a.row_stride + a.router_at[stream] + ch);
+        *reinterpret_cast<uint4*>(raw_s + (r + 2) * kThreads + 8 * chunk) = v;
+        if (r >= 0) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.raw[stream]) + (seq * a.max_t + start + r) * kD + ch) = v;
+    }
+    // token features
+    const auto copy = [&](int at, int width, void* to, int64_t row0) {
+        const int chunks = width / 8;
+#pragma unroll 4
+        for (int i = tid; i < bs * chunks; i += kSeqThreads) {
+            const int r = i / chunks, c = i - r * chunks;
+            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(to) + (row0 + r) * width + 8 * c) =
+                *reinterpret_cast<const uint4*>(rows + r * a.row_stride + at + 8 * c);
+        }
+    };
+    copy(a.key_at[0], kD, a.key[0], seq * a.max_t + start);
+    copy(a.key_at[1], kD, a.key[1], seq * a.max_t + start);
+    copy(a.partner_anchor_at, 128, a.partner_anchor, seq * a.max_t + start);
+    if (slot == 0) copy(a.operand_at, a.rdim, a.operand, static_cast<int64_t>(b) * a.max_t + start);
+    __syncthreads();
+    for (int r = tid >> 4; r < bs; r += kSeqThreads / 16) {
+        const int p = start + r;
+        float cur[8], prev1[8], prev2[8], y[8];
+        load8(raw_s + (r + 2) * kThreads, 8 * chunk, kDt, cur);
+        load8(raw_s + (r + 1) * kThreads, 8 * chunk, kDt, prev1);
+        load8(raw_s + r * kThreads, 8 * chunk, kDt, prev2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            float v = __fmul_rn(cur[e], w[2][e]);
+            v = __fadd_rn(v, __fmul_rn(__fmul_rn(prev1[e], w[1][e]), p >= 1 ? 1.0f : 0.0f));
+            y[e] = __fadd_rn(v, __fmul_rn(__fmul_rn(prev2[e], w[0][e]), p >= 2 ? 1.0f : 0.0f));
+            if (r == bs - 1) last[8 * chunk + e] = y[e];
+        }
+        uint32_t packed[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (kDt == RLM_BF16) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
+                packed[e] = *reinterpret_cast<const uint32_t*>(&h);
+            } else {
+                const __half2 h = __floats2half2_rn(y[2 * e], y[2 * e + 1]);
+                packed[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        }
+        const uint4 v = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        *reinterpret_cast<uint4*>(conv_s + r * kThreads + 8 * chunk) = v;
+        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.conv[stream]) + (seq * a.max_t + p) * kD + ch) = v;
+    }
+    __syncthreads();
+    if (tid >= kThreads) return;
+    // statistics: rounded values for the rows before the block's last, the fp32 value for that row
+    float sum = 0.0f;
+    for (int r = 0; r < bs - 1; ++r) sum = __fadd_rn(sum, load_scalar(conv_s, r * kThreads + tid, kDt));
+    sum = __fadd_rn(sum, last[tid]);
+    const float mean = __fdiv_rn(sum, static_cast<float>(bs));
+    float acc = 0.0f;
+    for (int r = 0; r < bs; ++r) {
+        const float d = __fsub_rn(r == bs - 1 ? last[tid] : load_scalar(conv_s, r * kThreads + tid, kDt), mean);
+        acc = __fmaf_rn(d, d, acc);
+    }
+    const float sd = __fsqrt_rn(__fdiv_rn(acc, static_cast<float>(bs)));
+    const int64_t stat = (seq * a.n_blocks + blk) * kD + tid % kD;
+    store_scalar(a.mean[tid / kD], stat, kDt, mean);
+    store_scalar(a.stdv[tid / kD], stat, kDt, sd);
+}
+
 int validate_and_launch(RouterArgs& a, void* stream, const char* who) {
     if (a.batch == 0 || a.layers == 0) return RLM_OK;
     if (a.batch < 0 || a.layers < 0 || a.max_t < 1 || a.n_blocks < 1 || a.block_size < 1 ||
@@ -370,4 +482,62 @@ extern "C" int rlm_router_cache_prefill(
     launch_kernel(router_cache_prefill_kernel, dim3(grid), dim3(kThreads), 0, stream, a);
     count_launch();
     return check_launch("router_cache_prefill_kernel");
+}
+
+extern "C" int rlm_sequence_state(
+    const void* packed, int64_t row_stride, int slots, int relation_dim, void* anchor_keys, void* partner_keys,
+    void* operand_cache, void* partner_anchor_cache, void* anchor_raw_cache, void* partner_raw_cache,
+    void* anchor_conv_cache, void* partner_conv_cache, void* anchor_mean, void* anchor_std, void* partner_mean,
+    void* partner_std, const void* anchor_conv_weight, const void* partner_conv_weight, int batch, int max_t,
+    int block_size, int dtype, int weight_dtype, void* stream) {
+    using namespace rlm;
+    if (batch == 0 || max_t == 0) return RLM_OK;
+    const void* need[] = {packed, anchor_keys, partner_keys, operand_cache, partner_anchor_cache, anchor_raw_cache,
+                          partner_raw_cache, anchor_conv_cache, partner_conv_cache, anchor_mean, anchor_std, partner_mean,
+                          partner_std, anchor_conv_weight, partner_conv_weight};
+    for (const void* q : need)
+        if (!q) { set_error("sequence_state: NULL pointer"); return RLM_ERR_NULL; }
+    const int width = slots > 0 ? 384 * slots + relation_dim : 384 + relation_dim;
+    if (batch < 0 || max_t < 0 || slots < 0 || block_size < 1 || max_t % block_size != 0 || relation_dim < 8 ||
+        relation_dim % 8 != 0 || row_stride < width || row_stride % 8 != 0 || batch > 65535 || slots > 65535) {
+        set_error("sequence_state: need whole blocks, a relation width that is a multiple of 8 and rows of that layout");
+        return RLM_ERR_SHAPE;
+    }
+    if ((dtype != RLM_BF16 && dtype != RLM_F16) || !valid_dtype(weight_dtype)) {
+        set_error("sequence_state: rows and caches must be bfloat16 or float16");
+        return RLM_ERR_DTYPE;
+    }
+    for (int i = 0; i < 9; ++i)
+        if (!aligned16(need[i])) { set_error("sequence_state: rows and caches must be 16-byte aligned"); return RLM_ERR_ALIGN; }
+    SequenceArgs a{};
+    a.packed = static_cast<const uint16_t*>(packed);
+    a.row_stride = row_stride;
+    a.rdim = relation_dim;
+    a.slot_stride = 384;
+    a.key_at[0] = 0;
+    a.key_at[1] = 64;
+    // one layer: keys | operand | partner-anchor | router keys; slots: (keys | partner-anchor | router keys) * S | operand
+    a.operand_at = slots > 0 ? 384 * slots : 128;
+    a.partner_anchor_at = slots > 0 ? 128 : 128 + relation_dim;
+    a.router_at[0] = a.partner_anchor_at + 128;
+    a.router_at[1] = a.partner_anchor_at + 192;
+    a.key[0] = anchor_keys; a.key[1] = partner_keys;
+    a.partner_anchor = partner_anchor_cache; a.operand = operand_cache;
+    a.raw[0] = anchor_raw_cache; a.raw[1] = partner_raw_cache;
+    a.conv[0] = anchor_conv_cache; a.conv[1] = partner_conv_cache;
+    a.mean[0] = anchor_mean; a.mean[1] = partner_mean;
+    a.stdv[0] = anchor_std; a.stdv[1] = partner_std;
+    a.weight[0] = anchor_conv_weight; a.weight[1] = partner_conv_weight;
+    a.batch = batch; a.max_t = max_t; a.n_blocks = max_t / block_size; a.block_size = block_size; a.weight_dtype = weight_dtype;
+    const int smem_bytes = (2 * block_size + 2) * kThreads * 2;
+    auto kernel = dtype == RLM_BF16 ? sequence_state_kernel<RLM_BF16> : sequence_state_kernel<RLM_F16>;
+    if (smem_bytes > kSmemDynamicLimit) {
+        set_error("sequence_state: block tile exceeds 227 KB of shared memory");
+        return RLM_ERR_SMEM;
+    }
+    if (smem_bytes > 48 * 1024)
+        if (int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta)) return rc;
+    launch_kernel(kernel, dim3(a.n_blocks, batch, slots > 0 ? slots : 1), dim3(kSeqThreads), smem_bytes, stream, a);
+    count_launch();
+    return check_launch("sequence_state_kernel");
 }

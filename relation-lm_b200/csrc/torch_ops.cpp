@@ -19,6 +19,7 @@
 #include <mutex>
 #include <optional>
 #include <tuple>
+#include <vector>
 
 #include "../../include/relation_lm_b200.h"
 
@@ -412,6 +413,35 @@ void router_cache_prefill(const Tensor& anchor_raw, const Tensor& partner_raw, R
                                    partner_raw.stride(1), partner_raw.stride(0), ROUTER_POINTERS, anchor_raw.size(1),
                                    anchor_raw.size(0), anchor_raw_cache.size(1), anchor_mean.size(1), block_size,
                                    same_dtype("raw key", {&anchor_raw, &partner_raw}), ROUTER_DTYPES, launch.stream));
+}
+
+std::vector<Tensor> sequence_state(const Tensor& packed, int64_t slots, int64_t relation_dim, int64_t block_size,
+                                   const Tensor& anchor_conv_weight, const Tensor& partner_conv_weight) {
+    const c10::Device device = contiguous({ARG(packed), ARG(anchor_conv_weight), ARG(partner_conv_weight)});
+    const int64_t n = slots > 0 ? slots : 1;
+    TORCH_CHECK_VALUE(packed.dim() == 3 && slots >= 0 && block_size >= 1 && packed.size(2) == 384 * n + relation_dim &&
+                          anchor_conv_weight.numel() == n * 192 && partner_conv_weight.numel() == n * 192,
+                      "packed must be [B, T, 384 * slots + R] and the conv weights [slots, 64, 3]");
+    const int64_t batch = packed.size(0), length = packed.size(1);
+    const int dtype = code(packed), weight = same_dtype("conv weight", {&anchor_conv_weight, &partner_conv_weight});
+    Launch launch(device);
+    const auto make = [&](std::initializer_list<int64_t> tail, bool slotted) {
+        std::vector<int64_t> shape;
+        if (slotted && slots > 0) shape.push_back(slots);
+        shape.push_back(batch);
+        shape.insert(shape.end(), tail);
+        return empty(shape, packed.scalar_type(), device);
+    };
+    const int64_t nb = length / block_size;
+    std::vector<Tensor> t = {make({length, 64}, true), make({length, 64}, true), make({length, relation_dim}, false),
+                             make({length, 128}, true)};
+    for (int i = 0; i < 4; ++i) t.push_back(make({length, 64}, true));
+    for (int i = 0; i < 4; ++i) t.push_back(make({nb, 4, 16}, true));
+    check(rlm_sequence_state(ptr(packed), packed.size(2), slots, relation_dim, ptr(t[0]), ptr(t[1]), ptr(t[2]), ptr(t[3]),
+                             ptr(t[4]), ptr(t[5]), ptr(t[6]), ptr(t[7]), ptr(t[8]), ptr(t[9]), ptr(t[10]), ptr(t[11]),
+                             ptr(anchor_conv_weight), ptr(partner_conv_weight), batch, length, block_size, dtype, weight,
+                             launch.stream));
+    return t;
 }
 
 // ------------------------------------------------------------------ relation hidden rows
@@ -948,6 +978,8 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
             "Tensor(a4!) anchor_conv_cache, Tensor(a5!) partner_conv_cache, Tensor(a6!) anchor_mean, "                   \
             "Tensor(a7!) anchor_std, Tensor(a8!) partner_mean, Tensor(a9!) partner_std, Tensor anchor_conv_weight, "     \
             "Tensor partner_conv_weight, SymInt block_size) -> ()")                                                      \
+    PURE(sequence_state, "(Tensor packed, SymInt slots, SymInt relation_dim, SymInt block_size, "                        \
+         "Tensor anchor_conv_weight, Tensor partner_conv_weight) -> Tensor[]")                                           \
     PURE(relation_hidden_cached, "(Tensor expanded_cache, Tensor operand_cache, Tensor anchor_index, "                   \
          "Tensor partner_index, Tensor product_weight) -> Tensor")                                                       \
     MUTATES(relation_hidden_cached_out, "(Tensor(a0!) out, Tensor expanded_cache, Tensor operand_cache, "                \

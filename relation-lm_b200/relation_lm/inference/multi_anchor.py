@@ -10,7 +10,7 @@ below is the routed form of the reference's ``forward`` for all positions at onc
 1. per block, memory side (``build_state``): one packed projection of ``memory`` for all slots
    — per slot anchor key | partner key | anchor half of the partner query (exact 64 + router 64)
    | anchor router key | partner router key, then the shared operand — split into per-slot
-   caches; ``router_cache_prefill`` per slot and stream; the expanded cache of the factorised
+   caches with every slot's and stream's router state (``sequence_state``); the expanded cache of the factorised
    first relation-MLP layer;
 2. query side (``forward``): LayerNorm -> one projection for all slots' queries ->
    ``relation_select_multi_rows`` (distinct anchors, anchors barred from every partner set) ->
@@ -188,7 +188,7 @@ class MultiAnchorPrefill:
         if dtype not in (torch.bfloat16, torch.float16):
             raise ValueError("the routed pass runs its projections on the tensor cores: bfloat16 or float16")
         self.config, self.device, self.dtype = stack.config, torch.device(device), dtype
-        self.tiled_select = bool(tiled_select)           # whole-sequence selector (bfloat16) instead of the per-row one
+        self.tiled_select = bool(tiled_select)           # whole-sequence selector instead of the per-row one
         cfg = stack.config
         # one launch for the relation MLP, norm-reduce and (slot counts that are powers of two) the slot mixing
         sizes = (cfg.relation_dim, cfg.hidden_dim, cfg.d_model, dtype)
@@ -206,31 +206,14 @@ class MultiAnchorPrefill:
     def build_state(self, layer: int, memory: Tensor) -> dict[str, Tensor]:
         """Per-slot caches and block statistics of layer ``layer`` for ``memory [B, T, d]`` (16-bit)."""
         from relation_lm.kernels.packed_projection import packed_projection
-        from relation_lm.kernels.router_cache import router_cache_prefill
+        from relation_lm.kernels.router_cache import sequence_state
 
         cfg, w = self.config, self.layers[layer]
         B, T, d = memory.shape
-        S, R, H, nb = cfg.anchors_per_block, cfg.relation_dim, cfg.hidden_dim, T // cfg.block_size
+        S, R, H = cfg.anchors_per_block, cfg.relation_dim, cfg.hidden_dim
         packed = packed_projection(memory.reshape(B * T, d), w["w_memory"]).view(B, T, S * 384 + R)
-        slots = packed[..., :S * 384].view(B, T, S, 384)
-
-        def per_slot(lo, hi):
-            return slots[..., lo:hi].permute(2, 0, 1, 3).contiguous()          # [S, B, T, width]
-
-        state = {"anchor_keys": per_slot(0, 64), "partner_keys": per_slot(64, 128),
-                 "partner_anchor_cache": per_slot(128, 256),
-                 "operand_cache": packed[..., S * 384:].contiguous(), "packed": packed}
-        zeros = lambda *shape: torch.zeros(*shape, device=self.device, dtype=self.dtype)  # noqa: E731
-        for n in ("anchor_raw_cache", "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache"):
-            state[n] = zeros(S, B, T, 64)
-        for n in ("anchor_mean", "anchor_std", "partner_mean", "partner_std"):
-            state[n] = zeros(S, B, nb, 4, 16)
-        for s in range(S):
-            router_cache_prefill(slots[:, :, s, 256:320], slots[:, :, s, 320:384], state["anchor_raw_cache"][s],
-                                 state["partner_raw_cache"][s], state["anchor_conv_cache"][s],
-                                 state["partner_conv_cache"][s], state["anchor_mean"][s], state["anchor_std"][s],
-                                 state["partner_mean"][s], state["partner_std"][s], w["anchor_conv_weight"][s],
-                                 w["partner_conv_weight"][s], cfg.block_size)
+        state = sequence_state(packed, S, R, cfg.block_size, w["anchor_conv_weight"], w["partner_conv_weight"])
+        state["packed"] = packed
         state["expanded_cache"] = packed_projection(state["operand_cache"].view(B * T, R), w["w_expand"],
                                                     w["b_expand"]).view(B, T, 2 * H)
         return state

@@ -9,9 +9,9 @@ whole-sequence form: the per-row operators of this library (``*_rows``) applied 
 bulk first:
 
 * ``build_state``: one packed projection of the memory stream for all positions
-  (src/relation_lm/inference/packed_cache.py:52-57), split into the four token caches;
-  ``router_cache_prefill`` (conv + block statistics of both router streams, equal to ``T``
-  successive ``router_cache_update`` calls); the expanded cache ``[W_a o + b, W_p o]`` of the
+  (src/relation_lm/inference/packed_cache.py:52-57), split into the four token caches with the conv and
+  block statistics of both router streams (``sequence_state``, equal to ``T`` successive
+  ``router_cache_update`` calls); the expanded cache ``[W_a o + b, W_p o]`` of the
   factorised first relation-MLP layer (src/relation_lm/kernels/relation_reduce.py:42-49).
 * ``forward``: LayerNorm -> 256-wide query projection -> ``relation_select_packed_rows`` ->
   ``relation_hidden_cached_rows`` (16-bit) -> second relation-MLP layer (tensor-core projection) ->
@@ -30,7 +30,7 @@ from relation_lm.kernels.packed_projection import layer_norm_cast, packed_projec
 from relation_lm.kernels.relation_reduce import (MLP_ROWS_MIN_PAIRS, relation_hidden_cached_rows_out, relation_mlp_rows,
                                                  relation_mlp_rows_supported, relation_norm_reduce_rows)
 from relation_lm.kernels.relation_select import relation_select_packed_prefill, relation_select_packed_rows
-from relation_lm.kernels.router_cache import router_cache_prefill
+from relation_lm.kernels.router_cache import sequence_state
 
 
 class RoutedPrefillLayer:
@@ -74,25 +74,11 @@ class RoutedPrefillLayer:
         B, T, d = x.shape
         if T != cfg.max_context:
             raise ValueError("the sequences must fill the configured context")
-        R, H, nb = cfg.relation_dim, cfg.hidden_dim, T // cfg.block_size
+        R, H = cfg.relation_dim, cfg.hidden_dim
         memory = torch.empty(B * T, d, device=self.device, dtype=self.dtype)
         layer_norm_cast(x.view(B * T, d), w["memory_norm_w"], w["memory_norm_b"], cfg.norm_eps, memory)
         packed = packed_projection(memory, w["w_packed"]).view(B, T, cfg.packed_width)
-        state = {
-            "anchor_keys": packed[..., 0:64].contiguous(), "partner_keys": packed[..., 64:128].contiguous(),
-            "operand_cache": packed[..., 128:128 + R].contiguous(),
-            "partner_anchor_cache": packed[..., 128 + R:256 + R].contiguous(),
-        }
-        zeros = lambda *s: torch.zeros(*s, device=self.device, dtype=self.dtype)  # noqa: E731
-        names = ("anchor_raw_cache", "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache")
-        for n in names:
-            state[n] = zeros(B, T, 64)
-        for n in ("anchor_mean", "anchor_std", "partner_mean", "partner_std"):
-            state[n] = zeros(B, nb, 4, 16)
-        router_cache_prefill(packed[..., 256 + R:320 + R], packed[..., 320 + R:384 + R],
-                             *[state[n] for n in names], state["anchor_mean"], state["anchor_std"],
-                             state["partner_mean"], state["partner_std"], w["anchor_conv_weight"],
-                             w["partner_conv_weight"], cfg.block_size)
+        state = sequence_state(packed, 0, R, cfg.block_size, w["anchor_conv_weight"], w["partner_conv_weight"])
         state["expanded_cache"] = packed_projection(state["operand_cache"].view(B * T, R), w["w_expand"],
                                                     w["b_expand"]).view(B, T, 2 * H)
         state["packed"] = packed

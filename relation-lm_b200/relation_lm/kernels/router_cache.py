@@ -14,6 +14,7 @@ from relation_lm.kernels import _abi
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
 _router_cache_update = torch.ops.relation_lm.router_cache_update.default
 _sparse_cache_append = torch.ops.relation_lm.sparse_cache_append.default
+_sequence_state = torch.ops.relation_lm.sequence_state.default
 _router_cache_prefill = torch.ops.relation_lm.router_cache_prefill.default
 
 _MUTATED = ("anchor_raw_cache", "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache",
@@ -118,6 +119,29 @@ def _(anchor_raw, partner_raw, anchor_raw_cache, partner_raw_cache, anchor_conv_
       partner_conv_cache, anchor_mean, anchor_std, partner_mean, partner_std,
       anchor_conv_weight, partner_conv_weight, block_size):
     return None
+
+
+STATE_NAMES = ("anchor_keys", "partner_keys", "operand_cache", "partner_anchor_cache", "anchor_raw_cache",
+               "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache", "anchor_mean", "anchor_std",
+               "partner_mean", "partner_std")
+
+
+def sequence_state(packed: Tensor, slots: int, relation_dim: int, block_size: int, anchor_conv_weight: Tensor,
+                   partner_conv_weight: Tensor) -> dict[str, Tensor]:
+    """The memory-side state of whole sequences from their packed projection rows ``[B, T, W]`` (16-bit) in one
+    launch (extension), keyed by ``STATE_NAMES``: the token caches, and what ``router_cache_prefill`` leaves of
+    both router streams.  ``slots = 0``: one layer's column order (``W = 384 + R``), caches ``[B, T, width]``;
+    ``slots = S``: ``S`` slots of 384 columns, then the operand, slot caches ``[S, B, T, width]``."""
+    return dict(zip(STATE_NAMES, _sequence_state(packed, slots, relation_dim, block_size, anchor_conv_weight,
+                                                 partner_conv_weight)))
+
+
+@torch.library.register_fake("relation_lm::sequence_state")
+def _(packed, slots, relation_dim, block_size, anchor_conv_weight, partner_conv_weight):
+    batch, length, lead = packed.size(0), packed.size(1), (slots,) if slots > 0 else ()
+    wide = [packed.new_empty((*lead, batch, length, w)) for w in (64, 64, 128, 64, 64, 64, 64)]
+    stats = [packed.new_empty((*lead, batch, length // block_size, 4, 16)) for _ in range(4)]
+    return [wide[0], wide[1], packed.new_empty((batch, length, relation_dim)), *wide[2:], *stats]
 
 
 @torch.library.custom_op("relation_lm::packed_projection_append", mutates_args=_APPEND_MUTATED, device_types="cuda")
