@@ -21,7 +21,7 @@ struct EmbedArgs {
     int32_t* status;
     float scale;
     int batch, d_model, vocab, boundary_vocab, max_t, table_dtype;
-    // optional LayerNorm outputs of the embedded row (16-bit, [B, d]): two affine parameter sets
+    // optional LayerNorm outputs of the embedded row (norm_dtype, [B, d]): two affine parameter sets
     const float* norm_w[2];
     const float* norm_b[2];
     void* norm_out[2];
@@ -60,9 +60,9 @@ __global__ void __launch_bounds__(256) decode_embed_kernel(const EmbedArgs a) {
         for (int i = 0; i < 4; ++i) v[i] = embed(c + i);
         *reinterpret_cast<float4*>(a.out + static_cast<int64_t>(b) * a.d_model + c) = make_float4(v[0], v[1], v[2], v[3]);
     }
-    const size_t row = static_cast<size_t>(b) * a.d_model;
-    NormTarget t0{a.norm_w[0], a.norm_b[0], a.norm_out[0] ? static_cast<uint16_t*>(a.norm_out[0]) + row : nullptr};
-    NormTarget t1{a.norm_w[1], a.norm_b[1], a.norm_out[1] ? static_cast<uint16_t*>(a.norm_out[1]) + row : nullptr};
+    const size_t row = static_cast<size_t>(b) * a.d_model * (a.norm_dtype == RLM_F32 ? 4 : 2);
+    NormTarget t0{a.norm_w[0], a.norm_b[0], a.norm_out[0] ? static_cast<unsigned char*>(a.norm_out[0]) + row : nullptr};
+    NormTarget t1{a.norm_w[1], a.norm_b[1], a.norm_out[1] ? static_cast<unsigned char*>(a.norm_out[1]) + row : nullptr};
     block_layer_norm4(v, live, c, a.d_model, a.norm_eps, t0, t1, a.norm_dtype, scratch);
 }
 
@@ -93,13 +93,13 @@ extern "C" int rlm_decode_embed(const int64_t* tokens, const int64_t* boundaries
         return RLM_ERR_NULL;
     }
     if (norm1_out || norm2_out) {
-        if (d_model % 4 != 0 || d_model > 1024 || (norm_out_dtype != RLM_BF16 && norm_out_dtype != RLM_F16)) {
-            set_error("decode_embed: LayerNorm outputs need d_model a multiple of 4 up to 1024 and a 16-bit dtype");
+        if (d_model % 4 != 0 || d_model > 1024 || !valid_dtype(norm_out_dtype)) {
+            set_error("decode_embed: LayerNorm outputs need d_model a multiple of 4 up to 1024 and a known dtype");
             return RLM_ERR_SHAPE;
         }
         if (!aligned16(out) || !aligned16(norm1_weight) || !aligned16(norm1_bias) || !aligned16(norm2_weight) ||
-            !aligned16(norm2_bias) || (reinterpret_cast<uintptr_t>(norm1_out) & 7u) ||
-            (reinterpret_cast<uintptr_t>(norm2_out) & 7u)) {
+            !aligned16(norm2_bias) || (reinterpret_cast<uintptr_t>(norm1_out) & (norm_out_dtype == RLM_F32 ? 15u : 7u)) ||
+            (reinterpret_cast<uintptr_t>(norm2_out) & (norm_out_dtype == RLM_F32 ? 15u : 7u))) {
             set_error("decode_embed: LayerNorm tensors must be 16-byte aligned");
             return RLM_ERR_ALIGN;
         }

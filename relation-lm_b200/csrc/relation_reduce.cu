@@ -406,7 +406,7 @@ struct NormArgs {
     int raw_splits;           // raw is the sum of this many slices, raw_split_stride elements apart (split-K GEMM)
     int64_t raw_split_stride;
     const void* raw_bias;     // optional [D] (param dtype): added to every partner row
-    const float* next_w;      // optional: LayerNorm of the updated residual row, written as 16-bit
+    const float* next_w;      // optional: LayerNorm of the updated residual row, written as next_dtype
     const float* next_b;      //   values to next_out [N, D] (the next layer's normalised input)
     void* next_out;
     float next_eps;
@@ -666,7 +666,7 @@ __device__ __forceinline__ void norm_reduce_vec_row(const NormArgs& a, int row, 
     }
     if (a.next_out) {
         __shared__ float scratch[18];
-        NormTarget t0{a.next_w, a.next_b, static_cast<uint16_t*>(a.next_out) + static_cast<size_t>(row) * D};
+        NormTarget t0{a.next_w, a.next_b, static_cast<unsigned char*>(a.next_out) + static_cast<size_t>(row) * D * (next_dtype == RLM_F32 ? 4 : 2)};
         NormTarget t1{a.next_w, a.next_b, normalized_copy};
         block_layer_norm4(updated, live, c, D, a.next_eps, t0, t1, next_dtype, scratch,
                           kEarly ? &next_g : nullptr, kEarly ? &next_b : nullptr);
@@ -919,14 +919,14 @@ int norm_reduce_launch(
     if (next_normalized) {
         if (!residual || !next_norm_weight || !next_norm_bias || !vec || !aligned16(next_norm_weight) ||
             !aligned16(next_norm_bias) || !aligned16(next_normalized) ||
-            (next_dtype != RLM_BF16 && next_dtype != RLM_F16)) {
+            !valid_dtype(next_dtype)) {
             set_error("relation_norm_reduce: the normalised output needs the residual form, dim a multiple "
-                      "of 8, 16-byte aligned tensors and a 16-bit dtype");
+                      "of 8, 16-byte aligned tensors and a known dtype");
             return RLM_ERR_UNSUPPORTED;
         }
     }
     if (proj_out) {
-        if (!proj_weight || !next_normalized || dim % 64 != 0 || proj_out_dim < kProjCols ||
+        if (!proj_weight || !next_normalized || next_dtype == RLM_F32 || dim % 64 != 0 || proj_out_dim < kProjCols ||
             proj_out_dim % kProjCols != 0 || proj_out_dim > 8 * kProjCols || !aligned16(proj_weight)) {
             set_error("relation_norm_reduce_project: needs the normalised output, dim a multiple of 64, "
                       "32..256 projection outputs in steps of 32 and a 16-byte aligned weight");

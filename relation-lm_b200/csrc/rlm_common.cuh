@@ -392,6 +392,10 @@ __device__ __forceinline__ void block_layer_norm4(const float (&v)[4], bool live
         const float4 b = loaded_beta ? *loaded_beta : *reinterpret_cast<const float4*>(t.beta + c);
         const float y0 = fmaf(d[0] * inv, g.x, b.x), y1 = fmaf(d[1] * inv, g.y, b.y);
         const float y2 = fmaf(d[2] * inv, g.z, b.z), y3 = fmaf(d[3] * inv, g.w, b.w);
+        if (out_dtype == RLM_F32) {
+            *reinterpret_cast<float4*>(static_cast<float*>(t.out_row) + c) = make_float4(y0, y1, y2, y3);
+            continue;
+        }
         uint2 packed;
         if (out_dtype == RLM_BF16) {
             __nv_bfloat162 lo = __floats2bfloat162_rn(y0, y1), hi = __floats2bfloat162_rn(y2, y3);

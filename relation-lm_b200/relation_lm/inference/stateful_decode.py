@@ -8,7 +8,7 @@ docs/benchmarks.md:87-113 of the reference project):
    every layer (packed_cache.py:52-57) followed by ``sparse_cache_append`` (token-cache rows
    + ``router_cache_update`` of all layers, one launch);
 2. per layer: ``LayerNorm(hidden)`` -> one 256-wide query-side projection ->
-   ``relation_select_packed`` -> ``relation_hidden_cache_update`` -> second relation-MLP layer
+   ``relation_select_packed`` -> ``relation_hidden_cache_update_out`` -> second relation-MLP layer
    -> ``relation_norm_reduce`` -> ``hidden += sigmoid(mix) * context``;
 3. final LayerNorm, tied token head, boundary head.
 
@@ -16,6 +16,8 @@ Every state tensor is allocated once and mutated in place; ``position`` lives on
 and is advanced there, so a captured CUDA graph of ``step`` replays for successive positions.
 """
 from __future__ import annotations
+
+from types import SimpleNamespace
 
 import torch
 import torch.nn.functional as F
@@ -30,15 +32,13 @@ from relation_lm.kernels.packed_projection import (decode_embed_norm, decode_fro
                                                     skinny_projection_greedy, skinny_projection_greedy_into,
                                                     skinny_projection_supported)
 from relation_lm.kernels.relation_reduce import (expanded_cache_append, expanded_cache_append_packed,
-                                                 relation_hidden_cache_update,
                                                  relation_layer_tail, relation_layer_tail_supported,
                                                  relation_hidden_cached_out,
                                                  relation_hidden_cache_update_out,
                                                  relation_norm_reduce_residual_norm,
                                                  relation_norm_reduce_residual_norm_project,
                                                  relation_norm_reduce_residual_norm_slices,
-                                                 relation_norm_reduce,
-                                                 relation_norm_reduce_residual, relation_tail)
+                                                 relation_norm_reduce, relation_tail)
 from relation_lm.kernels.relation_select import relation_select_packed
 from relation_lm.kernels.relation_layer import relation_layer, relation_layer_supported
 from relation_lm.kernels.router_cache import packed_projection_append, sparse_cache_append, state_slide
@@ -110,8 +110,7 @@ class StatefulDecoder:
         self.layer_tail = can_tail if layer_tail is None else (bool(layer_tail) and can_tail)
         if self.layer_tail:
             self.fused_query = False
-        if self.fused_query or self.layer_tail:
-            self.query = zeros(B, n_query)
+        self.query = zeros(B, n_query) if self.fused else zeros(L, B, n_query)
         # ... and the selector can run in front of the tail inside the same cluster: one launch per layer.
         # Off by default: with the step's working set cold in L2 it measured 3-5 % slower than the two
         # launches (equal when warm), whose selector overlaps the tail's weight loads just as well.
@@ -144,10 +143,15 @@ class StatefulDecoder:
         self._project = skinny_projection if self.skinny else packed_projection
         if self.skinny:
             self.argmax_scratch = torch.zeros(skinny_argmax_scratch_bytes(), device=self.device, dtype=torch.uint8)
-        if self.fused:
-            self.relation_hidden = zeros(B, cfg.k_max, H)
-            self.normalized = zeros(B, cfg.d_model)             # LayerNorm'd input of the next projection
-            self.memory_normalized = zeros(B, cfg.d_model)      # memory-norm'd input of the packed projection
+        self.relation_hidden = zeros(B, cfg.k_max, H)
+        self.normalized = zeros(B, cfg.d_model)                 # LayerNorm'd input of the next projection
+        self.memory_normalized = zeros(B, cfg.d_model)          # memory-norm'd input of the packed projection
+        if not self.fused:
+            # rows of whole 16-byte chunks up to 1024 wide: LayerNorms inside the kernels that make their input
+            self.kernel_norms = cfg.d_model % 8 == 0 and cfg.d_model <= 1024
+            self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
+            self.head_bias = torch.cat((zeros(cfg.vocab_size), self.w["boundary_b"]))
+        else:
             self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
             pad = (-self.head_weight.size(0)) % 128        # whole 128-column tiles for the projection kernel
             if pad:
@@ -155,6 +159,8 @@ class StatefulDecoder:
             # the boundary head's bias rides in the projection's epilogue (token columns: zero)
             self.head_bias = torch.zeros(self.head_weight.size(0), device=self.device, dtype=torch.float32)
             self.head_bias[cfg.vocab_size:cfg.vocab_size + cfg.boundary_vocab_size] = self.w["boundary_b"].float()
+
+        self._layers = [self._layer_views(l) for l in range(L)]
 
     # ------------------------------------------------------------------ state
     def reset(self) -> None:
@@ -223,44 +229,65 @@ class StatefulDecoder:
             _abi.set_programmatic_launch(previous)
 
     def _step_unfused(self, tokens: Tensor, boundaries: Tensor, keep_selection: bool):
+        """The step without the tensor-core projections (single precision, widths they do not take).  A step
+        of one sequence is bound by the host, so what can ride in a kernel does: the embedding with both its
+        LayerNorms, and norm-reduce with the residual update and the next LayerNorm."""
         cfg, w = self.config, self.w
-        pos = self.position
-        x = (F.embedding(tokens, w["token_embedding"]) + F.embedding(boundaries, w["boundary_embedding"])).float()
-        x = x * self.input_scale + w["position_embedding"].index_select(0, pos.view(1))
-        memory = F.layer_norm(x, (cfg.d_model,), w["memory_norm_w"], w["memory_norm_b"], cfg.norm_eps).to(self.dtype)
-        hidden = x
-        packed = F.linear(memory, w["w_packed"])                      # [B, layers * 512]
+        pos, K = self.position, cfg.k_max
+        if self.kernel_norms:
+            hidden = decode_embed_norm(tokens.contiguous(), boundaries.contiguous(), w["token_embedding"],
+                                       w["boundary_embedding"], w["position_embedding"], pos, self.input_scale,
+                                       w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized,
+                                       w["input_norm_w"][0], w["input_norm_b"][0], self.normalized, cfg.norm_eps)
+        else:
+            x = (F.embedding(tokens, w["token_embedding"]) + F.embedding(boundaries, w["boundary_embedding"])).float()
+            hidden = x * self.input_scale + w["position_embedding"].index_select(0, pos.view(1))
+            self._normalize(hidden, w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized)
+            self._normalize(hidden, w["input_norm_w"][0], w["input_norm_b"][0], self.normalized)
+        packed = F.linear(self.memory_normalized, w["w_packed"])      # [B, layers * 512]
         sparse_cache_append(packed, self.anchor_keys, self.partner_keys, self.operand_cache,
                             self.partner_anchor_cache, *self.router_caches, *self.router_stats,
                             w["anchor_conv_weight"], w["partner_conv_weight"], pos, cfg.block_size)
         if keep_selection:
             self.last_selection = []
-        B, K = self.batch, cfg.k_max
-        for l in range(cfg.layers):
-            normalized = F.layer_norm(hidden, (cfg.d_model,), w["input_norm_w"][l], w["input_norm_b"][l],
-                                      cfg.norm_eps).to(self.dtype)
-            q = F.linear(normalized, w["w_query"][l])                 # [B, 256]
+        for layer in self._layers:
+            torch.mm(self.normalized, layer.w_query_t, out=layer.query)                 # [B, 256]
             anchor, _, partner, partner_score = relation_select_packed(
-                q[:, 0:64], self.anchor_keys[l], q[:, 64:128], self.router_stats[0][l],
-                self.router_stats[1][l], w["anchor_gamma"][l], w["anchor_bias"][l], q[:, 128:256],
-                self.partner_anchor_cache[l], self.partner_keys[l], self.router_stats[2][l],
-                self.router_stats[3][l], w["partner_gamma"][l], w["partner_bias"][l], pos,
-                cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
-            relation_hidden = relation_hidden_cache_update(
-                self.expanded_cache[l], self.operand_cache[l], anchor, partner, w["anchor_weight"][l],
-                w["partner_weight"][l], w["product_weight"][l], w["first_bias"][l], pos)
-            raw = F.linear(relation_hidden.to(self.dtype), w["w2"][l], w["b2"][l])      # [B, K, d]
-            context = relation_norm_reduce(raw, partner_score, w["relation_norm_w"][l],
-                                           w["relation_norm_b"][l], pos, cfg.norm_eps)
-            hidden = torch.addcmul(hidden, context, w["mix"][l])
+                *layer.selection, pos, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
+            relation_hidden_cache_update_out(self.relation_hidden, *layer.caches, anchor, partner, *layer.first_layer, pos)
+            raw = F.linear(self.relation_hidden, *layer.second_layer)                   # [B, K, d]
+            if self.kernel_norms:
+                relation_norm_reduce_residual_norm(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps, hidden,
+                                                   layer.mix, *layer.next_norm, cfg.norm_eps, self.normalized)
+            else:
+                context = relation_norm_reduce(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps)
+                torch.addcmul(hidden, context, layer.mix, out=hidden)
+                self._normalize(hidden, *layer.next_norm, self.normalized)
             if keep_selection:
                 self.last_selection.append((anchor, partner))
-        final = F.layer_norm(hidden, (cfg.d_model,), w["final_norm_w"], w["final_norm_b"], cfg.norm_eps).to(self.dtype)
-        self.last_final = final
-        token_logits = F.linear(final, w["token_embedding"])
-        boundary_logits = F.linear(final, w["boundary_w"], w["boundary_b"])
+        self.last_final = self.normalized
+        logits = F.linear(self.normalized, self.head_weight, self.head_bias)
         pos.add_(1)
-        return token_logits, boundary_logits
+        return logits[:, :cfg.vocab_size], logits[:, cfg.vocab_size:]
+
+    def _normalize(self, rows: Tensor, weight: Tensor, bias: Tensor, out: Tensor) -> None:
+        out.copy_(F.layer_norm(rows, (self.config.d_model,), weight, bias, self.config.norm_eps))
+
+    def _layer_views(self, l: int) -> SimpleNamespace:
+        """What a step hands the operators of layer ``l``: indexing the stacked tensors once a step costs more
+        host time than launching on them."""
+        w, q, last = self.w, self.query if self.fused else self.query[l], l + 1 == self.config.layers
+        following = (w["final_norm_w"], w["final_norm_b"]) if last else (w["input_norm_w"][l + 1], w["input_norm_b"][l + 1])
+        return SimpleNamespace(
+            query=q, w_query=w["w_query"][l], next_query=None if last else w["w_query"][l + 1],
+            selection=(q[:, 0:64], self.anchor_keys[l], q[:, 64:128], self.router_stats[0][l], self.router_stats[1][l],
+                       w["anchor_gamma"][l], w["anchor_bias"][l], q[:, 128:256], self.partner_anchor_cache[l],
+                       self.partner_keys[l], self.router_stats[2][l], self.router_stats[3][l], w["partner_gamma"][l],
+                       w["partner_bias"][l]),
+            caches=(self.expanded_cache[l], self.operand_cache[l]),
+            first_layer=(w["anchor_weight"][l], w["partner_weight"][l], w["product_weight"][l], w["first_bias"][l]),
+            second_layer=(w["w2"][l], w["b2"][l]), relation_norm=(w["relation_norm_w"][l], w["relation_norm_b"][l]),
+            w_query_t=w["w_query"][l].t(), mix=w["mix"][l], next_norm=following)
 
     def _step_fused(self, tokens: Tensor, boundaries: Tensor, keep_selection: bool, advance: bool = True,
                     greedy: bool = False, chosen_out: Tensor | None = None):
@@ -327,24 +354,22 @@ class StatefulDecoder:
         for l in range(cfg.layers):
             # layer 0 projects the embedding's normalised rows; later layers find their queries
             # written by the previous layer's norm-reduce when that fusion is on
-            q = self.query if ((self.fused_query or self.layer_tail) and (l > 0 or self.fused_front)) \
-                else self._project(self.normalized, w["w_query"][l])
-            last = l + 1 == cfg.layers
-            next_w = w["final_norm_w"] if last else w["input_norm_w"][l + 1]
-            next_b = w["final_norm_b"] if last else w["input_norm_b"][l + 1]
+            layer, last = self._layers[l], l + 1 == cfg.layers
+            next_w, next_b = layer.next_norm
+            if (self.fused_query or self.layer_tail) and (l > 0 or self.fused_front):
+                q, selection = self.query, layer.selection
+            else:
+                q = self._project(self.normalized, layer.w_query)
+                selection = (q[:, 0:64], *layer.selection[1:2], q[:, 64:128], *layer.selection[3:7], q[:, 128:256],
+                             *layer.selection[8:])
             if self.whole_layer:
                 if trace is not None:
                     entry = {"stage": "layer", "layer": l, "query": q.clone(), "hidden_before": hidden.clone()}
                     trace.append(entry)
                 anchor, _, partner, partner_score = relation_layer(
-                    q[:, 0:64], self.anchor_keys[l], q[:, 64:128], self.router_stats[0][l],
-                    self.router_stats[1][l], w["anchor_gamma"][l], w["anchor_bias"][l], q[:, 128:256],
-                    self.partner_anchor_cache[l], self.partner_keys[l], self.router_stats[2][l],
-                    self.router_stats[3][l], w["partner_gamma"][l], w["partner_bias"][l], pos,
-                    cfg.local_window, cfg.top_blocks, K, cfg.strict_valid,
-                    self.expanded_cache[l], self.operand_cache[l], w["product_weight"][l], w["w2"][l], w["b2"][l],
-                    w["relation_norm_w"][l], w["relation_norm_b"][l], cfg.norm_eps, hidden, w["mix"][l], next_w,
-                    next_b, cfg.norm_eps, self.normalized, None if last else w["w_query"][l + 1],
+                    *selection, pos, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid,
+                    *layer.caches, layer.first_layer[2], *layer.second_layer, *layer.relation_norm, cfg.norm_eps, hidden,
+                    layer.mix, next_w, next_b, cfg.norm_eps, self.normalized, layer.next_query,
                     None if last else self.query)
                 if trace is not None:
                     entry.update(anchor=anchor.clone(), partner=partner.clone(), partner_score=partner_score.clone(),
@@ -355,21 +380,16 @@ class StatefulDecoder:
                     self.last_selection.append((anchor, partner))
                 continue
             anchor, _, partner, partner_score = relation_select_packed(
-                q[:, 0:64], self.anchor_keys[l], q[:, 64:128], self.router_stats[0][l],
-                self.router_stats[1][l], w["anchor_gamma"][l], w["anchor_bias"][l], q[:, 128:256],
-                self.partner_anchor_cache[l], self.partner_keys[l], self.router_stats[2][l],
-                self.router_stats[3][l], w["partner_gamma"][l], w["partner_bias"][l], pos,
-                cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
+                *selection, pos, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
             if trace is not None:
                 entry = {"stage": "layer", "layer": l, "query": q.clone(), "anchor": anchor.clone(),
                          "partner": partner.clone(), "partner_score": partner_score.clone(),
                          "hidden_before": hidden.clone()}
                 trace.append(entry)
             if self.layer_tail:
-                relation_layer_tail(self.expanded_cache[l], self.operand_cache[l], anchor, partner, partner_score,
-                                    w["product_weight"][l], w["w2"][l], w["b2"][l], w["relation_norm_w"][l],
-                                    w["relation_norm_b"][l], pos, cfg.norm_eps, hidden, w["mix"][l], next_w, next_b,
-                                    cfg.norm_eps, self.normalized, None if last else w["w_query"][l + 1],
+                relation_layer_tail(*layer.caches, anchor, partner, partner_score, layer.first_layer[2],
+                                    *layer.second_layer, *layer.relation_norm, pos, cfg.norm_eps, hidden, layer.mix,
+                                    next_w, next_b, cfg.norm_eps, self.normalized, layer.next_query,
                                     None if last else self.query)
                 if trace is not None:
                     entry.update(hidden_after=hidden.clone(), next_normalized=self.normalized.clone())
@@ -379,13 +399,10 @@ class StatefulDecoder:
                     self.last_selection.append((anchor, partner))
                 continue
             if self.stacked_expand:
-                relation_hidden_cached_out(self.relation_hidden, self.expanded_cache[l], self.operand_cache[l],
-                                           anchor, partner, w["product_weight"][l])
+                relation_hidden_cached_out(self.relation_hidden, *layer.caches, anchor, partner, layer.first_layer[2])
             else:
-                relation_hidden_cache_update_out(
-                    self.relation_hidden, self.expanded_cache[l], self.operand_cache[l], anchor, partner,
-                    w["anchor_weight"][l], w["partner_weight"][l], w["product_weight"][l],
-                    w["first_bias"][l], pos)
+                relation_hidden_cache_update_out(self.relation_hidden, *layer.caches, anchor, partner, *layer.first_layer,
+                                                 pos)
             if self.fused_tail:
                 relation_tail(self.relation_hidden, w["w2"][l], w["b2"][l], partner_score,
                               w["relation_norm_w"][l], w["relation_norm_b"][l], pos, cfg.norm_eps,
@@ -400,18 +417,16 @@ class StatefulDecoder:
                     w["relation_norm_w"][l], w["relation_norm_b"][l], pos, cfg.norm_eps, hidden, w["mix"][l],
                     next_w, next_b, cfg.norm_eps, self.normalized)
             else:
-                raw = F.linear(self.relation_hidden, w["w2"][l], w["b2"][l])            # [B, K, d]
+                raw = F.linear(self.relation_hidden, *layer.second_layer)               # [B, K, d]
                 if trace is not None:
                     entry["raw"] = raw.clone()
                 if self.fused_query and not last:
                     relation_norm_reduce_residual_norm_project(
-                        raw, partner_score, w["relation_norm_w"][l], w["relation_norm_b"][l], pos, cfg.norm_eps,
-                        hidden, w["mix"][l], next_w, next_b, cfg.norm_eps, self.normalized,
-                        w["w_query"][l + 1], self.query)
+                        raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps, hidden, layer.mix, next_w, next_b,
+                        cfg.norm_eps, self.normalized, layer.next_query, self.query)
                 else:
-                    relation_norm_reduce_residual_norm(raw, partner_score, w["relation_norm_w"][l],
-                                                       w["relation_norm_b"][l], pos, cfg.norm_eps, hidden,
-                                                       w["mix"][l], next_w, next_b, cfg.norm_eps, self.normalized)
+                    relation_norm_reduce_residual_norm(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps, hidden,
+                                                       layer.mix, next_w, next_b, cfg.norm_eps, self.normalized)
             if trace is not None:
                 entry.update(relation_hidden=self.relation_hidden.clone(), hidden_after=hidden.clone(),
                              next_normalized=self.normalized.clone())
