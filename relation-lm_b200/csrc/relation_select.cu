@@ -146,118 +146,122 @@ __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(cons
 // L2), anchor, partner queries, partner scores, top-K — with warp-level synchronisation only.
 // The arithmetic is the per-row kernel's own (the same device functions), so indices and scores
 // are bit-identical to relation_select_kernel's.
-// CTAs of kTileWarps warps serve 4 kTileWarps positions (16 warps when the shared memory allows, else 8).
+// CTAs of kTileWarps warps serve one, two or four positions per warp (tile_shape).
 
-// ---- warp-per-query primitives (16-bit bf16 caches).  The arithmetic is the canonical one: every
-// sum below is a sum of the per-row kernel with its operands possibly swapped, so scores are
-// bit-identical.  A lane owns a whole key row (or block) and keeps the 64-wide query in
-// registers, paired for the two-wide fma: v[c][j] = (q[16 c + j], q[16 c + 8 + j]), element j of
-// chunks 2c and 2c + 1.  Staged rows are kPadRow bytes apart, so the eight lanes of a quarter
-// warp read eight different 16-byte chunk indices without rotating their chunk order.
-constexpr uint32_t kPadRow = 2 * kD + 16;
+// ---- warp-per-query primitives (caches, statistics and queries in one 16-bit dtype kDt).  The arithmetic is the
+// canonical one: every sum below is a sum of the per-row kernel with its operands possibly swapped, so scores are
+// bit-identical.  A row is eight 16-byte chunks, lane = 8 rq + chunk: one load instruction of a warp covers four
+// whole rows (512 contiguous bytes of a window, of a block's statistics or of a picked block in the key cache), a
+// lane keeps only its chunk of the query, and the eight chunk sums of a row meet in a butterfly whose level l adds
+// what the per-row kernel's tree adds at level l.  A lane that owned a whole row needed the 64-wide query in
+// registers (128 per thread, 16 warps per SM), and remote rows had to pass through shared memory to be read that
+// way: 96 cycles of the SM's shared-memory pipe for 32 rows against 39 here.
+// Whole-sequence selection of 8 x 4096 rows (384 candidates, 64 blocks): 466 -> 341 us; 16 x 2048 rows of four slots:
+// 1233 -> 955 us.  Issue slots are 71 % taken now (56 % before).
+constexpr uint32_t kRow = 2 * kD;
 
-struct QueryRegs { float2 v[4][8]; };
+// This lane's chunk of a query, every element twice: operands of the two-wide fma over two rows.
+struct QueryChunk { float2 v[8]; };
 
-// Shared-memory copies of a query keep the same pairing (element e at paired_index(e)), so that
-// a 16-byte load fills two register pairs as they are used.
-__device__ __forceinline__ int paired_index(int e) { return (e & ~15) | ((e & 7) << 1) | ((e >> 3) & 1); }
-
-__device__ __forceinline__ void load_query_regs(const float* paired, QueryRegs& r) {
+__device__ __forceinline__ void load_query_chunk(const float* query, QueryChunk& q) {
+    const float* src = query + 8 * (threadIdx.x & 7);
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const float4 v = *reinterpret_cast<const float4*>(paired + 16 * c + 4 * m);
-            r.v[c][2 * m] = make_float2(v.x, v.y);
-            r.v[c][2 * m + 1] = make_float2(v.z, v.w);
-        }
+    for (int h = 0; h < 2; ++h) {
+        const float4 x = *reinterpret_cast<const float4*>(src + 4 * h);
+        q.v[4 * h + 0] = make_float2(x.x, x.x);
+        q.v[4 * h + 1] = make_float2(x.y, x.y);
+        q.v[4 * h + 2] = make_float2(x.z, x.z);
+        q.v[4 * h + 3] = make_float2(x.w, x.w);
+    }
 }
 
-// seg8(chunk 2c, q) + seg8(chunk 2c + 1, q): the two chains advance together in one two-wide fma
-__device__ __forceinline__ float pair_dot_bf16(const uint4 w0, const uint4 w1, const float2 (&q)[8]) {
+// Element pair i of the chunks of two rows, (lower halves, upper halves), widened to fp32 (exact).
+template <int kDt>
+__device__ __forceinline__ void widen_pair(uint32_t a, uint32_t b, float2& lower, float2& upper) {
+    if (kDt == RLM_BF16) {
+        lower = make_float2(__uint_as_float(a << 16), __uint_as_float(b << 16));
+        upper = make_float2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u));
+    } else {
+        const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&a)), y = __half22float2(*reinterpret_cast<const __half2*>(&b));
+        lower = make_float2(x.x, y.x);
+        upper = make_float2(x.y, y.y);
+    }
+}
+
+// seg8 of this lane's chunk for two rows
+template <int kDt>
+__device__ __forceinline__ float2 seg_pair(const uint4 w0, const uint4 w1, const QueryChunk& q) {
     const uint32_t a[4] = {w0.x, w0.y, w0.z, w0.w}, b[4] = {w1.x, w1.y, w1.z, w1.w};
     float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        acc = __ffma2_rn(make_float2(__uint_as_float(a[i] << 16), __uint_as_float(b[i] << 16)), q[2 * i], acc);
-        acc = __ffma2_rn(make_float2(__uint_as_float(a[i] & 0xffff0000u), __uint_as_float(b[i] & 0xffff0000u)),
-                         q[2 * i + 1], acc);
+        float2 lower, upper;
+        widen_pair<kDt>(a[i], b[i], lower, upper);
+        acc = __ffma2_rn(lower, q.v[2 * i], acc);
+        acc = __ffma2_rn(upper, q.v[2 * i + 1], acc);
     }
-    return __fadd_rn(acc.x, acc.y);
+    return acc;
 }
 
-// the same with |q| (the deviation term of the block scores)
-__device__ __forceinline__ float pair_dot_abs_bf16(const uint4 w0, const uint4 w1, const float2 (&q)[8]) {
-    const uint32_t a[4] = {w0.x, w0.y, w0.z, w0.w}, b[4] = {w1.x, w1.y, w1.z, w1.w};
-    float x = 0.0f, y = 0.0f;
+// One level of the butterfly over the chunk lanes: of kN values (a row each) a lane keeps those whose index has the
+// parity of its lane bit, adds the partner's halves of them and hands over its own halves of the others.
+template <int kN, int kXor>
+__device__ __forceinline__ void fold_level(const float (&s)[kN], float (&out)[kN / 2]) {
+    const bool odd = threadIdx.x & kXor;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        x = __fmaf_rn(__uint_as_float(a[i] << 16), fabsf(q[2 * i].x), x);
-        y = __fmaf_rn(__uint_as_float(b[i] << 16), fabsf(q[2 * i].y), y);
-        x = __fmaf_rn(__uint_as_float(a[i] & 0xffff0000u), fabsf(q[2 * i + 1].x), x);
-        y = __fmaf_rn(__uint_as_float(b[i] & 0xffff0000u), fabsf(q[2 * i + 1].y), y);
+    for (int j = 0; j < kN / 2; ++j) {
+        const float keep = odd ? s[2 * j + 1] : s[2 * j], give = odd ? s[2 * j] : s[2 * j + 1];
+        out[j] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, kXor));
     }
-    return __fadd_rn(x, y);
 }
 
-// score_rows_split<true, 1> for one warp with the query in registers (same arguments otherwise;
-// no exclusion list, rows already in place).  `stride`: bytes between rows.
+// Chunk sums of rows load(0) .. load(7) (row i: rows 4 i + rq of a pass), two rows at a time.
+template <int kDt, typename Load>
+__device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q, float (&s)[8]) {
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        uint4 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = load(h + i);
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+            const float2 p = seg_pair<kDt>(w[i], w[i + 1], q);
+            s[h + i] = p.x;
+            s[h + i + 1] = p.y;
+        }
+    }
+}
+
+// Score of the row that this lane owns after the butterfly: row 4 chunk + rq of the pass.
+template <int kDt, typename Load>
+__device__ __forceinline__ float pass_score(const Load& load, const QueryChunk& q) {
+    float s[8], v[4], u[2], t[1];
+    chunk_sums<kDt>(load, q, s);
+    fold_level<8, 1>(s, v);
+    fold_level<4, 2>(v, u);
+    fold_level<2, 4>(u, t);
+    return __fmul_rn(t[0], 0.125f);
+}
+
 // Further excluded positions of a query (the anchors of a multi-anchor row's slots; -1 = none).
 struct ExclRegs { int v[kMaxExclude]; int n; };
 
 template <bool kExcl>
 __device__ __forceinline__ bool not_excluded(int pos, const ExclRegs* ex) {
     bool keep = true;
-    if (kExcl) {
+    if (kExcl) {                       // unused entries are -1, which no position equals
 #pragma unroll
-        for (int x = 0; x < kMaxExclude; ++x) keep = keep && (x >= ex->n || pos != ex->v[x]);
+        for (int x = 0; x < kMaxExclude / 2; ++x) keep = keep && pos != ex->v[x];
+        if (ex->n > kMaxExclude / 2) {
+#pragma unroll
+            for (int x = kMaxExclude / 2; x < kMaxExclude; ++x) keep = keep && pos != ex->v[x];
+        }
     }
     return keep;
 }
 
-template <bool kAtPosition, bool kExcl = false>
-__device__ __forceinline__ void score_rows_warp(const unsigned char* rows, uint32_t stride, int n_rows, const int* sel,
-                                                int bs, int bs_shift, int first_valid, int pos0, int exclude,
-                                                const QueryRegs& q, float* cand, int slot0, uint32_t& best_key,
-                                                int& best_pos, const ExclRegs* ex = nullptr) {
-    const int lane = threadIdx.x & 31;
-    uint32_t my_key = 0;
-    int my_pos = 0x7fffffff;
-    for (int base = 0; base < n_rows; base += 32) {
-        const int r = base + lane;
-        int pos;
-        bool valid;
-        if (sel) {
-            const int rank = bs_shift >= 0 ? r >> bs_shift : r / bs, o = r - rank * bs;
-            const bool in = r < n_rows;
-            pos = in ? sel[3 * rank] * bs + o : -1;
-            valid = in && o < sel[3 * rank + 2];
-        } else {
-            pos = pos0 + r;
-            valid = r < n_rows && r >= first_valid;
-        }
-        valid = valid && pos != exclude && not_excluded<kExcl>(pos, ex);
-        float sc = kNegInf;
-        if (valid) {
-            const uint4* row = reinterpret_cast<const uint4*>(rows + static_cast<size_t>(kAtPosition ? pos : r) * stride);
-            uint4 w[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) w[c] = row[c];
-            const float s01 = __fadd_rn(pair_dot_bf16(w[0], w[1], q.v[0]), pair_dot_bf16(w[2], w[3], q.v[1]));
-            const float s23 = __fadd_rn(pair_dot_bf16(w[4], w[5], q.v[2]), pair_dot_bf16(w[6], w[7], q.v[3]));
-            sc = __fmul_rn(__fadd_rn(s01, s23), 0.125f);
-        }
-        if (cand) {
-            if (r < n_rows) cand[slot0 + r] = sc;
-            continue;
-        }
-        const uint32_t key = float_key(sc);
-        if (valid && (key > my_key || my_pos == 0x7fffffff || (key == my_key && pos < my_pos))) {
-            my_key = key;
-            my_pos = pos;
-        }
-    }
-    if (cand) return;
+// Best (score, lowest position on ties) of the warp into the running best.
+__device__ __forceinline__ void fold_best(uint32_t my_key, int my_pos, uint32_t& best_key, int& best_pos) {
     warp_argmax_key(my_key, my_pos);
     if (my_pos != 0x7fffffff &&
         (my_key > best_key || best_pos == 0x7fffffff || (my_key == best_key && my_pos < best_pos))) {
@@ -266,105 +270,139 @@ __device__ __forceinline__ void score_rows_warp(const unsigned char* rows, uint3
     }
 }
 
-// Rows scored where they lie in the key cache (the picked remote blocks), one warp.  A lane that
-// reads its own 128-byte row makes every load instruction of the warp touch 32 cache lines, and
-// the L1 tag rate then bounds the whole selector; so a pass of 32 rows is fetched coalesced (a
-// load instruction covers four whole rows: lane = 8 (row % 4) + chunk), parked in the warp's
-// padded staging buffer (32 rows of kPadRow bytes) and scored from there a row per lane, exactly
-// like the local window.  Arguments as score_rows_warp with sel != nullptr.
-template <bool kExcl = false>
-__device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
-                                                  int bs_shift, int exclude, const QueryRegs& q, unsigned char* stage,
-                                                  float* cand, int slot0, uint32_t& best_key, int& best_pos,
-                                                  const ExclRegs* ex = nullptr) {
+__device__ __forceinline__ void keep_best(bool valid, float score, int pos, uint32_t& my_key, int& my_pos) {
+    const uint32_t key = float_key(score);
+    if (valid && (key > my_key || my_pos == 0x7fffffff || (key == my_key && pos < my_pos))) {
+        my_key = key;
+        my_pos = pos;
+    }
+}
+
+// The local window, staged in shared memory: row r is position pos0 + r; rows below first_valid are none (and
+// not staged).  Scores go to cand[slot0 + r], or, without cand, into the running best.
+template <int kDt, bool kExcl = false>
+__device__ __forceinline__ void score_window_warp(const unsigned char* rows, int n_rows, int first_valid, int pos0, int exclude,
+                                                  const QueryChunk& q, float* cand, int slot0, uint32_t& best_key,
+                                                  int& best_pos, const ExclRegs* ex = nullptr) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
-    unsigned char* park = stage + rq * kPadRow + 16 * chunk;        // this lane's cell of rows rq, rq + 4, ...
+    const unsigned char* mine = rows + 16 * chunk;
     for (int base = 0; base < n_rows; base += 32) {
-        int pos;                                         // position of row base + lane, or -1
-        uint4 v[8];
-        if (bs_shift >= 5) {
-            // the pass lies in one picked block: rows base + 4 i + rq are 512 bytes apart
-            const int rank = base >> bs_shift, o0 = base - (rank << bs_shift);
-            const int first = sel[3 * rank] * bs, lim = sel[3 * rank + 2];
-            const unsigned char* src = keys + static_cast<size_t>(first + o0 + rq) * (2 * kD) + 16 * chunk;
-            // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint4*>(src + i * (8 * kD));
-            pos = o0 + lane < lim ? first + o0 + lane : -1;
+        float sc;
+        if (base >= first_valid && base + 32 <= n_rows) {
+            const unsigned char* src = mine + (base + rq) * static_cast<int>(kRow);
+            sc = pass_score<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
         } else {
-            auto row_pos = [&](int r) -> int {
-                if (r >= n_rows) return -1;
-                const int rank = bs_shift >= 0 ? r >> bs_shift : r / bs, o = r - rank * bs;
-                return o < sel[3 * rank + 2] ? sel[3 * rank] * bs + o : -1;
-            };
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int p = row_pos(base + 4 * i + rq);
-                v[i] = make_uint4(0, 0, 0, 0);
-                if (p >= 0) v[i] = *reinterpret_cast<const uint4*>(keys + static_cast<size_t>(p) * (2 * kD) + 16 * chunk);
-            }
-            pos = row_pos(base + lane);
+            // the ragged ends read a staged row in place of each missing one
+            sc = pass_score<kDt>([&](int i) {
+                const int r = min(max(base + 4 * i + rq, first_valid), n_rows - 1);
+                return *reinterpret_cast<const uint4*>(mine + r * static_cast<int>(kRow));
+            }, q);
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(park + i * (4 * kPadRow)) = v[i];
-        __syncwarp();
-        const int r = base + lane;
-        const bool valid = pos >= 0 && pos != exclude && not_excluded<kExcl>(pos, ex);
-        float sc = kNegInf;
-        if (valid) {
-            const uint4* row = reinterpret_cast<const uint4*>(stage + lane * kPadRow);
-            uint4 w[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) w[c] = row[c];
-            const float s01 = __fadd_rn(pair_dot_bf16(w[0], w[1], q.v[0]), pair_dot_bf16(w[2], w[3], q.v[1]));
-            const float s23 = __fadd_rn(pair_dot_bf16(w[4], w[5], q.v[2]), pair_dot_bf16(w[6], w[7], q.v[3]));
-            sc = __fmul_rn(__fadd_rn(s01, s23), 0.125f);
-        }
-        __syncwarp();                                   // the staging buffer is free again
+        const int r = base + 4 * chunk + rq, pos = pos0 + r;
+        const bool valid = r < n_rows && r >= first_valid && pos != exclude && not_excluded<kExcl>(pos, ex);
+        sc = valid ? sc : kNegInf;
         if (cand) {
             if (r < n_rows) cand[slot0 + r] = sc;
-            continue;
-        }
-        const uint32_t key = float_key(sc);
-        if (valid && (key > my_key || my_pos == 0x7fffffff || (key == my_key && pos < my_pos))) {
-            my_key = key;
-            my_pos = pos;
+        } else {
+            keep_best(valid, sc, pos, my_key, my_pos);
         }
     }
-    if (cand) return;
-    warp_argmax_key(my_key, my_pos);
-    if (my_pos != 0x7fffffff &&
-        (my_key > best_key || best_pos == 0x7fffffff || (my_key == best_key && my_pos < best_pos))) {
-        best_key = my_key;
-        best_pos = my_pos;
-    }
+    if (!cand) fold_best(my_key, my_pos, best_key, best_pos);
 }
 
-// score_blocks for one warp, a block per lane with all four heads (no shuffles): out[n] for the
-// first n_complete blocks, -inf up to the next multiple of four of nb.
-__device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, const unsigned char* stdv, uint32_t stride,
-                                                  int nb, int n_complete, int bs, int t, int ls, int strict,
-                                                  int buckets, const QueryRegs& rq, const float* sp4, const float* bias,
-                                                  float* out) {
-    const int lane = threadIdx.x & 31;
+// The picked remote blocks (sel: block, picked, rows), scored where they lie in the key cache.
+template <int kDt, bool kExcl = false>
+__device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
+                                                  int bs_shift, int exclude, const QueryChunk& q, float* cand, int slot0,
+                                                  uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr) {
+    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
+    uint32_t my_key = 0;
+    int my_pos = 0x7fffffff;
+    const unsigned char* mine = keys + 16 * chunk;
+    for (int base = 0; base < n_rows; base += 32) {
+        const int r = base + 4 * chunk + rq;
+        int pos;                                         // position of row r, or -1
+        float sc;
+        if (bs_shift >= 5) {
+            // the pass lies in one picked block: rows 4 i + rq are 512 bytes apart
+            const int rank = base >> bs_shift, o0 = base - (rank << bs_shift);
+            const int first = sel[3 * rank] * bs + o0, lim = sel[3 * rank + 2] - o0;
+            const unsigned char* src = mine + static_cast<size_t>(first + rq) * kRow;
+            // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
+            sc = pass_score<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+            pos = 4 * chunk + rq < lim ? first + 4 * chunk + rq : -1;
+        } else {
+            auto row_pos = [&](int row) -> int {
+                if (row >= n_rows) return -1;
+                const int rank = bs_shift >= 0 ? row >> bs_shift : row / bs, o = row - rank * bs;
+                return o < sel[3 * rank + 2] ? sel[3 * rank] * bs + o : -1;
+            };
+            sc = pass_score<kDt>([&](int i) {
+                const int p = row_pos(base + 4 * i + rq);
+                return p >= 0 ? *reinterpret_cast<const uint4*>(mine + static_cast<size_t>(p) * kRow) : make_uint4(0, 0, 0, 0);
+            }, q);
+            pos = row_pos(r);
+        }
+        const bool valid = pos >= 0 && pos != exclude && not_excluded<kExcl>(pos, ex);
+        sc = valid ? sc : kNegInf;
+        if (cand) {
+            if (r < n_rows) cand[slot0 + r] = sc;
+        } else {
+            keep_best(valid, sc, pos, my_key, my_pos);
+        }
+    }
+    if (!cand) fold_best(my_key, my_pos, best_key, best_pos);
+}
+
+// score_blocks for one warp, 32 blocks a pass: chunks 2 h and 2 h + 1 of a block's statistics are head h, so the
+// first butterfly level completes a head's sums; a 4 x 4 transpose between the head lanes then leaves every lane
+// with the four heads of one block.  out[n] for the first n_complete blocks, -inf up to the next multiple of four
+// of nb.
+template <int kDt>
+__device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, const unsigned char* stdv, int nb, int n_complete,
+                                                  int bs, int t, int ls, int strict, int buckets, const QueryChunk& q,
+                                                  const float* sp4, const float* bias, float* out) {
+    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
-    for (int n = lane; n < n_complete; n += 32) {
+    QueryChunk qa;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
+    const float sp = sp4[chunk >> 1];
+    const bool x2 = lane & 2, x4 = lane & 4;
+    for (int base = 0; base < n_complete; base += 32) {
+        float sums[8], md[4], sd[4];
+        const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
+        chunk_sums<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+        fold_level<8, 1>(sums, md);
+        chunk_sums<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+        fold_level<8, 1>(sums, sd);
+        // v[j]: head (chunk >> 1) of block 4 (2 j + (chunk & 1)) + rq
+        float v[4], w[2][2], sh[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(__fadd_rn(md[j], __fmul_rn(sp, sd[j])), 0.25f);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float got = __shfl_xor_sync(0xffffffffu, x2 ? v[2 * j] : v[2 * j + 1], 2), own = x2 ? v[2 * j + 1] : v[2 * j];
+            w[j][0] = x2 ? got : own;
+            w[j][1] = x2 ? own : got;
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const float got = __shfl_xor_sync(0xffffffffu, x4 ? w[0][x] : w[1][x], 4), own = x4 ? w[1][x] : w[0][x];
+            sh[x] = x4 ? got : own;
+            sh[2 + x] = x4 ? own : got;
+        }
+        const int n = base + 4 * chunk + rq;
+        if (n >= n_complete) continue;                   // no lane-collective operation follows in the pass
         const int end = (n + 1) * bs - 1;
         int dist = t - end;
         if (dist < 0) dist = 0;
         int bucket = 31 - __clz(dist + 1);
         if (bucket > buckets - 1) bucket = buckets - 1;
-        const uint4* m = reinterpret_cast<const uint4*>(mean + static_cast<size_t>(n) * stride);
-        const uint4* sd4 = reinterpret_cast<const uint4*>(stdv + static_cast<size_t>(n) * stride);
-        float sh[4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const float md = pair_dot_bf16(m[2 * h], m[2 * h + 1], rq.v[h]);
-            const float sd = pair_dot_abs_bf16(sd4[2 * h], sd4[2 * h + 1], rq.v[h]);
-            sh[h] = __fadd_rn(__fmul_rn(__fadd_rn(md, __fmul_rn(sp4[h], sd)), 0.25f), bias[h * buckets + bucket]);
-        }
+        for (int h = 0; h < 4; ++h) sh[h] = __fadd_rn(sh[h], bias[h * buckets + bucket]);
         const float mx = fmaxf(fmaxf(sh[0], sh[1]), fmaxf(sh[2], sh[3]));
         const float e01 = __fadd_rn(canon_exp(__fsub_rn(sh[0], mx)), canon_exp(__fsub_rn(sh[1], mx)));
         const float e23 = __fadd_rn(canon_exp(__fsub_rn(sh[2], mx)), canon_exp(__fsub_rn(sh[3], mx)));
@@ -473,28 +511,28 @@ __device__ __forceinline__ bool topk_filter(const float* cand, int cap4, int K, 
 struct TileArgs {
     SelectArgs base;          // packed mode; queries [n_seq * q_len, ...]; row = b * q_len + t
     int q_len;                // query positions 0 .. q_len - 1 of every sequence
+    int tile_queries;         // positions per CTA
     int warp_bytes, stats_bytes, window_rows, param_bytes;
 };
 
-template <bool kBf16, int kTileWarps>
-__global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_select_tile_kernel(const TileArgs m) {
-    constexpr int kTileQ = 4 * kTileWarps, kTileThreads = 32 * kTileWarps;
+template <int kDt, int kTileWarps>
+__global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / kTileWarps) relation_select_tile_kernel(const TileArgs m) {
+    constexpr bool kFast = kDt != RLM_F32;            // one 16-bit dtype throughout (else run-time dtypes)
+    constexpr int kTileThreads = 32 * kTileWarps;
+    const int tile_q = m.tile_queries;
     extern __shared__ __align__(128) unsigned char smem[];
     const SelectArgs& a = m.base;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int key_dtype = kBf16 ? RLM_BF16 : a.key_dtype, stats_dtype = kBf16 ? RLM_BF16 : a.stats_dtype,
-              query_dtype = kBf16 ? RLM_BF16 : a.query_dtype;
-    const int tiles_per_seq = (m.q_len + kTileQ - 1) / kTileQ;
-    const int b = blockIdx.x / tiles_per_seq, t0 = (blockIdx.x - b * tiles_per_seq) * kTileQ;
-    const int t_end = min(t0 + kTileQ, m.q_len);               // exclusive
+    const int key_dtype = kFast ? kDt : a.key_dtype, stats_dtype = kFast ? kDt : a.stats_dtype,
+              query_dtype = kFast ? kDt : a.query_dtype;
+    const int tiles_per_seq = (m.q_len + tile_q - 1) / tile_q;
+    const int b = blockIdx.x / tiles_per_seq, t0 = (blockIdx.x - b * tiles_per_seq) * tile_q;
+    const int t_end = min(t0 + tile_q, m.q_len);               // exclusive
     const int nb = a.n_blocks, bs = a.block_size, L = a.local_window, top = a.top_blocks, K = a.k_out;
     const int bs_shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
     const int ks = key_dtype == RLM_F32 ? 4 : 2, ss = stats_dtype == RLM_F32 ? 4 : 2;
     const size_t key_row = static_cast<size_t>(kD) * ks, stat_row = static_cast<size_t>(kD) * ss;
-    // bf16 rows are staged with 16 bytes of padding (see kPadRow); the other dtypes keep the
-    // per-row kernel's scoring functions and their dense rows
-    const uint32_t key_stride = kBf16 ? kPadRow : static_cast<uint32_t>(key_row);
-    const uint32_t stat_stride = kBf16 ? kPadRow : static_cast<uint32_t>(stat_row);
+    const uint32_t key_stride = static_cast<uint32_t>(key_row), stat_stride = static_cast<uint32_t>(stat_row);
     const int buckets4 = 4 * a.buckets;
     griddep_sync();
 
@@ -545,7 +583,6 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
     float* cand = bscore + ((nb + 3) & ~3);
     const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
     int* sel = reinterpret_cast<int*>(cand + cap4);
-    unsigned char* stage = warp_base + m.warp_bytes - 32 * kPadRow;          // remote rows of a pass (bf16 caches)
     for (int i = cap + lane; i < cap4; i += 32) cand[i] = kNegInf;
     cp_async_wait_all();
     __syncthreads();
@@ -560,7 +597,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
             if (i < kD) v = load_scalar(a.anchor_query, row * a.aq_stride + i, query_dtype);
             else if (i < 2 * kD) v = load_scalar(a.anchor_router_query, row * a.arq_stride + i - kD, query_dtype);
             else v = load_scalar(a.partner_base, row * a.pbase_stride + i - 2 * kD, query_dtype);
-            queries[kBf16 ? (i & ~(kD - 1)) | paired_index(i & (kD - 1)) : i] = v;
+            queries[i] = v;
         }
         __syncwarp();
         const float* aq = queries, *arq = queries + kD;
@@ -575,34 +612,34 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
         // ---- anchor
         uint32_t bk = 0;
         int bp = 0x7fffffff;
-        if constexpr (kBf16) {
-            QueryRegs q;
+        if constexpr (kFast) {
+            QueryChunk q;
             if (top > 0) {
-                load_query_regs(arq, q);
-                score_blocks_warp(st[0], st[1], stat_stride, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                load_query_chunk(arq, q);
+                score_blocks_warp<kDt>(st[0], st[1], nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
                                   sp_a, bias_a, bscore);
             }
-            load_query_regs(aq, q);
-            score_rows_warp<false>(local_a, key_stride, L, nullptr, bs, bs_shift, first_local, t - L + 1, -1, q, nullptr,
+            load_query_chunk(aq, q);
+            score_window_warp<kDt>(local_a, L, first_local, t - L + 1, -1, q, nullptr,
                                    0, bk, bp);
             if (top > 0) {
                 __syncwarp();
                 if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
                 else pick_blocks(bscore, nb, top, bs, ls, sel);
-                score_remote_warp(seq_a, top * bs, sel, bs, bs_shift, -1, q, stage, nullptr, 0, bk, bp);
+                score_remote_warp<kDt>(seq_a, top * bs, sel, bs, bs_shift, -1, q, nullptr, 0, bk, bp);
             }
         } else {
             if (top > 0)
-                score_blocks_any<kBf16>(st[0], st[1], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<false>(st[0], st[1], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         arq, sp_a, bias_a, bscore, 0, 1);
-            score_rows_split<kBf16, 1>(local_a, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1, nullptr, 0, aq,
+            score_rows_split<false, 1>(local_a, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1, nullptr, 0, aq,
                                        nullptr, 0, 0, 1, bk, bp, 0u, ok);
             if (top > 0) {
                 __syncwarp();
                 pick_blocks(bscore, nb, top, bs, ls, sel);
                 uint32_t rk = 0;
                 int rp = 0x7fffffff;
-                score_rows_split<kBf16, 1, true>(seq_a, key_dtype, top * bs, sel, bs, 0, 0, -1, nullptr, 0, aq, nullptr, 0,
+                score_rows_split<false, 1, true>(seq_a, key_dtype, top * bs, sel, bs, 0, 0, -1, nullptr, 0, aq, nullptr, 0,
                                                  0, 1, rk, rp, 0u, ok);
                 if (rp != 0x7fffffff && (rk > bk || bp == 0x7fffffff || (rk == bk && rp < bp))) { bk = rk; bp = rp; }
             }
@@ -617,39 +654,38 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
         for (int i = lane; i < 2 * kD; i += 32) {
             const float add = load_scalar(a.partner_anchor_cache,
                                           (static_cast<size_t>(b) * a.max_t + anchor_pos) * 2 * kD + i, key_dtype);
-            const int at = kBf16 ? (i & ~(kD - 1)) | paired_index(i & (kD - 1)) : i;
-            pq[at] = __fadd_rn(pq[at], add);
+            pq[i] = __fadd_rn(pq[i], add);
         }
         __syncwarp();
         // ---- partners
         uint32_t dk = 0;
         int dp = 0x7fffffff;
-        if constexpr (kBf16) {
-            QueryRegs q;
+        if constexpr (kFast) {
+            QueryChunk q;
             if (top > 0) {
-                load_query_regs(prq, q);
-                score_blocks_warp(st[2], st[3], stat_stride, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                load_query_chunk(prq, q);
+                score_blocks_warp<kDt>(st[2], st[3], nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
                                   sp_p, bias_p, bscore);
             }
-            load_query_regs(pq, q);
-            score_rows_warp<false>(local_p, key_stride, L, nullptr, bs, bs_shift, first_local, t - L + 1, anchor_pos, q,
+            load_query_chunk(pq, q);
+            score_window_warp<kDt>(local_p, L, first_local, t - L + 1, anchor_pos, q,
                                    cand, 0, dk, dp);
             if (top > 0) {
                 __syncwarp();
                 if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
                 else pick_blocks(bscore, nb, top, bs, ls, sel);
-                score_remote_warp(seq_p, top * bs, sel, bs, bs_shift, anchor_pos, q, stage, cand, L, dk, dp);
+                score_remote_warp<kDt>(seq_p, top * bs, sel, bs, bs_shift, anchor_pos, q, cand, L, dk, dp);
             }
         } else {
             if (top > 0)
-                score_blocks_any<kBf16>(st[2], st[3], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<false>(st[2], st[3], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         prq, sp_p, bias_p, bscore, 0, 1);
-            score_rows_split<kBf16, 1>(local_p, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos, nullptr, 0,
+            score_rows_split<false, 1>(local_p, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos, nullptr, 0,
                                        pq, cand, 0, 0, 1, dk, dp, 0u, ok);
             if (top > 0) {
                 __syncwarp();
                 pick_blocks(bscore, nb, top, bs, ls, sel);
-                score_rows_split<kBf16, 1, true>(seq_p, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, nullptr, 0, pq, cand,
+                score_rows_split<false, 1, true>(seq_p, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, nullptr, 0, pq, cand,
                                                  L, 0, 1, dk, dp, 0u, ok);
             }
         }
@@ -670,9 +706,9 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
     }
 }
 
-// ---- whole-sequence multi-anchor selection: the tiled form of relation_select_multi_kernel (bf16)
+// ---- whole-sequence multi-anchor selection: the tiled form of relation_select_multi_kernel (one 16-bit dtype)
 //
-// A CTA of kTileWarps warps serves 4 kTileWarps consecutive positions of one sequence; every warp
+// A CTA of kTileWarps warps serves up to 4 kTileWarps consecutive positions of one sequence; every warp
 // keeps its queries and walks them through 2 S phases — the anchors of slot 0 .. S - 1 (each barring
 // the positions taken before it), then the partners of slot 0 .. S - 1 (each barring all anchors).
 // A phase's block statistics and window union (one slot, one stream) are staged for the whole CTA
@@ -680,24 +716,25 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
 // relation_select_multi_kernel's (same results bit for bit).
 struct MultiTileArgs {
     MultiSelectArgs m;
-    int q_len;
-    int warp_bytes, stats_bytes, window_rows, param_bytes, stage_bytes;
+    int q_len, tile_queries;
+    int warp_bytes, stats_bytes, param_bytes, stage_bytes;
 };
 
-template <int kTileWarps>
-__global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_select_multi_tile_kernel(const MultiTileArgs ta) {
-    constexpr int kTileQ = 4 * kTileWarps, kTileThreads = 32 * kTileWarps;
+template <int kDt, int kTileWarps>
+__global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_select_multi_tile_kernel(const MultiTileArgs ta) {
+    constexpr int kTileThreads = 32 * kTileWarps;
+    const int tile_q = ta.tile_queries;
     extern __shared__ __align__(128) unsigned char smem[];
     const MultiSelectArgs& m = ta.m;
     const SelectArgs& a = m.base;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = m.slots, K = a.k_out;
-    const int tiles_per_seq = (ta.q_len + kTileQ - 1) / kTileQ;
-    const int b = blockIdx.x / tiles_per_seq, t0 = (blockIdx.x - b * tiles_per_seq) * kTileQ;
-    const int t_end = min(t0 + kTileQ, ta.q_len);
+    const int tiles_per_seq = (ta.q_len + tile_q - 1) / tile_q;
+    const int b = blockIdx.x / tiles_per_seq, t0 = (blockIdx.x - b * tiles_per_seq) * tile_q;
+    const int t_end = min(t0 + tile_q, ta.q_len);
     const int nb = a.n_blocks, bs = a.block_size, L = a.local_window, top = a.top_blocks;
     const int bs_shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
-    constexpr size_t key_row = 2 * kD, stat_row = 2 * kD;
+    constexpr size_t key_row = kRow, stat_row = kRow;
     const int buckets4 = 4 * a.buckets;
     griddep_sync();
 
@@ -721,12 +758,12 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
             const int stat_chunks = n_stage * 8;
             for (int i = tid; i < 2 * stat_chunks; i += kTileThreads) {
                 const int which = i >= stat_chunks, c = i - which * stat_chunks;
-                cp_async16(smem_u32(dst) + which * ta.stats_bytes + (c >> 3) * kPadRow + 16 * (c & 7),
+                cp_async16(smem_u32(dst) + which * ta.stats_bytes + 16 * c,
                            (which ? stdv : mean) + 16 * c);
             }
             const int win_chunks = (t_end - w_lo) * 8;
             for (int i = tid; i < win_chunks; i += kTileThreads)
-                cp_async16(smem_u32(dst) + 2 * ta.stats_bytes + (i >> 3) * kPadRow + 16 * (i & 7), keys + 16 * i);
+                cp_async16(smem_u32(dst) + 2 * ta.stats_bytes + 16 * i, keys + 16 * i);
         }
         cp_async_commit();
     };
@@ -745,17 +782,15 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
         params[i] = v;
     }
     // per-warp scratch
-    float* queries = reinterpret_cast<float*>(warp_base);                     // exact query | router query (paired layout)
+    float* queries = reinterpret_cast<float*>(warp_base);                     // exact query | router query
     uint32_t* short_list = reinterpret_cast<uint32_t*>(queries + 2 * kD);     // 64 words of the top-K filter
     int* taken = reinterpret_cast<int*>(short_list + 64);                     // [4 queries][kMaxSlots]
     float* bscore = reinterpret_cast<float*>(taken + 4 * kMaxSlots);
     float* cand = bscore + ((nb + 3) & ~3);
     const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
     int* sel = reinterpret_cast<int*>(cand + cap4);
-    unsigned char* park = warp_base + ta.warp_bytes - 32 * kPadRow;           // remote rows of a pass
     for (int i = cap + lane; i < cap4; i += 32) cand[i] = kNegInf;
     for (int i = lane; i < 4 * kMaxSlots; i += 32) taken[i] = -1;
-    const size_t esz = 2;
 
     for (int ph = 0; ph < 2 * S; ++ph) {
         request_phase(ph + 1);                       // into the buffer phase ph - 1 has left
@@ -776,7 +811,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
             const int ls = max(t - L + 1, 0), first_local = ls - (t - L + 1);
             const int n_complete = min((t + 1) / bs, nb);
             int* mine = taken + qi * kMaxSlots;
-            const unsigned char* local = win + static_cast<ptrdiff_t>(t - L + 1 - w_lo) * static_cast<ptrdiff_t>(kPadRow);
+            const unsigned char* local = win + static_cast<ptrdiff_t>(t - L + 1 - w_lo) * static_cast<ptrdiff_t>(kRow);
             ExclRegs ex;
             if (!partner) {
                 // ---- anchor of slot s: active iff s <= t; the positions taken by slots 0 .. s - 1 are barred
@@ -788,30 +823,30 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
                     continue;                        // taken[s] stays -1
                 }
                 for (int i = lane; i < 2 * kD; i += 32) {
-                    const float v = i < kD ? load_scalar(a.anchor_query, row * a.aq_stride + s * kD + i, RLM_BF16)
-                                           : load_scalar(a.anchor_router_query, row * a.arq_stride + s * kD + i - kD, RLM_BF16);
-                    queries[(i & ~(kD - 1)) | paired_index(i & (kD - 1))] = v;
+                    const float v = i < kD ? load_scalar(a.anchor_query, row * a.aq_stride + s * kD + i, kDt)
+                                           : load_scalar(a.anchor_router_query, row * a.arq_stride + s * kD + i - kD, kDt);
+                    queries[i] = v;
                 }
                 ex.n = s;
 #pragma unroll
                 for (int x = 0; x < kMaxExclude; ++x) ex.v[x] = x < s ? mine[x] : -1;
                 __syncwarp();
-                QueryRegs q;
+                QueryChunk q;
                 if (top > 0) {
-                    load_query_regs(queries + kD, q);
-                    score_blocks_warp(st_mean, st_std, kPadRow, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp,
+                    load_query_chunk(queries + kD, q);
+                    score_blocks_warp<kDt>(st_mean, st_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp,
                                       bias, bscore);
                 }
-                load_query_regs(queries, q);
+                load_query_chunk(queries, q);
                 uint32_t bk = 0;
                 int bp = 0x7fffffff;
-                score_rows_warp<false, true>(local, kPadRow, L, nullptr, bs, bs_shift, first_local, t - L + 1, -1, q, nullptr,
+                score_window_warp<kDt, true>(local, L, first_local, t - L + 1, -1, q, nullptr,
                                              0, bk, bp, &ex);
                 if (top > 0) {
                     __syncwarp();
                     if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
                     else pick_blocks(bscore, nb, top, bs, ls, sel);
-                    score_remote_warp<true>(seq_keys, top * bs, sel, bs, bs_shift, -1, q, park, nullptr, 0, bk, bp, &ex);
+                    score_remote_warp<kDt, true>(seq_keys, top * bs, sel, bs, bs_shift, -1, q, nullptr, 0, bk, bp, &ex);
                 }
                 const float score = bp == 0x7fffffff ? kNegInf : key_float(bk);
                 const bool live = score > kNegInf;
@@ -833,30 +868,30 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
                 }
                 const unsigned char* pac = static_cast<const unsigned char*>(a.partner_anchor_cache) + s * m.pac_slot;
                 for (int i = lane; i < 2 * kD; i += 32) {
-                    const float base = load_scalar(a.partner_base, row * a.pbase_stride + s * 2 * kD + i, RLM_BF16);
-                    const float add = load_scalar(pac, (static_cast<size_t>(b) * a.max_t + anchor_pos) * 2 * kD + i, RLM_BF16);
-                    queries[(i & ~(kD - 1)) | paired_index(i & (kD - 1))] = __fadd_rn(base, add);
+                    const float base = load_scalar(a.partner_base, row * a.pbase_stride + s * 2 * kD + i, kDt);
+                    const float add = load_scalar(pac, (static_cast<size_t>(b) * a.max_t + anchor_pos) * 2 * kD + i, kDt);
+                    queries[i] = __fadd_rn(base, add);
                 }
                 ex.n = S;
 #pragma unroll
                 for (int x = 0; x < kMaxExclude; ++x) ex.v[x] = x < S ? mine[x] : -1;
                 __syncwarp();
-                QueryRegs q;
+                QueryChunk q;
                 if (top > 0) {
-                    load_query_regs(queries + kD, q);
-                    score_blocks_warp(st_mean, st_std, kPadRow, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp,
+                    load_query_chunk(queries + kD, q);
+                    score_blocks_warp<kDt>(st_mean, st_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp,
                                       bias, bscore);
                 }
-                load_query_regs(queries, q);
+                load_query_chunk(queries, q);
                 uint32_t dk = 0;
                 int dp = 0x7fffffff;
-                score_rows_warp<false, true>(local, kPadRow, L, nullptr, bs, bs_shift, first_local, t - L + 1, anchor_pos, q,
+                score_window_warp<kDt, true>(local, L, first_local, t - L + 1, anchor_pos, q,
                                              cand, 0, dk, dp, &ex);
                 if (top > 0) {
                     __syncwarp();
                     if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
                     else pick_blocks(bscore, nb, top, bs, ls, sel);
-                    score_remote_warp<true>(seq_keys, top * bs, sel, bs, bs_shift, anchor_pos, q, park, cand, L, dk, dp, &ex);
+                    score_remote_warp<kDt, true>(seq_keys, top * bs, sel, bs, bs_shift, anchor_pos, q, cand, L, dk, dp, &ex);
                 }
                 __syncwarp();
                 bool exact = false;
@@ -876,7 +911,46 @@ __global__ void __launch_bounds__(32 * kTileWarps, 16 / kTileWarps) relation_sel
         __syncthreads();                             // everybody has left buffer ph & 1
     }
     cp_async_wait_all();
-    (void)esz;
+}
+
+// A tile's shape: warps per CTA and positions per warp.  A launch lasts as many waves of a tile per SM as its tiles
+// need, each as long as the tile's rounds of a position per warp; a round of 32 warps fills the SM, fewer warps
+// leave issue slots unused but end sooner (relative lengths below from one round of each: 27, 23, 21 and 19 us for
+// 512 positions, launch and staging included, and 341, 339, 403 and 477 us for 8 x 4096).  The shape of least waves x
+// rounds x length that fits the shared memory is taken: 8 x 4096 positions run as 1024 tiles of 32, 3 x 1984 as 126 of
+// 48 (as 249 of 24 they take 53 us, as 186 of 32 67 us), 512 as 64 of 8.
+struct TileShape { int warps, per_warp, smem_bytes; };
+
+template <typename Smem>
+TileShape tile_shape(int n_seq, int q_len, int most_warps, const Smem& smem) {
+    static constexpr int kShapes[4][2] = {{32, 32}, {24, 24}, {16, 19}, {8, 13}};
+    TileShape best{0, 0, 0};
+    int64_t best_cost = INT64_MAX;
+    for (const auto& shape : kShapes) {
+        const int warps = shape[0];
+        if (warps > most_warps || (warps == 24 && most_warps < 32)) continue;
+        for (int per_warp = 4; per_warp >= 1; per_warp /= 2) {
+            const int total = smem(warps, per_warp * warps);
+            if (total > kSmemDynamicLimit) continue;
+            const int64_t tiles = static_cast<int64_t>(n_seq) * ((q_len + per_warp * warps - 1) / (per_warp * warps));
+            const int64_t waves = (tiles + sm_count() - 1) / sm_count();
+            const int64_t cost = waves * (32 * per_warp * shape[1] + shape[1]);      // staging: 1/32 of a round
+            if (cost < best_cost) { best_cost = cost; best = {warps, per_warp, total}; }
+        }
+    }
+    return best;
+}
+
+template <int kDt>
+auto multi_tile_kernel(int warps) {
+    return warps == 32 ? relation_select_multi_tile_kernel<kDt, 32> : warps == 24 ? relation_select_multi_tile_kernel<kDt, 24>
+           : warps == 16 ? relation_select_multi_tile_kernel<kDt, 16> : relation_select_multi_tile_kernel<kDt, 8>;
+}
+
+template <int kDt>
+auto tile_kernel(int warps) {
+    return warps == 32 ? relation_select_tile_kernel<kDt, 32> : warps == 24 ? relation_select_tile_kernel<kDt, 24>
+           : warps == 16 ? relation_select_tile_kernel<kDt, 16> : relation_select_tile_kernel<kDt, 8>;
 }
 
 int launch_multi_tile(MultiTileArgs& ta, void* stream) {
@@ -889,8 +963,9 @@ int launch_multi_tile(MultiTileArgs& ta, void* stream) {
                   "K <= 32, query length <= T");
         return RLM_ERR_SHAPE;
     }
-    if (a.query_dtype != RLM_BF16 || a.key_dtype != RLM_BF16 || a.stats_dtype != RLM_BF16 || !valid_dtype(a.param_dtype)) {
-        set_error("relation_select_multi_prefill: queries, caches and block statistics must be bfloat16 "
+    if ((a.query_dtype != RLM_BF16 && a.query_dtype != RLM_F16) || a.key_dtype != a.query_dtype ||
+        a.stats_dtype != a.query_dtype || !valid_dtype(a.param_dtype)) {
+        set_error("relation_select_multi_prefill: queries, caches and block statistics must share bfloat16 or float16 "
                   "(relation_select_multi_rows serves the other dtypes)");
         return RLM_ERR_UNSUPPORTED;
     }
@@ -925,24 +1000,24 @@ int launch_multi_tile(MultiTileArgs& ta, void* stream) {
     }
     const int cap4 = (cap + 3) & ~3;
     const int floats = 2 * kD + 64 + 4 * kMaxSlots + ((a.n_blocks + 3) & ~3) + cap4;
-    ta.warp_bytes = align16(floats * 4 + 3 * (a.top_blocks > 0 ? a.top_blocks : 1) * 4) + 16 + 32 * static_cast<int>(kPadRow);
-    ta.stats_bytes = align16(a.n_blocks * static_cast<int>(kPadRow));
+    ta.warp_bytes = align16(floats * 4 + 3 * (a.top_blocks > 0 ? a.top_blocks : 1) * 4) + 16;
+    ta.stats_bytes = a.n_blocks * static_cast<int>(kRow);
     ta.param_bytes = align16(m.slots * (8 + 8 * a.buckets) * 4);
-    int warps = 16, total = 0;
-    for (;; warps = 8) {
-        ta.window_rows = a.local_window + 4 * warps;
-        ta.stage_bytes = (2 * ta.stats_bytes + ta.window_rows * static_cast<int>(kPadRow) + 127) & ~127;
-        total = 2 * ta.stage_bytes + ta.param_bytes + warps * ta.warp_bytes;
-        if (total <= kSmemDynamicLimit || warps == 8) break;
-    }
-    if (total > kSmemDynamicLimit) {
+    const TileShape shape = tile_shape(a.n_seq, ta.q_len, 32, [&](int warps, int tile) {
+        ta.stage_bytes = (2 * ta.stats_bytes + (a.local_window + tile) * static_cast<int>(kRow) + 127) & ~127;
+        return 2 * ta.stage_bytes + ta.param_bytes + warps * ta.warp_bytes;
+    });
+    if (shape.warps == 0) {
         set_error("relation_select_multi_prefill: block statistics + window union exceed 227 KB of shared memory");
         return RLM_ERR_SMEM;
     }
-    auto kernel = warps == 16 ? relation_select_multi_tile_kernel<16> : relation_select_multi_tile_kernel<8>;
+    const int warps = shape.warps, total = shape.smem_bytes;
+    ta.tile_queries = shape.per_warp * warps;
+    ta.stage_bytes = (2 * ta.stats_bytes + (a.local_window + ta.tile_queries) * static_cast<int>(kRow) + 127) & ~127;
+    auto kernel = a.key_dtype == RLM_BF16 ? multi_tile_kernel<RLM_BF16>(warps) : multi_tile_kernel<RLM_F16>(warps);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
-    const int tiles = a.n_seq * ((ta.q_len + 4 * warps - 1) / (4 * warps));
+    const int tiles = a.n_seq * ((ta.q_len + ta.tile_queries - 1) / ta.tile_queries);
     launch_kernel(kernel, dim3(tiles), dim3(32 * warps), total, stream, ta);
     count_launch();
     return check_launch("relation_select_multi_tile_kernel");
@@ -951,7 +1026,7 @@ int launch_multi_tile(MultiTileArgs& ta, void* stream) {
 int tile_warp_bytes(const SelectArgs& a) {
     const int cap4 = (a.local_window + a.top_blocks * a.block_size + 3) & ~3;
     const int floats = 4 * kD + 64 + ((a.n_blocks + 3) & ~3) + cap4;
-    return align16(floats * 4 + 3 * (a.top_blocks > 0 ? a.top_blocks : 1) * 4) + 16 + 32 * static_cast<int>(kPadRow);
+    return align16(floats * 4 + 3 * (a.top_blocks > 0 ? a.top_blocks : 1) * 4) + 16;
 }
 
 int launch_tile(TileArgs& m, void* stream) {
@@ -985,27 +1060,26 @@ int launch_tile(TileArgs& m, void* stream) {
         set_error("relation_select_packed_prefill: at most 512 candidates per query (window + remote blocks)");
         return RLM_ERR_UNSUPPORTED;
     }
-    const bool bf16 = a.query_dtype == RLM_BF16 && a.key_dtype == RLM_BF16 && a.stats_dtype == RLM_BF16;
-    const int key_stride = bf16 ? static_cast<int>(kPadRow) : kD * dtype_size(a.key_dtype);
-    const int stat_stride = bf16 ? static_cast<int>(kPadRow) : kD * dtype_size(a.stats_dtype);
+    const bool fast = a.query_dtype != RLM_F32 && a.key_dtype == a.query_dtype && a.stats_dtype == a.query_dtype;
+    const int key_stride = kD * dtype_size(a.key_dtype), stat_stride = kD * dtype_size(a.stats_dtype);
     m.warp_bytes = tile_warp_bytes(a);
     m.stats_bytes = align16(a.n_blocks * stat_stride);
     m.param_bytes = align16((8 + 8 * a.buckets) * 4);
-    int warps = 16, total = 0;
-    for (;; warps = 8) {
-        m.window_rows = a.local_window + 4 * warps;
-        total = 4 * m.stats_bytes + 2 * m.window_rows * key_stride + m.param_bytes + warps * m.warp_bytes;
-        if (total <= kSmemDynamicLimit || warps == 8) break;
-    }
-    if (total > kSmemDynamicLimit) {
+    const TileShape shape = tile_shape(a.n_seq, m.q_len, fast ? 32 : 16, [&](int warps, int tile) {
+        return 4 * m.stats_bytes + 2 * (a.local_window + tile) * key_stride + m.param_bytes + warps * m.warp_bytes;
+    });
+    if (shape.warps == 0) {
         set_error("relation_select_packed_prefill: block statistics + window union exceed 227 KB of shared memory");
         return RLM_ERR_SMEM;
     }
-    auto kernel = bf16 ? (warps == 16 ? relation_select_tile_kernel<true, 16> : relation_select_tile_kernel<true, 8>)
-                       : (warps == 16 ? relation_select_tile_kernel<false, 16> : relation_select_tile_kernel<false, 8>);
+    const int warps = shape.warps, total = shape.smem_bytes;
+    m.tile_queries = shape.per_warp * warps;
+    m.window_rows = a.local_window + m.tile_queries;
+    auto kernel = !fast ? (warps == 16 ? relation_select_tile_kernel<RLM_F32, 16> : relation_select_tile_kernel<RLM_F32, 8>)
+                  : a.key_dtype == RLM_BF16 ? tile_kernel<RLM_BF16>(warps) : tile_kernel<RLM_F16>(warps);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
-    const int tiles = a.n_seq * ((m.q_len + 4 * warps - 1) / (4 * warps));
+    const int tiles = a.n_seq * ((m.q_len + m.tile_queries - 1) / m.tile_queries);
     launch_kernel(kernel, dim3(tiles), dim3(32 * warps), total, stream, m);
     count_launch();
     return check_launch("relation_select_tile_kernel");
