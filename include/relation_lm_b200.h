@@ -208,7 +208,7 @@ int rlm_relation_hidden_cache_update(
  *   *position.  residual (optional, [N,D] f32, updated in place): residual += (*mix) * context,
  *   the `hidden + sigmoid(mix_logit) * context` of the reference's relation layer
  *   (src/relation_lm/models/stacked_relation.py:124) with mix a device fp32 scalar.
- *   next_normalized (optional, with residual; [N,D] bfloat16 / float16 = next_dtype): LayerNorm of the
+ *   next_normalized (optional, with residual; [N,D] next_dtype): LayerNorm of the
  *   updated residual row with next_norm_weight / next_norm_bias [D] f32 and next_norm_eps, i.e. the
  *   normalised input of the next layer's query projection (or of the output heads).
  *   raw_splits > 1: raw is the sum of raw_splits slices raw_split_stride ELEMENTS apart (the output of
@@ -290,13 +290,13 @@ int rlm_norm_projection(const float* x, int64_t x_row_stride, const float* gamma
                         void* stream);
 
 /*
- * LayerNorm of fp32 rows into a 16-bit matrix (extension): the first half of
+ * LayerNorm of fp32 rows into a matrix of any dtype (extension): the first half of
  * rlm_norm_projection for batches beyond one row tile, where normalising once and streaming
  * the result through rlm_packed_projection beats normalising per output-column tile.  Same
  * arithmetic as rlm_norm_projection; gamma = beta = NULL gives a plain cast.  No reference
  * counterpart beyond `layer_norm(...).to(dtype)` in the model code.
  *   x [rows, d_in] fp32, row stride in ELEMENTS; d_in a multiple of 8 up to 1024;
- *   out [rows, d_in] contiguous bfloat16 / float16.
+ *   out [rows, d_in] contiguous, out_dtype.
  */
 int rlm_layer_norm_cast(const float* x, int64_t x_row_stride, const float* gamma, const float* beta,
                         float eps, void* out, int rows, int d_in, int out_dtype, void* stream);
@@ -487,7 +487,7 @@ int rlm_relation_tail_static(const void* relation_hidden, const void* second_wei
  * out[b] = (token_table[tokens[b]] + boundary_table[boundaries[b]]) * scale + position_table[*position]
  *   tokens, boundaries [B] int64; tables [V, d] / [Vb, d] table_dtype; position_table [T, d] f32;
  *   out [B, d] f32.  Ids outside the tables set RLM_DEV_POSITION and leave the row unwritten.
- *   norm1_out / norm2_out (optional, [B, d] bfloat16 / float16 = norm_out_dtype): LayerNorm of the
+ *   norm1_out / norm2_out (optional, [B, d] norm_out_dtype): LayerNorm of the
  *   embedded row with norm{1,2}_weight / norm{1,2}_bias [d] f32 and norm_eps — the normalised inputs of
  *   the packed projection (memory norm) and of the first layer's query projection (input norm).
  */

@@ -632,13 +632,14 @@ __global__ void __launch_bounds__(kGemmThreads) norm_projection_kernel(
                      ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
-// ------------------------------------------------------------------ LayerNorm -> 16-bit rows
+// ------------------------------------------------------------------ LayerNorm of many rows
 //
 // For batches beyond one row tile the normalisation is done once (a warp per row) into a 16-bit matrix that
 // packed_projection_kernel then streams with TMA, instead of once per output-column tile.  Arithmetic
 // identical to the fused kernel above.  A stream of 6 bytes per element: bound by DRAM as long as nothing
 // else is loaded per row, so a warp keeps its lanes' affine parameters in registers and walks rows.  (With
-// one row per warp and the parameters read element by element: 41 us for 32 768 x 512, 2.4 TB/s.)
+// one row per warp and the parameters read element by element 32 768 x 512 took 41 us, 2.4 TB/s; now 20 us.)
+// fp32 outputs (kDt = RLM_F32) are the end of a stack.
 constexpr int kCastThreads = 256;
 
 struct NormCastArgs {
@@ -651,7 +652,7 @@ struct NormCastArgs {
     int m, k;
 };
 
-template <int kChunks, bool kBf16>
+template <int kChunks, int kDt>
 __global__ void __launch_bounds__(kCastThreads) layer_norm_cast_kernel(const NormCastArgs a) {
     const int lane = threadIdx.x & 31, chunks = a.k / 8;
     float4 g[kChunks][2], b[kChunks][2];
@@ -701,26 +702,33 @@ __global__ void __launch_bounds__(kCastThreads) layer_norm_cast_kernel(const Nor
             if (c >= chunks) continue;
             const float ge[8] = {g[i][0].x, g[i][0].y, g[i][0].z, g[i][0].w, g[i][1].x, g[i][1].y, g[i][1].z, g[i][1].w};
             const float be[8] = {b[i][0].x, b[i][0].y, b[i][0].z, b[i][0].w, b[i][1].x, b[i][1].y, b[i][1].z, b[i][1].w};
-            uint32_t packed[4];
+            float y[8];
 #pragma unroll
-            for (int e = 0; e < 8; e += 2)
-                packed[e / 2] = pack2(fmaf((v[i][e] - mean) * inv, ge[e], be[e]), fmaf((v[i][e + 1] - mean) * inv, ge[e + 1], be[e + 1]),
-                                      kBf16 ? RLM_BF16 : RLM_F16);
-            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + static_cast<size_t>(r) * a.k + 8 * c) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            for (int e = 0; e < 8; ++e) y[e] = fmaf((v[i][e] - mean) * inv, ge[e], be[e]);
+            if constexpr (kDt == RLM_F32) {
+                float4* out = reinterpret_cast<float4*>(static_cast<float*>(a.out) + static_cast<size_t>(r) * a.k + 8 * c);
+                out[0] = make_float4(y[0], y[1], y[2], y[3]);
+                out[1] = make_float4(y[4], y[5], y[6], y[7]);
+            } else {
+                uint32_t packed[4];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) packed[e / 2] = pack2(y[e], y[e + 1], kDt);
+                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + static_cast<size_t>(r) * a.k + 8 * c) =
+                    make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            }
         }
     }
 }
 
-template <bool kBf16>
+template <int kDt>
 void launch_norm_cast(const NormCastArgs& a, void* stream) {
     const int per_cta = kCastThreads / 32, most = 8 * sm_count(), need = (a.m + per_cta - 1) / per_cta;
     const dim3 grid(need < most ? need : most), block(kCastThreads);
     switch ((a.k + 255) / 256) {
-        case 1: launch_kernel(layer_norm_cast_kernel<1, kBf16>, grid, block, 0, stream, a); break;
-        case 2: launch_kernel(layer_norm_cast_kernel<2, kBf16>, grid, block, 0, stream, a); break;
-        case 3: launch_kernel(layer_norm_cast_kernel<3, kBf16>, grid, block, 0, stream, a); break;
-        default: launch_kernel(layer_norm_cast_kernel<4, kBf16>, grid, block, 0, stream, a); break;
+        case 1: launch_kernel(layer_norm_cast_kernel<1, kDt>, grid, block, 0, stream, a); break;
+        case 2: launch_kernel(layer_norm_cast_kernel<2, kDt>, grid, block, 0, stream, a); break;
+        case 3: launch_kernel(layer_norm_cast_kernel<3, kDt>, grid, block, 0, stream, a); break;
+        default: launch_kernel(layer_norm_cast_kernel<4, kDt>, grid, block, 0, stream, a); break;
     }
 }
 
@@ -821,9 +829,9 @@ extern "C" int rlm_layer_norm_cast(const float* x, int64_t x_row_stride, const f
         set_error("layer_norm_cast: need d_in a multiple of 8 up to 1024");
         return RLM_ERR_SHAPE;
     }
-    if (out_dtype != RLM_BF16 && out_dtype != RLM_F16) {
-        set_error("layer_norm_cast: the output must be bfloat16 or float16");
-        return RLM_ERR_UNSUPPORTED;
+    if (!valid_dtype(out_dtype)) {
+        set_error("layer_norm_cast: unknown dtype code");
+        return RLM_ERR_DTYPE;
     }
     if (!aligned16(x) || !aligned16(out) || (gamma && (!aligned16(gamma) || !aligned16(beta)))) {
         set_error("layer_norm_cast: tensors must be 16-byte aligned");
@@ -832,8 +840,9 @@ extern "C" int rlm_layer_norm_cast(const float* x, int64_t x_row_stride, const f
     NormCastArgs a{};
     a.x = x; a.gamma = gamma; a.beta = beta; a.out = out; a.x_stride = x_row_stride; a.eps = eps;
     a.m = rows; a.k = d_in;
-    if (out_dtype == RLM_BF16) launch_norm_cast<true>(a, stream);
-    else launch_norm_cast<false>(a, stream);
+    if (out_dtype == RLM_BF16) launch_norm_cast<RLM_BF16>(a, stream);
+    else if (out_dtype == RLM_F16) launch_norm_cast<RLM_F16>(a, stream);
+    else launch_norm_cast<RLM_F32>(a, stream);
     count_launch();
     return check_launch("layer_norm_cast_kernel");
 }

@@ -29,6 +29,7 @@ using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 using Two = std::tuple<Tensor, Tensor>;
 using Four = std::tuple<Tensor, Tensor, Tensor, Tensor>;
+using Five = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>;
 using Six = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor>;
 
 // ------------------------------------------------------------------ checks
@@ -244,7 +245,7 @@ Four relation_select_packed_prefill(SELECT_PARAMS, int64_t query_length, int64_t
 
 // Shared by the two multi-anchor forms: shapes, outputs and the call.  The kernels write the anchors'
 // activity as bytes 0 / 1, which is the storage of a bool tensor.
-Six select_multi(const char* name, const SelectTensors& s, const Tensor* row_batch, const Tensor* row_position,
+Five select_multi(const char* name, const SelectTensors& s, const Tensor* row_batch, const Tensor* row_position,
                  int64_t query_length, int64_t local_window, int64_t top_blocks, int64_t k_out, bool strict_valid) {
     for (const Named& a : {Named{"anchor_query", &s.anchor_query}, Named{"anchor_router_query", &s.anchor_router_query},
                            Named{"partner_base", &s.partner_base}})
@@ -292,17 +293,28 @@ Six select_multi(const char* name, const SelectTensors& s, const Tensor* row_bat
             s.anchor_query.stride(0), s.anchor_router_query.stride(0), s.partner_base.stride(0), query_length, batch, slots,
             max_t, nb, s.anchor_bias.size(2), local_window, top_blocks, k_out, strict_valid, q, k, st, p, launch.status,
             launch.stream));
-    return {anchor, anchor_score, active, partner, score, at::isfinite(score)};
+    return {anchor, anchor_score, active, partner, score};
+}
+
+Six with_partner_active(const Five& s) {
+    return std::tuple_cat(s, std::make_tuple(at::isfinite(std::get<4>(s))));
 }
 
 Six relation_select_multi_rows(SELECT_PARAMS, const Tensor& row_batch, const Tensor& row_position, int64_t local_window,
                                int64_t top_blocks, int64_t partners_per_anchor, bool strict_valid) {
-    return select_multi("relation_select_multi_rows", SELECT_TENSORS, &row_batch, &row_position, 0, local_window, top_blocks,
-                        partners_per_anchor, strict_valid);
+    return with_partner_active(select_multi("relation_select_multi_rows", SELECT_TENSORS, &row_batch, &row_position, 0,
+                                            local_window, top_blocks, partners_per_anchor, strict_valid));
 }
 
 Six relation_select_multi_prefill(SELECT_PARAMS, int64_t query_length, int64_t local_window, int64_t top_blocks,
                                   int64_t partners_per_anchor, bool strict_valid) {
+    return with_partner_active(select_multi("relation_select_multi_prefill", SELECT_TENSORS, nullptr, nullptr, query_length,
+                                            local_window, top_blocks, partners_per_anchor, strict_valid));
+}
+
+// ... without the partners' activity (finite scores), four elementwise launches that the fused layer has no use for
+Five relation_select_multi_prefill_scores(SELECT_PARAMS, int64_t query_length, int64_t local_window, int64_t top_blocks,
+                                          int64_t partners_per_anchor, bool strict_valid) {
     return select_multi("relation_select_multi_prefill", SELECT_TENSORS, nullptr, nullptr, query_length, local_window,
                         top_blocks, partners_per_anchor, strict_valid);
 }
@@ -838,7 +850,7 @@ Tensor decode_embed_norm(const Tensor& tokens, const Tensor& boundaries, const T
         TORCH_CHECK_VALUE(is_f32(*t) && t->numel() == d_model, "LayerNorm parameters must be float32 [d_model]");
     TORCH_CHECK_VALUE(is_shape(normalized1, {batch, d_model}) && is_shape(normalized2, {batch, d_model}) &&
                           normalized1.scalar_type() == normalized2.scalar_type(),
-                      "normalized outputs must be [B, d_model] of one 16-bit dtype");
+                      "normalized outputs must be [B, d_model] of one dtype");
     const int table = same_dtype("embedding table", {&token_table, &boundary_table});
     Launch launch(device);
     Tensor out = empty({batch, d_model}, at::kFloat, device);
@@ -962,6 +974,9 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
     PURE(relation_select_multi_prefill, "(" SELECT_SCHEMA "SymInt query_length, SymInt local_window, "                   \
          "SymInt top_blocks, SymInt partners_per_anchor, bool strict_valid) -> "                                         \
          "(Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)")                                                             \
+    PURE(relation_select_multi_prefill_scores, "(" SELECT_SCHEMA "SymInt query_length, SymInt local_window, "            \
+         "SymInt top_blocks, SymInt partners_per_anchor, bool strict_valid) -> "                                         \
+         "(Tensor, Tensor, Tensor, Tensor, Tensor)")                                                                     \
     MUTATES(router_cache_update,                                                                                         \
             "(Tensor anchor_raw, Tensor partner_raw, Tensor(a2!) anchor_raw_cache, Tensor(a3!) partner_raw_cache, "      \
             "Tensor(a4!) anchor_conv_cache, Tensor(a5!) partner_conv_cache, Tensor(a6!) anchor_mean, "                   \

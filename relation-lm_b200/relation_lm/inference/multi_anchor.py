@@ -29,7 +29,8 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor, nn
 
-from relation_lm.kernels.relation_reduce import MLP_ROWS_MIN_PAIRS, relation_mlp_rows, relation_mlp_rows_supported
+from relation_lm.kernels import _abi
+from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
 
 
 @dataclass
@@ -203,6 +204,7 @@ class MultiAnchorPrefill:
         rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
         return rb, rp
 
+    @_abi.programmatic_launch
     def build_state(self, layer: int, memory: Tensor) -> dict[str, Tensor]:
         """Per-slot caches and block statistics of layer ``layer`` for ``memory [B, T, d]`` (16-bit)."""
         from relation_lm.kernels.packed_projection import packed_projection
@@ -218,18 +220,26 @@ class MultiAnchorPrefill:
                                                     w["b_expand"]).view(B, T, 2 * H)
         return state
 
-    def forward_layer(self, layer: int, hidden: Tensor, state: dict[str, Tensor], keep: dict | None = None) -> Tensor:
-        """Updates the residual stream ``hidden [B, T, d]`` (fp32) in place and returns it."""
-        from relation_lm.kernels.multi_select import (relation_select_multi_prefill, relation_select_multi_rows,
-                                                      slot_mix_residual)
+    @_abi.programmatic_launch
+    def forward_layer(self, layer: int, hidden: Tensor, state: dict[str, Tensor], keep: dict | None = None,
+                      source: Tensor | None = None) -> Tensor:
+        """Updates the residual stream ``hidden [B, T, d]`` (fp32) in place and returns it; with ``source``
+        the stream enters there, untouched, and only the result goes to ``hidden``."""
+        from relation_lm.kernels.multi_select import (relation_select_multi_prefill, relation_select_multi_prefill_scores,
+                                                      relation_select_multi_rows, slot_mix_residual)
         from relation_lm.kernels.packed_projection import layer_norm_cast, packed_projection
         from relation_lm.kernels.relation_reduce import relation_hidden_cached_rows_out, relation_norm_reduce_rows
 
         cfg, w = self.config, self.layers[layer]
         B, T, d = hidden.shape
         N, S, K, H = B * T, cfg.anchors_per_block, cfg.partners_per_anchor, cfg.hidden_dim
+        fused = self.fused_mlp and keep is None
+        if source is None:
+            source = hidden
+        elif not (fused and self.fused_mix):
+            source = hidden.copy_(source)
         normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
-        layer_norm_cast(hidden.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
+        layer_norm_cast(source.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
         q = packed_projection(normalized, w["w_query"])                          # [N, S * 256]
         anchor_query = q[:, :S * 64].unflatten(1, (S, 64))                       # column slices of one projection
         anchor_router_query = q[:, S * 64:S * 128].unflatten(1, (S, 64))
@@ -238,32 +248,30 @@ class MultiAnchorPrefill:
                        w["anchor_gamma"], w["anchor_bias"], partner_base, state["partner_anchor_cache"],
                        state["partner_keys"], state["partner_mean"], state["partner_std"], w["partner_gamma"],
                        w["partner_bias"])
-        tiled = (self.tiled_select and self.dtype == torch.bfloat16
-                 and cfg.local_window + cfg.top_blocks * cfg.block_size <= 512)
+        tiled = self.tiled_select and cfg.local_window + cfg.top_blocks * cfg.block_size <= 512
         selected = None
         if tiled:
             # whole sequences: tiles of consecutive positions share the staged statistics and windows
             try:
-                selected = relation_select_multi_prefill(*select_args, T, cfg.local_window, cfg.top_blocks, K,
-                                                         cfg.strict_valid)
+                select = relation_select_multi_prefill if keep is not None else relation_select_multi_prefill_scores
+                selected = select(*select_args, T, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
             except (ValueError, RuntimeError) as error:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
-        fused = self.fused_mlp and keep is None and N * S * K >= MLP_ROWS_MIN_PAIRS
         if selected is None or not fused:
             rb, rp = self.rows(B, T)
         if selected is None:
             selected = relation_select_multi_rows(*select_args, rb, rp, cfg.local_window, cfg.top_blocks, K,
                                                   cfg.strict_valid)
-        anchor, anchor_score, anchor_active, partner, partner_score, partner_active = selected
+        anchor, anchor_score, anchor_active, partner, partner_score = selected[:5]
         if fused:
             mlp = (state["expanded_cache"], state["operand_cache"], anchor, partner, partner_score)
             weights = (w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"], cfg.norm_eps)
             # softmax over the finite partner scores of a slot, no active-K limit
             if self.fused_mix:
                 relation_mlp_rows(hidden.view(N, d), *mlp, anchor_active, w["slot_weight"], w["gate"], *weights,
-                                  hidden.view(N, d), S, T, False)
+                                  source.view(N, d), S, T, False)
             else:
                 slot_context = torch.empty(N * S, d, device=self.device, dtype=torch.float32)
                 relation_mlp_rows(slot_context, *mlp, None, None, None, *weights, None, 1, T * S, False)
@@ -281,20 +289,23 @@ class MultiAnchorPrefill:
         slot_mix_residual(slot_context, anchor_active, w["slot_weight"], w["gate"], hidden.view(N, d))
         if keep is not None:
             keep.update(query=q, anchor=anchor, anchor_score=anchor_score, anchor_active=anchor_active,
-                        partner=partner, partner_score=partner_score, partner_active=partner_active,
+                        partner=partner, partner_score=partner_score, partner_active=selected[5],
                         hidden_rel=hidden_rel, raw=raw, slot_context=slot_context, row_batch=rb, row_position=rp)
         return hidden
 
     def forward(self, hidden: Tensor, memory: Tensor, keep: list | None = None) -> Tensor:
         """The stack's output ``[B, T, d]`` (fp32): ``depth`` layers on a copy of ``hidden`` with one
         shared ``memory`` (16-bit), then the final LayerNorm."""
-        current = hidden.clone()
+        from relation_lm.kernels.packed_projection import layer_norm_cast
+
+        current, source = torch.empty_like(hidden, memory_format=torch.contiguous_format), hidden.contiguous()
         for l in range(self.config.depth):
             state = self.build_state(l, memory)
             kept = {} if keep is not None else None
-            self.forward_layer(l, current, state, kept)
+            self.forward_layer(l, current, state, kept, source if l == 0 else None)
             if keep is not None:
                 kept["state"] = state
                 keep.append(kept)
-        return torch.nn.functional.layer_norm(current, (current.size(-1),), self.final_norm_w, self.final_norm_b,
-                                              self.config.norm_eps)
+        out, d = torch.empty_like(current), current.size(-1)
+        layer_norm_cast(current.view(-1, d), self.final_norm_w, self.final_norm_b, self.config.norm_eps, out.view(-1, d))
+        return out

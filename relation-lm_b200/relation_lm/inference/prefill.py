@@ -26,8 +26,9 @@ import torch
 from torch import Tensor
 
 from relation_lm.inference.routed_model import RoutedRelationLM
+from relation_lm.kernels import _abi
 from relation_lm.kernels.packed_projection import layer_norm_cast, packed_projection
-from relation_lm.kernels.relation_reduce import (MLP_ROWS_MIN_PAIRS, relation_hidden_cached_rows_out, relation_mlp_rows,
+from relation_lm.kernels.relation_reduce import (relation_hidden_cached_rows_out, relation_mlp_rows,
                                                  relation_mlp_rows_supported, relation_norm_reduce_rows)
 from relation_lm.kernels.relation_select import relation_select_packed_prefill, relation_select_packed_rows
 from relation_lm.kernels.router_cache import sequence_state
@@ -39,6 +40,7 @@ class RoutedPrefillLayer:
     def __init__(self, model: RoutedRelationLM, layer: int = 0, device="cuda",
                  dtype: torch.dtype = torch.bfloat16, tiled_select: bool = True) -> None:
         self.tiled_select = bool(tiled_select)
+        self._rows: tuple | None = None
         if dtype not in (torch.bfloat16, torch.float16):
             raise ValueError("the prefill path runs its projections on the tensor cores: bfloat16 or float16")
         self.config, self.layer, self.device, self.dtype = model.config, int(layer), torch.device(device), dtype
@@ -63,11 +65,16 @@ class RoutedPrefillLayer:
         }
 
     def rows(self, batch: int, length: int) -> tuple[Tensor, Tensor]:
-        """``(row_batch, row_position)`` of all ``batch * length`` query rows, sequence-major."""
-        rb = torch.arange(batch, device=self.device, dtype=torch.int32).repeat_interleave(length)
-        rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
-        return rb, rp
+        """``(row_batch, row_position)`` of all ``batch * length`` query rows, sequence-major; the tables of the
+        last size are kept (building them takes four launches)."""
+        kept = self._rows
+        if kept is None or kept[0] != (batch, length):
+            rb = torch.arange(batch, device=self.device, dtype=torch.int32).repeat_interleave(length)
+            rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
+            kept = self._rows = ((batch, length), rb, rp)
+        return kept[1], kept[2]
 
+    @_abi.programmatic_launch
     def build_state(self, x: Tensor) -> dict[str, Tensor]:
         """Caches and block statistics of sequences whose embedded inputs are ``x [B, T, d]`` (fp32)."""
         cfg, w = self.config, self.w
@@ -84,6 +91,7 @@ class RoutedPrefillLayer:
         state["packed"] = packed
         return state
 
+    @_abi.programmatic_launch
     def forward(self, x: Tensor, state: dict[str, Tensor], keep: dict | None = None) -> Tensor:
         """The layer's output ``[B, T, d]`` (fp32) for residual inputs ``x [B, T, d]`` (fp32).  With a
         dict in ``keep`` the intermediates (queries, selections, hidden states, second-layer
@@ -108,7 +116,7 @@ class RoutedPrefillLayer:
                 if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
                     raise
                 self.tiled_select = False                   # rejected before anything was launched
-        fused = self.fused_mlp and keep is None and N * K >= MLP_ROWS_MIN_PAIRS
+        fused = self.fused_mlp and keep is None
         if selected is None or not fused:
             rb, rp = self.rows(B, T)
         if selected is None:

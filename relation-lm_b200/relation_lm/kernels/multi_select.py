@@ -25,6 +25,8 @@ from relation_lm.kernels import _abi  # noqa: F401  (loads the libraries)
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
 _relation_select_multi_rows = torch.ops.relation_lm.relation_select_multi_rows.default
 _relation_select_multi_prefill = torch.ops.relation_lm.relation_select_multi_prefill.default
+# the same without its last output (the partners' activity)
+relation_select_multi_prefill_scores = torch.ops.relation_lm.relation_select_multi_prefill_scores.default
 _slot_mix_residual = torch.ops.relation_lm.slot_mix_residual.default
 
 
@@ -95,7 +97,7 @@ def relation_select_multi_prefill(
     partners_per_anchor: int,
     strict_valid: bool,
 ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
-    """Whole-sequence form of ``relation_select_multi_rows`` (bfloat16 tensors): query row
+    """Whole-sequence form of ``relation_select_multi_rows`` (one 16-bit dtype throughout): query row
     ``b * query_length + t`` is position ``t`` of sequence ``b``; same results, bit for bit.  A CTA
     serves a tile of consecutive positions and stages each slot's block statistics and window union
     once per tile."""
@@ -118,6 +120,19 @@ def _(anchor_query, anchor_keys, anchor_router_query, anchor_block_mean, anchor_
             anchor_query.new_empty((rows, slots, k), dtype=torch.int32),
             anchor_query.new_empty((rows, slots, k), dtype=f32),
             anchor_query.new_empty((rows, slots, k), dtype=torch.bool))
+
+
+@torch.library.register_fake("relation_lm::relation_select_multi_prefill_scores")
+def _(anchor_query, anchor_keys, anchor_router_query, anchor_block_mean, anchor_block_std, anchor_gamma,
+      anchor_bias, partner_base, partner_anchor_cache, partner_keys, partner_block_mean, partner_block_std,
+      partner_gamma, partner_bias, query_length, local_window, top_blocks, partners_per_anchor, strict_valid):
+    rows, slots = anchor_query.size(0), anchor_query.size(1)
+    k = partners_per_anchor
+    f32 = torch.float32
+    return (anchor_query.new_empty((rows, slots), dtype=torch.int32), anchor_query.new_empty((rows, slots), dtype=f32),
+            anchor_query.new_empty((rows, slots), dtype=torch.bool),
+            anchor_query.new_empty((rows, slots, k), dtype=torch.int32),
+            anchor_query.new_empty((rows, slots, k), dtype=f32))
 
 
 def slot_mix_residual(slot_context: Tensor, anchor_active: Tensor, slot_weight: Tensor, gate: Tensor,

@@ -65,7 +65,7 @@ def _(x, weight, splits):
 
 
 def layer_norm_cast(x: Tensor, norm_weight: Tensor, norm_bias: Tensor, norm_eps: float, out: Tensor) -> None:
-    """``out = layer_norm(x)`` for fp32 rows ``[rows, d]`` into a bfloat16 / float16 matrix."""
+    """``out = layer_norm(x)`` for fp32 rows ``[rows, d]``, in the dtype of ``out``."""
     _layer_norm_cast(x, norm_weight, norm_bias, norm_eps, out)
 
 
@@ -138,7 +138,7 @@ def decode_embed_norm(tokens: Tensor, boundaries: Tensor, token_table: Tensor, b
                       position_table: Tensor, position: Tensor, scale: float, norm1_weight: Tensor,
                       norm1_bias: Tensor, normalized1: Tensor, norm2_weight: Tensor, norm2_bias: Tensor,
                       normalized2: Tensor, norm_eps: float) -> Tensor:
-    """``decode_embed`` that also writes two LayerNorms of the embedded rows as 16-bit matrices
+    """``decode_embed`` that also writes two LayerNorms of the embedded rows in the outputs' dtype
     (``normalized1`` with the memory norm for the packed projection, ``normalized2`` with the first
     layer's input norm for its query projection); returns the fp32 rows."""
     return _decode_embed_norm(tokens, boundaries, token_table, boundary_table, position_table, position, scale,

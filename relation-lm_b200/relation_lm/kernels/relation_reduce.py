@@ -285,7 +285,7 @@ def relation_norm_reduce_residual_norm(
     normalized: Tensor,
 ) -> None:
     """``relation_norm_reduce_residual`` that also writes ``normalized = layer_norm(hidden)`` of
-    the updated rows (extension): ``normalized [B, D]`` bfloat16 / float16 with the next layer's
+    the updated rows (extension): ``normalized [B, D]`` in its own dtype, with the next layer's
     (or the output head's) fp32 LayerNorm parameters, ready for the next projection."""
     _relation_norm_reduce_residual_norm(raw, partner_scores, norm_weight, norm_bias, position, norm_eps, hidden, mix,
                                         next_norm_weight, next_norm_bias, next_norm_eps, normalized)
@@ -480,15 +480,11 @@ def _(raw, partner_scores, norm_weight, norm_bias, row_position, norm_eps):
     return raw.new_empty((raw.size(0), raw.size(2)), dtype=torch.float32)
 
 
-# Half a tile of 128 pairs for each of a B200's 148 SMs.  The one-launch form walks a tile's hidden columns one
-# after another (37 us for a tile of 256 pairs at d 256); below this the three launches, which spread the
-# hidden columns over the SMs, take less (27 us for 4096 pairs at d 256).
-MLP_ROWS_MIN_PAIRS = 9472
-
-
 def relation_mlp_rows_supported(k_out: int, slots: int, relation_dim: int, hidden_dim: int, d_model: int,
                                 dtype: torch.dtype) -> bool:
-    """Whether ``relation_mlp_rows`` serves these sizes.  Worth it from ``MLP_ROWS_MIN_PAIRS`` pairs up."""
+    """Whether ``relation_mlp_rows`` serves these sizes.  Worth it from the smallest pass up: 256 rows of d 256 with
+    K 4 take 27 us in three kernels against 37 in one, but the pass is then bound by its launches (122 us against 99
+    with five fewer); 1024 pairs of d 768 are even, and everything above is faster in one."""
     return dtype in (torch.bfloat16, torch.float16) and bool(_abi.LIB.rlm_relation_mlp_rows_supported(
         int(k_out), int(slots), int(relation_dim), int(hidden_dim), int(d_model), _abi.DTYPE_CODE[dtype]))
 
