@@ -58,8 +58,10 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
     const int most = kLtMaxPairs / tail.k_out < kLtMaxSeq ? kLtMaxPairs / tail.k_out : kLtMaxSeq;
     tail.seqs_per_cluster = (tail.n_seq + 3) / 4 < most ? (tail.n_seq + 3) / 4 : most;
     if (tail.seqs_per_cluster > tail.cluster) tail.seqs_per_cluster = tail.cluster;   // a selecting CTA per sequence
-    const LtPlan whole = lt_plan(tail.rdim, tail.d, kLtMaxPairs);
-    if (sel.plan.total > static_cast<int>(whole.total - whole.p)) {
+    const uint32_t smem_bytes = lt_smem_bytes_with_stage(tail.rdim, tail.d, tail.query_weight ? tail.n_query / tail.cluster : 0,
+                                                         sel.plan.total);
+    const LtPlan whole = lt_plan(tail.rdim, tail.d, kLtMaxPairs, 0);
+    if (sel.plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) {
         set_error("relation_layer: the selector's working set does not fit the tail's tile memory (use the two launches)");
         return RLM_ERR_UNSUPPORTED;
     }
@@ -78,7 +80,6 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), tail.cluster);
     if (rc != RLM_OK) return rc;
     const int clusters = (tail.n_seq + tail.seqs_per_cluster - 1) / tail.seqs_per_cluster;
-    const size_t smem_bytes = lt_plan(tail.rdim, tail.d, kLtMaxPairs).total + 1024;
     launch_kernel_cluster(kernel, dim3(tail.cluster, clusters), dim3(kLtThreads), static_cast<unsigned>(tail.cluster),
                           smem_bytes, stream, mwm, mw2, tail, sel);
     count_launch();
@@ -104,14 +105,15 @@ extern "C" int rlm_relation_layer_supported(int n_seq, int k_out, int relation_d
     const int cluster = hidden_dim / kLtHC;
     const Plan plan = make_plan(n_blocks, max_t / n_blocks, local_window, top_blocks, buckets, dtype_size(dtype),
                                 dtype_size(dtype), kPacked, false);
-    const LtPlan whole = lt_plan(relation_dim, d_model, kLtMaxPairs);
-    if (plan.total > static_cast<int>(whole.total - whole.p)) return 0;
+    const uint32_t smem_bytes = lt_smem_bytes_with_stage(relation_dim, d_model, n_query / cluster, plan.total);
+    const LtPlan whole = lt_plan(relation_dim, d_model, kLtMaxPairs, 0);
+    if (plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) return 0;
     auto kernel = dtype == RLM_BF16 ? relation_layer_kernel<true> : relation_layer_kernel<false>;
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(cluster, 1, 1);
     config.blockDim = dim3(kLtThreads, 1, 1);
-    config.dynamicSmemBytes = lt_plan(relation_dim, d_model, kLtMaxPairs).total + 1024;
+    config.dynamicSmemBytes = smem_bytes;
     cudaLaunchAttribute attribute[1];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
     attribute[0].val.clusterDim.x = cluster;

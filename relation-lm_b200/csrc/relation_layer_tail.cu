@@ -18,19 +18,23 @@
 // expanded-cache terms, runs the product GEMM with the hidden columns on the TMEM lanes
 // (tcgen05.mma, pairs on the TMEM columns), applies GELU and writes its hidden slice as the
 // K-major B tile of the second GEMM, whose A operand is the resident W_2 slice: a split-K GEMM
-// over the cluster, each CTA holding a partial raw^T [d, pairs] in TMEM.  The partials are dumped
-// to shared memory and reduced through distributed shared memory: CTA c pulls the d / C output
-// rows it owns from all CTAs in a fixed order (deterministic sums), adds the bias and keeps
-// raw[pairs, d / C].  LayerNorm statistics over the full width are combined across the cluster
-// from per-CTA (mean, M2) pairs (Chan's parallel variance), which every CTA stores into the
-// shared memory of all the others before the barrier (no remote load after it); softmax weights,
-// context, residual update and the next LayerNorm follow the same way, and the normalised rows
-// are handed to every CTA for its share of the query projection.  Four cluster barriers in total.
+// over the cluster, each CTA holding a partial raw^T [d, pairs] in TMEM.
+//
+// What bounds the launch is a chain of some twenty dependent phases, so the CTAs hand their results on by pushing
+// them into the receiver's shared memory with stores that count towards a barrier of the receiver (st.async), and a
+// receiver waits for exactly what it needs: no cluster-wide barrier lies in the chain and no remote load.  Three
+// exchanges: the partial sums go from the accumulators straight to the CTA that owns the output row (d / C rows
+// each, summed in rank order: deterministic); (mean, M2) of a CTA's 32 columns per pair to every CTA (Chan's
+// parallel variance); the updated residual columns to every CTA, which then normalises whole rows for its share of
+// the query projection.  Cluster barriers remain off the chain: one split in two halves around the second GEMM (the
+// weight slice whose place receives the partial sums has been consumed everywhere), one around the projection (no
+// CTA leaves while another may still push to it).  With four cluster barriers, partial sums dumped and pulled and
+// normalised rows stored value by value, a step of the 6-layer model took 150 us at batch 1, now 139 us.
 //
 // Semantics follow src/relation_lm/kernels/relation_reduce.py:72-146 and 360-417 of the
 // reference project with the cuBLAS second layer of benchmarks/benchmark_relation_reduce.py:55-64
 // in between, and `hidden + sigmoid(mix) * context` of models/stacked_relation.py:124.
-// Every wait is bounded; on expiry the kernel sets RLM_DEV_TIMEOUT, still passes every cluster
+// Every wait is bounded; on expiry the kernel sets RLM_DEV_TIMEOUT, still pushes what it owes and passes every cluster
 // barrier (so no CTA waits for a peer that left), frees its TMEM and returns.
 
 #include "relation_layer_tail_body.cuh"
@@ -65,7 +69,7 @@ extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relat
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(cluster, 1, 1);
     config.blockDim = dim3(kLtThreads, 1, 1);
-    config.dynamicSmemBytes = lt_plan(relation_dim, d_model, kLtMaxPairs).total + 1024;
+    config.dynamicSmemBytes = lt_smem_bytes(relation_dim, d_model, n_query / cluster);
     cudaLaunchAttribute attribute[1];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
     attribute[0].val.clusterDim.x = cluster;
@@ -127,7 +131,7 @@ extern "C" int rlm_relation_layer_tail(
     auto kernel = dtype == RLM_BF16 ? relation_layer_tail_kernel<true> : relation_layer_tail_kernel<false>;
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), a.cluster);
     if (rc != RLM_OK) return rc;
-    const size_t smem_bytes = lt_plan(relation_dim, d_model, kLtMaxPairs).total + 1024;
+    const size_t smem_bytes = lt_smem_bytes(relation_dim, d_model, a.n_query / a.cluster);
     launch_kernel_cluster(kernel, dim3(a.cluster, clusters), dim3(kLtThreads),
                           static_cast<unsigned>(a.cluster), smem_bytes, stream, mwm, mw2, a);
     count_launch();

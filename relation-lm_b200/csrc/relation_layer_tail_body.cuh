@@ -43,24 +43,52 @@ struct LayerTailArgs {
 
 // Shared-memory plan (byte offsets from the 1024-aligned dynamic base).
 struct LtPlan {
-    uint32_t wm, w2, p, hid, term_p, term_a, op_a, total;
+    uint32_t wm, w2, p, hid, term_p, term_a, op_a, wq, total;
 };
 
-__host__ __device__ inline LtPlan lt_plan(int rdim, int d, int pairs_pad) {
+// The partial sums that a CTA receives, [sender][four pairs][owned column][pair] of 512 d pairs / 128 bytes in all,
+// take the place of a consumed weight slice: W_m's for 16 pairs, W_2's for more (the W_q slice then waits for W_m's).
+// nq_own: rows of the query-projection weight per CTA.
+__host__ __device__ inline LtPlan lt_plan(int rdim, int d, int pairs_pad, int nq_own) {
     LtPlan p;
     uint32_t off = 0;
-    p.wm = off;     off += static_cast<uint32_t>(rdim / kBK) * kBM * 128u;           // W_m slice; later the W_q slice
-    p.w2 = off;     off += static_cast<uint32_t>(d / kBM) * 2u * kBM * 128u;         // W_2 slice; later the partial dump
-    p.p = off;      off += static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u;     // product tile; later the owned raw values
-    if (off - p.p < kLtMaxPairs * kLtOwnStride * 4u) off = p.p + kLtMaxPairs * kLtOwnStride * 4u;
+    const uint32_t received = 4u * static_cast<uint32_t>(d) * pairs_pad;
+    p.wm = off;     off += static_cast<uint32_t>(rdim / kBK) * kBM * 128u;           // W_m slice
+    if (pairs_pad == 16 && off < received) off = received;
+    p.w2 = off;     off += static_cast<uint32_t>(d / kBM) * 2u * kBM * 128u;         // W_2 slice
+    p.p = off;      off += static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u;     // product tile; later normalised pairs, then rows
+    if (off - p.p < pairs_pad * kLtOwnStride * 4u) off = p.p + pairs_pad * kLtOwnStride * 4u;
+    if (off - p.p < static_cast<uint32_t>(kLtMaxSeq) * d * 2u) off = p.p + kLtMaxSeq * d * 2u;
     off = (off + 1023u) & ~1023u;
-    p.hid = off;    off += 2u * pairs_pad * 128u;                                    // hidden tile; later the normalised rows
-    if (off - p.hid < static_cast<uint32_t>(kLtMaxSeq) * d * 2u) off = p.hid + kLtMaxSeq * d * 2u;
-    p.term_p = off; off += kLtMaxPairs * kLtTermStride;
+    p.hid = off;    off += 2u * pairs_pad * 128u;                                    // hidden tile; later the residual rows
+    if (off - p.hid < static_cast<uint32_t>(kLtMaxSeq) * d * 4u) off = p.hid + kLtMaxSeq * d * 4u;
+    p.term_p = off; off += pairs_pad * kLtTermStride;
     p.term_a = off; off += kLtMaxSeq * kLtTermStride;
     p.op_a = off;   off += kLtMaxSeq * static_cast<uint32_t>(rdim) * 2u;
+    p.wq = p.wm;
+    if (pairs_pad == 16) { p.wq = off; off += static_cast<uint32_t>(nq_own) * (2u * d + 256u); }
     p.total = off;
     return p;
+}
+
+// Dynamic shared memory of a launch, whatever its pairs per cluster.
+inline uint32_t lt_smem_bytes(int rdim, int d, int nq_own) {
+    uint32_t most = 0;
+    for (int pairs = 16; pairs <= kLtMaxPairs; pairs *= 2) {
+        const uint32_t total = lt_plan(rdim, d, pairs, nq_own).total;
+        if (total > most) most = total;
+    }
+    return most + 1024;
+}
+
+// Dynamic shared memory of a whole-layer launch, whose stage needs `stage` bytes behind the weight slices.
+inline uint32_t lt_smem_bytes_with_stage(int rdim, int d, int nq_own, int stage) {
+    uint32_t most = lt_smem_bytes(rdim, d, nq_own);
+    for (int pairs = 16; pairs <= kLtMaxPairs; pairs *= 2) {
+        const uint32_t total = lt_plan(rdim, d, pairs, nq_own).p + static_cast<uint32_t>(stage) + 1024u;
+        if (total > most) most = total;
+    }
+    return most;
 }
 
 __device__ __forceinline__ uint32_t lt_cluster_rank() {
@@ -77,17 +105,37 @@ __device__ __forceinline__ uint32_t lt_peer(uint32_t local_addr, uint32_t rank) 
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
     return remote;
 }
-__device__ __forceinline__ float4 lt_ld_peer16(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
+__device__ __forceinline__ void lt_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void lt_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Stores into another CTA's shared memory that count towards a barrier of that CTA (both addresses from lt_peer).
+__device__ __forceinline__ void lt_push16(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void lt_st_peer8(uint32_t addr, float x, float y) {
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+__device__ __forceinline__ void lt_push8(uint32_t addr, uint32_t bar, float x, float y) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                 ::"r"(addr), "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void lt_st_peer2(uint32_t addr, uint16_t v) {
-    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+__device__ __forceinline__ void lt_push4(uint32_t addr, uint32_t bar, float x) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+                 ::"r"(addr), "r"(__float_as_uint(x)), "r"(bar) : "memory");
+}
+
+// Sum of a[j] over the warp, for j = lane / 8.
+__device__ __forceinline__ float lt_fold4(const float (&a)[4]) {
+    const bool hi = threadIdx.x & 16, mid = threadIdx.x & 8;
+    const float b0 = (hi ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], 16);
+    const float b1 = (hi ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], 16);
+    float c = (mid ? b1 : b0) + __shfl_xor_sync(0xffffffffu, mid ? b0 : b1, 8);
+    c += __shfl_xor_sync(0xffffffffu, c, 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
+__device__ __forceinline__ void lt_tmem_ld4(uint32_t addr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
 }
 
 __device__ __forceinline__ float lt_from16(uint16_t bits, int dtype) {
@@ -111,12 +159,12 @@ struct NoStage {
 template <bool kBf16, typename Stage>
 __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const CUtensorMap& map_w2,
                                                 const LayerTailArgs& a, unsigned char* lt_smem_raw, const Stage& stage) {
-    __shared__ __align__(8) unsigned long long bars[4];          // W_m, W_2, product GEMM done, second GEMM done
+    // W_m, W_2, product GEMM done, second GEMM done; partial sums, pair statistics, residual rows received
+    __shared__ __align__(8) unsigned long long bars[7];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
     __shared__ int pair_seq_s[kLtMaxPairs];
     __shared__ float weight_s[kLtMaxPairs];
-    __shared__ __align__(8) float2 ln_s[kLtMaxPairs];            // (mean, rstd) per pair over the full width
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dtype = kBf16 ? static_cast<int>(RLM_BF16) : static_cast<int>(RLM_F16);
@@ -134,7 +182,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    const LtPlan plan = lt_plan(R, D, pairs_pad);
+    const int nq_own = a.query_weight ? a.n_query / C : 0;
+    const LtPlan plan = lt_plan(R, D, pairs_pad, nq_own);
     unsigned char* wm_tile = base + plan.wm;
     unsigned char* w2_tile = base + plan.w2;
     unsigned char* p_tile = base + plan.p;
@@ -143,26 +192,53 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     unsigned char* term_a = base + plan.term_a;
     unsigned char* op_a = base + plan.op_a;
     const uint32_t p_kblock = static_cast<uint32_t>(pairs_pad) * 128u;
-    // Once every CTA has dumped its partial sums, the term rows are dead in the whole cluster: their
-    // place receives the LayerNorm statistics that the CTAs push to one another, [sender][pair]
-    // and [sender][sequence] of (mean, M2) over the sender's 32 columns.
+    // A CTA that has received all partial sums knows that every CTA is past its epilogue and its second GEMM: the
+    // term rows' place receives the statistics that the CTAs push to one another, [sender][pair] of (mean, M2) over
+    // the sender's 32 columns, and the hidden tile's place the residual rows [sequence][d].
     float2* stats_in = reinterpret_cast<float2*>(term_p);
-    float2* stats2_in = reinterpret_cast<float2*>(term_a);
-    // LayerNorm parameters of this thread's owned column (thread = sequence x owned column at the
-    // end of the kernel): parameters, read before the dependency wait
+    float* rows_in = reinterpret_cast<float*>(hid_tile);
+    const int row_chunks = pairs_pad / 4, quads = (pairs + 3) >> 2;
+    // LayerNorm parameters of this thread's owned column (column = lane), read before the dependency wait
     const int own0 = static_cast<int>(rank) * kLtOwn;
     const float pre_g = a.norm_w[own0 + lane], pre_bt = a.norm_b[own0 + lane];
-    const float pre_nw = a.next_w[own0 + lane], pre_nb = a.next_b[own0 + lane];
-    const int row_chunks = pairs_pad / 4;                      // 16-byte chunks per row of partial sums: 4, 8 or 16
-    const float pre_bias = tid < kLtOwn * row_chunks ? load_scalar(a.second_bias, own0 + tid / row_chunks, dtype) : 0.0f;
+    const float pre_bias = load_scalar(a.second_bias, own0 + lane, dtype);
+    // warps that share a sequence at the end: warp = part x nseq + sequence
+    const int my_seq = warp % nseq, part = warp / nseq, parts = (kLtThreads / 32) / nseq;
+    // ... and the parameters of the next LayerNorm for the 128-column chunks part, part + parts, ... of a row
+    float4 next_g[4], next_b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (part + i * parts < mtiles && part < parts) {
+            next_g[i] = *reinterpret_cast<const float4*>(a.next_w + 128 * (part + i * parts) + 4 * lane);
+            next_b[i] = *reinterpret_cast<const float4*>(a.next_b + 128 * (part + i * parts) + 4 * lane);
+        }
+    int tpo = 16;                                              // threads per projection output: 2 .. 16
+    while (tpo > 2 && (nseq * nq_own * tpo > kLtThreads || (D / 8) / tpo < 2)) tpo >>= 1;
+    const uint32_t wq_stride = static_cast<uint32_t>(D) * 2u + 16u * static_cast<uint32_t>(tpo);
+    unsigned char* wq_tile = base + plan.wq;
+    // this CTA's rows of the query-projection weight (rows padded by one 16-byte chunk per cooperating thread:
+    // conflict-free reads in the projection)
+    const auto request_wq = [&] {
+        const int w_chunks = D / 8;
+        for (int i = tid; i < nq_own * w_chunks; i += kLtThreads) {
+            const int j = i / w_chunks, c = i - j * w_chunks;
+            cp_async16(smem_u32(wq_tile) + j * wq_stride + 16 * c,
+                       static_cast<const char*>(a.query_weight) +
+                           (static_cast<size_t>(rank) * nq_own + j) * D * 2 + 16 * c);
+        }
+    };
 
     const uint32_t bar_wm = smem_u32(&bars[0]), bar_w2 = smem_u32(&bars[1]);
     const uint32_t bar_d1 = smem_u32(&bars[2]), bar_d2 = smem_u32(&bars[3]);
+    const uint32_t bar_part = smem_u32(&bars[4]), bar_stat = smem_u32(&bars[5]), bar_rows = smem_u32(&bars[6]);
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_wm) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
-        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&bars[i]), 1);
+        for (int i = 0; i < 7; ++i) mbar_init(smem_u32(&bars[i]), 1);
         fence_barrier_init();
+        mbar_expect_tx(bar_part, static_cast<uint32_t>(C * quads) * 512u);
+        mbar_expect_tx(bar_stat, static_cast<uint32_t>(C * pairs) * 8u);
+        mbar_expect_tx(bar_rows, static_cast<uint32_t>(nseq * D) * 4u);
         failed = 0;
         // the weight slices do not depend on earlier kernels: requested before the dependency wait
         mbar_expect_tx(bar_wm, static_cast<uint32_t>(kblocks) * kBM * 128u);
@@ -178,6 +254,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                      ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (!Stage::kActive && pairs_pad == 16) request_wq();       // a parameter: before the dependency wait
     if (Stage::kActive) {
         // the stage's results reach the other CTAs of the cluster through global memory, ordered by
         // the cluster barrier
@@ -186,9 +263,9 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     } else {
         griddep_sync();
     }
+    if (Stage::kActive && pairs_pad == 16) request_wq();        // its place was the stage's until here
     // the residual stream was written by the previous kernel: requested now, used at the very end
-    float pre_res = 0.0f;
-    if (warp < nseq) pre_res = a.residual[static_cast<size_t>(s0 + warp) * D + own0 + lane];
+    const float pre_res = a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane];
     const float pre_mix = *a.mix;
 
     // ---- gathers.  Four threads share a row to gather: they read its index themselves (one
@@ -303,44 +380,37 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     __syncwarp();
     if (!mbar_wait(bar_d1, 0)) failed = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    const int nq_own = a.query_weight ? a.n_query / C : 0;
-    int tpo = 16;                                              // threads per projection output: 2 .. 16
-    while (tpo > 2 && (nseq * nq_own * tpo > kLtThreads || (D / 8) / tpo < 2)) tpo >>= 1;
-    const uint32_t wq_stride = static_cast<uint32_t>(D) * 2u + 16u * static_cast<uint32_t>(tpo);
+    if (pairs_pad == 16) { __syncwarp(); lt_cluster_arrive(); }      // the W_m slice is consumed: its place may receive
     cp_async_wait_all();                                       // the expanded-cache terms have arrived
     __syncthreads();
 
     // ---- epilogue of the product GEMM: + expanded-cache terms, GELU, hidden slice as the K-major
-    // B tile of the second GEMM (row = pair, K = this CTA's hidden columns).  Warps 0-3 take the
-    // first half of the pair columns, warps 4-7 the second half (eight columns at a time).
-    const int half_cols = pairs_pad >> 1;                     // 8, 16 or 32 pair columns per warp half
+    // B tile of the second GEMM (row = pair, K = this CTA's hidden columns).  Warps 0-3 and 4-7 take
+    // every other four pair columns; the columns of pairs that do not exist stay unwritten (their
+    // results are never read).
     {
         const int hc = 32 * (warp & 3) + lane;                // hidden column == TMEM lane
-        const int col0 = half_cols * (warp >> 2);
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
         const unsigned char* ta = term_a + hc * 2;
         const unsigned char* tp = term_p + hc * 2;
         unsigned char* hrow = hid_tile + static_cast<uint32_t>(hc >> 6) * p_kblock + (hc & 7) * 2;
         const int hchunk = (hc >> 3) & 7;
-        for (int c = col0; c < col0 + half_cols; c += 8) {
-            uint32_t v[8];
-            tmem_ld8(tmem_base + lane_base + c, v);
-            float term[8];
+        for (int c = 4 * (warp >> 2); c < pairs; c += 8) {
+            uint32_t v[4];
+            lt_tmem_ld4(tmem_base + lane_base + c, v);
+            float term[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int pr = c + j;
-                term[j] = 0.0f;
-                if (pr < pairs)
-                    term[j] = lt_from16(*reinterpret_cast<const uint16_t*>(ta + pair_seq_s[pr] * kLtTermStride), dtype) +
-                              lt_from16(*reinterpret_cast<const uint16_t*>(tp + pr * kLtTermStride), dtype);
+            for (int j = 0; j < 4; ++j) {
+                const int pr = min(c + j, pairs - 1);
+                term[j] = lt_from16(*reinterpret_cast<const uint16_t*>(ta + pair_seq_s[pr] * kLtTermStride), dtype) +
+                          lt_from16(*reinterpret_cast<const uint16_t*>(tp + pr * kLtTermStride), dtype);
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
                 const int pr = c + j;
-                const float x = pr < pairs ? gelu_tc(__uint_as_float(v[j]) + term[j]) : 0.0f;
-                *reinterpret_cast<uint16_t*>(hrow + (pr >> 3) * 1024 + (pr & 7) * 128 + ((hchunk ^ (pr & 7)) << 4)) = lt_to16(x, dtype);
+                *reinterpret_cast<uint16_t*>(hrow + (pr >> 3) * 1024 + (pr & 7) * 128 + ((hchunk ^ (pr & 7)) << 4)) =
+                    lt_to16(gelu_tc(__uint_as_float(v[j]) + term[j]), dtype);
             }
         }
     }
@@ -369,175 +439,167 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         umma_commit(bar_d2);
     }
     __syncwarp();
-    // the W_m slice was consumed by the first GEMM: while the second one runs, its place takes this
-    // CTA's rows of the query-projection weight (rows padded by one 16-byte chunk per cooperating
-    // thread: conflict-free reads in the projection below)
-    if (nq_own > 0) {
-        const int w_chunks = D / 8;
-        for (int i = tid; i < nq_own * w_chunks; i += kLtThreads) {
-            const int j = i / w_chunks, c = i - j * w_chunks;
-            cp_async16(smem_u32(wm_tile) + j * wq_stride + 16 * c,
-                       static_cast<const char*>(a.query_weight) +
-                           (static_cast<size_t>(rank) * nq_own + j) * D * 2 + 16 * c);
-        }
-        cp_async_commit();
-    }
+    if (pairs_pad > 16) request_wq();                          // in the consumed W_m slice's place, while the GEMM runs
+    cp_async_commit();
     if (!mbar_wait(bar_d2, 0)) failed = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (pairs_pad > 16) { __syncwarp(); lt_cluster_arrive(); }      // the W_2 slice is consumed: its place may receive
+    lt_cluster_wait();                                         // every CTA's receiving place is free
 
-    // ---- dump the partial raw^T [d, pairs_pad] (fp32) over the consumed W_2 slice; 16-byte chunk
-    // j of row r sits at chunk j ^ (r mod chunks per row): conflict-free for writers and readers
-    const uint32_t part_row = static_cast<uint32_t>(pairs_pad) * 4u;
+    // ---- reduce-scatter: the 32 output rows that a warp reads from the tensor memory belong to one CTA, which
+    // receives them from every CTA of the cluster as [sender][four pairs][column][pair]: 512 contiguous bytes a store
+    // of the warp, and the receiver's barrier counts them in
+    unsigned char* recv = pairs_pad == 16 ? wm_tile : w2_tile;
     {
-        const int lr = 32 * (warp & 3) + lane;
-        const int col0 = half_cols * (warp >> 2);
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        for (int mt = 0; mt < mtiles; ++mt) {
-            const int r = mt * kBM + lr;
-            for (int c = col0; c < col0 + half_cols; c += 8) {
-                uint32_t v[8];
+        for (int mt = warp >> 2; mt < mtiles; mt += 2) {
+            const uint32_t owner = static_cast<uint32_t>(4 * mt + (warp & 3));
+            const uint32_t bar = lt_peer(bar_part, owner);
+            const uint32_t dst = lt_peer(smem_u32(recv), owner) + (rank * row_chunks * 32u + lane) * 16u;
+            for (int c = 0; c < pairs; c += 16) {              // the accumulator has 16, 32 or 64 columns
+                uint32_t v[8], w[8];
                 tmem_ld8(tmem_d2 + lane_base + static_cast<uint32_t>(mt * pairs_pad + c), v);
+                tmem_ld8(tmem_d2 + lane_base + static_cast<uint32_t>(mt * pairs_pad + c + 8), w);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int ch = ((c >> 2) + q) ^ (r & (row_chunks - 1));
-                    *reinterpret_cast<uint4*>(w2_tile + r * part_row + ch * 16) =
-                        make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                }
+                const uint32_t at = dst + static_cast<uint32_t>(c >> 2) * 512u;
+                lt_push16(at, bar, v[0], v[1], v[2], v[3]);
+                if (c + 4 < pairs) lt_push16(at + 512u, bar, v[4], v[5], v[6], v[7]);
+                if (c + 8 < pairs) lt_push16(at + 1024u, bar, w[0], w[1], w[2], w[3]);
+                if (c + 12 < pairs) lt_push16(at + 1536u, bar, w[4], w[5], w[6], w[7]);
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    lt_cluster_sync();                                         // (1) every CTA's partial is in its shared memory
+
+    // ---- a warp owns four pairs (32 columns, a lane each): partial sums in rank order, so that the result does not
+    // depend on timing, and (mean, M2) of the 32 columns, pushed to every CTA
+    if (!mbar_wait(bar_part, 0)) failed = 1;
+    float x[2][4];
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const int q = warp + 8 * it;
+        if (q >= quads) break;
+        const unsigned char* src = recv + (static_cast<uint32_t>(q) * 32u + lane) * 16u;
+        float4 v[16];
+#pragma unroll
+        for (int s = 0; s < 16; ++s)
+            v[s] = s < C ? *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(s * row_chunks) * 512u)
+                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int s = 0; s < 16; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
+        x[it][0] = acc.x + pre_bias; x[it][1] = acc.y + pre_bias; x[it][2] = acc.z + pre_bias; x[it][3] = acc.w + pre_bias;
+        const float mean = lt_fold4(x[it]) * (1.0f / kLtOwn);
+        float dv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float d = x[it][j] - __shfl_sync(0xffffffffu, mean, 8 * j);
+            dv[j] = d * d;
+        }
+        const float m2 = lt_fold4(dv);
+        const int pr = 4 * q + (lane >> 3);
+        if (pr < pairs) {
+            const uint32_t at = smem_u32(&stats_in[rank * pairs_pad + pr]);
+            for (uint32_t to = lane & 7; to < static_cast<uint32_t>(C); to += 8) lt_push8(lt_peer(at, to), lt_peer(bar_stat, to), mean, m2);
+        }
+    }
+
+    // ---- the pairs' statistics over the full width (equal counts: Chan's parallel variance), eight lanes a pair, and
+    // the normalised pairs [pair][kLtOwnStride] for the sequences' weighted sums
+    float* own_y = reinterpret_cast<float*>(p_tile);
+    if (!mbar_wait(bar_stat, 0)) failed = 1;
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+        const int q = warp + 8 * it;
+        if (q >= quads) break;
+        const int pr = min(4 * q + (lane >> 3), pairs - 1), from = lane & 7;
+        float2 st[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            st[i] = from + 8 * i < C ? stats_in[(from + 8 * i) * pairs_pad + pr] : make_float2(0.0f, 0.0f);
+        float msum = st[0].x + st[1].x;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
+        const float mean = msum / static_cast<float>(C);
+        float m2 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (from + 8 * i < C) { const float dm = st[i].x - mean; m2 += st[i].y + static_cast<float>(kLtOwn) * dm * dm; }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        const float rstd = rsqrtf(m2 / static_cast<float>(D) + a.eps);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float mj = __shfl_sync(0xffffffffu, mean, 8 * j), rj = __shfl_sync(0xffffffffu, rstd, 8 * j);
+            if (4 * q + j < pairs) own_y[(4 * q + j) * kLtOwnStride + lane] = fmaf((x[it][j] - mj) * rj, pre_g, pre_bt);
+        }
+    }
+    __syncthreads();
     // every warp has read its accumulators: the tensor memory goes back now, off the kernel's exit path
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
 
-    // ---- reduce-scatter: this CTA owns output rows [own0, own0 + 32); partial sums are pulled
-    // from the CTAs in rank order, so the result does not depend on timing
-    float* own_raw = reinterpret_cast<float*>(p_tile);        // [pair][kLtOwnStride]
-    {
-        const uint32_t part_base = smem_u32(w2_tile);
-        for (int i = tid; i < kLtOwn * row_chunks; i += kLtThreads) {
-            const int r = i / row_chunks, j = i - r * row_chunks;
-            const int row = own0 + r;
-            const uint32_t off = static_cast<uint32_t>(row) * part_row + static_cast<uint32_t>((j ^ (row & (row_chunks - 1))) * 16);
-            float4 v[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q)
-                v[q] = q < C ? lt_ld_peer16(lt_peer(part_base, static_cast<uint32_t>(q)) + off)
-                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) { acc.x += v[q].x; acc.y += v[q].y; acc.z += v[q].z; acc.w += v[q].w; }
-            const float bias = i == tid ? pre_bias : load_scalar(a.second_bias, row, dtype);
-            const int pr = 4 * j;
-            own_raw[(pr + 0) * kLtOwnStride + r] = acc.x + bias;
-            own_raw[(pr + 1) * kLtOwnStride + r] = acc.y + bias;
-            own_raw[(pr + 2) * kLtOwnStride + r] = acc.z + bias;
-            own_raw[(pr + 3) * kLtOwnStride + r] = acc.w + bias;
-        }
-    }
-    __syncthreads();
-
-    // ---- LayerNorm statistics of every pair over the full width: (mean, M2) of this CTA's 32
-    // columns, combined over the cluster (equal counts: Chan's parallel variance)
-    {
-        const int pr = tid >> 2, q = tid & 3;                  // four threads per pair, eight columns each
-        float x[8], sum = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            x[i] = pr < pairs ? own_raw[pr * kLtOwnStride + 8 * q + i] : 0.0f;
-            sum += x[i];
-        }
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const float mean = sum * (1.0f / kLtOwn);
-        float m2 = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { const float dv = x[i] - mean; m2 = fmaf(dv, dv, m2); }
-        m2 += __shfl_xor_sync(0xffffffffu, m2, 1);
-        m2 += __shfl_xor_sync(0xffffffffu, m2, 2);
-        // pushed to every CTA of the cluster (the four threads of a pair share the receivers), so that
-        // nobody waits for a remote load after the barrier
-        if (pr < pairs) {
-            const uint32_t at = smem_u32(&stats_in[rank * kLtMaxPairs + pr]);
-            for (int i = 0; i < (C >> 2); ++i) lt_st_peer8(lt_peer(at, static_cast<uint32_t>(q * (C >> 2) + i)), mean, m2);
-        }
-    }
-    lt_cluster_sync();                                         // (2) every CTA's pair statistics are written
-    {
-        // four lanes per pair, each reading the statistics of C / 4 CTAs (C = 4, 8 or 16)
-        const int pr = tid >> 2, q = tid & 3, per = C >> 2;
-        float2 st[4];
-        float msum = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            st[i] = make_float2(0.0f, 0.0f);
-            if (i < per && pr < pairs)
-                st[i] = stats_in[(q * per + i) * kLtMaxPairs + pr];
-            msum += st[i].x;
-        }
-        msum += __shfl_xor_sync(0xffffffffu, msum, 1);
-        msum += __shfl_xor_sync(0xffffffffu, msum, 2);
-        const float mean = msum / static_cast<float>(C);
-        float m2 = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (i < per) { const float dm = st[i].x - mean; m2 += st[i].y + static_cast<float>(kLtOwn) * dm * dm; }
-        m2 += __shfl_xor_sync(0xffffffffu, m2, 1);
-        m2 += __shfl_xor_sync(0xffffffffu, m2, 2);
-        if (q == 0 && pr < pairs) ln_s[pr] = make_float2(mean, rsqrtf(m2 / static_cast<float>(D) + a.eps));
-    }
-    __syncthreads();
-
-    // ---- context, residual update and the next LayerNorm: thread (sequence = warp, owned column = lane)
-    const int bl = warp, col = own0 + lane;
-    const bool live = bl < nseq && !bad_position;
-    float hval = 0.0f;
-    if (live) {
-        const float g = pre_g, bt = pre_bt;
+    // ---- context and residual update: column = lane; the warps of a sequence share out the CTAs that its updated
+    // columns are pushed to
+    if (part < parts) {
         float ctx = 0.0f;
         for (int k = 0; k < K; ++k) {
-            const float wk = weight_s[bl * K + k];
+            const float wk = weight_s[my_seq * K + k];
             if (wk == 0.0f) continue;                          // inactive slots contribute nothing
-            const float2 ms = ln_s[bl * K + k];
-            const float x = own_raw[(bl * K + k) * kLtOwnStride + lane];
-            ctx = fmaf(wk, fmaf((x - ms.x) * ms.y, g, bt), ctx);
+            ctx = fmaf(wk, own_y[(my_seq * K + k) * kLtOwnStride + lane], ctx);
         }
-        float* res = a.residual + static_cast<size_t>(s0 + bl) * D + col;
-        hval = fmaf(pre_mix, ctx, pre_res);
-        *res = hval;
+        const float hval = bad_position ? pre_res : fmaf(pre_mix, ctx, pre_res);
+        if (part == 0 && !bad_position) a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane] = hval;
+        const uint32_t at = smem_u32(&rows_in[my_seq * D + own0 + lane]);
+        for (uint32_t to = part; to < static_cast<uint32_t>(C); to += parts) lt_push4(lt_peer(at, to), lt_peer(bar_rows, to), hval);
     }
-    {
-        const float mean = warp_sum(hval) * (1.0f / kLtOwn);
-        const float dv = hval - mean;
-        const float m2 = warp_sum(dv * dv);
-        if (lane < C && bl < kLtMaxSeq)
-            lt_st_peer8(lt_peer(smem_u32(&stats2_in[rank * kLtMaxSeq + bl]), static_cast<uint32_t>(lane)), mean, m2);
-    }
-    lt_cluster_sync();                                         // (3) every CTA's residual statistics are written
-    {
-        float2 st = make_float2(0.0f, 0.0f);
-        if (lane < C && bl < nseq) st = stats2_in[lane * kLtMaxSeq + bl];
-        const float mean = warp_sum(st.x) / static_cast<float>(C);
-        const float dm = st.x - mean;
-        const float m2 = warp_sum(lane < C ? st.y + static_cast<float>(kLtOwn) * dm * dm : 0.0f);
-        const float rstd = rsqrtf(m2 / static_cast<float>(D) + a.next_eps);
-        if (live) {
-            const uint16_t nv = lt_to16(fmaf((hval - mean) * rstd, pre_nw, pre_nb), dtype);
-            static_cast<uint16_t*>(a.normalized)[static_cast<size_t>(s0 + bl) * D + col] = nv;
-            if (nq_own > 0) {
-                // the normalised rows go to every CTA of the cluster for its share of the projection
-                const uint32_t at = smem_u32(hid_tile) + static_cast<uint32_t>((bl * D + col) * 2);
-                for (int p = 0; p < C; ++p) lt_st_peer2(lt_peer(at, static_cast<uint32_t>(p)), nv);
-            }
-        }
-    }
+
+    // ---- the next LayerNorm, of whole rows in every CTA: the warps of a sequence share its 128-column chunks
     cp_async_wait_all();                                       // this thread's pieces of the W_q slice
-    lt_cluster_sync();                                         // (4) normalised rows everywhere; no remote access after this
+    if (!mbar_wait(bar_rows, 0)) failed = 1;
+    __syncwarp();
+    lt_cluster_arrive();                                       // nothing more is pushed to this CTA, nor by it
+    uint16_t* rows16 = reinterpret_cast<uint16_t*>(p_tile);    // [sequence][d]
+    if (part < parts) {
+        const float* row = rows_in + my_seq * D;
+        float4 h[4];
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            h[i] = i < mtiles ? *reinterpret_cast<const float4*>(row + 128 * i + 4 * lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            sum += (h[i].x + h[i].y) + (h[i].z + h[i].w);
+        }
+        const float mean = warp_sum(sum) / static_cast<float>(D);
+        float sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < mtiles) {
+                h[i].x -= mean; h[i].y -= mean; h[i].z -= mean; h[i].w -= mean;
+                sq = fmaf(h[i].x, h[i].x, sq); sq = fmaf(h[i].y, h[i].y, sq);
+                sq = fmaf(h[i].z, h[i].z, sq); sq = fmaf(h[i].w, h[i].w, sq);
+            }
+        const float rstd = rsqrtf(warp_sum(sq) / static_cast<float>(D) + a.next_eps);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int chunk = part + i * parts;
+            if (chunk >= mtiles) break;
+            float4 v = h[0];
+#pragma unroll
+            for (int k = 1; k < 4; ++k)
+                if (chunk == k) v = h[k];
+            const float4 g = next_g[i], b = next_b[i];
+            const uint2 out = make_uint2(
+                pack2(fmaf(v.x * rstd, g.x, b.x), fmaf(v.y * rstd, g.y, b.y), dtype),
+                pack2(fmaf(v.z * rstd, g.z, b.z), fmaf(v.w * rstd, g.w, b.w), dtype));
+            const int at = 128 * chunk + 4 * lane;
+            *reinterpret_cast<uint2*>(rows16 + my_seq * D + at) = out;
+            if (at / kLtOwn == static_cast<int>(rank) && !bad_position)
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.normalized) + static_cast<size_t>(s0 + my_seq) * D + at) = out;
+        }
+    }
+    __syncthreads();
 
     // ---- this CTA's share of the next query projection: outputs [rank * nq_own, + nq_own) of every
     // sequence, two threads per (sequence, output), fp32 accumulation
@@ -548,8 +610,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             const int o = o0 + tid / tpo;
             const bool in = o < n_out;
             const int b = in ? o / nq_own : 0, j = in ? o - b * nq_own : 0;
-            const unsigned char* wrow = wm_tile + j * wq_stride;
-            const unsigned char* xrow = hid_tile + (b * D) * 2;
+            const unsigned char* wrow = wq_tile + j * wq_stride;
+            const unsigned char* xrow = p_tile + (b * D) * 2;
             float acc0 = 0.0f, acc1 = 0.0f;
             for (int i = 0; i < my_chunks; i += 2) {
                 float wf[8], xf[8], wg[8], xg[8];
@@ -567,6 +629,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 static_cast<uint16_t*>(a.query)[static_cast<size_t>(s0 + b) * a.n_query + rank * nq_own + j] = lt_to16(acc, dtype);
         }
     }
+    __syncwarp();
+    lt_cluster_wait();                                         // no CTA leaves while another may still push to it
     if (tid == 0 && a.status) {
         if (*reinterpret_cast<volatile int*>(&failed)) atomicOr(a.status, RLM_DEV_TIMEOUT);
         if (bad_position) atomicOr(a.status, RLM_DEV_POSITION);
@@ -593,7 +657,7 @@ int lt_validate(const LayerTailArgs& a) {
         set_error("relation_layer_tail: query projection width must be a multiple of 16 outputs per CTA (H / 128 CTAs), at most 64 each");
         return RLM_ERR_UNSUPPORTED;
     }
-    if (lt_plan(a.rdim, a.d, kLtMaxPairs).total + 1024 > static_cast<uint32_t>(kSmemDynamicLimit)) {
+    if (lt_smem_bytes(a.rdim, a.d, a.query_weight ? a.n_query / cluster : 0) > static_cast<uint32_t>(kSmemDynamicLimit)) {
         set_error("relation_layer_tail: the weight slices exceed 227 KB of shared memory");
         return RLM_ERR_SMEM;
     }
