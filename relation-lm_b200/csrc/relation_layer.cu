@@ -15,7 +15,7 @@ namespace {
 // shared memory the tail uses from its gathers on (product tile, hidden tile, term rows), while the
 // weight slices stream in.  The indices travel through global memory (they are outputs anyway) and
 // the cluster barrier.
-template <bool kBf16>
+template <int kDt>
 struct SelectInFront {
     static constexpr bool kActive = true;
     const SelectArgs* args;
@@ -23,7 +23,7 @@ struct SelectInFront {
     __device__ __forceinline__ bool operator()(unsigned char* scratch, uint32_t rank, int s0, int nseq) const {
         if (static_cast<int>(rank) >= nseq) return false;
         // the selector waits for the previous launch itself, as late as its queries allow
-        select_row<kBf16, true, false>(*args, s0 + static_cast<int>(rank), scratch, bars);
+        select_row<kDt, true, false>(*args, s0 + static_cast<int>(rank), scratch, bars);
         return true;
     }
 };
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) relation_layer_kernel(
     const LayerTailArgs tail, const SelectArgs sel) {
     extern __shared__ __align__(1024) unsigned char layer_smem_raw[];
     __shared__ __align__(8) unsigned long long select_bars[4];
-    layer_tail_body<kBf16>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16>{&sel, smem_u32(select_bars)});
+    layer_tail_body<kBf16>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16 ? RLM_BF16 : RLM_F16>{&sel, smem_u32(select_bars)});
 }
 
 int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weight, const void* second_weight,

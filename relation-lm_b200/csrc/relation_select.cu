@@ -19,13 +19,11 @@ namespace rlm {
 namespace {
 
 // kMinCtas = 3: the latency-oriented build (decode batches: one wave or less).  kMinCtas = 4:
-// launches of many rows, where rows in flight per SM set the throughput.  kBf16: queries, key
-// caches and block statistics are all bf16 (the decode configuration); the dtype branches
-// fold away, which matters because a row's time is largely instruction fetch.
-template <int kMinCtas, bool kBf16, bool kDecode, bool kResident = false>
+// launches of many rows, where rows in flight per SM set the throughput.
+template <int kMinCtas, int kDt, bool kDecode>
 __global__ void __launch_bounds__(kThreads, kMinCtas) relation_select_kernel(const SelectArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    select_row<kBf16, kDecode, false, kResident>(a, blockIdx.x, smem, smem_u32(smem + a.plan.bars));
+    select_row<kDt, kDecode, false>(a, blockIdx.x, smem, smem_u32(smem + a.plan.bars));
 }
 
 // ---- routed multi-anchor selection: S anchor slots per query row, one launch
@@ -55,7 +53,7 @@ __device__ __forceinline__ const void* slot_ptr(const void* p, size_t bytes) {
     return static_cast<const char*>(p) + bytes;
 }
 
-template <bool kBf16>
+template <int kDt>
 __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(const MultiSelectArgs m) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long call_bars[4 * 2 * kMaxSlots];
@@ -91,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(cons
             a.exclude_count = s;
             a.out_anchor = out_idx - row;                    // [row] lands on (row, s)
             a.out_anchor_score = out_sc - row;
-            select_row<kBf16, false, true>(a, row, smem, smem_u32(&call_bars[4 * s]));
+            select_row<kDt, false, true>(a, row, smem, smem_u32(&call_bars[4 * s]));
         }
         __syncthreads();
         if (tid == 0) {                                      // the thread that stored the slot's result
@@ -125,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(cons
             a.exclude_count = S;
             a.out_partner = out_idx - static_cast<ptrdiff_t>(row) * K;
             a.out_partner_score = out_sc - static_cast<ptrdiff_t>(row) * K;
-            select_row<kBf16, false, true>(a, row, smem, smem_u32(&call_bars[4 * (S + s)]));
+            select_row<kDt, false, true>(a, row, smem, smem_u32(&call_bars[4 * (S + s)]));
         }
         __syncthreads();
         if (tid < K) {                                       // the threads that stored the slot's results
@@ -278,17 +276,19 @@ __device__ __forceinline__ void keep_best(bool valid, float score, int pos, uint
     }
 }
 
+// The passes first, first + step, ... of a score function are this warp's (all of them by default).
+
 // The local window, staged in shared memory: row r is position pos0 + r; rows below first_valid are none (and
 // not staged).  Scores go to cand[slot0 + r], or, without cand, into the running best.
 template <int kDt, bool kExcl = false>
 __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int n_rows, int first_valid, int pos0, int exclude,
                                                   const QueryChunk& q, float* cand, int slot0, uint32_t& best_key,
-                                                  int& best_pos, const ExclRegs* ex = nullptr) {
+                                                  int& best_pos, const ExclRegs* ex = nullptr, int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
     const unsigned char* mine = rows + 16 * chunk;
-    for (int base = 0; base < n_rows; base += 32) {
+    for (int base = 32 * first; base < n_rows; base += 32 * step) {
         float sc;
         if (base >= first_valid && base + 32 <= n_rows) {
             const unsigned char* src = mine + (base + rq) * static_cast<int>(kRow);
@@ -316,23 +316,24 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
 template <int kDt, bool kExcl = false>
 __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
                                                   int bs_shift, int exclude, const QueryChunk& q, float* cand, int slot0,
-                                                  uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr) {
+                                                  uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr,
+                                                  int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
     const unsigned char* mine = keys + 16 * chunk;
-    for (int base = 0; base < n_rows; base += 32) {
+    for (int base = 32 * first; base < n_rows; base += 32 * step) {
         const int r = base + 4 * chunk + rq;
         int pos;                                         // position of row r, or -1
         float sc;
         if (bs_shift >= 5) {
             // the pass lies in one picked block: rows 4 i + rq are 512 bytes apart
             const int rank = base >> bs_shift, o0 = base - (rank << bs_shift);
-            const int first = sel[3 * rank] * bs + o0, lim = sel[3 * rank + 2] - o0;
-            const unsigned char* src = mine + static_cast<size_t>(first + rq) * kRow;
+            const int start = sel[3 * rank] * bs + o0, lim = sel[3 * rank + 2] - o0;
+            const unsigned char* src = mine + static_cast<size_t>(start + rq) * kRow;
             // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
             sc = pass_score<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
-            pos = 4 * chunk + rq < lim ? first + 4 * chunk + rq : -1;
+            pos = 4 * chunk + rq < lim ? start + 4 * chunk + rq : -1;
         } else {
             auto row_pos = [&](int row) -> int {
                 if (row >= n_rows) return -1;
@@ -363,15 +364,16 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
 template <int kDt>
 __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, const unsigned char* stdv, int nb, int n_complete,
                                                   int bs, int t, int ls, int strict, int buckets, const QueryChunk& q,
-                                                  const float* sp4, const float* bias, float* out) {
+                                                  const float* sp4, const float* bias, float* out, int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
-    for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
+    if (first == 0)
+        for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
     QueryChunk qa;
 #pragma unroll
     for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
     const float sp = sp4[chunk >> 1];
     const bool x2 = lane & 2, x4 = lane & 4;
-    for (int base = 0; base < n_complete; base += 32) {
+    for (int base = 32 * first; base < n_complete; base += 32 * step) {
         float sums[8], md[4], sd[4];
         const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
         chunk_sums<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
@@ -508,6 +510,184 @@ __device__ __forceinline__ bool topk_filter(const float* cand, int cap4, int K, 
     return true;
 }
 
+// Exact top-K of up to 512 candidate slots by one warp.
+__device__ __forceinline__ void topk_warp(const float* cand, int cap4, int K, int L, int t, int bs, int bs_shift, const int* sel,
+                                          uint32_t* scratch, int32_t* out_pos, float* out_score) {
+    if (cap4 <= 128) {
+        if (!topk_filter<4>(cand, cap4, K, L, t, bs, bs_shift, sel, scratch, out_pos, out_score))
+            topk_tournament<4>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_score);
+    } else if (cap4 <= 256) {
+        if (!topk_filter<8>(cand, cap4, K, L, t, bs, bs_shift, sel, scratch, out_pos, out_score))
+            topk_tournament<8>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_score);
+    } else {
+        if (!topk_filter<16>(cand, cap4, K, L, t, bs, bs_shift, sel, scratch, out_pos, out_score))
+            topk_tournament<16>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_score);
+    }
+}
+
+// ---- the decode form in one 16-bit dtype: a query row by a CTA of eight warps
+//
+// A row's time is a chain of dependent phases, so what counts is their number and length, not their work.  Here a
+// phase is a pass of 32 rows or blocks by a warp (the primitives above: a handful of loads, 64 multiply-adds a lane, a
+// three-step butterfly): complete blocks and local window side by side, then every warp that has picked rows to score
+// ranks the block scores for itself (top rounds of two redux instructions) and scores its passes, all warps merge the
+// eight warps' bests, add the anchor's partner-query row and do the same for the partners, and the top K come from
+// one warp's threshold filter.  Six block-wide barriers; with the shared-memory scoring loops, the all-pairs ranking
+// and the tournament of select_row the same chain took ten.
+// kResident: both key caches of the sequence in shared memory (requested before the dependency wait), else the window
+// there and the picked rows from L2.
+template <int kDt, bool kResident>
+__global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_decode_kernel(const SelectArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint32_t best_key_s[2 * kWarps], short_list[64];
+    __shared__ int best_pos_s[2 * kWarps], sel_s[kWarps][3 * kDecodeTop];
+    __shared__ float softplus_s[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = blockIdx.x, buckets4 = 4 * a.buckets;
+    const Plan& p = a.plan;
+    const uint32_t bar_a = smem_u32(smem + p.bars), bar_p = bar_a + 8;
+    // The caches, statistics and the position were written before the previous kernel of the stream started, so
+    // everything up to the bulk-copy requests may run while that kernel (which makes the queries) is still executing.
+    const int t = static_cast<int>(*a.position);
+    const int nb = a.n_blocks, bs = a.block_size, L = a.local_window, top = a.top_blocks;
+    const int bs_shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
+    const int ls = max(t - L + 1, 0), first_local = ls - (t - L + 1), n_complete = min((t + 1) / bs, nb);
+    const size_t seq_keys = static_cast<size_t>(row) * a.max_t * kRow, seq_stats = static_cast<size_t>(row) * nb * kRow;
+    const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
+    const bool bad_position = t < 0 || t >= a.max_t;
+    if (tid == 0 && !bad_position) {
+        mbar_init(bar_a, 1);
+        mbar_init(bar_p, 1);
+        fence_barrier_init();
+        const uint32_t sbytes = top > 0 ? n_complete * kRow : 0u;
+        const uint32_t lbytes = (kResident ? t + 1 : t - ls + 1) * kRow;
+        const size_t loff = seq_keys + (kResident ? 0 : static_cast<size_t>(ls) * kRow);
+        const uint32_t ldst = kResident ? 0u : first_local * kRow;
+        const auto request = [&](const void* mean, const void* stdv, const void* keys, int mean_at, int std_at, int keys_at,
+                                 uint32_t bar) {
+            mbar_expect_tx(bar, 2 * sbytes + lbytes);
+            if (sbytes) {
+                bulk_g2s(smem_u32(smem + mean_at), static_cast<const char*>(mean) + seq_stats, sbytes, bar);
+                bulk_g2s(smem_u32(smem + std_at), static_cast<const char*>(stdv) + seq_stats, sbytes, bar);
+            }
+            bulk_g2s(smem_u32(smem + keys_at) + ldst, static_cast<const char*>(keys) + loff, lbytes, bar);
+        };
+        request(a.anchor_mean, a.anchor_std, a.anchor_keys, p.a_mean, p.a_std, p.a_local, bar_a);
+        request(a.partner_mean, a.partner_std, a.partner_keys, p.p_mean, p.p_std, p.p_local, bar_p);
+    }
+    float* queries = reinterpret_cast<float*>(smem + p.queries);                 // aq | arq | pq | prq
+    float* bias_a = reinterpret_cast<float*>(smem + p.params), *bias_p = bias_a + buckets4;
+    float* bscore = reinterpret_cast<float*>(smem + p.block_scores);
+    float* cand = reinterpret_cast<float*>(smem + p.cand);
+    for (int i = tid; i < buckets4; i += kThreads) {
+        bias_a[i] = load_scalar(a.anchor_bias, i, a.param_dtype);
+        bias_p[i] = load_scalar(a.partner_bias, i, a.param_dtype);
+    }
+    if (tid < cap4 - cap) cand[cap + tid] = kNegInf;             // padding slots never win a comparison
+    if (tid >= 32 && tid < 40)
+        softplus_s[tid - 32] = canon_log(__fadd_rn(1.0f, canon_exp(load_scalar(tid < 36 ? a.anchor_gamma : a.partner_gamma, tid & 3, a.param_dtype))));
+    griddep_sync();
+    if (bad_position) {
+        if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_POSITION);
+        return;
+    }
+    queries[tid] = tid < kD       ? load_scalar(a.anchor_query, row * a.aq_stride + tid, kDt)
+                   : tid < 2 * kD ? load_scalar(a.anchor_router_query, row * a.arq_stride + tid - kD, kDt)
+                                  : load_scalar(a.partner_base, row * a.pbase_stride + tid - 2 * kD, kDt);
+    __syncthreads();
+
+    // blocks and window side by side: up to half of the warps walk the passes of blocks
+    const int block_warps = top > 0 ? max(1, min((n_complete + 31) >> 5, kWarps / 2)) : 0;
+    const int picked_rows = top * bs;
+    int* sel = sel_s[warp];
+    // row r of a window is position t - L + 1 + r (only rows that are staged are read)
+    const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(kRow) : 0;
+    const auto pick = [&] {
+        if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
+        else pick_blocks(bscore, nb, top, bs, ls, sel);
+    };
+    bool ok = mbar_wait(bar_a, 0);
+    {
+        QueryChunk q;
+        uint32_t bk = 0;
+        int bp = 0x7fffffff;
+        if (warp < block_warps) {
+            load_query_chunk(queries + kD, q);
+            score_blocks_warp<kDt>(smem + p.a_mean, smem + p.a_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                                   softplus_s, bias_a, bscore, warp, block_warps);
+            load_query_chunk(queries, q);
+        } else {
+            load_query_chunk(queries, q);
+            score_window_warp<kDt>(smem + p.a_local + window_offset, L, first_local, t - L + 1, -1, q, nullptr, 0, bk, bp,
+                                   nullptr, warp - block_warps, kWarps - block_warps);
+        }
+        if (lane == 0) { best_key_s[warp] = bk; best_pos_s[warp] = bp; }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
+            return;
+        }
+        bk = 0;
+        bp = 0x7fffffff;
+        if (32 * warp < picked_rows) {
+            pick();
+            score_remote_warp<kDt>(kResident ? smem + p.a_local : static_cast<const unsigned char*>(a.anchor_keys) + seq_keys,
+                                   picked_rows, sel, bs, bs_shift, -1, q, nullptr, 0, bk, bp, nullptr, warp, kWarps);
+        }
+        if (lane == 0) { best_key_s[kWarps + warp] = bk; best_pos_s[kWarps + warp] = bp; }
+    }
+    __syncthreads();
+    // highest score wins; equal scores go to the lowest position (the reference's left-most local arg-max followed by
+    // its "equal and earlier" merge rule)
+    uint32_t best_key = lane < 2 * kWarps ? best_key_s[lane] : 0u;
+    int anchor_pos = lane < 2 * kWarps ? best_pos_s[lane] : 0x7fffffff;
+    if (anchor_pos == 0x7fffffff) best_key = 0u;
+    warp_argmax_key(best_key, anchor_pos);
+    if (anchor_pos == 0x7fffffff) {       // no candidate
+        anchor_pos = 0;
+        best_key = float_key(kNegInf);
+    }
+    if (tid < 2 * kD)       // the anchor's contribution to the partner queries
+        queries[2 * kD + tid] = __fadd_rn(queries[2 * kD + tid],
+                                          load_scalar(a.partner_anchor_cache, (static_cast<size_t>(row) * a.max_t + anchor_pos) * 2 * kD + tid, kDt));
+    if (tid == kThreads - 1) {
+        a.out_anchor[row] = anchor_pos;
+        a.out_anchor_score[row] = key_float(best_key);
+    }
+    ok = mbar_wait(bar_p, 0);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
+        return;
+    }
+    {
+        QueryChunk q;
+        uint32_t bk = 0;
+        int bp = 0x7fffffff;
+        if (warp < block_warps) {
+            load_query_chunk(queries + 3 * kD, q);
+            score_blocks_warp<kDt>(smem + p.p_mean, smem + p.p_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                                   softplus_s + 4, bias_p, bscore, warp, block_warps);
+            load_query_chunk(queries + 2 * kD, q);
+        } else {
+            load_query_chunk(queries + 2 * kD, q);
+            score_window_warp<kDt>(smem + p.p_local + window_offset, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp,
+                                   nullptr, warp - block_warps, kWarps - block_warps);
+        }
+        __syncthreads();
+        if (32 * warp < picked_rows) {
+            pick();
+            score_remote_warp<kDt>(kResident ? smem + p.p_local : static_cast<const unsigned char*>(a.partner_keys) + seq_keys,
+                                   picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr, warp, kWarps);
+        }
+    }
+    __syncthreads();
+    // Exact top-K of the candidate table: output slot k holds the k-th best candidate (higher score first, equal scores
+    // by the earlier slot); results without a finite score report -inf and the position of candidate slot 0.
+    int32_t* out_pos = a.out_partner + static_cast<size_t>(row) * a.k_out;
+    float* out_score = a.out_partner_score + static_cast<size_t>(row) * a.k_out;
+    if (cap4 > 512) topk_large(cand, cap, a.k_out, L, t, bs, sel_s[0], out_pos, out_score);
+    else if (warp == 0) topk_warp(cand, cap4, a.k_out, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);
+}
+
 struct TileArgs {
     SelectArgs base;          // packed mode; queries [n_seq * q_len, ...]; row = b * q_len + t
     int q_len;                // query positions 0 .. q_len - 1 of every sequence
@@ -630,16 +810,16 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             }
         } else {
             if (top > 0)
-                score_blocks_any<false>(st[0], st[1], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<kAnyDtype>(st[0], st[1], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         arq, sp_a, bias_a, bscore, 0, 1);
-            score_rows_split<false, 1>(local_a, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1, nullptr, 0, aq,
+            score_rows_split<kAnyDtype, 1>(local_a, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1, nullptr, 0, aq,
                                        nullptr, 0, 0, 1, bk, bp, 0u, ok);
             if (top > 0) {
                 __syncwarp();
                 pick_blocks(bscore, nb, top, bs, ls, sel);
                 uint32_t rk = 0;
                 int rp = 0x7fffffff;
-                score_rows_split<false, 1, true>(seq_a, key_dtype, top * bs, sel, bs, 0, 0, -1, nullptr, 0, aq, nullptr, 0,
+                score_rows_split<kAnyDtype, 1, true>(seq_a, key_dtype, top * bs, sel, bs, 0, 0, -1, nullptr, 0, aq, nullptr, 0,
                                                  0, 1, rk, rp, 0u, ok);
                 if (rp != 0x7fffffff && (rk > bk || bp == 0x7fffffff || (rk == bk && rp < bp))) { bk = rk; bp = rp; }
             }
@@ -678,30 +858,21 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             }
         } else {
             if (top > 0)
-                score_blocks_any<false>(st[2], st[3], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<kAnyDtype>(st[2], st[3], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         prq, sp_p, bias_p, bscore, 0, 1);
-            score_rows_split<false, 1>(local_p, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos, nullptr, 0,
+            score_rows_split<kAnyDtype, 1>(local_p, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos, nullptr, 0,
                                        pq, cand, 0, 0, 1, dk, dp, 0u, ok);
             if (top > 0) {
                 __syncwarp();
                 pick_blocks(bscore, nb, top, bs, ls, sel);
-                score_rows_split<false, 1, true>(seq_p, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, nullptr, 0, pq, cand,
+                score_rows_split<kAnyDtype, 1, true>(seq_p, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, nullptr, 0, pq, cand,
                                                  L, 0, 1, dk, dp, 0u, ok);
             }
         }
         __syncwarp();
         int32_t* out_pos = a.out_partner + static_cast<size_t>(row) * K;
         float* out_sc = a.out_partner_score + static_cast<size_t>(row) * K;
-        if (cap4 <= 128) {
-            if (!topk_filter<4>(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_sc))
-                topk_tournament<4>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_sc);
-        } else if (cap4 <= 256) {
-            if (!topk_filter<8>(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_sc))
-                topk_tournament<8>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_sc);
-        } else {
-            if (!topk_filter<16>(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_sc))
-                topk_tournament<16>(cand, cap4, K, L, t, bs, bs_shift, sel, out_pos, out_sc);
-        }
+        topk_warp(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_sc);
         __syncwarp();
     }
 }
@@ -1085,18 +1256,29 @@ int launch_tile(TileArgs& m, void* stream) {
     return check_launch("relation_select_tile_kernel");
 }
 
+// The decode form in one 16-bit dtype has the kernel of warp passes; launches of more rows than the SMs hold at once
+// (rows in flight count there, not a row's chain) and the other forms take a select_row build.
+template <int kDt>
+auto select_kernel(bool many_rows, bool decode, bool passes, bool resident) {
+    return resident ? relation_select_decode_kernel<kDt, true>
+           : passes && !many_rows ? relation_select_decode_kernel<kDt, false>
+           : many_rows ? (decode ? relation_select_kernel<4, kDt, true> : relation_select_kernel<4, kDt, false>)
+                       : relation_select_kernel<3, kDt, false>;
+}
+
 int launch(SelectArgs& a, void* stream) {
     if (a.n_rows == 0) return RLM_OK;
     bool many_rows = false;
     const int ready = prepare(a, many_rows, true);
     if (ready != RLM_OK) return ready;
     const Plan& plan = a.plan;
-    const bool bf16 = a.query_dtype == RLM_BF16 && a.key_dtype == RLM_BF16 && a.stats_dtype == RLM_BF16;
-    const bool decode = bf16 && a.mode == kPacked && !a.row_batch && !a.row_position && !a.exclude_list;
-    auto kernel = a.resident ? relation_select_kernel<1, true, true, true> : many_rows ? (decode ? relation_select_kernel<4, true, true>
-                                      : bf16 ? relation_select_kernel<4, true, false> : relation_select_kernel<4, false, false>)
-                            : (decode ? relation_select_kernel<3, true, true>
-                                      : bf16 ? relation_select_kernel<3, true, false> : relation_select_kernel<3, false, false>);
+    const int dtype = a.key_dtype == a.query_dtype && a.stats_dtype == a.query_dtype ? a.query_dtype : kAnyDtype;
+    const bool decode = a.mode == kPacked && !a.row_batch && !a.row_position && !a.exclude_list;
+    const bool passes = decode && a.top_blocks <= kDecodeTop && plan.total <= kSmemDynamicLimit - kDecodeStatic;
+    auto kernel = dtype == RLM_BF16 ? select_kernel<RLM_BF16>(many_rows, decode, passes, a.resident)
+                  : dtype == RLM_F16 ? select_kernel<RLM_F16>(many_rows, decode, passes, a.resident)
+                  : dtype == RLM_F32 && decode ? (many_rows ? relation_select_kernel<4, RLM_F32, true> : relation_select_kernel<3, RLM_F32, true>)
+                                               : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     launch_kernel(kernel, dim3(a.n_rows), dim3(kThreads), plan.total, stream, a);
@@ -1150,8 +1332,9 @@ int launch_multi(MultiSelectArgs& m, void* stream) {
         set_error("relation_select_multi_rows: a query row stride is shorter than the slots it holds");
         return RLM_ERR_SHAPE;
     }
-    const bool bf16 = a.query_dtype == RLM_BF16 && a.key_dtype == RLM_BF16 && a.stats_dtype == RLM_BF16;
-    auto kernel = bf16 ? relation_select_multi_kernel<true> : relation_select_multi_kernel<false>;
+    const int dtype = a.key_dtype == a.query_dtype && a.stats_dtype == a.query_dtype ? a.query_dtype : kAnyDtype;
+    auto kernel = dtype == RLM_BF16 ? relation_select_multi_kernel<RLM_BF16>
+                  : dtype == RLM_F16 ? relation_select_multi_kernel<RLM_F16> : relation_select_multi_kernel<kAnyDtype>;
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     launch_kernel(kernel, dim3(a.n_rows), dim3(kThreads), total, stream, m);

@@ -14,6 +14,12 @@ namespace {
 
 
 constexpr int kThreads = 256;
+// Template argument kDt of the functions below: the one dtype of queries, key caches and block statistics, known at
+// compile time (the dtype branches fold away, which matters because a row's time is largely instruction fetch), or
+// kAnyDtype: run-time dtypes, each its own.
+constexpr int kAnyDtype = -1;
+constexpr int kDecodeTop = 32;        // picked blocks that relation_select_decode_kernel takes at most
+constexpr int kDecodeStatic = 6144;   // static shared memory kept free for it
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxKOut = 32;  // partner slots per query
 constexpr int kMaxExclude = 8; // extra excluded positions per query (multi-anchor selection)
@@ -69,7 +75,7 @@ struct SelectArgs {
     int mode;
     int shared_streams;                  // the partner's staging buffers alias the anchor's (see make_plan)
     int sm_count;                        // streaming multiprocessors of the device the launch goes to
-    int resident;                        // decode form with the whole key caches staged (see select_row)
+    int resident;                        // decode form with the whole key caches staged (relation_select_decode_kernel)
     Plan plan;
 };
 
@@ -144,7 +150,7 @@ __device__ __forceinline__ float chunk_dot(const unsigned char* row, const float
 // (score, lowest position on ties) is folded into (best_key, best_pos), identical in all lanes.
 // kAtPosition: `rows` is the sequence's whole key cache and a candidate row is read where it lies
 // (row = its position), straight from global memory / L2, instead of from a staged copy.
-template <bool kBf16, int kLpr, bool kAtPosition = false>
+template <int kDt, int kLpr, bool kAtPosition = false>
 __device__ __noinline__ void score_rows_split(const unsigned char* rows, int key_dtype_arg, int n_rows,
                                               const int* sel, int bs, int first_valid, int pos0,
                                               int exclude, const int* excl, int n_excl, const float* query,
@@ -153,7 +159,7 @@ __device__ __noinline__ void score_rows_split(const unsigned char* rows, int key
     constexpr int kRows = 32 / kLpr;                 // rows per warp pass
     const int lane = threadIdx.x & 31;
     const int sub = lane & (kLpr - 1), rl = lane / kLpr;
-    const int key_dtype = kBf16 ? RLM_BF16 : key_dtype_arg;
+    const int key_dtype = kDt >= 0 ? kDt : key_dtype_arg;
     const int row_bytes = kD * (key_dtype == RLM_F32 ? 4 : 2);
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
@@ -226,7 +232,7 @@ __device__ __noinline__ void score_rows_split(const unsigned char* rows, int key
 
 // Picks the split that keeps every lane of the group busy in the fewest passes (launches of at
 // most one CTA per SM, where a row's latency is what counts).
-template <bool kBf16, bool kAtPosition = false>
+template <int kDt>
 __device__ __forceinline__ void score_rows(const unsigned char* rows, int key_dtype, int n_rows,
                                            const int* sel, int bs, int first_valid, int pos0,
                                            int exclude, const int* excl, int n_excl, const float* query,
@@ -234,26 +240,26 @@ __device__ __forceinline__ void score_rows(const unsigned char* rows, int key_dt
                                            int& best_pos, uint32_t bar, bool& arrived, int sm_count_arg) {
     const int lanes = static_cast<int>(gridDim.x) <= sm_count_arg ? 32 * nw : 0;   // a row per lane when CTAs share the SMs: fewer instructions in total
     if (4 * n_rows <= lanes)
-        score_rows_split<kBf16, 4, kAtPosition>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
+        score_rows_split<kDt, 4>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
                                    query, cand, slot0, wi, nw, best_key, best_pos, bar, arrived);
     else if (2 * n_rows <= lanes)
-        score_rows_split<kBf16, 2, kAtPosition>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
+        score_rows_split<kDt, 2>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
                                    query, cand, slot0, wi, nw, best_key, best_pos, bar, arrived);
     else
-        score_rows_split<kBf16, 1, kAtPosition>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
+        score_rows_split<kDt, 1>(rows, key_dtype, n_rows, sel, bs, first_valid, pos0, exclude, excl, n_excl,
                                    query, cand, slot0, wi, nw, best_key, best_pos, bar, arrived);
 }
 
 // Block scores of the first `n_complete` blocks with the `nw` warps of a group; the other
 // entries of `out` (up to the next multiple of four) are set to -inf.
-template <bool kBf16>
+template <int kDt>
 __device__ __noinline__ void score_blocks(const unsigned char* mean, const unsigned char* stdv,
                                           int stats_dtype_arg, int nb, int n_complete, int bs, int t,
                                           int ls, int strict, int buckets, const float* rq,
                                           const float* sp4, const float* bias, float* out, int wi, int nw) {
     const int lane = threadIdx.x & 31;
     const int j = lane & 7, sub = lane >> 3, head = j >> 1;
-    const int stats_dtype = kBf16 ? RLM_BF16 : stats_dtype_arg;
+    const int stats_dtype = kDt >= 0 ? kDt : stats_dtype_arg;
     const int row_bytes = kD * (stats_dtype == RLM_F32 ? 4 : 2);
     const float sp = sp4[head];
     float q[8], aq[8];
@@ -301,14 +307,14 @@ __device__ __noinline__ void score_blocks(const unsigned char* mean, const unsig
 // lanes of a quarter warp read eight different 16-byte chunk indices (rows are 128 or 256 bytes
 // apart in shared memory).  Every sum is one of the eight-lane form's sums with its operands
 // possibly swapped, so the scores are bit-identical.
-template <bool kBf16>
+template <int kDt>
 __device__ __noinline__ void score_blocks_head(const unsigned char* mean, const unsigned char* stdv,
                                                int stats_dtype_arg, int nb, int n_complete, int bs, int t,
                                                int ls, int strict, int buckets, const float* rq,
                                                const float* sp4, const float* bias, float* out, int wi, int nw) {
     const int lane = threadIdx.x & 31;
     const int head = lane & 3, bl = lane >> 2;
-    const int stats_dtype = kBf16 ? RLM_BF16 : stats_dtype_arg;
+    const int stats_dtype = kDt >= 0 ? kDt : stats_dtype_arg;
     const int row_bytes = kD * (stats_dtype == RLM_F32 ? 4 : 2);
     const int c0 = 2 * head + (bl & 1), c1 = c0 ^ 1;
     float q0[8], q1[8], a0[8], a1[8];
@@ -354,16 +360,16 @@ __device__ __noinline__ void score_blocks_head(const unsigned char* mean, const 
 }
 
 // Eight lanes per block up to 16 complete blocks (one pass of four warps), a head per lane beyond.
-template <bool kBf16>
+template <int kDt>
 __device__ __forceinline__ void score_blocks_any(const unsigned char* mean, const unsigned char* stdv,
                                                  int stats_dtype, int nb, int n_complete, int bs, int t,
                                                  int ls, int strict, int buckets, const float* rq,
                                                  const float* sp4, const float* bias, float* out, int wi, int nw) {
     if (n_complete > 16)
-        score_blocks_head<kBf16>(mean, stdv, stats_dtype, nb, n_complete, bs, t, ls, strict, buckets, rq, sp4,
+        score_blocks_head<kDt>(mean, stdv, stats_dtype, nb, n_complete, bs, t, ls, strict, buckets, rq, sp4,
                                  bias, out, wi, nw);
     else
-        score_blocks<kBf16>(mean, stdv, stats_dtype, nb, n_complete, bs, t, ls, strict, buckets, rq, sp4, bias,
+        score_blocks<kDt>(mean, stdv, stats_dtype, nb, n_complete, bs, t, ls, strict, buckets, rq, sp4, bias,
                             out, wi, nw);
 }
 
@@ -642,11 +648,7 @@ __device__ __forceinline__ void issue_remote(const unsigned char* keys, unsigned
 // kernel (one call per slot and phase): the caller has already ordered itself after earlier
 // kernels, hands in the four mbarriers of this call, and in partner-only mode the partner queries
 // are completed here with the anchor's row of the partner-anchor cache.
-// kResident (decode form): the sequence's whole key caches up to the position are requested at entry
-// in place of the local windows, so the remote blocks need no second round of copies once they
-// are picked — two dependent memory round trips fewer per row, for contexts whose caches fit the
-// shared memory (2 x T x 128 bytes at 16 bits).
-template <bool kBf16, bool kDecode, bool kMulti, bool kResident = false>
+template <int kDt, bool kDecode, bool kMulti>
 __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, unsigned char* smem,
                                            const uint32_t bars) {
     __shared__ uint32_t warp_key[2 * kWarps];
@@ -659,8 +661,8 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
     const int32_t* row_batch = kDecode ? nullptr : a.row_batch;
     const int32_t* row_position = kDecode ? nullptr : a.row_position;
     const int32_t* exclude_list = kDecode ? nullptr : a.exclude_list;
-    const int key_dtype = kBf16 ? RLM_BF16 : a.key_dtype, stats_dtype = kBf16 ? RLM_BF16 : a.stats_dtype,
-              query_dtype = kBf16 ? RLM_BF16 : a.query_dtype;
+    const int key_dtype = kDt >= 0 ? kDt : a.key_dtype, stats_dtype = kDt >= 0 ? kDt : a.stats_dtype,
+              query_dtype = kDt >= 0 ? kDt : a.query_dtype;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool do_anchor = mode != kPartnerOnly, do_partner = mode != kAnchorOnly;
     const int buckets4 = 4 * a.buckets;
@@ -711,9 +713,6 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
     const size_t seq_keys = static_cast<size_t>(b) * a.max_t * key_row;
     const size_t seq_stats = static_cast<size_t>(b) * nb * stat_row;
     const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
-    // resident form: row r of the window is position t - L + 1 + r of the resident cache (rows before
-    // position 0 are never valid, hence never read)
-    const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(key_row) : 0;
 
     if (tid == 0) {
         // the issuing thread initialises the barriers itself; the others first touch them
@@ -721,10 +720,9 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
         for (int i = 0; i < 4; ++i) mbar_init(bars + 8 * i, 1);
         fence_barrier_init();
         const uint32_t sbytes = top > 0 ? static_cast<uint32_t>(n_complete * stat_row) : 0u;
-        // resident form: positions 0 .. t at rows 0 .. t; otherwise the local window at its slots
-        const uint32_t lbytes = static_cast<uint32_t>((kResident ? t + 1 : n_local) * key_row);
-        const size_t loff = seq_keys + (kResident ? 0 : static_cast<size_t>(ls) * key_row);
-        const uint32_t ldst = kResident ? 0u : static_cast<uint32_t>(first_local * key_row);
+        const uint32_t lbytes = static_cast<uint32_t>(n_local * key_row);
+        const size_t loff = seq_keys + static_cast<size_t>(ls) * key_row;
+        const uint32_t ldst = static_cast<uint32_t>(first_local * key_row);
         if (do_anchor) {
             mbar_expect_tx(bar_a, 2 * sbytes + lbytes);
             if (sbytes) {
@@ -789,10 +787,10 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
         uint32_t bk = 0;
         int bp = 0x7fffffff;
         if (warp < block_warps)
-            score_blocks_any<kBf16>(smem + p.a_mean, smem + p.a_std, stats_dtype, nb, n_complete, bs, t, ls,
+            score_blocks_any<kDt>(smem + p.a_mean, smem + p.a_std, stats_dtype, nb, n_complete, bs, t, ls,
                                     a.strict_valid, a.buckets, arq, sp_a, bias_a, bscore, warp, block_warps);
         else
-            score_rows<kBf16>(smem + p.a_local + window_offset, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1,
+            score_rows<kDt>(smem + p.a_local, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1,
                        excl_s, n_excl, aq, nullptr, 0, row_wi, row_nw, bk, bp, 0u, ok, a.sm_count);
         if (lane == 0) { warp_key[warp] = bk; warp_pos[warp] = bp; }
         __syncthreads();
@@ -813,9 +811,7 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
         }
         if (top > 0) {
             if (warp == 0) {
-                if (kResident) {
-                    pick_blocks(bscore, nb, top, bs, ls, sel);
-                } else if (nb <= 128 && top <= 32) {
+                if (nb <= 128 && top <= 32) {
                     pick_and_issue(bscore, nb, top, bs, ls, sel, static_cast<const unsigned char*>(a.anchor_keys),
                                    smem + p.remote, key_row, seq_keys, bar_ra);
                 } else {
@@ -828,12 +824,9 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
             __syncthreads();
             bk = 0;
             bp = 0x7fffffff;
-            if (kResident)      // the picked blocks' rows are already here, at their positions
-                score_rows<kBf16, true>(smem + p.a_local, key_dtype, top * bs, sel, bs, 0, 0, -1, excl_s, n_excl, aq,
-                                        nullptr, 0, warp, kWarps, bk, bp, 0u, ok, a.sm_count);
-            else                // each warp works out its rows' positions first and only then waits for the copies
-                score_rows<kBf16>(smem + p.remote, key_dtype, top * bs, sel, bs, 0, 0, -1, excl_s, n_excl, aq,
-                           nullptr, 0, warp, kWarps, bk, bp, bar_ra, ok, a.sm_count);
+            // each warp works out its rows' positions first and only then waits for the copies
+            score_rows<kDt>(smem + p.remote, key_dtype, top * bs, sel, bs, 0, 0, -1, excl_s, n_excl, aq,
+                            nullptr, 0, warp, kWarps, bk, bp, bar_ra, ok, a.sm_count);
             if (lane == 0) { warp_key[kWarps + warp] = bk; warp_pos[kWarps + warp] = bp; }
             if (__syncthreads_or(!ok)) {
                 if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
@@ -882,17 +875,15 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
     uint32_t dk = 0;
     int dp = 0x7fffffff;
     if (warp < block_warps)
-        score_blocks_any<kBf16>(smem + p.p_mean, smem + p.p_std, stats_dtype, nb, n_complete, bs, t, ls,
+        score_blocks_any<kDt>(smem + p.p_mean, smem + p.p_std, stats_dtype, nb, n_complete, bs, t, ls,
                                 a.strict_valid, a.buckets, prq, sp_p, bias_p, bscore, warp, block_warps);
     else
-        score_rows<kBf16>(smem + p.p_local + window_offset, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos,
+        score_rows<kDt>(smem + p.p_local, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos,
                    excl_s, n_excl, pq, cand, 0, row_wi, row_nw, dk, dp, 0u, okp, a.sm_count);
     __syncthreads();
     if (top > 0) {
         if (warp == 0) {
-            if (kResident) {
-                pick_blocks(bscore, nb, top, bs, ls, sel);
-            } else if (nb <= 128 && top <= 32) {
+            if (nb <= 128 && top <= 32) {
                 pick_and_issue(bscore, nb, top, bs, ls, sel, static_cast<const unsigned char*>(a.partner_keys),
                                smem + p.remote, key_row, seq_keys, bar_rp);
             } else {
@@ -906,12 +897,8 @@ __device__ __forceinline__ void select_row(const SelectArgs& a, const int row, u
         }
         __syncthreads();
         bool ok = true;
-        if (kResident)
-            score_rows<kBf16, true>(smem + p.p_local, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, excl_s, n_excl, pq,
-                                    cand, L, warp, kWarps, dk, dp, 0u, ok, a.sm_count);
-        else
-            score_rows<kBf16>(smem + p.remote, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, excl_s, n_excl, pq,
-                       cand, L, warp, kWarps, dk, dp, bar_rp, ok, a.sm_count);
+        score_rows<kDt>(smem + p.remote, key_dtype, top * bs, sel, bs, 0, 0, anchor_pos, excl_s, n_excl, pq,
+                        cand, L, warp, kWarps, dk, dp, bar_rp, ok, a.sm_count);
         if (__syncthreads_or(!ok)) {
             if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
             return;
@@ -997,15 +984,15 @@ int prepare(SelectArgs& a, bool& many_rows, bool allow_resident = false) {
         a.plan = make_plan(a.n_blocks, a.block_size, a.local_window, a.top_blocks, a.buckets,
                            dtype_size(a.key_dtype), dtype_size(a.stats_dtype), a.mode, true);
     }
-    // At most one row per SM, 16-bit bf16 decode form, caches that fit: stage the whole key caches
-    // (see select_row, kResident)
+    // At most one row per SM, decode form in one 16-bit dtype, caches that fit: stage the whole key caches
+    // (relation_select_decode_kernel)
     a.resident = 0;
     if (allow_resident && !many_rows && a.n_rows <= kSms && a.mode == kPacked && !a.row_batch && !a.row_position &&
-        !a.exclude_list && a.top_blocks > 0 && a.query_dtype == RLM_BF16 && a.key_dtype == RLM_BF16 &&
-        a.stats_dtype == RLM_BF16) {
+        !a.exclude_list && a.top_blocks > 0 && a.top_blocks <= kDecodeTop && a.query_dtype != RLM_F32 && a.key_dtype == a.query_dtype &&
+        a.stats_dtype == a.query_dtype) {
         const Plan whole = make_plan(a.n_blocks, a.block_size, a.local_window, a.top_blocks, a.buckets,
                                      dtype_size(a.key_dtype), dtype_size(a.stats_dtype), a.mode, false, a.max_t);
-        if (whole.total <= kSmemDynamicLimit - 4096) {
+        if (whole.total <= kSmemDynamicLimit - kDecodeStatic) {
             a.plan = whole;
             a.resident = 1;
         }

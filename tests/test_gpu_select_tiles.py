@@ -1,11 +1,12 @@
-"""Whole-sequence selectors at each tile size (one, two or four positions per warp, chosen by the number of
-tiles against the SMs) and 16-bit dtype, against the per-row kernels bit for bit."""
+"""The selectors of warp passes: whole-sequence forms at each tile size (one, two or four
+positions per warp, chosen by the number of tiles against the SMs) and the decode form, in either 16-bit dtype,
+against the per-row kernels bit for bit."""
 from __future__ import annotations
 
 import pytest
 import torch
 
-from gpu_util import assert_status_clear
+from gpu_util import assert_status_clear, position_tensor
 
 pytestmark = pytest.mark.gpu
 
@@ -63,4 +64,32 @@ def test_pass_shapes_of_the_tiled_selector(T, NB, L, top, strict):
     want = relation_select_packed_rows(*x, row_batch, row_pos, L, top, 8, strict)
     for mine, theirs in zip(got, want):
         assert torch.equal(mine.view(torch.int32), theirs.view(torch.int32))
+    assert_status_clear()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,NB,L,top,K,positions", [
+    (128, 8, 17, 2, 8, (0, 15, 16, 127)),            # resident caches, ragged window, no complete block at first
+    (2048, 32, 128, 2, 8, (63, 1000, 2047)),         # picked rows from L2
+    (600, 150, 40, 5, 4, (3, 300, 599)),             # more than 128 blocks, blocks of 4, passes of several blocks
+    (1024, 16, 400, 3, 8, (500, 1023)),              # more than 512 candidates: the block-wide top-K
+    (320, 5, 33, 0, 8, (0, 32, 319)),                # no remote blocks
+])
+def test_decode_form_equals_the_rows_form(T, NB, L, top, K, positions, dtype):
+    from relation_lm.kernels.relation_select import relation_select_packed, relation_select_packed_rows
+
+    B = 3
+    g = torch.Generator(device="cuda").manual_seed(T + L)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    stats = lambda: (r(B, NB, 4, 16).to(dtype), r(B, NB, 4, 16).abs().to(dtype), r(4), r(4, 16))  # noqa: E731
+    x = [r(B, 64).to(dtype), r(B, T, 64).to(dtype), r(B, 64).to(dtype), *stats(), r(B, 128).to(dtype),
+         r(B, T, 128).to(dtype), r(B, T, 64).to(dtype), *stats()]
+    x[1][:, 5] = x[1][:, 3]                          # equal keys: the lower position wins
+    x[9][:, 5] = x[9][:, 3]
+    row_batch = torch.arange(B, dtype=torch.int32, device="cuda")
+    for t in positions:
+        got = relation_select_packed(*x, position_tensor(t), L, top, K, False)
+        want = relation_select_packed_rows(*x, row_batch, torch.full_like(row_batch, t), L, top, K, False)
+        for mine, theirs in zip(got, want):
+            assert torch.equal(mine.view(torch.int32), theirs.view(torch.int32)), t
     assert_status_clear()
