@@ -105,7 +105,9 @@ __device__ __forceinline__ uint32_t lt_peer(uint32_t local_addr, uint32_t rank) 
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
     return remote;
 }
-__device__ __forceinline__ void lt_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// Relaxed: no data travels with these barriers (a consumed tile's place is free; nothing more will be pushed), and a
+// release would wait a thousand cycles for the warp's earlier stores and copies.
+__device__ __forceinline__ void lt_cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void lt_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // Stores into another CTA's shared memory that count towards a barrier of that CTA (both addresses from lt_peer).
@@ -122,15 +124,59 @@ __device__ __forceinline__ void lt_push4(uint32_t addr, uint32_t bar, float x) {
                  ::"r"(addr), "r"(__float_as_uint(x)), "r"(bar) : "memory");
 }
 
-// Sum of a[j] over the warp, for j = lane / 8.
-__device__ __forceinline__ float lt_fold4(const float (&a)[4]) {
+// Mean and sum of squared deviations of x[j] over the warp's 32 lanes, for j = lane / 8: equal halves are merged level
+// by level (Chan's parallel variance), both values in the same five exchanges.
+__device__ __forceinline__ float2 lt_moments4(const float (&x)[4]) {
     const bool hi = threadIdx.x & 16, mid = threadIdx.x & 8;
-    const float b0 = (hi ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], 16);
-    const float b1 = (hi ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], 16);
-    float c = (mid ? b1 : b0) + __shfl_xor_sync(0xffffffffu, mid ? b0 : b1, 8);
-    c += __shfl_xor_sync(0xffffffffu, c, 4);
-    c += __shfl_xor_sync(0xffffffffu, c, 2);
-    return c + __shfl_xor_sync(0xffffffffu, c, 1);
+    float m[2], v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float mine = hi ? x[2 + j] : x[j], other = __shfl_xor_sync(0xffffffffu, hi ? x[j] : x[2 + j], 16), d = mine - other;
+        m[j] = 0.5f * (mine + other);
+        v[j] = 0.5f * d * d;
+    }
+    float mean = mid ? m[1] : m[0], m2 = mid ? v[1] : v[0], count = 2.0f;
+    float give_mean = mid ? m[0] : m[1], give_m2 = mid ? v[0] : v[1];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, give_mean, o), other2 = __shfl_xor_sync(0xffffffffu, give_m2, o);
+        const float d = mean - other;
+        m2 = fmaf(d * d, 0.5f * count, m2 + other2);
+        mean = 0.5f * (mean + other);
+        count += count;
+        give_mean = mean;
+        give_m2 = m2;
+    }
+    return make_float2(mean, m2);
+}
+
+// MMAs are issued by a whole warp, each instruction predicated on one elected lane: inside an `if (tid == 0)` every
+// descriptor is moved from vector to uniform registers one instruction at a time, 85 cycles an MMA where the operands
+// stream in 32.
+__device__ __forceinline__ bool lt_elect() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void lt_umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                        bool issue) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
+}
+__device__ __forceinline__ void lt_commit(uint32_t bar, bool issue) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "setp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n"
+        ::"r"(bar), "r"(static_cast<uint32_t>(issue)) : "memory");
 }
 
 __device__ __forceinline__ void lt_tmem_ld4(uint32_t addr, uint32_t (&v)[4]) {
@@ -273,14 +319,24 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // trip lies between the selector's indices and the first gather.  Partner operand rows go
     // straight into the swizzled product tile; copy group 0 = operand rows (needed by the
     // product GEMM), group 1 = this CTA's 128 columns of the two expanded-cache terms (needed by
-    // its epilogue).
+    // its epilogue).  Indices and scores are all requested before the first is used, and the
+    // anchors' rows are gathered by threads that a small batch's partner rows leave free.
     const size_t op_row = static_cast<size_t>(R) * 2, ex_row = static_cast<size_t>(H) * 4;
     const int entry = tid >> 2, quarter = tid & 3;
-    int my_pair_row = 0, my_anchor_row = 0;
+    const int a_entry = (tid - kLtThreads / 2) >> 2;          // sequence whose anchor this thread gathers
+    const bool gathers_anchor = tid >= kLtThreads / 2 && a_entry < nseq;
+    const int partner = entry < pairs ? a.partner_index[static_cast<size_t>(s0) * K + entry] : 0;
+    const int anchor = gathers_anchor ? a.anchor_index[s0 + a_entry] : 0;
+    // scores of sequence = warp, for the softmax weights below
+    const float* score_row = a.partner_scores + static_cast<size_t>(s0 + warp) * K;
+    const float score0 = warp < nseq && lane < K ? score_row[lane] : kNegInf;
+    const float score1 = warp < nseq && lane + 32 < K ? score_row[lane + 32] : kNegInf;
+    const int t = static_cast<int>(*a.position);
+    const bool bad_position = t < 0 || t >= a.max_t;          // the same in every CTA of the grid
+    const int my_pair_row = min(max(partner, 0), a.max_t - 1);      // empty slots carry a sentinel that may be negative
+    const int my_anchor_row = min(max(anchor, 0), a.max_t - 1);
     if (entry < pairs) {
         const int bl = entry / K;
-        const int p = a.partner_index[static_cast<size_t>(s0) * K + entry];
-        my_pair_row = min(max(p, 0), a.max_t - 1);            // empty slots carry a sentinel that may be negative
         if (quarter == 0) pair_seq_s[entry] = bl;
         const char* src = static_cast<const char*>(a.operand_cache) +
                           (static_cast<size_t>(s0 + bl) * a.max_t + my_pair_row) * op_row;
@@ -291,13 +347,11 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};"
                          ::"r"(smem_u32(p_tile) + swizzled(entry, c, p_kblock)), "r"(0) : "memory");
     }
-    if (entry < nseq) {
-        const int an = a.anchor_index[s0 + entry];
-        my_anchor_row = min(max(an, 0), a.max_t - 1);
+    if (gathers_anchor) {
         const char* src = static_cast<const char*>(a.operand_cache) +
-                          (static_cast<size_t>(s0 + entry) * a.max_t + my_anchor_row) * op_row;
+                          (static_cast<size_t>(s0 + a_entry) * a.max_t + my_anchor_row) * op_row;
         for (int c = quarter; c < chunks; c += 4)
-            cp_async16(smem_u32(op_a) + static_cast<uint32_t>(entry * R * 2 + 16 * c), src + 16 * c);
+            cp_async16(smem_u32(op_a) + static_cast<uint32_t>(a_entry * R * 2 + 16 * c), src + 16 * c);
     }
     cp_async_commit();
     if (entry < pairs) {
@@ -308,35 +362,28 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         for (int i = 0; i < 4; ++i)
             cp_async16(smem_u32(term_p) + entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
     }
-    if (entry < nseq) {
+    if (gathers_anchor) {
         const char* src = static_cast<const char*>(a.expanded_cache) +
-                          (static_cast<size_t>(s0 + entry) * a.max_t + my_anchor_row) * ex_row +
+                          (static_cast<size_t>(s0 + a_entry) * a.max_t + my_anchor_row) * ex_row +
                           static_cast<size_t>(h0) * 2;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            cp_async16(smem_u32(term_a) + entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
+            cp_async16(smem_u32(term_a) + a_entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
     }
     cp_async_commit();
-    // softmax weights over the active partner slots of every sequence (needed much later): a few
-    // threads of the last warp read the scores themselves while the gathers are in flight
-    const int t = static_cast<int>(*a.position);
-    const bool bad_position = t < 0 || t >= a.max_t;          // the same in every CTA of the grid
-    if (tid >= kLtThreads - kLtMaxSeq && tid - (kLtThreads - kLtMaxSeq) < nseq) {
-        const int b = tid - (kLtThreads - kLtMaxSeq);
-        const float* sc = a.partner_scores + static_cast<size_t>(s0 + b) * K;
+    // softmax weights over the active partner slots of a sequence (needed much later), by a warp while the gathers are
+    // in flight
+    if (warp < nseq) {
         int k_limit = 32 - __clz(max(t, 0) + 1);               // ceil(log2(t + 2))
         k_limit = min(max(k_limit, 1), K);
-        float mx = -1.0e4f;
-        for (int k = 0; k < K; ++k)
-            if (k < k_limit && sc[k] > -1.0e30f) mx = fmaxf(mx, sc[k]);
-        float den = 0.0f;
-        for (int k = 0; k < K; ++k) {
-            const float e = (k < k_limit && sc[k] > -1.0e30f) ? expf(sc[k] - mx) : 0.0f;
-            weight_s[b * K + k] = e;
-            den += e;
-        }
-        den = 1.0f / fmaxf(den, 1.0e-9f);
-        for (int k = 0; k < K; ++k) weight_s[b * K + k] *= den;
+        const bool live0 = lane < k_limit && score0 > -1.0e30f, live1 = lane + 32 < k_limit && score1 > -1.0e30f;
+        float mx = fmaxf(live0 ? score0 : -1.0e4f, live1 ? score1 : -1.0e4f);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float e0 = live0 ? expf(score0 - mx) : 0.0f, e1 = live1 ? expf(score1 - mx) : 0.0f;
+        const float scale = 1.0f / fmaxf(warp_sum(e0 + e1), 1.0e-9f);
+        if (lane < K) weight_s[warp * K + lane] = e0 * scale;
+        if (lane + 32 < K) weight_s[warp * K + lane + 32] = e1 * scale;
     }
     cp_async_wait_group1();                                    // the operand rows have arrived
     __syncthreads();
@@ -362,20 +409,18 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const uint32_t tmem_d2 = tmem_base + 64u;                 // second GEMM: mtiles x pairs_pad columns from column 64
 
     // ---- product GEMM: D1[hidden column, pair] = W_m slice x products^T
-    if (tid == 0) {
-        if (mbar_wait(bar_wm, 0)) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int kb = 0; kb < kblocks; ++kb) {
-                const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kBM * 128u);
-                const uint64_t dp = smem_desc_sw128(smem_u32(p_tile) + kb * p_kblock);
+    if (warp == 0) {
+        const bool ok = mbar_wait(bar_wm, 0), issue = lt_elect();
+        if (!ok) failed = 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = 0; kb < kblocks; ++kb) {
+            const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kBM * 128u);
+            const uint64_t dp = smem_desc_sw128(smem_u32(p_tile) + kb * p_kblock);
 #pragma unroll
-                for (int kk = 0; kk < kBK / 16; ++kk)
-                    umma_f16(tmem_base, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            }
-        } else {
-            failed = 1;
+            for (int kk = 0; kk < kBK / 16; ++kk)
+                lt_umma(tmem_base, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
         }
-        umma_commit(bar_d1);
+        lt_commit(bar_d1, issue);
     }
     __syncwarp();
     if (!mbar_wait(bar_d1, 0)) failed = 1;
@@ -421,22 +466,21 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     // ---- second GEMM, split over the cluster along the hidden width:
     // D2[output row, pair] (partial) = W_2[:, this CTA's hidden columns] x hidden slice^T
-    if (tid == 0) {
-        if (mbar_wait(bar_w2, 0)) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int mt = 0; mt < mtiles; ++mt)
-                for (int kb = 0; kb < 2; ++kb) {
-                    const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + (mt * 2 + kb) * kBM * 128u);
-                    const uint64_t dh = smem_desc_sw128(smem_u32(hid_tile) + kb * p_kblock);
+    if (warp == 0) {
+        const bool ok = mbar_wait(bar_w2, 0), issue = lt_elect();
+        if (!ok) failed = 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int mt = 0; mt < mtiles; ++mt)
 #pragma unroll
-                    for (int kk = 0; kk < kBK / 16; ++kk)
-                        umma_f16(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
-                                 (kb > 0 || kk > 0) ? 1u : 0u);
-                }
-        } else {
-            failed = 1;
-        }
-        umma_commit(bar_d2);
+            for (int kb = 0; kb < 2; ++kb) {
+                const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + (mt * 2 + kb) * kBM * 128u);
+                const uint64_t dh = smem_desc_sw128(smem_u32(hid_tile) + kb * p_kblock);
+#pragma unroll
+                for (int kk = 0; kk < kBK / 16; ++kk)
+                    lt_umma(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
+                            (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+            }
+        lt_commit(bar_d2, issue);
     }
     __syncwarp();
     if (pairs_pad > 16) request_wq();                          // in the consumed W_m slice's place, while the GEMM runs
@@ -489,18 +533,11 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 #pragma unroll
         for (int s = 0; s < 16; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
         x[it][0] = acc.x + pre_bias; x[it][1] = acc.y + pre_bias; x[it][2] = acc.z + pre_bias; x[it][3] = acc.w + pre_bias;
-        const float mean = lt_fold4(x[it]) * (1.0f / kLtOwn);
-        float dv[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float d = x[it][j] - __shfl_sync(0xffffffffu, mean, 8 * j);
-            dv[j] = d * d;
-        }
-        const float m2 = lt_fold4(dv);
+        const float2 moments = lt_moments4(x[it]);
         const int pr = 4 * q + (lane >> 3);
         if (pr < pairs) {
             const uint32_t at = smem_u32(&stats_in[rank * pairs_pad + pr]);
-            for (uint32_t to = lane & 7; to < static_cast<uint32_t>(C); to += 8) lt_push8(lt_peer(at, to), lt_peer(bar_stat, to), mean, m2);
+            for (uint32_t to = lane & 7; to < static_cast<uint32_t>(C); to += 8) lt_push8(lt_peer(at, to), lt_peer(bar_stat, to), moments.x, moments.y);
         }
     }
 
@@ -513,20 +550,26 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         const int q = warp + 8 * it;
         if (q >= quads) break;
         const int pr = min(4 * q + (lane >> 3), pairs - 1), from = lane & 7;
-        float2 st[2];
+        // sums of the means' distances from the first one, of their squares and of the M2, in the same three exchanges
+        const float pivot = stats_in[pr].x;
+        float d1 = 0.0f, d2 = 0.0f, m2 = 0.0f;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
-            st[i] = from + 8 * i < C ? stats_in[(from + 8 * i) * pairs_pad + pr] : make_float2(0.0f, 0.0f);
-        float msum = st[0].x + st[1].x;
+            if (from + 8 * i < C) {
+                const float2 st = stats_in[(from + 8 * i) * pairs_pad + pr];
+                const float d = st.x - pivot;
+                d1 += d;
+                d2 = fmaf(d, d, d2);
+                m2 += st.y;
+            }
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
-        const float mean = msum / static_cast<float>(C);
-        float m2 = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (from + 8 * i < C) { const float dm = st[i].x - mean; m2 += st[i].y + static_cast<float>(kLtOwn) * dm * dm; }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        for (int o = 4; o > 0; o >>= 1) {
+            d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+            d2 += __shfl_xor_sync(0xffffffffu, d2, o);
+            m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        }
+        const float per = 1.0f / static_cast<float>(C), mean = fmaf(d1, per, pivot);
+        m2 = fmaf(static_cast<float>(kLtOwn), fmaxf(fmaf(-d1 * per, d1, d2), 0.0f), m2);
         const float rstd = rsqrtf(m2 / static_cast<float>(D) + a.eps);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -545,10 +588,10 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // columns are pushed to
     if (part < parts) {
         float ctx = 0.0f;
+#pragma unroll 4
         for (int k = 0; k < K; ++k) {
-            const float wk = weight_s[my_seq * K + k];
-            if (wk == 0.0f) continue;                          // inactive slots contribute nothing
-            ctx = fmaf(wk, own_y[(my_seq * K + k) * kLtOwnStride + lane], ctx);
+            const float wk = weight_s[my_seq * K + k], y = own_y[(my_seq * K + k) * kLtOwnStride + lane];
+            ctx = wk == 0.0f ? ctx : fmaf(wk, y, ctx);         // inactive slots contribute nothing
         }
         const float hval = bad_position ? pre_res : fmaf(pre_mix, ctx, pre_res);
         if (part == 0 && !bad_position) a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane] = hval;
