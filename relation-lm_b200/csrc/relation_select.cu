@@ -279,8 +279,9 @@ __device__ __forceinline__ void keep_best(bool valid, float score, int pos, uint
 // The passes first, first + step, ... of a score function are this warp's (all of them by default).
 
 // The local window, staged in shared memory: row r is position pos0 + r; rows below first_valid are none (and
-// not staged).  Scores go to cand[slot0 + r], or, without cand, into the running best.
-template <int kDt, bool kExcl = false>
+// not staged).  Scores go to cand[slot0 + r], or, without cand, into the running
+// best (kBoth: to both).
+template <int kDt, bool kExcl = false, bool kBoth = false>
 __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int n_rows, int first_valid, int pos0, int exclude,
                                                   const QueryChunk& q, float* cand, int slot0, uint32_t& best_key,
                                                   int& best_pos, const ExclRegs* ex = nullptr, int first = 0, int step = 1) {
@@ -303,17 +304,15 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
         const int r = base + 4 * chunk + rq, pos = pos0 + r;
         const bool valid = r < n_rows && r >= first_valid && pos != exclude && not_excluded<kExcl>(pos, ex);
         sc = valid ? sc : kNegInf;
-        if (cand) {
+        if (kBoth || cand)
             if (r < n_rows) cand[slot0 + r] = sc;
-        } else {
-            keep_best(valid, sc, pos, my_key, my_pos);
-        }
+        if (kBoth || !cand) keep_best(valid, sc, pos, my_key, my_pos);
     }
-    if (!cand) fold_best(my_key, my_pos, best_key, best_pos);
+    if (kBoth || !cand) fold_best(my_key, my_pos, best_key, best_pos);
 }
 
 // The picked remote blocks (sel: block, picked, rows), scored where they lie in the key cache.
-template <int kDt, bool kExcl = false>
+template <int kDt, bool kExcl = false, bool kBoth = false>
 __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
                                                   int bs_shift, int exclude, const QueryChunk& q, float* cand, int slot0,
                                                   uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr,
@@ -348,13 +347,11 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
         }
         const bool valid = pos >= 0 && pos != exclude && not_excluded<kExcl>(pos, ex);
         sc = valid ? sc : kNegInf;
-        if (cand) {
+        if (kBoth || cand)
             if (r < n_rows) cand[slot0 + r] = sc;
-        } else {
-            keep_best(valid, sc, pos, my_key, my_pos);
-        }
+        if (kBoth || !cand) keep_best(valid, sc, pos, my_key, my_pos);
     }
-    if (!cand) fold_best(my_key, my_pos, best_key, best_pos);
+    if (kBoth || !cand) fold_best(my_key, my_pos, best_key, best_pos);
 }
 
 // score_blocks for one warp, 32 blocks a pass: chunks 2 h and 2 h + 1 of a block's statistics are head h, so the
@@ -531,16 +528,16 @@ __device__ __forceinline__ void topk_warp(const float* cand, int cap4, int K, in
 // phase is a pass of 32 rows or blocks by a warp (the primitives above: a handful of loads, 64 multiply-adds a lane, a
 // three-step butterfly): complete blocks and local window side by side, then every warp that has picked rows to score
 // ranks the block scores for itself (top rounds of two redux instructions) and scores its passes, all warps merge the
-// eight warps' bests, add the anchor's partner-query row and do the same for the partners, and the top K come from
-// one warp's threshold filter.  Six block-wide barriers; with the shared-memory scoring loops, the all-pairs ranking
-// and the tournament of select_row the same chain took ten.
+// eight warps' bests, add the anchor's partner-query row and do the same for the partners; the top K come from ranking
+// every candidate against all others by the whole CTA.  Half of a cold phase is instruction fetch (a pass of blocks
+// takes 2300 cycles where its arithmetic needs some 900), so both streams run through one copy of the code.
 // kResident: both key caches of the sequence in shared memory (requested before the dependency wait), else the window
 // there and the picked rows from L2.
 template <int kDt, bool kResident>
 __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_decode_kernel(const SelectArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ uint32_t best_key_s[2 * kWarps], short_list[64];
-    __shared__ int best_pos_s[2 * kWarps], sel_s[kWarps][3 * kDecodeTop];
+    __shared__ uint32_t best_key_s[kWarps], short_list[64];
+    __shared__ int best_pos_s[kWarps], sel_s[kWarps][3 * kDecodeTop];
     __shared__ float softplus_s[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.x, buckets4 = 4 * a.buckets;
@@ -602,90 +599,98 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     int* sel = sel_s[warp];
     // row r of a window is position t - L + 1 + r (only rows that are staged are read)
     const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(kRow) : 0;
-    const auto pick = [&] {
-        if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
-        else pick_blocks(bscore, nb, top, bs, ls, sel);
-    };
-    bool ok = mbar_wait(bar_a, 0);
-    {
+    int anchor_pos = -1;
+    // the anchor's stream, then the partner's: one copy of the code, so that the second finds it in the instruction cache
+#pragma unroll 1
+    for (int stream = 0; stream < 2; ++stream) {
+        const unsigned char* mean = smem + (stream ? p.p_mean : p.a_mean), *stdv = smem + (stream ? p.p_std : p.a_std);
+        const unsigned char* staged = smem + (stream ? p.p_local : p.a_local);
+        const unsigned char* keys = static_cast<const unsigned char*>(stream ? a.partner_keys : a.anchor_keys) + seq_keys;
+        const float* query = queries + 2 * kD * stream;            // exact query | router query
+        const bool ok = mbar_wait(stream ? bar_p : bar_a, 0);
         QueryChunk q;
         uint32_t bk = 0;
         int bp = 0x7fffffff;
         if (warp < block_warps) {
-            load_query_chunk(queries + kD, q);
-            score_blocks_warp<kDt>(smem + p.a_mean, smem + p.a_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
-                                   softplus_s, bias_a, bscore, warp, block_warps);
-            load_query_chunk(queries, q);
+            load_query_chunk(query + kD, q);
+            score_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, softplus_s + 4 * stream,
+                                   stream ? bias_p : bias_a, bscore, warp, block_warps);
         } else {
-            load_query_chunk(queries, q);
-            score_window_warp<kDt>(smem + p.a_local + window_offset, L, first_local, t - L + 1, -1, q, nullptr, 0, bk, bp,
-                                   nullptr, warp - block_warps, kWarps - block_warps);
+            load_query_chunk(query, q);
+            score_window_warp<kDt, false, true>(staged + window_offset, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp,
+                                                nullptr, warp - block_warps, kWarps - block_warps);
         }
-        if (lane == 0) { best_key_s[warp] = bk; best_pos_s[warp] = bp; }
         if (__syncthreads_or(!ok)) {
             if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
             return;
         }
-        bk = 0;
-        bp = 0x7fffffff;
         if (32 * warp < picked_rows) {
-            pick();
-            score_remote_warp<kDt>(kResident ? smem + p.a_local : static_cast<const unsigned char*>(a.anchor_keys) + seq_keys,
-                                   picked_rows, sel, bs, bs_shift, -1, q, nullptr, 0, bk, bp, nullptr, warp, kWarps);
+            load_query_chunk(query, q);
+            if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
+            else pick_blocks(bscore, nb, top, bs, ls, sel);
+            score_remote_warp<kDt, false, true>(kResident ? staged : keys, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L,
+                                                bk, bp, nullptr, warp, kWarps);
         }
-        if (lane == 0) { best_key_s[kWarps + warp] = bk; best_pos_s[kWarps + warp] = bp; }
-    }
-    __syncthreads();
-    // highest score wins; equal scores go to the lowest position (the reference's left-most local arg-max followed by
-    // its "equal and earlier" merge rule)
-    uint32_t best_key = lane < 2 * kWarps ? best_key_s[lane] : 0u;
-    int anchor_pos = lane < 2 * kWarps ? best_pos_s[lane] : 0x7fffffff;
-    if (anchor_pos == 0x7fffffff) best_key = 0u;
-    warp_argmax_key(best_key, anchor_pos);
-    if (anchor_pos == 0x7fffffff) {       // no candidate
-        anchor_pos = 0;
-        best_key = float_key(kNegInf);
-    }
-    if (tid < 2 * kD)       // the anchor's contribution to the partner queries
-        queries[2 * kD + tid] = __fadd_rn(queries[2 * kD + tid],
-                                          load_scalar(a.partner_anchor_cache, (static_cast<size_t>(row) * a.max_t + anchor_pos) * 2 * kD + tid, kDt));
-    if (tid == kThreads - 1) {
-        a.out_anchor[row] = anchor_pos;
-        a.out_anchor_score[row] = key_float(best_key);
-    }
-    ok = mbar_wait(bar_p, 0);
-    if (__syncthreads_or(!ok)) {
-        if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
-        return;
-    }
-    {
-        QueryChunk q;
-        uint32_t bk = 0;
-        int bp = 0x7fffffff;
-        if (warp < block_warps) {
-            load_query_chunk(queries + 3 * kD, q);
-            score_blocks_warp<kDt>(smem + p.p_mean, smem + p.p_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
-                                   softplus_s + 4, bias_p, bscore, warp, block_warps);
-            load_query_chunk(queries + 2 * kD, q);
-        } else {
-            load_query_chunk(queries + 2 * kD, q);
-            score_window_warp<kDt>(smem + p.p_local + window_offset, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp,
-                                   nullptr, warp - block_warps, kWarps - block_warps);
+        if (lane == 0) { best_key_s[warp] = bk; best_pos_s[warp] = bp; }
+        __syncthreads();
+        if (stream) break;
+        // highest score wins; equal scores go to the lowest position (the reference's left-most local arg-max followed
+        // by its "equal and earlier" merge rule)
+        uint32_t best_key = lane < kWarps ? best_key_s[lane] : 0u;
+        anchor_pos = lane < kWarps ? best_pos_s[lane] : 0x7fffffff;
+        if (anchor_pos == 0x7fffffff) best_key = 0u;
+        warp_argmax_key(best_key, anchor_pos);
+        if (anchor_pos == 0x7fffffff) {   // no candidate
+            anchor_pos = 0;
+            best_key = float_key(kNegInf);
+        }
+        if (tid < 2 * kD)       // the anchor's contribution to the partner queries
+            queries[2 * kD + tid] = __fadd_rn(queries[2 * kD + tid],
+                                              load_scalar(a.partner_anchor_cache, (static_cast<size_t>(row) * a.max_t + anchor_pos) * 2 * kD + tid, kDt));
+        if (tid == kThreads - 1) {
+            a.out_anchor[row] = anchor_pos;
+            a.out_anchor_score[row] = key_float(best_key);
         }
         __syncthreads();
-        if (32 * warp < picked_rows) {
-            pick();
-            score_remote_warp<kDt>(kResident ? smem + p.p_local : static_cast<const unsigned char*>(a.partner_keys) + seq_keys,
-                                   picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr, warp, kWarps);
-        }
     }
-    __syncthreads();
     // Exact top-K of the candidate table: output slot k holds the k-th best candidate (higher score first, equal scores
     // by the earlier slot); results without a finite score report -inf and the position of candidate slot 0.
-    int32_t* out_pos = a.out_partner + static_cast<size_t>(row) * a.k_out;
-    float* out_score = a.out_partner_score + static_cast<size_t>(row) * a.k_out;
-    if (cap4 > 512) topk_large(cand, cap, a.k_out, L, t, bs, sel_s[0], out_pos, out_score);
-    else if (warp == 0) topk_warp(cand, cap4, a.k_out, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);
+    const int K = a.k_out;
+    int32_t* out_pos = a.out_partner + static_cast<size_t>(row) * K;
+    float* out_score = a.out_partner_score + static_cast<size_t>(row) * K;
+    if (cap4 <= kThreads) {
+        // every candidate's rank, two threads a candidate for up to 128 of them: cap^2 / 256 comparisons a thread
+        uint32_t* rank_keys = reinterpret_cast<uint32_t*>(queries);      // 256 words, no longer needed
+        if (tid < cap4) rank_keys[tid] = float_key(cand[tid] + 0.0f);
+        __syncthreads();
+        const bool two = cap4 <= kThreads / 2;
+        const int slot = two ? tid >> 1 : tid, groups = cap4 >> 2, from = two && (tid & 1) ? groups >> 1 : 0,
+                  to = two && !(tid & 1) ? groups >> 1 : groups;
+        const uint32_t mine = rank_keys[slot < cap ? slot : 0], before = mine - 1u;      // keys of scores are positive
+        int rank = 0;
+        for (int g = from; g < to; ++g) {
+            const uint4 k = *reinterpret_cast<const uint4*>(rank_keys + 4 * g);
+            rank += (k.x > (4 * g + 0 < slot ? before : mine)) + (k.y > (4 * g + 1 < slot ? before : mine)) +
+                    (k.z > (4 * g + 2 < slot ? before : mine)) + (k.w > (4 * g + 3 < slot ? before : mine));
+        }
+        if (two) rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+        if (slot < cap && rank < K && !(two && (tid & 1))) {
+            const float score = cand[slot];
+            int pos = t - L + 1;
+            if (score > kNegInf) {
+                if (slot < L) pos += slot;
+                else { const int r = bs_shift >= 0 ? (slot - L) >> bs_shift : (slot - L) / bs; pos = sel_s[0][3 * r] * bs + (slot - L - r * bs); }
+            }
+            out_pos[rank] = pos;
+            out_score[rank] = score;
+        }
+        // more partners than candidates
+        for (int k = cap + tid; k < K; k += kThreads) { out_pos[k] = t - L + 1; out_score[k] = kNegInf; }
+    } else if (cap4 > 512) {
+        topk_large(cand, cap, K, L, t, bs, sel_s[0], out_pos, out_score);
+    } else if (warp == 0) {
+        topk_warp(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);
+    }
 }
 
 struct TileArgs {
