@@ -206,7 +206,7 @@ template <bool kBf16, typename Stage>
 __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const CUtensorMap& map_w2,
                                                 const LayerTailArgs& a, unsigned char* lt_smem_raw, const Stage& stage) {
     // W_m, W_2, product GEMM done, second GEMM done; partial sums, pair statistics, residual rows received
-    __shared__ __align__(8) unsigned long long bars[7];
+    __shared__ __align__(8) unsigned long long bars[10];         // the second GEMM has one per tile of 128 output rows
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
     __shared__ int pair_seq_s[kLtMaxPairs];
@@ -275,12 +275,12 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     };
 
     const uint32_t bar_wm = smem_u32(&bars[0]), bar_w2 = smem_u32(&bars[1]);
-    const uint32_t bar_d1 = smem_u32(&bars[2]), bar_d2 = smem_u32(&bars[3]);
-    const uint32_t bar_part = smem_u32(&bars[4]), bar_stat = smem_u32(&bars[5]), bar_rows = smem_u32(&bars[6]);
+    const uint32_t bar_d1 = smem_u32(&bars[2]), bar_part = smem_u32(&bars[3]), bar_stat = smem_u32(&bars[4]), bar_rows = smem_u32(&bars[5]);
+    const uint32_t bar_d2 = smem_u32(&bars[6]);                // + 8 per tile
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_wm) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
-        for (int i = 0; i < 7; ++i) mbar_init(smem_u32(&bars[i]), 1);
+        for (int i = 0; i < 10; ++i) mbar_init(smem_u32(&bars[i]), 1);
         fence_barrier_init();
         mbar_expect_tx(bar_part, static_cast<uint32_t>(C * quads) * 512u);
         mbar_expect_tx(bar_stat, static_cast<uint32_t>(C * pairs) * 8u);
@@ -327,10 +327,11 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const bool gathers_anchor = tid >= kLtThreads / 2 && a_entry < nseq;
     const int partner = entry < pairs ? a.partner_index[static_cast<size_t>(s0) * K + entry] : 0;
     const int anchor = gathers_anchor ? a.anchor_index[s0 + a_entry] : 0;
-    // scores of sequence = warp, for the softmax weights below
-    const float* score_row = a.partner_scores + static_cast<size_t>(s0 + warp) * K;
-    const float score0 = warp < nseq && lane < K ? score_row[lane] : kNegInf;
-    const float score1 = warp < nseq && lane + 32 < K ? score_row[lane + 32] : kNegInf;
+    // scores of one sequence per warp, for the softmax weights
+    const int weighted = kLtThreads / 32 - 1 - warp;
+    const float* score_row = a.partner_scores + static_cast<size_t>(s0 + weighted) * K;
+    const float score0 = weighted < nseq && lane < K ? score_row[lane] : kNegInf;
+    const float score1 = weighted < nseq && lane + 32 < K ? score_row[lane + 32] : kNegInf;
     const int t = static_cast<int>(*a.position);
     const bool bad_position = t < 0 || t >= a.max_t;          // the same in every CTA of the grid
     const int my_pair_row = min(max(partner, 0), a.max_t - 1);      // empty slots carry a sentinel that may be negative
@@ -371,20 +372,6 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             cp_async16(smem_u32(term_a) + a_entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
     }
     cp_async_commit();
-    // softmax weights over the active partner slots of a sequence (needed much later), by a warp while the gathers are
-    // in flight
-    if (warp < nseq) {
-        int k_limit = 32 - __clz(max(t, 0) + 1);               // ceil(log2(t + 2))
-        k_limit = min(max(k_limit, 1), K);
-        const bool live0 = lane < k_limit && score0 > -1.0e30f, live1 = lane + 32 < k_limit && score1 > -1.0e30f;
-        float mx = fmaxf(live0 ? score0 : -1.0e4f, live1 ? score1 : -1.0e4f);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const float e0 = live0 ? expf(score0 - mx) : 0.0f, e1 = live1 ? expf(score1 - mx) : 0.0f;
-        const float scale = 1.0f / fmaxf(warp_sum(e0 + e1), 1.0e-9f);
-        if (lane < K) weight_s[warp * K + lane] = e0 * scale;
-        if (lane + 32 < K) weight_s[warp * K + lane + 32] = e1 * scale;
-    }
     cp_async_wait_group1();                                    // the operand rows have arrived
     __syncthreads();
     // products o[a] * o[p], in fp32, rounded to the operand dtype, in place
@@ -470,7 +457,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         const bool ok = mbar_wait(bar_w2, 0), issue = lt_elect();
         if (!ok) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int mt = 0; mt < mtiles; ++mt)
+        for (int mt = 0; mt < mtiles; ++mt) {
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb) {
                 const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + (mt * 2 + kb) * kBM * 128u);
@@ -480,14 +467,31 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                     lt_umma(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
                             (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
             }
-        lt_commit(bar_d2, issue);
+            lt_commit(bar_d2 + 8u * mt, issue);                // each tile's partial sums leave while the next is computed
+        }
     }
     __syncwarp();
     if (pairs_pad > 16) request_wq();                          // in the consumed W_m slice's place, while the GEMM runs
     cp_async_commit();
-    if (!mbar_wait(bar_d2, 0)) failed = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (pairs_pad > 16) { __syncwarp(); lt_cluster_arrive(); }      // the W_2 slice is consumed: its place may receive
+    // meanwhile the softmax weights over the active partner slots of every sequence (the last warps first: warp 0 issues)
+    if (weighted < nseq) {
+        int k_limit = 32 - __clz(max(t, 0) + 1);               // ceil(log2(t + 2))
+        k_limit = min(max(k_limit, 1), K);
+        const bool live0 = lane < k_limit && score0 > -1.0e30f, live1 = lane + 32 < k_limit && score1 > -1.0e30f;
+        float mx = fmaxf(live0 ? score0 : -1.0e4f, live1 ? score1 : -1.0e4f);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float e0 = live0 ? expf(score0 - mx) : 0.0f, e1 = live1 ? expf(score1 - mx) : 0.0f;
+        const float scale = 1.0f / fmaxf(warp_sum(e0 + e1), 1.0e-9f);
+        if (lane < K) weight_s[weighted * K + lane] = e0 * scale;
+        if (lane + 32 < K) weight_s[weighted * K + lane + 32] = e1 * scale;
+    }
+    if (pairs_pad > 16) {
+        for (int mt = 0; mt < mtiles; ++mt)
+            if (!mbar_wait(bar_d2 + 8u * mt, 0)) failed = 1;
+        __syncwarp();
+        lt_cluster_arrive();                                   // the W_2 slice is consumed: its place may receive
+    }
     lt_cluster_wait();                                         // every CTA's receiving place is free
 
     // ---- reduce-scatter: the 32 output rows that a warp reads from the tensor memory belong to one CTA, which
@@ -497,6 +501,9 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     {
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
         for (int mt = warp >> 2; mt < mtiles; mt += 2) {
+            if (!mbar_wait(bar_d2 + 8u * mt, 0)) failed = 1;
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t owner = static_cast<uint32_t>(4 * mt + (warp & 3));
             const uint32_t bar = lt_peer(bar_part, owner);
             const uint32_t dst = lt_peer(smem_u32(recv), owner) + (rank * row_chunks * 32u + lane) * 16u;

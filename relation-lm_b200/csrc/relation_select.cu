@@ -213,16 +213,17 @@ __device__ __forceinline__ void fold_level(const float (&s)[kN], float (&out)[kN
     }
 }
 
-// Chunk sums of rows load(0) .. load(7) (row i: rows 4 i + rq of a pass), two rows at a time.
-template <int kDt, typename Load>
-__device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q, float (&s)[8]) {
+// Chunk sums of rows load(0) .. load(kN - 1) (row i: rows 4 i + rq of a pass), two rows at a time.
+template <int kDt, int kN, typename Load>
+__device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q, float (&s)[kN]) {
+    constexpr int kStep = kN < 4 ? kN : 4;
 #pragma unroll
-    for (int h = 0; h < 8; h += 4) {
-        uint4 w[4];
+    for (int h = 0; h < kN; h += kStep) {
+        uint4 w[kStep];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = load(h + i);
+        for (int i = 0; i < kStep; ++i) w[i] = load(h + i);
 #pragma unroll
-        for (int i = 0; i < 4; i += 2) {
+        for (int i = 0; i < kStep; i += 2) {
             const float2 p = seg_pair<kDt>(w[i], w[i + 1], q);
             s[h + i] = p.x;
             s[h + i + 1] = p.y;
@@ -230,15 +231,31 @@ __device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q
     }
 }
 
-// Score of the row that this lane owns after the butterfly: row 4 chunk + rq of the pass.
-template <int kDt, typename Load>
+// Score of the row that this lane owns after the butterfly: row 4 (chunk mod kN) + rq of a pass of 4 kN rows (with
+// fewer than eight rows per lane group, lanes own rows in common).  A pass of 32 rows costs the least per row; one of
+// 16 or 8 ends sooner, where warps are idle.
+template <int kDt, int kN, typename Load>
 __device__ __forceinline__ float pass_score(const Load& load, const QueryChunk& q) {
-    float s[8], v[4], u[2], t[1];
-    chunk_sums<kDt>(load, q, s);
-    fold_level<8, 1>(s, v);
-    fold_level<4, 2>(v, u);
-    fold_level<2, 4>(u, t);
-    return __fmul_rn(t[0], 0.125f);
+    float s[kN], total;
+    chunk_sums<kDt, kN>(load, q, s);
+    if constexpr (kN == 8) {
+        float v[4], u[2], t[1];
+        fold_level<8, 1>(s, v);
+        fold_level<4, 2>(v, u);
+        fold_level<2, 4>(u, t);
+        total = t[0];
+    } else if constexpr (kN == 4) {
+        float v[2], u[1];
+        fold_level<4, 1>(s, v);
+        fold_level<2, 2>(v, u);
+        total = __fadd_rn(u[0], __shfl_xor_sync(0xffffffffu, u[0], 4));
+    } else {
+        float v[1];
+        fold_level<2, 1>(s, v);
+        const float u = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 2));
+        total = __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, 4));
+    }
+    return __fmul_rn(total, 0.125f);
 }
 
 // Further excluded positions of a query (the anchors of a multi-anchor row's slots; -1 = none).
@@ -281,7 +298,7 @@ __device__ __forceinline__ void keep_best(bool valid, float score, int pos, uint
 // The local window, staged in shared memory: row r is position pos0 + r; rows below first_valid are none (and
 // not staged).  Scores go to cand[slot0 + r], or, without cand, into the running
 // best (kBoth: to both).
-template <int kDt, bool kExcl = false, bool kBoth = false>
+template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8>
 __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int n_rows, int first_valid, int pos0, int exclude,
                                                   const QueryChunk& q, float* cand, int slot0, uint32_t& best_key,
                                                   int& best_pos, const ExclRegs* ex = nullptr, int first = 0, int step = 1) {
@@ -289,19 +306,19 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
     const unsigned char* mine = rows + 16 * chunk;
-    for (int base = 32 * first; base < n_rows; base += 32 * step) {
+    for (int base = 4 * kN * first; base < n_rows; base += 4 * kN * step) {
         float sc;
-        if (base >= first_valid && base + 32 <= n_rows) {
+        if (base >= first_valid && base + 4 * kN <= n_rows) {
             const unsigned char* src = mine + (base + rq) * static_cast<int>(kRow);
-            sc = pass_score<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+            sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
         } else {
             // the ragged ends read a staged row in place of each missing one
-            sc = pass_score<kDt>([&](int i) {
+            sc = pass_score<kDt, kN>([&](int i) {
                 const int r = min(max(base + 4 * i + rq, first_valid), n_rows - 1);
                 return *reinterpret_cast<const uint4*>(mine + r * static_cast<int>(kRow));
             }, q);
         }
-        const int r = base + 4 * chunk + rq, pos = pos0 + r;
+        const int r = base + 4 * (chunk & (kN - 1)) + rq, pos = pos0 + r;
         const bool valid = r < n_rows && r >= first_valid && pos != exclude && not_excluded<kExcl>(pos, ex);
         sc = valid ? sc : kNegInf;
         if (kBoth || cand)
@@ -312,7 +329,7 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
 }
 
 // The picked remote blocks (sel: block, picked, rows), scored where they lie in the key cache.
-template <int kDt, bool kExcl = false, bool kBoth = false>
+template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8>
 __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
                                                   int bs_shift, int exclude, const QueryChunk& q, float* cand, int slot0,
                                                   uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr,
@@ -321,25 +338,25 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
     const unsigned char* mine = keys + 16 * chunk;
-    for (int base = 32 * first; base < n_rows; base += 32 * step) {
-        const int r = base + 4 * chunk + rq;
+    for (int base = 4 * kN * first; base < n_rows; base += 4 * kN * step) {
+        const int r = base + 4 * (chunk & (kN - 1)) + rq;
         int pos;                                         // position of row r, or -1
         float sc;
-        if (bs_shift >= 5) {
+        if (bs_shift >= (kN == 8 ? 5 : kN == 4 ? 4 : 3)) {
             // the pass lies in one picked block: rows 4 i + rq are 512 bytes apart
             const int rank = base >> bs_shift, o0 = base - (rank << bs_shift);
             const int start = sel[3 * rank] * bs + o0, lim = sel[3 * rank + 2] - o0;
             const unsigned char* src = mine + static_cast<size_t>(start + rq) * kRow;
             // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
-            sc = pass_score<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
-            pos = 4 * chunk + rq < lim ? start + 4 * chunk + rq : -1;
+            sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+            pos = r - base < lim ? start + (r - base) : -1;
         } else {
             auto row_pos = [&](int row) -> int {
                 if (row >= n_rows) return -1;
                 const int rank = bs_shift >= 0 ? row >> bs_shift : row / bs, o = row - rank * bs;
                 return o < sel[3 * rank + 2] ? sel[3 * rank] * bs + o : -1;
             };
-            sc = pass_score<kDt>([&](int i) {
+            sc = pass_score<kDt, kN>([&](int i) {
                 const int p = row_pos(base + 4 * i + rq);
                 return p >= 0 ? *reinterpret_cast<const uint4*>(mine + static_cast<size_t>(p) * kRow) : make_uint4(0, 0, 0, 0);
             }, q);
@@ -373,9 +390,9 @@ __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, con
     for (int base = 32 * first; base < n_complete; base += 32 * step) {
         float sums[8], md[4], sd[4];
         const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
-        chunk_sums<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+        chunk_sums<kDt, 8>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
         fold_level<8, 1>(sums, md);
-        chunk_sums<kDt>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+        chunk_sums<kDt, 8>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
         fold_level<8, 1>(sums, sd);
         // v[j]: head (chunk >> 1) of block 4 (2 j + (chunk & 1)) + rq
         float v[4], w[2][2], sh[4];
@@ -410,10 +427,66 @@ __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, con
     }
 }
 
+// The same, eight blocks a pass: a lane pair has one head of one block, and the heads of a block meet in two more
+// exchanges.  Half the time of a pass of 32, for few blocks and warps to spare.
+template <int kDt>
+__device__ __forceinline__ void score_few_blocks_warp(const unsigned char* mean, const unsigned char* stdv, int nb, int n_complete,
+                                                      int bs, int t, int ls, int strict, int buckets, const QueryChunk& q,
+                                                      const float* sp4, const float* bias, float* out, int first, int step) {
+    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3, head = chunk >> 1;
+    if (first == 0)
+        for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
+    QueryChunk qa;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
+    const float sp = sp4[head];
+    for (int base = 8 * first; base < n_complete; base += 8 * step) {
+        float sums[2], md[1], sd[1];
+        const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
+        const int n = base + 4 * (chunk & 1) + rq, end = (n + 1) * bs - 1;
+        int bucket = 31 - __clz(max(t - end, 0) + 1);
+        if (bucket > buckets - 1) bucket = buckets - 1;
+        const float shift = bias[head * buckets + bucket];
+        chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+        fold_level<2, 1>(sums, md);
+        chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+        fold_level<2, 1>(sums, sd);
+        const float sh = __fadd_rn(__fmul_rn(__fadd_rn(md[0], __fmul_rn(sp, sd[0])), 0.25f), shift);
+        float mx = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, 2));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        float e = canon_exp(__fsub_rn(sh, mx));
+        e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 2));
+        e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 4));
+        const float acc = __fadd_rn(mx, canon_log(e));
+        if (n < n_complete) out[n] = (!strict || end < ls) ? acc : kNegInf;
+    }
+}
+
 // pick_blocks for one warp and up to 128 blocks: `top` rounds of (largest score, lowest block on
 // ties) through two redux instructions each, instead of ranking every block against all others.
 __device__ __forceinline__ void pick_blocks_warp(const float* scores, int nb, int top, int bs, int ls, int* sel) {
     const int lane = threadIdx.x & 31;
+    if (nb <= 32) {                                          // a block a lane; top <= nb
+        int picked = -1;                                     // lane r keeps the r-th choice
+
+        const float v = lane < nb ? scores[lane] : kNegInf;
+        uint32_t key = v > -1.0e30f ? float_key(v + 0.0f) : 0u;
+        for (int r = 0; r < min(top, 32); ++r) {
+            const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+            if (best == 0u) break;
+            const int n = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
+            picked = lane == r ? n : picked;
+            key = lane == n ? 0u : key;
+        }
+        if (lane < top) {
+            const int rows = picked < 0 ? 0 : min(max(ls - picked * bs, 0), bs);
+            sel[3 * lane] = max(picked, 0);
+            sel[3 * lane + 1] = picked >= 0;
+            sel[3 * lane + 2] = rows;
+        }
+        __syncwarp();
+        return;
+    }
     uint32_t key[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -594,7 +667,8 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     __syncthreads();
 
     // blocks and window side by side: up to half of the warps walk the passes of blocks
-    const int block_warps = top > 0 ? max(1, min((n_complete + 31) >> 5, kWarps / 2)) : 0;
+    const bool few_blocks = n_complete <= 32;
+    const int block_warps = top > 0 ? max(1, min(few_blocks ? (n_complete + 7) >> 3 : (n_complete + 31) >> 5, kWarps / 2)) : 0;
     const int picked_rows = top * bs;
     int* sel = sel_s[warp];
     // row r of a window is position t - L + 1 + r (only rows that are staged are read)
@@ -613,23 +687,43 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         int bp = 0x7fffffff;
         if (warp < block_warps) {
             load_query_chunk(query + kD, q);
-            score_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, softplus_s + 4 * stream,
-                                   stream ? bias_p : bias_a, bscore, warp, block_warps);
+            const float* sp = softplus_s + 4 * stream, *bias = stream ? bias_p : bias_a;
+            if (few_blocks)
+                score_few_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp, bias, bscore,
+                                           warp, block_warps);
+            else
+                score_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp, bias, bscore, warp,
+                                       block_warps);
         } else {
             load_query_chunk(query, q);
-            score_window_warp<kDt, false, true>(staged + window_offset, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp,
-                                                nullptr, warp - block_warps, kWarps - block_warps);
+            const unsigned char* window = staged + window_offset;
+            const int first = warp - block_warps, step = kWarps - block_warps;
+            if (L <= 16 * step)
+                score_window_warp<kDt, false, true, 4>(window, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp, nullptr,
+                                                       first, step);
+            else
+                score_window_warp<kDt, false, true>(window, L, first_local, t - L + 1, anchor_pos, q, cand, 0, bk, bp, nullptr,
+                                                    first, step);
         }
         if (__syncthreads_or(!ok)) {
             if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
             return;
         }
-        if (32 * warp < picked_rows) {
+        const int pass_rows = picked_rows <= 8 * kWarps ? 8 : picked_rows <= 16 * kWarps ? 16 : 32;
+        if (pass_rows * warp < picked_rows) {
             load_query_chunk(query, q);
             if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
             else pick_blocks(bscore, nb, top, bs, ls, sel);
-            score_remote_warp<kDt, false, true>(kResident ? staged : keys, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L,
-                                                bk, bp, nullptr, warp, kWarps);
+            const unsigned char* rows = kResident ? staged : keys;
+            if (pass_rows == 8)
+                score_remote_warp<kDt, false, true, 2>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
+                                                       warp, kWarps);
+            else if (pass_rows == 16)
+                score_remote_warp<kDt, false, true, 4>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
+                                                       warp, kWarps);
+            else
+                score_remote_warp<kDt, false, true>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
+                                                    warp, kWarps);
         }
         if (lane == 0) { best_key_s[warp] = bk; best_pos_s[warp] = bp; }
         __syncthreads();
@@ -666,13 +760,18 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         const bool two = cap4 <= kThreads / 2;
         const int slot = two ? tid >> 1 : tid, groups = cap4 >> 2, from = two && (tid & 1) ? groups >> 1 : 0,
                   to = two && !(tid & 1) ? groups >> 1 : groups;
+        // candidates of earlier slots go first where they tie: theirs is the comparison with >=
         const uint32_t mine = rank_keys[slot < cap ? slot : 0], before = mine - 1u;      // keys of scores are positive
+        const int own = slot >> 2;
         int rank = 0;
+#pragma unroll 4
         for (int g = from; g < to; ++g) {
             const uint4 k = *reinterpret_cast<const uint4*>(rank_keys + 4 * g);
-            rank += (k.x > (4 * g + 0 < slot ? before : mine)) + (k.y > (4 * g + 1 < slot ? before : mine)) +
-                    (k.z > (4 * g + 2 < slot ? before : mine)) + (k.w > (4 * g + 3 < slot ? before : mine));
+            const uint32_t bar = g < own ? before : mine;
+            rank += (k.x > bar) + (k.y > bar) + (k.z > bar) + (k.w > bar);
         }
+        if (own >= from && own < to)
+            for (int j = 4 * own; j < slot; ++j) rank += rank_keys[j] == mine;
         if (two) rank += __shfl_xor_sync(0xffffffffu, rank, 1);
         if (slot < cap && rank < K && !(two && (tid & 1))) {
             const float score = cand[slot];

@@ -187,9 +187,7 @@ __device__ __forceinline__ void convert8(const Raw8& r, int dtype, float (&f)[8]
 // makes block scores reproducible bit for bit by a CPU following the same steps.
 
 __device__ __forceinline__ float canon_exp(float x) {
-    if (x != x) return x;
-    if (x < -86.0f) return 0.0f;
-    if (x > 88.0f) return __int_as_float(0x7f800000);
+    // the special cases are selected at the end: as early returns their branches took longer than the evaluation
     const float magic = 12582912.0f;  // 1.5 * 2^23
     float kf = __fsub_rn(__fmaf_rn(x, 1.44269502f, magic), magic);
     float r = __fmaf_rn(kf, -0.693145752f, x);
@@ -202,17 +200,17 @@ __device__ __forceinline__ float canon_exp(float x) {
     p = __fmaf_rn(p, r, 0.5f);
     p = __fmaf_rn(p, r, 1.0f);
     p = __fmaf_rn(p, r, 1.0f);
-    int k = static_cast<int>(kf);
-    return __int_as_float(__float_as_int(p) + k * (1 << 23));
+    const uint32_t k = static_cast<uint32_t>(static_cast<int>(kf));
+    float y = __uint_as_float(__float_as_uint(p) + (k << 23));
+    y = x < -86.0f ? 0.0f : y;
+    y = x > 88.0f ? __int_as_float(0x7f800000) : y;
+    return x != x ? x : y;
 }
 
 __device__ __forceinline__ float canon_log(float y) {
-    if (y != y || y < 0.0f) return __int_as_float(0x7fc00000);
-    if (y == 0.0f) return kNegInf;
-    if (y == __int_as_float(0x7f800000)) return y;
     int bits = __float_as_int(y);
     int e = (bits - 0x3f3504f3) >> 23;
-    float m = __int_as_float(bits - e * (1 << 23));
+    float m = __uint_as_float(static_cast<uint32_t>(bits) - (static_cast<uint32_t>(e) << 23));
     float f = __fsub_rn(m, 1.0f);
     float z = __fdiv_rn(f, __fadd_rn(2.0f, f));
     float w = __fmul_rn(z, z);
@@ -226,7 +224,10 @@ __device__ __forceinline__ float canon_log(float y) {
     float lm = __fmaf_rn(z2, p, z2);
     float ef = static_cast<float>(e);
     float r = __fmaf_rn(ef, 1.42860677e-06f, lm);
-    return __fmaf_rn(ef, 0.693145752f, r);
+    r = __fmaf_rn(ef, 0.693145752f, r);
+    r = y == 0.0f ? kNegInf : r;
+    r = y == __int_as_float(0x7f800000) ? y : r;
+    return y != y || y < 0.0f ? __int_as_float(0x7fc00000) : r;
 }
 
 // acc = 0; acc = fma(a[i], b[i], acc) for ascending i.
