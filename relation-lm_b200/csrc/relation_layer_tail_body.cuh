@@ -300,7 +300,12 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                      ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    const int entry = tid >> 2, quarter = tid & 3, bl = entry / K;      // bl: sequence of pair `entry`
     if (!Stage::kActive && pairs_pad == 16) request_wq();       // a parameter: before the dependency wait
+    // the kernel's parameters that are first used behind the wait, into the constant cache
+    asm volatile("" ::"l"(a.operand_cache), "l"(a.expanded_cache), "l"(a.anchor_index), "l"(a.partner_index), "l"(a.partner_scores),
+                 "l"(a.position), "l"(a.residual), "l"(a.mix), "l"(a.normalized), "l"(a.query), "r"(a.max_t), "f"(a.eps),
+                 "f"(a.next_eps));
     if (Stage::kActive) {
         // the stage's results reach the other CTAs of the cluster through global memory, ordered by
         // the cluster barrier
@@ -322,7 +327,6 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // its epilogue).  Indices and scores are all requested before the first is used, and the
     // anchors' rows are gathered by threads that a small batch's partner rows leave free.
     const size_t op_row = static_cast<size_t>(R) * 2, ex_row = static_cast<size_t>(H) * 4;
-    const int entry = tid >> 2, quarter = tid & 3;
     const int a_entry = (tid - kLtThreads / 2) >> 2;          // sequence whose anchor this thread gathers
     const bool gathers_anchor = tid >= kLtThreads / 2 && a_entry < nseq;
     const int partner = entry < pairs ? a.partner_index[static_cast<size_t>(s0) * K + entry] : 0;
@@ -337,7 +341,6 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const int my_pair_row = min(max(partner, 0), a.max_t - 1);      // empty slots carry a sentinel that may be negative
     const int my_anchor_row = min(max(anchor, 0), a.max_t - 1);
     if (entry < pairs) {
-        const int bl = entry / K;
         if (quarter == 0) pair_seq_s[entry] = bl;
         const char* src = static_cast<const char*>(a.operand_cache) +
                           (static_cast<size_t>(s0 + bl) * a.max_t + my_pair_row) * op_row;
@@ -357,7 +360,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     cp_async_commit();
     if (entry < pairs) {
         const char* src = static_cast<const char*>(a.expanded_cache) +
-                          (static_cast<size_t>(s0 + entry / K) * a.max_t + my_pair_row) * ex_row +
+                          (static_cast<size_t>(s0 + bl) * a.max_t + my_pair_row) * ex_row +
                           static_cast<size_t>(H + h0) * 2;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -500,7 +503,9 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     unsigned char* recv = pairs_pad == 16 ? wm_tile : w2_tile;
     {
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        for (int mt = warp >> 2; mt < mtiles; mt += 2) {
+        // few pairs: by the last four warps alone, a tile behind the GEMM that warp 0 is still issuing
+        const int first = pairs_pad > 16 ? warp >> 2 : warp >= 4 ? 0 : mtiles, step = pairs_pad > 16 ? 2 : 1;
+        for (int mt = first; mt < mtiles; mt += step) {
             if (!mbar_wait(bar_d2 + 8u * mt, 0)) failed = 1;
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -522,8 +527,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 
-    // ---- a warp owns four pairs (32 columns, a lane each): partial sums in rank order, so that the result does not
-    // depend on timing, and (mean, M2) of the 32 columns, pushed to every CTA
+    // ---- a warp owns four pairs (32 columns, a lane each): partial sums in a fixed order, so that the result does
+    // not depend on timing, and (mean, M2) of the 32 columns, pushed to every CTA
     if (!mbar_wait(bar_part, 0)) failed = 1;
     float x[2][4];
 #pragma unroll
@@ -531,14 +536,24 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         const int q = warp + 8 * it;
         if (q >= quads) break;
         const unsigned char* src = recv + (static_cast<uint32_t>(q) * 32u + lane) * 16u;
-        float4 v[16];
+        float4 part_sum[4];                                    // senders of equal rank modulo four (C is 4, 8 or 16)
 #pragma unroll
-        for (int s = 0; s < 16; ++s)
-            v[s] = s < C ? *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(s * row_chunks) * 512u)
-                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int k = 0; k < 4; ++k)
+            part_sum[k] = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(k * row_chunks) * 512u);
 #pragma unroll
-        for (int s = 0; s < 16; ++s) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
+        for (int s = 4; s < 16; s += 4) {
+            if (s >= C) break;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 v = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>((s + k) * row_chunks) * 512u);
+                part_sum[k].x += v.x; part_sum[k].y += v.y; part_sum[k].z += v.z; part_sum[k].w += v.w;
+            }
+        }
+        float4 acc;
+        acc.x = (part_sum[0].x + part_sum[1].x) + (part_sum[2].x + part_sum[3].x);
+        acc.y = (part_sum[0].y + part_sum[1].y) + (part_sum[2].y + part_sum[3].y);
+        acc.z = (part_sum[0].z + part_sum[1].z) + (part_sum[2].z + part_sum[3].z);
+        acc.w = (part_sum[0].w + part_sum[1].w) + (part_sum[2].w + part_sum[3].w);
         x[it][0] = acc.x + pre_bias; x[it][1] = acc.y + pre_bias; x[it][2] = acc.z + pre_bias; x[it][3] = acc.w + pre_bias;
         const float2 moments = lt_moments4(x[it]);
         const int pr = 4 * q + (lane >> 3);
@@ -595,10 +610,16 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // columns are pushed to
     if (part < parts) {
         float ctx = 0.0f;
-#pragma unroll 4
-        for (int k = 0; k < K; ++k) {
-            const float wk = weight_s[my_seq * K + k], y = own_y[(my_seq * K + k) * kLtOwnStride + lane];
-            ctx = wk == 0.0f ? ctx : fmaf(wk, y, ctx);         // inactive slots contribute nothing
+        for (int k0 = 0; k0 < K; k0 += 8) {
+            float wk[8], y[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int at = my_seq * K + min(k0 + k, K - 1);
+                wk[k] = k0 + k < K ? weight_s[at] : 0.0f;
+                y[k] = own_y[at * kLtOwnStride + lane];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ctx = wk[k] == 0.0f ? ctx : fmaf(wk[k], y[k], ctx);     // inactive slots contribute nothing
         }
         const float hval = bad_position ? pre_res : fmaf(pre_mix, ctx, pre_res);
         if (part == 0 && !bad_position) a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane] = hval;
@@ -614,6 +635,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     uint16_t* rows16 = reinterpret_cast<uint16_t*>(p_tile);    // [sequence][d]
     if (part < parts) {
         const float* row = rows_in + my_seq * D;
+        // local moments of the lane's 4 mtiles columns, then five exchanges of (mean, M2) of equal halves
         float4 h[4];
         float sum = 0.0f;
 #pragma unroll
@@ -621,16 +643,21 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             h[i] = i < mtiles ? *reinterpret_cast<const float4*>(row + 128 * i + 4 * lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             sum += (h[i].x + h[i].y) + (h[i].z + h[i].w);
         }
-        const float mean = warp_sum(sum) / static_cast<float>(D);
-        float sq = 0.0f;
+        float count = 4.0f * static_cast<float>(mtiles), mean = sum * (1.0f / count), m2 = 0.0f;      // a power of two
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (i < mtiles) {
-                h[i].x -= mean; h[i].y -= mean; h[i].z -= mean; h[i].w -= mean;
-                sq = fmaf(h[i].x, h[i].x, sq); sq = fmaf(h[i].y, h[i].y, sq);
-                sq = fmaf(h[i].z, h[i].z, sq); sq = fmaf(h[i].w, h[i].w, sq);
+                const float dx = h[i].x - mean, dy = h[i].y - mean, dz = h[i].z - mean, dw = h[i].w - mean;
+                m2 += fmaf(dx, dx, dy * dy) + fmaf(dz, dz, dw * dw);
             }
-        const float rstd = rsqrtf(warp_sum(sq) / static_cast<float>(D) + a.next_eps);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float other = __shfl_xor_sync(0xffffffffu, mean, o), other2 = __shfl_xor_sync(0xffffffffu, m2, o), d = mean - other;
+            m2 = fmaf(d * d, 0.5f * count, m2 + other2);
+            mean = 0.5f * (mean + other);
+            count += count;
+        }
+        const float rstd = rsqrtf(fmaf(m2, 1.0f / static_cast<float>(D), a.next_eps));
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int chunk = part + i * parts;
@@ -641,8 +668,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 if (chunk == k) v = h[k];
             const float4 g = next_g[i], b = next_b[i];
             const uint2 out = make_uint2(
-                pack2(fmaf(v.x * rstd, g.x, b.x), fmaf(v.y * rstd, g.y, b.y), dtype),
-                pack2(fmaf(v.z * rstd, g.z, b.z), fmaf(v.w * rstd, g.w, b.w), dtype));
+                pack2(fmaf((v.x - mean) * rstd, g.x, b.x), fmaf((v.y - mean) * rstd, g.y, b.y), dtype),
+                pack2(fmaf((v.z - mean) * rstd, g.z, b.z), fmaf((v.w - mean) * rstd, g.w, b.w), dtype));
             const int at = 128 * chunk + 4 * lane;
             *reinterpret_cast<uint2*>(rows16 + my_seq * D + at) = out;
             if (at / kLtOwn == static_cast<int>(rank) && !bad_position)
