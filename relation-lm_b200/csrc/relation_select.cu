@@ -427,63 +427,91 @@ __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, con
     }
 }
 
-// The same, eight blocks a pass: a lane pair has one head of one block, and the heads of a block meet in two more
-// exchanges.  Half the time of a pass of 32, for few blocks and warps to spare.
+// Scores of eight blocks, first .. first + 7: a lane pair has one head of one block, and the heads of a block meet in
+// two more exchanges.  Half the time of a pass of 32, for few blocks and warps to spare.  `sp` and `shift`: this lane's
+// head's softplus(gamma) and its bias at the block's distance (block_shift).
+__device__ __forceinline__ int lane_block(int first) { return first + 4 * (threadIdx.x & 1) + ((threadIdx.x & 31) >> 3); }
+
+__device__ __forceinline__ float block_shift(const void* bias, int block, int bs, int t, int buckets, int dtype) {
+    int bucket = 31 - __clz(max(t - ((block + 1) * bs - 1), 0) + 1);
+    if (bucket > buckets - 1) bucket = buckets - 1;
+    return load_scalar(bias, ((threadIdx.x & 7) >> 1) * buckets + bucket, dtype);
+}
+
 template <int kDt>
-__device__ __forceinline__ void score_few_blocks_warp(const unsigned char* mean, const unsigned char* stdv, int nb, int n_complete,
-                                                      int bs, int t, int ls, int strict, int buckets, const QueryChunk& q,
-                                                      const float* sp4, const float* bias, float* out, int first, int step) {
-    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3, head = chunk >> 1;
-    if (first == 0)
-        for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
+__device__ __forceinline__ void score_eight_blocks(const unsigned char* mean, const unsigned char* stdv, int first, int n_complete,
+                                                   int bs, int ls, int strict, const QueryChunk& q, float sp, float shift,
+                                                   float* out) {
+    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     QueryChunk qa;
 #pragma unroll
     for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
-    const float sp = sp4[head];
-    for (int base = 8 * first; base < n_complete; base += 8 * step) {
-        float sums[2], md[1], sd[1];
-        const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
-        const int n = base + 4 * (chunk & 1) + rq, end = (n + 1) * bs - 1;
-        int bucket = 31 - __clz(max(t - end, 0) + 1);
-        if (bucket > buckets - 1) bucket = buckets - 1;
-        const float shift = bias[head * buckets + bucket];
-        chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
-        fold_level<2, 1>(sums, md);
-        chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
-        fold_level<2, 1>(sums, sd);
-        const float sh = __fadd_rn(__fmul_rn(__fadd_rn(md[0], __fmul_rn(sp, sd[0])), 0.25f), shift);
-        float mx = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, 2));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-        float e = canon_exp(__fsub_rn(sh, mx));
-        e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 2));
-        e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 4));
-        const float acc = __fadd_rn(mx, canon_log(e));
-        if (n < n_complete) out[n] = (!strict || end < ls) ? acc : kNegInf;
+    float sums[2], md[1], sd[1];
+    const auto at = [&](int i) { return static_cast<uint32_t>(min(first + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
+    chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+    fold_level<2, 1>(sums, md);
+    chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+    fold_level<2, 1>(sums, sd);
+    const float sh = __fadd_rn(__fmul_rn(__fadd_rn(md[0], __fmul_rn(sp, sd[0])), 0.25f), shift);
+    float mx = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, 2));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    float e = canon_exp(__fsub_rn(sh, mx));
+    e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 2));
+    e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 4));
+    const int n = lane_block(first);
+    if (n < n_complete) out[n] = (!strict || (n + 1) * bs - 1 < ls) ? __fadd_rn(mx, canon_log(e)) : kNegInf;
+}
+
+// The choices of pick_blocks among up to 32 blocks, a block a lane: lane r gets the r-th, or -1.
+__device__ __forceinline__ int pick_small(const float* scores, int nb, int top) {
+    const int lane = threadIdx.x & 31;
+    const float v = lane < nb ? scores[lane] : kNegInf;
+    uint32_t key = v > -1.0e30f ? float_key(v + 0.0f) : 0u;
+    int picked = -1;
+    for (int r = 0; r < top; ++r) {
+        const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+        if (best == 0u) break;
+        const int n = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
+        picked = lane == r ? n : picked;
+        key = lane == n ? 0u : key;
     }
+    return picked;
+}
+
+// The list entry (block, picked, rows) of a choice.
+__device__ __forceinline__ void write_pick(int* entry, int picked, int bs, int ls) {
+    entry[0] = max(picked, 0);
+    entry[1] = picked >= 0;
+    entry[2] = picked < 0 ? 0 : min(max(ls - picked * bs, 0), bs);
+}
+
+// Pass `first` of the picked rows with the choices in registers (lane r: the r-th) and a pass inside one block.
+template <int kDt, int kN>
+__device__ __forceinline__ void score_picked_pass(const unsigned char* keys, int first, int picked, int bs, int bs_shift, int ls,
+                                                  int exclude, const QueryChunk& q, float* cand, uint32_t& best_key, int& best_pos) {
+    const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3, base = 4 * kN * first;
+    const int rank = base >> bs_shift, o0 = base - (rank << bs_shift), block = __shfl_sync(0xffffffffu, picked, rank);
+    const int start = max(block, 0) * bs + o0, lim = block < 0 ? 0 : min(max(ls - block * bs, 0), bs) - o0;
+    const unsigned char* src = keys + static_cast<size_t>(start + rq) * kRow + 16 * chunk;
+    // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
+    float sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+    const int o = 4 * (chunk & (kN - 1)) + rq, pos = start + o;
+    const bool valid = o < lim && pos != exclude;
+    sc = valid ? sc : kNegInf;
+    cand[base + o] = sc;
+    uint32_t my_key = 0;
+    int my_pos = 0x7fffffff;
+    keep_best(valid, sc, pos, my_key, my_pos);
+    fold_best(my_key, my_pos, best_key, best_pos);
 }
 
 // pick_blocks for one warp and up to 128 blocks: `top` rounds of (largest score, lowest block on
 // ties) through two redux instructions each, instead of ranking every block against all others.
 __device__ __forceinline__ void pick_blocks_warp(const float* scores, int nb, int top, int bs, int ls, int* sel) {
     const int lane = threadIdx.x & 31;
-    if (nb <= 32) {                                          // a block a lane; top <= nb
-        int picked = -1;                                     // lane r keeps the r-th choice
-
-        const float v = lane < nb ? scores[lane] : kNegInf;
-        uint32_t key = v > -1.0e30f ? float_key(v + 0.0f) : 0u;
-        for (int r = 0; r < min(top, 32); ++r) {
-            const uint32_t best = __reduce_max_sync(0xffffffffu, key);
-            if (best == 0u) break;
-            const int n = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
-            picked = lane == r ? n : picked;
-            key = lane == n ? 0u : key;
-        }
-        if (lane < top) {
-            const int rows = picked < 0 ? 0 : min(max(ls - picked * bs, 0), bs);
-            sel[3 * lane] = max(picked, 0);
-            sel[3 * lane + 1] = picked >= 0;
-            sel[3 * lane + 2] = rows;
-        }
+    if (nb <= 32) {
+        const int picked = pick_small(scores, nb, top);
+        if (lane < top) write_pick(sel + 3 * lane, picked, bs, ls);
         __syncwarp();
         return;
     }
@@ -595,6 +623,26 @@ __device__ __forceinline__ void topk_warp(const float* cand, int cap4, int K, in
     }
 }
 
+// How many of 4 n_groups keys come before `mine`, number `index` of them: the larger, and the equal ones of lower
+// number; mine > 0.  Four counters, so that the additions do not wait for one another.
+template <int kUnroll>
+__device__ __forceinline__ int rank_among(const uint32_t* keys, int n_groups, uint32_t mine, int index) {
+    const uint32_t before = mine - 1u;                       // k > before: k >= mine
+    const int own = index >> 2, at = index & 3;
+    const uint4 k0 = *reinterpret_cast<const uint4*>(keys + 4 * own);
+    int r0 = k0.x == mine && at > 0, r1 = k0.y == mine && at > 1, r2 = k0.z == mine && at > 2, r3 = 0;
+#pragma unroll kUnroll
+    for (int g = 0; g < n_groups; ++g) {
+        const uint4 k = *reinterpret_cast<const uint4*>(keys + 4 * g);
+        const uint32_t bar = g < own ? before : mine;
+        if (k.x > bar) ++r0;
+        if (k.y > bar) ++r1;
+        if (k.z > bar) ++r2;
+        if (k.w > bar) ++r3;
+    }
+    return (r0 + r1) + (r2 + r3);
+}
+
 // ---- the decode form in one 16-bit dtype: a query row by a CTA of eight warps
 //
 // A row's time is a chain of dependent phases, so what counts is their number and length, not their work.  Here a
@@ -610,7 +658,7 @@ template <int kDt, bool kResident>
 __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_decode_kernel(const SelectArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t best_key_s[kWarps], short_list[64];
-    __shared__ int best_pos_s[kWarps], sel_s[kWarps][3 * kDecodeTop];
+    __shared__ __align__(16) int best_pos_s[kWarps], sel_s[kWarps * 3 * kDecodeTop];
     __shared__ float softplus_s[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.x, buckets4 = 4 * a.buckets;
@@ -621,7 +669,7 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     const int t = static_cast<int>(*a.position);
     const int nb = a.n_blocks, bs = a.block_size, L = a.local_window, top = a.top_blocks;
     const int bs_shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
-    const int ls = max(t - L + 1, 0), first_local = ls - (t - L + 1), n_complete = min((t + 1) / bs, nb);
+    const int ls = max(t - L + 1, 0), first_local = ls - (t - L + 1), n_complete = max(min((t + 1) / bs, nb), 0);
     const size_t seq_keys = static_cast<size_t>(row) * a.max_t * kRow, seq_stats = static_cast<size_t>(row) * nb * kRow;
     const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
     const bool bad_position = t < 0 || t >= a.max_t;
@@ -654,6 +702,21 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         bias_p[i] = load_scalar(a.partner_bias, i, a.param_dtype);
     }
     if (tid < cap4 - cap) cand[cap + tid] = kNegInf;             // padding slots never win a comparison
+    const bool few_blocks = n_complete <= 32;
+    for (int n = n_complete + tid; n < ((nb + 3) & ~3); n += kThreads) bscore[n] = kNegInf;
+    // few blocks: eight to a warp, whose lanes keep their head's parameters for both streams
+    float lane_sp[2] = {0.0f, 0.0f}, lane_shift[2] = {0.0f, 0.0f};
+    if (few_blocks && !bad_position && 8 * warp < n_complete) {
+        const int head = (tid & 7) >> 1, block = lane_block(8 * warp);
+        lane_sp[0] = canon_log(__fadd_rn(1.0f, canon_exp(load_scalar(a.anchor_gamma, head, a.param_dtype))));
+        lane_sp[1] = canon_log(__fadd_rn(1.0f, canon_exp(load_scalar(a.partner_gamma, head, a.param_dtype))));
+        lane_shift[0] = block_shift(a.anchor_bias, block, bs, t, a.buckets, a.param_dtype);
+        lane_shift[1] = block_shift(a.partner_bias, block, bs, t, a.buckets, a.param_dtype);
+    }
+    // parameters that are first used behind the wait, into the constant cache
+    asm volatile("" ::"l"(a.anchor_query), "l"(a.anchor_router_query), "l"(a.partner_base), "l"(a.partner_anchor_cache),
+                 "l"(a.out_anchor), "l"(a.out_anchor_score), "l"(a.out_partner), "l"(a.out_partner_score), "l"(a.aq_stride),
+                 "l"(a.arq_stride), "l"(a.pbase_stride), "r"(a.k_out), "r"(a.strict_valid));
     if (tid >= 32 && tid < 40)
         softplus_s[tid - 32] = canon_log(__fadd_rn(1.0f, canon_exp(load_scalar(tid < 36 ? a.anchor_gamma : a.partner_gamma, tid & 3, a.param_dtype))));
     griddep_sync();
@@ -667,10 +730,9 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     __syncthreads();
 
     // blocks and window side by side: up to half of the warps walk the passes of blocks
-    const bool few_blocks = n_complete <= 32;
     const int block_warps = top > 0 ? max(1, min(few_blocks ? (n_complete + 7) >> 3 : (n_complete + 31) >> 5, kWarps / 2)) : 0;
     const int picked_rows = top * bs;
-    int* sel = sel_s[warp];
+    int* sel = sel_s + warp * 3 * kDecodeTop;
     // row r of a window is position t - L + 1 + r (only rows that are staged are read)
     const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(kRow) : 0;
     int anchor_pos = -1;
@@ -687,13 +749,13 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         int bp = 0x7fffffff;
         if (warp < block_warps) {
             load_query_chunk(query + kD, q);
-            const float* sp = softplus_s + 4 * stream, *bias = stream ? bias_p : bias_a;
-            if (few_blocks)
-                score_few_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp, bias, bscore,
-                                           warp, block_warps);
-            else
-                score_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp, bias, bscore, warp,
-                                       block_warps);
+            if (!few_blocks)
+                score_blocks_warp<kDt>(mean, stdv, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, softplus_s + 4 * stream,
+                                       stream ? bias_p : bias_a, bscore, warp, block_warps);
+            else if (n_complete > 0)
+                score_eight_blocks<kDt>(mean, stdv, 8 * warp, n_complete, bs, ls, a.strict_valid, q, stream ? lane_sp[1] : lane_sp[0],
+                                        stream ? lane_shift[1] : lane_shift[0], bscore);
+            load_query_chunk(query, q);
         } else {
             load_query_chunk(query, q);
             const unsigned char* window = staged + window_offset;
@@ -709,21 +771,23 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
             if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_TIMEOUT);
             return;
         }
-        const int pass_rows = picked_rows <= 8 * kWarps ? 8 : picked_rows <= 16 * kWarps ? 16 : 32;
-        if (pass_rows * warp < picked_rows) {
-            load_query_chunk(query, q);
+        const unsigned char* rows = kResident ? staged : keys;
+        if (nb <= 32 && bs_shift >= 4 && picked_rows <= 16 * kWarps) {
+            // a pass of 8 or 16 rows per warp, each inside one block; the first warp leaves the list for the top K
+            const int pass_rows = picked_rows <= 8 * kWarps ? 8 : 16;
+            if (pass_rows * warp < picked_rows) {
+                const int picked = pick_small(bscore, nb, top);
+                if (pass_rows == 8)
+                    score_picked_pass<kDt, 2>(rows, warp, picked, bs, bs_shift, ls, anchor_pos, q, cand + L, bk, bp);
+                else
+                    score_picked_pass<kDt, 4>(rows, warp, picked, bs, bs_shift, ls, anchor_pos, q, cand + L, bk, bp);
+                if (warp == 0 && lane < top) write_pick(sel + 3 * lane, picked, bs, ls);
+            }
+        } else if (32 * warp < picked_rows) {
             if (nb <= 128) pick_blocks_warp(bscore, nb, top, bs, ls, sel);
             else pick_blocks(bscore, nb, top, bs, ls, sel);
-            const unsigned char* rows = kResident ? staged : keys;
-            if (pass_rows == 8)
-                score_remote_warp<kDt, false, true, 2>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
-                                                       warp, kWarps);
-            else if (pass_rows == 16)
-                score_remote_warp<kDt, false, true, 4>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
-                                                       warp, kWarps);
-            else
-                score_remote_warp<kDt, false, true>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr,
-                                                    warp, kWarps);
+            score_remote_warp<kDt, false, true>(rows, picked_rows, sel, bs, bs_shift, anchor_pos, q, cand, L, bk, bp, nullptr, warp,
+                                                kWarps);
         }
         if (lane == 0) { best_key_s[warp] = bk; best_pos_s[warp] = bp; }
         __syncthreads();
@@ -753,40 +817,37 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     int32_t* out_pos = a.out_partner + static_cast<size_t>(row) * K;
     float* out_score = a.out_partner_score + static_cast<size_t>(row) * K;
     if (cap4 <= kThreads) {
-        // every candidate's rank, two threads a candidate for up to 128 of them: cap^2 / 256 comparisons a thread
-        uint32_t* rank_keys = reinterpret_cast<uint32_t*>(queries);      // 256 words, no longer needed
-        if (tid < cap4) rank_keys[tid] = float_key(cand[tid] + 0.0f);
-        __syncthreads();
-        const bool two = cap4 <= kThreads / 2;
-        const int slot = two ? tid >> 1 : tid, groups = cap4 >> 2, from = two && (tid & 1) ? groups >> 1 : 0,
-                  to = two && !(tid & 1) ? groups >> 1 : groups;
-        // candidates of earlier slots go first where they tie: theirs is the comparison with >=
-        const uint32_t mine = rank_keys[slot < cap ? slot : 0], before = mine - 1u;      // keys of scores are positive
-        const int own = slot >> 2;
-        int rank = 0;
-#pragma unroll 4
-        for (int g = from; g < to; ++g) {
-            const uint4 k = *reinterpret_cast<const uint4*>(rank_keys + 4 * g);
-            const uint32_t bar = g < own ? before : mine;
-            rank += (k.x > bar) + (k.y > bar) + (k.z > bar) + (k.w > bar);
-        }
-        if (own >= from && own < to)
-            for (int j = 4 * own; j < slot; ++j) rank += rank_keys[j] == mine;
-        if (two) rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-        if (slot < cap && rank < K && !(two && (tid & 1))) {
-            const float score = cand[slot];
-            int pos = t - L + 1;
-            if (score > kNegInf) {
-                if (slot < L) pos += slot;
-                else { const int r = bs_shift >= 0 ? (slot - L) >> bs_shift : (slot - L) / bs; pos = sel_s[0][3 * r] * bs + (slot - L - r * bs); }
+        // ranks among a warp's 32 candidates first, then among the warps' K best each
+        uint32_t* keys = reinterpret_cast<uint32_t*>(queries);                   // 256 words, no longer needed
+        uint32_t* kept_keys = reinterpret_cast<uint32_t*>(sel_s + 3 * kDecodeTop);       // nor are the other warps' lists
+        int* kept_slots = sel_s + 3 * kDecodeTop + kThreads;
+        const int n_kept = ((cap4 + 31) >> 5) * K;
+        const uint32_t key = tid < cap4 ? float_key(cand[tid] + 0.0f) : 1u;      // below every score's key, and not 0 (rank_among)
+        keys[tid] = key;
+        __syncwarp();
+        if (32 * warp < cap4) {
+            const int rank = rank_among<8>(keys + 32 * warp, 8, key, lane);
+            if (rank < K) {
+                kept_keys[warp * K + rank] = key;
+                kept_slots[warp * K + rank] = tid;
             }
-            out_pos[rank] = pos;
-            out_score[rank] = score;
+        }
+        if (tid < ((n_kept + 3) & ~3) - n_kept) kept_keys[n_kept + tid] = 0u;
+        __syncthreads();
+        if (tid < n_kept) {
+            const int slot = kept_slots[tid], rank = rank_among<4>(kept_keys, (n_kept + 3) >> 2, kept_keys[tid], tid);
+            if (rank < K && slot < cap) {
+                const float score = cand[slot];
+                const int r = bs_shift >= 0 ? (slot - L) >> bs_shift : (slot - L) / bs;
+                const int pos = slot < L ? t - L + 1 + slot : sel_s[3 * max(r, 0)] * bs + (slot - L - r * bs);
+                out_pos[rank] = score > kNegInf ? pos : t - L + 1;
+                out_score[rank] = score;
+            }
         }
         // more partners than candidates
         for (int k = cap + tid; k < K; k += kThreads) { out_pos[k] = t - L + 1; out_score[k] = kNegInf; }
     } else if (cap4 > 512) {
-        topk_large(cand, cap, K, L, t, bs, sel_s[0], out_pos, out_score);
+        topk_large(cand, cap, K, L, t, bs, sel_s, out_pos, out_score);
     } else if (warp == 0) {
         topk_warp(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);
     }
