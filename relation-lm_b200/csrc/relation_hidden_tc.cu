@@ -57,6 +57,7 @@ struct HiddenTcArgs {
     int rows_per_tile;      // 128 / K
     int inv_k16;            // ceil(65536 / K): r / K == (r * inv_k16) >> 16 for r < 256
     uint32_t idesc;
+    int separate;                   // gathered rows beside the tiles, not in their place (see GatherPlan)
 };
 
 struct RowUpdateArgs {
@@ -81,14 +82,18 @@ constexpr uint32_t kRowBytes = kTcBN * 2;            // one tile row of a 16-bit
 constexpr uint32_t kRowStride = kRowBytes + 16;      // padded: conflict-free 16-byte row accesses
 
 // Shared-memory plan of the gather kernel (bytes past the 1024-aligned base): the A and weight
-// tiles first; once the MMA has consumed them the same bytes hold the gathered expanded-cache
-// rows (anchor terms, then partner terms), which the epilogue overwrites with its results.
-struct GatherPlan { uint32_t partner_rows, total; };
+// tiles first, then the gathered expanded-cache rows (anchor terms, partner terms), which the epilogue
+// overwrites with its results.  Launches of several CTAs per SM keep them small: the rows take the
+// consumed tiles' bytes, and the CTAs of an SM overlap each other.  A launch of at most two per SM is one
+// chain of round trips instead, so its rows have bytes of their own and are requested together with the
+// operand rows (512 pairs, H 3072: LABELHIDDEN).
+struct GatherPlan { uint32_t rows, partner_rows, total; };
 
-__host__ __device__ inline GatherPlan gather_plan(int rdim, int rows_per_tile) {
+__host__ __device__ inline GatherPlan gather_plan(int rdim, int rows_per_tile, bool separate) {
     GatherPlan p;
     const uint32_t tile_bytes = static_cast<uint32_t>(rdim / kBK) * kBM * 128u;
-    p.partner_rows = static_cast<uint32_t>(rows_per_tile) * kRowStride;
+    p.rows = separate ? 2 * tile_bytes : 0u;
+    p.partner_rows = p.rows + static_cast<uint32_t>(rows_per_tile) * kRowStride;
     const uint32_t staged = p.partner_rows + kBM * kRowStride;
     p.total = 2 * tile_bytes > staged ? 2 * tile_bytes : staged;
     return p;
@@ -114,11 +119,11 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
 
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    const GatherPlan plan = gather_plan(R, RPT);
+    const GatherPlan plan = gather_plan(R, RPT, a.separate);
     const uint32_t tile_bytes = static_cast<uint32_t>(kblocks) * kBM * 128u;   // one 128 x R tile
     unsigned char* a_tile = base;
     unsigned char* wm_tile = a_tile + tile_bytes;
-    unsigned char* g_anchor = base;                        // after the MMA: [RPT][kRowStride] expanded[a, h0 ..]
+    unsigned char* g_anchor = base + plan.rows;            // [RPT][kRowStride] expanded[a, h0 ..]
     unsigned char* g_partner = base + plan.partner_rows;   // [128][kRowStride] expanded[p, H + h0 ..], then results
 
     const uint32_t bar_w = smem_u32(&bars[0]), bar_acc = smem_u32(&bars[1]);
@@ -158,6 +163,25 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
     }
     __syncthreads();      // also publishes the barrier initialisation
 
+    // The expanded-cache segments of the epilogue as 16-byte asynchronous copies (a warp covers two 256-byte tile rows
+    // per instruction): row j < RPT of the staging area is the anchor term of sequence j, row RPT + r the partner term
+    // of pair r.
+    const auto request_terms = [&] {
+        const int c = tid & 15, n_rows_staged = RPT + tile_pairs;
+#pragma unroll 1
+        for (int g = tid >> 4; g < n_rows_staged; g += kTcThreads / 16) {
+            const int r = g - RPT;
+            const int rb = g < RPT ? g : (r * a.inv_k16) >> 16;
+            if (row0 + rb >= a.n_rows || seq_s[rb] < 0) continue;
+            const int at = g < RPT ? idx_s[rb * (K + 1)] : idx_s[rb * (K + 1) + (r - rb * K) + 1];
+            const char* src = static_cast<const char*>(a.expanded_cache) +
+                              ((static_cast<size_t>(seq_s[rb]) * a.max_t + at) * 2 * H + (g < RPT ? 0 : H) + h0) * 2;
+            // the partner rows follow the anchor rows in shared memory
+            cp_async16(smem_u32(g_anchor) + g * kRowStride + 16 * c, src + 16 * c);
+        }
+        cp_async_commit();
+    };
+
     // A tile: the partner operand rows go straight to their swizzled places in the A tile as
     // 16-byte asynchronous copies while the anchor chunks they are multiplied with wait in
     // registers; once this thread's copies have landed it multiplies them in place (fp32).
@@ -167,6 +191,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
         constexpr int kRound = 8;
         const int rows_per_pass = kTcThreads / chunks;
         const int bc = tid % chunks, r_first = tid / chunks;
+        bool early = a.separate;
         for (int r0 = r_first < rows_per_pass ? r_first : kBM; r0 < kBM; r0 += kRound * rows_per_pass) {
             uint4 anchor_chunk[kRound];
 #pragma unroll
@@ -186,7 +211,13 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
                 }
             }
             cp_async_commit();
-            cp_async_wait_all();
+            if (early) {                                      // behind the first operand rows
+                early = false;
+                request_terms();
+                cp_async_wait_group1();
+            } else {
+                cp_async_wait_all();
+            }
 #pragma unroll
             for (int u = 0; u < kRound; ++u) {
                 const int r = r0 + u * rows_per_pass;
@@ -199,6 +230,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
                                    pack2(fp[4] * fa[4], fp[5] * fa[5], kDt), pack2(fp[6] * fa[6], fp[7] * fa[7], kDt));
             }
         }
+        if (early) request_terms();                           // a thread without operand rows
     }
     fence_proxy_async();     // generic-proxy writes of the tile -> visible to the tensor core
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -229,25 +261,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
     ready = ready && (*reinterpret_cast<volatile int*>(&failed) == 0);
     const bool staged = kOut != RLM_F32;
     if (!__syncthreads_or(!ready)) {
-    // The operand tiles are consumed: all threads request the expanded-cache segments of the
-        // epilogue into the same bytes as 16-byte asynchronous copies (a warp covers two 256-byte
-        // tile rows per instruction): row j < RPT of the staging area is the anchor term of
-        // sequence j, row RPT + r the partner term of pair r.
-            {
-            const int c = tid & 15, n_rows_staged = RPT + tile_pairs;
-#pragma unroll 1
-            for (int g = tid >> 4; g < n_rows_staged; g += kTcThreads / 16) {
-                const int r = g - RPT;
-                const int rb = g < RPT ? g : (r * a.inv_k16) >> 16;
-                if (row0 + rb >= a.n_rows || seq_s[rb] < 0) continue;
-                const int at = g < RPT ? idx_s[rb * (K + 1)] : idx_s[rb * (K + 1) + (r - rb * K) + 1];
-                const char* src = static_cast<const char*>(a.expanded_cache) +
-                                  ((static_cast<size_t>(seq_s[rb]) * a.max_t + at) * 2 * H + (g < RPT ? 0 : H) + h0) * 2;
-                // the partner rows follow the anchor rows in shared memory
-                cp_async16(smem_u32(g_anchor) + g * kRowStride + 16 * c, src + 16 * c);
-            }
-            cp_async_commit();
-        }
+        if (!a.separate) request_terms();      // the operand tiles are consumed: into their bytes
         cp_async_wait_all();
         __syncthreads();
         // This thread's share: pair row `pr`, hidden columns [h0 + 64 ch, h0 + 64 ch + 64).
@@ -714,7 +728,7 @@ __global__ void __launch_bounds__(kUpdThreads) expanded_row_update_kernel(
     if (early) griddep_sync();       // every kernel waits for its predecessor before it lets its successor go
 }
 
-size_t gather_smem_bytes(int rdim, int k_out) { return 1024 + gather_plan(rdim, kBM / k_out).total; }
+size_t gather_smem_bytes(int rdim, int k_out, bool separate) { return 1024 + gather_plan(rdim, kBM / k_out, separate).total; }
 
 size_t update_smem_bytes(int rdim, int n_seq) {
     const int n_cols = ((n_seq < kUpdMaxSeq ? n_seq : kUpdMaxSeq) + 15) & ~15;
@@ -730,7 +744,7 @@ bool hidden_tc_applicable(bool update, int n_rows, int rdim, int hdim, int k_out
     if (rdim % kBK != 0 || hdim % kTcBN != 0 || k_out < 1 || k_out > 16) return false;
     if (static_cast<long long>(n_rows) * k_out < 256) return false;    // small launches: latency-bound form
     if (!aligned16(expanded_cache) || !aligned16(out)) return false;
-    if (gather_smem_bytes(rdim, k_out) > static_cast<size_t>(kSmemDynamicLimit)) return false;
+    if (gather_smem_bytes(rdim, k_out, false) > static_cast<size_t>(kSmemDynamicLimit)) return false;
     if (update && update_smem_bytes(rdim, n_rows) > static_cast<size_t>(kSmemDynamicLimit)) return false;
     return true;
 }
@@ -817,7 +831,8 @@ int launch_hidden_tc(bool update, void* expanded_cache, const void* operand_cach
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     dim3 grid(hdim / kTcBN, row_tiles);
-    launch_kernel(kernel, dim3(grid), dim3(kTcThreads), gather_smem_bytes(rdim, k_out), stream, mm, a);
+    a.separate = static_cast<int64_t>(grid.x) * grid.y <= 2 * sm_count() && 2 * gather_smem_bytes(rdim, k_out, true) <= static_cast<size_t>(kSmemPerCta);
+    launch_kernel(kernel, dim3(grid), dim3(kTcThreads), gather_smem_bytes(rdim, k_out, a.separate), stream, mm, a);
     count_launch();
     return check_launch("relation_hidden_tc_kernel");
 }

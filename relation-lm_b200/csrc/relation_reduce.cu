@@ -673,11 +673,11 @@ __device__ __forceinline__ void norm_reduce_vec_row(const NormArgs& a, int row, 
     }
 }
 
-template <int kVecChunks, bool kPlain>
-__global__ void __launch_bounds__(kNormThreads, kVecChunks <= 2 ? 4 : (kVecChunks == 3 ? 3 : 2)) relation_norm_reduce_vec_kernel(const NormArgs a) {
+template <int kVecChunks, bool kPlain, bool kEarly = false>
+__global__ void __launch_bounds__(kNormThreads, kEarly ? 1 : kVecChunks <= 2 ? 4 : (kVecChunks == 3 ? 3 : 2)) relation_norm_reduce_vec_kernel(const NormArgs a) {
     extern __shared__ __align__(16) float partial[];   // [warps][dim]
     griddep_sync();
-    norm_reduce_vec_row<kVecChunks, false, kPlain>(a, blockIdx.x, partial, nullptr);
+    norm_reduce_vec_row<kVecChunks, kEarly, kPlain>(a, blockIdx.x, partial, nullptr);
 }
 
 // ---- thousands of rows (whole-sequence passes): a warp per row
@@ -960,7 +960,12 @@ int norm_reduce_launch(
     // the decode step's dtypes (bf16 rows in one slice, fp32 parameters) take builds without dtype branches
     const bool plain_rows = raw_dtype == RLM_BF16 && param_dtype == RLM_F32 && a.raw_splits == 1 && !raw_bias &&
                             (!next_normalized || next_dtype == RLM_BF16);
-    if (vec) {
+    if (vec && plain_rows && n_rows <= sm_count()) {
+        // a row per SM at most: a row's latency counts, so everything it needs is requested at the top
+        auto kernel = dim <= 512 ? relation_norm_reduce_vec_kernel<2, true, true> : dim <= 768 ? relation_norm_reduce_vec_kernel<3, true, true>
+                                                                                               : relation_norm_reduce_vec_kernel<4, true, true>;
+        launch_kernel(kernel, dim3(n_rows), dim3(kNormThreads), smem_bytes, stream, a);
+    } else if (vec) {
         auto kernel = dim <= 512 ? (plain_rows ? relation_norm_reduce_vec_kernel<2, true> : relation_norm_reduce_vec_kernel<2, false>)
                     : dim <= 768 ? (plain_rows ? relation_norm_reduce_vec_kernel<3, true> : relation_norm_reduce_vec_kernel<3, false>)
                                  : (plain_rows ? relation_norm_reduce_vec_kernel<4, true> : relation_norm_reduce_vec_kernel<4, false>);
