@@ -86,7 +86,7 @@ constexpr uint32_t kRowStride = kRowBytes + 16;      // padded: conflict-free 16
 // overwrites with its results.  Launches of several CTAs per SM keep them small: the rows take the
 // consumed tiles' bytes, and the CTAs of an SM overlap each other.  A launch of at most two per SM is one
 // chain of round trips instead, so its rows have bytes of their own and are requested together with the
-// operand rows (512 pairs, H 3072: LABELHIDDEN).
+// operand rows (512 pairs, H 3072, with the 512-thread build: 8.2 us of a tile's chain -> about 4).
 struct GatherPlan { uint32_t rows, partner_rows, total; };
 
 __host__ __device__ inline GatherPlan gather_plan(int rdim, int rows_per_tile, bool separate) {
@@ -100,16 +100,16 @@ __host__ __device__ inline GatherPlan gather_plan(int rdim, int rows_per_tile, b
 }
 
 // kDt: dtype of the caches and weights, kOut: dtype of the output (compile-time, so that the
-// conversions carry no branches).
-template <int kDt, int kOut>
-__global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
+// conversions carry no branches).  kThr: 256 threads, three CTAs per SM, for launches that fill the SMs; 512 for at
+// most a CTA per SM, where the tile's time is what one CTA's warps issue (gather addresses, GELU, stores).
+template <int kDt, int kOut, int kThr>
+__global__ void __launch_bounds__(kThr, kThr == kTcThreads ? 3 : 1) relation_hidden_tc_kernel(
     const __grid_constant__ CUtensorMap map_wm, const HiddenTcArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
-    __shared__ int idx_s[2 * kBM];      // [rows_per_tile][K + 1]
-    __shared__ int seq_s[kBM];
+    __shared__ int row_s[2 * kBM];      // [rows_per_tile][K + 1]: cache rows (sequence x max_t + index) of anchor and partners, -1: none
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int R = a.rdim, H = a.hdim, K = a.k_out, RPT = a.rows_per_tile;
@@ -144,22 +144,18 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
     }
 
     griddep_sync();      // weight tile requested, tensor memory allocated: now the previous kernel's outputs
-    // gathered indices of the tile's sequences
+    // gathered rows of the tile's sequences
 #pragma unroll 1
-    for (int i = tid; i < RPT * (K + 1); i += kTcThreads) {
+    for (int i = tid; i < RPT * (K + 1); i += kThr) {
         const int rb = i / (K + 1), j = i - rb * (K + 1), row = row0 + rb;
-        int v = 0;
-        if (row < a.n_rows)
-            v = j == 0 ? a.anchor_index[row] : a.partner_index[static_cast<size_t>(row) * K + j - 1];
-        idx_s[i] = min(max(v, 0), a.max_t - 1);
-        if (j == 0) {
-            int b = row < a.n_rows ? (a.row_batch ? a.row_batch[row] : row) : -1;
-            if (row < a.n_rows && (b < 0 || b >= a.n_seq)) {
-                if (a.status) atomicOr(a.status, RLM_DEV_POSITION);
-                b = -1;
-            }
-            seq_s[rb] = b;
+        int at = -1;
+        if (row < a.n_rows) {
+            const int v = j == 0 ? a.anchor_index[row] : a.partner_index[static_cast<size_t>(row) * K + j - 1];
+            const int b = a.row_batch ? a.row_batch[row] : row;
+            if (b >= 0 && b < a.n_seq) at = b * a.max_t + min(max(v, 0), a.max_t - 1);      // n_seq * max_t < 2^31
+            else if (j == 0 && a.status) atomicOr(a.status, RLM_DEV_POSITION);
         }
+        row_s[i] = at;
     }
     __syncthreads();      // also publishes the barrier initialisation
 
@@ -168,16 +164,14 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
     // of pair r.
     const auto request_terms = [&] {
         const int c = tid & 15, n_rows_staged = RPT + tile_pairs;
-#pragma unroll 1
-        for (int g = tid >> 4; g < n_rows_staged; g += kTcThreads / 16) {
-            const int r = g - RPT;
-            const int rb = g < RPT ? g : (r * a.inv_k16) >> 16;
-            if (row0 + rb >= a.n_rows || seq_s[rb] < 0) continue;
-            const int at = g < RPT ? idx_s[rb * (K + 1)] : idx_s[rb * (K + 1) + (r - rb * K) + 1];
-            const char* src = static_cast<const char*>(a.expanded_cache) +
-                              ((static_cast<size_t>(seq_s[rb]) * a.max_t + at) * 2 * H + (g < RPT ? 0 : H) + h0) * 2;
+        const char* source = static_cast<const char*>(a.expanded_cache) + 2 * h0 + 16 * c;
+        const size_t ex_row = static_cast<size_t>(H) * 4;
+#pragma unroll 3
+        for (int g = tid >> 4; g < n_rows_staged; g += kThr / 16) {
+            const int r = g - RPT, rb = g < RPT ? g : (r * a.inv_k16) >> 16;
+            const int at = row_s[rb * (K + 1) + (g < RPT ? 0 : r - rb * K + 1)];
             // the partner rows follow the anchor rows in shared memory
-            cp_async16(smem_u32(g_anchor) + g * kRowStride + 16 * c, src + 16 * c);
+            if (at >= 0) cp_async16(smem_u32(g_anchor) + g * kRowStride + 16 * c, source + at * ex_row + (g < RPT ? 0 : 2 * H));
         }
         cp_async_commit();
     };
@@ -185,27 +179,32 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
     // A tile: the partner operand rows go straight to their swizzled places in the A tile as
     // 16-byte asynchronous copies while the anchor chunks they are multiplied with wait in
     // registers; once this thread's copies have landed it multiplies them in place (fp32).
-    // A thread keeps one chunk column and walks the pair rows, eight rows per round.
+    // A thread keeps one chunk column and walks the pair rows, kRound rows per round.
     const size_t op_row = static_cast<size_t>(R) * 2;
     {
-        constexpr int kRound = 8;
-        const int rows_per_pass = kTcThreads / chunks;
+        constexpr int kRound = kThr == kTcThreads ? 8 : 4;
+        const int rows_per_pass = kThr / chunks;
         const int bc = tid % chunks, r_first = tid / chunks;
         bool early = a.separate;
         for (int r0 = r_first < rows_per_pass ? r_first : kBM; r0 < kBM; r0 += kRound * rows_per_pass) {
             uint4 anchor_chunk[kRound];
+            int anchor_row[kRound], partner_row[kRound];
+#pragma unroll
+            for (int u = 0; u < kRound; ++u) {
+                const int r = r0 + u * rows_per_pass, rb = (r * a.inv_k16) >> 16, e = r < tile_pairs ? rb * (K + 1) : 0;
+                anchor_row[u] = r < tile_pairs ? row_s[e] : -1;
+                partner_row[u] = row_s[e + (r < tile_pairs ? r - rb * K + 1 : 0)];
+            }
+            const char* operand = static_cast<const char*>(a.operand_cache) + 16 * bc;
 #pragma unroll
             for (int u = 0; u < kRound; ++u) {
                 const int r = r0 + u * rows_per_pass;
                 anchor_chunk[u] = make_uint4(0, 0, 0, 0);
                 if (r >= kBM) continue;
-                const int rb = (r * a.inv_k16) >> 16, k = r - rb * K;
                 const uint32_t dst = smem_u32(a_tile) + swizzled(r, bc, kBM * 128u);
-                if (r < tile_pairs && seq_s[rb < RPT ? rb : 0] >= 0) {
-                    const char* operand = static_cast<const char*>(a.operand_cache) +
-                                          static_cast<size_t>(seq_s[rb]) * a.max_t * op_row + 16 * bc;
-                    cp_async16(dst, operand + idx_s[rb * (K + 1) + k + 1] * op_row);
-                    anchor_chunk[u] = *reinterpret_cast<const uint4*>(operand + idx_s[rb * (K + 1)] * op_row);
+                if (anchor_row[u] >= 0) {
+                    cp_async16(dst, operand + partner_row[u] * op_row);
+                    anchor_chunk[u] = *reinterpret_cast<const uint4*>(operand + anchor_row[u] * op_row);
                 } else {
                     asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0) : "memory");
                 }
@@ -264,18 +263,19 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
         if (!a.separate) request_terms();      // the operand tiles are consumed: into their bytes
         cp_async_wait_all();
         __syncthreads();
-        // This thread's share: pair row `pr`, hidden columns [h0 + 64 ch, h0 + 64 ch + 64).
+        // This thread's share: pair row `pr`, kCols hidden columns from h0 + kCols ch on.
+        constexpr int kCols = kTcBN / (kThr / kBM);
         const int pr = 32 * (warp & 3) + lane, ch = warp >> 2;
         const int prb = (pr * a.inv_k16) >> 16;
-        const bool pair_live = pr < tile_pairs && row0 + prb < a.n_rows && seq_s[prb < RPT ? prb : 0] >= 0;
+        const bool pair_live = pr < tile_pairs && row_s[prb * (K + 1)] >= 0;
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        const unsigned char* ga = g_anchor + (prb < RPT ? prb : 0) * kRowStride + 128 * ch;
-        const unsigned char* gp = g_partner + pr * kRowStride + 128 * ch;
-        unsigned char* so = g_partner + pr * kRowStride + 128 * ch;      // results replace the partner term
+        const unsigned char* ga = g_anchor + (prb < RPT ? prb : 0) * kRowStride + 2 * kCols * ch;
+        const unsigned char* gp = g_partner + pr * kRowStride + 2 * kCols * ch;
+        unsigned char* so = g_partner + pr * kRowStride + 2 * kCols * ch;        // results replace the partner term
 #pragma unroll 1      // the body is large and runs once per warp: keep the instruction footprint small
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < kCols / 16; ++q) {
             uint32_t v[16];
-            tmem_ld16(tmem_base + lane_base + 64 * ch + 16 * q, v);
+            tmem_ld16(tmem_base + lane_base + kCols * ch + 16 * q, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (!pair_live) continue;
             float y[16];
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
                 }
             }
             if (!staged) {
-                const size_t at = (static_cast<size_t>(row0) * K + pr) * H + h0 + 64 * ch + 16 * q;
+                const size_t at = (static_cast<size_t>(row0) * K + pr) * H + h0 + kCols * ch + 16 * q;
                 float4* o = reinterpret_cast<float4*>(static_cast<float*>(a.out) + at);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) o[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
@@ -309,13 +309,13 @@ __global__ void __launch_bounds__(kTcThreads, 3) relation_hidden_tc_kernel(
             // 16-bit outputs leave row by row: a warp stores two 256-byte pair rows per instruction
             __syncthreads();
             const int c = tid & 15;
-#pragma unroll 2
-            for (int r = tid >> 4; r < tile_pairs; r += kTcThreads / 16) {
+#pragma unroll 4
+            for (int r = tid >> 4; r < tile_pairs; r += kThr / 16) {
                 const int rb = (r * a.inv_k16) >> 16;
-                if (row0 + rb >= a.n_rows || seq_s[rb] < 0) continue;
-                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) +
-                                          (static_cast<size_t>(row0) * K + r) * H + h0 + 8 * c) =
-                    *reinterpret_cast<const uint4*>(g_partner + r * kRowStride + 16 * c);
+                if (row_s[rb * (K + 1)] >= 0)
+                    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) +
+                                              (static_cast<size_t>(row0) * K + r) * H + h0 + 8 * c) =
+                        *reinterpret_cast<const uint4*>(g_partner + r * kRowStride + 16 * c);
             }
         }
     } else if (tid == 0 && a.status) {
@@ -728,6 +728,18 @@ __global__ void __launch_bounds__(kUpdThreads) expanded_row_update_kernel(
     if (early) griddep_sync();       // every kernel waits for its predecessor before it lets its successor go
 }
 
+using HiddenTcKernel = void (*)(const CUtensorMap, const HiddenTcArgs);
+
+template <int kDt, int kThr>
+HiddenTcKernel hidden_tc_kernel(int out_dtype) {
+    return out_dtype == RLM_F32 ? relation_hidden_tc_kernel<kDt, RLM_F32, kThr>
+           : out_dtype == RLM_BF16 ? relation_hidden_tc_kernel<kDt, RLM_BF16, kThr> : relation_hidden_tc_kernel<kDt, RLM_F16, kThr>;
+}
+template <int kDt>
+HiddenTcKernel hidden_tc_kernel(int out_dtype, bool few) {
+    return few ? hidden_tc_kernel<kDt, 2 * kTcThreads>(out_dtype) : hidden_tc_kernel<kDt, kTcThreads>(out_dtype);
+}
+
 size_t gather_smem_bytes(int rdim, int k_out, bool separate) { return 1024 + gather_plan(rdim, kBM / k_out, separate).total; }
 
 size_t update_smem_bytes(int rdim, int n_seq) {
@@ -802,16 +814,7 @@ int launch_hidden_tc(bool update, void* expanded_cache, const void* operand_cach
         set_error("relation_hidden: cuTensorMapEncodeTiled failed");
         return RLM_ERR_LAUNCH;
     }
-    using Kernel = void (*)(const CUtensorMap, const HiddenTcArgs);
-    Kernel kernel = nullptr;
-    if (dtype == RLM_BF16)
-        kernel = out_dtype == RLM_F32 ? relation_hidden_tc_kernel<RLM_BF16, RLM_F32>
-               : out_dtype == RLM_BF16 ? relation_hidden_tc_kernel<RLM_BF16, RLM_BF16>
-                                       : relation_hidden_tc_kernel<RLM_BF16, RLM_F16>;
-    else
-        kernel = out_dtype == RLM_F32 ? relation_hidden_tc_kernel<RLM_F16, RLM_F32>
-               : out_dtype == RLM_BF16 ? relation_hidden_tc_kernel<RLM_F16, RLM_BF16>
-                                       : relation_hidden_tc_kernel<RLM_F16, RLM_F16>;
+    using Kernel = HiddenTcKernel;
     const int row_tiles = (n_rows + a.rows_per_tile - 1) / a.rows_per_tile;
     const size_t rows_smem = 1024 + rows_plan(rdim, a.rows_per_tile).total;
     if (out_dtype != RLM_F32 && row_tiles >= 2 * sm_count() && hdim / kTcBN >= 2 &&
@@ -828,11 +831,14 @@ int launch_hidden_tc(bool update, void* expanded_cache, const void* operand_cach
         count_launch();
         return check_launch("relation_hidden_rows_kernel");
     }
+    dim3 grid(hdim / kTcBN, row_tiles);
+    const int ctas = static_cast<int>(grid.x * grid.y);
+    const bool few = ctas <= sm_count();
+    Kernel kernel = dtype == RLM_BF16 ? hidden_tc_kernel<RLM_BF16>(out_dtype, few) : hidden_tc_kernel<RLM_F16>(out_dtype, few);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
-    dim3 grid(hdim / kTcBN, row_tiles);
-    a.separate = static_cast<int64_t>(grid.x) * grid.y <= 2 * sm_count() && 2 * gather_smem_bytes(rdim, k_out, true) <= static_cast<size_t>(kSmemPerCta);
-    launch_kernel(kernel, dim3(grid), dim3(kTcThreads), gather_smem_bytes(rdim, k_out, a.separate), stream, mm, a);
+    a.separate = ctas <= 2 * sm_count() && 2 * gather_smem_bytes(rdim, k_out, true) <= static_cast<size_t>(kSmemPerCta);
+    launch_kernel(kernel, grid, dim3(few ? 2 * kTcThreads : kTcThreads), gather_smem_bytes(rdim, k_out, a.separate), stream, mm, a);
     count_launch();
     return check_launch("relation_hidden_tc_kernel");
 }
