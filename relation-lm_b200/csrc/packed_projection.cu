@@ -21,8 +21,10 @@ constexpr int kGemmThreads = 128;
 
 // Ring depth: wide tiles use three stages (96 KB) so that two CTAs share an SM and one CTA's
 // epilogue overlaps the other's main loop; narrow tiles (few rows, latency-bound) use eight so
-// that a whole K = 512 reduction is requested at once.
-__host__ __device__ constexpr int stages_for(int bn) { return bn >= 128 ? 3 : 8; }
+// that a whole K = 512 reduction is requested at once, and wide tiles of launches with at most a CTA
+// per SM six (deep): the output head of a decode batch streams its weights from DRAM, and three
+// stages in flight per SM do not cover the latency (64 x 768 x 16384 in a step: 12.8 -> 10.6 us).
+__host__ __device__ constexpr int stages_for(int bn, bool deep) { return bn < 128 ? 8 : deep ? 6 : 3; }
 
 struct GemmArgs {
     void* out;
@@ -37,7 +39,7 @@ struct GemmArgs {
     int k_splits;
 };
 
-template <int BN>
+template <int BN, bool kDeep>
 __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
     const GemmArgs a) {
@@ -46,9 +48,9 @@ __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
 
-    constexpr int kStages = stages_for(BN);
+    constexpr int kStages = stages_for(BN, kDeep);
     // one or two warps issue MMAs (K-blocks dealt round-robin into accumulators of their own, summed by
-    // the epilogue): a single thread issues a tcgen05.mma every ~60 cycles, which bounds short
+    // the epilogue): one warp issues a tcgen05.mma every ~50 cycles, which bounds short
     // K loops; tensor-memory columns = issuers * BN, at least 32
     const int issuers = a.issuers;
     uint32_t tmem_cols = 32;
@@ -113,8 +115,8 @@ __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
     } else if (warp <= issuers) {
         const int me = warp - 1;                              // issuer index: K-blocks me, me + issuers, ...
         const uint32_t my_acc = tmem_base + static_cast<uint32_t>(me * BN);
-        // tensor-core issue: four UMMA K-steps of 16 per stage.  The whole warp walks the loop so
-        // that addresses and descriptors stay warp-uniform; one lane issues the instructions.
+        // tensor-core issue: four UMMA K-steps of 16 per stage
+        const bool elected = elect_lane();
         bool ok = true;
         for (int it = me; it < k_iters && ok; it += issuers) {
             const int s = it % kStages;
@@ -124,18 +126,14 @@ __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t da = smem_desc_sw128(ring_addr + s * (kABytes + kBBytes));
             const uint64_t db = smem_desc_sw128(ring_addr + s * (kABytes + kBBytes) + kABytes);
-            if (lane == 0) {
 #pragma unroll
-                for (int kk = 0; kk < kBK / 16; ++kk)      // +32 bytes along K inside the swizzle atom
-                    umma_f16(my_acc, da + 2 * kk, db + 2 * kk, a.idesc, (it >= issuers || kk > 0) ? 1u : 0u);
-                umma_commit(empty(s));                       // stage reusable once these MMAs retire
-            }
-            __syncwarp();
+            for (int kk = 0; kk < kBK / 16; ++kk)          // +32 bytes along K inside the swizzle atom
+                umma_f16_if(my_acc, da + 2 * kk, db + 2 * kk, a.idesc, (it >= issuers || kk > 0) ? 1u : 0u, elected);
+            umma_commit_if(empty(s), elected);               // stage reusable once these MMAs retire
         }
-        if (lane == 0) {
-            if (!ok) failed = 1;
-            umma_commit(acc_full);                           // accumulator complete (or abandoned)
-        }
+        if (lane == 0 && !ok) failed = 1;
+        __syncwarp();
+        umma_commit_if(acc_full, elected);                   // accumulator complete (or abandoned)
     }
     __syncwarp();
 
@@ -732,10 +730,10 @@ void launch_norm_cast(const NormCastArgs& a, void* stream) {
     }
 }
 
-template <int BN>
+template <int BN, bool kDeep = false>
 int launch_gemm(const CUtensorMap& mx, const CUtensorMap& mw, const GemmArgs& a, void* stream) {
-    const int smem_bytes = stages_for(BN) * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
-    auto kernel = packed_projection_kernel<BN>;
+    const int smem_bytes = stages_for(BN, kDeep) * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
+    auto kernel = packed_projection_kernel<BN, kDeep>;
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     dim3 grid(a.n / BN, (a.m + kBM - 1) / kBM, a.k_splits);
@@ -906,17 +904,18 @@ extern "C" int rlm_packed_projection(const void* x, int64_t x_row_stride, const 
     GemmArgs a{};
     a.out = out; a.bias = bias; a.status = status; a.m = rows; a.n = n_out; a.k = d_in; a.out_dtype = out_dtype;
     a.a_bytes = static_cast<uint32_t>(box_rows) * kBK * 2;
-    // a single thread issues one tcgen05.mma per ~60 cycles, more than a 128-wide MMA runs: two warps issue
+    // one warp issues a tcgen05.mma per ~50 cycles, more than a narrow one runs: two warps issue those
     const int k_blocks = ((d_in + kBK - 1) / kBK) / k_splits;
     a.k_blocks_per_split = k_blocks;
     a.k_splits = k_splits;
     // (with an even ring depth each issuer owns its own stages, so every stage barrier is consumed in order)
-    a.issuers = (k_blocks >= 2 && stages_for(bn) % 2 == 0) ? 2 : 1;
+    a.issuers = k_blocks >= 2 && bn < 128 ? 2 : 1;
     const uint32_t fmt = in_dtype == RLM_BF16 ? 1u : 0u;
     a.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(bn >> 3) << 17) |
               (static_cast<uint32_t>(kBM >> 4) << 24);
     if (bn == 32) return launch_gemm<32>(mx, mw, a, stream);
     if (bn == 64) return launch_gemm<64>(mx, mw, a, stream);
-    return launch_gemm<128>(mx, mw, a, stream);
+    const bool deep = n_out / 128 * m_tiles * k_splits <= sm_count() && k_blocks > stages_for(128, false);
+    return deep ? launch_gemm<128, true>(mx, mw, a, stream) : launch_gemm<128>(mx, mw, a, stream);
 }
 

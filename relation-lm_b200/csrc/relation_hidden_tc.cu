@@ -693,11 +693,11 @@ __global__ void __launch_bounds__(kUpdThreads) expanded_row_update_kernel(
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     ready = ready && (*reinterpret_cast<volatile int*>(&failed) == 0);
     if (!__syncthreads_or(!ready)) {
-        // this thread owns hidden column h0 + tid of the half: one 2-byte store per sequence,
-        // a warp's 32 stores of one sequence are 64 contiguous bytes of its cache row
+        // this thread owns hidden column h0 + tid of the half: its values of all sequences are laid out as rows in the
+        // consumed tiles' place, and leave 256 contiguous bytes of a cache row per half-warp (as one 2-byte store per
+        // sequence they took most of the launch: 20 us for 12 layers x 64 sequences of H 3072, now 17)
         const float bias = half == 0 ? load_scalar(a.first_bias, static_cast<int64_t>(layer) * H + h0 + tid, a.dtype) : 0.0f;
         const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;
-        uint16_t* cache = static_cast<uint16_t*>(a.expanded_cache);
         for (int c = 0; c < n_cols; c += 16) {
             uint32_t v[16];
             tmem_ld16(tmem_base + lane_base + c, v);
@@ -714,9 +714,16 @@ __global__ void __launch_bounds__(kUpdThreads) expanded_row_update_kernel(
                     __half hv = __float2half_rn(val);
                     bits = *reinterpret_cast<uint16_t*>(&hv);
                 }
-                cache[((static_cast<size_t>(layer) * a.n_seq + s0 + c + j) * a.max_t + t) * 2 * H + half * H + h0 + tid] = bits;
+                *reinterpret_cast<uint16_t*>(base + (c + j) * kRowStride + 2 * tid) = bits;
             }
         }
+        __syncthreads();
+        const int c = tid & 15;
+        char* cache = static_cast<char*>(a.expanded_cache) + 2 * (half * H + h0) + 16 * c;
+#pragma unroll 4
+        for (int j = tid >> 4; j < n_here; j += kUpdThreads / 16)
+            *reinterpret_cast<uint4*>(cache + ((static_cast<size_t>(layer) * a.n_seq + s0 + j) * a.max_t + t) * (4 * static_cast<size_t>(H))) =
+                *reinterpret_cast<const uint4*>(base + j * kRowStride + 16 * c);
     } else if (tid == 0 && a.status) {
         atomicOr(a.status, RLM_DEV_TIMEOUT);
     }

@@ -150,35 +150,6 @@ __device__ __forceinline__ float2 lt_moments4(const float (&x)[4]) {
     return make_float2(mean, m2);
 }
 
-// MMAs are issued by a whole warp, each instruction predicated on one elected lane: inside an `if (tid == 0)` every
-// descriptor is moved from vector to uniform registers one instruction at a time, 85 cycles an MMA where the operands
-// stream in 32.
-__device__ __forceinline__ bool lt_elect() {
-    uint32_t p;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
-    return p != 0;
-}
-__device__ __forceinline__ void lt_umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
-                                        bool issue) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "setp.ne.b32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
-}
-__device__ __forceinline__ void lt_commit(uint32_t bar, bool issue) {
-    asm volatile(
-        "{\n"
-        ".reg .pred q;\n"
-        "setp.ne.b32 q, %1, 0;\n"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-        "}\n"
-        ::"r"(bar), "r"(static_cast<uint32_t>(issue)) : "memory");
-}
-
 __device__ __forceinline__ void lt_tmem_ld4(uint32_t addr, uint32_t (&v)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
@@ -400,7 +371,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     // ---- product GEMM: D1[hidden column, pair] = W_m slice x products^T
     if (warp == 0) {
-        const bool ok = mbar_wait(bar_wm, 0), issue = lt_elect();
+        const bool ok = mbar_wait(bar_wm, 0), issue = elect_lane();
         if (!ok) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int kb = 0; kb < kblocks; ++kb) {
@@ -408,9 +379,9 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             const uint64_t dp = smem_desc_sw128(smem_u32(p_tile) + kb * p_kblock);
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
-                lt_umma(tmem_base, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+                umma_f16_if(tmem_base, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
         }
-        lt_commit(bar_d1, issue);
+        umma_commit_if(bar_d1, issue);
     }
     __syncwarp();
     if (!mbar_wait(bar_d1, 0)) failed = 1;
@@ -457,7 +428,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // ---- second GEMM, split over the cluster along the hidden width:
     // D2[output row, pair] (partial) = W_2[:, this CTA's hidden columns] x hidden slice^T
     if (warp == 0) {
-        const bool ok = mbar_wait(bar_w2, 0), issue = lt_elect();
+        const bool ok = mbar_wait(bar_w2, 0), issue = elect_lane();
         if (!ok) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int mt = 0; mt < mtiles; ++mt) {
@@ -467,10 +438,10 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 const uint64_t dh = smem_desc_sw128(smem_u32(hid_tile) + kb * p_kblock);
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; ++kk)
-                    lt_umma(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
+                    umma_f16_if(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
                             (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
             }
-            lt_commit(bar_d2 + 8u * mt, issue);                // each tile's partial sums leave while the next is computed
+            umma_commit_if(bar_d2 + 8u * mt, issue);                // each tile's partial sums leave while the next is computed
         }
     }
     __syncwarp();

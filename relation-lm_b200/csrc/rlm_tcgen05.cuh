@@ -48,6 +48,35 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                  ::"r"(bar) : "memory");
 }
 
+// MMAs are issued by a whole warp, each instruction predicated on one elected lane: inside an `if (tid == 0)` every
+// descriptor is moved from vector to uniform registers one instruction at a time, 85 cycles an MMA where the operands
+// stream in 32.
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void umma_f16_if(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate, bool issue) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue)) : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t bar, bool issue) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "setp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n"
+        ::"r"(bar), "r"(static_cast<uint32_t>(issue)) : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
