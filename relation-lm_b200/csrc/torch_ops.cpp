@@ -8,11 +8,18 @@
 // operators the reference project defines (src/relation_lm/kernels/relation_select.py:311,
 // triton_select.py:255-298, router_cache.py:175, relation_reduce.py:149-420) and this library's
 // extensions.  Fake implementations and documentation stay in the Python modules.
+#include <torch/csrc/python_headers.h>
+
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/record_function.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
 #include <initializer_list>
@@ -1079,3 +1086,159 @@ TORCH_LIBRARY_IMPL(relation_lm, ADInplaceOrView, m) { FOR_EACH_OP(NOTHING, BUMP_
 TORCH_LIBRARY_FRAGMENT(relationlex, m) { FOR_EACH_LEX_OP(DEFINE) }
 TORCH_LIBRARY_IMPL(relationlex, CUDA, m) { FOR_EACH_LEX_OP(IMPLEMENT) }
 TORCH_LIBRARY_IMPL(relationlex, Autograd, m) { FOR_EACH_LEX_OP(NO_DERIVATIVE) }
+
+// ------------------------------------------------------------------ direct calls from Python
+//
+// An operator call through the dispatcher costs the host 2-4 us (boxing twenty arguments, the autograd and
+// version-counter fallbacks), as much as its launch, and the passes of a small model are bound by exactly that.
+// Each operator is therefore a plain extension function too.  It returns NotImplemented, and the caller takes the
+// dispatcher, whenever the dispatcher would have anything to do: arguments that are not plain CUDA tensors, a
+// derivative to record, a mode, a tracer, a transform or a profiler at work.
+namespace {
+
+using c10::DispatchKey;
+using c10::DispatchKeySet;
+
+constexpr DispatchKeySet kInterposing({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::PythonDispatcher,
+                                       DispatchKey::PreDispatch, DispatchKey::Functionalize, DispatchKey::Tracer,
+                                       DispatchKey::Batched, DispatchKey::VmapMode, DispatchKey::FuncTorchBatched,
+                                       DispatchKey::FuncTorchVmapMode, DispatchKey::FuncTorchGradWrapper,
+                                       DispatchKey::FuncTorchDynamicLayerFrontMode, DispatchKey::FuncTorchDynamicLayerBackMode,
+                                       DispatchKey::FuncTorchBatchedDecomposition, DispatchKey::TESTING_ONLY_GenericWrapper,
+                                       DispatchKey::TESTING_ONLY_GenericMode});
+
+bool nothing_interposed() {
+    return !c10::impl::tls_local_dispatch_key_set().included_.has_any(kInterposing) && !at::impl::torch_function_mode_enabled() &&
+           !at::hasThreadLocalCallbacks() && !at::hasGlobalCallbacks();
+}
+
+const Tensor* plain_tensor(PyObject* o, bool grad) {
+    if (!THPVariable_CheckExact(o)) return nullptr;
+    const Tensor& t = THPVariable_Unpack(o);
+    if (!t.is_cuda() || t.key_set().has_any(kInterposing) || t.is_inference() || (grad && t.requires_grad())) return nullptr;
+    return &t;
+}
+
+// An argument on its way from Python: load() says whether it is of the plain kind.
+template <typename T> struct Arg;
+template <> struct Arg<const Tensor&> {
+    const Tensor* t;
+    bool load(PyObject* o, bool grad) { return (t = plain_tensor(o, grad)) != nullptr; }
+    const Tensor& get() { return *t; }
+    void written() {}
+};
+template <> struct Arg<Tensor&> {
+    Tensor t;
+    bool load(PyObject* o, bool grad) {
+        const Tensor* p = plain_tensor(o, grad);
+        if (p) t = *p;
+        return p != nullptr;
+    }
+    Tensor& get() { return t; }
+    void written() { t.unsafeGetTensorImpl()->bump_version(); }
+};
+template <> struct Arg<const OptTensor&> {
+    OptTensor t;
+    bool load(PyObject* o, bool grad) {
+        if (o == Py_None) return true;
+        const Tensor* p = plain_tensor(o, grad);
+        if (p) t = *p;
+        return p != nullptr;
+    }
+    const OptTensor& get() { return t; }
+    void written() {}
+};
+template <> struct Arg<int64_t> {
+    int64_t v;
+    bool load(PyObject* o, bool) {
+        if (!PyLong_CheckExact(o)) return false;
+        v = PyLong_AsLongLong(o);
+        if (v != -1 || !PyErr_Occurred()) return true;
+        PyErr_Clear();
+        return false;
+    }
+    int64_t get() { return v; }
+    void written() {}
+};
+template <> struct Arg<double> {
+    double v;
+    bool load(PyObject* o, bool) {
+        if (!PyFloat_CheckExact(o)) return false;
+        v = PyFloat_AS_DOUBLE(o);
+        return true;
+    }
+    double get() { return v; }
+    void written() {}
+};
+template <> struct Arg<bool> {
+    bool v;
+    bool load(PyObject* o, bool) {
+        v = o == Py_True;
+        return v || o == Py_False;
+    }
+    bool get() { return v; }
+    void written() {}
+};
+
+PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+PyObject* wrap(const std::vector<Tensor>& ts) {
+    PyObject* list = PyList_New(static_cast<Py_ssize_t>(ts.size()));
+    for (size_t i = 0; list && i < ts.size(); ++i) PyList_SET_ITEM(list, static_cast<Py_ssize_t>(i), THPVariable_Wrap(ts[i]));
+    return list;
+}
+template <typename... T>
+PyObject* wrap(const std::tuple<T...>& ts) {
+    PyObject* tuple = PyTuple_New(sizeof...(T));
+    Py_ssize_t i = 0;
+    if (tuple) std::apply([&](const auto&... t) { (PyTuple_SET_ITEM(tuple, i++, wrap(t)), ...); }, ts);
+    return tuple;
+}
+
+template <typename R, typename... A, size_t... I>
+PyObject* call_direct(R (*function)(A...), PyObject* const* args, std::index_sequence<I...>) {
+    const bool grad = at::GradMode::is_enabled();
+    std::tuple<Arg<A>...> loaded;
+    if (!(std::get<I>(loaded).load(args[I], grad) && ...)) Py_RETURN_NOTIMPLEMENTED;
+    if constexpr (std::is_void_v<R>) {
+        {
+            pybind11::gil_scoped_release no_gil;
+            function(std::get<I>(loaded).get()...);
+        }
+        (std::get<I>(loaded).written(), ...);
+        Py_RETURN_NONE;
+    } else {
+        std::optional<R> result;
+        {
+            pybind11::gil_scoped_release no_gil;
+            result.emplace(function(std::get<I>(loaded).get()...));
+        }
+        (std::get<I>(loaded).written(), ...);
+        return wrap(*result);
+    }
+}
+template <typename R, typename... A>
+PyObject* call_checked(R (*function)(A...), PyObject* const* args, Py_ssize_t n) {
+    if (n != static_cast<Py_ssize_t>(sizeof...(A)) || !nothing_interposed()) Py_RETURN_NOTIMPLEMENTED;
+    return call_direct(function, args, std::index_sequence_for<A...>{});
+}
+template <auto kFunction>
+PyObject* direct(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    return call_checked(kFunction, args, n);
+    END_HANDLE_TH_ERRORS
+}
+
+#define METHOD(name) \
+    {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct<&name>)), METH_FASTCALL, nullptr}
+PyMethodDef kMethods[] = {METHOD(relation_select_packed), METHOD(relation_select_packed_rows), METHOD(relation_select_packed_prefill),
+                          METHOD(relation_select_multi_prefill_scores), METHOD(router_cache_update), METHOD(sparse_cache_append),
+                          METHOD(sequence_state), METHOD(relation_hidden_cached), METHOD(relation_hidden_cached_out),
+                          METHOD(relation_hidden_cache_update), METHOD(relation_hidden_cache_update_out),
+                          METHOD(relation_norm_reduce), METHOD(relation_norm_reduce_residual_norm), METHOD(relation_mlp_rows),
+                          METHOD(packed_projection), METHOD(layer_norm_cast), METHOD(decode_embed_norm),
+                          {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "librelation_lm_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit_librelation_lm_torch() { return PyModule_Create(&kModule); }

@@ -5,12 +5,23 @@ Names, field order and validation follow the reference project's
 """
 from __future__ import annotations
 
+import functools
 from collections.abc import Sequence
 from dataclasses import dataclass
 
 import torch
 import torch.nn.functional as F
 from torch import Tensor
+
+_TENSOR_CORE = (torch.bfloat16, torch.float16)
+
+
+@functools.cache
+def _kernel():
+    from relation_lm.kernels.packed_projection import packed_projection      # loads the native library
+
+    return packed_projection
+
 
 SPARSE_CACHE_NAMES = (
     "anchor_key",
@@ -52,21 +63,21 @@ class PackedSparseCacheProjection:
     def project(self, memory: Tensor) -> tuple[Tensor, ...]:
         """Project ``memory [..., d]``; the pieces come back in ``names`` order as views of
         one packed result (so the router slices keep the packed row stride)."""
-        if memory.size(-1) != self.input_width:
+        weight = self.weight
+        if memory.size(-1) != weight.size(1):
             raise ValueError("memory width does not match packed projection input")
-        if memory.is_cuda and memory.dtype in (torch.bfloat16, torch.float16) \
-                and self.weight.dtype == memory.dtype and self.output_width % 32 == 0 \
-                and self.input_width % 8 == 0:
+        if memory.is_cuda and memory.dtype in _TENSOR_CORE and weight.dtype == memory.dtype \
+                and weight.size(0) % 32 == 0 and weight.size(1) % 8 == 0:
             # tensor-core kernel of this library (tcgen05); fp32 operands use the library GEMM
-            from relation_lm.kernels.packed_projection import packed_projection
-
-            rows = memory.reshape(-1, self.input_width) if memory.dim() != 2 else memory
+            rows = memory if memory.dim() == 2 else memory.reshape(-1, weight.size(1))
             if rows.stride(-1) != 1 or rows.stride(0) % 8 != 0:
                 rows = rows.contiguous()
-            packed = packed_projection(rows, self.weight).view(*memory.shape[:-1], self.output_width)
+            packed = _kernel()(rows, weight)
+            if memory.dim() != 2:
+                packed = packed.view(*memory.shape[:-1], weight.size(0))
         else:
-            packed = F.linear(memory, self.weight)
-        return packed.split(self.split_sizes, dim=-1)
+            packed = F.linear(memory, weight)
+        return packed.split_with_sizes(self.split_sizes, dim=-1)
 
     def project_dict(self, memory: Tensor) -> dict[str, Tensor]:
         return dict(zip(self.names, self.project(memory), strict=True))

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.util
 from pathlib import Path
 
 import torch
@@ -84,6 +85,25 @@ def _load() -> ctypes.CDLL:
 
 LIB = _load()
 torch.ops.load_library(str(_OPS_PATH))
+_DIRECT = importlib.util.module_from_spec(importlib.util.spec_from_file_location(_OPS_PATH.stem, _OPS_PATH))
+
+
+def operator(name: str):
+    """``torch.ops.relation_lm.<name>``, called without the dispatcher where that would have nothing to do (plain
+    CUDA tensors, no derivative, mode, tracer or transform): 2-4 us of host time less per call."""
+    op = getattr(torch.ops.relation_lm, name).default
+    direct = getattr(_DIRECT, name, None)
+    if direct is None:
+        return op
+
+    def call(*args):
+        if not torch.compiler.is_compiling():
+            out = direct(*args)
+            if out is not NotImplemented:
+                return out
+        return op(*args)
+
+    return call
 
 _STATUS: dict[int, torch.Tensor] = {}
 

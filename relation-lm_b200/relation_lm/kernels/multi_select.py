@@ -23,11 +23,11 @@ from torch import Tensor
 from relation_lm.kernels import _abi  # noqa: F401  (loads the libraries)
 
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
-_relation_select_multi_rows = torch.ops.relation_lm.relation_select_multi_rows.default
-_relation_select_multi_prefill = torch.ops.relation_lm.relation_select_multi_prefill.default
+_relation_select_multi_rows = _abi.operator("relation_select_multi_rows")
+_relation_select_multi_prefill = _abi.operator("relation_select_multi_prefill")
 # the same without its last output (the partners' activity)
-relation_select_multi_prefill_scores = torch.ops.relation_lm.relation_select_multi_prefill_scores.default
-_slot_mix_residual = torch.ops.relation_lm.slot_mix_residual.default
+relation_select_multi_prefill_scores = _abi.operator("relation_select_multi_prefill_scores")
+_slot_mix_residual = _abi.operator("slot_mix_residual")
 
 
 def relation_select_multi_rows(

@@ -14,14 +14,14 @@ from torch import Tensor
 from relation_lm.kernels import _abi
 
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
-_packed_projection = torch.ops.relation_lm.packed_projection.default
-_layer_norm_cast = torch.ops.relation_lm.layer_norm_cast.default
-_decode_embed_norm = torch.ops.relation_lm.decode_embed_norm.default
-_decode_front = torch.ops.relation_lm.decode_front.default
-_greedy_token = torch.ops.relation_lm.greedy_token.default
-_skinny_projection = torch.ops.relation_lm.skinny_projection.default
-_skinny_projection_greedy = torch.ops.relation_lm.skinny_projection_greedy.default
-_skinny_projection_greedy_into = torch.ops.relation_lm.skinny_projection_greedy_into.default
+_packed_projection = _abi.operator("packed_projection")
+_layer_norm_cast = _abi.operator("layer_norm_cast")
+_decode_embed_norm = _abi.operator("decode_embed_norm")
+_decode_front = _abi.operator("decode_front")
+_greedy_token = _abi.operator("greedy_token")
+_skinny_projection = _abi.operator("skinny_projection")
+_skinny_projection_greedy = _abi.operator("skinny_projection_greedy")
+_skinny_projection_greedy_into = _abi.operator("skinny_projection_greedy_into")
 
 _FUSED_NORM_ROWS = 16    # beyond this many rows normalising once beats normalising in every column tile
 

@@ -16,21 +16,21 @@ from torch import Tensor
 from relation_lm.kernels import _abi
 
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
-_relation_hidden_cached = torch.ops.relation_lm.relation_hidden_cached.default
-_relation_hidden_cached_out = torch.ops.relation_lm.relation_hidden_cached_out.default
-_expanded_cache_append = torch.ops.relation_lm.expanded_cache_append.default
-_expanded_cache_append_packed = torch.ops.relation_lm.expanded_cache_append_packed.default
-_relation_hidden_cache_update = torch.ops.relation_lm.relation_hidden_cache_update.default
-_relation_norm_reduce = torch.ops.relation_lm.relation_norm_reduce.default
-_relation_hidden_cache_update_out = torch.ops.relation_lm.relation_hidden_cache_update_out.default
-_relation_norm_reduce_residual = torch.ops.relation_lm.relation_norm_reduce_residual.default
-_relation_norm_reduce_residual_norm_project = torch.ops.relation_lm.relation_norm_reduce_residual_norm_project.default
-_relation_norm_reduce_residual_norm = torch.ops.relation_lm.relation_norm_reduce_residual_norm.default
-_relation_hidden_cached_rows = torch.ops.relation_lm.relation_hidden_cached_rows.default
-_relation_hidden_cached_rows_out = torch.ops.relation_lm.relation_hidden_cached_rows_out.default
-_relation_norm_reduce_rows = torch.ops.relation_lm.relation_norm_reduce_rows.default
-_relation_mlp_rows = torch.ops.relation_lm.relation_mlp_rows.default
-_relation_layer_tail = torch.ops.relation_lm.relation_layer_tail.default
+_relation_hidden_cached = _abi.operator("relation_hidden_cached")
+_relation_hidden_cached_out = _abi.operator("relation_hidden_cached_out")
+_expanded_cache_append = _abi.operator("expanded_cache_append")
+_expanded_cache_append_packed = _abi.operator("expanded_cache_append_packed")
+_relation_hidden_cache_update = _abi.operator("relation_hidden_cache_update")
+_relation_norm_reduce = _abi.operator("relation_norm_reduce")
+_relation_hidden_cache_update_out = _abi.operator("relation_hidden_cache_update_out")
+_relation_norm_reduce_residual = _abi.operator("relation_norm_reduce_residual")
+_relation_norm_reduce_residual_norm_project = _abi.operator("relation_norm_reduce_residual_norm_project")
+_relation_norm_reduce_residual_norm = _abi.operator("relation_norm_reduce_residual_norm")
+_relation_hidden_cached_rows = _abi.operator("relation_hidden_cached_rows")
+_relation_hidden_cached_rows_out = _abi.operator("relation_hidden_cached_rows_out")
+_relation_norm_reduce_rows = _abi.operator("relation_norm_reduce_rows")
+_relation_mlp_rows = _abi.operator("relation_mlp_rows")
+_relation_layer_tail = _abi.operator("relation_layer_tail")
 
 
 @dataclass(frozen=True)

@@ -15,9 +15,9 @@ from torch import Tensor
 from relation_lm.kernels import _abi  # noqa: F401  (loads the libraries)
 
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
-_relation_select_packed = torch.ops.relation_lm.relation_select_packed.default
-_relation_select_packed_rows = torch.ops.relation_lm.relation_select_packed_rows.default
-_relation_select_packed_prefill = torch.ops.relation_lm.relation_select_packed_prefill.default
+_relation_select_packed = _abi.operator("relation_select_packed")
+_relation_select_packed_rows = _abi.operator("relation_select_packed_rows")
+_relation_select_packed_prefill = _abi.operator("relation_select_packed_prefill")
 
 
 def relation_select_packed(

@@ -12,10 +12,10 @@ from torch import Tensor
 from relation_lm.kernels import _abi
 
 # The operators themselves are registered by csrc/torch_ops.cpp; the functions below document them.
-_router_cache_update = torch.ops.relation_lm.router_cache_update.default
-_sparse_cache_append = torch.ops.relation_lm.sparse_cache_append.default
-_sequence_state = torch.ops.relation_lm.sequence_state.default
-_router_cache_prefill = torch.ops.relation_lm.router_cache_prefill.default
+_router_cache_update = _abi.operator("router_cache_update")
+_sparse_cache_append = _abi.operator("sparse_cache_append")
+_sequence_state = _abi.operator("sequence_state")
+_router_cache_prefill = _abi.operator("router_cache_prefill")
 
 _MUTATED = ("anchor_raw_cache", "partner_raw_cache", "anchor_conv_cache", "partner_conv_cache",
             "anchor_mean", "anchor_std", "partner_mean", "partner_std")
