@@ -819,7 +819,7 @@ def run_prefill(args) -> None:
     from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
     from relation_lm.kernels import _abi
     from relation_lm.kernels.packed_projection import packed_projection
-    from relation_lm.kernels.relation_reduce import relation_hidden_cached_rows_out, relation_norm_reduce_rows
+    from relation_lm.kernels.relation_reduce import relation_hidden_cached_rows_out, relation_mlp_rows, relation_norm_reduce_rows
     from relation_lm.kernels.relation_select import relation_select_packed_prefill, relation_select_packed_rows
 
     rank = int(os.environ.get("RANK", "0"))
@@ -860,7 +860,10 @@ def run_prefill(args) -> None:
     layer.build_state(x)                                     # warm-up of every kernel of the build
     build_ms, state = timed(lambda: layer.build_state(x))
     flush = torch.empty(256 * 1024 * 1024, dtype=torch.uint8, device=device)
-    for _ in range(max(3, args.warmup)):
+    launches_before = _abi.launch_count()
+    layer.forward(x, state)
+    launches = _abi.launch_count() - launches_before
+    for _ in range(max(3, args.warmup) - 1):
         layer.forward(x, state)
     sampler = ClockSampler(local) if rank == 0 else None
     barrier()
@@ -896,6 +899,7 @@ def run_prefill(args) -> None:
         w = layer.w
         q, rb, rp = keep["query"], keep["row_batch"], keep["row_position"]
         hidden_rel = torch.empty(N, K, H, device=device, dtype=torch.bfloat16)
+        mlp_out = torch.empty(N, d, device=device, dtype=torch.float32)
         select_args = (q[:, 0:64], state["anchor_keys"], q[:, 64:128], state["anchor_mean"], state["anchor_std"],
                        w["anchor_gamma"], w["anchor_bias"], q[:, 128:256], state["partner_anchor_cache"],
                        state["partner_keys"], state["partner_mean"], state["partner_std"], w["partner_gamma"],
@@ -905,6 +909,10 @@ def run_prefill(args) -> None:
                 *select_args, T, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid),
             "relation_select_kernel(rows)": lambda: relation_select_packed_rows(
                 *select_args, rb, rp, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid),
+            "relation_mlp_rows_kernel": lambda: relation_mlp_rows(
+                mlp_out, state["expanded_cache"], state["operand_cache"], keep["anchor"], keep["partner"], keep["partner_score"],
+                None, None, w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"],
+                cfg.norm_eps, x.view(N, d), 1, T, True),
             "relation_hidden_tc_kernel(rows)": lambda: relation_hidden_cached_rows_out(
                 hidden_rel, state["expanded_cache"], state["operand_cache"], keep["anchor"], keep["partner"],
                 w["product_weight"], rb),
@@ -934,11 +942,15 @@ def run_prefill(args) -> None:
                 compulsory_bytes=compulsory, logical_bytes=logical, fp32_flops=flops,
                 compulsory_gb_per_s=compulsory / us / 1e3, logical_gb_per_s=logical / us / 1e3,
                 tflops=flops / us / 1e6, frac_of_fp32_fma_peak=flops / us / 1e6 / fma_peak)
-        kernels["relation_select_kernel(rows)"]["note"] = "the per-row form, not on the pass's path: timed for comparison"
+        off_path = ("relation_select_kernel(rows)", "relation_hidden_tc_kernel(rows)", "packed_projection_kernel(second layer)",
+                    "relation_norm_reduce_kernel(rows)")
+        for name in off_path:
+            kernels[name]["note"] = "not on the pass's path: timed for comparison"
+        kernels["relation_mlp_rows_kernel"]["tflops"] = 2 * N * K * H * (cfg.relation_dim + d) / kernels["relation_mlp_rows_kernel"]["us_per_launch"] / 1e6
         sel_us = kernels["relation_select_tile_kernel"]["us_per_launch"]
         kernels["relation_hidden_tc_kernel(rows)"]["tflops"] = 2 * N * K * cfg.relation_dim * H / kernels["relation_hidden_tc_kernel(rows)"]["us_per_launch"] / 1e6
         kernels["packed_projection_kernel(second layer)"]["tflops"] = 2 * N * K * H * d / kernels["packed_projection_kernel(second layer)"]["us_per_launch"] / 1e6
-        dominant = max((k for k in kernels if k != "relation_select_kernel(rows)"), key=lambda k: kernels[k]["us_per_launch"])
+        dominant = max((k for k in kernels if k not in off_path), key=lambda k: kernels[k]["us_per_launch"])
         line = {
             "metric": "relation prefill tokens/s at ctx4096 K=8", "value": world * N * args.steps / (total_ms / 1e3),
             "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": max(3, args.warmup),
@@ -950,7 +962,7 @@ def run_prefill(args) -> None:
                        "l2": "flushed between steps", "state_build_ms": build_ms},
             "e2e": {"value": world * N * e2e_steps / (e2e_ms / 1e3), "unit": UNIT,
                     "h2d_bytes_per_step": N * d * 4, "d2h_bytes_per_step": N * d * 4, "steps": e2e_steps},
-            "gpu_launches": 6 * args.steps, "clocks": clocks, "kernels": kernels,
+            "gpu_launches": launches * args.steps, "launches_per_step": launches, "clocks": clocks, "kernels": kernels,
             "roofline": {"kernel": "relation_select_tile_kernel", "bound": "hbm", "achieved": compulsory / sel_us / 1e3,
                          "peak": peak, "unit": "GB/s", "frac": compulsory / sel_us / 1e3 / peak,
                          "peak_source": "measured" if peaks else "fallback", "traffic": None,
