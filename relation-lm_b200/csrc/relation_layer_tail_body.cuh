@@ -197,8 +197,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(pairs_pad >> 3) << 17) |
                            (static_cast<uint32_t>(kBM >> 4) << 24);
 
-    unsigned char* base = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* base = smem_align1024(lt_smem_raw);
     const int nq_own = a.query_weight ? a.n_query / C : 0;
     const LtPlan plan = lt_plan(R, D, pairs_pad, nq_own);
     unsigned char* wm_tile = base + plan.wm;

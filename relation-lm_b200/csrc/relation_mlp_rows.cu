@@ -394,8 +394,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
     const int n_super = (a.n_tiles + kG - 1) / kG;
     const int anchors = kBM >> a.k_shift, sel_k = kG * anchors;                      // anchors of a tile, of the pair
 
-    unsigned char* base = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* base = smem_align1024(smem_raw);
     const MlpPlan plan = mlp_plan(R, NC, C, wide, a.term_stages, a.wm_stages, a.w2_stages, a.k_shift);
     const uint32_t s_a = smem_u32(base + plan.a), s_wm = smem_u32(base + plan.wm), s_w2 = smem_u32(base + plan.w2);
     const uint32_t s_hid = smem_u32(base + plan.hid), s_term = smem_u32(base + plan.term), s_anc = smem_u32(base + plan.anc);
@@ -486,10 +485,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         const int row = 32 * (warp & 3) + lane, turn = warp >> 3, half = (warp >> 2) & 1;
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
         unsigned char* block = base + plan.hid + static_cast<uint32_t>(turn * C + o) * kMlpBlock;
-        uint4* cell[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            cell[c] = reinterpret_cast<uint4*>(block + (row >> 3) * 1024 + (row & 7) * 128 + (((4 * half + c) ^ (row & 7)) << 4));
+        // this thread's chunk c of the block lies at cell ^ (c << 4): 128-byte rows, chunks swizzled by the row
+        const uint32_t cell = smem_u32(block) + static_cast<uint32_t>((row >> 3) * 1024 + (row & 7) * 128 + (((4 * half) ^ (row & 7)) << 4));
         const uint32_t full = smem_u32(&bars.hid_full[turn][o]), part = smem_u32(block) + static_cast<uint32_t>(warp & 3) * 4096u;
         const int q = warp >> 2, quarter = NC / 4;                   // output columns of this warp in the last stage
         const int group = 1 << a.group_shift;
@@ -525,7 +522,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             // the block's previous content has been consumed, here and where it was copied to
             ok = ok && mlp_wait(smem_u32(&bars.hid_empty[turn]), (unit & 1) ^ 1, failed);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) *cell[c] = w[c];
+            for (int c = 0; c < 4; ++c)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                             ::"r"(cell ^ static_cast<uint32_t>(c << 4)), "r"(w[c].x), "r"(w[c].y), "r"(w[c].z), "r"(w[c].w) : "memory");
             fence_proxy_async();                                  // the block -> tensor core, bulk copy
             if (C == 1) {
                 __syncwarp();

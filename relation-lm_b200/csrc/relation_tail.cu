@@ -60,8 +60,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) relation_tail_kernel(
     griddep_sync();
 
     constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = kTailBN * kBK * 2;
-    unsigned char* ring = reinterpret_cast<unsigned char*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* ring = smem_align1024(smem_raw);
     const uint32_t ring_addr = smem_u32(ring);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * kTailBN, m0 = blockIdx.z * kBM;

@@ -244,6 +244,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Dynamic shared memory from its first multiple of 1024 bytes (the swizzle atom).  By an offset, not by rounding the
+// address as an integer: through an integer the compiler loses that it is shared memory, and every access by pointer
+// becomes a generic one with a 64-bit address (the relation MLP spilled 252 bytes a thread that way, 136 this way;
+// a pass over 8 x 4096 rows 1375 -> 1335 us).
+__device__ __forceinline__ unsigned char* smem_align1024(unsigned char* raw) {
+    return raw + ((0u - smem_u32(raw)) & 1023u);
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
