@@ -883,7 +883,9 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
 
     // ---- shared staging: statistics of the blocks complete at the tile's last position, and the
     // union of the local windows: positions [w_lo, t_end)
-    unsigned char* st[4] = {smem, smem + m.stats_bytes, smem + 2 * m.stats_bytes, smem + 3 * m.stats_bytes};
+    // (offsets from `smem`, not a table of pointers indexed at run time: through such a table the compiler loses that
+    // they are shared memory, and every load becomes a generic one with a 64-bit address)
+    const auto st = [&](int which) { return smem + which * m.stats_bytes; };
     unsigned char* win_a = smem + 4 * m.stats_bytes;
     unsigned char* win_p = win_a + static_cast<size_t>(m.window_rows) * key_stride;
     float* params = reinterpret_cast<float*>(win_p + static_cast<size_t>(m.window_rows) * key_stride);
@@ -899,7 +901,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
         for (int i = tid; i < 4 * stat_chunks; i += kTileThreads) {
             const int which = i / stat_chunks, c = i - which * stat_chunks;
             const int r = c / stat_cpr, cc = c - r * stat_cpr;
-            cp_async16(smem_u32(st[which]) + r * stat_stride + 16 * cc, src[which] + 16 * c);
+            cp_async16(smem_u32(st(which)) + r * stat_stride + 16 * cc, src[which] + 16 * c);
         }
         const int win_chunks = (t_end - w_lo) * key_cpr;
         const char* ka = static_cast<const char*>(a.anchor_keys) + seq_keys + w_lo * key_row;
@@ -961,7 +963,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             QueryChunk q;
             if (top > 0) {
                 load_query_chunk(arq, q);
-                score_blocks_warp<kDt>(st[0], st[1], nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                score_blocks_warp<kDt>(st(0), st(1), nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
                                   sp_a, bias_a, bscore);
             }
             load_query_chunk(aq, q);
@@ -975,7 +977,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             }
         } else {
             if (top > 0)
-                score_blocks_any<kAnyDtype>(st[0], st[1], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<kAnyDtype>(st(0), st(1), stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         arq, sp_a, bias_a, bscore, 0, 1);
             score_rows_split<kAnyDtype, 1>(local_a, key_dtype, L, nullptr, bs, first_local, t - L + 1, -1, nullptr, 0, aq,
                                        nullptr, 0, 0, 1, bk, bp, 0u, ok);
@@ -1009,7 +1011,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             QueryChunk q;
             if (top > 0) {
                 load_query_chunk(prq, q);
-                score_blocks_warp<kDt>(st[2], st[3], nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
+                score_blocks_warp<kDt>(st(2), st(3), nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
                                   sp_p, bias_p, bscore);
             }
             load_query_chunk(pq, q);
@@ -1023,7 +1025,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
             }
         } else {
             if (top > 0)
-                score_blocks_any<kAnyDtype>(st[2], st[3], stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
+                score_blocks_any<kAnyDtype>(st(2), st(3), stats_dtype, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets,
                                         prq, sp_p, bias_p, bscore, 0, 1);
             score_rows_split<kAnyDtype, 1>(local_p, key_dtype, L, nullptr, bs, first_local, t - L + 1, anchor_pos, nullptr, 0,
                                        pq, cand, 0, 0, 1, dk, dp, 0u, ok);
@@ -1075,7 +1077,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_sel
     griddep_sync();
 
     // two staging buffers: mean | std | window union of one slot and stream
-    unsigned char* stage_buf[2] = {smem, smem + ta.stage_bytes};
+    const auto stage_buf = [&](int ph) { return smem + (ph & 1) * ta.stage_bytes; };     // an offset, not a table of pointers
     float* params = reinterpret_cast<float*>(smem + 2 * ta.stage_bytes);      // per slot: softplus a[4] p[4], bias a, bias p
     const int slot_params = 8 + 2 * buckets4;
     unsigned char* warp_base = reinterpret_cast<unsigned char*>(params) + ta.param_bytes + static_cast<size_t>(warp) * ta.warp_bytes;
@@ -1085,7 +1087,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_sel
         if (ph < 2 * S) {
             const int s = ph < S ? ph : ph - S;
             const bool partner = ph >= S;
-            unsigned char* dst = stage_buf[ph & 1];
+            unsigned char* dst = stage_buf(ph);
             const size_t seq_stats = s * m.stats_slot + static_cast<size_t>(b) * nb * stat_row;
             const size_t seq_keys = s * m.keys_slot + static_cast<size_t>(b) * a.max_t * key_row;
             const char* mean = static_cast<const char*>(partner ? a.partner_mean : a.anchor_mean) + seq_stats;
@@ -1134,7 +1136,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_sel
         __syncthreads();                             // phase ph is staged (and, first time, the parameters are written)
         const int s = ph < S ? ph : ph - S;
         const bool partner = ph >= S;
-        const unsigned char* st_mean = stage_buf[ph & 1];
+        const unsigned char* st_mean = stage_buf(ph);
         const unsigned char* st_std = st_mean + ta.stats_bytes;
         const unsigned char* win = st_mean + 2 * ta.stats_bytes;
         const float* sp = params + s * slot_params + (partner ? 4 : 0);
