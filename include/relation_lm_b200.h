@@ -690,6 +690,14 @@ int rlm_selftest_bounded_wait(int32_t* status, int64_t cycle_limit, int64_t* wai
                               void* stream);
 
 /*
+ * Where rlm_relation_layer_tail keeps, in a CTA's shared memory, what its warps use at the same time at its end
+ * (extension; test support, host only): ranges[2 i], ranges[2 i + 1] = first byte and end of i = 0 the normalised
+ * pairs, 1 the last LayerNorm's 16-bit rows, 2 the received residual rows, 3 the received statistics, 4 the
+ * query-projection weights, 5 all of it.  `pairs`, `n_seq`: of one cluster.
+ */
+int rlm_selftest_layer_tail_plan(int pairs, int n_seq, int relation_dim, int d_model, int n_query, int64_t* ranges);
+
+/*
  * The relation MLP of a whole-sequence pass in one launch (extension): rlm_relation_hidden_cached (rows
  * form) -> second relation-MLP layer -> rlm_relation_norm_reduce (rows form) -> residual, and with
  * slot_weight / anchor_active (both or neither) rlm_slot_mix_residual as well.  Neither the hidden states

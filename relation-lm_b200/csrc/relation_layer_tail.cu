@@ -85,6 +85,24 @@ extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relat
     return clusters > 0 ? 1 : 0;
 }
 
+extern "C" int rlm_selftest_layer_tail_plan(int pairs, int n_seq, int relation_dim, int d_model, int n_query, int64_t* ranges) {
+    using namespace rlm;
+    if (!ranges) { set_error("selftest_layer_tail_plan: result required"); return RLM_ERR_NULL; }
+    const int cluster = 4 * d_model / kLtHC, pairs_pad = pairs <= 16 ? 16 : (pairs <= 32 ? 32 : 64);
+    if (pairs < 1 || pairs > kLtMaxPairs || n_seq < 1 || n_seq > kLtMaxSeq || d_model % kBM != 0 || d_model < kBM || cluster > 16 ||
+        relation_dim % kBK != 0 || n_query % cluster != 0) {
+        set_error("selftest_layer_tail_plan: sizes outside the kernel's range");
+        return RLM_ERR_SHAPE;
+    }
+    const int nq_own = n_query / cluster;
+    const LtPlan p = lt_plan(relation_dim, d_model, pairs_pad, nq_own);
+    const int64_t begin[] = {p.own_y, p.rows, p.hid, p.term_p, p.wq, 0};
+    const int64_t bytes[] = {pairs * kLtOwnStride * 4, n_seq * d_model * 2, n_seq * d_model * 4, cluster * pairs_pad * 8,
+                             nq_own * (2 * d_model + 256), p.total};
+    for (int i = 0; i < 6; ++i) { ranges[2 * i] = begin[i]; ranges[2 * i + 1] = begin[i] + bytes[i]; }
+    return RLM_OK;
+}
+
 extern "C" int rlm_relation_layer_tail(
     const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
     const int32_t* partner_index, const float* partner_scores, const void* product_weight,

@@ -44,6 +44,7 @@ struct LayerTailArgs {
 // Shared-memory plan (byte offsets from the 1024-aligned dynamic base).
 struct LtPlan {
     uint32_t wm, w2, p, hid, term_p, term_a, op_a, wq, total;
+    uint32_t own_y, rows;                // later uses of p and w2: see lt_plan
 };
 
 // The partial sums that a CTA receives, [sender][four pairs][owned column][pair] of 512 d pairs / 128 bytes in all,
@@ -56,9 +57,8 @@ __host__ __device__ inline LtPlan lt_plan(int rdim, int d, int pairs_pad, int nq
     p.wm = off;     off += static_cast<uint32_t>(rdim / kBK) * kBM * 128u;           // W_m slice
     if (pairs_pad == 16 && off < received) off = received;
     p.w2 = off;     off += static_cast<uint32_t>(d / kBM) * 2u * kBM * 128u;         // W_2 slice
-    p.p = off;      off += static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u;     // product tile; later normalised pairs, then rows
+    p.p = off;      off += static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u;     // product tile; later the normalised pairs
     if (off - p.p < pairs_pad * kLtOwnStride * 4u) off = p.p + pairs_pad * kLtOwnStride * 4u;
-    if (off - p.p < static_cast<uint32_t>(kLtMaxSeq) * d * 2u) off = p.p + kLtMaxSeq * d * 2u;
     off = (off + 1023u) & ~1023u;
     p.hid = off;    off += 2u * pairs_pad * 128u;                                    // hidden tile; later the residual rows
     if (off - p.hid < static_cast<uint32_t>(kLtMaxSeq) * d * 4u) off = p.hid + kLtMaxSeq * d * 4u;
@@ -68,6 +68,12 @@ __host__ __device__ inline LtPlan lt_plan(int rdim, int d, int pairs_pad, int nq
     p.wq = p.wm;
     if (pairs_pad == 16) { p.wq = off; off += static_cast<uint32_t>(nq_own) * (2u * d + 256u); }
     p.total = off;
+    // The last LayerNorm's rows take W_2's place, not the normalised pairs': a warp may write its rows while another
+    // of its CTA still sums its pairs (the barrier between them counts what this CTA is sent, and only one warp a
+    // sequence sends to it).  W_2's place is free in every warp by then: the statistics that a CTA waits for include
+    // its own, and those follow its second GEMM and its reads of the partial sums.
+    p.own_y = p.p;
+    p.rows = p.w2;
     return p;
 }
 
@@ -535,7 +541,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     // ---- the pairs' statistics over the full width (equal counts: Chan's parallel variance), eight lanes a pair, and
     // the normalised pairs [pair][kLtOwnStride] for the sequences' weighted sums
-    float* own_y = reinterpret_cast<float*>(p_tile);
+    float* own_y = reinterpret_cast<float*>(base + plan.own_y);
     if (!mbar_wait(bar_stat, 0)) failed = 1;
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
@@ -602,7 +608,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     if (!mbar_wait(bar_rows, 0)) failed = 1;
     __syncwarp();
     lt_cluster_arrive();                                       // nothing more is pushed to this CTA, nor by it
-    uint16_t* rows16 = reinterpret_cast<uint16_t*>(p_tile);    // [sequence][d]
+    unsigned char* rows16 = base + plan.rows;                  // [sequence][d] of 16 bits
     if (part < parts) {
         const float* row = rows_in + my_seq * D;
         // local moments of the lane's 4 mtiles columns, then five exchanges of (mean, M2) of equal halves
@@ -641,7 +647,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 pack2(fmaf((v.x - mean) * rstd, g.x, b.x), fmaf((v.y - mean) * rstd, g.y, b.y), dtype),
                 pack2(fmaf((v.z - mean) * rstd, g.z, b.z), fmaf((v.w - mean) * rstd, g.w, b.w), dtype));
             const int at = 128 * chunk + 4 * lane;
-            *reinterpret_cast<uint2*>(rows16 + my_seq * D + at) = out;
+            *reinterpret_cast<uint2*>(rows16 + (my_seq * D + at) * 2) = out;
             if (at / kLtOwn == static_cast<int>(rank) && !bad_position)
                 *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.normalized) + static_cast<size_t>(s0 + my_seq) * D + at) = out;
         }
@@ -658,7 +664,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             const bool in = o < n_out;
             const int b = in ? o / nq_own : 0, j = in ? o - b * nq_own : 0;
             const unsigned char* wrow = wq_tile + j * wq_stride;
-            const unsigned char* xrow = p_tile + (b * D) * 2;
+            const unsigned char* xrow = rows16 + (b * D) * 2;
             float acc0 = 0.0f, acc1 = 0.0f;
             for (int i = 0; i < my_chunks; i += 2) {
                 float wf[8], xf[8], wg[8], xg[8];

@@ -90,6 +90,20 @@ def test_layer_tail_matches_unfused_oracle(B, K, d, R, T, n_query, t, dtype):
     assert_status_clear()
 
 
+@pytest.mark.parametrize("B,d", [(1, 512), (7, 512), (16, 256), (9, 128)])
+def test_layer_tail_repeats_bit_for_bit(B, d):
+    """One to four sequences a cluster, several warps a sequence: no result may depend on which warp is first."""
+    from relation_lm.kernels.relation_reduce import relation_layer_tail_supported
+
+    if not relation_layer_tail_supported(B, 8, 128, 4 * d, d, 256, torch.bfloat16):
+        pytest.skip("clusters of this size are not available on this device")
+    x = _case(B, 8, d, 128, 40, 256, torch.bfloat16, 77 + B)
+    first = _run(x, 39, torch.bfloat16)
+    for _ in range(50):
+        assert all(torch.equal(a, b) for a, b in zip(first, _run(x, 39, torch.bfloat16)))
+    assert_status_clear()
+
+
 def test_layer_tail_rejects_shapes_it_does_not_serve():
     from relation_lm.kernels.relation_reduce import relation_layer_tail_supported
 
