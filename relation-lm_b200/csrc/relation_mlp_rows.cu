@@ -124,7 +124,7 @@ __host__ __device__ inline MlpPlan mlp_plan(int rdim, int cols, int outs, int wi
 }
 
 struct MlpBars {
-    unsigned long long a_full, a_empty, d2_full, d2_empty, stats_full, rows_full[2], u_full[3];
+    unsigned long long a_full, a_empty, d2_full, d2_empty, stats_full, rows_full[2], u_full[3], u_empty[3];
     unsigned long long d1_full[2], d1_empty[2], wm_full[2], wm_empty[2];
     unsigned long long w2_full[kMlpMaxStages], w2_empty[kMlpMaxStages];
     unsigned long long hid_full[kMlpHidden][2], hid_empty[kMlpHidden];
@@ -421,7 +421,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         init(&bars.d2_full, 1);
         init(&bars.d2_empty, kMlpEpiWarps * kG);
         init(&bars.stats_full, C == 1 ? kMlpEpiWarps : 1);
-        for (int i = 0; i < 3; ++i) init(&bars.u_full[i], kBM / 32);
+        for (int i = 0; i < 3; ++i) {
+            init(&bars.u_full[i], kBM / 32);
+            init(&bars.u_empty[i], kMlpEpiWarps);
+        }
         for (int i = 0; i < 2; ++i) {
             init(&bars.rows_full[i], kBM / 32);
             init(&bars.d1_full[i], 1);
@@ -613,6 +616,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             const float rstd = rsqrtf(fmaf(total, a.inv_d, a.eps));
             ok = ok && mlp_wait(smem_u32(&bars.u_full[tix3]), u_phase, failed);
             const float u = u_s[tix3 * kBM + row];
+            __syncwarp();
+            if (ok && lane == 0) mlp_arrive(smem_u32(&bars.u_empty[tix3]));
             if (++tix3 == 3) { tix3 = 0; u_phase ^= 1; }
             const float ur = u == 0.0f ? 0.0f : u * rstd;
             float u_sum = u, urm_sum = u == 0.0f ? 0.0f : ur * mean;
@@ -830,7 +835,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         const size_t op_row = static_cast<size_t>(R) * 2;
         const char* operand = static_cast<const char*>(a.operand_cache);
         const int cc = lane % chunks, r_first = gw * rows_per_warp + lane / chunks, r_step = kMlpOperandWarps * rows_per_warp;
-        int tix = 0, u_at = 0;
+        int tix = 0, u_at = 0, u_phase = 0;
         bool ok = true;
         // Tile `super`'s cache rows (its partners; the anchors of both of the pair's tiles) into buffer `b` and this
         // thread's pair's weight into u.
@@ -875,13 +880,16 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                     arow = srow / a.slots / a.rows_per_seq * a.max_t + min(max(a.anchor_index[srow], 0), a.max_t - 1);
                 arow_s[b * sel_k + gt] = arow;
             }
+            // The weights are read in a tile's last stage, the first layer runs ahead of it: with two or three units a
+            // tile the slot may still be waiting to be read.
+            ok = ok && mlp_wait(smem_u32(&bars.u_empty[u_at]), u_phase ^ 1, failed);
             u_s[u_at * kBM + gt] = u;
             __syncwarp();
             if (ok && lane == 0) {
                 mlp_arrive(smem_u32(&bars.rows_full[b]));
                 mlp_arrive(smem_u32(&bars.u_full[u_at]));
             }
-            if (++u_at == 3) u_at = 0;
+            if (++u_at == 3) { u_at = 0; u_phase ^= 1; }
         };
         if (cluster < n_super) indices(cluster, 0);
         for (int super = cluster; super < n_super; super += n_clusters, ++tix) {

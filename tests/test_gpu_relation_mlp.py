@@ -10,10 +10,10 @@ from gpu_util import assert_status_clear
 pytestmark = pytest.mark.gpu
 
 
-def _case(dtype, batch, length, slots, k, rdim, d, seed):
+def _case(dtype, batch, length, slots, k, rdim, d, seed, hidden=0):
     g = torch.Generator(device="cuda").manual_seed(seed)
     rn = lambda *s, scale=1.0: torch.randn(*s, generator=g, device="cuda") * scale  # noqa: E731
-    H, N = 4 * d, batch * length
+    H, N = hidden or 4 * d, batch * length
     x = {
         "expanded": rn(batch, length, 2 * H, scale=0.5).to(dtype), "operand": rn(batch, length, rdim).to(dtype),
         "anchor": torch.randint(-1, length, (N, slots), generator=g, device="cuda", dtype=torch.int32),
@@ -72,10 +72,24 @@ def _expected(x, length, limited, mixed):
     (3, 600, 4, 4, 128, 512, False), (3, 800, 1, 8, 128, 768, True),
 ])
 def test_matches_the_composition(dtype, batch, length, slots, k, rdim, d, limited):
+    _check(dtype, batch, length, slots, k, rdim, d, 4 * d, limited)
+
+
+# the fewest hidden units a CTA can have (two and three; d 64 .. 256 and 512: the wide form, 384 and 768: the other), with
+# five tiles or more for every cluster: the first layer then runs two tiles ahead of the weights' last use
+@pytest.mark.parametrize("batch,slots,k,rdim,d,hidden", [
+    (56, 4, 8, 64, 64, 256), (56, 4, 8, 64, 64, 384), (56, 2, 16, 128, 256, 256), (28, 4, 8, 128, 512, 512),
+    (28, 4, 8, 64, 512, 768), (56, 4, 8, 64, 384, 256), (28, 4, 8, 128, 768, 512), (28, 4, 8, 64, 768, 768),
+])
+def test_few_hidden_units_and_many_tiles(batch, slots, k, rdim, d, hidden):
+    _check(torch.bfloat16, batch, 53, slots, k, rdim, d, hidden, False)
+
+
+def _check(dtype, batch, length, slots, k, rdim, d, hidden, limited):
     from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
 
-    assert relation_mlp_rows_supported(k, slots, rdim, 4 * d, d, dtype)
-    x = _case(dtype, batch, length, slots, k, rdim, d, seed=d + 7 * k + length)
+    assert relation_mlp_rows_supported(k, slots, rdim, hidden, d, dtype)
+    x = _case(dtype, batch, length, slots, k, rdim, d, d + 7 * k + length, hidden)
     mixed = slots > 1
     out = x["residual"].clone()
     relation_mlp_rows(out, x["expanded"], x["operand"], x["anchor"], x["partner"], x["score"], x["active"] if mixed else None,
