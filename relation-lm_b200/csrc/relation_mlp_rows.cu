@@ -26,7 +26,10 @@
 // The expanded-cache terms join the first layer's accumulator as matrix products, so that the epilogue is GELU
 // and nothing else: the partners' segments, gathered as a 128 x 64 block in operand layout, times the identity,
 // and the anchors' segments selected by a one-hot matrix.  Both are exact in the fp32 accumulator.  (Added
-// in the epilogue instead they cost a third of its instructions, and the epilogue was the bound.)
+// in the epilogue instead they cost a third of its instructions, and the epilogue was the bound.)  An infinity or NaN
+// in an anchor's segment would reach every row of the product (zero times infinity), so the gathering threads look at
+// what they place: such a chunk enters as zeros, and its anchor is marked for the epilogue, which makes the rows
+// that selected it NaN.  (A partner's segment only meets its own row.)
 //
 // One CTA (32 warps, registers shifted to the epilogue by setmaxnreg), a persistent loop over tiles:
 //   warps 0-15   epilogue: thread = pair row x 32 columns of a hidden block; then the LayerNorm and the
@@ -34,8 +37,8 @@
 //   warps 16, 17 TMA producers of W_2 and of W_m tiles (apart: a full W_2 ring must not hold up W_m)
 //   warps 18, 19 tcgen05.mma issue of the first and of the second layer (the first CTA of a pair; in the
 //                second they forward its barriers to the first)
-//   warps 20-23  gathers of the expanded-cache segments (cp.async; as TMA row gathers, tile::gather4, a block of
-//                128 + 32 rows took 3 500 cycles instead of 1 000)
+//   warps 20-23  gathers of the expanded-cache segments (the partners' by cp.async, the anchors' through registers; as
+//                TMA row gathers, tile::gather4, a block of 128 + 32 rows took 3 500 cycles instead of 1 000)
 //   warps 24-31  indices, weights u, and the operand products of the next tile (the A tile): in registers
 //                while the current tile runs, into shared memory the moment its last product is done
 // Hidden columns go in units of 128 (two blocks of 64, one per epilogue group): up to 256 output columns per
@@ -92,7 +95,7 @@ struct MlpArgs {
 
 // Shared-memory plan (byte offsets from the 1024-aligned dynamic base).
 struct MlpPlan {
-    uint32_t a, wm, w2, hid, term, anc, onehot, ident, bias, gamma, beta, stats, u, prow, arow, total;
+    uint32_t a, wm, w2, hid, term, anc, onehot, ident, bias, gamma, beta, stats, u, poison, prow, arow, total;
 };
 
 // Anchor segments of one block: the anchors of both of the pair's tiles, this CTA's half of the columns.
@@ -117,6 +120,7 @@ __host__ __device__ inline MlpPlan mlp_plan(int rdim, int cols, int outs, int wi
     p.beta = off;   off += static_cast<uint32_t>(cols) * 4u;
     p.stats = off;  off += static_cast<uint32_t>(4 * outs) * kBM * 8u;
     p.u = off;      off += 3u * kBM * 4u;
+    p.poison = off; off += 4u * (kBM >> k_shift) * 4u;
     p.prow = off;   off += 2u * kBM * 4u;
     p.arow = off;   off += 4u * (kBM >> k_shift) * 4u;
     p.total = off;
@@ -174,6 +178,16 @@ __device__ __forceinline__ void mlp_store_remote(uint32_t remote_dst, float x, f
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
                  ::"r"(remote_dst), "f"(x), "f"(y), "r"(remote_bar) : "memory");
 }
+// Marks the anchors r (bit 0 of `which`) and r + 32 (bit 1) of a CTA pair's two tiles in the CTA of their tile: NaN at
+// `marks` + anchor, visible there before anything that this thread announces afterwards.
+__device__ __noinline__ void mlp_mark(uint32_t marks, uint32_t leader, int anchors, int r, uint32_t which) {
+    for (int i = 0; i < 2; ++i, r += 32)
+        if (which >> i & 1) {
+            const int of = r >= anchors ? 1 : 0;
+            asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(mlp_peer(marks + 4u * (r - of * anchors), leader + of)), "r"(0x7fc00000) : "memory");
+        }
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+}
 template <bool kCluster>
 __device__ __forceinline__ bool mlp_try_wait(uint32_t bar, uint32_t parity) {
     if (!kCluster) return mbar_try_wait(bar, parity);
@@ -208,6 +222,14 @@ template <int kRegs>
 __device__ __forceinline__ void mlp_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs)); }
 __device__ __forceinline__ void mlp_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Whether one of eight 16-bit values is an infinity or NaN (an exponent of all ones).
+template <int kDt>
+__device__ __forceinline__ bool mlp_not_finite(const uint4& v) {
+    constexpr uint32_t kExp = kDt == RLM_BF16 ? 0x7f807f80u : 0x7c007c00u, kUnit = kDt == RLM_BF16 ? 0x00800080u : 0x04000400u;
+    const uint32_t carry = ((v.x & kExp) + kUnit) | ((v.y & kExp) + kUnit) | ((v.z & kExp) + kUnit) | ((v.w & kExp) + kUnit);
+    return (carry & 0x80008000u) != 0;
 }
 
 // ---- tcgen05 on CTA pairs
@@ -410,6 +432,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
     float* u_s = reinterpret_cast<float*>(base + plan.u);
     int* prow_s = reinterpret_cast<int*>(base + plan.prow);
     int* arow_s = reinterpret_cast<int*>(base + plan.arow);
+    float* poison_s = reinterpret_cast<float*>(base + plan.poison);      // [four tiles in turn][anchor]: 0, or NaN for one that is not finite
 
     if (tid == 0) {
         failed_s = 0;
@@ -441,7 +464,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             init(&bars.hid_empty[i], C);
         }
         for (int i = 0; i < kMlpMaxTerms; ++i) {
-            init(&bars.term_full[i], 32 * kMlpGatherWarps + both - 1);
+            init(&bars.term_full[i], (32 + 1) * kMlpGatherWarps + both - 1);
             init(&bars.term_empty[i], 1);
         }
         fence_barrier_init();
@@ -455,6 +478,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         gamma_s[i] = a.norm_w[o * NC + i];
         beta_s[i] = a.norm_b[o * NC + i];
     }
+    for (int i = tid; i < 4 * anchors; i += kMlpThreads) poison_s[i] = 0.0f;
     const uint16_t one = kDt == RLM_BF16 ? 0x3f80 : 0x3c00;
     for (int i = tid; i < kBM * sel_k / 8; i += kMlpThreads) {          // one-hot rows: K-chunk major core matrices, no swizzle
         const int c = i / kBM, r = i - c * kBM;
@@ -586,7 +610,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                 }
             }
             const float inv_quarter = 1.0f / static_cast<float>(quarter);
-            const float mean_q = fmaf(s1, inv_quarter, shift), m2 = fmaf(-s1 * inv_quarter, s1, s2);
+            // (a row whose anchor is not finite becomes NaN here, and through the statistics in every output part)
+            const float mean_q = fmaf(s1, inv_quarter, shift) + *static_cast<volatile float*>(poison_s + (tix & 3) * anchors + (row >> a.k_shift));
+            const float m2 = fmaf(-s1 * inv_quarter, s1, s2);
             // every CTA of the tile receives (mean, sum of squares) of all quarters
             float2* mine = stats_s + (o * 4 + q) * kBM + row;
             if (C == 1) {
@@ -788,22 +814,39 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         mlp_fewer_registers<kMlpIssueRegs>();
         // ------------------------------------------------------------ expanded-cache segments of every block
         // 64 columns of the tile's 128 partner rows (128-byte swizzle), this CTA's 32 of the 64 columns of the pair's
-        // anchor rows (64-byte swizzle), a thread per 16-byte chunk.
+        // anchor rows (64-byte swizzle), a thread per 16-byte chunk.  The anchors' chunks are requested a block ahead
+        // into registers, where they are looked at (see the top).  What that costs, and the other places measured for
+        // it, as us a pass of 8 x 4096 rows of d 512: 1266 without looking, 1300 here; the operand warps over the
+        // anchors' whole rows 1306 (another read of them); the issuing warp 1433 (in the way of every block's products).
         const int gt = tid - 32 * (kMlpEpiWarps + 4), c = gt & 7, ac = gt & 3;
         const size_t ex_row = static_cast<size_t>(H) * 4;
         const char* expanded = static_cast<const char*>(a.expanded_cache);
+        const char* partners = expanded + static_cast<size_t>(H) * 2 + 16 * c;
         const uint32_t to = swizzled(gt >> 3, c, kMlpBlock);               // rows 16 apart: 2048 bytes apart
+        const uint32_t anchor_to = static_cast<uint32_t>((gt >> 2) * 64 + ((ac ^ ((gt >> 3) & 3)) << 4));      // ... 32 apart alike
         int ts = 0, tphase = 0, tix = 0;
         bool ok = true;
         for (int super = cluster; super < n_super; super += n_clusters, ++tix) {
             ok = ok && mlp_wait(smem_u32(&bars.rows_full[tix & 1]), (tix >> 1) & 1, failed);
-            const int* arow_t = arow_s + (tix & 1) * sel_k;
-            const char* from[8];
+            int prow[8], arow[2];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int row = prow_s[(tix & 1) * kBM + (gt >> 3) + 16 * i];
-                from[i] = row < 0 ? nullptr : expanded + row * ex_row + static_cast<size_t>(H) * 2 + 16 * c;
+            for (int i = 0; i < 8; ++i) prow[i] = prow_s[(tix & 1) * kBM + (gt >> 3) + 16 * i];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int r = (gt >> 2) + 8 * kMlpGatherWarps * i;
+                arow[i] = r < sel_k ? arow_s[(tix & 1) * sel_k + r] : -1;
             }
+            uint4 ahead[2];
+            uint32_t bad = 0;                                     // this thread's anchors that are not finite
+            const auto request_anchors = [&](int n) {
+                const char* from = expanded + static_cast<size_t>(column(n, o)) * 2 + g * (kMlpHC / kG) * 2 + 16 * ac;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {      // beyond the last row: every row's product reads it (times zero)
+                    ahead[i] = make_uint4(0, 0, 0, 0);
+                    if (arow[i] >= 0) ahead[i] = *reinterpret_cast<const uint4*>(from + arow[i] * ex_row);
+                }
+            };
+            if (ok) request_anchors(0);
             for (int n = 0; n < 2 * U; ++n) {
                 const size_t h_bytes = static_cast<size_t>(column(n, o)) * 2;
                 const uint32_t block = s_term + static_cast<uint32_t>(ts) * kMlpBlock + to;
@@ -811,18 +854,23 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                 if (ok) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        if (from[i]) cp_async16(block + 2048u * i, from[i] + h_bytes);
-                    for (int r = gt >> 2; r < sel_k; r += 8 * kMlpGatherWarps) {
-                        const int arow = arow_t[r];
-                        const uint32_t at = plan.anc + static_cast<uint32_t>(ts) * anc_stage +
-                                            static_cast<uint32_t>(r * 64 + ((ac ^ ((r >> 1) & 3)) << 4));
-                        if (arow >= 0)
-                            cp_async16(smem_u32(base + at), expanded + arow * ex_row + h_bytes + g * (kMlpHC / kG) * 2 + 16 * ac);
-                        else      // beyond the last row: every row's product reads it (times zero)
-                            *reinterpret_cast<uint4*>(base + at) = make_uint4(0, 0, 0, 0);
+                        if (prow[i] >= 0) cp_async16(block + 2048u * i, partners + prow[i] * ex_row + h_bytes);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int r = (gt >> 2) + 8 * kMlpGatherWarps * i;
+                        if (r >= sel_k) break;
+                        if (mlp_not_finite<kDt>(ahead[i])) {
+                            ahead[i] = make_uint4(0, 0, 0, 0);
+                            bad |= 1u << i;
+                        }
+                        *reinterpret_cast<uint4*>(base + plan.anc + static_cast<uint32_t>(ts) * anc_stage + anchor_to + 2048u * i) = ahead[i];
                     }
+                    if (n + 1 < 2 * U) request_anchors(n + 1);
+                    else if (bad) mlp_mark(smem_u32(poison_s + (tix & 3) * anchors), leader, anchors, gt >> 2, bad);
                     mlp_cp_async_arrive(smem_u32(&bars.term_full[ts]));
                 }
+                __syncwarp();                                 // the warp's stores -> its one arrival for them
+                if (ok && lane == 0) mlp_arrive(smem_u32(&bars.term_full[ts]));
                 if (++ts == a.term_stages) { ts = 0; tphase ^= 1; }
             }
         }
@@ -835,7 +883,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         const size_t op_row = static_cast<size_t>(R) * 2;
         const char* operand = static_cast<const char*>(a.operand_cache);
         const int cc = lane % chunks, r_first = gw * rows_per_warp + lane / chunks, r_step = kMlpOperandWarps * rows_per_warp;
-        int tix = 0, u_at = 0, u_phase = 0;
+        int tix = 0, u_at = 0, u_phase = 0, made = 0;
         bool ok = true;
         // Tile `super`'s cache rows (its partners; the anchors of both of the pair's tiles) into buffer `b` and this
         // thread's pair's weight into u.
@@ -884,6 +932,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             // tile the slot may still be waiting to be read.
             ok = ok && mlp_wait(smem_u32(&bars.u_empty[u_at]), u_phase ^ 1, failed);
             u_s[u_at * kBM + gt] = u;
+            // the next tile's marks, last read three tiles ago; nothing of that tile is gathered before this one is announced
+            ++made;
+            if (gt < anchors) poison_s[(made & 3) * anchors + gt] = 0.0f;
             __syncwarp();
             if (ok && lane == 0) {
                 mlp_arrive(smem_u32(&bars.rows_full[b]));

@@ -106,6 +106,44 @@ def _check(dtype, batch, length, slots, k, rdim, d, hidden, limited):
     assert float((context - expected).abs().max()) <= bound * float(expected.abs().max().clamp_min(1.0))
 
 
+# d 256: one output part, 512 and 768: two, each finding its own columns; the first and the last hidden column
+@pytest.mark.parametrize("dtype,value", [(torch.bfloat16, torch.inf), (torch.float16, torch.nan), (torch.float16, -torch.inf)])
+@pytest.mark.parametrize("slots,k,d", [(1, 8, 256), (2, 4, 512), (1, 16, 768), (4, 4, 512)])
+def test_a_cache_row_that_is_not_finite_reaches_the_rows_that_selected_it(dtype, value, slots, k, d):
+    from relation_lm.kernels.relation_reduce import relation_mlp_rows
+
+    length = 90
+    x = _case(dtype, 2, length, slots, k, 128, d, seed=d + k)
+    mixed = slots > 1
+
+    def run(expanded):
+        out = torch.empty_like(x["residual"])
+        relation_mlp_rows(out, expanded, x["operand"], x["anchor"], x["partner"], x["score"], x["active"] if mixed else None,
+                          x["slot_weight"] if mixed else None, x["scale"], x["wm"], x["w2"], x["b2"], x["nw"], x["nb"], 1e-5,
+                          x["residual"], slots, length, False)
+        assert_status_clear()
+        return out
+
+    before = run(x["expanded"])
+    N, H = 2 * length, 4 * d
+    seq = torch.arange(N, device="cuda")[:, None] // length
+    used = torch.isfinite(x["score"])                                       # pairs with a weight
+    if mixed:
+        used &= x["active"][..., None]
+    for column in (0, 65, H // 2 + 31, H - 1):
+        for half, row in ((0, 0), (1, 41), (0, 77)):
+            expanded = x["expanded"].clone()
+            expanded[1, row, half * H + column] = value
+            if half:
+                hit = ((x["partner"].clamp(0, length - 1) == row) & used).flatten(1).any(1)
+            else:
+                hit = ((x["anchor"].clamp(0, length - 1) == row)[..., None] & used).flatten(1).any(1)
+            hit &= (seq == 1).squeeze(1)
+            out = run(expanded)
+            assert bool(hit.any()) and bool(out[hit].isnan().all())
+            assert torch.equal(out[~hit], before[~hit])
+
+
 def test_new_output_without_residual_or_scale():
     from relation_lm.kernels.relation_reduce import relation_mlp_rows
 
