@@ -40,7 +40,6 @@ class RoutedPrefillLayer:
     def __init__(self, model: RoutedRelationLM, layer: int = 0, device="cuda",
                  dtype: torch.dtype = torch.bfloat16, tiled_select: bool = True) -> None:
         self.tiled_select = bool(tiled_select)
-        self._rows: tuple | None = None
         if dtype not in (torch.bfloat16, torch.float16):
             raise ValueError("the prefill path runs its projections on the tensor cores: bfloat16 or float16")
         self.config, self.layer, self.device, self.dtype = model.config, int(layer), torch.device(device), dtype
@@ -65,14 +64,11 @@ class RoutedPrefillLayer:
         }
 
     def rows(self, batch: int, length: int) -> tuple[Tensor, Tensor]:
-        """``(row_batch, row_position)`` of all ``batch * length`` query rows, sequence-major; the tables of the
-        last size are kept (building them takes four launches)."""
-        kept = self._rows
-        if kept is None or kept[0] != (batch, length):
-            rb = torch.arange(batch, device=self.device, dtype=torch.int32).repeat_interleave(length)
-            rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
-            kept = self._rows = ((batch, length), rb, rp)
-        return kept[1], kept[2]
+        """``(row_batch, row_position)`` of all ``batch * length`` query rows, sequence-major.  Made for each pass: a
+        table kept from another one would have been filled on that one's stream, or only in its captured graph."""
+        rb = torch.arange(batch, device=self.device, dtype=torch.int32).repeat_interleave(length)
+        rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
+        return rb, rp
 
     @_abi.programmatic_launch
     def build_state(self, x: Tensor) -> dict[str, Tensor]:

@@ -1,0 +1,21 @@
+"""Host-side behaviour of the whole-sequence passes."""
+from __future__ import annotations
+
+import torch
+
+from relation_lm.inference.prefill import RoutedPrefillLayer
+from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+
+
+def _layer(**sizes):
+    cfg = RoutedRelationConfig(**{**dict(vocab_size=32, boundary_vocab_size=4, d_model=64, layers=1, max_context=32, block_size=8,
+                                         local_window=8, top_blocks=1), **sizes})
+    return RoutedPrefillLayer(RoutedRelationLM(cfg, seed=0), 0, "cpu")
+
+
+def test_row_tables_belong_to_their_pass():
+    """Every pass fills its own tables on its own stream (or in its own graph): none is handed from one to the next."""
+    layer = _layer()
+    first, second = layer.rows(2, 32), layer.rows(2, 32)
+    for a, b in zip(first, second):
+        assert torch.equal(a, b) and a.data_ptr() != b.data_ptr()
