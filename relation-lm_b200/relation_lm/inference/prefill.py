@@ -123,7 +123,7 @@ class RoutedPrefillLayer:
             out = torch.empty(N, d, device=self.device, dtype=torch.float32)
             relation_mlp_rows(out, state["expanded_cache"], state["operand_cache"], anchor, partner, partner_score, None, None,
                               w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"],
-                              cfg.norm_eps, x.view(N, d), 1, T, True)
+                              cfg.norm_eps, x.view(N, d).contiguous(), 1, T, True)       # (a copy only of strided rows)
             return out.view(B, T, d)
         hidden_rel = torch.empty(N, K, H, device=self.device, dtype=self.dtype)
         relation_hidden_cached_rows_out(hidden_rel, state["expanded_cache"], state["operand_cache"], anchor,
