@@ -132,8 +132,43 @@ def sequence_state(packed: Tensor, slots: int, relation_dim: int, block_size: in
     launch (extension), keyed by ``STATE_NAMES``: the token caches, and what ``router_cache_prefill`` leaves of
     both router streams.  ``slots = 0``: one layer's column order (``W = 384 + R``), caches ``[B, T, width]``;
     ``slots = S``: ``S`` slots of 384 columns, then the operand, slot caches ``[S, B, T, width]``."""
+    if block_size > _STATE_BLOCK:
+        return _sequence_state_by_parts(packed, slots, relation_dim, block_size, anchor_conv_weight, partner_conv_weight)
     return dict(zip(STATE_NAMES, _sequence_state(packed, slots, relation_dim, block_size, anchor_conv_weight,
                                                  partner_conv_weight)))
+
+
+# Positions of the largest block whose router rows, with two rows of history, and convolved rows the kernel can hold in
+# shared memory: (2 n + 2) rows of 256 bytes in 226 KB.  Longer blocks are copied and walked in device memory.
+_STATE_BLOCK = 451
+
+
+def _sequence_state_by_parts(packed: Tensor, slots: int, relation_dim: int, block_size: int, anchor_conv_weight: Tensor,
+                             partner_conv_weight: Tensor) -> dict[str, Tensor]:
+    (batch, length, width), n = packed.shape, max(slots, 1)
+    if packed.dtype not in (torch.bfloat16, torch.float16) or slots < 0 or length % block_size != 0 \
+            or width != 384 * n + relation_dim or anchor_conv_weight.numel() != 192 * n \
+            or partner_conv_weight.numel() != 192 * n:
+        raise ValueError("packed must be 16-bit [B, T, 384 * slots + R] of whole blocks and the conv weights [slots, 64, 3]")
+    operand_at, anchor_at = (384 * n, 128) if slots else (128, 128 + relation_dim)
+
+    def columns(at: int, size: int) -> Tensor:
+        if not slots:
+            return packed[..., at:at + size].contiguous()
+        return torch.stack([packed[..., 384 * s + at:384 * s + at + size] for s in range(n)])
+
+    state = {"anchor_keys": columns(0, 64), "partner_keys": columns(64, 64),
+             "operand_cache": packed[..., operand_at:operand_at + relation_dim].contiguous(),
+             "partner_anchor_cache": columns(anchor_at, 128)}
+    for name in STATE_NAMES[4:]:
+        tail = (length, 64) if name.endswith("cache") else (length // block_size, 4, 16)
+        state[name] = packed.new_zeros((n, batch, *tail))
+    weights = anchor_conv_weight.view(n, 64, 3), partner_conv_weight.view(n, 64, 3)
+    for s in range(n):
+        router = packed[..., 384 * s + anchor_at + 128:384 * s + anchor_at + 256]
+        router_cache_prefill(router[..., :64], router[..., 64:], *[state[name][s] for name in STATE_NAMES[4:]],
+                             weights[0][s], weights[1][s], block_size)
+    return {name: t if slots or name in STATE_NAMES[:4] else t[0] for name, t in state.items()}
 
 
 @torch.library.register_fake("relation_lm::sequence_state")

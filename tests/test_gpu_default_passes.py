@@ -33,3 +33,14 @@ def test_prefill_takes_rows_of_a_wider_tensor():
     assert all(torch.equal(state[n], dense[n]) for n in state)
     assert torch.equal(layer.forward(x, state), layer.forward(x.contiguous(), state))
     assert_status_clear()
+
+
+@pytest.mark.parametrize("block", [448, 512])
+def test_prefill_of_blocks_beyond_the_state_kernels_tile(block):
+    layer = _layer(max_context=2 * block, block_size=block, local_window=48, top_blocks=1)
+    x = _rows(2, 2 * block, 256)
+    state, keep = layer.build_state(x), {}
+    kept = layer.forward(x, state, keep)
+    # one selection on both sides, the relation MLP in one kernel or three: its rounding steps (see test_gpu_relation_mlp)
+    assert float((layer.forward(x, state) - kept).abs().max()) <= 2 * 2 ** -8 * float(keep["context"].abs().max().clamp_min(1.0))
+    assert_status_clear()

@@ -34,7 +34,8 @@ def _by_parts(packed, slots, rdim, bs, wa, wp):
 
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
 @pytest.mark.parametrize("batch,blocks,bs,slots,rdim", [(1, 1, 1, 0, 128), (2, 3, 2, 0, 64), (1, 4, 8, 0, 128), (3, 5, 16, 2, 128),
-                                                       (2, 2, 33, 1, 64), (2, 3, 64, 0, 128), (1, 2, 64, 4, 128), (1, 1, 256, 8, 8)])
+                                                       (2, 2, 33, 1, 64), (2, 3, 64, 0, 128), (1, 2, 64, 4, 128), (1, 1, 256, 8, 8),
+                                                       (1, 2, 451, 0, 64), (1, 2, 452, 0, 64), (2, 1, 600, 2, 128)])
 def test_equals_copies_and_router_prefill(dtype, batch, blocks, bs, slots, rdim):
     from relation_lm.kernels.router_cache import STATE_NAMES, sequence_state
 
