@@ -298,6 +298,9 @@ class MultiAnchorPrefill:
         shared ``memory`` (16-bit), then the final LayerNorm."""
         from relation_lm.kernels.packed_projection import layer_norm_cast
 
+        if not self.config.depth:                           # a stack without layers is its final LayerNorm
+            return torch.nn.functional.layer_norm(hidden, (hidden.size(-1),), self.final_norm_w, self.final_norm_b,
+                                                  self.config.norm_eps)
         current, source = torch.empty_like(hidden, memory_format=torch.contiguous_format), hidden.contiguous()
         for l in range(self.config.depth):
             state = self.build_state(l, memory)

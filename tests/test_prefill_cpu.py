@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import torch
 
+from relation_lm.inference.multi_anchor import MultiAnchorConfig, MultiAnchorPrefill, MultiAnchorRoutedStack
 from relation_lm.inference.prefill import RoutedPrefillLayer
 from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
 
@@ -19,3 +20,10 @@ def test_row_tables_belong_to_their_pass():
     first, second = layer.rows(2, 32), layer.rows(2, 32)
     for a, b in zip(first, second):
         assert torch.equal(a, b) and a.data_ptr() != b.data_ptr()
+
+
+def test_a_stack_without_layers_is_its_final_norm():
+    stack = MultiAnchorRoutedStack(MultiAnchorConfig(d_model=64, depth=0), seed=0)
+    hidden = torch.randn(2, 5, 64, generator=torch.Generator().manual_seed(1))
+    out = MultiAnchorPrefill(stack, "cpu").forward(hidden, hidden.bfloat16())
+    assert torch.equal(out, torch.nn.functional.layer_norm(hidden, (64,), stack.final_norm.weight, stack.final_norm.bias, 1e-5))
