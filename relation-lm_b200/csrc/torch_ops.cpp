@@ -853,6 +853,8 @@ Tensor decode_embed_norm(const Tensor& tokens, const Tensor& boundaries, const T
     TORCH_CHECK_VALUE(tokens.scalar_type() == at::kLong && boundaries.scalar_type() == at::kLong && is_f32(position_table),
                       "ids must be int64 and the position table float32");
     const int64_t batch = tokens.numel(), d_model = token_table.size(1);
+    TORCH_CHECK_VALUE(boundaries.numel() == batch && boundary_table.size(1) == d_model && position_table.size(1) == d_model,
+                      "decode_embed_norm: one boundary id per token and tables of one width");
     for (const Tensor* t : {&norm1_weight, &norm1_bias, &norm2_weight, &norm2_bias})
         TORCH_CHECK_VALUE(is_f32(*t) && t->numel() == d_model, "LayerNorm parameters must be float32 [d_model]");
     TORCH_CHECK_VALUE(is_shape(normalized1, {batch, d_model}) && is_shape(normalized2, {batch, d_model}) &&

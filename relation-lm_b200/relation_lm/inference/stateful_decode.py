@@ -151,8 +151,10 @@ class StatefulDecoder:
         if not self.fused:
             # rows of whole 16-byte chunks up to 1024 wide: LayerNorms inside the kernels that make their input
             self.kernel_norms = cfg.d_model % 8 == 0 and cfg.d_model <= 1024
-            self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
-            self.head_bias = torch.cat((zeros(cfg.vocab_size), self.w["boundary_b"]))
+            # one product for both heads where its column slices are dense matrices, as two products' results are
+            if B == 1:
+                self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
+                self.head_bias = torch.cat((zeros(cfg.vocab_size), self.w["boundary_b"]))
         else:
             self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
             pad = (-self.head_weight.size(0)) % 128        # whole 128-column tiles for the projection kernel
@@ -237,8 +239,9 @@ class StatefulDecoder:
         cfg, w = self.config, self.w
         pos, K = self.position, cfg.k_max
         if self.kernel_norms:
-            hidden = decode_embed_norm(tokens.contiguous(), boundaries.contiguous(), w["token_embedding"],
-                                       w["boundary_embedding"], w["position_embedding"], pos, self.input_scale,
+            tokens, boundaries = self._ids(tokens, boundaries)
+            hidden = decode_embed_norm(tokens, boundaries, w["token_embedding"], w["boundary_embedding"],
+                                       w["position_embedding"], pos, self.input_scale,
                                        w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized,
                                        w["input_norm_w"][0], w["input_norm_b"][0], self.normalized, cfg.norm_eps)
         else:
@@ -253,6 +256,8 @@ class StatefulDecoder:
         if keep_selection:
             self.last_selection = []
         for layer in self._layers:
+            # the last layer's goes to a tensor of this step's own: it stays behind as `last_final`
+            normalized = torch.empty_like(self.normalized) if layer is self._layers[-1] else self.normalized
             torch.mm(self.normalized, layer.w_query_t, out=layer.query)                 # [B, 256]
             anchor, _, partner, partner_score = relation_select_packed(
                 *layer.selection, pos, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
@@ -260,17 +265,36 @@ class StatefulDecoder:
             raw = F.linear(self.relation_hidden, *layer.second_layer)                   # [B, K, d]
             if self.kernel_norms:
                 relation_norm_reduce_residual_norm(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps, hidden,
-                                                   layer.mix, *layer.next_norm, cfg.norm_eps, self.normalized)
+                                                   layer.mix, *layer.next_norm, cfg.norm_eps, normalized)
             else:
                 context = relation_norm_reduce(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps)
                 torch.addcmul(hidden, context, layer.mix, out=hidden)
-                self._normalize(hidden, *layer.next_norm, self.normalized)
+                self._normalize(hidden, *layer.next_norm, normalized)
             if keep_selection:
                 self.last_selection.append((anchor, partner))
-        self.last_final = self.normalized
-        logits = F.linear(self.normalized, self.head_weight, self.head_bias)
+        self.last_final = normalized
+        if self.batch == 1:
+            logits = F.linear(normalized, self.head_weight, self.head_bias)
+            heads = logits[:, :cfg.vocab_size], logits[:, cfg.vocab_size:]
+        else:
+            heads = F.linear(normalized, w["token_embedding"]), F.linear(normalized, w["boundary_w"], w["boundary_b"])
         pos.add_(1)
-        return logits[:, :cfg.vocab_size], logits[:, cfg.vocab_size:]
+        return heads
+
+    @staticmethod
+    def _ids(tokens: Tensor, boundaries: Tensor) -> tuple[Tensor, Tensor]:
+        """Ids as an embedding lookup takes them (32 bits, one for all sequences), as the kernel does: int64 ``[B]`` each."""
+        if tokens.shape != boundaries.shape:
+            tokens, boundaries = torch.broadcast_tensors(tokens, boundaries)
+        if tokens.dim() != 1:
+            if tokens.dim() > 1:
+                raise ValueError("token and boundary ids must be [B]")
+            tokens, boundaries = tokens.view(1), boundaries.view(1)
+        if tokens.dtype == torch.int32:
+            tokens = tokens.long()
+        if boundaries.dtype == torch.int32:
+            boundaries = boundaries.long()
+        return tokens.contiguous(), boundaries.contiguous()
 
     def _normalize(self, rows: Tensor, weight: Tensor, bias: Tensor, out: Tensor) -> None:
         out.copy_(F.layer_norm(rows, (self.config.d_model,), weight, bias, self.config.norm_eps))

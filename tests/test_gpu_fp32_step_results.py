@@ -1,0 +1,50 @@
+"""What a single-precision step takes and returns, beside its values."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from gpu_util import assert_status_clear
+
+pytestmark = pytest.mark.gpu
+
+
+def _decoder(batch):
+    from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+    from relation_lm.inference.stateful_decode import StatefulDecoder
+
+    cfg = RoutedRelationConfig(vocab_size=50, boundary_vocab_size=6, d_model=64, layers=2, max_context=32, block_size=8,
+                               local_window=8, top_blocks=1)
+    return StatefulDecoder(RoutedRelationLM(cfg, seed=1), batch, "cuda", torch.float32)
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_results_belong_to_their_step(batch):
+    dec = _decoder(batch)
+    tokens, bounds = (torch.randint(0, n, (4, batch), device="cuda") for n in (50, 6))
+    kept, copies = [], []
+    for t in range(4):
+        results = (*dec.step(tokens[t], bounds[t]), dec.last_final)
+        assert results[0].is_contiguous() and results[1].is_contiguous()
+        assert results[0].shape == (batch, 50) and results[1].shape == (batch, 6)
+        kept.append(results)
+        copies.append([r.clone() for r in results])
+    assert all(torch.equal(a, b) for k, c in zip(kept, copies) for a, b in zip(k, c))
+    assert not torch.equal(kept[0][2], kept[1][2])
+    assert_status_clear()
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_ids_as_an_embedding_takes_them(batch):
+    """32-bit ids, and one id for all sequences."""
+    tokens = torch.arange(batch, device="cuda") + 7
+    for other in (torch.tensor([2], device="cuda"), torch.tensor(2, device="cuda"),
+                  torch.full((batch,), 2, device="cuda", dtype=torch.int32)):
+        want, got = _decoder(batch), _decoder(batch)
+        a = want.step(tokens, torch.full((batch,), 2, device="cuda"))
+        b = got.step(tokens.int(), other)
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    dec = _decoder(batch)
+    with pytest.raises(ValueError):
+        dec.step(tokens.view(batch, 1), tokens.view(batch, 1))
+    assert_status_clear()
