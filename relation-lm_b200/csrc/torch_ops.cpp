@@ -390,7 +390,9 @@ Tensor router_cache_update(const Tensor& anchor_raw, const Tensor& partner_raw, 
                           " must be a [B, 64] CUDA tensor with unit inner stride");
     require_position(position, device);
     const int64_t batch = anchor_raw.size(0);
-    TORCH_CHECK_VALUE(anchor_raw_cache.size(2) == 64 && anchor_mean.dim() == 4 && anchor_mean.size(2) * anchor_mean.size(3) == 64,
+    // a block's statistics are 64 values, split into heads or not
+    TORCH_CHECK_VALUE(anchor_raw_cache.size(2) == 64 && anchor_mean.dim() >= 3 &&
+                          c10::multiply_integers(anchor_mean.sizes().slice(2)) == 64,
                       "this build supports router width 64");
     Launch launch(device);
     Tensor out = empty({batch, 2, 64}, at::kFloat, device);

@@ -199,3 +199,21 @@ def test_projection_with_state_append_in_its_epilogue_equals_the_two_launch_form
     for mine, theirs in zip(tok1 + router1 + stats1, tok2 + router2 + stats2):
         assert torch.equal(mine, theirs)
     assert_status_clear()
+
+
+def test_update_takes_block_statistics_that_are_not_split_into_heads():
+    """``[B, NB, 64]`` as well as ``[B, NB, 4, 16]``: the same 64 values."""
+    case = cases.all_cases()["router_p8_b2"]
+    split, flat = to_cuda(cases.make_inputs(case)), to_cuda(cases.make_inputs(case))
+    for n in STATE[4:]:
+        flat[n] = flat[n].flatten(2)
+    for x in (split, flat):
+        x["anchor_raw"], x["partner_raw"] = x["packed"][:, 384:448], x["packed"][:, 448:512]
+    t, bs = case["position"], case["block_size"]
+    assert torch.equal(_run(split, t, bs), _run(flat, t, bs))
+    for n in STATE:
+        assert torch.equal(split[n].flatten(2), flat[n].flatten(2)), n
+    flat["anchor_mean"] = flat["anchor_mean"][..., :32].contiguous()
+    with pytest.raises(ValueError):
+        _run(flat, t, bs)
+    assert_status_clear()
