@@ -28,13 +28,13 @@ struct SelectInFront {
     }
 };
 
-template <bool kBf16>
+template <bool kBf16, bool kAligned>
 __global__ void __launch_bounds__(kLtThreads, 1) relation_layer_kernel(
     const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2,
     const LayerTailArgs tail, const SelectArgs sel) {
     extern __shared__ __align__(1024) unsigned char layer_smem_raw[];
     __shared__ __align__(8) unsigned long long select_bars[4];
-    layer_tail_body<kBf16>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16 ? RLM_BF16 : RLM_F16>{&sel, smem_u32(select_bars)});
+    layer_tail_body<kBf16, kAligned>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16 ? RLM_BF16 : RLM_F16>{&sel, smem_u32(select_bars)});
 }
 
 int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weight, const void* second_weight,
@@ -76,7 +76,8 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
         set_error("relation_layer: cuTensorMapEncodeTiled failed");
         return RLM_ERR_LAUNCH;
     }
-    auto kernel = tail.dtype == RLM_BF16 ? relation_layer_kernel<true> : relation_layer_kernel<false>;
+    auto kernel = lt_aligned(tail) ? (tail.dtype == RLM_BF16 ? relation_layer_kernel<true, true> : relation_layer_kernel<false, true>)
+                                   : (tail.dtype == RLM_BF16 ? relation_layer_kernel<true, false> : relation_layer_kernel<false, false>);
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), tail.cluster);
     if (rc != RLM_OK) return rc;
     const int clusters = (tail.n_seq + tail.seqs_per_cluster - 1) / tail.seqs_per_cluster;
@@ -108,7 +109,7 @@ extern "C" int rlm_relation_layer_supported(int n_seq, int k_out, int relation_d
     const uint32_t smem_bytes = lt_smem_bytes_with_stage(relation_dim, d_model, n_query / cluster, plan.total);
     const LtPlan whole = lt_plan(relation_dim, d_model, kLtMaxPairs, 0);
     if (plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) return 0;
-    auto kernel = dtype == RLM_BF16 ? relation_layer_kernel<true> : relation_layer_kernel<false>;
+    auto kernel = dtype == RLM_BF16 ? relation_layer_kernel<true, true> : relation_layer_kernel<false, true>;
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(cluster, 1, 1);

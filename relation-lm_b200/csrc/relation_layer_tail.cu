@@ -42,12 +42,12 @@
 namespace rlm {
 namespace {
 
-template <bool kBf16>
+template <bool kBf16, bool kAligned>
 __global__ void __launch_bounds__(kLtThreads, 1) relation_layer_tail_kernel(
     const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2,
     const LayerTailArgs a) {
     extern __shared__ __align__(1024) unsigned char lt_smem_raw[];
-    layer_tail_body<kBf16>(map_wm, map_w2, a, lt_smem_raw, NoStage{});
+    layer_tail_body<kBf16, kAligned>(map_wm, map_w2, a, lt_smem_raw, NoStage{});
 }
 
 }  // namespace
@@ -63,7 +63,7 @@ extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relat
     a.query = n_query > 0 ? &a : nullptr;
     if (lt_validate(a) != RLM_OK) return 0;
     const int cluster = hidden_dim / kLtHC;
-    auto kernel = dtype == RLM_BF16 ? relation_layer_tail_kernel<true> : relation_layer_tail_kernel<false>;
+    auto kernel = dtype == RLM_BF16 ? relation_layer_tail_kernel<true, true> : relation_layer_tail_kernel<false, true>;
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     // one cluster of this size, with this much shared memory per CTA, must fit the device
     cudaLaunchConfig_t config = {};
@@ -146,7 +146,8 @@ extern "C" int rlm_relation_layer_tail(
         set_error("relation_layer_tail: cuTensorMapEncodeTiled failed");
         return RLM_ERR_LAUNCH;
     }
-    auto kernel = dtype == RLM_BF16 ? relation_layer_tail_kernel<true> : relation_layer_tail_kernel<false>;
+    auto kernel = lt_aligned(a) ? (dtype == RLM_BF16 ? relation_layer_tail_kernel<true, true> : relation_layer_tail_kernel<false, true>)
+                                : (dtype == RLM_BF16 ? relation_layer_tail_kernel<true, false> : relation_layer_tail_kernel<false, false>);
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), a.cluster);
     if (rc != RLM_OK) return rc;
     const size_t smem_bytes = lt_smem_bytes(relation_dim, d_model, a.n_query / a.cluster);

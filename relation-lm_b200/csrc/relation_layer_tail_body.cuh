@@ -161,6 +161,11 @@ __device__ __forceinline__ void lt_tmem_ld4(uint32_t addr, uint32_t (&v)[4]) {
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
 }
 
+template <bool kAligned>
+__device__ __forceinline__ float4 lt_load4(const float* p) {
+    return kAligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
 __device__ __forceinline__ float lt_from16(uint16_t bits, int dtype) {
     return dtype == RLM_BF16 ? bf16_bits_to_float(bits) : __half2float(*reinterpret_cast<const __half*>(&bits));
 }
@@ -179,7 +184,10 @@ struct NoStage {
     __device__ __forceinline__ bool operator()(unsigned char*, uint32_t, int, int) const { return false; }
 };
 
-template <bool kBf16, typename Stage>
+// kAligned: the next LayerNorm's parameters lie on 16-byte boundaries and its rows on 8-byte ones.  Contiguous slices of
+// other tensors need not; they take a build of their own, because the test in the kernel costs every launch
+// instructions to fetch (a step of the 6-layer model at batch 1: 94.5 us, with the test 96.9).
+template <bool kBf16, bool kAligned, typename Stage>
 __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const CUtensorMap& map_w2,
                                                 const LayerTailArgs& a, unsigned char* lt_smem_raw, const Stage& stage) {
     // W_m, W_2, product GEMM done, second GEMM done; partial sums, pair statistics, residual rows received
@@ -231,8 +239,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         if (part + i * parts < mtiles && part < parts) {
-            next_g[i] = *reinterpret_cast<const float4*>(a.next_w + 128 * (part + i * parts) + 4 * lane);
-            next_b[i] = *reinterpret_cast<const float4*>(a.next_b + 128 * (part + i * parts) + 4 * lane);
+            next_g[i] = lt_load4<kAligned>(a.next_w + 128 * (part + i * parts) + 4 * lane);
+            next_b[i] = lt_load4<kAligned>(a.next_b + 128 * (part + i * parts) + 4 * lane);
         }
     int tpo = 16;                                              // threads per projection output: 2 .. 16
     while (tpo > 2 && (nseq * nq_own * tpo > kLtThreads || (D / 8) / tpo < 2)) tpo >>= 1;
@@ -648,8 +656,15 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 pack2(fmaf((v.z - mean) * rstd, g.z, b.z), fmaf((v.w - mean) * rstd, g.w, b.w), dtype));
             const int at = 128 * chunk + 4 * lane;
             *reinterpret_cast<uint2*>(rows16 + (my_seq * D + at) * 2) = out;
-            if (at / kLtOwn == static_cast<int>(rank) && !bad_position)
-                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(a.normalized) + static_cast<size_t>(s0 + my_seq) * D + at) = out;
+            if (at / kLtOwn == static_cast<int>(rank) && !bad_position) {
+                uint16_t* to = static_cast<uint16_t*>(a.normalized) + static_cast<size_t>(s0 + my_seq) * D + at;
+                if (kAligned) {
+                    *reinterpret_cast<uint2*>(to) = out;
+                } else {
+                    to[0] = static_cast<uint16_t>(out.x); to[1] = static_cast<uint16_t>(out.x >> 16);
+                    to[2] = static_cast<uint16_t>(out.y); to[3] = static_cast<uint16_t>(out.y >> 16);
+                }
+            }
         }
     }
     __syncthreads();
@@ -688,6 +703,10 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         if (*reinterpret_cast<volatile int*>(&failed)) atomicOr(a.status, RLM_DEV_TIMEOUT);
         if (bad_position) atomicOr(a.status, RLM_DEV_POSITION);
     }
+}
+
+inline bool lt_aligned(const LayerTailArgs& a) {
+    return aligned16(a.next_w) && aligned16(a.next_b) && (reinterpret_cast<uintptr_t>(a.normalized) & 7u) == 0;
 }
 
 int lt_validate(const LayerTailArgs& a) {

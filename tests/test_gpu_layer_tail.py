@@ -104,6 +104,26 @@ def test_layer_tail_repeats_bit_for_bit(B, d):
     assert_status_clear()
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_layer_tail_takes_slices_that_start_anywhere(offset):
+    """The next LayerNorm's parameters and the normalised rows as contiguous slices at 4-byte and 2-byte offsets."""
+    from relation_lm.kernels.relation_reduce import relation_layer_tail, relation_layer_tail_supported
+
+    if not relation_layer_tail_supported(5, 8, 128, 1024, 256, 256, torch.bfloat16):
+        pytest.skip("clusters of this size are not available on this device")
+    x = _case(5, 8, 256, 128, 40, 256, torch.bfloat16, 91)
+    want = _run(x, 39, torch.bfloat16)
+    dev = {k: (v.cuda() if isinstance(v, torch.Tensor) else v) for k, v in x.items()}
+    at = lambda t: torch.cat((t.new_zeros(offset), t.flatten()))[offset:].view(t.shape)  # noqa: E731
+    hidden, normalized = at(dev["hidden"]), at(torch.zeros(5, 256, device="cuda", dtype=torch.bfloat16))
+    query = at(torch.zeros(5, 256, device="cuda", dtype=torch.bfloat16))
+    relation_layer_tail(dev["expanded"], dev["operand"], dev["anchor"], dev["partner"], dev["scores"], dev["wm"],
+                        dev["w2"], at(dev["b2"]), at(dev["gamma"]), at(dev["beta"]), position_tensor(39), 1e-5, hidden,
+                        dev["mix"], at(dev["next_w"]), at(dev["next_b"]), 1e-5, normalized, dev["wq"], query)
+    assert torch.equal(hidden, want[0]) and torch.equal(normalized, want[1]) and torch.equal(query, want[2])
+    assert_status_clear()
+
+
 def test_layer_tail_rejects_shapes_it_does_not_serve():
     from relation_lm.kernels.relation_reduce import relation_layer_tail_supported
 
