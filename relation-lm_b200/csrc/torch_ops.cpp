@@ -18,7 +18,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/pybind11.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
@@ -957,6 +959,60 @@ Tensor skinny_projection_greedy_into(const Tensor& x, const Tensor& weight, cons
     return skinny_greedy(x, weight, bias, vocab, scratch, position, next_token, dense_rows({ARG(x)}));
 }
 
+// ------------------------------------------------------------------ what surrounds an operator
+
+using Stack = torch::jit::Stack;
+
+template <typename F>
+void for_each_tensor(const c10::IValue& v, F&& f) {
+    if (v.isTensor()) {
+        f(v.toTensor());
+    } else if (v.isTensorList()) {
+        for (const Tensor& t : v.toTensorList().vec()) f(t);
+    }
+}
+
+// Derivatives are not implemented: in grad mode floating-point results of arguments that require one carry a node that
+// raises when it is asked for it.  Arguments that are written stay as they are, a leaf included.  (PyTorch's own
+// fallback for such operators refuses to write a leaf that requires a derivative, and any forward-mode tangent.)
+void no_derivative(const c10::OperatorHandle& op, c10::DispatchKeySet keys, Stack* stack) {
+    const c10::FunctionSchema& schema = op.schema();
+    torch::autograd::variable_list inputs;
+    if (at::GradMode::is_enabled())
+        for (const c10::IValue& v : torch::jit::last(*stack, schema.arguments().size()))
+            for_each_tensor(v, [&](const Tensor& t) {
+                if (t.defined() && t.requires_grad()) inputs.push_back(t);
+            });
+    {
+        at::AutoDispatchBelowAutograd below;
+        op.redispatchBoxed(keys & c10::after_autograd_keyset, stack);
+    }
+    if (inputs.empty() || schema.returns().empty()) return;
+    const auto node = std::make_shared<torch::autograd::NotImplemented>(schema.name());
+    node->set_next_edges(torch::autograd::collect_next_edges(inputs));
+    for (const c10::IValue& v : torch::jit::last(*stack, schema.returns().size()))
+        for_each_tensor(v, [&](const Tensor& t) {
+            if (t.defined() && torch::autograd::isDifferentiableType(t.scalar_type())) torch::autograd::set_history(t, node);
+        });
+}
+
+// The version counters of the arguments that the schema marks as written advance.
+void bump_versions(const c10::OperatorHandle& op, c10::DispatchKeySet keys, Stack* stack) {
+    const auto& arguments = op.schema().arguments();
+    std::vector<Tensor> written;
+    const auto values = torch::jit::last(*stack, arguments.size());
+    for (size_t i = 0; i < arguments.size(); ++i)
+        if (arguments[i].alias_info() && arguments[i].alias_info()->isWrite())
+            for_each_tensor(values[i], [&](const Tensor& t) {
+                if (t.defined() && !t.is_inference()) written.push_back(t);
+            });
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        op.redispatchBoxed(keys & c10::after_ADInplaceOrView_keyset, stack);
+    }
+    for (const Tensor& t : written) t.unsafeGetTensorImpl()->bump_version();
+}
+
 Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int>(device_index)); }
 
 }  // namespace
@@ -969,9 +1025,8 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
     "Tensor partner_anchor_cache, Tensor partner_keys, Tensor partner_block_mean, Tensor partner_block_std, "            \
     "Tensor partner_gamma, Tensor partner_bias, "
 
-// Every operator with its schema, its implementation and the fallbacks that custom operators have:
-// derivatives are not implemented (an error when they are asked for), and with `MUTATES` the version
-// counters of the arguments that are written advance.
+// Every operator with its schema, its implementation and what surrounds it (above); with `MUTATES`, arguments that
+// are written.
 #define FOR_EACH_OP(PURE, MUTATES)                                                                                       \
     PURE(relation_select_packed, "(" SELECT_SCHEMA "Tensor position, SymInt local_window, SymInt top_blocks, "           \
          "SymInt k_out, bool strict_valid) -> (Tensor, Tensor, Tensor, Tensor)")                                         \
@@ -1067,8 +1122,8 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
 
 #define DEFINE(name, schema) m.def(#name schema, {at::Tag::pt2_compliant_tag});
 #define IMPLEMENT(name, schema) m.impl(#name, TORCH_FN(name));
-#define NO_DERIVATIVE(name, schema) m.impl(#name, torch::autograd::autogradNotImplementedFallback());
-#define BUMP_VERSIONS(name, schema) m.impl(#name, torch::autograd::autogradNotImplementedInplaceOrViewFallback());
+#define NO_DERIVATIVE(name, schema) m.impl(#name, torch::CppFunction::makeFromBoxedFunction<&no_derivative>());
+#define BUMP_VERSIONS(name, schema) m.impl(#name, torch::CppFunction::makeFromBoxedFunction<&bump_versions>());
 #define NOTHING(name, schema)
 
 TORCH_LIBRARY_FRAGMENT(relation_lm, m) {

@@ -60,3 +60,19 @@ def test_modes_see_the_operator():
     with Watch():
         relation_norm_reduce(*_reduce_args())
     assert any("relation_norm_reduce" in name for name in seen)
+
+
+@pytest.mark.parametrize("direct", [True, False])
+def test_a_saved_tensor_that_an_operator_overwrites_is_noticed(direct):
+    """By an operator that is called directly and by one that goes through the dispatcher."""
+    from relation_lm.kernels.relation_reduce import relation_norm_reduce_residual, relation_norm_reduce_residual_norm
+
+    raw, scores, weight, bias, position, eps = _reduce_args()
+    hidden, x = torch.randn(2, 64, device="cuda"), torch.ones(2, 64, device="cuda", requires_grad=True)
+    y, mix = (x * hidden).sum(), torch.ones((), device="cuda")          # keeps `hidden` for the backward pass
+    if direct:
+        relation_norm_reduce_residual_norm(raw, scores, weight, bias, position, eps, hidden, mix, weight, bias, eps, torch.empty_like(hidden))
+    else:
+        relation_norm_reduce_residual(raw, scores, weight, bias, position, eps, hidden, mix)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
