@@ -1151,8 +1151,9 @@ TORCH_LIBRARY_IMPL(relationlex, Autograd, m) { FOR_EACH_LEX_OP(NO_DERIVATIVE) }
 // An operator call through the dispatcher costs the host 2-4 us (boxing twenty arguments, the autograd and
 // version-counter fallbacks), as much as its launch, and the passes of a small model are bound by exactly that.
 // Each operator is therefore a plain extension function too.  It returns NotImplemented, and the caller takes the
-// dispatcher, whenever the dispatcher would have anything to do: arguments that are not plain CUDA tensors, a
-// derivative to record, a mode, a tracer, a transform or a profiler at work.
+// dispatcher, whenever the dispatcher would have anything to do: arguments that are not plain CUDA tensors (views that
+// are still to be negated, tensors of zeros without memory and the like among them), a derivative to record, a mode, a
+// tracer, a transform or a profiler at work.
 namespace {
 
 using c10::DispatchKey;
@@ -1163,7 +1164,9 @@ constexpr DispatchKeySet kInterposing({DispatchKey::Python, DispatchKey::PythonT
                                        DispatchKey::Batched, DispatchKey::VmapMode, DispatchKey::FuncTorchBatched,
                                        DispatchKey::FuncTorchVmapMode, DispatchKey::FuncTorchGradWrapper,
                                        DispatchKey::FuncTorchDynamicLayerFrontMode, DispatchKey::FuncTorchDynamicLayerBackMode,
-                                       DispatchKey::FuncTorchBatchedDecomposition, DispatchKey::TESTING_ONLY_GenericWrapper,
+                                       DispatchKey::FuncTorchBatchedDecomposition, DispatchKey::Negative, DispatchKey::Conjugate,
+                                       DispatchKey::ZeroTensor, DispatchKey::Sparse, DispatchKey::SparseCsr,
+                                       DispatchKey::Quantized, DispatchKey::NestedTensor, DispatchKey::TESTING_ONLY_GenericWrapper,
                                        DispatchKey::TESTING_ONLY_GenericMode});
 
 bool nothing_interposed() {

@@ -76,3 +76,13 @@ def test_a_saved_tensor_that_an_operator_overwrites_is_noticed(direct):
         relation_norm_reduce_residual(raw, scores, weight, bias, position, eps, hidden, mix)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.backward()
+
+
+def test_views_that_are_still_to_be_negated():
+    """The imaginary part of a conjugate is a view with a sign that the dispatcher resolves before the kernel."""
+    from relation_lm.kernels.relation_reduce import relation_norm_reduce
+
+    args = _reduce_args()
+    lazy = torch._neg_view(args[1])
+    assert lazy.is_neg()
+    assert torch.equal(relation_norm_reduce(args[0], lazy, *args[2:]), relation_norm_reduce(args[0], lazy.resolve_neg(), *args[2:]))
