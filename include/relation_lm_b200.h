@@ -62,8 +62,10 @@ typedef enum {
  * provided the caller keeps one rule: the key caches, block statistics and the `position` scalar
  * passed to a selector must not be written by the kernel launched immediately before it on the
  * same stream (in a decode step they are written by the cache append, several launches earlier).
- * Returns the previous setting.  The setting belongs to the calling host thread (another thread's
- * launches are not affected) and is read at launch (capture) time.
+ * enabled = 2: from the second launch on, for a composition whose first kernel must not read its weights
+ * and parameters ahead of a kernel of the caller's that writes them.
+ * Returns the previous setting (2 until that first launch).  The setting belongs to the calling host thread
+ * (another thread's launches are not affected) and is read at launch (capture) time.
  */
 int rlm_set_programmatic_launch(int enabled);
 

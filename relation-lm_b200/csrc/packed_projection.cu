@@ -666,6 +666,8 @@ struct NormCastArgs {
 
 template <int kChunks, int kDt>
 __global__ void __launch_bounds__(kCastThreads) layer_norm_cast_kernel(const NormCastArgs a) {
+    // Whole-sequence passes begin with this kernel, so its parameters may have been written by whatever ran before.
+    griddep_sync();
     const int lane = threadIdx.x & 31, chunks = a.k / 8;
     float4 g[kChunks][2], b[kChunks][2];
 #pragma unroll
@@ -678,7 +680,6 @@ __global__ void __launch_bounds__(kCastThreads) layer_norm_cast_kernel(const Nor
             b[i][h] = live ? *reinterpret_cast<const float4*>(a.beta + 8 * c + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-    griddep_sync();
     const int warps = gridDim.x * (kCastThreads / 32);
     for (int r = blockIdx.x * (kCastThreads / 32) + (threadIdx.x >> 5); r < a.m; r += warps) {
         const float* row = a.x + r * a.x_stride;

@@ -24,7 +24,11 @@ void set_error(const char* message) {
 // thread's launches (for instance the plain operators, whose callers know nothing of the
 // ordering rule that comes with programmatic launch) are issued.
 thread_local int g_programmatic = 0;
-bool programmatic_launch_enabled() { return g_programmatic != 0; }
+bool programmatic_launch_enabled() {
+    if (g_programmatic != 2) return g_programmatic != 0;
+    g_programmatic = 1;                // from the next launch on
+    return false;
+}
 
 int sm_count() {
     static std::atomic<int> cached[64];
@@ -81,7 +85,7 @@ int allow_large_smem(const void* kernel, int bytes) {
 
 extern "C" int rlm_set_programmatic_launch(int enabled) {
     const int previous = rlm::g_programmatic;
-    rlm::g_programmatic = enabled ? 1 : 0;
+    rlm::g_programmatic = enabled == 2 ? 2 : enabled ? 1 : 0;
     return previous;
 }
 extern "C" int rlm_abi_version(void) { return RLM_ABI_VERSION; }

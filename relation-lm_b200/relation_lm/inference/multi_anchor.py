@@ -204,7 +204,7 @@ class MultiAnchorPrefill:
         rp = torch.arange(length, device=self.device, dtype=torch.int32).repeat(batch)
         return rb, rp
 
-    @_abi.programmatic_launch
+    @_abi.programmatic_launch(first=False)                   # the memory projection requests its weights early
     def build_state(self, layer: int, memory: Tensor) -> dict[str, Tensor]:
         """Per-slot caches and block statistics of layer ``layer`` for ``memory [B, T, d]`` (16-bit)."""
         from relation_lm.kernels.packed_projection import packed_projection
@@ -293,6 +293,7 @@ class MultiAnchorPrefill:
                         hidden_rel=hidden_rel, raw=raw, slot_context=slot_context, row_batch=rb, row_position=rp)
         return hidden
 
+    @_abi.programmatic_launch(first=False)
     def forward(self, hidden: Tensor, memory: Tensor, keep: list | None = None) -> Tensor:
         """The stack's output ``[B, T, d]`` (fp32): ``depth`` layers on a copy of ``hidden`` with one
         shared ``memory`` (16-bit), then the final LayerNorm."""

@@ -145,16 +145,24 @@ def set_programmatic_launch(enabled: bool) -> bool:
     return bool(LIB.rlm_set_programmatic_launch(1 if enabled else 0))
 
 
-def programmatic_launch(function):
+def programmatic_launch(function=None, *, first: bool = True):
     """Decorator: programmatic dependent launch for the kernels that ``function`` launches.  For compositions that
-    keep the rule above: each kernel's set-up then overlaps its predecessor's end (1-2 us a launch)."""
+    keep the rule above: each kernel's set-up then overlaps its predecessor's end (1-2 us a launch).  What comes before
+    a composition is the caller's and may still be writing its weights: ``first = False`` launches the first kernel in
+    the ordinary way, for compositions whose first kernel reads any before its dependency wait."""
+    if function is None:
+        return functools.partial(programmatic_launch, first=first)
+
     @functools.wraps(function)
     def wrapped(*args, **kwargs):
-        previous = set_programmatic_launch(True)
+        previous = LIB.rlm_set_programmatic_launch(1 if first else 2)
+        if previous:                                        # part of another composition
+            LIB.rlm_set_programmatic_launch(previous)
+            return function(*args, **kwargs)
         try:
             return function(*args, **kwargs)
         finally:
-            set_programmatic_launch(previous)
+            LIB.rlm_set_programmatic_launch(0)
     return wrapped
 
 

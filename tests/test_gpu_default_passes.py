@@ -44,3 +44,14 @@ def test_prefill_of_blocks_beyond_the_state_kernels_tile(block):
     # one selection on both sides, the relation MLP in one kernel or three: its rounding steps (see test_gpu_relation_mlp)
     assert float((layer.forward(x, state) - kept).abs().max()) <= 2 * 2 ** -8 * float(keep["context"].abs().max().clamp_min(1.0))
     assert_status_clear()
+
+
+def test_only_the_first_launch_of_a_composition_is_ordinary():
+    from relation_lm.kernels import _abi
+    from relation_lm.kernels.packed_projection import layer_norm_cast
+
+    x, w = _rows(1, 4, 64).view(4, 64), torch.ones(64, device="cuda")
+    assert _abi.LIB.rlm_set_programmatic_launch(2) == 0
+    layer_norm_cast(x, w, w, 1e-5, torch.empty_like(x))
+    assert _abi.LIB.rlm_set_programmatic_launch(0) == 1
+    assert_status_clear()
