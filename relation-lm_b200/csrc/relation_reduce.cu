@@ -961,7 +961,8 @@ int norm_reduce_launch(
     const bool plain_rows = raw_dtype == RLM_BF16 && param_dtype == RLM_F32 && a.raw_splits == 1 && !raw_bias &&
                             (!next_normalized || next_dtype == RLM_BF16);
     if (vec && plain_rows && n_rows <= sm_count()) {
-        // a row per SM at most: a row's latency counts, so everything it needs is requested at the top
+        // a row per SM at most: a row's latency counts, so everything it needs is requested at the top (measured, and
+        // built, for bfloat16 rows; float16 rows take the general build below)
         auto kernel = dim <= 512 ? relation_norm_reduce_vec_kernel<2, true, true> : dim <= 768 ? relation_norm_reduce_vec_kernel<3, true, true>
                                                                                                : relation_norm_reduce_vec_kernel<4, true, true>;
         launch_kernel(kernel, dim3(n_rows), dim3(kNormThreads), smem_bytes, stream, a);

@@ -1256,7 +1256,8 @@ __global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_sel
 // leave issue slots unused but end sooner (relative lengths below from one round of each: 27, 23, 21 and 19 us for
 // 512 positions, launch and staging included, and 341, 339, 403 and 477 us for 8 x 4096).  The shape of least waves x
 // rounds x length that fits the shared memory is taken: 8 x 4096 positions run as 1024 tiles of 32, 3 x 1984 as 126 of
-// 48 (as 249 of 24 they take 53 us, as 186 of 32 67 us), 512 as 64 of 8.
+// 48 (as 249 of 24 they take 53 us, as 186 of 32 67 us), 512 as 64 of 8.  The lengths are those of the single-anchor
+// 16-bit builds; the multi-anchor and the fp32 builds follow the same rule without having been measured for it.
 struct TileShape { int warps, per_warp, smem_bytes; };
 
 template <typename Smem>

@@ -246,8 +246,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // Dynamic shared memory from its first multiple of 1024 bytes (the swizzle atom).  By an offset, not by rounding the
 // address as an integer: through an integer the compiler loses that it is shared memory, and every access by pointer
-// becomes a generic one with a 64-bit address (the relation MLP spilled 252 bytes a thread that way, 136 this way;
-// a pass over 8 x 4096 rows 1375 -> 1335 us).
+// becomes a generic one with a 64-bit address (the relation MLP spilled 232 bytes a thread and loaded 252
+// back that way, 136 and 228 this way; a pass over 8 x 4096 rows 1375 -> 1335 us).
 __device__ __forceinline__ unsigned char* smem_align1024(unsigned char* raw) {
     return raw + ((0u - smem_u32(raw)) & 1023u);
 }

@@ -1290,6 +1290,9 @@ PyObject* direct(PyObject*, PyObject* const* args, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// The operators that passes without a captured graph call: a position operator by operator, the single-precision step
+// and the whole-sequence passes.  The 16-bit step is replayed from a graph, where a call costs the host nothing; the
+// operators that only it uses go through the dispatcher.
 #define METHOD(name) \
     {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&direct<&name>)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {METHOD(relation_select_packed), METHOD(relation_select_packed_rows), METHOD(relation_select_packed_prefill),
