@@ -67,11 +67,19 @@ def _step(dtype):
     (torch.float16, {"d_model": 512, "top_blocks": 4, "block_size": 32}), (torch.bfloat16, {"k_max": 6}),          # K 6: three kernels
 ])
 def test_prefill_equals_its_form_of_separate_kernels(dtype, sizes):
+    _prefill_equals_separate_kernels(dtype, sizes, 3)
+
+
+def test_prefill_of_eight_long_contexts_equals_its_form_of_separate_kernels():
+    _prefill_equals_separate_kernels(torch.bfloat16, dict(d_model=512, max_context=4096, block_size=64, local_window=128, top_blocks=4), 8)
+
+
+def _prefill_equals_separate_kernels(dtype, sizes, batch):
     """From the same state and rows: one selection on both sides, values within the relation MLP's rounding steps."""
     layer = _layer(dtype, **sizes)
     cfg = layer.config
     assert layer.fused_mlp == (cfg.k_max != 6)
-    x = _rows(3, cfg.max_context, cfg.d_model)
+    x = _rows(batch, cfg.max_context, cfg.d_model)
     state, keep = layer.build_state(x), {}
     kept, out = layer.forward(x, state, keep), layer.forward(x, state)
     assert float((out - kept).abs().max()) <= _step(dtype) * float(keep["context"].abs().max().clamp_min(1.0)) * float(layer.w["mix"])
@@ -90,11 +98,19 @@ def _stack(dtype, **sizes):
 @pytest.mark.parametrize("dtype,slots,d", [(torch.bfloat16, 4, 256), (torch.float16, 2, 256), (torch.bfloat16, 3, 256),
                                            (torch.bfloat16, 4, 512), (torch.float16, 3, 512)])
 def test_multi_anchor_equals_its_form_of_separate_kernels(dtype, slots, d):
+    _multi_anchor_equals_separate_kernels(dtype, slots, d, 2, 192)
+
+
+def test_multi_anchor_of_long_contexts_equals_its_form_of_separate_kernels():
+    _multi_anchor_equals_separate_kernels(torch.bfloat16, 4, 512, 16, 2048, block_size=32, local_window=64, top_blocks=3)
+
+
+def _multi_anchor_equals_separate_kernels(dtype, slots, d, batch, length, **sizes):
     """Layer by layer from the same residual stream (over several layers a rounding may decide a near tie), then the
     whole pass as the chain of its layers: entry of the first one from its source, and the final LayerNorm."""
-    stack = _stack(dtype, anchors_per_block=slots, d_model=d)
+    stack = _stack(dtype, anchors_per_block=slots, d_model=d, max_context=length, **sizes)
     assert stack.fused_mlp and stack.fused_mix == (slots != 3)                          # three slots: mixed on their own
-    hidden, memory = _rows(2, 192, d), _rows(2, 192, d, seed=6).to(dtype)
+    hidden, memory = _rows(batch, length, d), _rows(batch, length, d, seed=6).to(dtype)
     stream = hidden.clone()
     for layer in range(2):
         state, keep = stack.build_state(layer, memory), {}
