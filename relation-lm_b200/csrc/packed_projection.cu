@@ -218,7 +218,14 @@ __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
 //   warp 0, one lane: TMA producer, a ring of stages (x rows x 64 | w 256 x 64);
 //   warp 1, one lane: tcgen05.mma 128 x 256 x 16;
 //   warps 2-9: epilogue (tcgen05.ld, bias, convert, store; two warps per quarter of the TMEM lanes,
-//   128 columns each).
+//   128 columns each).  16-bit results go through shared memory, 32 rows x 64 columns at a time, and leave by
+//   TMA stores, which also clip the last row and column tiles: whole 128-byte segments, and nobody waits for them.
+//   Stored by the threads instead, a warp's instruction touched 32 rows, 16 bytes of each, and the bias came as 32
+//   scalar loads per 32 columns.  us, before and now: 32768 x 128 x 4096 with bias 126 -> 56 (268 MB written: 4.9 of
+//   6.5 TB/s), 5952 x 128 x 6144 with bias 47 -> 20, 32768 x 512 x 1664 84 -> 54 (1.03 PFLOP/s; by the kernel
+//   above, before ragged widths came here), 262144 x 2048 x 512 with bias 454 -> 415.
+// Ring depth: with short reductions the output is what counts and three stages leave room for two output boxes a warp;
+//   longer ones without a bias take four stages and one box (32768 x 512 x 1664: 58.7 -> 54.1 us).
 // kRowTiles = 1: tiles of 128 x 256, two accumulators (2 x 256 TMEM columns) used by alternate
 // tiles, so that a tile's epilogue runs behind the next tile's main loop.
 // kRowTiles = 2: tiles of 256 x 256 — two row tiles share every w tile, which halves the weight
@@ -228,6 +235,9 @@ __global__ void __launch_bounds__(kGemmThreads) packed_projection_kernel(
 // start as soon as the epilogue has read it out.
 constexpr int kPgThreads = 320;
 constexpr int kPgBN = 256;
+constexpr uint32_t kPgBox = 32 * 128;            // 32 rows x 64 columns of 16 bits
+// Output boxes per epilogue warp: two, where the ring of 48 KB stages leaves room for them.
+__host__ __device__ constexpr int pg_buffers(int row_tiles, int stages) { return row_tiles == 1 && stages == 3 ? 2 : 1; }
 
 struct PersistentGemmArgs {
     void* out;
@@ -236,19 +246,29 @@ struct PersistentGemmArgs {
     int m, n, k, out_dtype;
     uint32_t idesc;
     int tiles_n, tiles;
+    int staged;              // 16-bit results through shared memory and map_out
+    int bias_vec;            // bias on a 16-byte boundary
 };
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-template <int kRowTiles>
+template <int kRowTiles, int kStages>
 __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-    const PersistentGemmArgs a) {
+    const __grid_constant__ CUtensorMap map_out, const PersistentGemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    constexpr int kStages = kRowTiles == 2 ? 3 : 4;
+    constexpr int kBuffers = pg_buffers(kRowTiles, kStages);
+    constexpr bool kBiasRows = kRowTiles == 1 && kStages == 3;
     __shared__ __align__(8) unsigned long long bars[2 * kStages + 4];
+    __shared__ __align__(16) float bias_rows[kBiasRows ? 8 * kPgBN / 2 : 4];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
 
@@ -341,11 +361,24 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
         // epilogue warps 2 .. 9: TMEM lanes 32 (warp % 4) .., one output row and 128 columns per thread
         const int quarter = warp & 3, col_half = (warp - 2) >> 2;
         const uint32_t lane_base = static_cast<uint32_t>(32 * quarter) << 16;
+        float* bias_s = bias_rows + (kBiasRows ? (warp - 2) * (kPgBN / 2) : 0);
+        const uint32_t box = ring_addr + kStages * kStageBytes + static_cast<uint32_t>((warp - 2) * kBuffers) * kPgBox;
+        const uint32_t cell = box + static_cast<uint32_t>(lane * 128 + ((lane & 7) << 4));      // chunk c: cell ^ (c << 4)
         int j = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < a.tiles && ok; tile += gridDim.x, ++j) {
             const int b = kRowTiles == 1 ? (j & 1) : 0;
-            const int m0 = (tile / a.tiles_n) * kTileRows, n0 = (tile % a.tiles_n) * kPgBN;
+            const int m0 = (tile / a.tiles_n) * kTileRows, n0 = (tile % a.tiles_n) * kPgBN + col_half * (kPgBN / 2);
+            if (kBiasRows && a.bias) {                      // this warp's columns, a lane four of them
+                const int col = n0 + 4 * lane;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (col < a.n)                                   // (a.n is a multiple of 32)
+                    v = a.bias_vec ? *reinterpret_cast<const float4*>(a.bias + col)
+                                   : make_float4(a.bias[col], a.bias[col + 1], a.bias[col + 2], a.bias[col + 3]);
+                __syncwarp();                                    // the previous tile's reads
+                *reinterpret_cast<float4*>(bias_s + 4 * lane) = v;
+                __syncwarp();
+            }
             ok = mbar_wait(acc_full(b), kRowTiles == 1 ? ((j >> 1) & 1) : (j & 1));
             ok = __all_sync(0xffffffffu, ok) && (*reinterpret_cast<volatile int*>(&failed) == 0);
             if (!ok) break;
@@ -353,14 +386,20 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
 #pragma unroll 1
             for (int r = 0; r < kRowTiles; ++r) {
                 const int accn = kRowTiles == 1 ? b : r;
-                const int row = m0 + kBM * r + 32 * quarter + lane;
+                const int first_row = m0 + kBM * r + 32 * quarter, row = first_row + lane;
+                const uint32_t acc = tmem_base + lane_base + static_cast<uint32_t>(accn * kPgBN + col_half * (kPgBN / 2));
 #pragma unroll 1
-                for (int c = col_half * (kPgBN / 2); c < (col_half + 1) * (kPgBN / 2); c += 32) {
+                for (int c = 0; c < kPgBN / 2; c += 32) {
                     uint32_t v[32];
-                    tmem_ld16(tmem_base + lane_base + accn * kPgBN + c, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
-                    tmem_ld16(tmem_base + lane_base + accn * kPgBN + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&v[16]));
+                    tmem_ld16(acc + c, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
+                    tmem_ld16(acc + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&v[16]));
+                    const uint32_t buffer = kBuffers == 2 ? static_cast<uint32_t>(c >> 6) * kPgBox : 0u;
+                    if (a.staged && (c & 32) == 0) {             // the buffer's previous store has read it
+                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kBuffers - 1) : "memory");
+                        __syncwarp();
+                    }
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (c + 32 == (col_half + 1) * (kPgBN / 2)) {
+                    if (c + 32 == kPgBN / 2) {
                         // this warp's share of the accumulator is in registers: hand it back to the MMA warp
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
@@ -368,36 +407,42 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
                     }
                     if (a.bias) {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + a.bias[n0 + c + i]);
+                        for (int i = 0; i < 32; i += 4) {
+                            const float* at = a.bias + n0 + c + i;
+                            const float4 add = kBiasRows ? *reinterpret_cast<const float4*>(bias_s + c + i) : make_float4(at[0], at[1], at[2], at[3]);
+                            v[i] = __float_as_uint(__uint_as_float(v[i]) + add.x);
+                            v[i + 1] = __float_as_uint(__uint_as_float(v[i + 1]) + add.y);
+                            v[i + 2] = __float_as_uint(__uint_as_float(v[i + 2]) + add.z);
+                            v[i + 3] = __float_as_uint(__uint_as_float(v[i + 3]) + add.w);
+                        }
                     }
-                    if (row >= a.m) continue;
-                    const size_t at = static_cast<size_t>(row) * a.n + n0 + c;
-                    if (a.out_dtype == RLM_F32) {
-                        float4* o = reinterpret_cast<float4*>(static_cast<float*>(a.out) + at);
+                    if (!a.staged) {                             // fp32 results (a.n a multiple of 256)
+                        if (row >= a.m) continue;
+                        float4* o = reinterpret_cast<float4*>(static_cast<float*>(a.out) + static_cast<size_t>(row) * a.n + n0 + c);
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             o[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                                                __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-                    } else {
-                        uint32_t packed[16];
+                        continue;
+                    }
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float lo = __uint_as_float(v[2 * i]), hi = __uint_as_float(v[2 * i + 1]);
-                            if (a.out_dtype == RLM_BF16) {
-                                __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                                packed[i] = *reinterpret_cast<uint32_t*>(&h);
-                            } else {
-                                __half2 h = __floats2half2_rn(lo, hi);
-                                packed[i] = *reinterpret_cast<uint32_t*>(&h);
-                            }
-                        }
-                        uint4* o = reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.out) + at);
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t w[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) o[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+                        for (int e = 0; e < 4; ++e)
+                            w[e] = pack2(__uint_as_float(v[8 * i + 2 * e]), __uint_as_float(v[8 * i + 2 * e + 1]), a.out_dtype);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"((cell ^ static_cast<uint32_t>((((c & 32) >> 3) + i) << 4)) + buffer), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+                    }
+                    if (c & 32) {
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0 && first_row < a.m && n0 + c - 32 < a.n) tma_store_2d(&map_out, box + buffer, n0 + c - 32, first_row);
                     }
                 }
             }
         }
+        if (a.staged && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (!ok && lane == 0) failed = 1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -408,17 +453,16 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
                      ::"r"(tmem_base), "r"(2 * kPgBN) : "memory");
 }
 
-template <int kRowTiles>
-int launch_persistent_gemm(const CUtensorMap& mx, const CUtensorMap& mw, PersistentGemmArgs& a, void* stream) {
-    constexpr int kStages = kRowTiles == 2 ? 3 : 4;
-    const int smem_bytes = kStages * (kRowTiles * kBM * kBK * 2 + kPgBN * kBK * 2) + 1024;
-    auto kernel = packed_projection_persistent_kernel<kRowTiles>;
+template <int kRowTiles, int kStages>
+int launch_persistent_gemm(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, PersistentGemmArgs& a, void* stream) {
+    const int smem_bytes = kStages * (kRowTiles * kBM * kBK * 2 + kPgBN * kBK * 2) + 8 * pg_buffers(kRowTiles, kStages) * static_cast<int>(kPgBox) + 1024;
+    auto kernel = packed_projection_persistent_kernel<kRowTiles, kStages>;
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
-    a.tiles_n = a.n / kPgBN;
+    a.tiles_n = (a.n + kPgBN - 1) / kPgBN;
     a.tiles = a.tiles_n * ((a.m + kRowTiles * kBM - 1) / (kRowTiles * kBM));
     const int ctas = a.tiles < sm_count() ? a.tiles : sm_count();
-    launch_kernel(kernel, dim3(ctas), dim3(kPgThreads), smem_bytes, stream, mx, mw, a);
+    launch_kernel(kernel, dim3(ctas), dim3(kPgThreads), smem_bytes, stream, mx, mw, mo, a);
     count_launch();
     return check_launch("packed_projection_persistent_kernel");
 }
@@ -885,22 +929,30 @@ extern "C" int rlm_packed_projection(const void* x, int64_t x_row_stride, const 
         return RLM_ERR_SHAPE;
     }
     const int m_tiles = (rows + kBM - 1) / kBM;
-    if (k_splits == 1 && n_out % kPgBN == 0 && d_in % kBK == 0 && m_tiles * (n_out / kPgBN) >= 2 * sm_count()) {
-        // at least two 128 x 256 tiles per SM: persistent CTAs; 256 x 256 tiles when there are two of those per SM
+    // Persistent CTAs from 5 tiles of 128 x 256 for 8 SMs on (us by the other kernel -> here: 3168 x 256 x 896, 100 tiles,
+    // 6.6 -> 6.2; 5952 x 768 x 512, 94 tiles, 9.4 -> 8.9; 3168 x 128 x 2048, 200 tiles, 12.5 -> 7.9; 9001 x 512 x 256,
+    // 71 tiles, 6.8 -> 7.5).  fp32 results are stored by the threads: at least two tiles per SM, whole tiles of columns.
+    const int wide_tiles = (n_out + kPgBN - 1) / kPgBN, big_tiles = m_tiles * wide_tiles;
+    const bool staged = out_dtype != RLM_F32;
+    if (k_splits == 1 && d_in % kBK == 0 && (staged ? rows >= kBM && 8 * big_tiles >= 5 * sm_count() : n_out % kPgBN == 0 && big_tiles >= 2 * sm_count())) {
+        // 256 x 256 tiles when there are two of those per SM
         // (a 256-row tile's epilogue is not hidden behind the next main loop: it pays only with a long reduction)
-        const bool tall = d_in >= 1024 && ((rows + 2 * kBM - 1) / (2 * kBM)) * (n_out / kPgBN) >= 2 * sm_count();
-        CUtensorMap px, pw;
+        const bool tall = d_in >= 1024 && n_out % kPgBN == 0 && ((rows + 2 * kBM - 1) / (2 * kBM)) * (n_out / kPgBN) >= 2 * sm_count();
+        CUtensorMap px, pw, po;
         if (!make_map(&px, x, rows, d_in, x_row_stride, tall ? 2 * kBM : kBM, in_dtype) ||
-            !make_map(&pw, weight, n_out, d_in, d_in, kPgBN, in_dtype)) {
+            !make_map(&pw, weight, n_out, d_in, d_in, kPgBN, in_dtype) ||
+            !make_map(&po, out, rows, n_out, n_out, 32, staged ? out_dtype : in_dtype)) {
             set_error("packed_projection: cuTensorMapEncodeTiled failed");
             return RLM_ERR_LAUNCH;
         }
         PersistentGemmArgs p{};
         p.out = out; p.bias = bias; p.status = status; p.m = rows; p.n = n_out; p.k = d_in; p.out_dtype = out_dtype;
+        p.staged = staged; p.bias_vec = aligned16(bias);
         const uint32_t pfmt = in_dtype == RLM_BF16 ? 1u : 0u;
         p.idesc = (1u << 4) | (pfmt << 7) | (pfmt << 10) | (static_cast<uint32_t>(kPgBN >> 3) << 17) |
                   (static_cast<uint32_t>(kBM >> 4) << 24);
-        return tall ? launch_persistent_gemm<2>(px, pw, p, stream) : launch_persistent_gemm<1>(px, pw, p, stream);
+        if (tall) return launch_persistent_gemm<2, 3>(px, pw, po, p, stream);
+        return bias || d_in <= 4 * kBK ? launch_persistent_gemm<1, 3>(px, pw, po, p, stream) : launch_persistent_gemm<1, 4>(px, pw, po, p, stream);
     }
     // Tile width: with few rows the weight read dominates, so pick the widest tile that still
     // gives about one CTA per SM; with many rows use wide tiles.

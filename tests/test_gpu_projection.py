@@ -324,3 +324,29 @@ def test_many_rows_projection_matches_torch_and_oracle(rows, d_in, n_out, dtype,
     again = packed_projection(xg, wg, b.cuda() if bias else None)
     assert torch.equal(got, again)
     assert_status_clear()
+
+
+@pytest.mark.parametrize("rows,d_in,n_out,dtype,bias", [
+    (2999, 128, 1664, torch.bfloat16, True),       # last column tile half empty, last rows inside an output box
+    (6273, 320, 288, torch.float16, False),        # 32 columns and one row of the last tiles; ring of four, five K-blocks
+    (5952, 64, 512, torch.bfloat16, True),         # 94 tiles (the fewest), one K-block
+    (24065, 128, 160, torch.float16, True),        # one column tile, a box of 32 columns
+    (12000, 576, 224, torch.bfloat16, False),
+])
+def test_persistent_projection_at_ragged_edges(rows, d_in, n_out, dtype, bias):
+    """Output boxes that the last rows and columns cut, and a bias off a 16-byte boundary, on persistent CTAs: within
+    1e-2 of the row's largest magnitude of torch's fp32 product, and nothing written beyond the result."""
+    from relation_lm.kernels import _abi
+
+    g = torch.Generator().manual_seed(rows + n_out)
+    x = torch.randn(rows, d_in, generator=g).to(dtype).cuda()
+    w = (torch.randn(n_out, d_in, generator=g) * 0.05).to(dtype).cuda()
+    b = torch.randn(n_out + 1, generator=g).cuda()[1:] if bias else None
+    room = torch.full((rows * n_out + 4096,), 7.0, dtype=dtype, device="cuda")
+    _abi.check(_abi.LIB.rlm_packed_projection(_abi.ptr(x), x.stride(0), _abi.ptr(w), _abi.ptr(b) if bias else None, _abi.ptr(room), rows,
+                                              d_in, n_out, _abi.code(x), _abi.code(room), 1,
+                                              _abi.ptr(_abi.status_tensor(x.device)), _abi.stream_ptr(x.device)))
+    want = x.float() @ w.float().T + (b if bias else 0.0)
+    assert_rel_close(room[:rows * n_out].view(rows, n_out), want, 1e-2)
+    assert bool((room[rows * n_out:] == 7.0).all())
+    assert_status_clear()
