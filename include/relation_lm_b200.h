@@ -576,6 +576,17 @@ int rlm_skinny_projection(const void* x, int64_t x_row_stride, const void* weigh
                           void* argmax_scratch, int64_t* next_token, int64_t* position, void* stream);
 
 /*
+ * Projection of a few rows in single precision (extension): out [rows, n_out] = x [rows, d_in] @ weight [n_out, d_in].T
+ * (+ bias [n_out], optional) and, in the same launch, out2 [rows, n_out2] with weight2 / bias2 (optional: n_out2 0).  fp32
+ * throughout, sums in a fixed order.  Stands where the reference calls F.linear on the rows of one decode position
+ * (src/relation_lm/inference/packed_cache.py:52-57 and the heads of src/relation_lm/models/relation_lm.py:121-124).
+ * rows <= 64, d_in and the row stride of x multiples of 4; x and the weights 16-byte aligned.
+ */
+int rlm_few_rows_projection(const float* x, int64_t x_row_stride, const float* weight, const float* bias, float* out,
+                            const float* weight2, const float* bias2, float* out2, int rows, int d_in, int n_out,
+                            int n_out2, void* stream);
+
+/*
  * Packed sparse-cache projection of one decode position for every layer, with the state update in
  * its epilogue (extension): what a reference decode step does with
  * PackedSparseCacheProjection.project (src/relation_lm/inference/packed_cache.py:52-57), the four

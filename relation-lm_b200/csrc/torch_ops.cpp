@@ -918,6 +918,34 @@ Tensor greedy_token(const Tensor& logits, int64_t vocab, const OptTensor& positi
     return out;
 }
 
+void few_rows(Tensor& out, Tensor* out2, const Tensor& x, const Tensor& weight, const Tensor* weight2, const OptTensor& bias,
+              const OptTensor& bias2) {
+    const c10::Device device = dense_rows({ARG(x)});
+    TORCH_CHECK_VALUE(contiguous({ARG(out), ARG(weight), Named{"out2", out2}, Named{"weight2", weight2}, OPT(bias), OPT(bias2)}) == device,
+                      "weights and results must be on the device of x");
+    const auto fits = [&](const Tensor& o, const Tensor& w, const OptTensor& b) {
+        TORCH_CHECK_VALUE(is_f32(x) && is_f32(w) && is_f32(o) && (!b.has_value() || is_f32(*b)), "few_rows_projection takes float32 tensors");
+        TORCH_CHECK_VALUE(w.dim() == 2 && w.size(1) == x.size(1) && is_shape(o, {x.size(0), w.size(0)}) &&
+                              (!b.has_value() || b->numel() == w.size(0)),
+                          "few_rows_projection: weight [n, d], bias [n], result [rows, n]");
+    };
+    fits(out, weight, bias);
+    if (out2) fits(*out2, *weight2, bias2);
+    Launch launch(device);
+    check(rlm_few_rows_projection(f32(x), x.stride(0), f32(weight), f32(bias), f32(out), weight2 ? f32(*weight2) : nullptr, f32(bias2),
+                                  out2 ? f32(*out2) : nullptr, x.size(0), x.size(1), weight.size(0), weight2 ? weight2->size(0) : 0,
+                                  launch.stream));
+}
+
+void few_rows_projection(Tensor& out, const Tensor& x, const Tensor& weight, const OptTensor& bias) {
+    few_rows(out, nullptr, x, weight, nullptr, bias, std::nullopt);
+}
+
+void few_rows_projection_pair(Tensor& out, Tensor& out2, const Tensor& x, const Tensor& weight, const Tensor& weight2,
+                              const OptTensor& bias2) {
+    few_rows(out, &out2, x, weight, &weight2, std::nullopt, bias2);
+}
+
 Tensor skinny_projection(const Tensor& x, const Tensor& weight, const OptTensor& bias) {
     const c10::Device device = dense_rows({ARG(x)});
     check_projection(x, weight, bias, device);
@@ -1114,6 +1142,9 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
             "Tensor norm2_weight, Tensor norm2_bias, float norm_eps, Tensor weight, SymInt n_first, "                    \
             "Tensor(a14!) norm1_out, Tensor(a15!) norm2_out, Tensor(a16!) out_second) -> (Tensor, Tensor)")              \
     MUTATES(greedy_token, "(Tensor logits, SymInt vocab, Tensor(a2!)? position) -> Tensor")                              \
+    MUTATES(few_rows_projection, "(Tensor(a0!) out, Tensor x, Tensor weight, Tensor? bias=None) -> ()")                  \
+    MUTATES(few_rows_projection_pair, "(Tensor(a0!) out, Tensor(a1!) out2, Tensor x, Tensor weight, Tensor weight2, "     \
+            "Tensor? bias2=None) -> ()")                                                                                 \
     PURE(skinny_projection, "(Tensor x, Tensor weight, Tensor? bias=None) -> Tensor")                                    \
     MUTATES(skinny_projection_greedy, "(Tensor x, Tensor weight, Tensor? bias, SymInt vocab, Tensor(a4!) scratch, "      \
             "Tensor(a5!)? position) -> (Tensor, Tensor)")                                                                \
@@ -1300,7 +1331,8 @@ PyMethodDef kMethods[] = {METHOD(relation_select_packed), METHOD(relation_select
                           METHOD(sequence_state), METHOD(relation_hidden_cached), METHOD(relation_hidden_cached_out),
                           METHOD(relation_hidden_cache_update), METHOD(relation_hidden_cache_update_out),
                           METHOD(relation_norm_reduce), METHOD(relation_norm_reduce_residual_norm), METHOD(relation_mlp_rows),
-                          METHOD(packed_projection), METHOD(layer_norm_cast), METHOD(decode_embed_norm),
+                          METHOD(packed_projection), METHOD(layer_norm_cast), METHOD(decode_embed_norm), METHOD(few_rows_projection),
+                          METHOD(few_rows_projection_pair),
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "librelation_lm_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -26,6 +26,8 @@ from torch import Tensor
 from relation_lm.inference.routed_model import RoutedRelationLM
 from relation_lm.kernels import _abi
 from relation_lm.kernels.packed_projection import (decode_embed_norm, decode_front, decode_front_supported,
+                                                    few_rows_projection, few_rows_projection_pair,
+                                                    few_rows_projection_supported,
                                                     greedy_token, l2_prefetch, layer_norm_cast,
                                                     mapped_host_view, packed_projection, packed_projection_slices,
                                                     skinny_argmax_scratch_bytes, skinny_projection,
@@ -151,8 +153,16 @@ class StatefulDecoder:
         if not self.fused:
             # rows of whole 16-byte chunks up to 1024 wide: LayerNorms inside the kernels that make their input
             self.kernel_norms = cfg.d_model % 8 == 0 and cfg.d_model <= 1024
+            # The products of a position's rows by the library's own kernel, and with it the whole step under
+            # programmatic launch (libraries' kernels in between would wait for nothing that it lets run early).
+            # From nine sequences on libraries have the better products (16 rows of the 16 256 heads at d 768: 36 us, 28).
+            self.few_rows = (self.kernel_norms and B <= 8 and H % 4 == 0
+                             and few_rows_projection_supported(B * cfg.k_max, cfg.d_model, dtype))
+            if self.few_rows:
+                self.packed_rows = zeros(B, self.w["w_packed"].shape[0])
+                self.second_rows = zeros(B, cfg.k_max, cfg.d_model)
             # one product for both heads where its column slices are dense matrices, as two products' results are
-            if B == 1:
+            elif B == 1:
                 self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
                 self.head_bias = torch.cat((zeros(cfg.vocab_size), self.w["boundary_b"]))
         else:
@@ -211,7 +221,11 @@ class StatefulDecoder:
                 return self._step_fused(tokens, boundaries, keep_selection)
             finally:
                 _abi.set_programmatic_launch(previous)
-        return self._step_unfused(tokens, boundaries, keep_selection)
+        previous = _abi.set_programmatic_launch(self.programmatic_launch and self.few_rows)
+        try:
+            return self._step_unfused(tokens, boundaries, keep_selection)
+        finally:
+            _abi.set_programmatic_launch(previous)
 
     def step_greedy(self, tokens: Tensor, boundaries: Tensor, chosen_out: Tensor | None = None) -> Tensor:
         """One step followed by the greedy choice: returns the next token ids ``[B]`` (int64) and
@@ -249,7 +263,11 @@ class StatefulDecoder:
             hidden = x * self.input_scale + w["position_embedding"].index_select(0, pos.view(1))
             self._normalize(hidden, w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized)
             self._normalize(hidden, w["input_norm_w"][0], w["input_norm_b"][0], self.normalized)
-        packed = F.linear(self.memory_normalized, w["w_packed"])      # [B, layers * 512]
+        if self.few_rows:
+            packed = self.packed_rows                                 # [B, layers * 512]
+            few_rows_projection(packed, self.memory_normalized, w["w_packed"], None)
+        else:
+            packed = F.linear(self.memory_normalized, w["w_packed"])
         sparse_cache_append(packed, self.anchor_keys, self.partner_keys, self.operand_cache,
                             self.partner_anchor_cache, *self.router_caches, *self.router_stats,
                             w["anchor_conv_weight"], w["partner_conv_weight"], pos, cfg.block_size)
@@ -258,11 +276,18 @@ class StatefulDecoder:
         for layer in self._layers:
             # the last layer's goes to a tensor of this step's own: it stays behind as `last_final`
             normalized = torch.empty_like(self.normalized) if layer is self._layers[-1] else self.normalized
-            torch.mm(self.normalized, layer.w_query_t, out=layer.query)                 # [B, 256]
+            if self.few_rows:
+                few_rows_projection(layer.query, self.normalized, layer.w_query, None)        # [B, 256]
+            else:
+                torch.mm(self.normalized, layer.w_query_t, out=layer.query)
             anchor, _, partner, partner_score = relation_select_packed(
                 *layer.selection, pos, cfg.local_window, cfg.top_blocks, K, cfg.strict_valid)
             relation_hidden_cache_update_out(self.relation_hidden, *layer.caches, anchor, partner, *layer.first_layer, pos)
-            raw = F.linear(self.relation_hidden, *layer.second_layer)                   # [B, K, d]
+            if self.few_rows:
+                raw = self.second_rows                                                  # [B, K, d]
+                few_rows_projection(raw.view(-1, cfg.d_model), self.relation_hidden.view(-1, cfg.hidden_dim), *layer.second_layer)
+            else:
+                raw = F.linear(self.relation_hidden, *layer.second_layer)
             if self.kernel_norms:
                 relation_norm_reduce_residual_norm(raw, partner_score, *layer.relation_norm, pos, cfg.norm_eps, hidden,
                                                    layer.mix, *layer.next_norm, cfg.norm_eps, normalized)
@@ -273,7 +298,10 @@ class StatefulDecoder:
             if keep_selection:
                 self.last_selection.append((anchor, partner))
         self.last_final = normalized
-        if self.batch == 1:
+        if self.few_rows:
+            heads = normalized.new_empty(self.batch, cfg.vocab_size), normalized.new_empty(self.batch, cfg.boundary_vocab_size)
+            few_rows_projection_pair(*heads, normalized, w["token_embedding"], w["boundary_w"], w["boundary_b"])
+        elif self.batch == 1:
             logits = F.linear(normalized, self.head_weight, self.head_bias)
             heads = logits[:, :cfg.vocab_size], logits[:, cfg.vocab_size:]
         else:

@@ -19,6 +19,8 @@ _layer_norm_cast = _abi.operator("layer_norm_cast")
 _decode_embed_norm = _abi.operator("decode_embed_norm")
 _decode_front = _abi.operator("decode_front")
 _greedy_token = _abi.operator("greedy_token")
+_few_rows_projection = _abi.operator("few_rows_projection")
+_few_rows_projection_pair = _abi.operator("few_rows_projection_pair")
 _skinny_projection = _abi.operator("skinny_projection")
 _skinny_projection_greedy = _abi.operator("skinny_projection_greedy")
 _skinny_projection_greedy_into = _abi.operator("skinny_projection_greedy_into")
@@ -208,6 +210,34 @@ def greedy_token(logits: Tensor, vocab: int, position: Tensor | None = None) -> 
 @torch.library.register_fake("relation_lm::greedy_token")
 def _(logits, vocab, position):
     return logits.new_empty((logits.size(0),), dtype=torch.int64)
+
+
+def few_rows_projection_supported(rows: int, d_in: int, dtype: torch.dtype) -> bool:
+    """Whether ``few_rows_projection`` takes these sizes."""
+    return 1 <= rows <= 64 and d_in % 4 == 0 and dtype == torch.float32
+
+
+def few_rows_projection(out: Tensor, x: Tensor, weight: Tensor, bias: Tensor | None = None) -> None:
+    """``out = x [rows <= 64, d] @ weight [n, d].T (+ bias)`` in single precision (extension): the products of one
+    decode position, streams of their weight matrices."""
+    _few_rows_projection(out, x, weight, bias)
+
+
+@torch.library.register_fake("relation_lm::few_rows_projection")
+def _(out, x, weight, bias=None):
+    return None
+
+
+def few_rows_projection_pair(out: Tensor, out2: Tensor, x: Tensor, weight: Tensor, weight2: Tensor,
+                             bias2: Tensor | None = None) -> None:
+    """``few_rows_projection`` with two weights for the same rows in one launch: ``out = x @ weight.T``,
+    ``out2 = x @ weight2.T (+ bias2)``."""
+    _few_rows_projection_pair(out, out2, x, weight, weight2, bias2)
+
+
+@torch.library.register_fake("relation_lm::few_rows_projection_pair")
+def _(out, out2, x, weight, weight2, bias2=None):
+    return None
 
 
 def skinny_projection_supported(rows: int, d_in: int, dtype: torch.dtype) -> bool:
