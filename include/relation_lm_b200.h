@@ -415,6 +415,21 @@ int rlm_relation_layer_tail(
     int hidden_dim, int d_model, int n_query, int dtype, int32_t* status, void* stream);
 
 /*
+ * The same for d = 768, H = 3072 (extension): clusters of 16 CTAs of 192 hidden and 48 output columns each, whose slices
+ * of second_weight are streamed.  R 64 or 128, NQ a multiple of 256; arguments and results as above.
+ */
+int rlm_relation_layer_tail_wide_supported(int n_seq, int k_out, int relation_dim, int hidden_dim,
+                                           int d_model, int n_query, int dtype);
+int rlm_relation_layer_tail_wide(
+    const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
+    const int32_t* partner_index, const float* partner_scores, const void* product_weight,
+    const void* second_weight, const void* second_bias, const float* norm_weight, const float* norm_bias,
+    const int64_t* position, float norm_eps, float* residual, const float* mix,
+    const float* next_norm_weight, const float* next_norm_bias, float next_norm_eps, void* normalized,
+    const void* query_weight, void* query, int n_seq, int k_out, int max_t, int relation_dim,
+    int hidden_dim, int d_model, int n_query, int dtype, int32_t* status, void* stream);
+
+/*
  * A whole relation layer of a decode step in one launch (extension): rlm_relation_select_packed in
  * its decode form (one query row per sequence, all at *position) followed by
  * rlm_relation_layer_tail, in the tail's cluster.  The first CTAs of a cluster each select for one

@@ -28,14 +28,23 @@ struct SelectInFront {
     }
 };
 
-template <bool kBf16, bool kAligned>
+template <bool kBf16, bool kAligned, bool kMany>
 __global__ void __launch_bounds__(kLtThreads, 1) relation_layer_kernel(
     const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2,
     const LayerTailArgs tail, const SelectArgs sel) {
     extern __shared__ __align__(1024) unsigned char layer_smem_raw[];
     __shared__ __align__(8) unsigned long long select_bars[4];
-    layer_tail_body<kBf16, kAligned>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16 ? RLM_BF16 : RLM_F16>{&sel, smem_u32(select_bars)});
+    layer_tail_body<kBf16, kAligned, false, kMany>(map_wm, map_w2, tail, layer_smem_raw, SelectInFront<kBf16 ? RLM_BF16 : RLM_F16>{&sel, smem_u32(select_bars)});
 }
+
+using LayerKernel = void (*)(const CUtensorMap, const CUtensorMap, const LayerTailArgs, const SelectArgs);
+
+template <bool kMany>
+LayerKernel layer_kernel(bool bf16, bool aligned) {
+    return aligned ? (bf16 ? relation_layer_kernel<true, true, kMany> : relation_layer_kernel<false, true, kMany>)
+                   : (bf16 ? relation_layer_kernel<true, false, kMany> : relation_layer_kernel<false, false, kMany>);
+}
+LayerKernel layer_kernel(bool bf16, bool aligned, bool many) { return many ? layer_kernel<true>(bf16, aligned) : layer_kernel<false>(bf16, aligned); }
 
 int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weight, const void* second_weight,
                  void* stream) {
@@ -60,7 +69,7 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
     if (tail.seqs_per_cluster > tail.cluster) tail.seqs_per_cluster = tail.cluster;   // a selecting CTA per sequence
     const uint32_t smem_bytes = lt_smem_bytes_with_stage(tail.rdim, tail.d, tail.query_weight ? tail.n_query / tail.cluster : 0,
                                                          sel.plan.total);
-    const LtPlan whole = lt_plan(tail.rdim, tail.d, kLtMaxPairs, 0);
+    const LtPlan whole = lt_plan(tail.rdim, tail.d, true, kLtMaxPairs, 0);
     if (sel.plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) {
         set_error("relation_layer: the selector's working set does not fit the tail's tile memory (use the two launches)");
         return RLM_ERR_UNSUPPORTED;
@@ -76,8 +85,7 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
         set_error("relation_layer: cuTensorMapEncodeTiled failed");
         return RLM_ERR_LAUNCH;
     }
-    auto kernel = lt_aligned(tail) ? (tail.dtype == RLM_BF16 ? relation_layer_kernel<true, true> : relation_layer_kernel<false, true>)
-                                   : (tail.dtype == RLM_BF16 ? relation_layer_kernel<true, false> : relation_layer_kernel<false, false>);
+    auto kernel = layer_kernel(tail.dtype == RLM_BF16, lt_aligned(tail), lt_many(tail.seqs_per_cluster, tail.k_out));
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), tail.cluster);
     if (rc != RLM_OK) return rc;
     const int clusters = (tail.n_seq + tail.seqs_per_cluster - 1) / tail.seqs_per_cluster;
@@ -107,9 +115,9 @@ extern "C" int rlm_relation_layer_supported(int n_seq, int k_out, int relation_d
     const Plan plan = make_plan(n_blocks, max_t / n_blocks, local_window, top_blocks, buckets, dtype_size(dtype),
                                 dtype_size(dtype), kPacked, false);
     const uint32_t smem_bytes = lt_smem_bytes_with_stage(relation_dim, d_model, n_query / cluster, plan.total);
-    const LtPlan whole = lt_plan(relation_dim, d_model, kLtMaxPairs, 0);
+    const LtPlan whole = lt_plan(relation_dim, d_model, true, kLtMaxPairs, 0);
     if (plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) return 0;
-    auto kernel = dtype == RLM_BF16 ? relation_layer_kernel<true, true> : relation_layer_kernel<false, true>;
+    auto kernel = layer_kernel(dtype == RLM_BF16, true, true);
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(cluster, 1, 1);

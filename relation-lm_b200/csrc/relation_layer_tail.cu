@@ -10,7 +10,7 @@
 //   residual[b]  += mix * context[b];  normalized[b] = LayerNorm'(residual[b])
 //   query[b]      = W_q normalized[b]                                              (optional)
 //
-// Geometry.  A thread-block cluster of C = H / 128 CTAs serves up to 64 (sequence, partner)
+// Geometry (d <= 512, few pairs).  A thread-block cluster of C = H / 128 CTAs serves up to 64 (sequence, partner)
 // pairs; CTA c owns hidden columns [128 c, 128 c + 128).  Its weight slices — W_m[128 c .., :]
 // (128 x R) and W_2[:, 128 c ..] (d x 128) — are requested by TMA before the dependency wait and
 // stay resident in shared memory.  After the selector's indices arrive every CTA gathers the
@@ -19,6 +19,20 @@
 // (tcgen05.mma, pairs on the TMEM columns), applies GELU and writes its hidden slice as the
 // K-major B tile of the second GEMM, whose A operand is the resident W_2 slice: a split-K GEMM
 // over the cluster, each CTA holding a partial raw^T [d, pairs] in TMEM.
+//
+// Launches of more than 16 pairs a cluster (d >= 256): the partial sums, C x d x pairs floats through distributed shared
+// memory at some 15 bytes a cycle and CTA, become what takes the time (64 pairs: 8 300 of 28 000 cycles).  There
+// neighbouring CTAs exchange their 16-bit hidden slices and divide the output rows: each has half of the rows over both
+// slices, the partial sums are half as many, and the other's slice travels while the own one is multiplied.
+//
+// d = 768 (kWide): 16 CTAs of 192 hidden columns (two overlapping tiles of the product GEMM) and 48 output columns, always
+// sharing; a CTA's part of W_2, 288 KB, does not fit beside the rest and goes through a ring of six to nine tiles of
+// 16 KB, three warps issuing a tile of output rows each and a fourth refilling.  us a step of 12 layers in a graph, five
+// launches a layer -> here: batch 1 319 -> 239, batch 8 338 -> 255, batch 16 405 -> 318, batch 28 481 -> 387.
+//
+// us a step of 6 layers of d 512 before sharing, the gathers through registers, two issuing warps and the statistics in
+// messages of two pairs -> with them: batch 1 84.0 -> 81.9, 5 98.4 -> 94.3, 8 97.5 -> 94.3, 16 128.5 -> 122.5,
+// 32 167.6 -> 157.3, 48 174.1 -> 164.0.
 //
 // What bounds the launch is a chain of some twenty dependent phases, so the CTAs hand their results on by pushing
 // them into the receiver's shared memory with stores that count towards a barrier of the receiver (st.async), and a
@@ -42,28 +56,42 @@
 namespace rlm {
 namespace {
 
-template <bool kBf16, bool kAligned>
+template <bool kBf16, bool kAligned, bool kWide, bool kMany>
 __global__ void __launch_bounds__(kLtThreads, 1) relation_layer_tail_kernel(
     const __grid_constant__ CUtensorMap map_wm, const __grid_constant__ CUtensorMap map_w2,
     const LayerTailArgs a) {
     extern __shared__ __align__(1024) unsigned char lt_smem_raw[];
-    layer_tail_body<kBf16, kAligned>(map_wm, map_w2, a, lt_smem_raw, NoStage{});
+    layer_tail_body<kBf16, kAligned, kWide, kMany>(map_wm, map_w2, a, lt_smem_raw, NoStage{});
 }
 
-}  // namespace
-}  // namespace rlm
+using TailKernel = void (*)(const CUtensorMap, const CUtensorMap, const LayerTailArgs);
 
-extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relation_dim, int hidden_dim,
-                                                 int d_model, int n_query, int dtype) {
-    using namespace rlm;
+template <bool kWide, bool kMany>
+TailKernel tail_kernel(bool bf16, bool aligned) {
+    return aligned ? (bf16 ? relation_layer_tail_kernel<true, true, kWide, kMany> : relation_layer_tail_kernel<false, true, kWide, kMany>)
+                   : (bf16 ? relation_layer_tail_kernel<true, false, kWide, kMany> : relation_layer_tail_kernel<false, false, kWide, kMany>);
+}
+TailKernel tail_kernel(bool bf16, bool aligned, bool wide, bool many) {
+    return wide ? (many ? tail_kernel<true, true>(bf16, aligned) : tail_kernel<true, false>(bf16, aligned))
+                : (many ? tail_kernel<false, true>(bf16, aligned) : tail_kernel<false, false>(bf16, aligned));
+}
+
+// A few sequences per cluster: up to four clusters share the work of a small batch (each
+// streams the layer's weights from L2 once), more clusters only for batches beyond 32.
+int tail_seqs_per_cluster(int n_seq, int k_out) {
+    const int most = kLtMaxPairs / k_out < kLtMaxSeq ? kLtMaxPairs / k_out : kLtMaxSeq;
+    return (n_seq + 3) / 4 < most ? (n_seq + 3) / 4 : most;
+}
+
+int tail_supported(bool wide, int n_seq, int k_out, int relation_dim, int hidden_dim, int d_model, int n_query, int dtype) {
     LayerTailArgs a{};
     a.n_seq = n_seq; a.k_out = k_out; a.max_t = 1; a.rdim = relation_dim; a.hdim = hidden_dim; a.d = d_model;
     a.n_query = n_query; a.dtype = dtype;
     a.query_weight = n_query > 0 ? &a : nullptr;      // only tested for NULL
     a.query = n_query > 0 ? &a : nullptr;
-    if (lt_validate(a) != RLM_OK) return 0;
-    const int cluster = hidden_dim / kLtHC;
-    auto kernel = dtype == RLM_BF16 ? relation_layer_tail_kernel<true, true> : relation_layer_tail_kernel<false, true>;
+    if (lt_validate(a, wide) != RLM_OK) return 0;
+    const int cluster = lt_cluster(d_model);
+    auto kernel = tail_kernel(dtype == RLM_BF16, true, wide, lt_many(tail_seqs_per_cluster(n_seq, k_out), k_out));
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     // one cluster of this size, with this much shared memory per CTA, must fit the device
     cudaLaunchConfig_t config = {};
@@ -85,33 +113,13 @@ extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relat
     return clusters > 0 ? 1 : 0;
 }
 
-extern "C" int rlm_selftest_layer_tail_plan(int pairs, int n_seq, int relation_dim, int d_model, int n_query, int64_t* ranges) {
-    using namespace rlm;
-    if (!ranges) { set_error("selftest_layer_tail_plan: result required"); return RLM_ERR_NULL; }
-    const int cluster = 4 * d_model / kLtHC, pairs_pad = pairs <= 16 ? 16 : (pairs <= 32 ? 32 : 64);
-    if (pairs < 1 || pairs > kLtMaxPairs || n_seq < 1 || n_seq > kLtMaxSeq || d_model % kBM != 0 || d_model < kBM || cluster > 16 ||
-        relation_dim % kBK != 0 || n_query % cluster != 0) {
-        set_error("selftest_layer_tail_plan: sizes outside the kernel's range");
-        return RLM_ERR_SHAPE;
-    }
-    const int nq_own = n_query / cluster;
-    const LtPlan p = lt_plan(relation_dim, d_model, pairs_pad, nq_own);
-    const int64_t begin[] = {p.own_y, p.rows, p.hid, p.term_p, p.wq, 0};
-    const int64_t bytes[] = {pairs * kLtOwnStride * 4, n_seq * d_model * 2, n_seq * d_model * 4, cluster * pairs_pad * 8,
-                             nq_own * (2 * d_model + 256), p.total};
-    for (int i = 0; i < 6; ++i) { ranges[2 * i] = begin[i]; ranges[2 * i + 1] = begin[i] + bytes[i]; }
-    return RLM_OK;
-}
-
-extern "C" int rlm_relation_layer_tail(
-    const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
+int launch_tail(bool wide, const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
     const int32_t* partner_index, const float* partner_scores, const void* product_weight,
     const void* second_weight, const void* second_bias, const float* norm_weight, const float* norm_bias,
     const int64_t* position, float norm_eps, float* residual, const float* mix,
     const float* next_norm_weight, const float* next_norm_bias, float next_norm_eps, void* normalized,
     const void* query_weight, void* query, int n_seq, int k_out, int max_t, int relation_dim,
     int hidden_dim, int d_model, int n_query, int dtype, int32_t* status, void* stream) {
-    using namespace rlm;
     if (n_seq == 0) return RLM_OK;
     if (!expanded_cache || !operand_cache || !anchor_index || !partner_index || !partner_scores ||
         !product_weight || !second_weight || !second_bias || !norm_weight || !norm_bias || !position ||
@@ -127,27 +135,23 @@ extern "C" int rlm_relation_layer_tail(
     a.query_weight = query_weight; a.query = query; a.status = status; a.eps = norm_eps; a.next_eps = next_norm_eps;
     a.n_seq = n_seq; a.k_out = k_out; a.max_t = max_t; a.rdim = relation_dim; a.hdim = hidden_dim; a.d = d_model;
     a.n_query = query_weight ? n_query : 0; a.dtype = dtype;
-    int rc = lt_validate(a);
+    int rc = lt_validate(a, wide);
     if (rc != RLM_OK) return rc;
     if (!aligned16(expanded_cache) || !aligned16(operand_cache) || !aligned16(product_weight) ||
         !aligned16(second_weight) || (query_weight && !aligned16(query_weight))) {
         set_error("relation_layer_tail: caches and weights must be 16-byte aligned");
         return RLM_ERR_ALIGN;
     }
-    a.cluster = hidden_dim / kLtHC;
-    // a few sequences per cluster: up to four clusters share the work of a small batch (each
-    // streams the layer's weights from L2 once), more clusters only for batches beyond 32
-    const int most = kLtMaxPairs / k_out < kLtMaxSeq ? kLtMaxPairs / k_out : kLtMaxSeq;
-    a.seqs_per_cluster = (n_seq + 3) / 4 < most ? (n_seq + 3) / 4 : most;
+    a.cluster = lt_cluster(d_model);
+    a.seqs_per_cluster = tail_seqs_per_cluster(n_seq, k_out);
     const int clusters = (n_seq + a.seqs_per_cluster - 1) / a.seqs_per_cluster;
     CUtensorMap mwm, mw2;
-    if (!make_map(&mwm, product_weight, hidden_dim, relation_dim, relation_dim, kBM, dtype) ||
+    if (!make_map(&mwm, product_weight, hidden_dim, relation_dim, relation_dim, lt_hidden(d_model), dtype) ||
         !make_map(&mw2, second_weight, d_model, hidden_dim, hidden_dim, kBM, dtype)) {
         set_error("relation_layer_tail: cuTensorMapEncodeTiled failed");
         return RLM_ERR_LAUNCH;
     }
-    auto kernel = lt_aligned(a) ? (dtype == RLM_BF16 ? relation_layer_tail_kernel<true, true> : relation_layer_tail_kernel<false, true>)
-                                : (dtype == RLM_BF16 ? relation_layer_tail_kernel<true, false> : relation_layer_tail_kernel<false, false>);
+    auto kernel = tail_kernel(dtype == RLM_BF16, lt_aligned(a), wide, lt_many(a.seqs_per_cluster, k_out));
     rc = lt_prepare(reinterpret_cast<const void*>(kernel), a.cluster);
     if (rc != RLM_OK) return rc;
     const size_t smem_bytes = lt_smem_bytes(relation_dim, d_model, a.n_query / a.cluster);
@@ -155,4 +159,59 @@ extern "C" int rlm_relation_layer_tail(
                           static_cast<unsigned>(a.cluster), smem_bytes, stream, mwm, mw2, a);
     count_launch();
     return check_launch("relation_layer_tail_kernel");
+}
+
+}  // namespace
+}  // namespace rlm
+
+extern "C" int rlm_relation_layer_tail_supported(int n_seq, int k_out, int relation_dim, int hidden_dim, int d_model, int n_query,
+                                                 int dtype) {
+    return rlm::tail_supported(false, n_seq, k_out, relation_dim, hidden_dim, d_model, n_query, dtype);
+}
+
+extern "C" int rlm_relation_layer_tail_wide_supported(int n_seq, int k_out, int relation_dim, int hidden_dim, int d_model,
+                                                      int n_query, int dtype) {
+    return rlm::tail_supported(true, n_seq, k_out, relation_dim, hidden_dim, d_model, n_query, dtype);
+}
+
+extern "C" int rlm_relation_layer_tail(
+
+    const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
+    const int32_t* partner_index, const float* partner_scores, const void* product_weight,
+    const void* second_weight, const void* second_bias, const float* norm_weight, const float* norm_bias,
+    const int64_t* position, float norm_eps, float* residual, const float* mix,
+    const float* next_norm_weight, const float* next_norm_bias, float next_norm_eps, void* normalized,
+    const void* query_weight, void* query, int n_seq, int k_out, int max_t, int relation_dim,
+    int hidden_dim, int d_model, int n_query, int dtype, int32_t* status, void* stream) {
+    return rlm::launch_tail(false, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight, second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, residual, mix, next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query, n_seq, k_out, max_t, relation_dim, hidden_dim, d_model, n_query, dtype, status, stream);
+}
+
+extern "C" int rlm_relation_layer_tail_wide(
+
+    const void* expanded_cache, const void* operand_cache, const int32_t* anchor_index,
+    const int32_t* partner_index, const float* partner_scores, const void* product_weight,
+    const void* second_weight, const void* second_bias, const float* norm_weight, const float* norm_bias,
+    const int64_t* position, float norm_eps, float* residual, const float* mix,
+    const float* next_norm_weight, const float* next_norm_bias, float next_norm_eps, void* normalized,
+    const void* query_weight, void* query, int n_seq, int k_out, int max_t, int relation_dim,
+    int hidden_dim, int d_model, int n_query, int dtype, int32_t* status, void* stream) {
+    return rlm::launch_tail(true, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight, second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, residual, mix, next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query, n_seq, k_out, max_t, relation_dim, hidden_dim, d_model, n_query, dtype, status, stream);
+}
+
+extern "C" int rlm_selftest_layer_tail_plan(int pairs, int n_seq, int relation_dim, int d_model, int n_query, int64_t* ranges) {
+    using namespace rlm;
+    if (!ranges) { set_error("selftest_layer_tail_plan: result required"); return RLM_ERR_NULL; }
+    const int cluster = d_model < kBM ? 1 : lt_cluster(d_model), pairs_pad = pairs <= 16 ? 16 : (pairs <= 32 ? 32 : 64);
+    if (pairs < 1 || pairs > kLtMaxPairs || n_seq < 1 || n_seq > kLtMaxSeq || d_model % kBM != 0 || d_model < kBM || cluster > 16 ||
+        (lt_wide(d_model) && d_model != 768) || relation_dim % kBK != 0 || n_query % cluster != 0) {
+        set_error("selftest_layer_tail_plan: sizes outside the kernel's range");
+        return RLM_ERR_SHAPE;
+    }
+    const int nq_own = n_query / cluster;
+    const LtPlan p = lt_plan(relation_dim, d_model, pairs > 16, pairs_pad, nq_own);
+    const int64_t begin[] = {p.own_y, p.rows, p.rows_in, p.term_p, p.wq, 0};
+    const int64_t bytes[] = {pairs * (lt_owned(d_model) + 1) * 4, n_seq * d_model * 2, n_seq * d_model * 4, cluster * pairs_pad * 8,
+                             nq_own * (2 * d_model + 256), p.total};
+    for (int i = 0; i < 6; ++i) { ranges[2 * i] = begin[i]; ranges[2 * i + 1] = begin[i] + bytes[i]; }
+    return RLM_OK;
 }

@@ -11,12 +11,18 @@ namespace rlm {
 namespace {
 
 constexpr int kLtThreads = 256;
-constexpr int kLtHC = 128;            // hidden columns per CTA
+constexpr int kLtHC = 128;            // hidden columns per CTA (192 at d = 768)
 constexpr int kLtMaxPairs = 64;       // (sequence, partner) pairs per cluster
 constexpr int kLtMaxSeq = 8;          // sequences per cluster
-constexpr int kLtOwn = 32;            // output columns a CTA owns after the reduce-scatter (d / C)
-constexpr int kLtOwnStride = 33;      // padded row of the owned raw values (floats)
-constexpr uint32_t kLtTermStride = kLtHC * 2 + 16;   // padded row of the staged expanded-cache terms
+constexpr int kLtOwn = 32;            // output columns a CTA owns after the reduce-scatter (d / C; 48 at d = 768)
+constexpr uint32_t kLtW2Tile = kBM * 128u;           // 128 output rows x 64 hidden columns
+constexpr int kLtMaxRing = 10;        // W_2 tiles in flight where the slice is streamed
+
+// d = 768: 16 CTAs of 192 hidden and 48 output columns, whose W_2 slice is streamed; otherwise H / 128 CTAs.
+__host__ __device__ inline bool lt_wide(int d) { return d > 512; }
+__host__ __device__ inline int lt_hidden(int d) { return lt_wide(d) ? 192 : kLtHC; }
+__host__ __device__ inline int lt_cluster(int d) { return 4 * d / lt_hidden(d); }
+__host__ __device__ inline int lt_owned(int d) { return lt_wide(d) ? 48 : kLtOwn; }
 
 struct LayerTailArgs {
     const void* expanded_cache;      // [B, T, 2H]
@@ -43,47 +49,75 @@ struct LayerTailArgs {
 
 // Shared-memory plan (byte offsets from the 1024-aligned dynamic base).
 struct LtPlan {
-    uint32_t wm, w2, p, hid, term_p, term_a, op_a, wq, total;
-    uint32_t own_y, rows;                // later uses of p and w2: see lt_plan
+    uint32_t wm, w2, p, hid, term_p, term_a, stats_out, wq, total;
+    uint32_t own_y, rows, rows_in;       // later uses of p, w2 and hid: see lt_plan
+    int ring;                            // W_2 tiles in flight (wide: the slice has 18)
 };
 
-// The partial sums that a CTA receives, [sender][four pairs][owned column][pair] of 512 d pairs / 128 bytes in all,
-// take the place of a consumed weight slice: W_m's for 16 pairs, W_2's for more (the W_q slice then waits for W_m's).
-// nq_own: rows of the query-projection weight per CTA.
-__host__ __device__ inline LtPlan lt_plan(int rdim, int d, int pairs_pad, int nq_own) {
+// Launches of more than 16 pairs a cluster.
+__host__ __device__ inline bool lt_many(int seqs_per_cluster, int k_out) { return seqs_per_cluster * k_out > 16; }
+// CTAs that share their hidden slices and divide the output rows (neighbours in the cluster): see relation_layer_tail.cu.
+// The partial sums of few pairs are too short for that (us a step of 6 layers of d 512, batch 1 and 8: 84.0 and 94.6
+// without, 84.0 and 94.5 with it; of 4 layers of d 256, batch 1: 57.5, 59.4).
+__host__ __device__ inline int lt_sharing(int d, bool many) { return lt_wide(d) || (d >= 2 * kBM && many) ? 2 : 1; }
+
+// The partial sums that a CTA receives, [sender][four pairs][owned column][pair] of 512 d pairs / 128 bytes (half of it from
+// sharing CTAs) in all, take the place of a consumed weight slice: W_m's for 16 pairs, W_2's for more (the W_q slice then
+// waits for W_m's).  nq_own: rows of the query-projection weight per CTA.
+__host__ __device__ inline LtPlan lt_plan(int rdim, int d, bool many, int pairs_pad, int nq_own) {
     LtPlan p;
+    const bool wide = lt_wide(d);
+    const uint32_t hc = lt_hidden(d), own = lt_owned(d), term_stride = 2u * hc + 16u;
     uint32_t off = 0;
-    const uint32_t received = 4u * static_cast<uint32_t>(d) * pairs_pad;
-    p.wm = off;     off += static_cast<uint32_t>(rdim / kBK) * kBM * 128u;           // W_m slice
+    const uint32_t received = 4u * static_cast<uint32_t>(d) * pairs_pad / lt_sharing(d, many);
+    p.wm = off;     off += static_cast<uint32_t>(rdim / kBK) * hc * 128u;            // W_m slice
     if (pairs_pad == 16 && off < received) off = received;
-    p.w2 = off;     off += static_cast<uint32_t>(d / kBM) * 2u * kBM * 128u;         // W_2 slice
-    p.p = off;      off += static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u;     // product tile; later the normalised pairs
-    if (off - p.p < pairs_pad * kLtOwnStride * 4u) off = p.p + pairs_pad * kLtOwnStride * 4u;
+    p.w2 = off;     if (!wide) off += static_cast<uint32_t>(d / kBM) * 2u * kLtW2Tile;      // W_2 slice (wide: at the end)
+    // product tile; later this CTA's hidden slice, which is written when the product GEMM is done; later the normalised pairs
+    const uint32_t product = static_cast<uint32_t>(rdim / kBK) * pairs_pad * 128u, slice = hc / kBK * pairs_pad * 128u;
+    const uint32_t normalised = pairs_pad * (own + 1u) * 4u, rows_in = static_cast<uint32_t>(kLtMaxSeq) * d * 4u;
+    p.p = off;      off += product > slice ? product : slice;
+    if (off - p.p < normalised) off = p.p + normalised;
     off = (off + 1023u) & ~1023u;
-    p.hid = off;    off += 2u * pairs_pad * 128u;                                    // hidden tile; later the residual rows
-    if (off - p.hid < static_cast<uint32_t>(kLtMaxSeq) * d * 4u) off = p.hid + kLtMaxSeq * d * 4u;
-    p.term_p = off; off += pairs_pad * kLtTermStride;
-    p.term_a = off; off += kLtMaxSeq * kLtTermStride;
-    p.op_a = off;   off += kLtMaxSeq * static_cast<uint32_t>(rdim) * 2u;
+    p.hid = p.rows_in = off; off += slice;                                           // the sharing CTA's slice; later the residual rows
+    if (!wide && off - p.hid < rows_in) off = p.hid + rows_in;
+    p.term_p = off; off += pairs_pad * term_stride;
+    p.term_a = off; off += kLtMaxSeq * term_stride;
+    p.stats_out = off; off += kLtMaxPairs * 8u;
     p.wq = p.wm;
-    if (pairs_pad == 16) { p.wq = off; off += static_cast<uint32_t>(nq_own) * (2u * d + 256u); }
-    p.total = off;
     // The last LayerNorm's rows take W_2's place, not the normalised pairs': a warp may write its rows while another
     // of its CTA still sums its pairs (the barrier between them counts what this CTA is sent, and only one warp a
     // sequence sends to it).  W_2's place is free in every warp by then: the statistics that a CTA waits for include
     // its own, and those follow its second GEMM and its reads of the partial sums.
     p.own_y = p.p;
-    p.rows = p.w2;
+    p.ring = 0;
+    if (wide) {
+        // the ring takes what is left; in its place, later: the residual rows that come in, the last LayerNorm's rows and,
+        // where W_m's place receives the partial sums, the W_q slice
+        p.w2 = (off + 1023u) & ~1023u;
+        const int left = kSmemDynamicLimit - 1024 - static_cast<int>(p.w2);
+        p.ring = left < 0 ? 0 : left / static_cast<int>(kLtW2Tile);
+        if (p.ring > kLtMaxRing) p.ring = kLtMaxRing;
+        off = p.w2 + p.ring * kLtW2Tile;
+        p.rows_in = p.w2;
+        p.rows = p.w2 + rows_in;
+        if (pairs_pad == 16) p.wq = p.rows + rows_in / 2;
+    } else {
+        if (pairs_pad == 16) { p.wq = off; off += static_cast<uint32_t>(nq_own) * (2u * d + 256u); }
+        p.rows = p.w2;
+    }
+    p.total = off;
     return p;
 }
 
 // Dynamic shared memory of a launch, whatever its pairs per cluster.
 inline uint32_t lt_smem_bytes(int rdim, int d, int nq_own) {
     uint32_t most = 0;
-    for (int pairs = 16; pairs <= kLtMaxPairs; pairs *= 2) {
-        const uint32_t total = lt_plan(rdim, d, pairs, nq_own).total;
-        if (total > most) most = total;
-    }
+    for (int pairs = 16; pairs <= kLtMaxPairs; pairs *= 2)
+        for (int many = pairs > 16; many < 2; ++many) {
+            const uint32_t total = lt_plan(rdim, d, many, pairs, nq_own).total;
+            if (total > most) most = total;
+        }
     return most + 1024;
 }
 
@@ -91,7 +125,7 @@ inline uint32_t lt_smem_bytes(int rdim, int d, int nq_own) {
 inline uint32_t lt_smem_bytes_with_stage(int rdim, int d, int nq_own, int stage) {
     uint32_t most = lt_smem_bytes(rdim, d, nq_own);
     for (int pairs = 16; pairs <= kLtMaxPairs; pairs *= 2) {
-        const uint32_t total = lt_plan(rdim, d, pairs, nq_own).p + static_cast<uint32_t>(stage) + 1024u;
+        const uint32_t total = lt_plan(rdim, d, pairs > 16, pairs, nq_own).p + static_cast<uint32_t>(stage) + 1024u;
         if (total > most) most = total;
     }
     return most;
@@ -111,6 +145,10 @@ __device__ __forceinline__ uint32_t lt_peer(uint32_t local_addr, uint32_t rank) 
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
     return remote;
 }
+__device__ __forceinline__ void lt_copy_cluster(uint32_t remote_dst, uint32_t src, uint32_t bytes, uint32_t remote_bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(remote_dst), "r"(src), "r"(bytes), "r"(remote_bar) : "memory");
+}
 // Relaxed: no data travels with these barriers (a consumed tile's place is free; nothing more will be pushed), and a
 // release would wait a thousand cycles for the warp's earlier stores and copies.
 __device__ __forceinline__ void lt_cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
@@ -120,10 +158,6 @@ __device__ __forceinline__ void lt_cluster_wait() { asm volatile("barrier.cluste
 __device__ __forceinline__ void lt_push16(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
                  ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void lt_push8(uint32_t addr, uint32_t bar, float x, float y) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
-                 ::"r"(addr), "r"(__float_as_uint(x)), "r"(__float_as_uint(y)), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void lt_push4(uint32_t addr, uint32_t bar, float x) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
@@ -145,6 +179,40 @@ __device__ __forceinline__ float2 lt_moments4(const float (&x)[4]) {
     float give_mean = mid ? m[0] : m[1], give_m2 = mid ? v[0] : v[1];
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, give_mean, o), other2 = __shfl_xor_sync(0xffffffffu, give_m2, o);
+        const float d = mean - other;
+        m2 = fmaf(d * d, 0.5f * count, m2 + other2);
+        mean = 0.5f * (mean + other);
+        count += count;
+        give_mean = mean;
+        give_m2 = m2;
+    }
+    return make_float2(mean, m2);
+}
+
+// The same over a half-warp's 16 lanes of three columns each, x[column][j], for j = (lane % 16) / 4.
+__device__ __forceinline__ float2 lt_moments4(const float (&x)[3][4]) {
+    const bool hi = threadIdx.x & 8, mid = threadIdx.x & 4;
+    float m4[4], v4[4], m[2], v[2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        m4[j] = (x[0][j] + x[1][j] + x[2][j]) * (1.0f / 3.0f);
+        const float d0 = x[0][j] - m4[j], d1 = x[1][j] - m4[j], d2 = x[2][j] - m4[j];
+        v4[j] = fmaf(d0, d0, fmaf(d1, d1, d2 * d2));
+    }
+    float count = 3.0f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float other = __shfl_xor_sync(0xffffffffu, hi ? m4[j] : m4[2 + j], 8), other2 = __shfl_xor_sync(0xffffffffu, hi ? v4[j] : v4[2 + j], 8);
+        const float mine = hi ? m4[2 + j] : m4[j], d = mine - other;
+        m[j] = 0.5f * (mine + other);
+        v[j] = fmaf(d * d, 0.5f * count, (hi ? v4[2 + j] : v4[j]) + other2);
+    }
+    count += count;
+    float mean = mid ? m[1] : m[0], m2 = mid ? v[1] : v[0];
+    float give_mean = mid ? m[0] : m[1], give_m2 = mid ? v[0] : v[1];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
         const float other = __shfl_xor_sync(0xffffffffu, give_mean, o), other2 = __shfl_xor_sync(0xffffffffu, give_m2, o);
         const float d = mean - other;
         m2 = fmaf(d * d, 0.5f * count, m2 + other2);
@@ -187,11 +255,15 @@ struct NoStage {
 // kAligned: the next LayerNorm's parameters lie on 16-byte boundaries and its rows on 8-byte ones.  Contiguous slices of
 // other tensors need not; they take a build of their own, because the test in the kernel costs every launch
 // instructions to fetch (a step of the 6-layer model at batch 1: 94.5 us, with the test 96.9).
-template <bool kBf16, bool kAligned, typename Stage>
+template <bool kBf16, bool kAligned, bool kWide, bool kMany, typename Stage>
 __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const CUtensorMap& map_w2,
                                                 const LayerTailArgs& a, unsigned char* lt_smem_raw, const Stage& stage) {
-    // W_m, W_2, product GEMM done, second GEMM done; partial sums, pair statistics, residual rows received
-    __shared__ __align__(8) unsigned long long bars[10];         // the second GEMM has one per tile of 128 output rows
+    // W_m, W_2 (own columns), product GEMM done; partial sums, pair statistics, residual rows, shared slice received; W_2 (the
+    // sharing CTA's columns)
+    __shared__ __align__(8) unsigned long long bars[12 + (kWide ? 2 * kLtMaxRing : 0)];      // behind them one per tile of 128 output rows: second GEMM done
+    constexpr int kHC = kWide ? 192 : kLtHC, kOwn = kWide ? 48 : kLtOwn, kOwnStride = kOwn + 1, kSlices = kHC / kBK;
+    constexpr uint32_t kTermStride = 2 * kHC + 16;               // padded row of the staged expanded-cache terms
+    constexpr int kChunks128 = kWide ? 6 : 4;                    // most 128-column chunks of a row
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
     __shared__ int pair_seq_s[kLtMaxPairs];
@@ -204,44 +276,57 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const int s0 = blockIdx.y * a.seqs_per_cluster;
     const int nseq = min(a.n_seq - s0, a.seqs_per_cluster);
     const int pairs = nseq * K;
-    const int pairs_pad = pairs <= 16 ? 16 : (pairs <= 32 ? 32 : 64);
-    const int kblocks = R / kBK, chunks = R / 8, mtiles = D / kBM;
-    const int h0 = static_cast<int>(rank) * kLtHC;
+    const int pairs_pad = !kMany || pairs <= 16 ? 16 : (pairs <= 32 ? 32 : 64);
+    const int kblocks = R / kBK, chunks = R / 8, mtiles = (D / (kWide || kMany ? lt_sharing(D, kMany) : 1)) / kBM, row_tiles = D / kBM;
+    const int h0 = static_cast<int>(rank) * kHC;
+    // this CTA's half of the output rows (g), its place among the CTAs of that half, the CTA that it shares with
+    const int share = kWide ? 2 : kMany ? lt_sharing(D, true) : 1, gs = share - 1, g = static_cast<int>(rank) & gs, place = static_cast<int>(rank) >> gs;
+    const int d_rows = D >> gs, senders = C >> gs;
+    const uint32_t sharer = rank ^ static_cast<uint32_t>(gs);
     const uint32_t fmt = dtype == RLM_BF16 ? 1u : 0u;
     const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(pairs_pad >> 3) << 17) |
                            (static_cast<uint32_t>(kBM >> 4) << 24);
 
     unsigned char* base = smem_align1024(lt_smem_raw);
     const int nq_own = a.query_weight ? a.n_query / C : 0;
-    const LtPlan plan = lt_plan(R, D, pairs_pad, nq_own);
+    const LtPlan plan = lt_plan(R, D, kMany, pairs_pad, nq_own);
     unsigned char* wm_tile = base + plan.wm;
     unsigned char* w2_tile = base + plan.w2;
     unsigned char* p_tile = base + plan.p;
     unsigned char* hid_tile = base + plan.hid;
     unsigned char* term_p = base + plan.term_p;
     unsigned char* term_a = base + plan.term_a;
-    unsigned char* op_a = base + plan.op_a;
+    float2* stats_out = reinterpret_cast<float2*>(base + plan.stats_out);      // this CTA's [pair] (mean, M2)
     const uint32_t p_kblock = static_cast<uint32_t>(pairs_pad) * 128u;
     // A CTA that has received all partial sums knows that every CTA is past its epilogue and its second GEMM: the
     // term rows' place receives the statistics that the CTAs push to one another, [sender][pair] of (mean, M2) over
-    // the sender's 32 columns, and the hidden tile's place the residual rows [sequence][d].
+    // the sender's columns, and the shared slice's place (or W_2's) the residual rows [sequence][d].
     float2* stats_in = reinterpret_cast<float2*>(term_p);
-    float* rows_in = reinterpret_cast<float*>(hid_tile);
+    float* rows_in = reinterpret_cast<float*>(base + plan.rows_in);
     const int row_chunks = pairs_pad / 4, quads = (pairs + 3) >> 2;
-    // LayerNorm parameters of this thread's owned column (column = lane), read before the dependency wait
-    const int own0 = static_cast<int>(rank) * kLtOwn;
-    const float pre_g = a.norm_w[own0 + lane], pre_bt = a.norm_b[own0 + lane];
-    const float pre_bias = load_scalar(a.second_bias, own0 + lane, dtype);
+    // LayerNorm parameters of this thread's owned columns, read before the dependency wait
+    const int own0 = g * d_rows + place * kOwn;
+    // (wide: a half-warp has the owned columns, three to a lane)
+    const int column = kWide ? lane & 15 : lane;
+    constexpr int kOwnPer = kWide ? 3 : 1;
+    float pre_g[kOwnPer], pre_bt[kOwnPer], pre_bias[kOwnPer];
+#pragma unroll
+    for (int i = 0; i < kOwnPer; ++i) {
+        pre_g[i] = a.norm_w[own0 + column + 16 * i];
+        pre_bt[i] = a.norm_b[own0 + column + 16 * i];
+        pre_bias[i] = load_scalar(a.second_bias, own0 + column + 16 * i, dtype);
+    }
     // warps that share a sequence at the end: warp = part x nseq + sequence
     const int my_seq = warp % nseq, part = warp / nseq, parts = (kLtThreads / 32) / nseq;
     // ... and the parameters of the next LayerNorm for the 128-column chunks part, part + parts, ... of a row
-    float4 next_g[4], next_b[4];
+    float4 next_g[kChunks128], next_b[kChunks128];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        if (part + i * parts < mtiles && part < parts) {
+    for (int i = 0; i < kChunks128; ++i)
+        if (part + i * parts < row_tiles && part < parts) {
             next_g[i] = lt_load4<kAligned>(a.next_w + 128 * (part + i * parts) + 4 * lane);
             next_b[i] = lt_load4<kAligned>(a.next_b + 128 * (part + i * parts) + 4 * lane);
         }
+    const float per = 1.0f / static_cast<float>(C), inv_d = 1.0f / static_cast<float>(D);
     int tpo = 16;                                              // threads per projection output: 2 .. 16
     while (tpo > 2 && (nseq * nq_own * tpo > kLtThreads || (D / 8) / tpo < 2)) tpo >>= 1;
     const uint32_t wq_stride = static_cast<uint32_t>(D) * 2u + 16u * static_cast<uint32_t>(tpo);
@@ -260,32 +345,62 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     const uint32_t bar_wm = smem_u32(&bars[0]), bar_w2 = smem_u32(&bars[1]);
     const uint32_t bar_d1 = smem_u32(&bars[2]), bar_part = smem_u32(&bars[3]), bar_stat = smem_u32(&bars[4]), bar_rows = smem_u32(&bars[5]);
-    const uint32_t bar_d2 = smem_u32(&bars[6]);                // + 8 per tile
+    const uint32_t bar_hid = smem_u32(&bars[6]), bar_w2b = smem_u32(&bars[7]);
+    const uint32_t bar_d2 = smem_u32(&bars[8]);                // + 8 per tile
+    // wide: W_2's tiles n = ([this CTA's, the sharing CTA's][K-block][tile_at(i)]) go through a ring
+    const int ring = plan.ring;
+    const auto bar_full = [&](int slot) { return smem_u32(&bars[12 + (kWide ? slot : 0)]); };
+    const auto bar_empty = [&](int slot) { return smem_u32(&bars[12 + (kWide ? kLtMaxRing + slot : 0)]); };
+    // The CTAs take the tiles of output rows in different orders, so that their partial sums go to all CTAs at any
+    // time: in one order, four of sixteen received and the last ones' sums came late.
+    const auto tile_at = [&](int i) { return kWide ? (i + place) % 3 : (i + place) & (mtiles - 1); };
+    const auto request_w2 = [&](int n) {
+        const int other = n / 9, kb = n / 3 - 3 * other, mt = tile_at(n % 3), slot = n % ring;
+        mbar_expect_tx(bar_full(slot), kLtW2Tile);
+        tma_load_2d(smem_u32(w2_tile) + slot * kLtW2Tile, &map_w2, (other ? static_cast<int>(sharer) : static_cast<int>(rank)) * kHC + kb * kBK,
+                    g * d_rows + mt * kBM, bar_full(slot));
+    };
+    const uint32_t slice_rows = static_cast<uint32_t>((pairs + 7) & ~7) * 128u;          // bytes of a K-block that hold pairs
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_wm) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
-        for (int i = 0; i < 10; ++i) mbar_init(smem_u32(&bars[i]), 1);
+        for (int i = 0; i < 12 + (kWide ? 2 * kLtMaxRing : 0); ++i) mbar_init(smem_u32(&bars[i]), 1);
         fence_barrier_init();
-        mbar_expect_tx(bar_part, static_cast<uint32_t>(C * quads) * 512u);
-        mbar_expect_tx(bar_stat, static_cast<uint32_t>(C * pairs) * 8u);
+        mbar_expect_tx(bar_part, static_cast<uint32_t>(senders * quads) * (kOwn * 16u));
+        mbar_expect_tx(bar_stat, static_cast<uint32_t>(C * ((pairs + 1) & ~1)) * 8u);
         mbar_expect_tx(bar_rows, static_cast<uint32_t>(nseq * D) * 4u);
         failed = 0;
         // the weight slices do not depend on earlier kernels: requested before the dependency wait
-        mbar_expect_tx(bar_wm, static_cast<uint32_t>(kblocks) * kBM * 128u);
+        mbar_expect_tx(bar_wm, static_cast<uint32_t>(kblocks) * kHC * 128u);
         for (int kb = 0; kb < kblocks; ++kb)
-            tma_load_2d(smem_u32(wm_tile) + kb * kBM * 128u, &map_wm, kb * kBK, h0, bar_wm);
-        mbar_expect_tx(bar_w2, static_cast<uint32_t>(mtiles) * 2u * kBM * 128u);
-        for (int mt = 0; mt < mtiles; ++mt)
+            tma_load_2d(smem_u32(wm_tile) + kb * kHC * 128u, &map_wm, kb * kBK, h0, bar_wm);
+        // W_2: this half's output rows, by K-block of hidden columns: this CTA's two, then the sharing CTA's
+        if (kWide)
+            for (int n = 0; n < ring; ++n) request_w2(n);
+        for (int other = 0; !kWide && other < share; ++other) {
+            const uint32_t bar = other ? bar_w2b : bar_w2;
+            const int from = (other ? static_cast<int>(sharer) : static_cast<int>(rank)) * kLtHC;
+            mbar_expect_tx(bar, static_cast<uint32_t>(mtiles) * 2u * kBM * 128u);
             for (int kb = 0; kb < 2; ++kb)
-                tma_load_2d(smem_u32(w2_tile) + (mt * 2 + kb) * kBM * 128u, &map_w2, h0 + kb * kBK, mt * kBM, bar_w2);
+                for (int mt = 0; mt < mtiles; ++mt)
+                    tma_load_2d(smem_u32(w2_tile) + ((2 * other + kb) * mtiles + mt) * kBM * 128u, &map_w2, from + kb * kBK,
+                                g * d_rows + mt * kBM, bar);
+        }
+        if (share > 1) mbar_expect_tx(bar_hid, kSlices * slice_rows);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    const int entry = tid >> 2, quarter = tid & 3, bl = entry / K;      // bl: sequence of pair `entry`
-    if (!Stage::kActive && pairs_pad == 16) request_wq();       // a parameter: before the dependency wait
+    if (kWide || kMany) {                                      // every CTA's barriers are initialised (few: see the next barrier)
+        __syncwarp();
+        lt_cluster_sync();
+    }
+    // the threads of a pair (16, 8 or 4), this thread's place among them, the pair's sequence
+    const int tpp_shift = pairs_pad == 16 ? 4 : pairs_pad == 32 ? 3 : 2, tpp = 1 << tpp_shift;
+    const int entry = tid >> tpp_shift, sub = tid & (tpp - 1), bl = entry / K, quarter = tid & 3;
+    if (!kWide && !Stage::kActive && pairs_pad == 16) request_wq();       // a parameter: before the dependency wait
     // the kernel's parameters that are first used behind the wait, into the constant cache
     asm volatile("" ::"l"(a.operand_cache), "l"(a.expanded_cache), "l"(a.anchor_index), "l"(a.partner_index), "l"(a.partner_scores),
                  "l"(a.position), "l"(a.residual), "l"(a.mix), "l"(a.normalized), "l"(a.query), "r"(a.max_t), "f"(a.eps),
@@ -300,20 +415,23 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     }
     if (Stage::kActive && pairs_pad == 16) request_wq();        // its place was the stage's until here
     // the residual stream was written by the previous kernel: requested now, used at the very end
-    const float pre_res = a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane];
+    constexpr int kResPer = kWide ? 2 : 1;
+    float pre_res[kResPer];
+#pragma unroll
+    for (int i = 0; i < kResPer; ++i) pre_res[i] = a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + min(lane + 32 * i, kOwn - 1)];
     const float pre_mix = *a.mix;
 
-    // ---- gathers.  Four threads share a row to gather: they read its index themselves (one
-    // broadcast load) and issue their quarter of its copies at once, so no shared-memory round
-    // trip lies between the selector's indices and the first gather.  Partner operand rows go
-    // straight into the swizzled product tile; copy group 0 = operand rows (needed by the
-    // product GEMM), group 1 = this CTA's 128 columns of the two expanded-cache terms (needed by
-    // its epilogue).  Indices and scores are all requested before the first is used, and the
-    // anchors' rows are gathered by threads that a small batch's partner rows leave free.
+    // ---- gathers.  Some threads share a pair: they read its two indices themselves (broadcast loads) and request their
+    // parts of its operand rows into registers at once, so that neither a shared-memory round trip nor a barrier lies
+    // between the selector's indices and the products, which go straight into the swizzled tile.  Behind them, by
+    // cp.async, this CTA's columns of the two expanded-cache terms, needed by the epilogue.  (Operand rows by cp.async,
+    // multiplied in place behind a barrier: 2 850 cycles from the wait to the products at batch 1, now 1 360.)  The scores are
+    // requested with the indices; the anchors' terms are gathered by threads that a small batch's pairs leave free.
     const size_t op_row = static_cast<size_t>(R) * 2, ex_row = static_cast<size_t>(H) * 4;
-    const int a_entry = (tid - kLtThreads / 2) >> 2;          // sequence whose anchor this thread gathers
+    const int a_entry = (tid - kLtThreads / 2) >> 2;          // sequence whose anchor's terms this thread gathers
     const bool gathers_anchor = tid >= kLtThreads / 2 && a_entry < nseq;
     const int partner = entry < pairs ? a.partner_index[static_cast<size_t>(s0) * K + entry] : 0;
+    const int pair_anchor = entry < pairs ? a.anchor_index[s0 + bl] : 0;
     const int anchor = gathers_anchor ? a.anchor_index[s0 + a_entry] : 0;
     // scores of one sequence per warp, for the softmax weights
     const int weighted = kLtThreads / 32 - 1 - warp;
@@ -324,63 +442,59 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const bool bad_position = t < 0 || t >= a.max_t;          // the same in every CTA of the grid
     const int my_pair_row = min(max(partner, 0), a.max_t - 1);      // empty slots carry a sentinel that may be negative
     const int my_anchor_row = min(max(anchor, 0), a.max_t - 1);
-    if (entry < pairs) {
-        if (quarter == 0) pair_seq_s[entry] = bl;
-        const char* src = static_cast<const char*>(a.operand_cache) +
-                          (static_cast<size_t>(s0 + bl) * a.max_t + my_pair_row) * op_row;
-        for (int c = quarter; c < chunks; c += 4)
-            cp_async16(smem_u32(p_tile) + swizzled(entry, c, p_kblock), src + 16 * c);
-    } else if (entry < pairs_pad) {
-        for (int c = quarter; c < chunks; c += 4)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};"
-                         ::"r"(smem_u32(p_tile) + swizzled(entry, c, p_kblock)), "r"(0) : "memory");
-    }
-    if (gathers_anchor) {
-        const char* src = static_cast<const char*>(a.operand_cache) +
-                          (static_cast<size_t>(s0 + a_entry) * a.max_t + my_anchor_row) * op_row;
-        for (int c = quarter; c < chunks; c += 4)
-            cp_async16(smem_u32(op_a) + static_cast<uint32_t>(a_entry * R * 2 + 16 * c), src + 16 * c);
-    }
-    cp_async_commit();
-    if (entry < pairs) {
-        const char* src = static_cast<const char*>(a.expanded_cache) +
-                          (static_cast<size_t>(s0 + bl) * a.max_t + my_pair_row) * ex_row +
-                          static_cast<size_t>(H + h0) * 2;
+    const size_t seq_row = static_cast<size_t>(s0 + bl) * a.max_t;
+    const uint4* partner_op = reinterpret_cast<const uint4*>(static_cast<const char*>(a.operand_cache) + (seq_row + my_pair_row) * op_row) + sub;
+    const uint4* anchor_op = reinterpret_cast<const uint4*>(static_cast<const char*>(a.operand_cache) + (seq_row + min(max(pair_anchor, 0), a.max_t - 1)) * op_row) + sub;
+    uint4 pv[4], av[4];                                        // four chunks of a row at a time
+    const auto request = [&](int c0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            cp_async16(smem_u32(term_p) + entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
+        for (int i = 0; i < 4; ++i) {
+            const bool in = entry < pairs && c0 + tpp * i + sub < chunks;
+            pv[i] = in ? partner_op[c0 + tpp * i] : make_uint4(0, 0, 0, 0);
+            av[i] = in ? anchor_op[c0 + tpp * i] : make_uint4(0, 0, 0, 0);
+        }
+    };
+    request(0);
+    if (entry < pairs) {
+        if (sub == 0) pair_seq_s[entry] = bl;
+        const char* src = static_cast<const char*>(a.expanded_cache) + (seq_row + my_pair_row) * ex_row + static_cast<size_t>(H + h0) * 2;
+#pragma unroll
+        for (int i = 0; i < kHC / 32; ++i)
+            if (sub + tpp * i < kHC / 8) cp_async16(smem_u32(term_p) + entry * kTermStride + 16 * (sub + tpp * i), src + 16 * (sub + tpp * i));
     }
     if (gathers_anchor) {
         const char* src = static_cast<const char*>(a.expanded_cache) +
                           (static_cast<size_t>(s0 + a_entry) * a.max_t + my_anchor_row) * ex_row +
                           static_cast<size_t>(h0) * 2;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            cp_async16(smem_u32(term_a) + a_entry * kLtTermStride + 16 * (4 * quarter + i), src + 16 * (4 * quarter + i));
+        for (int i = 0; i < kHC / 32; ++i)
+            cp_async16(smem_u32(term_a) + a_entry * kTermStride + 16 * (kHC / 32 * quarter + i), src + 16 * (kHC / 32 * quarter + i));
     }
     cp_async_commit();
-    cp_async_wait_group1();                                    // the operand rows have arrived
-    __syncthreads();
-    // products o[a] * o[p], in fp32, rounded to the operand dtype, in place
-    for (int i = tid; i < pairs * chunks; i += kLtThreads) {
-        const int j = i / chunks, c = i - j * chunks;
-        unsigned char* at = p_tile + swizzled(j, c, p_kblock);
-        float pv[8], av[8];
-        unpack8(*reinterpret_cast<const uint4*>(at), dtype, pv);
-        unpack8(*reinterpret_cast<const uint4*>(op_a + pair_seq_s[j] * R * 2 + 16 * c), dtype, av);
-        uint4 out;
-        out.x = pack2(pv[0] * av[0], pv[1] * av[1], dtype);
-        out.y = pack2(pv[2] * av[2], pv[3] * av[3], dtype);
-        out.z = pack2(pv[4] * av[4], pv[5] * av[5], dtype);
-        out.w = pack2(pv[6] * av[6], pv[7] * av[7], dtype);
-        *reinterpret_cast<uint4*>(at) = out;
+    // products o[a] * o[p], in fp32, rounded to the operand dtype; zeros in the rows of pairs that do not exist
+    for (int c0 = 0;;) {
+        if (entry < pairs_pad)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (c0 + tpp * i + sub >= chunks) break;
+                float fp[8], fa[8];
+                unpack8(pv[i], dtype, fp);
+                unpack8(av[i], dtype, fa);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                             ::"r"(smem_u32(p_tile) + swizzled(entry, c0 + tpp * i + sub, p_kblock)), "r"(pack2(fp[0] * fa[0], fp[1] * fa[1], dtype)),
+                               "r"(pack2(fp[2] * fa[2], fp[3] * fa[3], dtype)), "r"(pack2(fp[4] * fa[4], fp[5] * fa[5], dtype)),
+                               "r"(pack2(fp[6] * fa[6], fp[7] * fa[7], dtype)) : "memory");
+            }
+        c0 += 4 * tpp;
+        if (c0 >= chunks) break;
+        request(c0);
     }
     fence_proxy_async();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_slot;
-    const uint32_t tmem_d2 = tmem_base + 64u;                 // second GEMM: mtiles x pairs_pad columns from column 64
+    const uint32_t tmem_d2 = tmem_base + (kWide ? 128u : 64u);      // second GEMM: mtiles x pairs_pad columns
 
     // ---- product GEMM: D1[hidden column, pair] = W_m slice x products^T
     if (warp == 0) {
@@ -388,49 +502,82 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         if (!ok) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int kb = 0; kb < kblocks; ++kb) {
-            const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kBM * 128u);
+            const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kHC * 128u);
             const uint64_t dp = smem_desc_sw128(smem_u32(p_tile) + kb * p_kblock);
+            // (192 hidden columns as two overlapping tiles of 128: rows 0 .. 127, rows 64 .. 191)
 #pragma unroll
-            for (int kk = 0; kk < kBK / 16; ++kk)
-                umma_f16_if(tmem_base, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+            for (int half = 0; half < (kWide ? 2 : 1); ++half)
+#pragma unroll
+                for (int kk = 0; kk < kBK / 16; ++kk)
+                    umma_f16_if(tmem_base + 64u * half, dw + half * (64 * 128 >> 4) + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
         }
         umma_commit_if(bar_d1, issue);
     }
     __syncwarp();
-    if (!mbar_wait(bar_d1, 0)) failed = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (pairs_pad == 16) { __syncwarp(); lt_cluster_arrive(); }      // the W_m slice is consumed: its place may receive
     cp_async_wait_all();                                       // the expanded-cache terms have arrived
     __syncthreads();
 
     // ---- epilogue of the product GEMM: + expanded-cache terms, GELU, hidden slice as the K-major
     // B tile of the second GEMM (row = pair, K = this CTA's hidden columns).  Warps 0-3 and 4-7 take
     // every other four pair columns; the columns of pairs that do not exist stay unwritten (their
-    // results are never read).
+    // results are never read).  The terms of the first eight pairs are added up while the GEMM runs.
     {
-        const int hc = 32 * (warp & 3) + lane;                // hidden column == TMEM lane
-        const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        const unsigned char* ta = term_a + hc * 2;
-        const unsigned char* tp = term_p + hc * 2;
-        unsigned char* hrow = hid_tile + static_cast<uint32_t>(hc >> 6) * p_kblock + (hc & 7) * 2;
-        const int hchunk = (hc >> 3) & 7;
-        for (int c = 4 * (warp >> 2); c < pairs; c += 8) {
-            uint32_t v[4];
-            lt_tmem_ld4(tmem_base + lane_base + c, v);
-            float term[4];
+        const int quadrant = warp & 3;
+        const uint32_t lane_base = static_cast<uint32_t>(32 * quadrant) << 16;
+        float term[8];
+        uint32_t ta, tp;
+        unsigned char* hrow;
+        int hchunk;
+        const auto at_column = [&](int hc) {                  // this thread's hidden column
+            ta = smem_u32(term_a) + hc * 2;
+            tp = smem_u32(term_p) + hc * 2;
+            hrow = p_tile + static_cast<uint32_t>(hc >> 6) * p_kblock + (hc & 7) * 2;
+            hchunk = (hc >> 3) & 7;
+        };
+        const auto terms = [&](int c, int step) {             // of pairs c .. c + 3 and c + step .. c + step + 3
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int pr = min(c + j, pairs - 1);
-                term[j] = lt_from16(*reinterpret_cast<const uint16_t*>(ta + pair_seq_s[pr] * kLtTermStride), dtype) +
-                          lt_from16(*reinterpret_cast<const uint16_t*>(tp + pr * kLtTermStride), dtype);
+            for (int j = 0; j < 8; ++j) {
+                const int pr = min(c + (j & 3) + (j & 4 ? step : 0), pairs - 1);
+                uint16_t from_a, from_p;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(from_a) : "r"(ta + pair_seq_s[pr] * kTermStride));
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(from_p) : "r"(tp + pr * kTermStride));
+                term[j] = lt_from16(from_a, dtype) + lt_from16(from_p, dtype);
             }
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        };
+        const auto finish = [&](uint32_t from, int c, int step) {      // fours of pairs c, c + step, .. of the accumulator at `from`
+            for (; c < pairs; c += 2 * step) {
+                uint32_t v[8];
+                lt_tmem_ld4(from + lane_base + c, *reinterpret_cast<uint32_t(*)[4]>(&v[0]));
+                if (c + step < pairs) lt_tmem_ld4(from + lane_base + c + step, *reinterpret_cast<uint32_t(*)[4]>(&v[4]));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const auto store = [&](int pr, float h) {
+                    *reinterpret_cast<uint16_t*>(hrow + (pr >> 3) * 1024 + (pr & 7) * 128 + ((hchunk ^ (pr & 7)) << 4)) = lt_to16(h, dtype);
+                };
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int pr = c + j;
-                *reinterpret_cast<uint16_t*>(hrow + (pr >> 3) * 1024 + (pr & 7) * 128 + ((hchunk ^ (pr & 7)) << 4)) =
-                    lt_to16(gelu_tc(__uint_as_float(v[j]) + term[j]), dtype);
+                for (int j = 0; j < 8; j += 2) {
+                    if (j >= 4 && c + step >= pairs) break;
+                    const int pr = c + (j & 3) + (j & 4 ? step : 0);
+                    const float2 h = gelu_pair(make_float2(__uint_as_float(v[j]) + term[j], __uint_as_float(v[j + 1]) + term[j + 1]));
+                    store(pr, h.x);
+                    store(pr + 1, h.y);
+                }
+                if (c + 2 * step < pairs) terms(c + 2 * step, step);
             }
+        };
+        // Wide: quadrants 0, 1 have columns 0 .. 63 in the first tile, quadrants 2, 3 columns 128 .. 191 in the second; of
+        // columns 64 .. 127, which both tiles hold, every quadrant of the four takes every fourth four of pairs.
+        const bool upper = kWide && quadrant >= 2;
+        at_column(32 * quadrant + lane + (upper ? 64 : 0));
+        terms(4 * (warp >> 2), 8);
+        if (!mbar_wait(bar_d1, 0)) failed = 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (pairs_pad == 16) { __syncwarp(); lt_cluster_arrive(); }      // the W_m slice is consumed: its place may receive
+        finish(tmem_base + (upper ? 64u : 0u), 4 * (warp >> 2), 8);
+        if (kWide) {
+            const int first = 4 * ((warp >> 2) + (upper ? 2 : 0));
+            at_column(64 + 32 * (quadrant & 1) + lane);
+            if (first < pairs) terms(first, 16);
+            finish(tmem_base + (upper ? 0u : 64u), first, 16);
         }
     }
     fence_proxy_async();
@@ -440,21 +587,57 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
 
     // ---- second GEMM, split over the cluster along the hidden width:
     // D2[output row, pair] (partial) = W_2[:, this CTA's hidden columns] x hidden slice^T
-    if (warp == 0) {
-        const bool ok = mbar_wait(bar_w2, 0), issue = elect_lane();
-        if (!ok) failed = 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int mt = 0; mt < mtiles; ++mt) {
-#pragma unroll
-            for (int kb = 0; kb < 2; ++kb) {
-                const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + (mt * 2 + kb) * kBM * 128u);
-                const uint64_t dh = smem_desc_sw128(smem_u32(hid_tile) + kb * p_kblock);
+    // (by two warps: one issues an instruction every 50 cycles, a narrow one takes 32)
+    // The sharing CTA's slice is on its way while this CTA's own is multiplied.
+    if (share > 1 && tid == 32 * 2)
+        for (int kb = 0; kb < kSlices; ++kb)
+            lt_copy_cluster(lt_peer(smem_u32(hid_tile) + kb * p_kblock, sharer), smem_u32(p_tile) + kb * p_kblock, slice_rows, lt_peer(bar_hid, sharer));
+    if (kWide) {
+        if (warp == 0 || warp == 1 || warp == 3) {             // a tile of output rows each
+            const int i = warp == 3 ? 2 : warp, mt = tile_at(i);
+            const bool issue = elect_lane();
+            bool ok = true;
+            for (int n = i; n < 18; n += 3) {
+                const int other = n / 9, kb = n / 3 - 3 * other, slot = n % ring;
+                if (n == 9 + i) ok = mbar_wait(bar_hid, 0) && ok;
+                ok = mbar_wait(bar_full(slot), (n / ring) & 1) && ok;
+                if (!ok) failed = 1;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + slot * kLtW2Tile);
+                const uint64_t dh = smem_desc_sw128(smem_u32(other ? hid_tile : p_tile) + kb * p_kblock);
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; ++kk)
-                    umma_f16_if(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
-                            (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+                    umma_f16_if(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc, (n > i || kk > 0) ? 1u : 0u, issue && ok);
+                umma_commit_if(bar_empty(slot), issue);
             }
-            umma_commit_if(bar_d2 + 8u * mt, issue);                // each tile's partial sums leave while the next is computed
+            umma_commit_if(bar_d2 + 8u * mt, issue);
+        } else if (warp == 2 && lane == 0) {
+            for (int n = ring; n < 18; ++n) {
+                if (!mbar_wait(bar_empty(n % ring), (n / ring - 1) & 1)) { failed = 1; break; }
+                request_w2(n);
+            }
+        }
+    } else if (warp < 2) {
+        const bool issue = elect_lane();
+        bool ok = true;
+        for (int other = 0; other < share; ++other) {
+            ok = mbar_wait(other ? bar_w2b : bar_w2, 0) && (!other || mbar_wait(bar_hid, 0)) && ok;
+            if (!ok) failed = 1;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t slice = smem_u32(other ? hid_tile : p_tile);
+            for (int i = warp; i < mtiles; i += 2) {
+                const int mt = tile_at(i);
+#pragma unroll
+                for (int kb = 0; kb < 2; ++kb) {
+                    const uint64_t dw = smem_desc_sw128(smem_u32(w2_tile) + ((2 * other + kb) * mtiles + mt) * kBM * 128u);
+                    const uint64_t dh = smem_desc_sw128(slice + kb * p_kblock);
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        umma_f16_if(tmem_d2 + static_cast<uint32_t>(mt * pairs_pad), dw + 2 * kk, dh + 2 * kk, idesc,
+                                (other > 0 || kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+                }
+                if (other + 1 == share) umma_commit_if(bar_d2 + 8u * mt, issue);      // each tile's partial sums leave while the next is computed
+            }
         }
     }
     __syncwarp();
@@ -487,100 +670,126 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     unsigned char* recv = pairs_pad == 16 ? wm_tile : w2_tile;
     {
         const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-        // few pairs: by the last four warps alone, a tile behind the GEMM that warp 0 is still issuing
-        const int first = pairs_pad > 16 ? warp >> 2 : warp >= 4 ? 0 : mtiles, step = pairs_pad > 16 ? 2 : 1;
-        for (int mt = first; mt < mtiles; mt += step) {
+        // few pairs in four tiles: by the last four warps alone, a tile behind the GEMM that the first two are still issuing
+        const bool behind = share == 1 && pairs_pad == 16;
+        for (int i = behind ? (warp >= 4 ? 0 : mtiles) : warp >> 2; i < mtiles; i += behind ? 1 : 2) {
+            const int mt = tile_at(i);
             if (!mbar_wait(bar_d2 + 8u * mt, 0)) failed = 1;
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t owner = static_cast<uint32_t>(4 * mt + (warp & 3));
+            const int row = mt * kBM + 32 * (warp & 3) + lane, owner_place = row / kOwn;      // (narrow: the same in the warp)
+            const uint32_t owner = static_cast<uint32_t>((owner_place << gs) | g);
             const uint32_t bar = lt_peer(bar_part, owner);
-            const uint32_t dst = lt_peer(smem_u32(recv), owner) + (rank * row_chunks * 32u + lane) * 16u;
+            const uint32_t dst = lt_peer(smem_u32(recv), owner) + static_cast<uint32_t>(place * row_chunks * kOwn + row - owner_place * kOwn) * 16u;
             for (int c = 0; c < pairs; c += 16) {              // the accumulator has 16, 32 or 64 columns
                 uint32_t v[8], w[8];
                 tmem_ld8(tmem_d2 + lane_base + static_cast<uint32_t>(mt * pairs_pad + c), v);
                 tmem_ld8(tmem_d2 + lane_base + static_cast<uint32_t>(mt * pairs_pad + c + 8), w);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const uint32_t at = dst + static_cast<uint32_t>(c >> 2) * 512u;
+                constexpr uint32_t kFour = kOwn * 16u;
+                const uint32_t at = dst + static_cast<uint32_t>(c >> 2) * kFour;
                 lt_push16(at, bar, v[0], v[1], v[2], v[3]);
-                if (c + 4 < pairs) lt_push16(at + 512u, bar, v[4], v[5], v[6], v[7]);
-                if (c + 8 < pairs) lt_push16(at + 1024u, bar, w[0], w[1], w[2], w[3]);
-                if (c + 12 < pairs) lt_push16(at + 1536u, bar, w[4], w[5], w[6], w[7]);
+                if (c + 4 < pairs) lt_push16(at + kFour, bar, v[4], v[5], v[6], v[7]);
+                if (c + 8 < pairs) lt_push16(at + 2 * kFour, bar, w[0], w[1], w[2], w[3]);
+                if (c + 12 < pairs) lt_push16(at + 3 * kFour, bar, w[4], w[5], w[6], w[7]);
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 
-    // ---- a warp owns four pairs (32 columns, a lane each): partial sums in a fixed order, so that the result does
-    // not depend on timing, and (mean, M2) of the 32 columns, pushed to every CTA
+    // ---- a warp (wide: a half-warp) owns four pairs and all owned columns: partial sums in a fixed order, so that the
+    // result does not depend on timing, and (mean, M2) of the owned columns, pushed to every CTA
+    if (kWide && pairs_pad == 16) {                            // the W_q slice, in the ring's place
+        for (int mt = 0; mt < mtiles; ++mt)
+            if (!mbar_wait(bar_d2 + 8u * mt, 0)) failed = 1;
+        request_wq();
+        cp_async_commit();
+    }
     if (!mbar_wait(bar_part, 0)) failed = 1;
-    float x[2][4];
+    constexpr int kIters = kWide ? 1 : 2, kPairLanes = kWide ? 4 : 8;
+    const int first_lane = kWide ? lane & 16 : 0, sub_lane = lane - first_lane;
+    const auto quad_at = [&](int it) { return kWide ? 2 * warp + (lane >> 4) : warp + 8 * it; };
+    const auto quad_none = [&](int it) { return (kWide ? 2 * warp : warp + 8 * it) >= quads; };      // for the whole warp
+    float x[kIters][kOwnPer][4];
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const int q = warp + 8 * it;
-        if (q >= quads) break;
-        const unsigned char* src = recv + (static_cast<uint32_t>(q) * 32u + lane) * 16u;
-        float4 part_sum[4];                                    // senders of equal rank modulo four (C is 4, 8 or 16)
+    for (int it = 0; it < kIters; ++it) {
+        if (quad_none(it)) break;
+        const int q = min(quad_at(it), quads - 1);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            part_sum[k] = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(k * row_chunks) * 512u);
+        for (int i = 0; i < kOwnPer; ++i) {
+            const unsigned char* src = recv + static_cast<uint32_t>(q * kOwn + column + 16 * i) * 16u;
+            const uint32_t sender = static_cast<uint32_t>(row_chunks * kOwn) * 16u;
+            float4 part_sum[4];                                // senders of equal place modulo four (4, 8 or 16 of them)
 #pragma unroll
-        for (int s = 4; s < 16; s += 4) {
-            if (s >= C) break;
+            for (int k = 0; k < 4; ++k) part_sum[k] = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(k) * sender);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float4 v = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>((s + k) * row_chunks) * 512u);
-                part_sum[k].x += v.x; part_sum[k].y += v.y; part_sum[k].z += v.z; part_sum[k].w += v.w;
+            for (int first = 4; first < (kWide ? 8 : 16); first += 4) {
+                if (first >= senders) break;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 v = *reinterpret_cast<const float4*>(src + static_cast<uint32_t>(first + k) * sender);
+                    part_sum[k].x += v.x; part_sum[k].y += v.y; part_sum[k].z += v.z; part_sum[k].w += v.w;
+                }
             }
+            x[it][i][0] = (part_sum[0].x + part_sum[1].x) + (part_sum[2].x + part_sum[3].x) + pre_bias[i];
+            x[it][i][1] = (part_sum[0].y + part_sum[1].y) + (part_sum[2].y + part_sum[3].y) + pre_bias[i];
+            x[it][i][2] = (part_sum[0].z + part_sum[1].z) + (part_sum[2].z + part_sum[3].z) + pre_bias[i];
+            x[it][i][3] = (part_sum[0].w + part_sum[1].w) + (part_sum[2].w + part_sum[3].w) + pre_bias[i];
         }
-        float4 acc;
-        acc.x = (part_sum[0].x + part_sum[1].x) + (part_sum[2].x + part_sum[3].x);
-        acc.y = (part_sum[0].y + part_sum[1].y) + (part_sum[2].y + part_sum[3].y);
-        acc.z = (part_sum[0].z + part_sum[1].z) + (part_sum[2].z + part_sum[3].z);
-        acc.w = (part_sum[0].w + part_sum[1].w) + (part_sum[2].w + part_sum[3].w);
-        x[it][0] = acc.x + pre_bias; x[it][1] = acc.y + pre_bias; x[it][2] = acc.z + pre_bias; x[it][3] = acc.w + pre_bias;
-        const float2 moments = lt_moments4(x[it]);
-        const int pr = 4 * q + (lane >> 3);
-        if (pr < pairs) {
-            const uint32_t at = smem_u32(&stats_in[rank * pairs_pad + pr]);
-            for (uint32_t to = lane & 7; to < static_cast<uint32_t>(C); to += 8) lt_push8(lt_peer(at, to), lt_peer(bar_stat, to), moments.x, moments.y);
+        float2 moments;
+        if constexpr (kWide) moments = lt_moments4(x[it]);
+        else moments = lt_moments4(x[it][0]);
+        const int pr = 4 * q + sub_lane / kPairLanes;
+        if (pr < pairs && quad_at(it) < quads && sub_lane % kPairLanes == 0) stats_out[pr] = moments;
+    }
+    __syncthreads();
+    // ... in messages of sixteen bytes (64 pairs: this exchange took 3 900 cycles with eight bytes a message)
+    if (lane < (pairs + 1) >> 1) {                             // a lane two pairs, a warp two or one of the CTAs
+        const float4 m = *reinterpret_cast<const float4*>(&stats_out[2 * lane]);
+        const uint32_t at = smem_u32(&stats_in[rank * pairs_pad + 2 * lane]);
+        for (uint32_t i = warp; i < static_cast<uint32_t>(C); i += kLtThreads / 32) {
+            const uint32_t to = (i + rank) & static_cast<uint32_t>(C - 1);
+            lt_push16(lt_peer(at, to), lt_peer(bar_stat, to), __float_as_uint(m.x), __float_as_uint(m.y), __float_as_uint(m.z), __float_as_uint(m.w));
         }
     }
 
-    // ---- the pairs' statistics over the full width (equal counts: Chan's parallel variance), eight lanes a pair, and
-    // the normalised pairs [pair][kLtOwnStride] for the sequences' weighted sums
+    // ---- the pairs' statistics over the full width (equal counts: Chan's parallel variance), eight (four) lanes a pair, and
+    // the normalised pairs [pair][kOwnStride] for the sequences' weighted sums
     float* own_y = reinterpret_cast<float*>(base + plan.own_y);
     if (!mbar_wait(bar_stat, 0)) failed = 1;
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const int q = warp + 8 * it;
-        if (q >= quads) break;
-        const int pr = min(4 * q + (lane >> 3), pairs - 1), from = lane & 7;
-        // sums of the means' distances from the first one, of their squares and of the M2, in the same three exchanges
+    for (int it = 0; it < kIters; ++it) {
+        if (quad_none(it)) break;
+        const int q = min(quad_at(it), quads - 1);
+        const int pr = min(4 * q + sub_lane / kPairLanes, pairs - 1), from = lane % kPairLanes;
+        // sums of the means' distances from the first one, of their squares and of the M2, in the same exchanges
         const float pivot = stats_in[pr].x;
         float d1 = 0.0f, d2 = 0.0f, m2 = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (from + 8 * i < C) {
-                const float2 st = stats_in[(from + 8 * i) * pairs_pad + pr];
+        for (int i = 0; i < 16 / kPairLanes; ++i)
+            if (from + kPairLanes * i < C) {
+                const float2 st = stats_in[(from + kPairLanes * i) * pairs_pad + pr];
                 const float d = st.x - pivot;
                 d1 += d;
                 d2 = fmaf(d, d, d2);
                 m2 += st.y;
             }
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
+        for (int o = kPairLanes / 2; o > 0; o >>= 1) {
             d1 += __shfl_xor_sync(0xffffffffu, d1, o);
             d2 += __shfl_xor_sync(0xffffffffu, d2, o);
             m2 += __shfl_xor_sync(0xffffffffu, m2, o);
         }
-        const float per = 1.0f / static_cast<float>(C), mean = fmaf(d1, per, pivot);
-        m2 = fmaf(static_cast<float>(kLtOwn), fmaxf(fmaf(-d1 * per, d1, d2), 0.0f), m2);
-        const float rstd = rsqrtf(m2 / static_cast<float>(D) + a.eps);
+        const float mean = fmaf(d1, per, pivot);
+        m2 = fmaf(static_cast<float>(kOwn), fmaxf(fmaf(-d1 * per, d1, d2), 0.0f), m2);
+        const float rstd = rsqrtf(fmaf(m2, inv_d, a.eps));
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float mj = __shfl_sync(0xffffffffu, mean, 8 * j), rj = __shfl_sync(0xffffffffu, rstd, 8 * j);
-            if (4 * q + j < pairs) own_y[(4 * q + j) * kLtOwnStride + lane] = fmaf((x[it][j] - mj) * rj, pre_g, pre_bt);
+            const float mj = __shfl_sync(0xffffffffu, mean, first_lane + kPairLanes * j), rj = __shfl_sync(0xffffffffu, rstd, first_lane + kPairLanes * j);
+            if (4 * q + j < pairs && quad_at(it) < quads)
+#pragma unroll
+                for (int i = 0; i < kOwnPer; ++i)
+                    own_y[(4 * q + j) * kOwnStride + column + 16 * i] = fmaf((x[it][i][j] - mj) * rj, pre_g[i], pre_bt[i]);
         }
     }
     __syncthreads();
@@ -590,25 +799,33 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
 
-    // ---- context and residual update: column = lane; the warps of a sequence share out the CTAs that its updated
-    // columns are pushed to
+    // ---- context and residual update: column = lane (wide: and 32 + lane); the warps of a sequence share out the CTAs
+    // that its updated columns are pushed to
     if (part < parts) {
-        float ctx = 0.0f;
-        for (int k0 = 0; k0 < K; k0 += 8) {
-            float wk[8], y[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int at = my_seq * K + min(k0 + k, K - 1);
-                wk[k] = k0 + k < K ? weight_s[at] : 0.0f;
-                y[k] = own_y[at * kLtOwnStride + lane];
+        for (int i = 0; i < kResPer; ++i) {
+            const int col = lane + 32 * i;
+            if (col >= kOwn) continue;
+            float ctx = 0.0f;
+            for (int k0 = 0; k0 < K; k0 += 8) {
+                float wk[8], y[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int at = my_seq * K + min(k0 + k, K - 1);
+                    wk[k] = k0 + k < K ? weight_s[at] : 0.0f;
+                    y[k] = own_y[at * kOwnStride + col];
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ctx = wk[k] == 0.0f ? ctx : fmaf(wk[k], y[k], ctx);     // inactive slots contribute nothing
             }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) ctx = wk[k] == 0.0f ? ctx : fmaf(wk[k], y[k], ctx);     // inactive slots contribute nothing
+            const float hval = bad_position ? pre_res[i] : fmaf(pre_mix, ctx, pre_res[i]);
+            if (part == 0 && !bad_position) a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + col] = hval;
+            const uint32_t at = smem_u32(&rows_in[my_seq * D + own0 + col]);
+            for (uint32_t to_i = part; to_i < static_cast<uint32_t>(C); to_i += parts) {
+                const uint32_t to = (to_i + rank) & static_cast<uint32_t>(C - 1);
+                lt_push4(lt_peer(at, to), lt_peer(bar_rows, to), hval);
+            }
         }
-        const float hval = bad_position ? pre_res : fmaf(pre_mix, ctx, pre_res);
-        if (part == 0 && !bad_position) a.residual[static_cast<size_t>(s0 + my_seq) * D + own0 + lane] = hval;
-        const uint32_t at = smem_u32(&rows_in[my_seq * D + own0 + lane]);
-        for (uint32_t to = part; to < static_cast<uint32_t>(C); to += parts) lt_push4(lt_peer(at, to), lt_peer(bar_rows, to), hval);
     }
 
     // ---- the next LayerNorm, of whole rows in every CTA: the warps of a sequence share its 128-column chunks
@@ -619,18 +836,18 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     unsigned char* rows16 = base + plan.rows;                  // [sequence][d] of 16 bits
     if (part < parts) {
         const float* row = rows_in + my_seq * D;
-        // local moments of the lane's 4 mtiles columns, then five exchanges of (mean, M2) of equal halves
-        float4 h[4];
+        // local moments of the lane's 4 row_tiles columns, then five exchanges of (mean, M2) of equal halves
+        float4 h[kChunks128];
         float sum = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            h[i] = i < mtiles ? *reinterpret_cast<const float4*>(row + 128 * i + 4 * lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int i = 0; i < kChunks128; ++i) {
+            h[i] = i < row_tiles ? *reinterpret_cast<const float4*>(row + 128 * i + 4 * lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             sum += (h[i].x + h[i].y) + (h[i].z + h[i].w);
         }
-        float count = 4.0f * static_cast<float>(mtiles), mean = sum * (1.0f / count), m2 = 0.0f;      // a power of two
+        float count = 4.0f * static_cast<float>(row_tiles), mean = sum * (1.0f / count), m2 = 0.0f;      
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (i < mtiles) {
+        for (int i = 0; i < kChunks128; ++i)
+            if (i < row_tiles) {
                 const float dx = h[i].x - mean, dy = h[i].y - mean, dz = h[i].z - mean, dw = h[i].w - mean;
                 m2 += fmaf(dx, dx, dy * dy) + fmaf(dz, dz, dw * dw);
             }
@@ -641,14 +858,14 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             mean = 0.5f * (mean + other);
             count += count;
         }
-        const float rstd = rsqrtf(fmaf(m2, 1.0f / static_cast<float>(D), a.next_eps));
+        const float rstd = rsqrtf(fmaf(m2, inv_d, a.next_eps));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kChunks128; ++i) {
             const int chunk = part + i * parts;
-            if (chunk >= mtiles) break;
+            if (chunk >= row_tiles) break;
             float4 v = h[0];
 #pragma unroll
-            for (int k = 1; k < 4; ++k)
+            for (int k = 1; k < kChunks128; ++k)
                 if (chunk == k) v = h[k];
             const float4 g = next_g[i], b = next_b[i];
             const uint2 out = make_uint2(
@@ -656,7 +873,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 pack2(fmaf((v.z - mean) * rstd, g.z, b.z), fmaf((v.w - mean) * rstd, g.w, b.w), dtype));
             const int at = 128 * chunk + 4 * lane;
             *reinterpret_cast<uint2*>(rows16 + (my_seq * D + at) * 2) = out;
-            if (at / kLtOwn == static_cast<int>(rank) && !bad_position) {
+            if (at >= own0 && at < own0 + kOwn && !bad_position) {
                 uint16_t* to = static_cast<uint16_t*>(a.normalized) + static_cast<size_t>(s0 + my_seq) * D + at;
                 if (kAligned) {
                     *reinterpret_cast<uint2*>(to) = out;
@@ -709,7 +926,7 @@ inline bool lt_aligned(const LayerTailArgs& a) {
     return aligned16(a.next_w) && aligned16(a.next_b) && (reinterpret_cast<uintptr_t>(a.normalized) & 7u) == 0;
 }
 
-int lt_validate(const LayerTailArgs& a) {
+int lt_validate(const LayerTailArgs& a, bool wide = false) {
     if (a.n_seq < 1 || a.k_out < 1 || a.k_out > kLtMaxPairs || a.max_t < 1) {
         set_error("relation_layer_tail: sizes must be positive and K at most 64");
         return RLM_ERR_SHAPE;
@@ -718,18 +935,20 @@ int lt_validate(const LayerTailArgs& a) {
         set_error("relation_layer_tail: caches and weights must share bfloat16 or float16");
         return RLM_ERR_UNSUPPORTED;
     }
-    if (a.hdim % kLtHC != 0 || (a.hdim / kLtHC != 4 && a.hdim / kLtHC != 8 && a.hdim / kLtHC != 16) ||
-        a.d % kBM != 0 || a.d > 512 || a.d / (a.hdim / kLtHC) != kLtOwn || a.rdim % kBK != 0 || a.rdim > 256) {
-        set_error("relation_layer_tail: needs H = 4 d with d in {128, 256, 512} and R a multiple of 64 up to 256");
+    if (a.hdim != 4 * a.d || (wide ? a.d != 768 : a.d != 128 && a.d != 256 && a.d != 512) || a.rdim < kBK || a.rdim % kBK != 0 || a.rdim > 256) {
+        set_error(wide ? "relation_layer_tail_wide: needs H = 4 d with d = 768 and R a multiple of 64"
+                       : "relation_layer_tail: needs H = 4 d with d in {128, 256, 512} and R a multiple of 64 up to 256");
         return RLM_ERR_UNSUPPORTED;
     }
-    const int cluster = a.hdim / kLtHC;
+    const int cluster = lt_cluster(a.d);
     if (a.query_weight && (a.n_query < cluster || a.n_query % (16 * cluster) != 0 || a.n_query / cluster > 64 || !a.query ||
-                           static_cast<size_t>(a.n_query / cluster) * (a.d * 2 + 256) > static_cast<size_t>(a.rdim / kBK) * kBM * 128)) {
+                           static_cast<size_t>(a.n_query / cluster) * (a.d * 2 + 256) > static_cast<size_t>(a.rdim / kBK) * lt_hidden(a.d) * 128)) {
         set_error("relation_layer_tail: query projection width must be a multiple of 16 outputs per CTA (H / 128 CTAs), at most 64 each");
         return RLM_ERR_UNSUPPORTED;
     }
-    if (lt_smem_bytes(a.rdim, a.d, a.query_weight ? a.n_query / cluster : 0) > static_cast<uint32_t>(kSmemDynamicLimit)) {
+    // (a ring has to hold what takes its place later: 64 pairs' partial sums are six tiles)
+    if (lt_smem_bytes(a.rdim, a.d, a.query_weight ? a.n_query / cluster : 0) > static_cast<uint32_t>(kSmemDynamicLimit) ||
+        (lt_wide(a.d) && lt_plan(a.rdim, a.d, true, kLtMaxPairs, 0).ring < 6)) {
         set_error("relation_layer_tail: the weight slices exceed 227 KB of shared memory");
         return RLM_ERR_SMEM;
     }

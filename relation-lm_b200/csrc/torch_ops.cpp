@@ -728,7 +728,9 @@ void slot_mix_residual(const Tensor& slot_context, const Tensor& anchor_active, 
                                 f32(gate), f32(hidden), rows, slots, dim, launch.stream));
 }
 
-void relation_layer_tail(const Tensor& expanded_cache, const Tensor& operand_cache, const Tensor& anchor_index,
+using TailCall = decltype(&rlm_relation_layer_tail);
+
+void layer_tail(TailCall launch_tail, const Tensor& expanded_cache, const Tensor& operand_cache, const Tensor& anchor_index,
                          const Tensor& partner_index, const Tensor& partner_scores, const Tensor& product_weight,
                          const Tensor& second_weight, const Tensor& second_bias, const Tensor& norm_weight,
                          const Tensor& norm_bias, const Tensor& position, double norm_eps, Tensor& hidden, const Tensor& mix,
@@ -763,12 +765,32 @@ void relation_layer_tail(const Tensor& expanded_cache, const Tensor& operand_cac
         dtype = same_dtype("16-bit operand", {&expanded_cache, &*query_weight, &*query});
     }
     Launch launch(device);
-    check(rlm_relation_layer_tail(ptr(expanded_cache), ptr(operand_cache), i32(anchor_index), i32(partner_index),
+    check(launch_tail(ptr(expanded_cache), ptr(operand_cache), i32(anchor_index), i32(partner_index),
                                   f32(partner_scores), ptr(product_weight), ptr(second_weight), ptr(second_bias),
                                   f32(norm_weight), f32(norm_bias), i64(position), static_cast<float>(norm_eps), f32(hidden),
                                   f32(mix), f32(next_norm_weight), f32(next_norm_bias), static_cast<float>(next_norm_eps),
                                   ptr(normalized), ptr(query_weight), ptr(query), batch, k_out, max_t, rdim, hdim, dim, n_query,
                                   dtype, launch.status, launch.stream));
+}
+
+#define TAIL_PARAMS                                                                                                      \
+    const Tensor& expanded_cache, const Tensor& operand_cache, const Tensor& anchor_index,                                  \
+        const Tensor &partner_index, const Tensor &partner_scores, const Tensor &product_weight,                          \
+        const Tensor &second_weight, const Tensor &second_bias, const Tensor &norm_weight, const Tensor &norm_bias,      \
+        const Tensor &position, double norm_eps, Tensor &hidden, const Tensor &mix, const Tensor &next_norm_weight,      \
+        const Tensor &next_norm_bias, double next_norm_eps, Tensor &normalized, const OptTensor &query_weight,           \
+        const OptTensor &query
+
+void relation_layer_tail(TAIL_PARAMS) {
+    layer_tail(&rlm_relation_layer_tail, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight, second_weight, second_bias,
+               norm_weight, norm_bias, position, norm_eps, hidden, mix, next_norm_weight, next_norm_bias, next_norm_eps, normalized,
+               query_weight, query);
+}
+
+void relation_layer_tail_wide(TAIL_PARAMS) {
+    layer_tail(&rlm_relation_layer_tail_wide, expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight, second_weight, second_bias,
+               norm_weight, norm_bias, position, norm_eps, hidden, mix, next_norm_weight, next_norm_bias, next_norm_eps, normalized,
+               query_weight, query);
 }
 
 void relation_mlp_rows(Tensor& out, const Tensor& expanded_cache, const Tensor& operand_cache, const Tensor& anchor_index,
@@ -1123,6 +1145,11 @@ Tensor status_word_of(int64_t device_index) { return status_word(static_cast<int
     MUTATES(slot_mix_residual, "(Tensor slot_context, Tensor anchor_active, Tensor slot_weight, Tensor gate, "           \
             "Tensor(a4!) hidden) -> ()")                                                                                 \
     MUTATES(relation_layer_tail, "(Tensor expanded_cache, Tensor operand_cache, Tensor anchor_index, "                   \
+            "Tensor partner_index, Tensor partner_scores, Tensor product_weight, Tensor second_weight, "                 \
+            "Tensor second_bias, Tensor norm_weight, Tensor norm_bias, Tensor position, float norm_eps, "                \
+            "Tensor(a12!) hidden, Tensor mix, Tensor next_norm_weight, Tensor next_norm_bias, float next_norm_eps, "     \
+            "Tensor(a17!) normalized, Tensor? query_weight, Tensor(a19!)? query) -> ()")                                 \
+    MUTATES(relation_layer_tail_wide, "(Tensor expanded_cache, Tensor operand_cache, Tensor anchor_index, "              \
             "Tensor partner_index, Tensor partner_scores, Tensor product_weight, Tensor second_weight, "                 \
             "Tensor second_bias, Tensor norm_weight, Tensor norm_bias, Tensor position, float norm_eps, "                \
             "Tensor(a12!) hidden, Tensor mix, Tensor next_norm_weight, Tensor next_norm_bias, float next_norm_eps, "     \

@@ -35,6 +35,7 @@ from relation_lm.kernels.packed_projection import (decode_embed_norm, decode_fro
                                                     skinny_projection_supported)
 from relation_lm.kernels.relation_reduce import (expanded_cache_append, expanded_cache_append_packed,
                                                  relation_layer_tail, relation_layer_tail_supported,
+                                                 relation_layer_tail_wide, relation_layer_tail_wide_supported,
                                                  relation_hidden_cached_out,
                                                  relation_hidden_cache_update_out,
                                                  relation_norm_reduce_residual_norm,
@@ -108,10 +109,16 @@ class StatefulDecoder:
         self.fused_query = can_fuse_query and (B <= 12 if fused_query is None else bool(fused_query))
         # The whole relation tail of a layer (relation hidden, second MLP layer, norm-reduce, residual,
         # next LayerNorm, next query projection) as ONE cluster launch with the hidden states on chip:
-        # two launches per layer and no library GEMM in the step, for small batches of d <= 512.
-        can_tail = (self.fused and not self.fused_tail and self.second_layer_splits == 1 and self.stacked_expand
-                    and B <= 64 and relation_layer_tail_supported(B, cfg.k_max, R, H, cfg.d_model, n_query, dtype))
-        self.layer_tail = can_tail if layer_tail is None else (bool(layer_tail) and can_tail)
+        # two launches per layer and no library GEMM in the step, for small batches of d <= 512 and of d 768.
+        sizes = (B, cfg.k_max, R, H, cfg.d_model, n_query, dtype)
+        wide = cfg.d_model == 768
+        can_tail = (self.fused and not self.fused_tail and self.second_layer_splits == 1 and self.stacked_expand and B <= 64
+                    and (relation_layer_tail_wide_supported(*sizes) if wide else relation_layer_tail_supported(*sizes)))
+        self._tail = relation_layer_tail_wide if wide else relation_layer_tail
+        # (d 768 below 256 pairs; us per step of 12 layers with the tail / with four or five launches a layer: 255 / 338
+        # for 8 sequences, 387 / 481 for 28, 397 / 355 for 32, whose hidden states take the tensor-core kernel there)
+        by_default = can_tail and not (wide and B * cfg.k_max >= 256)
+        self.layer_tail = by_default if layer_tail is None else (bool(layer_tail) and can_tail)
         if self.layer_tail:
             self.fused_query = False
         self.query = zeros(B, n_query) if self.fused else zeros(L, B, n_query)
@@ -441,10 +448,10 @@ class StatefulDecoder:
                          "hidden_before": hidden.clone()}
                 trace.append(entry)
             if self.layer_tail:
-                relation_layer_tail(*layer.caches, anchor, partner, partner_score, layer.first_layer[2],
-                                    *layer.second_layer, *layer.relation_norm, pos, cfg.norm_eps, hidden, layer.mix,
-                                    next_w, next_b, cfg.norm_eps, self.normalized, layer.next_query,
-                                    None if last else self.query)
+                self._tail(*layer.caches, anchor, partner, partner_score, layer.first_layer[2],
+                           *layer.second_layer, *layer.relation_norm, pos, cfg.norm_eps, hidden, layer.mix,
+                           next_w, next_b, cfg.norm_eps, self.normalized, layer.next_query,
+                           None if last else self.query)
                 if trace is not None:
                     entry.update(hidden_after=hidden.clone(), next_normalized=self.normalized.clone())
                     if not last:

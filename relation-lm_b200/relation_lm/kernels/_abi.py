@@ -52,6 +52,8 @@ PROTOTYPES = {
     "rlm_state_slide": [_P, _P, _P, _P, _P, _I, _P],
     "rlm_decode_front": [_P] * 6 + [_F] + [_P] * 4 + [_F] + [_P] * 6 + [_I] * 8 + [_P, _P],
     "rlm_relation_layer_tail_supported": [_I] * 7,
+    "rlm_relation_layer_tail_wide_supported": [_I] * 7,
+    "rlm_relation_layer_tail_wide": [_P] * 11 + [_F, _P, _P, _P, _P, _F, _P, _P, _P] + [_I] * 8 + [_P, _P],
     "rlm_relation_layer_tail": [_P] * 11 + [_F, _P, _P, _P, _P, _F, _P, _P, _P] + [_I] * 8 + [_P, _P],
     "rlm_sequence_state": [_P, _L, _I, _I] + [_P] * 14 + [_I] * 5 + [_P],
     "rlm_relation_mlp_rows_supported": [_I] * 6,

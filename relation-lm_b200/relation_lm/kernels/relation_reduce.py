@@ -31,6 +31,7 @@ _relation_hidden_cached_rows_out = _abi.operator("relation_hidden_cached_rows_ou
 _relation_norm_reduce_rows = _abi.operator("relation_norm_reduce_rows")
 _relation_mlp_rows = _abi.operator("relation_mlp_rows")
 _relation_layer_tail = _abi.operator("relation_layer_tail")
+_relation_layer_tail_wide = _abi.operator("relation_layer_tail_wide")
 
 
 @dataclass(frozen=True)
@@ -574,6 +575,34 @@ def relation_layer_tail(
 
 
 @torch.library.register_fake("relation_lm::relation_layer_tail")
+def _(expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight,
+      second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, hidden, mix,
+      next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query):
+    return None
+
+
+def relation_layer_tail_wide_supported(n_seq: int, k_out: int, relation_dim: int, hidden_dim: int, d_model: int,
+                                       n_query: int, dtype: torch.dtype) -> bool:
+    """Whether ``relation_layer_tail_wide`` serves these sizes on the current device."""
+    if dtype not in (torch.bfloat16, torch.float16):
+        return False
+    return bool(_abi.LIB.rlm_relation_layer_tail_wide_supported(int(n_seq), int(k_out), int(relation_dim),
+                                                                int(hidden_dim), int(d_model), int(n_query),
+                                                                _abi.DTYPE_CODE[dtype]))
+
+
+def relation_layer_tail_wide(expanded_cache: Tensor, operand_cache: Tensor, anchor_index: Tensor, partner_index: Tensor,
+                             partner_scores: Tensor, product_weight: Tensor, second_weight: Tensor, second_bias: Tensor,
+                             norm_weight: Tensor, norm_bias: Tensor, position: Tensor, norm_eps: float, hidden: Tensor,
+                             mix: Tensor, next_norm_weight: Tensor, next_norm_bias: Tensor, next_norm_eps: float,
+                             normalized: Tensor, query_weight: Tensor | None, query: Tensor | None) -> None:
+    """``relation_layer_tail`` for ``d`` 768 (extension): the second layer's weights are streamed."""
+    _relation_layer_tail_wide(expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight,
+                              second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, hidden, mix,
+                              next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query)
+
+
+@torch.library.register_fake("relation_lm::relation_layer_tail_wide")
 def _(expanded_cache, operand_cache, anchor_index, partner_index, partner_scores, product_weight,
       second_weight, second_bias, norm_weight, norm_bias, position, norm_eps, hidden, mix,
       next_norm_weight, next_norm_bias, next_norm_eps, normalized, query_weight, query):
