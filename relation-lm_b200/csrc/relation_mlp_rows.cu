@@ -15,7 +15,7 @@
 // round trip of 2 * pairs * H bytes each way: 1.07 GB written and read back for 262 144 pairs of
 // H = 2048, beside a GELU epilogue that nothing overlaps.  Kept on chip, the second layer needs an
 // fp32 accumulator of 128 pairs x d, all of an SM's tensor memory at d = 512; so a tile of 128 pairs
-// belongs to C = 2 CTAs of a cluster (C = 1 for d <= 384): each accumulates d / C output columns and
+// belongs to C = 2 CTAs of a cluster (C = 1 for d <= 384 and more than 33 pairs of tiles): each accumulates d / C output columns and
 // computes every C-th block of 64 hidden columns, which it passes on to the other through distributed
 // shared memory (one bulk copy per 32 rows, completing on the receiver's mbarrier).
 //
@@ -1003,13 +1003,14 @@ int log2_of(int v) {
     return s;
 }
 
+// `spread`: two output parts also where one would do.
 // Output columns per CTA (tensor memory: cols of the second layer + one or two units of the first) and the
 // first of a list of pipeline depths that fits the shared memory.  At d = 512, K = 8, where two fit, two gathered
 // blocks with three W_2 stages measured 745 us for 262 144 pairs, three with two 786 us.
-MlpShape mlp_shape(int rdim, int hdim, int d, int k_shift) {
+MlpShape mlp_shape(int rdim, int hdim, int d, int k_shift, bool spread = false) {
     static constexpr int kDepths[][3] = {{4, 4, 2}, {3, 4, 2}, {3, 3, 2}, {3, 3, 1}, {2, 4, 1}, {2, 3, 1}, {2, 2, 1}};
     MlpShape s{};
-    s.outs = d <= 384 ? 1 : 2;
+    s.outs = d <= 384 && !spread ? 1 : 2;
     s.cols = d / s.outs;
     if (d % s.outs != 0 || s.cols % 64 != 0 || s.cols > 384 || hdim % (2 * kMlpHC * s.outs) != 0 || hdim < 4 * kMlpHC * s.outs) return s;
     s.wide = s.cols <= 256;
@@ -1117,7 +1118,15 @@ extern "C" int rlm_relation_mlp_rows(
                           static_cast<const void*>(residual)})
         if (!aligned16(q)) { set_error("relation_mlp_rows: tensors must be 16-byte aligned"); return RLM_ERR_ALIGN; }
     const int k_shift = log2_of(k_out);
-    const MlpShape s = mlp_shape(relation_dim, hidden_dim, d_model, k_shift);
+    MlpShape s = mlp_shape(relation_dim, hidden_dim, d_model, k_shift);
+    // A launch that leaves more than half of the SMs idle divides its tiles' columns and hidden blocks over twice as many
+    // CTAs, up to the 33 clusters of four that run at a time (us, one part -> two: 2048 pairs of d 256 31.5 -> 25.2, 4096
+    // 31.7 -> 25.3, 8192 33.2 -> 27.4; beyond that a second wave would cost more).
+    const int supers = (static_cast<int>((static_cast<int64_t>(n_rows) * slots * k_out + kBM - 1) / kBM) + kG - 1) / kG;
+    if (s.outs == 1 && supers * 2 * kG <= sm_count() - 16) {
+        const MlpShape spread = mlp_shape(relation_dim, hidden_dim, d_model, k_shift, true);
+        if (spread.ok) s = spread;
+    }
     const int n_inst = s.cols > 256 ? 2 : 1;
     const uint32_t fmt = dtype == RLM_BF16 ? 1u : 0u;
     const auto idesc = [&](int n) {

@@ -85,6 +85,13 @@ def test_few_hidden_units_and_many_tiles(batch, slots, k, rdim, d, hidden):
     _check(torch.bfloat16, batch, 53, slots, k, rdim, d, hidden, False)
 
 
+# one output part or two for widths that fit in one: 33 pairs of tiles (the most that are spread) and 34, and a hidden
+# width that two parts cannot divide
+@pytest.mark.parametrize("length,d,hidden", [(1056, 256, 1024), (1057, 256, 1024), (1056, 128, 512), (40, 256, 256), (300, 384, 1536)])
+def test_tiles_over_one_or_two_parts(length, d, hidden):
+    _check(torch.bfloat16, 1, length, 1, 8, 128, d, hidden, True)
+
+
 def _check(dtype, batch, length, slots, k, rdim, d, hidden, limited):
     from relation_lm.kernels.relation_reduce import relation_mlp_rows, relation_mlp_rows_supported
 
