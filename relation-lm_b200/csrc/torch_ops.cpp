@@ -376,6 +376,9 @@ Two partner_topk(const Tensor& partner_query, const Tensor& partner_keys, const 
 #define ROUTER_ARGS                                                                                                      \
     ARG(anchor_raw_cache), ARG(partner_raw_cache), ARG(anchor_conv_cache), ARG(partner_conv_cache), ARG(anchor_mean),    \
         ARG(anchor_std), ARG(partner_mean), ARG(partner_std), ARG(anchor_conv_weight), ARG(partner_conv_weight)
+#define ROUTER_VALUES                                                                                                    \
+    anchor_raw_cache, partner_raw_cache, anchor_conv_cache, partner_conv_cache, anchor_mean, anchor_std, partner_mean,   \
+        partner_std, anchor_conv_weight, partner_conv_weight
 #define ROUTER_POINTERS                                                                                                  \
     ptr(anchor_raw_cache), ptr(partner_raw_cache), ptr(anchor_conv_cache), ptr(partner_conv_cache), ptr(anchor_mean),    \
         ptr(anchor_std), ptr(partner_mean), ptr(partner_std), ptr(anchor_conv_weight), ptr(partner_conv_weight)
@@ -1009,6 +1012,55 @@ Tensor skinny_projection_greedy_into(const Tensor& x, const Tensor& weight, cons
     return skinny_greedy(x, weight, bias, vocab, scratch, position, next_token, dense_rows({ARG(x)}));
 }
 
+// ------------------------------------------------------------------ the single-precision step in three calls
+//
+// A step without a captured graph is bound by the host: ten operator calls of 4-5 us each for one layer, whose kernels
+// take 42 us.  These are the same operators in the same order, a call for what comes before the layers, one per layer and
+// one for the heads; they exist as extension functions only, and where those decline the step makes its calls one by one.
+
+Tensor single_precision_front(const Tensor& tokens, const Tensor& boundaries, const Tensor& token_table, const Tensor& boundary_table,
+                              const Tensor& position_table, const Tensor& position, double scale, const Tensor& memory_norm_w,
+                              const Tensor& memory_norm_b, Tensor& memory_rows, const Tensor& input_norm_w,
+                              const Tensor& input_norm_b, Tensor& normalized, double norm_eps, Tensor& packed,
+                              const Tensor& packed_weight, Tensor& anchor_keys, Tensor& partner_keys, Tensor& operand_cache,
+                              Tensor& partner_anchor_cache, ROUTER_PARAMS, int64_t block_size) {
+    Tensor hidden = decode_embed_norm(tokens, boundaries, token_table, boundary_table, position_table, position, scale, memory_norm_w,
+                                      memory_norm_b, memory_rows, input_norm_w, input_norm_b, normalized, norm_eps);
+    few_rows_projection(packed, memory_rows, packed_weight, std::nullopt);
+    sparse_cache_append(packed, anchor_keys, partner_keys, operand_cache, partner_anchor_cache, ROUTER_VALUES, position, block_size);
+    return hidden;
+}
+
+Two single_precision_layer(const Tensor& normalized, const Tensor& query_weight, Tensor& query, SELECT_PARAMS, const Tensor& position,
+                           int64_t local_window, int64_t top_blocks, int64_t k_out, bool strict_valid, Tensor& relation_hidden,
+                           Tensor& expanded_cache, const Tensor& operand_cache, const Tensor& anchor_weight,
+                           const Tensor& partner_weight, const Tensor& product_weight, const Tensor& first_bias,
+                           Tensor& second_rows, const Tensor& second_weight, const Tensor& second_bias, const Tensor& norm_weight,
+                           const Tensor& norm_bias, double norm_eps, Tensor& hidden, const Tensor& mix,
+                           const Tensor& next_norm_weight, const Tensor& next_norm_bias, Tensor& next_normalized) {
+    few_rows_projection(query, normalized, query_weight, std::nullopt);
+    auto [anchor, anchor_score, partner, score] =
+        select(SELECT_TENSORS, &position, nullptr, nullptr, local_window, top_blocks, k_out, strict_valid);
+    relation_hidden_cache_update_out(relation_hidden, expanded_cache, operand_cache, anchor, partner, anchor_weight, partner_weight,
+                                     product_weight, first_bias, position);
+    Tensor rows = second_rows.view({-1, second_weight.size(0)});
+    few_rows_projection(rows, relation_hidden.view({-1, second_weight.size(1)}), second_weight, second_bias);
+    relation_norm_reduce_residual_norm(second_rows, score, norm_weight, norm_bias, position, norm_eps, hidden, mix, next_norm_weight,
+                                       next_norm_bias, norm_eps, next_normalized);
+    return {anchor, partner};
+}
+
+Two single_precision_heads(const Tensor& normalized, const Tensor& token_weight, const Tensor& boundary_weight, const Tensor& boundary_bias,
+                           Tensor& position) {
+    const c10::Device device = dense_rows({ARG(normalized)});
+    Tensor tokens = empty({normalized.size(0), token_weight.size(0)}, at::kFloat, device);
+    Tensor boundaries = empty({normalized.size(0), boundary_weight.size(0)}, at::kFloat, device);
+    few_rows_projection_pair(tokens, boundaries, normalized, token_weight, boundary_weight, boundary_bias);
+    at::AutoDispatchBelowADInplaceOrView below;          // (the version counter is advanced by the caller)
+    position.add_(1);
+    return {tokens, boundaries};
+}
+
 // ------------------------------------------------------------------ what surrounds an operator
 
 using Stack = torch::jit::Stack;
@@ -1359,7 +1411,8 @@ PyMethodDef kMethods[] = {METHOD(relation_select_packed), METHOD(relation_select
                           METHOD(relation_hidden_cache_update), METHOD(relation_hidden_cache_update_out),
                           METHOD(relation_norm_reduce), METHOD(relation_norm_reduce_residual_norm), METHOD(relation_mlp_rows),
                           METHOD(packed_projection), METHOD(layer_norm_cast), METHOD(decode_embed_norm), METHOD(few_rows_projection),
-                          METHOD(few_rows_projection_pair),
+                          METHOD(few_rows_projection_pair), METHOD(single_precision_front), METHOD(single_precision_layer),
+                          METHOD(single_precision_heads),
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "librelation_lm_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

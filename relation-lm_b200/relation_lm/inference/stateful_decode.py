@@ -182,6 +182,18 @@ class StatefulDecoder:
             self.head_bias[cfg.vocab_size:cfg.vocab_size + cfg.boundary_vocab_size] = self.w["boundary_b"].float()
 
         self._layers = [self._layer_views(l) for l in range(L)]
+        if not self.fused and self.few_rows:
+            # what the grouped calls of the single-precision step take before and behind the position
+            w = self.w
+            self._front = ((w["token_embedding"], w["boundary_embedding"], w["position_embedding"]),
+                           (self.input_scale, w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized, w["input_norm_w"][0],
+                            w["input_norm_b"][0], self.normalized, cfg.norm_eps, self.packed_rows, w["w_packed"], self.anchor_keys,
+                            self.partner_keys, self.operand_cache, self.partner_anchor_cache, *self.router_caches,
+                            *self.router_stats, w["anchor_conv_weight"], w["partner_conv_weight"], cfg.block_size))
+            for layer in self._layers:
+                layer.grouped = ((layer.w_query, layer.query, *layer.selection),
+                                 (cfg.local_window, cfg.top_blocks, cfg.k_max, cfg.strict_valid, self.relation_hidden, *layer.caches,
+                                  *layer.first_layer, self.second_rows, *layer.second_layer, *layer.relation_norm, cfg.norm_eps))
 
     # ------------------------------------------------------------------ state
     def reset(self) -> None:
@@ -261,28 +273,22 @@ class StatefulDecoder:
         pos, K = self.position, cfg.k_max
         if self.kernel_norms:
             tokens, boundaries = self._ids(tokens, boundaries)
-            hidden = decode_embed_norm(tokens, boundaries, w["token_embedding"], w["boundary_embedding"],
-                                       w["position_embedding"], pos, self.input_scale,
-                                       w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized,
-                                       w["input_norm_w"][0], w["input_norm_b"][0], self.normalized, cfg.norm_eps)
-        else:
-            x = (F.embedding(tokens, w["token_embedding"]) + F.embedding(boundaries, w["boundary_embedding"])).float()
-            hidden = x * self.input_scale + w["position_embedding"].index_select(0, pos.view(1))
-            self._normalize(hidden, w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized)
-            self._normalize(hidden, w["input_norm_w"][0], w["input_norm_b"][0], self.normalized)
-        if self.few_rows:
-            packed = self.packed_rows                                 # [B, layers * 512]
-            few_rows_projection(packed, self.memory_normalized, w["w_packed"], None)
-        else:
-            packed = F.linear(self.memory_normalized, w["w_packed"])
-        sparse_cache_append(packed, self.anchor_keys, self.partner_keys, self.operand_cache,
-                            self.partner_anchor_cache, *self.router_caches, *self.router_stats,
-                            w["anchor_conv_weight"], w["partner_conv_weight"], pos, cfg.block_size)
+        # ... and its operators are called from native code, a call for a whole group of them, where nobody wants the
+        # selections in between.
+        grouped = self.few_rows and not keep_selection
+        hidden = NotImplemented
+        if grouped:
+            hidden = _abi.direct_call("single_precision_front", tokens, boundaries, *self._front[0], pos, *self._front[1])
+        if hidden is NotImplemented:
+            hidden = self._front_unfused(tokens, boundaries)
         if keep_selection:
             self.last_selection = []
         for layer in self._layers:
             # the last layer's goes to a tensor of this step's own: it stays behind as `last_final`
             normalized = torch.empty_like(self.normalized) if layer is self._layers[-1] else self.normalized
+            if grouped and _abi.direct_call("single_precision_layer", self.normalized, *layer.grouped[0], pos, *layer.grouped[1],
+                                            hidden, layer.mix, *layer.next_norm, normalized) is not NotImplemented:
+                continue
             if self.few_rows:
                 few_rows_projection(layer.query, self.normalized, layer.w_query, None)        # [B, 256]
             else:
@@ -305,6 +311,10 @@ class StatefulDecoder:
             if keep_selection:
                 self.last_selection.append((anchor, partner))
         self.last_final = normalized
+        if grouped:
+            heads = _abi.direct_call("single_precision_heads", normalized, w["token_embedding"], w["boundary_w"], w["boundary_b"], pos)
+            if heads is not NotImplemented:
+                return heads
         if self.few_rows:
             heads = normalized.new_empty(self.batch, cfg.vocab_size), normalized.new_empty(self.batch, cfg.boundary_vocab_size)
             few_rows_projection_pair(*heads, normalized, w["token_embedding"], w["boundary_w"], w["boundary_b"])
@@ -315,6 +325,29 @@ class StatefulDecoder:
             heads = F.linear(normalized, w["token_embedding"]), F.linear(normalized, w["boundary_w"], w["boundary_b"])
         pos.add_(1)
         return heads
+
+    def _front_unfused(self, tokens: Tensor, boundaries: Tensor) -> Tensor:
+        """The embedded rows; their LayerNorms, packed projection and cache rows of the position on the way."""
+        cfg, w, pos = self.config, self.w, self.position
+        if self.kernel_norms:
+            hidden = decode_embed_norm(tokens, boundaries, w["token_embedding"], w["boundary_embedding"],
+                                       w["position_embedding"], pos, self.input_scale,
+                                       w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized,
+                                       w["input_norm_w"][0], w["input_norm_b"][0], self.normalized, cfg.norm_eps)
+        else:
+            x = (F.embedding(tokens, w["token_embedding"]) + F.embedding(boundaries, w["boundary_embedding"])).float()
+            hidden = x * self.input_scale + w["position_embedding"].index_select(0, pos.view(1))
+            self._normalize(hidden, w["memory_norm_w"], w["memory_norm_b"], self.memory_normalized)
+            self._normalize(hidden, w["input_norm_w"][0], w["input_norm_b"][0], self.normalized)
+        if self.few_rows:
+            packed = self.packed_rows                                 # [B, layers * 512]
+            few_rows_projection(packed, self.memory_normalized, w["w_packed"], None)
+        else:
+            packed = F.linear(self.memory_normalized, w["w_packed"])
+        sparse_cache_append(packed, self.anchor_keys, self.partner_keys, self.operand_cache,
+                            self.partner_anchor_cache, *self.router_caches, *self.router_stats,
+                            w["anchor_conv_weight"], w["partner_conv_weight"], pos, cfg.block_size)
+        return hidden
 
     @staticmethod
     def _ids(tokens: Tensor, boundaries: Tensor) -> tuple[Tensor, Tensor]:

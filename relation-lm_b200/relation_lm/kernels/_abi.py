@@ -109,6 +109,13 @@ def operator(name: str):
 
     return call
 
+
+def direct_call(name: str, *args):
+    """An extension function that stands for several operators; ``NotImplemented`` where they have to be called one by
+    one (anything but plain CUDA tensors, a derivative, mode, tracer or transform)."""
+    return NotImplemented if torch.compiler.is_compiling() else getattr(_DIRECT, name)(*args)
+
+
 _STATUS: dict[int, torch.Tensor] = {}
 
 

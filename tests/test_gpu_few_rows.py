@@ -52,3 +52,32 @@ def test_refuses_what_it_does_not_take():
                 (torch.empty(65, 8, device="cuda"), torch.randn(65, 16, device="cuda"), w)):
         with pytest.raises(ValueError):
             few_rows_projection(*bad)
+
+
+@pytest.mark.parametrize("batch,layers,strided", [(1, 1, False), (3, 3, True), (8, 2, False)])
+def test_grouped_calls_are_the_single_ones(batch, layers, strided):
+    """The single-precision step with its operators called in groups and one by one (as it does to keep the selections):
+    logits, state, position and version counters alike."""
+    from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+    from relation_lm.inference.stateful_decode import StatefulDecoder
+
+    cfg = RoutedRelationConfig(vocab_size=301, boundary_vocab_size=9, d_model=256, layers=layers, max_context=64, block_size=8,
+                               local_window=16, top_blocks=2)
+    model = RoutedRelationLM(cfg, seed=5)
+    one, two = StatefulDecoder(model, batch, "cuda", torch.float32), StatefulDecoder(model, batch, "cuda", torch.float32)
+    ids = torch.arange(40, device="cuda").view(20, 2)[:, 0] % 9
+    for t in range(20):
+        tokens, bounds = (ids[t] + torch.arange(batch, device="cuda") * 7) % 301, ids[t].expand(batch)
+        if strided:
+            tokens = torch.stack((tokens, tokens), 1)[:, 0]
+        before = [x.position._version for x in (one, two)]
+        a, b = one.step(tokens, bounds), two.step(tokens, bounds, keep_selection=True)
+        assert all(torch.equal(x, y) and x.is_contiguous() for x, y in zip(a, b))
+        assert [x.position._version for x in (one, two)] == [v + 1 for v in before]
+    for name in ("anchor_keys", "partner_keys", "operand_cache", "partner_anchor_cache", "expanded_cache", "position", "last_final"):
+        assert torch.equal(getattr(one, name), getattr(two, name)), name
+        if name != "last_final":
+            assert getattr(one, name)._version == getattr(two, name)._version, name
+    for x, y in zip(one.router_caches + one.router_stats, two.router_caches + two.router_stats):
+        assert torch.equal(x, y)
+    assert_status_clear()
