@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kThreads) router_cache_prefill_kernel(const Pr
 // 16-byte pieces; the convolution runs on a tile in shared memory, a thread per eight channels, and only the
 // statistics, whose sums are ordered by position, walk the block's rows, a thread per channel.  (As four
 // strided copies, eight fills and a kernel that walked the rows in global memory: 91 us for 8 sequences of
-// 4096 positions; per anchor slot 30 us more for each.)
+// 4096 positions; per anchor slot 30 us more for each.)  Loads go in rounds, each before the round's stores (16 x 2048
+// positions, 4 slots: 74 -> 63 us for 252 MB; 8 x 4096 without slots 15.9 -> 14.3).
 constexpr int kSeqThreads = 256;
 
 struct SequenceArgs {
@@ -250,7 +251,7 @@ struct SequenceArgs {
 };
 
 template <int kDt>
-__global__ void __launch_bounds__(kSeqThreads) sequence_state_kernel(const SequenceArgs a) {
+__global__ void __launch_bounds__(kSeqThreads, 4) sequence_state_kernel(const SequenceArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float last[kThreads];                            // the block's last row before rounding
     const int tid = threadIdx.x, blk = blockIdx.x, b = blockIdx.y, slot = blockIdx.z, bs = a.block_size, start = blk * bs;
@@ -258,37 +259,68 @@ __global__ void __launch_bounds__(kSeqThreads) sequence_state_kernel(const Seque
     uint16_t* conv_s = raw_s + (bs + 2) * kThreads;             // [bs][128]
     // this thread's eight channels of the convolution
     const int chunk = tid & 15, stream = chunk >> 3, ch = 8 * (chunk & 7);
+    griddep_sync();
+    const int64_t seq = static_cast<int64_t>(slot) * a.batch + b;
+    const uint16_t* rows = a.packed + (static_cast<int64_t>(b) * a.max_t + start) * a.row_stride + slot * a.slot_stride;
+    // Every load of a round is issued before its first store: the stores may alias the loads as far as the compiler knows,
+    // and a load behind each of six columns' stores made a block six DRAM round trips long.
+    constexpr int kRouterAhead = 3, kCopyAhead = 4;
+    const auto copy_at = [&](int i) { return rows + (i >> 5) * a.row_stride + ((i & 31) < 16 ? a.key_at[(i >> 3) & 1] + 8 * (i & 7) : a.partner_anchor_at + 8 * (i & 15)); };
+    for (int r0 = 0, c0 = 0; r0 < (bs + 2) * 16 || c0 < bs * 32; r0 += kRouterAhead * kSeqThreads, c0 += kCopyAhead * kSeqThreads) {
+        uint4 router[kRouterAhead], copied[kCopyAhead];
+#pragma unroll
+        for (int j = 0; j < kRouterAhead; ++j) {
+            const int i = r0 + tid + j * kSeqThreads, r = (i >> 4) - 2;
+            router[j] = make_uint4(0, 0, 0, 0);
+            if (i < (bs + 2) * 16 && start + r >= 0) router[j] = *reinterpret_cast<const uint4*>(rows + r * a.row_stride + a.router_at[stream] + ch);
+        }
+#pragma unroll
+        for (int j = 0; j < kCopyAhead; ++j) {
+            const int i = c0 + tid + j * kSeqThreads;
+            if (i < bs * 32) copied[j] = *reinterpret_cast<const uint4*>(copy_at(i));
+        }
+        // router keys into shared memory and the raw caches
+#pragma unroll
+        for (int j = 0; j < kRouterAhead; ++j) {
+            const int i = r0 + tid + j * kSeqThreads, r = (i >> 4) - 2;
+            if (i >= (bs + 2) * 16) break;
+            *reinterpret_cast<uint4*>(raw_s + (r + 2) * kThreads + 8 * chunk) = router[j];
+            if (r >= 0) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.raw[stream]) + (seq * a.max_t + start + r) * kD + ch) = router[j];
+        }
+        // token features: the two keys' eight chunks of a row each, the partner-anchor row's sixteen
+#pragma unroll
+        for (int j = 0; j < kCopyAhead; ++j) {
+            const int i = c0 + tid + j * kSeqThreads;
+            if (i >= bs * 32) break;
+            const int64_t row = seq * a.max_t + start + (i >> 5);
+            uint16_t* to = (i & 31) < 16 ? static_cast<uint16_t*>(a.key[(i >> 3) & 1]) + row * kD + 8 * (i & 7)
+                                         : static_cast<uint16_t*>(a.partner_anchor) + row * 128 + 8 * (i & 15);
+            *reinterpret_cast<uint4*>(to) = copied[j];
+        }
+    }
+    if (slot == 0) {
+        const int chunks = a.rdim / 8, n = bs * chunks;
+        const int64_t row0 = static_cast<int64_t>(b) * a.max_t + start;
+        for (int c0 = 0; c0 < n; c0 += 4 * kSeqThreads) {
+            uint4 copied[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = c0 + tid + j * kSeqThreads, r = i / chunks;
+                if (i < n) copied[j] = *reinterpret_cast<const uint4*>(rows + r * a.row_stride + a.operand_at + 8 * (i - r * chunks));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = c0 + tid + j * kSeqThreads;
+                if (i < n) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.operand) + row0 * a.rdim + 8 * i) = copied[j];
+            }
+        }
+    }
     float w[3][8];
 #pragma unroll
     for (int e = 0; e < 8; ++e)
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             w[k][e] = load_scalar(a.weight[stream], (static_cast<int64_t>(slot) * kD + ch + e) * 3 + k, a.weight_dtype);
-    griddep_sync();
-    const int64_t seq = static_cast<int64_t>(slot) * a.batch + b;
-    const uint16_t* rows = a.packed + (static_cast<int64_t>(b) * a.max_t + start) * a.row_stride + slot * a.slot_stride;
-    // router keys into shared memory and the raw caches
-    for (int i = tid; i < (bs + 2) * 16; i += kSeqThreads) {
-        const int r = (i >> 4) - 2;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (start + r >= 0) v = *reinterpret_cast<const uint4*>(rows + r * a.row_stride + a.router_at[stream] + ch);
-        *reinterpret_cast<uint4*>(raw_s + (r + 2) * kThreads + 8 * chunk) = v;
-        if (r >= 0) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(a.raw[stream]) + (seq * a.max_t + start + r) * kD + ch) = v;
-    }
-    // token features
-    const auto copy = [&](int at, int width, void* to, int64_t row0) {
-        const int chunks = width / 8;
-#pragma unroll 4
-        for (int i = tid; i < bs * chunks; i += kSeqThreads) {
-            const int r = i / chunks, c = i - r * chunks;
-            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(to) + (row0 + r) * width + 8 * c) =
-                *reinterpret_cast<const uint4*>(rows + r * a.row_stride + at + 8 * c);
-        }
-    };
-    copy(a.key_at[0], kD, a.key[0], seq * a.max_t + start);
-    copy(a.key_at[1], kD, a.key[1], seq * a.max_t + start);
-    copy(a.partner_anchor_at, 128, a.partner_anchor, seq * a.max_t + start);
-    if (slot == 0) copy(a.operand_at, a.rdim, a.operand, static_cast<int64_t>(b) * a.max_t + start);
     __syncthreads();
     for (int r = tid >> 4; r < bs; r += kSeqThreads / 16) {
         const int p = start + r;
