@@ -429,9 +429,11 @@ class StatefulDecoder:
             sparse_cache_append(packed, self.anchor_keys, self.partner_keys, self.operand_cache,
                                 self.partner_anchor_cache, *self.router_caches, *self.router_stats,
                                 w["anchor_conv_weight"], w["partner_conv_weight"], pos, cfg.block_size)
-        if self.stacked_expand and self.fused_front:
+        if self.stacked_expand and not self.append_in_projection and (self.fused_front or cfg.d_model <= 512):
             # every layer's operand row of this position is known: expand them all at once, straight from
-            # the packed rows (written two launches back), so that this launch overlaps the append
+            # the packed rows (written two launches back), so that this launch overlaps the append (us a step,
+            # from the operand cache -> from the packed rows: 24 sequences of d 256, 4 layers 89.0 -> 86.1, 32 of d 512,
+            # 6 layers 159.7 -> 158.0; of d 768, 12 layers, where the two compete for memory, 8 256.1 -> 257.3, 28 386.1 -> 388.9)
             expanded_cache_append_packed(self.expanded_cache, packed, w["anchor_weight"], w["partner_weight"],
                                          w["first_bias"], pos)
         elif self.stacked_expand:
