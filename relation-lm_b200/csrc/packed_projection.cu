@@ -253,7 +253,6 @@ struct PersistentGemmArgs {
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
                  ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -394,7 +393,9 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
                     tmem_ld16(acc + c, *reinterpret_cast<uint32_t(*)[16]>(&v[0]));
                     tmem_ld16(acc + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&v[16]));
                     const uint32_t buffer = kBuffers == 2 ? static_cast<uint32_t>(c >> 6) * kPgBox : 0u;
-                    if (a.staged && (c & 32) == 0) {             // the buffer's previous store has read it
+                    if (a.staged && (c & 32) == 0) {
+                        // the buffer's previous store has read it: every box commits one group, so the newest kBuffers - 1
+                        // groups are those of the other buffer and may stay
                         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kBuffers - 1) : "memory");
                         __syncwarp();
                     }
@@ -437,7 +438,12 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
                     if (c & 32) {
                         fence_proxy_async();
                         __syncwarp();
-                        if (lane == 0 && first_row < a.m && n0 + c - 32 < a.n) tma_store_2d(&map_out, box + buffer, n0 + c - 32, first_row);
+                        if (lane == 0) {
+                            // a box beyond the last row or column is not stored and commits an empty group: the wait above
+                            // counts one group a box
+                            if (first_row < a.m && n0 + c - 32 < a.n) tma_store_2d(&map_out, box + buffer, n0 + c - 32, first_row);
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
                     }
                 }
             }

@@ -350,3 +350,33 @@ def test_persistent_projection_at_ragged_edges(rows, d_in, n_out, dtype, bias):
     assert_rel_close(room[:rows * n_out].view(rows, n_out), want, 1e-2)
     assert bool((room[rows * n_out:] == 7.0).all())
     assert_status_clear()
+
+
+@pytest.mark.parametrize("rows,d_in,n_out,bias", [
+    (24065, 128, 448, True),       # second half of the last column tile: one box of two
+    (24065, 128, 448, False),
+    (40000, 64, 160, True),        # 32 columns in the second half
+    (40000, 192, 192, False),
+    (50001, 128, 320, True),       # second half of the last column tile: none of two
+    (40000, 512, 160, True),
+    (38016, 64, 256, True),        # whole columns; rows end before the last tile's last two warps
+    (38020, 128, 512, False),
+])
+def test_persistent_projection_leaves_each_box_to_its_store(rows, d_in, n_out, bias):
+    """Two output boxes a warp and boxes that are not stored, in CTAs of several tiles: a box is rewritten only behind its
+    store, so that the rows are, bit for bit and every time, those of the product with as many rows and columns as whole
+    tiles have (each box stored there).  One K-block or a few: the next tile is at the box soon after the store."""
+    from relation_lm.kernels.packed_projection import packed_projection
+
+    g = torch.Generator().manual_seed(rows + n_out)
+    full_rows, full_out = (rows + 127) // 128 * 128, (n_out + 255) // 256 * 256
+    x = torch.randn(full_rows, d_in, generator=g).bfloat16().cuda()
+    w = torch.randn(full_out, d_in, generator=g).bfloat16().cuda()
+    b = torch.randn(full_out, generator=g).cuda() if bias else None
+    want = packed_projection(x, w, b)[:rows, :n_out]
+    sample = torch.randperm(rows, generator=g)[:512].cuda()
+    full = x[sample].float() @ w[:n_out].float().T + (b[:n_out] if bias else 0.0)
+    assert_rel_close(want[sample], full, 1e-2)
+    for _ in range(20):
+        assert torch.equal(packed_projection(x[:rows], w[:n_out], b[:n_out] if bias else None), want)
+    assert_status_clear()
