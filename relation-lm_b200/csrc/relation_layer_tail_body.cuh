@@ -557,7 +557,8 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 for (int j = 0; j < 8; j += 2) {
                     if (j >= 4 && c + step >= pairs) break;
                     const int pr = c + (j & 3) + (j & 4 ? step : 0);
-                    const float2 h = gelu_pair(make_float2(__uint_as_float(v[j]) + term[j], __uint_as_float(v[j + 1]) + term[j + 1]));
+                    // (the two are different pairs, perhaps of different sequences: a reciprocal each)
+                    const float2 h = gelu_tc2(make_float2(__uint_as_float(v[j]) + term[j], __uint_as_float(v[j + 1]) + term[j + 1]));
                     store(pr, h.x);
                     store(pr + 1, h.y);
                 }

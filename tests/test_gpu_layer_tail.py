@@ -207,3 +207,34 @@ def test_whole_layer_rejects_a_selector_that_does_not_fit():
     # the tail's tile memory is about 50 KB: 64 blocks of statistics + a 128-row window + 4 blocks of 64 keys need more
     assert not relation_layer_supported(4, 8, 128, 512, 128, 0, torch.bfloat16, 4096, 64, 8, 128, 4)
     assert not relation_layer_supported(4, 8, 128, 3072, 768, 0, torch.bfloat16, 128, 8, 8, 16, 1)   # d 768
+
+
+# 10 and 14 pairs in two sequences a cluster, 21 in three, 24 of which each sequence's slots are a whole number of twos, and
+# the form for d 768 below and above 16 pairs
+@pytest.mark.parametrize("dtype,value", [(torch.bfloat16, torch.inf), (torch.float16, torch.nan), (torch.bfloat16, -torch.inf)])
+@pytest.mark.parametrize("B,K,d", [(8, 5, 512), (7, 7, 256), (12, 7, 512), (12, 8, 256), (12, 7, 128), (8, 5, 768), (12, 7, 768)])
+def test_a_cache_row_that_is_not_finite_stays_with_its_sequence_and_slot(B, K, d, dtype, value):
+    """A value that is not finite in a row that a sequence selected makes that sequence's results NaN and leaves every
+    other's bits alone; in the row of an empty slot it changes nothing."""
+    from test_gpu_layer_tail_wide import _run as run_wide
+
+    run = run_wide if d == 768 else _run
+    T, t, H = 40, 39, 4 * d
+    x = _case(B, K, d, 128, T, 256, dtype, 400 + B + d)
+    g = torch.Generator().manual_seed(B)
+    rows = torch.stack([torch.randperm(T, generator=g) for _ in range(B)])
+    x["partner"], x["anchor"] = rows[:, :K].int().contiguous(), rows[:, K].int().contiguous()
+    x["scores"] = torch.randn(B, K, generator=g)
+    x["scores"][2:, K // 2] = -torch.inf
+    before = run(x, t, dtype)
+    for seq in (0, B // 2, B - 1):
+        for slot in range(min(K, 5)):                              # the first five take part at this position
+            for column in (0, H // 2 + 7, H - 1):
+                poisoned = dict(x, expanded=x["expanded"].clone())
+                poisoned["expanded"][seq, x["partner"][seq, slot], H + column] = value
+                after = run(poisoned, t, dtype)
+                hit = (torch.arange(B) == seq) & bool(x["scores"][seq, slot] > -torch.inf)
+                for got, want in zip(after, before):
+                    assert torch.equal(got[~hit], want[~hit]), (seq, slot, column)
+                    assert bool(got[hit].isnan().all()), (seq, slot, column)
+    assert_status_clear()
