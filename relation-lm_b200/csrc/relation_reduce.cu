@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kHiddenThreads) relation_hidden_kernel(const H
         t = static_cast<int>(*a.position);
         if (t < 0 || t >= a.max_t) {
             if (tid == 0 && a.status) atomicOr(a.status, RLM_DEV_POSITION);
+            griddep_sync();      // here too: what is launched next relies on this kernel having waited for its predecessor
             return;
         }
     }

@@ -48,3 +48,31 @@ def test_ids_as_an_embedding_takes_them(batch):
     with pytest.raises(ValueError):
         dec.step(tokens.view(batch, 1), tokens.view(batch, 1))
     assert_status_clear()
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+@pytest.mark.parametrize("keep_selection", [False, True])
+def test_a_step_past_the_context_is_reported_and_changes_no_state(batch, keep_selection):
+    """Every kernel of that step still waits for its predecessor, so that the steps around it are what they are without
+    programmatic launch."""
+    from relation_lm.kernels import _abi
+
+    results = []
+    for early in (False, True):
+        dec = _decoder(batch)
+        dec.programmatic_launch = early
+        tokens, bounds = (torch.randint(0, n, (40, batch), generator=torch.Generator().manual_seed(n)).cuda() for n in (50, 6))
+        for t in range(32):
+            dec.step(tokens[t], bounds[t], keep_selection)
+        assert_status_clear()
+        names = ("anchor_keys", "partner_keys", "operand_cache", "partner_anchor_cache", "expanded_cache")
+        state = [getattr(dec, n).clone() for n in names] + [s.clone() for s in dec.router_caches + dec.router_stats]
+        dec.step(tokens[32], bounds[32], keep_selection)
+        assert _abi.read_status() != 0
+        now = [getattr(dec, n) for n in names] + dec.router_caches + dec.router_stats
+        assert all(torch.equal(a, b) for a, b in zip(state, now))
+        dec.slide(1)
+        dec.position.fill_(24)
+        results.append([r.clone() for t in range(33, 40) for r in dec.step(tokens[t], bounds[t], keep_selection)])
+        assert_status_clear()
+    assert all(torch.equal(a, b) for a, b in zip(*results))
