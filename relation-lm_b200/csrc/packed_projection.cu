@@ -459,6 +459,31 @@ __global__ void __launch_bounds__(kPgThreads, 1) packed_projection_persistent_ke
                      ::"r"(tmem_base), "r"(2 * kPgBN) : "memory");
 }
 
+// Whether 16-bit results of at least 128 rows are faster on persistent CTAs, whose tiles are 128 x 256, than from the kernel
+// above, whose tiles are 128, 64 or 32 wide (the widest that divides n).  us, the other kernel -> persistent; 148 SMs:
+// * fewer than 5 tiles for 8 SMs: no (9001 x 512 x 256, 71 tiles, 6.8 -> 7.5; 5952 x 768 x 512, 94 tiles, 9.4 -> 8.9);
+// * up to 64 columns most of a tile is empty (32768 x 512 x 64 12.7 -> 16.4, x 32 11.4 -> 17.3); only streams of short rows gain
+//   (131072 x 128 x 64, 1024 tiles: 1.45 x);
+// * where n is no odd multiple of 128, tiles fill or the other kernel's are narrow: yes (32768 x 512 x 160 2.7 x, x 96 1.45 x);
+// * an odd multiple leaves half a tile of columns empty beside 128-wide tiles that fit.  One column tile: the other kernel
+//   from its hundredth tile on (below, it halves them: 12032 x 128 x 128 1.3 x; 19067 x 512 x 128 9.7 -> 11.3), until three
+//   rounds of short rows (57 000 x 128 x 128 1.1 x).  More: the other kernel while it needs one CTA a SM (6016 x 512 x 384
+//   0.87 x), or one wave of two where these need a second round (9723 x 512 x 384, 152 tiles, 8.5 -> 10.6; 12 800 x 512 x
+//   384, 200 tiles, 1.19 x), or two waves against a third round of long rows (19195 x 1024 x 384 22.3 -> 23.3).  With a
+//   bias, which the other kernel reads as scalars, short rows gain all the same (9723 x 256 x 640 1.01 x, 6016 x 512 x 384 1.09 x).
+bool persistent_pays(int m_tiles, int n_out, int d_in, bool bias) {
+    const int sms = sm_count();
+    const int64_t tiles = static_cast<int64_t>(m_tiles) * ((n_out + kPgBN - 1) / kPgBN), narrow = static_cast<int64_t>(m_tiles) * (n_out / 128);
+    if (8 * tiles < 5 * sms) return false;
+    if (n_out <= 64) return n_out == 64 && d_in <= 128 && tiles >= 3 * sms;
+    if (n_out % 256 != 128) return true;
+    if (n_out == 128)
+        return tiles < 100 || (tiles <= sms && bias && d_in <= 128) || (tiles >= 3 * sms && (d_in <= 128 || (bias && d_in <= 512)));
+    if (narrow <= sms) return bias && d_in <= 512;
+    if (tiles > sms && narrow <= 2 * sms) return bias && d_in <= 256;
+    return !(tiles > 2 * sms && narrow <= 4 * sms) || bias || d_in <= 512;
+}
+
 template <int kRowTiles, int kStages>
 int launch_persistent_gemm(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, PersistentGemmArgs& a, void* stream) {
     const int smem_bytes = kStages * (kRowTiles * kBM * kBK * 2 + kPgBN * kBK * 2) + 8 * pg_buffers(kRowTiles, kStages) * static_cast<int>(kPgBox) + 1024;
@@ -935,12 +960,11 @@ extern "C" int rlm_packed_projection(const void* x, int64_t x_row_stride, const 
         return RLM_ERR_SHAPE;
     }
     const int m_tiles = (rows + kBM - 1) / kBM;
-    // Persistent CTAs from 5 tiles of 128 x 256 for 8 SMs on (us by the other kernel -> here: 3168 x 256 x 896, 100 tiles,
-    // 6.6 -> 6.2; 5952 x 768 x 512, 94 tiles, 9.4 -> 8.9; 3168 x 128 x 2048, 200 tiles, 12.5 -> 7.9; 9001 x 512 x 256,
-    // 71 tiles, 6.8 -> 7.5).  fp32 results are stored by the threads: at least two tiles per SM, whole tiles of columns.
     const int wide_tiles = (n_out + kPgBN - 1) / kPgBN, big_tiles = m_tiles * wide_tiles;
     const bool staged = out_dtype != RLM_F32;
-    if (k_splits == 1 && d_in % kBK == 0 && (staged ? rows >= kBM && 8 * big_tiles >= 5 * sm_count() : n_out % kPgBN == 0 && big_tiles >= 2 * sm_count())) {
+    // fp32 results are stored by the threads: at least two tiles per SM, whole tiles of columns
+    if (k_splits == 1 && d_in % kBK == 0 &&
+        (staged ? rows >= kBM && persistent_pays(m_tiles, n_out, d_in, bias != nullptr) : n_out % kPgBN == 0 && big_tiles >= 2 * sm_count())) {
         // 256 x 256 tiles when there are two of those per SM
         // (a 256-row tile's epilogue is not hidden behind the next main loop: it pays only with a long reduction)
         const bool tall = d_in >= 1024 && n_out % kPgBN == 0 && ((rows + 2 * kBM - 1) / (2 * kBM)) * (n_out / kPgBN) >= 2 * sm_count();

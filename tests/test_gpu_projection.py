@@ -380,3 +380,25 @@ def test_persistent_projection_leaves_each_box_to_its_store(rows, d_in, n_out, b
     for _ in range(20):
         assert torch.equal(packed_projection(x[:rows], w[:n_out], b[:n_out] if bias else None), want)
     assert_status_clear()
+
+
+@pytest.mark.parametrize("rows,d_in,n_out,bias", [
+    (32768, 512, 32, True), (57000, 128, 64, False), (32768, 512, 64, False),      # narrow results
+    (12670, 128, 128, False), (12801, 128, 128, False), (12801, 128, 128, True), (57000, 64, 128, False),
+    (6016, 128, 384, False), (6016, 128, 384, True), (6400, 64, 384, False),       # 141 and 150 tiles of 128 columns
+    (9723, 512, 384, False), (9723, 256, 384, True), (12800, 64, 384, False), (5999, 128, 1664, True),
+    (19195, 576, 384, False), (19195, 576, 384, True),
+])
+def test_many_rows_of_narrow_and_odd_widths(rows, d_in, n_out, bias):
+    """Widths and tile counts on either side of where the persistent kernel takes over: each element within 1e-2 of its
+    row's largest magnitude of torch's fp32 product."""
+    from relation_lm.kernels.packed_projection import packed_projection
+
+    g = torch.Generator().manual_seed(rows + n_out)
+    x = torch.randn(rows, d_in, generator=g).bfloat16().cuda()
+    w = torch.randn(n_out, d_in, generator=g).bfloat16().cuda()
+    b = torch.randn(n_out, generator=g).cuda() if bias else None
+    got = packed_projection(x, w, b)
+    assert_rel_close(got, x.float() @ w.float().T + (b if bias else 0.0), 1e-2)
+    assert torch.equal(packed_projection(x, w, b), got)
+    assert_status_clear()
