@@ -240,7 +240,9 @@ class StatefulDecoder:
                 return self._step_fused(tokens, boundaries, keep_selection)
             finally:
                 _abi.set_programmatic_launch(previous)
-        previous = _abi.set_programmatic_launch(self.programmatic_launch and self.few_rows)
+        if not self.few_rows or torch.compiler.is_compiling():      # (a tracer cannot follow the switch)
+            return self._step_unfused(tokens, boundaries, keep_selection)
+        previous = _abi.set_programmatic_launch(self.programmatic_launch)
         try:
             return self._step_unfused(tokens, boundaries, keep_selection)
         finally:

@@ -108,3 +108,25 @@ def test_relation_select_packed_fullgraph(strict):
         for a, b in zip(want, got):
             assert torch.equal(a, b), t
     assert_status_clear()
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_single_precision_step_fullgraph(batch):
+    """The decoder's step as one graph: logits, caches and position as from the eager step."""
+    from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+    from relation_lm.inference.stateful_decode import StatefulDecoder
+
+    cfg = RoutedRelationConfig(vocab_size=50, boundary_vocab_size=6, d_model=64, layers=2, max_context=32, block_size=8,
+                               local_window=8, top_blocks=1)
+    model = RoutedRelationLM(cfg, seed=4)
+    eager, traced = (StatefulDecoder(model, batch, "cuda", torch.float32) for _ in range(2))
+    torch._dynamo.reset()                   # no shapes of another decoder's trace
+    step = torch.compile(traced.step, fullgraph=True)
+    ids = torch.arange(batch, device="cuda")
+    with torch.no_grad():
+        for t in range(4):
+            want, got = eager.step(ids + t, ids % 6), step(ids + t, ids % 6)
+            assert all(torch.equal(a, b) for a, b in zip(want, got)), t
+    for name in ("position", "anchor_keys", "operand_cache", "expanded_cache"):
+        assert torch.equal(getattr(eager, name), getattr(traced, name)), name
+    assert_status_clear()
