@@ -168,8 +168,15 @@ class StatefulDecoder:
             if self.few_rows:
                 self.packed_rows = zeros(B, self.w["w_packed"].shape[0])
                 self.second_rows = zeros(B, cfg.k_max, cfg.d_model)
+            # The heads too, unless their weights, which may be the model's own, start off a 16-byte boundary, or are so many
+            # rows that libraries stream them faster (us, library / own kernel: one row of d 768, 16 256 columns 22.9 / 11.0,
+            # 32 000 18.9 / 21.1, 128 256 61 / 71; eight rows 16 256 26.2 / 22.5, 32 000 42.8 / 43.2, 50 304 64 / 66, of d 1024
+            # 128 256 169 / 212; two to four rows and d 256 are the kernel's at every size: four rows of d 768, 128 256 1.47 x).
+            columns = cfg.vocab_size + cfg.boundary_vocab_size
+            many = cfg.d_model > 256 and (columns > 24_000 if B == 1 else columns > 40_000 and B > 4)
+            self.few_heads = self.few_rows and not many and all(self.w[n].data_ptr() % 16 == 0 for n in ("token_embedding", "boundary_w"))
             # one product for both heads where its column slices are dense matrices, as two products' results are
-            elif B == 1:
+            if B == 1 and not self.few_heads:
                 self.head_weight = torch.cat((self.w["token_embedding"], self.w["boundary_w"]), 0).contiguous()
                 self.head_bias = torch.cat((zeros(cfg.vocab_size), self.w["boundary_b"]))
         else:
@@ -313,11 +320,11 @@ class StatefulDecoder:
             if keep_selection:
                 self.last_selection.append((anchor, partner))
         self.last_final = normalized
-        if grouped:
+        if grouped and self.few_heads:
             heads = _abi.direct_call("single_precision_heads", normalized, w["token_embedding"], w["boundary_w"], w["boundary_b"], pos)
             if heads is not NotImplemented:
                 return heads
-        if self.few_rows:
+        if self.few_heads:
             heads = normalized.new_empty(self.batch, cfg.vocab_size), normalized.new_empty(self.batch, cfg.boundary_vocab_size)
             few_rows_projection_pair(*heads, normalized, w["token_embedding"], w["boundary_w"], w["boundary_b"])
         elif self.batch == 1:

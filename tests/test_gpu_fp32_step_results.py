@@ -76,3 +76,49 @@ def test_a_step_past_the_context_is_reported_and_changes_no_state(batch, keep_se
         results.append([r.clone() for t in range(33, 40) for r in dec.step(tokens[t], bounds[t], keep_selection)])
         assert_status_clear()
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("batch", [1, 2])
+def test_weights_that_start_anywhere(batch):
+    """The heads' weights are the model's own where those are already on the device in single precision: slices of a flat
+    buffer, off a 16-byte boundary, included."""
+    from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+    from relation_lm.inference.stateful_decode import StatefulDecoder
+
+    cfg = RoutedRelationConfig(vocab_size=50, boundary_vocab_size=6, d_model=64, layers=1, max_context=32, block_size=8,
+                               local_window=8, top_blocks=1)
+    model = RoutedRelationLM(cfg, seed=1).cuda()
+    want = StatefulDecoder(model, batch, "cuda", torch.float32)
+    for weight in (model.token_embedding.weight, model.boundary_output.weight):
+        flat = torch.cat((weight.detach().new_zeros(1), weight.detach().flatten()))
+        weight.data = flat[1:].view_as(weight)
+    got = StatefulDecoder(model, batch, "cuda", torch.float32)
+    tokens, bounds = (torch.randint(0, n, (4, batch), device="cuda") for n in (50, 6))
+    for t in range(4):
+        a, b = want.step(tokens[t], bounds[t]), got.step(tokens[t], bounds[t])
+        # a sum of 64 products in another order: 64 roundings of a sum of magnitudes below 64 times the largest product
+        for x, y in zip(a, b):
+            assert float((x - y).abs().max()) <= 64 * 2.0 ** -24 * 64 * float(want.last_final.abs().max())
+    assert torch.equal(want.position, got.position) and torch.equal(want.expanded_cache, got.expanded_cache)
+    assert_status_clear()
+
+
+@pytest.mark.parametrize("batch,vocab", [(1, 24_100), (5, 40_100), (4, 40_100)])
+def test_heads_of_many_columns(batch, vocab):
+    """On either side of where a library's product takes the heads: both heads against 64-bit products of the step's rows."""
+    from relation_lm.inference.routed_model import RoutedRelationConfig, RoutedRelationLM
+    from relation_lm.inference.stateful_decode import StatefulDecoder
+
+    cfg = RoutedRelationConfig(vocab_size=vocab, boundary_vocab_size=6, d_model=264, layers=1, max_context=32, block_size=8,
+                               local_window=8, top_blocks=1)
+    dec = StatefulDecoder(RoutedRelationLM(cfg, seed=1), batch, "cuda", torch.float32)
+    assert dec.few_rows and dec.few_heads == (batch == 4)
+    for keep_selection in (False, True):
+        heads = dec.step(torch.arange(batch, device="cuda"), torch.zeros(batch, dtype=torch.int64, device="cuda"), keep_selection)
+        rows = dec.last_final.double()
+        for got, (weight, bias) in zip(heads, ((dec.w["token_embedding"], None), (dec.w["boundary_w"], dec.w["boundary_b"]))):
+            full = torch.nn.functional.linear(rows, weight.double(), bias.double() if bias is not None else None)
+            size = rows.abs() @ weight.double().abs().T + 1.0
+            assert got.is_contiguous() and bool(((got.double() - full).abs() <= 264 * 2.0 ** -24 * size).all())
+    assert int(dec.position) == 2
+    assert_status_clear()
