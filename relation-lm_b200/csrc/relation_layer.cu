@@ -69,8 +69,7 @@ int launch_layer(SelectArgs& sel, LayerTailArgs& tail, const void* product_weigh
     if (tail.seqs_per_cluster > tail.cluster) tail.seqs_per_cluster = tail.cluster;   // a selecting CTA per sequence
     const uint32_t smem_bytes = lt_smem_bytes_with_stage(tail.rdim, tail.d, tail.query_weight ? tail.n_query / tail.cluster : 0,
                                                          sel.plan.total);
-    const LtPlan whole = lt_plan(tail.rdim, tail.d, true, kLtMaxPairs, 0);
-    if (sel.plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) {
+    if (sel.plan.total > lt_stage_room(tail.rdim, tail.d) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) {
         set_error("relation_layer: the selector's working set does not fit the tail's tile memory (use the two launches)");
         return RLM_ERR_UNSUPPORTED;
     }
@@ -115,8 +114,7 @@ extern "C" int rlm_relation_layer_supported(int n_seq, int k_out, int relation_d
     const Plan plan = make_plan(n_blocks, max_t / n_blocks, local_window, top_blocks, buckets, dtype_size(dtype),
                                 dtype_size(dtype), kPacked, false);
     const uint32_t smem_bytes = lt_smem_bytes_with_stage(relation_dim, d_model, n_query / cluster, plan.total);
-    const LtPlan whole = lt_plan(relation_dim, d_model, true, kLtMaxPairs, 0);
-    if (plan.total > static_cast<int>(whole.total - whole.p) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) return 0;
+    if (plan.total > lt_stage_room(relation_dim, d_model) || smem_bytes > static_cast<uint32_t>(kSmemDynamicLimit)) return 0;
     auto kernel = layer_kernel(dtype == RLM_BF16, true, true);
     if (lt_prepare(reinterpret_cast<const void*>(kernel), cluster) != RLM_OK) return 0;
     cudaLaunchConfig_t config = {};

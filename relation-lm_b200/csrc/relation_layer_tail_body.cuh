@@ -131,6 +131,15 @@ inline uint32_t lt_smem_bytes_with_stage(int rdim, int d, int nq_own, int stage)
     return most;
 }
 
+// Bytes that a stage in front of the gathers may take: 64 pairs' product tile, the residual rows or hidden slice, the terms and
+// eight sequences' operand rows (which once stood there; what fitted then fits: a launch's shared memory counts the stage).
+inline int lt_stage_room(int rdim, int d) {
+    const int product = rdim / kBK * kLtMaxPairs * 128, normalised = kLtMaxPairs * (kLtOwn + 1) * 4;
+    const int slice = 2 * kLtMaxPairs * 128, rows_in = kLtMaxSeq * d * 4;
+    return (((product > normalised ? product : normalised) + 1023) & ~1023) + (slice > rows_in ? slice : rows_in) +
+           (kLtMaxPairs + kLtMaxSeq) * (2 * kLtHC + 16) + kLtMaxSeq * rdim * 2;
+}
+
 __device__ __forceinline__ uint32_t lt_cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -238,3 +238,14 @@ def test_a_cache_row_that_is_not_finite_stays_with_its_sequence_and_slot(B, K, d
                     assert torch.equal(got[~hit], want[~hit]), (seq, slot, column)
                     assert bool(got[hit].isnan().all()), (seq, slot, column)
     assert_status_clear()
+
+
+@pytest.mark.parametrize("B,d,window,fits", [(3, 256, 72, True), (8, 128, 72, True), (3, 256, 76, False)])
+def test_whole_layer_takes_a_selector_up_to_its_room(B, d, window, fits):
+    """16 blocks of 32 keys, six of them fetched, 16 buckets: 53 968 bytes in front of the tail with a window of 72, 55 008
+    with 76, of 54 400; the results are those of the two launches."""
+    from relation_lm.kernels.relation_layer import relation_layer_supported
+
+    assert relation_layer_supported(B, 8, 128, 4 * d, d, 256, torch.bfloat16, 512, 16, 16, window, 6) == fits
+    if fits:
+        test_whole_layer_equals_select_then_tail(B, 8, d, 128, 512, 16, window, 6, 256, torch.bfloat16)
