@@ -373,7 +373,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_wm) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
-        for (int i = 0; i < 12 + (kWide ? 2 * kLtMaxRing : 0); ++i) mbar_init(smem_u32(&bars[i]), 1);
+        for (int i = 0; i < 12 + (kWide ? 2 * kLtMaxRing : 0); ++i) mbar_init(smem_u32(&bars[i]), kWide && i == 2 ? 2 : 1);
         fence_barrier_init();
         mbar_expect_tx(bar_part, static_cast<uint32_t>(senders * quads) * (kOwn * 16u));
         mbar_expect_tx(bar_stat, static_cast<uint32_t>(C * ((pairs + 1) & ~1)) * 8u);
@@ -385,7 +385,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             tma_load_2d(smem_u32(wm_tile) + kb * kHC * 128u, &map_wm, kb * kBK, h0, bar_wm);
         // W_2: this half's output rows, by K-block of hidden columns: this CTA's two, then the sharing CTA's
         if (kWide)
-            for (int n = 0; n < ring; ++n) request_w2(n);
+            for (int n = 0; n < ring - 1; ++n) request_w2(n);   // (the last place holds the products' low parts first)
         for (int other = 0; !kWide && other < share; ++other) {
             const uint32_t bar = other ? bar_w2b : bar_w2;
             const int from = (other ? static_cast<int>(sharer) : static_cast<int>(rank)) * kLtHC;
@@ -480,7 +480,10 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             cp_async16(smem_u32(term_a) + a_entry * kTermStride + 16 * (kHC / 32 * quarter + i), src + 16 * (kHC / 32 * quarter + i));
     }
     cp_async_commit();
-    // products o[a] * o[p], in fp32, rounded to the operand dtype; zeros in the rows of pairs that do not exist
+    // products o[a] * o[p], in fp32, rounded to the operand dtype; zeros in the rows of pairs that do not exist.  Wide: the
+    // difference to the rounded product in a tile of its own, with which the product GEMM has all bits of the product
+    // (16 of two bfloat16 factors, 22 of two halves), as the separate kernels below 256 pairs have it.
+    const uint32_t low_tile = smem_u32(w2_tile) + static_cast<uint32_t>(kWide ? ring - 1 : 0) * kLtW2Tile;
     for (int c0 = 0;;) {
         if (entry < pairs_pad)
 #pragma unroll
@@ -489,10 +492,22 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
                 float fp[8], fa[8];
                 unpack8(pv[i], dtype, fp);
                 unpack8(av[i], dtype, fa);
+                const uint32_t at = swizzled(entry, c0 + tpp * i + sub, p_kblock);
+                uint32_t high[4], low[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float x = fp[2 * e] * fa[2 * e], y = fp[2 * e + 1] * fa[2 * e + 1];
+                    high[e] = pack2(x, y, dtype);
+                    if (kWide) {
+                        const float hx = lt_from16(static_cast<uint16_t>(high[e]), dtype), hy = lt_from16(static_cast<uint16_t>(high[e] >> 16), dtype);
+                        low[e] = pack2(isfinite(hx) ? x - hx : 0.0f, isfinite(hy) ? y - hy : 0.0f, dtype);
+                    }
+                }
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
-                             ::"r"(smem_u32(p_tile) + swizzled(entry, c0 + tpp * i + sub, p_kblock)), "r"(pack2(fp[0] * fa[0], fp[1] * fa[1], dtype)),
-                               "r"(pack2(fp[2] * fa[2], fp[3] * fa[3], dtype)), "r"(pack2(fp[4] * fa[4], fp[5] * fa[5], dtype)),
-                               "r"(pack2(fp[6] * fa[6], fp[7] * fa[7], dtype)) : "memory");
+                             ::"r"(smem_u32(p_tile) + at), "r"(high[0]), "r"(high[1]), "r"(high[2]), "r"(high[3]) : "memory");
+                if (kWide)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                                 ::"r"(low_tile + at), "r"(low[0]), "r"(low[1]), "r"(low[2]), "r"(low[3]) : "memory");
             }
         c0 += 4 * tpp;
         if (c0 >= chunks) break;
@@ -506,19 +521,21 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     const uint32_t tmem_d2 = tmem_base + (kWide ? 128u : 64u);      // second GEMM: mtiles x pairs_pad columns
 
     // ---- product GEMM: D1[hidden column, pair] = W_m slice x products^T
-    if (warp == 0) {
+    // (wide: 192 hidden columns as two overlapping tiles of 128, rows 0 .. 127 and rows 64 .. 191, a warp each)
+    if (warp < (kWide ? 2 : 1)) {
         const bool ok = mbar_wait(bar_wm, 0), issue = elect_lane();
         if (!ok) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tile = kWide ? static_cast<uint32_t>(warp) : 0u;
         for (int kb = 0; kb < kblocks; ++kb) {
-            const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kHC * 128u);
-            const uint64_t dp = smem_desc_sw128(smem_u32(p_tile) + kb * p_kblock);
-            // (192 hidden columns as two overlapping tiles of 128: rows 0 .. 127, rows 64 .. 191)
+            const uint64_t dw = smem_desc_sw128(smem_u32(wm_tile) + kb * kHC * 128u) + tile * (64 * 128 >> 4);
 #pragma unroll
-            for (int half = 0; half < (kWide ? 2 : 1); ++half)
+            for (int part = 0; part < (kWide ? 2 : 1); ++part) {
+                const uint64_t dp = smem_desc_sw128((part ? low_tile : smem_u32(p_tile)) + kb * p_kblock);
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; ++kk)
-                    umma_f16_if(tmem_base + 64u * half, dw + half * (64 * 128 >> 4) + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u, issue && ok);
+                    umma_f16_if(tmem_base + 64u * tile, dw + 2 * kk, dp + 2 * kk, idesc, (kb > 0 || part > 0 || kk > 0) ? 1u : 0u, issue && ok);
+            }
         }
         umma_commit_if(bar_d1, issue);
     }
@@ -622,6 +639,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
             }
             umma_commit_if(bar_d2 + 8u * mt, issue);
         } else if (warp == 2 && lane == 0) {
+            request_w2(ring - 1);                              // the low parts are consumed
             for (int n = ring; n < 18; ++n) {
                 if (!mbar_wait(bar_empty(n % ring), (n / ring - 1) & 1)) { failed = 1; break; }
                 request_w2(n);
@@ -956,9 +974,9 @@ int lt_validate(const LayerTailArgs& a, bool wide = false) {
         set_error("relation_layer_tail: query projection width must be a multiple of 16 outputs per CTA (H / 128 CTAs), at most 64 each");
         return RLM_ERR_UNSUPPORTED;
     }
-    // (a ring has to hold what takes its place later: 64 pairs' partial sums are six tiles)
+    // (a ring has to hold what takes its place: 64 pairs' partial sums are six tiles; in its last one the products' low parts)
     if (lt_smem_bytes(a.rdim, a.d, a.query_weight ? a.n_query / cluster : 0) > static_cast<uint32_t>(kSmemDynamicLimit) ||
-        (lt_wide(a.d) && lt_plan(a.rdim, a.d, true, kLtMaxPairs, 0).ring < 6)) {
+        (lt_wide(a.d) && (lt_plan(a.rdim, a.d, true, kLtMaxPairs, 0).ring < 6 || a.rdim > 2 * kBK))) {
         set_error("relation_layer_tail: the weight slices exceed 227 KB of shared memory");
         return RLM_ERR_SMEM;
     }

@@ -66,3 +66,40 @@ def test_wide_tail_rejects_other_widths():
     assert not relation_layer_tail_wide_supported(8, 8, 256, 3072, 768, 256, torch.bfloat16)      # the ring does not fit
     with pytest.raises(ValueError):
         _run(_case(2, 8, 512, 128, 16, 0, torch.bfloat16, 1), 5, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,K", [(1, 8), (4, 5), (8, 8), (28, 8), (56, 4)])
+def test_wide_tail_is_no_further_from_64_bits_than_the_separate_kernels(B, K, dtype):
+    """The separate launches that this tail stands for below 256 pairs keep the products of the operand rows in fp32 and
+    the second layer's rows in 16 bits; the tail has all bits of the products, too, and its rows in fp32.  Both against
+    the composition in 64 bits: residual rows and normalised rows, root mean square."""
+    import torch.nn.functional as F
+
+    from relation_lm.kernels.relation_reduce import relation_hidden_cached_out, relation_norm_reduce_residual_norm
+
+    T, t, R = 96, 95, 128
+    x = _case(B, K, 768, R, T, 256, dtype, 8600 + B)
+    x["partner"], x["scores"] = x["partner"].clamp(min=0), torch.randn(B, K, generator=torch.Generator().manual_seed(B))
+    hidden, normalized, _ = _run(x, t, dtype)
+
+    dev = {k: (v.cuda() if isinstance(v, torch.Tensor) else v) for k, v in x.items()}
+    rows = torch.empty(B, K, 3072, device="cuda", dtype=dtype)
+    relation_hidden_cached_out(rows, dev["expanded"], dev["operand"], dev["anchor"], dev["partner"], dev["wm"])
+    separate, separate_norm = dev["hidden"].clone(), torch.empty(B, 768, device="cuda", dtype=dtype)
+    relation_norm_reduce_residual_norm(F.linear(rows, dev["w2"], dev["b2"]), dev["scores"], dev["gamma"], dev["beta"], position_tensor(t),
+                                       1e-5, separate, dev["mix"], dev["next_w"], dev["next_b"], 1e-5, separate_norm)
+
+    w = {k: (v.double() if v.is_floating_point() else v.long()) for k, v in dev.items() if isinstance(v, torch.Tensor)}
+    seq = torch.arange(B, device="cuda")
+    products = w["operand"][seq, w["anchor"]][:, None] * w["operand"][seq[:, None], w["partner"]]
+    first = w["expanded"][seq, w["anchor"], :3072][:, None] + w["expanded"][seq[:, None], w["partner"], 3072:] + products @ w["wm"].T
+    second = F.layer_norm(F.gelu(first) @ w["w2"].T + w["b2"], (768,), w["gamma"], w["beta"], 1e-5)
+    active = torch.arange(K, device="cuda") < 7                                  # ceil(log2(t + 2)) partners take part
+    weight = torch.softmax(w["scores"].masked_fill(~active, -torch.inf), 1)
+    exact = w["hidden"] + w["mix"] * (weight[..., None] * second).sum(1)
+    exact_norm = F.layer_norm(exact, (768,), w["next_w"], w["next_b"], 1e-5)
+    off = lambda got, want: float((got.double() - want).square().mean().sqrt())  # noqa: E731
+    assert off(hidden, exact) <= off(separate, exact)
+    assert off(normalized, exact_norm) <= 1.02 * off(separate_norm, exact_norm)  # (both are its rounding to 16 bits)
+    assert_status_clear()
