@@ -416,7 +416,8 @@ int rlm_relation_layer_tail(
 
 /*
  * The same for d = 768, H = 3072 (extension): clusters of 16 CTAs of 192 hidden and 48 output columns each, whose slices
- * of second_weight are streamed.  R 64 or 128, NQ a multiple of 256; arguments and results as above.
+ * of second_weight are streamed and whose products of operand rows keep all their bits.  R 64 or 128; a query projection with
+ * R 128 only, NQ 256.  Arguments and results as above.
  */
 int rlm_relation_layer_tail_wide_supported(int n_seq, int k_out, int relation_dim, int hidden_dim,
                                            int d_model, int n_query, int dtype);

@@ -41,7 +41,8 @@ struct FewRowsArgs {
 };
 
 // kRows rows at a time, kCols columns per warp.  Fewer rows leave registers for more CTAs on an SM, whose loads are what
-// a stream needs (one row, 512 x 16256: 11.7 us with two CTAs, 8.4 with four).
+// a stream needs (one row, 512 x 16256: 11.7 us with two CTAs, 8.4 with four).  Under those caps <4, *> and <2, 4> spill
+// 4 to 20 bytes.
 template <int kRows, int kCols>
 __global__ void __launch_bounds__(kFewThreads, kRows <= 2 ? 4 : kRows <= 4 ? 3 : 2) few_rows_projection_kernel(const FewRowsArgs a) {
     constexpr int kSums = kRows * kCols;

@@ -14,21 +14,25 @@
 // pairs; CTA c owns hidden columns [128 c, 128 c + 128).  Its weight slices — W_m[128 c .., :]
 // (128 x R) and W_2[:, 128 c ..] (d x 128) — are requested by TMA before the dependency wait and
 // stay resident in shared memory.  After the selector's indices arrive every CTA gathers the
-// operand rows (multiplied in place into the swizzled B tile) and its 128 columns of the two
+// operand rows (multiplied from registers into the swizzled B tile) and its 128 columns of the two
 // expanded-cache terms, runs the product GEMM with the hidden columns on the TMEM lanes
 // (tcgen05.mma, pairs on the TMEM columns), applies GELU and writes its hidden slice as the
 // K-major B tile of the second GEMM, whose A operand is the resident W_2 slice: a split-K GEMM
 // over the cluster, each CTA holding a partial raw^T [d, pairs] in TMEM.
 //
 // Launches of more than 16 pairs a cluster (d >= 256): the partial sums, C x d x pairs floats through distributed shared
-// memory at some 15 bytes a cycle and CTA, become what takes the time (64 pairs: 8 300 of 28 000 cycles).  There
+// memory at some 15 bytes a cycle and CTA, become what takes the time (64 pairs: waited for during 8 300 of 32 000 cycles,
+// sharing 5 800 of 28 600; 32 pairs 5 300 of 22 500, 3 600 of 20 300).  There
 // neighbouring CTAs exchange their 16-bit hidden slices and divide the output rows: each has half of the rows over both
 // slices, the partial sums are half as many, and the other's slice travels while the own one is multiplied.
 //
 // d = 768 (kWide): 16 CTAs of 192 hidden columns (two overlapping tiles of the product GEMM) and 48 output columns, always
 // sharing; a CTA's part of W_2, 288 KB, does not fit beside the rest and goes through a ring of six to nine tiles of
-// 16 KB, three warps issuing a tile of output rows each and a fourth refilling.  us a step of 12 layers in a graph, five
-// launches a layer -> here: batch 1 319 -> 239, batch 8 338 -> 255, batch 16 405 -> 318, batch 28 481 -> 387.
+// 16 KB, three warps issuing a tile of output rows each and a fourth refilling.  The products of the operand rows keep all
+// their bits here (a second tile for what rounding to 16 bits takes off), because the separate kernels that this form
+// replaces keep them in fp32: residual rows are 1.61e-4 off 64 bits (bf16, 28 x 8 pairs, root mean square), 2.09e-4 without,
+// 2.27e-4 from the separate kernels, for 1 us a layer of 8 sequences.  us a step of 12 layers, context 1024, in a graph,
+// five launches a layer -> here: batch 1 303 -> 250, batch 8 341 -> 269, batch 16 407 -> 324, batch 28 483 -> 400.
 //
 // us a step of 6 layers of d 512 before sharing, the gathers through registers, two issuing warps and the statistics in
 // messages of two pairs -> with them: batch 1 84.0 -> 81.9, 5 98.4 -> 94.3, 8 97.5 -> 94.3, 16 128.5 -> 122.5,

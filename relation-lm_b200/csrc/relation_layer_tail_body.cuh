@@ -434,7 +434,7 @@ __device__ __forceinline__ void layer_tail_body(const CUtensorMap& map_wm, const
     // parts of its operand rows into registers at once, so that neither a shared-memory round trip nor a barrier lies
     // between the selector's indices and the products, which go straight into the swizzled tile.  Behind them, by
     // cp.async, this CTA's columns of the two expanded-cache terms, needed by the epilogue.  (Operand rows by cp.async,
-    // multiplied in place behind a barrier: 2 850 cycles from the wait to the products at batch 1, now 1 360.)  The scores are
+    // multiplied in place behind a barrier: 2 850 cycles from the wait to the products at batch 1, now 1 550.)  The scores are
     // requested with the indices; the anchors' terms are gathered by threads that a small batch's pairs leave free.
     const size_t op_row = static_cast<size_t>(R) * 2, ex_row = static_cast<size_t>(H) * 4;
     const int a_entry = (tid - kLtThreads / 2) >> 2;          // sequence whose anchor's terms this thread gathers

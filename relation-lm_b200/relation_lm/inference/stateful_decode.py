@@ -115,8 +115,11 @@ class StatefulDecoder:
         can_tail = (self.fused and not self.fused_tail and self.second_layer_splits == 1 and self.stacked_expand and B <= 64
                     and (relation_layer_tail_wide_supported(*sizes) if wide else relation_layer_tail_supported(*sizes)))
         self._tail = relation_layer_tail_wide if wide else relation_layer_tail
-        # (d 768 below 256 pairs; us per step of 12 layers with the tail / with four or five launches a layer: 255 / 338
-        # for 8 sequences, 387 / 481 for 28, 397 / 355 for 32, whose hidden states take the tensor-core kernel there)
+        # (d 768 below 256 pairs; us per step of 12 layers, context 1024, with the tail / with four or five launches a layer:
+        # 250 / 303 for one sequence, 269 / 341 for 8, 400 / 483 for 28; 397 / 355 for 32 at context 512, whose hidden states
+        # take the tensor-core kernel.  From 57 sequences on, K <= 4, its eight clusters of 16 CTAs take two waves, as seven
+        # run at a time, and it is still the faster: 373 / 622 for 56 of K 4, 537 / 653 for 57, 623 / 652 for 63, 616 / 653
+        # for 64 of K 3, 516 / 634 of K 1)
         by_default = can_tail and not (wide and B * cfg.k_max >= 256)
         self.layer_tail = by_default if layer_tail is None else (bool(layer_tail) and can_tail)
         if self.layer_tail:
@@ -442,7 +445,9 @@ class StatefulDecoder:
             # every layer's operand row of this position is known: expand them all at once, straight from
             # the packed rows (written two launches back), so that this launch overlaps the append (us a step,
             # from the operand cache -> from the packed rows: 24 sequences of d 256, 4 layers 89.0 -> 86.1, 32 of d 512,
-            # 6 layers 159.7 -> 158.0; of d 768, 12 layers, where the two compete for memory, 8 256.1 -> 257.3, 28 386.1 -> 388.9)
+            # 6 layers 159.7 -> 158.0; of d 768, 12 layers, where the two compete for memory, 8 256.1 -> 257.3, 28 386.1 -> 388.9).
+            # It reads `packed` ahead of its dependency wait: exactly one launch, which waits before it lets this one go, has
+            # to lie between the projection and this call: the append.
             expanded_cache_append_packed(self.expanded_cache, packed, w["anchor_weight"], w["partner_weight"],
                                          w["first_bias"], pos)
         elif self.stacked_expand:
