@@ -158,6 +158,19 @@ __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(cons
 // 1233 -> 955 us.  Issue slots are 71 % taken now (56 % before).
 constexpr uint32_t kRow = 2 * kD;
 
+// A row in kDt, and a lane's eighth of it: 16 bytes, in single precision (the decode form alone) 32.
+template <int kDt> constexpr uint32_t kRowOf = kDt == RLM_F32 ? 4 * kD : kRow;
+struct WideChunk { uint4 lo, hi; };
+template <int kDt> struct RowChunk { using type = uint4; };
+template <> struct RowChunk<RLM_F32> { using type = WideChunk; };
+template <int kDt> using Chunk = typename RowChunk<kDt>::type;
+
+template <int kDt>
+__device__ __forceinline__ Chunk<kDt> load_chunk(const unsigned char* p) {
+    if constexpr (kDt == RLM_F32) return {reinterpret_cast<const uint4*>(p)[0], reinterpret_cast<const uint4*>(p)[1]};
+    else return *reinterpret_cast<const uint4*>(p);
+}
+
 // This lane's chunk of a query, every element twice: operands of the two-wide fma over two rows.
 struct QueryChunk { float2 v[8]; };
 
@@ -188,7 +201,15 @@ __device__ __forceinline__ void widen_pair(uint32_t a, uint32_t b, float2& lower
 
 // seg8 of this lane's chunk for two rows
 template <int kDt>
-__device__ __forceinline__ float2 seg_pair(const uint4 w0, const uint4 w1, const QueryChunk& q) {
+__device__ __forceinline__ float2 seg_pair(const Chunk<kDt> w0, const Chunk<kDt> w1, const QueryChunk& q) {
+    if constexpr (kDt == RLM_F32) {
+        const uint32_t a[8] = {w0.lo.x, w0.lo.y, w0.lo.z, w0.lo.w, w0.hi.x, w0.hi.y, w0.hi.z, w0.hi.w};
+        const uint32_t b[8] = {w1.lo.x, w1.lo.y, w1.lo.z, w1.lo.w, w1.hi.x, w1.hi.y, w1.hi.z, w1.hi.w};
+        float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc = __ffma2_rn(make_float2(__uint_as_float(a[i]), __uint_as_float(b[i])), q.v[i], acc);
+        return acc;
+    } else {
     const uint32_t a[4] = {w0.x, w0.y, w0.z, w0.w}, b[4] = {w1.x, w1.y, w1.z, w1.w};
     float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
@@ -199,6 +220,7 @@ __device__ __forceinline__ float2 seg_pair(const uint4 w0, const uint4 w1, const
         acc = __ffma2_rn(upper, q.v[2 * i + 1], acc);
     }
     return acc;
+    }
 }
 
 // One level of the butterfly over the chunk lanes: of kN values (a row each) a lane keeps those whose index has the
@@ -219,7 +241,7 @@ __device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q
     constexpr int kStep = kN < 4 ? kN : 4;
 #pragma unroll
     for (int h = 0; h < kN; h += kStep) {
-        uint4 w[kStep];
+        Chunk<kDt> w[kStep];
 #pragma unroll
         for (int i = 0; i < kStep; ++i) w[i] = load(h + i);
 #pragma unroll
@@ -305,17 +327,17 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
-    const unsigned char* mine = rows + 16 * chunk;
+    const unsigned char* mine = rows + kRowOf<kDt> / 8 * chunk;
     for (int base = 4 * kN * first; base < n_rows; base += 4 * kN * step) {
         float sc;
         if (base >= first_valid && base + 4 * kN <= n_rows) {
-            const unsigned char* src = mine + (base + rq) * static_cast<int>(kRow);
-            sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+            const unsigned char* src = mine + (base + rq) * static_cast<int>(kRowOf<kDt>);
+            sc = pass_score<kDt, kN>([&](int i) { return load_chunk<kDt>(src + i * static_cast<int>(4 * kRowOf<kDt>)); }, q);
         } else {
             // the ragged ends read a staged row in place of each missing one
             sc = pass_score<kDt, kN>([&](int i) {
                 const int r = min(max(base + 4 * i + rq, first_valid), n_rows - 1);
-                return *reinterpret_cast<const uint4*>(mine + r * static_cast<int>(kRow));
+                return load_chunk<kDt>(mine + r * static_cast<int>(kRowOf<kDt>));
             }, q);
         }
         const int r = base + 4 * (chunk & (kN - 1)) + rq, pos = pos0 + r;
@@ -337,7 +359,7 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
     int my_pos = 0x7fffffff;
-    const unsigned char* mine = keys + 16 * chunk;
+    const unsigned char* mine = keys + kRowOf<kDt> / 8 * chunk;
     for (int base = 4 * kN * first; base < n_rows; base += 4 * kN * step) {
         const int r = base + 4 * (chunk & (kN - 1)) + rq;
         int pos;                                         // position of row r, or -1
@@ -346,9 +368,9 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
             // the pass lies in one picked block: rows 4 i + rq are 512 bytes apart
             const int rank = base >> bs_shift, o0 = base - (rank << bs_shift);
             const int start = sel[3 * rank] * bs + o0, lim = sel[3 * rank + 2] - o0;
-            const unsigned char* src = mine + static_cast<size_t>(start + rq) * kRow;
+            const unsigned char* src = mine + static_cast<size_t>(start + rq) * kRowOf<kDt>;
             // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
-            sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+            sc = pass_score<kDt, kN>([&](int i) { return load_chunk<kDt>(src + i * static_cast<int>(4 * kRowOf<kDt>)); }, q);
             pos = r - base < lim ? start + (r - base) : -1;
         } else {
             auto row_pos = [&](int row) -> int {
@@ -358,7 +380,7 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
             };
             sc = pass_score<kDt, kN>([&](int i) {
                 const int p = row_pos(base + 4 * i + rq);
-                return p >= 0 ? *reinterpret_cast<const uint4*>(mine + static_cast<size_t>(p) * kRow) : make_uint4(0, 0, 0, 0);
+                return p >= 0 ? load_chunk<kDt>(mine + static_cast<size_t>(p) * kRowOf<kDt>) : Chunk<kDt>{};
             }, q);
             pos = row_pos(r);
         }
@@ -389,10 +411,10 @@ __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, con
     const bool x2 = lane & 2, x4 = lane & 4;
     for (int base = 32 * first; base < n_complete; base += 32 * step) {
         float sums[8], md[4], sd[4];
-        const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
-        chunk_sums<kDt, 8>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+        const auto at = [&](int i) { return static_cast<uint32_t>(min(base + 4 * i + rq, n_complete - 1)) * kRowOf<kDt> + kRowOf<kDt> / 8 * chunk; };
+        chunk_sums<kDt, 8>([&](int i) { return load_chunk<kDt>(mean + at(i)); }, q, sums);
         fold_level<8, 1>(sums, md);
-        chunk_sums<kDt, 8>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+        chunk_sums<kDt, 8>([&](int i) { return load_chunk<kDt>(stdv + at(i)); }, qa, sums);
         fold_level<8, 1>(sums, sd);
         // v[j]: head (chunk >> 1) of block 4 (2 j + (chunk & 1)) + rq
         float v[4], w[2][2], sh[4];
@@ -447,10 +469,10 @@ __device__ __forceinline__ void score_eight_blocks(const unsigned char* mean, co
 #pragma unroll
     for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
     float sums[2], md[1], sd[1];
-    const auto at = [&](int i) { return static_cast<uint32_t>(min(first + 4 * i + rq, n_complete - 1)) * kRow + 16 * chunk; };
-    chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(mean + at(i)); }, q, sums);
+    const auto at = [&](int i) { return static_cast<uint32_t>(min(first + 4 * i + rq, n_complete - 1)) * kRowOf<kDt> + kRowOf<kDt> / 8 * chunk; };
+    chunk_sums<kDt, 2>([&](int i) { return load_chunk<kDt>(mean + at(i)); }, q, sums);
     fold_level<2, 1>(sums, md);
-    chunk_sums<kDt, 2>([&](int i) { return *reinterpret_cast<const uint4*>(stdv + at(i)); }, qa, sums);
+    chunk_sums<kDt, 2>([&](int i) { return load_chunk<kDt>(stdv + at(i)); }, qa, sums);
     fold_level<2, 1>(sums, sd);
     const float sh = __fadd_rn(__fmul_rn(__fadd_rn(md[0], __fmul_rn(sp, sd[0])), 0.25f), shift);
     float mx = fmaxf(sh, __shfl_xor_sync(0xffffffffu, sh, 2));
@@ -492,9 +514,9 @@ __device__ __forceinline__ void score_picked_pass(const unsigned char* keys, int
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3, base = 4 * kN * first;
     const int rank = base >> bs_shift, o0 = base - (rank << bs_shift), block = __shfl_sync(0xffffffffu, picked, rank);
     const int start = max(block, 0) * bs + o0, lim = block < 0 ? 0 : min(max(ls - block * bs, 0), bs) - o0;
-    const unsigned char* src = keys + static_cast<size_t>(start + rq) * kRow + 16 * chunk;
+    const unsigned char* src = keys + static_cast<size_t>(start + rq) * kRowOf<kDt> + kRowOf<kDt> / 8 * chunk;
     // rows past `lim` are read too (they lie inside the block, hence inside the cache) and ignored
-    float sc = pass_score<kDt, kN>([&](int i) { return *reinterpret_cast<const uint4*>(src + i * static_cast<int>(4 * kRow)); }, q);
+    float sc = pass_score<kDt, kN>([&](int i) { return load_chunk<kDt>(src + i * static_cast<int>(4 * kRowOf<kDt>)); }, q);
     const int o = 4 * (chunk & (kN - 1)) + rq, pos = start + o;
     const bool valid = o < lim && pos != exclude;
     sc = valid ? sc : kNegInf;
@@ -643,7 +665,7 @@ __device__ __forceinline__ int rank_among(const uint32_t* keys, int n_groups, ui
     return (r0 + r1) + (r2 + r3);
 }
 
-// ---- the decode form in one 16-bit dtype: a query row by a CTA of eight warps
+// ---- the decode form in one dtype: a query row by a CTA of eight warps
 //
 // A row's time is a chain of dependent phases, so what counts is their number and length, not their work.  Here a
 // phase is a pass of 32 rows or blocks by a warp (the primitives above: a handful of loads, 64 multiply-adds a lane, a
@@ -670,17 +692,17 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     const int nb = a.n_blocks, bs = a.block_size, L = a.local_window, top = a.top_blocks;
     const int bs_shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
     const int ls = max(t - L + 1, 0), first_local = ls - (t - L + 1), n_complete = max(min((t + 1) / bs, nb), 0);
-    const size_t seq_keys = static_cast<size_t>(row) * a.max_t * kRow, seq_stats = static_cast<size_t>(row) * nb * kRow;
+    const size_t seq_keys = static_cast<size_t>(row) * a.max_t * kRowOf<kDt>, seq_stats = static_cast<size_t>(row) * nb * kRowOf<kDt>;
     const int cap = L + top * bs, cap4 = (cap + 3) & ~3;
     const bool bad_position = t < 0 || t >= a.max_t;
     if (tid == 0 && !bad_position) {
         mbar_init(bar_a, 1);
         mbar_init(bar_p, 1);
         fence_barrier_init();
-        const uint32_t sbytes = top > 0 ? n_complete * kRow : 0u;
-        const uint32_t lbytes = (kResident ? t + 1 : t - ls + 1) * kRow;
-        const size_t loff = seq_keys + (kResident ? 0 : static_cast<size_t>(ls) * kRow);
-        const uint32_t ldst = kResident ? 0u : first_local * kRow;
+        const uint32_t sbytes = top > 0 ? n_complete * kRowOf<kDt> : 0u;
+        const uint32_t lbytes = (kResident ? t + 1 : t - ls + 1) * kRowOf<kDt>;
+        const size_t loff = seq_keys + (kResident ? 0 : static_cast<size_t>(ls) * kRowOf<kDt>);
+        const uint32_t ldst = kResident ? 0u : first_local * kRowOf<kDt>;
         const auto request = [&](const void* mean, const void* stdv, const void* keys, int mean_at, int std_at, int keys_at,
                                  uint32_t bar) {
             mbar_expect_tx(bar, 2 * sbytes + lbytes);
@@ -734,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
     const int picked_rows = top * bs;
     int* sel = sel_s + warp * 3 * kDecodeTop;
     // row r of a window is position t - L + 1 + r (only rows that are staged are read)
-    const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(kRow) : 0;
+    const ptrdiff_t window_offset = kResident ? static_cast<ptrdiff_t>(t - L + 1) * static_cast<ptrdiff_t>(kRowOf<kDt>) : 0;
     int anchor_pos = -1;
     // the anchor's stream, then the partner's: one copy of the code, so that the second finds it in the instruction cache
 #pragma unroll 1
@@ -1424,7 +1446,7 @@ int launch_tile(TileArgs& m, void* stream) {
     return check_launch("relation_select_tile_kernel");
 }
 
-// The decode form in one 16-bit dtype has the kernel of warp passes; launches of more rows than the SMs hold at once
+// The decode form in one dtype has the kernel of warp passes; launches of more rows than the SMs hold at once
 // (rows in flight count there, not a row's chain) and the other forms take a select_row build.
 template <int kDt>
 auto select_kernel(bool many_rows, bool decode, bool passes, bool resident) {
@@ -1432,6 +1454,14 @@ auto select_kernel(bool many_rows, bool decode, bool passes, bool resident) {
            : passes && !many_rows ? relation_select_decode_kernel<kDt, false>
            : many_rows ? (decode ? relation_select_kernel<4, kDt, true> : relation_select_kernel<4, kDt, false>)
                        : relation_select_kernel<3, kDt, false>;
+}
+
+template <>
+auto select_kernel<RLM_F32>(bool many_rows, bool decode, bool passes, bool resident) {
+    return resident ? relation_select_decode_kernel<RLM_F32, true>
+           : passes && !many_rows ? relation_select_decode_kernel<RLM_F32, false>
+           : decode ? (many_rows ? relation_select_kernel<4, RLM_F32, true> : relation_select_kernel<3, RLM_F32, true>)
+                    : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
 }
 
 int launch(SelectArgs& a, void* stream) {
@@ -1442,11 +1472,13 @@ int launch(SelectArgs& a, void* stream) {
     const Plan& plan = a.plan;
     const int dtype = a.key_dtype == a.query_dtype && a.stats_dtype == a.query_dtype ? a.query_dtype : kAnyDtype;
     const bool decode = a.mode == kPacked && !a.row_batch && !a.row_position && !a.exclude_list;
-    const bool passes = decode && a.top_blocks <= kDecodeTop && plan.total <= kSmemDynamicLimit - kDecodeStatic;
+    // (single precision: two such CTAs per SM, three of the general form, which therefore holds more rows at once)
+    const bool passes = decode && a.top_blocks <= kDecodeTop && plan.total <= kSmemDynamicLimit - kDecodeStatic &&
+                        (dtype != RLM_F32 || a.n_rows <= 2 * a.sm_count);
     auto kernel = dtype == RLM_BF16 ? select_kernel<RLM_BF16>(many_rows, decode, passes, a.resident)
                   : dtype == RLM_F16 ? select_kernel<RLM_F16>(many_rows, decode, passes, a.resident)
-                  : dtype == RLM_F32 && decode ? (many_rows ? relation_select_kernel<4, RLM_F32, true> : relation_select_kernel<3, RLM_F32, true>)
-                                               : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
+                  : dtype == RLM_F32 ? select_kernel<RLM_F32>(many_rows, decode, passes, a.resident)
+                                     : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     launch_kernel(kernel, dim3(a.n_rows), dim3(kThreads), plan.total, stream, a);

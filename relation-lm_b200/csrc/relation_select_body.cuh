@@ -984,11 +984,11 @@ int prepare(SelectArgs& a, bool& many_rows, bool allow_resident = false) {
         a.plan = make_plan(a.n_blocks, a.block_size, a.local_window, a.top_blocks, a.buckets,
                            dtype_size(a.key_dtype), dtype_size(a.stats_dtype), a.mode, true);
     }
-    // At most one row per SM, decode form in one 16-bit dtype, caches that fit: stage the whole key caches
+    // At most one row per SM, decode form in one dtype, caches that fit: stage the whole key caches
     // (relation_select_decode_kernel)
     a.resident = 0;
     if (allow_resident && !many_rows && a.n_rows <= kSms && a.mode == kPacked && !a.row_batch && !a.row_position &&
-        !a.exclude_list && a.top_blocks > 0 && a.top_blocks <= kDecodeTop && a.query_dtype != RLM_F32 && a.key_dtype == a.query_dtype &&
+        !a.exclude_list && a.top_blocks > 0 && a.top_blocks <= kDecodeTop && a.key_dtype == a.query_dtype &&
         a.stats_dtype == a.query_dtype) {
         const Plan whole = make_plan(a.n_blocks, a.block_size, a.local_window, a.top_blocks, a.buckets,
                                      dtype_size(a.key_dtype), dtype_size(a.stats_dtype), a.mode, false, a.max_t);
