@@ -37,6 +37,8 @@ constexpr int kSplit = 4;          // thread groups along the relation dimension
 constexpr int kGroupThreads = 128;
 constexpr int kHiddenThreads = kSplit * kGroupThreads;
 constexpr int kMaxK = 16;          // partner slots per row
+constexpr int kFewThreads = 128;   // relation_hidden_few_kernel: threads per CTA, hidden columns per warp
+constexpr int kFewColumns = 4;
 constexpr int kPad = 4;            // row padding (floats) of staged weight tiles: conflict-free float4 reads
 
 struct HiddenArgs {
@@ -350,6 +352,137 @@ int launch_hidden_as(const HiddenArgs& a, void* stream) {
     return check_launch("relation_hidden_kernel");
 }
 
+// ---- a handful of sequences in single precision
+//
+// A decode step's launch of a few sequences is a chain: indices, gathered rows, a short product, GELU.  The tiled kernel
+// above walks it through shared memory (weight tiles, product matrix, partial sums: four block-wide barriers) and always
+// computes four sequences.  Here a warp owns four hidden columns and keeps its weight elements in registers, four relation
+// columns a lane, requested before the dependency wait; the operand products of a sequence are made in registers from rows
+// read straight from the cache, and the 32 sums over the lanes (eight partners x four columns) meet in a transposing
+// butterfly that leaves lane 8 c + k with column c of partner k: no shared memory, no barrier.
+template <bool kUpdate>
+__global__ void __launch_bounds__(kFewThreads) relation_hidden_few_kernel(const HiddenArgs a) {
+    const int lane = threadIdx.x & 31, R = a.rdim, H = a.hdim, K = a.k_out;
+    const int h0 = (blockIdx.x * (kFewThreads / 32) + (threadIdx.x >> 5)) * kFewColumns;
+    const bool in = 4 * lane < R;                        // lanes beyond the relation width hold zeros
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 wm[kFewColumns], wa[kFewColumns], wp[kFewColumns];
+#pragma unroll
+    for (int c = 0; c < kFewColumns; ++c) {
+        const bool live = in && h0 + c < H;
+        const size_t at = static_cast<size_t>(h0 + c) * R + 4 * lane;
+        wm[c] = wa[c] = wp[c] = zero;
+        if (live) wm[c] = *reinterpret_cast<const float4*>(static_cast<const float*>(a.product_weight) + at);
+        if (kUpdate && live) {
+            wa[c] = *reinterpret_cast<const float4*>(static_cast<const float*>(a.anchor_weight) + at);
+            wp[c] = *reinterpret_cast<const float4*>(static_cast<const float*>(a.partner_weight) + at);
+        }
+    }
+    // this lane's output: column `col` of partner `k`
+    const int k = lane & 7, col = h0 + (lane >> 3);
+    float bias = 0.0f;
+    if (kUpdate && col < H) bias = static_cast<const float*>(a.first_bias)[col];
+    int t = -1;
+    if (kUpdate) {
+        t = static_cast<int>(*a.position);
+        if (t < 0 || t >= a.max_t) {
+            if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && a.status) atomicOr(a.status, RLM_DEV_POSITION);
+            griddep_sync();      // here too: what is launched next relies on this kernel having waited for its predecessor
+            return;
+        }
+    }
+    griddep_sync();      // the weights are requested; indices and caches may come from the previous kernel
+    const bool live = k < K && col < H;
+    for (int row = blockIdx.y; row < a.n_rows; row += gridDim.y) {
+        // lane k: partner k's row; lane 8: the anchor's
+        int index = 0;
+        if (lane < K) index = a.partner_index[static_cast<size_t>(row) * K + lane];
+        else if (lane == 8) index = a.anchor_index[row];
+        index = min(max(index, 0), a.max_t - 1);
+        const int ai = __shfl_sync(0xffffffffu, index, 8), pi = __shfl_sync(0xffffffffu, index, k);
+        const size_t first = static_cast<size_t>(row) * a.max_t;
+        const float* operand = static_cast<const float*>(a.operand_cache) + first * R + 4 * lane;
+        float* expanded = static_cast<float*>(a.expanded_cache) + first * 2 * H;
+        float4 oa = zero, cur = zero, op[8];
+        if (in) oa = *reinterpret_cast<const float4*>(operand + static_cast<size_t>(ai) * R);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int p = __shfl_sync(0xffffffffu, index, i);
+            op[i] = zero;
+            if (in && i < K) op[i] = *reinterpret_cast<const float4*>(operand + static_cast<size_t>(p) * R);
+        }
+        if (kUpdate && in) cur = *reinterpret_cast<const float4*>(operand + static_cast<size_t>(t) * R);
+        // the position's own expanded row is being written by this launch: its terms come from the sums below
+        const bool fresh_a = kUpdate && ai == t, fresh_p = kUpdate && pi == t;
+        float base_a = 0.0f, base_p = 0.0f;
+        if (live && !fresh_a) base_a = expanded[static_cast<size_t>(ai) * 2 * H + col];
+        if (live && !fresh_p) base_p = expanded[static_cast<size_t>(pi) * 2 * H + H + col];
+        float y[32];                                     // [column][partner]
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 pr = make_float4(op[i].x * oa.x, op[i].y * oa.y, op[i].z * oa.z, op[i].w * oa.w);
+#pragma unroll
+            for (int c = 0; c < kFewColumns; ++c) y[8 * c + i] = dot4(wm[c], pr, 0.0f);
+        }
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            const int w = 16 >> s;
+            const bool upper = (lane & w) != 0;
+#pragma unroll
+            for (int i = 0; i < w; ++i) {
+                const float send = upper ? y[i] : y[i + w], keep = upper ? y[i + w] : y[i];
+                y[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+            }
+        }
+        if (kUpdate) {
+            float f[8];                                  // [anchor or partner half][column]
+#pragma unroll
+            for (int c = 0; c < kFewColumns; ++c) {
+                f[c] = dot4(wa[c], cur, 0.0f);
+                f[4 + c] = dot4(wp[c], cur, 0.0f);
+            }
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const int w = 4 >> s, bit = 16 >> s;
+                const bool upper = (lane & bit) != 0;
+#pragma unroll
+                for (int i = 0; i < w; ++i) {
+                    const float send = upper ? f[i] : f[i + w], keep = upper ? f[i + w] : f[i];
+                    f[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+                }
+            }
+            f[0] += __shfl_xor_sync(0xffffffffu, f[0], 2);
+            f[0] += __shfl_xor_sync(0xffffffffu, f[0], 1);       // lanes 16 half + 4 column + ...
+            const float row_a = __shfl_sync(0xffffffffu, f[0], 4 * (lane >> 3)) + bias;
+            const float row_p = __shfl_sync(0xffffffffu, f[0], 16 + 4 * (lane >> 3));
+            if (fresh_a) base_a = row_a;
+            if (fresh_p) base_p = row_p;
+            if (k < 2 && col < H) expanded[static_cast<size_t>(t) * 2 * H + k * H + col] = k == 0 ? row_a : row_p;
+        }
+        if (live) store_scalar(a.out, (static_cast<int64_t>(row) * K + k) * H + col, a.out_dtype, gelu_erf(y[0] + (base_a + base_p)));
+    }
+}
+
+// Where it is the faster one (us a launch in a graph, tiled kernel -> this one; K 8, R 128, H 4 d).  With the update: d 256,
+// 1 sequence 6.9 -> 2.5, 16 7.7 -> 6.7, 48 16.4 -> 15.0; d 576, 1 7.2 -> 2.8, 8 7.7 -> 6.2, 48 29.5 -> 26.5; d 768, 1 7.2 -> 3.1,
+// 6 10.6 -> 6.4, 48 39.3 -> 34.7.  Without it the tiled kernel stages a third of the weights: d 256, 1 4.6 -> 2.1,
+// 12 5.3 -> 4.4 (16 5.3 -> 5.7); d 512, 12 7.3 -> 7.0 (16 7.3 -> 8.8); d 768, 8 7.3 -> 6.4 (12 7.3 -> 8.9).
+bool hidden_few_applicable(const HiddenArgs& a, bool update) {
+    return a.cache_dtype == RLM_F32 && a.weight_dtype == RLM_F32 && !a.row_batch && a.k_out <= 8 && a.rdim <= 128 &&
+           (update ? a.n_rows <= 48 : a.n_rows <= 12 && a.n_rows * static_cast<int64_t>(a.hdim) <= 28800);
+}
+
+template <bool kUpdate>
+int launch_hidden_few(const HiddenArgs& a, void* stream) {
+    constexpr int kCtaColumns = kFewThreads / 32 * kFewColumns;
+    const int gx = (a.hdim + kCtaColumns - 1) / kCtaColumns;
+    int gy = (3 * sm_count() + gx - 1) / gx;             // three CTAs fit an SM; beyond that a CTA takes several sequences
+    if (gy > a.n_rows) gy = a.n_rows;
+    launch_kernel(relation_hidden_few_kernel<kUpdate>, dim3(gx, gy), dim3(kFewThreads), 0, stream, a);
+    count_launch();
+    return check_launch("relation_hidden_few_kernel");
+}
+
 int launch_hidden(HiddenArgs& a, bool update, void* stream) {
     if (a.n_rows == 0) return RLM_OK;
     if (!a.expanded_cache || !a.operand_cache || !a.anchor_index || !a.partner_index ||
@@ -382,6 +515,7 @@ int launch_hidden(HiddenArgs& a, bool update, void* stream) {
                                 a.anchor_weight, a.partner_weight, a.product_weight, a.first_bias,
                                 a.position, a.row_batch, a.out, a.n_rows, a.n_seq, a.max_t, a.rdim, a.hdim,
                                 a.k_out, a.cache_dtype, a.out_dtype, a.status, stream);
+    if (hidden_few_applicable(a, update)) return update ? launch_hidden_few<true>(a, stream) : launch_hidden_few<false>(a, stream);
     const bool wide = kRB * a.k_out > 32;      // more than 4 relation rows per thread
     if (update) return wide ? launch_hidden_as<true, 8>(a, stream) : launch_hidden_as<true, 4>(a, stream);
     return wide ? launch_hidden_as<false, 8>(a, stream) : launch_hidden_as<false, 4>(a, stream);
