@@ -1061,6 +1061,50 @@ Two single_precision_heads(const Tensor& normalized, const Tensor& token_weight,
     return {tokens, boundaries};
 }
 
+// ------------------------------------------------------------------ a whole-sequence layer, its operators in two groups
+//
+// One after the other from Python a short prompt's eight launches took the host longer than the device.
+
+// The state of sequences x [B, T, d]: what sequence_state leaves, the expanded cache, the packed rows.
+std::vector<Tensor> prefill_state(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps,
+                                  const Tensor& packed_weight, int64_t relation_dim, int64_t block_size,
+                                  const Tensor& anchor_conv_weight, const Tensor& partner_conv_weight,
+                                  const Tensor& expand_weight, const Tensor& expand_bias) {
+    const int64_t batch = x.size(0), length = x.size(1);
+    const Tensor rows = x.view({batch * length, x.size(2)});
+    Tensor memory = empty(rows.sizes(), packed_weight.scalar_type(), x.device());
+    layer_norm_cast(rows, norm_weight, norm_bias, norm_eps, memory);
+    const Tensor packed = packed_projection(memory, packed_weight, std::nullopt).view({batch, length, packed_weight.size(0)});
+    std::vector<Tensor> state = sequence_state(packed, 0, relation_dim, block_size, anchor_conv_weight, partner_conv_weight);
+    state.push_back(packed_projection(state[2].view({batch * length, relation_dim}), expand_weight, expand_bias)
+                        .view({batch, length, expand_weight.size(0)}));
+    state.push_back(packed);
+    return state;
+}
+
+// The layer's output [B, T, d] for residual inputs x and their state.
+Tensor prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps, const Tensor& query_weight,
+                     const Tensor& anchor_keys, const Tensor& anchor_mean, const Tensor& anchor_std, const Tensor& anchor_gamma,
+                     const Tensor& anchor_bias, const Tensor& partner_anchor_cache, const Tensor& partner_keys,
+                     const Tensor& partner_mean, const Tensor& partner_std, const Tensor& partner_gamma, const Tensor& partner_bias,
+                     int64_t local_window, int64_t top_blocks, int64_t k_out, bool strict_valid, const Tensor& expanded_cache,
+                     const Tensor& operand_cache, const Tensor& mix, const Tensor& product_weight, const Tensor& second_weight,
+                     const Tensor& second_bias, const Tensor& relation_norm_weight, const Tensor& relation_norm_bias) {
+    const int64_t batch = x.size(0), length = x.size(1), dim = x.size(2);
+    const Tensor rows = x.view({batch * length, dim});
+    Tensor normalized = empty(rows.sizes(), query_weight.scalar_type(), x.device());
+    layer_norm_cast(rows, norm_weight, norm_bias, norm_eps, normalized);
+    const Tensor q = packed_projection(normalized, query_weight, std::nullopt);
+    const auto [anchor, anchor_score, partner, score] = relation_select_packed_prefill(
+        q.narrow(1, 0, 64), anchor_keys, q.narrow(1, 64, 64), anchor_mean, anchor_std, anchor_gamma, anchor_bias, q.narrow(1, 128, 128),
+        partner_anchor_cache, partner_keys, partner_mean, partner_std, partner_gamma, partner_bias, length, local_window, top_blocks,
+        k_out, strict_valid);
+    Tensor out = empty(rows.sizes(), at::kFloat, x.device());
+    relation_mlp_rows(out, expanded_cache, operand_cache, anchor, partner, score, std::nullopt, std::nullopt, mix, product_weight,
+                      second_weight, second_bias, relation_norm_weight, relation_norm_bias, norm_eps, rows.contiguous(), 1, length, true);
+    return out.view({batch, length, dim});
+}
+
 // ------------------------------------------------------------------ what surrounds an operator
 
 using Stack = torch::jit::Stack;
@@ -1412,7 +1456,7 @@ PyMethodDef kMethods[] = {METHOD(relation_select_packed), METHOD(relation_select
                           METHOD(relation_norm_reduce), METHOD(relation_norm_reduce_residual_norm), METHOD(relation_mlp_rows),
                           METHOD(packed_projection), METHOD(layer_norm_cast), METHOD(decode_embed_norm), METHOD(few_rows_projection),
                           METHOD(few_rows_projection_pair), METHOD(single_precision_front), METHOD(single_precision_layer),
-                          METHOD(single_precision_heads),
+                          METHOD(single_precision_heads), METHOD(prefill_state), METHOD(prefill_layer),
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "librelation_lm_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -132,7 +132,7 @@ def sequence_state(packed: Tensor, slots: int, relation_dim: int, block_size: in
     launch (extension), keyed by ``STATE_NAMES``: the token caches, and what ``router_cache_prefill`` leaves of
     both router streams.  ``slots = 0``: one layer's column order (``W = 384 + R``), caches ``[B, T, width]``;
     ``slots = S``: ``S`` slots of 384 columns, then the operand, slot caches ``[S, B, T, width]``."""
-    if block_size > _STATE_BLOCK:
+    if not sequence_state_in_one_launch(block_size):
         return _sequence_state_by_parts(packed, slots, relation_dim, block_size, anchor_conv_weight, partner_conv_weight)
     return dict(zip(STATE_NAMES, _sequence_state(packed, slots, relation_dim, block_size, anchor_conv_weight,
                                                  partner_conv_weight)))
@@ -141,6 +141,10 @@ def sequence_state(packed: Tensor, slots: int, relation_dim: int, block_size: in
 # Positions of the largest block whose router rows, with two rows of history, and convolved rows the kernel can hold in
 # shared memory: (2 n + 2) rows of 256 bytes in 226 KB.  Longer blocks are copied and walked in device memory.
 _STATE_BLOCK = 451
+
+
+def sequence_state_in_one_launch(block_size: int) -> bool:
+    return block_size <= _STATE_BLOCK
 
 
 def _sequence_state_by_parts(packed: Tensor, slots: int, relation_dim: int, block_size: int, anchor_conv_weight: Tensor,
