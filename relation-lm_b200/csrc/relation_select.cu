@@ -171,6 +171,14 @@ __device__ __forceinline__ Chunk<kDt> load_chunk(const unsigned char* p) {
     else return *reinterpret_cast<const uint4*>(p);
 }
 
+// Two values of the 16-bit type kDt, from fp32 (exact).
+template <int kDt>
+__device__ __forceinline__ uint32_t pack_exact(float lo, float hi) {
+    if (kDt == RLM_BF16) return (__float_as_uint(lo) >> 16) | (__float_as_uint(hi) & 0xffff0000u);
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // This lane's chunk of a query, every element twice: operands of the two-wide fma over two rows.
 struct QueryChunk { float2 v[8]; };
 
@@ -184,6 +192,60 @@ __device__ __forceinline__ void load_query_chunk(const float* query, QueryChunk&
         q.v[4 * h + 2] = make_float2(x.z, x.z);
         q.v[4 * h + 3] = make_float2(x.w, x.w);
     }
+}
+
+__device__ __forceinline__ QueryChunk magnitude(const QueryChunk& q) {
+    QueryChunk m;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) m.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
+    return m;
+}
+
+// The chunk of a query whose values are kDt's own (the anchor stream's: a partner query is a sum, rounded to fp32), as
+// they lie: the mixed-precision fma takes both factors in 16 bits, widens them exactly and rounds once, the same sums
+// as of widened rows in two thirds of the instructions (16 instead of 24 for two rows' chunks; 0.54 against 0.68 ms for
+// 19 G of them on all SMs).  A multi-anchor pass, us: 16 x 2048 rows of four slots, four layers 11 440 -> 11 270,
+// 3 x 1056 rows of two slots, two layers 260 -> 256.
+template <int kDt>
+struct NarrowChunk { uint32_t v[4]; };
+
+template <int kDt>
+__device__ __forceinline__ void load_query_chunk(const float* query, NarrowChunk<kDt>& q) {
+    const float* src = query + 8 * (threadIdx.x & 7);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float4 x = *reinterpret_cast<const float4*>(src + 4 * h);
+        q.v[2 * h] = pack_exact<kDt>(x.x, x.y);
+        q.v[2 * h + 1] = pack_exact<kDt>(x.z, x.w);
+    }
+}
+
+template <int kDt>
+__device__ __forceinline__ NarrowChunk<kDt> magnitude(const NarrowChunk<kDt>& q) {
+    NarrowChunk<kDt> m;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m.v[e] = q.v[e] & 0x7fff7fffu;
+    return m;
+}
+
+// acc + the lower (upper) halves' product, rounded once
+template <int kDt>
+__device__ __forceinline__ float fma_lower(uint32_t a, uint32_t b, float acc) {
+    float d;
+    if (kDt == RLM_BF16)
+        asm("{.reg .b16 x, y, u, v; mov.b32 {x, y}, %1; mov.b32 {u, v}, %2; fma.rn.f32.bf16 %0, x, u, %3;}" : "=f"(d) : "r"(a), "r"(b), "f"(acc));
+    else
+        asm("{.reg .b16 x, y, u, v; mov.b32 {x, y}, %1; mov.b32 {u, v}, %2; fma.rn.f32.f16 %0, x, u, %3;}" : "=f"(d) : "r"(a), "r"(b), "f"(acc));
+    return d;
+}
+template <int kDt>
+__device__ __forceinline__ float fma_upper(uint32_t a, uint32_t b, float acc) {
+    float d;
+    if (kDt == RLM_BF16)
+        asm("{.reg .b16 x, y, u, v; mov.b32 {x, y}, %1; mov.b32 {u, v}, %2; fma.rn.f32.bf16 %0, y, v, %3;}" : "=f"(d) : "r"(a), "r"(b), "f"(acc));
+    else
+        asm("{.reg .b16 x, y, u, v; mov.b32 {x, y}, %1; mov.b32 {u, v}, %2; fma.rn.f32.f16 %0, y, v, %3;}" : "=f"(d) : "r"(a), "r"(b), "f"(acc));
+    return d;
 }
 
 // Element pair i of the chunks of two rows, (lower halves, upper halves), widened to fp32 (exact).
@@ -223,6 +285,20 @@ __device__ __forceinline__ float2 seg_pair(const Chunk<kDt> w0, const Chunk<kDt>
     }
 }
 
+template <int kDt>
+__device__ __forceinline__ float2 seg_pair(const uint4 w0, const uint4 w1, const NarrowChunk<kDt>& q) {
+    const uint32_t a[4] = {w0.x, w0.y, w0.z, w0.w}, b[4] = {w1.x, w1.y, w1.z, w1.w};
+    float x = 0.0f, y = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x = fma_lower<kDt>(a[i], q.v[i], x);
+        y = fma_lower<kDt>(b[i], q.v[i], y);
+        x = fma_upper<kDt>(a[i], q.v[i], x);
+        y = fma_upper<kDt>(b[i], q.v[i], y);
+    }
+    return make_float2(x, y);
+}
+
 // One level of the butterfly over the chunk lanes: of kN values (a row each) a lane keeps those whose index has the
 // parity of its lane bit, adds the partner's halves of them and hands over its own halves of the others.
 template <int kN, int kXor>
@@ -236,8 +312,8 @@ __device__ __forceinline__ void fold_level(const float (&s)[kN], float (&out)[kN
 }
 
 // Chunk sums of rows load(0) .. load(kN - 1) (row i: rows 4 i + rq of a pass), two rows at a time.
-template <int kDt, int kN, typename Load>
-__device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q, float (&s)[kN]) {
+template <int kDt, int kN, typename Load, typename Query>
+__device__ __forceinline__ void chunk_sums(const Load& load, const Query& q, float (&s)[kN]) {
     constexpr int kStep = kN < 4 ? kN : 4;
 #pragma unroll
     for (int h = 0; h < kN; h += kStep) {
@@ -256,8 +332,8 @@ __device__ __forceinline__ void chunk_sums(const Load& load, const QueryChunk& q
 // Score of the row that this lane owns after the butterfly: row 4 (chunk mod kN) + rq of a pass of 4 kN rows (with
 // fewer than eight rows per lane group, lanes own rows in common).  A pass of 32 rows costs the least per row; one of
 // 16 or 8 ends sooner, where warps are idle.
-template <int kDt, int kN, typename Load>
-__device__ __forceinline__ float pass_score(const Load& load, const QueryChunk& q) {
+template <int kDt, int kN, typename Load, typename Query>
+__device__ __forceinline__ float pass_score(const Load& load, const Query& q) {
     float s[kN], total;
     chunk_sums<kDt, kN>(load, q, s);
     if constexpr (kN == 8) {
@@ -320,9 +396,9 @@ __device__ __forceinline__ void keep_best(bool valid, float score, int pos, uint
 // The local window, staged in shared memory: row r is position pos0 + r; rows below first_valid are none (and
 // not staged).  Scores go to cand[slot0 + r], or, without cand, into the running
 // best (kBoth: to both).
-template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8>
+template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8, typename Query>
 __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int n_rows, int first_valid, int pos0, int exclude,
-                                                  const QueryChunk& q, float* cand, int slot0, uint32_t& best_key,
+                                                  const Query& q, float* cand, int slot0, uint32_t& best_key,
                                                   int& best_pos, const ExclRegs* ex = nullptr, int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     uint32_t my_key = 0;
@@ -351,9 +427,9 @@ __device__ __forceinline__ void score_window_warp(const unsigned char* rows, int
 }
 
 // The picked remote blocks (sel: block, picked, rows), scored where they lie in the key cache.
-template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8>
+template <int kDt, bool kExcl = false, bool kBoth = false, int kN = 8, typename Query>
 __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int n_rows, const int* sel, int bs,
-                                                  int bs_shift, int exclude, const QueryChunk& q, float* cand, int slot0,
+                                                  int bs_shift, int exclude, const Query& q, float* cand, int slot0,
                                                   uint32_t& best_key, int& best_pos, const ExclRegs* ex = nullptr,
                                                   int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
@@ -397,16 +473,14 @@ __device__ __forceinline__ void score_remote_warp(const unsigned char* keys, int
 // first butterfly level completes a head's sums; a 4 x 4 transpose between the head lanes then leaves every lane
 // with the four heads of one block.  out[n] for the first n_complete blocks, -inf up to the next multiple of four
 // of nb.
-template <int kDt>
+template <int kDt, typename Query>
 __device__ __forceinline__ void score_blocks_warp(const unsigned char* mean, const unsigned char* stdv, int nb, int n_complete,
-                                                  int bs, int t, int ls, int strict, int buckets, const QueryChunk& q,
+                                                  int bs, int t, int ls, int strict, int buckets, const Query& q,
                                                   const float* sp4, const float* bias, float* out, int first = 0, int step = 1) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
     if (first == 0)
         for (int n = n_complete + lane; n < ((nb + 3) & ~3); n += 32) out[n] = kNegInf;
-    QueryChunk qa;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
+    const auto qa = magnitude(q);
     const float sp = sp4[chunk >> 1];
     const bool x2 = lane & 2, x4 = lane & 4;
     for (int base = 32 * first; base < n_complete; base += 32 * step) {
@@ -465,9 +539,7 @@ __device__ __forceinline__ void score_eight_blocks(const unsigned char* mean, co
                                                    int bs, int ls, int strict, const QueryChunk& q, float sp, float shift,
                                                    float* out) {
     const int lane = threadIdx.x & 31, chunk = lane & 7, rq = lane >> 3;
-    QueryChunk qa;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) qa.v[e] = make_float2(fabsf(q.v[e].x), fabsf(q.v[e].y));
+    const auto qa = magnitude(q);
     float sums[2], md[1], sd[1];
     const auto at = [&](int i) { return static_cast<uint32_t>(min(first + 4 * i + rq, n_complete - 1)) * kRowOf<kDt> + kRowOf<kDt> / 8 * chunk; };
     chunk_sums<kDt, 2>([&](int i) { return load_chunk<kDt>(mean + at(i)); }, q, sums);
@@ -982,7 +1054,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, (kDt == RLM_F32 ? 16 : 32) / 
         uint32_t bk = 0;
         int bp = 0x7fffffff;
         if constexpr (kFast) {
-            QueryChunk q;
+            NarrowChunk<kDt> q;
             if (top > 0) {
                 load_query_chunk(arq, q);
                 score_blocks_warp<kDt>(st(0), st(1), nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q,
@@ -1191,7 +1263,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 32 / kTileWarps) relation_sel
 #pragma unroll
                 for (int x = 0; x < kMaxExclude; ++x) ex.v[x] = x < s ? mine[x] : -1;
                 __syncwarp();
-                QueryChunk q;
+                NarrowChunk<kDt> q;
                 if (top > 0) {
                     load_query_chunk(queries + kD, q);
                     score_blocks_warp<kDt>(st_mean, st_std, nb, n_complete, bs, t, ls, a.strict_valid, a.buckets, q, sp,
