@@ -67,6 +67,10 @@ constexpr uint32_t kMlpBlock = kBM * 128u;       // a 128 x 64 16-bit block
 constexpr int kMlpMaxStages = 4;
 constexpr int kMlpHidden = 2;                    // hidden blocks in flight per part
 constexpr int kMlpMaxTerms = 4;                  // gathered blocks in flight
+// Tiles whose marks (anchors that are not finite) have slots of their own.  A slot is cleared with the rows of the tile
+// before its next one, a moment that knows the epilogue only to be past the tile five before: the first layer, which
+// paces the rows, runs ahead of a tile's last stage, where the marks are read.
+constexpr int kMlpMarks = 8;
 
 struct MlpArgs {
     const void* expanded_cache;      // [B, T, 2H]
@@ -120,7 +124,7 @@ __host__ __device__ inline MlpPlan mlp_plan(int rdim, int cols, int outs, int wi
     p.beta = off;   off += static_cast<uint32_t>(cols) * 4u;
     p.stats = off;  off += static_cast<uint32_t>(4 * outs) * kBM * 8u;
     p.u = off;      off += 3u * kBM * 4u;
-    p.poison = off; off += 4u * (kBM >> k_shift) * 4u;
+    p.poison = off; off += static_cast<uint32_t>(kMlpMarks) * (kBM >> k_shift) * 4u;
     p.prow = off;   off += 2u * kBM * 4u;
     p.arow = off;   off += 4u * (kBM >> k_shift) * 4u;
     p.total = off;
@@ -432,7 +436,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
     float* u_s = reinterpret_cast<float*>(base + plan.u);
     int* prow_s = reinterpret_cast<int*>(base + plan.prow);
     int* arow_s = reinterpret_cast<int*>(base + plan.arow);
-    float* poison_s = reinterpret_cast<float*>(base + plan.poison);      // [four tiles in turn][anchor]: 0, or NaN for one that is not finite
+    float* poison_s = reinterpret_cast<float*>(base + plan.poison);      // [kMlpMarks tiles in turn][anchor]: 0, or NaN for one that is not finite
 
     if (tid == 0) {
         failed_s = 0;
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
         gamma_s[i] = a.norm_w[o * NC + i];
         beta_s[i] = a.norm_b[o * NC + i];
     }
-    for (int i = tid; i < 4 * anchors; i += kMlpThreads) poison_s[i] = 0.0f;
+    for (int i = tid; i < kMlpMarks * anchors; i += kMlpThreads) poison_s[i] = 0.0f;
     const uint16_t one = kDt == RLM_BF16 ? 0x3f80 : 0x3c00;
     for (int i = tid; i < kBM * sel_k / 8; i += kMlpThreads) {          // one-hot rows: K-chunk major core matrices, no swizzle
         const int c = i / kBM, r = i - c * kBM;
@@ -611,7 +615,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
             }
             const float inv_quarter = 1.0f / static_cast<float>(quarter);
             // (a row whose anchor is not finite becomes NaN here, and through the statistics in every output part)
-            const float mean_q = fmaf(s1, inv_quarter, shift) + *static_cast<volatile float*>(poison_s + (tix & 3) * anchors + (row >> a.k_shift));
+            const float mean_q = fmaf(s1, inv_quarter, shift) + *static_cast<volatile float*>(poison_s + (tix & (kMlpMarks - 1)) * anchors + (row >> a.k_shift));
             const float m2 = fmaf(-s1 * inv_quarter, s1, s2);
             // every CTA of the tile receives (mean, sum of squares) of all quarters
             float2* mine = stats_s + (o * 4 + q) * kBM + row;
@@ -866,7 +870,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                         *reinterpret_cast<uint4*>(base + plan.anc + static_cast<uint32_t>(ts) * anc_stage + anchor_to + 2048u * i) = ahead[i];
                     }
                     if (n + 1 < 2 * U) request_anchors(n + 1);
-                    else if (bad) mlp_mark(smem_u32(poison_s + (tix & 3) * anchors), leader, anchors, gt >> 2, bad);
+                    else if (bad) mlp_mark(smem_u32(poison_s + (tix & (kMlpMarks - 1)) * anchors), leader, anchors, gt >> 2, bad);
                     mlp_cp_async_arrive(smem_u32(&bars.term_full[ts]));
                 }
                 __syncwarp();                                 // the warp's stores -> its one arrival for them
@@ -900,9 +904,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) relation_mlp_rows_kernel(
                     arow = srow / a.slots / a.rows_per_seq * a.max_t + min(max(a.anchor_index[srow], 0), a.max_t - 1);
                 arow_s[b * sel_k + gt] = arow;
             }
-            // the next tile's marks, last read three tiles ago; nothing of that tile is gathered before this one is announced
+            // The next tile's marks: the slot was the tile's seven before this one, which the epilogue has read (`weights` of
+            // two tiles ago waited for the tile five before); nothing of the next tile is gathered before this one is announced.
             ++made;
-            if (gt < anchors) poison_s[(made & 3) * anchors + gt] = 0.0f;
+            if (gt < anchors) poison_s[(made & (kMlpMarks - 1)) * anchors + gt] = 0.0f;
             __syncwarp();
             if (ok && lane == 0) mlp_arrive(smem_u32(&bars.rows_full[b]));
         };

@@ -151,6 +151,44 @@ def test_a_cache_row_that_is_not_finite_reaches_the_rows_that_selected_it(dtype,
             assert torch.equal(out[~hit], before[~hit])
 
 
+# The shapes of test_few_hidden_units_and_many_tiles with eight tiles or more for every cluster (74 of two CTAs, 33 of
+# four): a tile's marks are read in its last stage, when the rows of tiles three ahead have been announced.
+@pytest.mark.parametrize("value", (torch.inf, torch.nan))
+@pytest.mark.parametrize("batch,slots,k,rdim,d,hidden", [
+    (93, 4, 8, 64, 64, 256), (93, 4, 8, 64, 64, 384), (93, 2, 16, 128, 256, 256), (42, 4, 8, 128, 512, 512),
+    (42, 4, 8, 64, 512, 768), (93, 4, 8, 64, 384, 256), (42, 4, 8, 128, 768, 512), (42, 4, 8, 64, 768, 768),
+])
+def test_anchors_that_are_not_finite_in_every_tile_of_a_cluster(value, batch, slots, k, rdim, d, hidden):
+    from relation_lm.kernels.relation_reduce import relation_mlp_rows
+
+    length = 53
+    x = _case(torch.bfloat16, batch, length, slots, k, rdim, d, d + hidden, hidden)
+    # a pair of tiles is eight rows: the first of each selects both of the rows that will not be finite
+    x["anchor"][::8, :2] = torch.tensor([17, 40], device="cuda", dtype=torch.int32)
+    x["active"][::8, :2] = True
+    x["score"][::8, :2, 0] = 1.0
+
+    def run(expanded):
+        out = torch.empty_like(x["residual"])
+        relation_mlp_rows(out, expanded, x["operand"], x["anchor"], x["partner"], x["score"], x["active"], x["slot_weight"], x["scale"],
+                          x["wm"], x["w2"], x["b2"], x["nw"], x["nb"], 1e-5, x["residual"], slots, length, False)
+        assert_status_clear()
+        return out
+
+    before = run(x["expanded"])
+    assert bool(before.isfinite().all())
+    anchor = x["anchor"].clamp(0, length - 1)
+    used = torch.isfinite(x["score"]).any(-1) & x["active"]                  # [row, slot]: some pair has a weight
+    for row, column in ((17, 0), (40, hidden - 1)):
+        expanded = x["expanded"].clone()
+        expanded[:, row, column] = value
+        hit = ((anchor == row) & used).any(1)
+        assert bool(hit[::8].all())
+        out = run(expanded)
+        assert bool(out[hit].isnan().all())
+        assert torch.equal(out[~hit], before[~hit])
+
+
 def test_new_output_without_residual_or_scale():
     from relation_lm.kernels.relation_reduce import relation_mlp_rows
 
