@@ -942,7 +942,7 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         }
         // more partners than candidates
         for (int k = cap + tid; k < K; k += kThreads) { out_pos[k] = t - L + 1; out_score[k] = kNegInf; }
-    } else if (cap4 > 512) {
+    } else if (cap4 > 512 || kDt == RLM_F32) {       // (fp32: the position of a score that is NaN, as select_row)
         topk_large(cand, cap, K, L, t, bs, sel_s, out_pos, out_score);
     } else if (warp == 0) {
         topk_warp(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);

@@ -592,14 +592,18 @@ __device__ __noinline__ void topk_large(float* cand, int cap, int K, int L, int 
 // one pass.  Lane l holds the scores of blocks l, l + 32, ...; each of the `top` rounds takes
 // the best remaining block of the warp (two redux instructions; ties to the lowest index) and
 // hands it to lane `round`, which then requests its own block, after lane 0 has posted the byte
-// count of all of them.  Same result as pick_blocks + issue_remote.
+// count of all of them.  Same result as pick_blocks + issue_remote: a block whose score is NaN is no choice, as in every
+// other form (taken by its key it would come before all others and end the choice).
 __device__ __noinline__ void pick_and_issue(const float* scores, int nb, int top, int bs, int ls, int* sel,
                                             const unsigned char* keys, unsigned char* dst, size_t key_row,
                                             size_t seq_keys, uint32_t bar) {
     const int lane = threadIdx.x & 31;
     uint32_t k[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) k[i] = lane + 32 * i < nb ? float_key(scores[lane + 32 * i]) : 0u;
+    for (int i = 0; i < 4; ++i) {
+        const float v = lane + 32 * i < nb ? scores[lane + 32 * i] : kNegInf;
+        k[i] = v > -1.0e30f ? float_key(v) : 0u;
+    }
     int my_block = 0, my_rows = 0;
     for (int r = 0; r < top; ++r) {
         uint32_t bk = 0;
@@ -608,7 +612,7 @@ __device__ __noinline__ void pick_and_issue(const float* scores, int nb, int top
         for (int i = 0; i < 4; ++i)
             if (k[i] > bk) { bk = k[i]; bn = lane + 32 * i; }
         warp_argmax_key(bk, bn);
-        if (!(key_float(bk) > -1.0e30f)) break;          // no usable block is left
+        if (bk == 0u) break;                             // no usable block is left
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (lane + 32 * i == bn) k[i] = 0u;

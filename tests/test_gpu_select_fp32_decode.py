@@ -77,6 +77,28 @@ def test_caches_with_values_that_are_not_finite(B, T, NB, L, top, K):
     assert_status_clear()
 
 
+# blocks a lane each, four a lane, blocks ranked against one another; up to 256 candidates, 320 and 552
+@pytest.mark.parametrize("B,T,NB,L,top,K", [SHAPES[i] for i in (0, 2, 3, 4, 6, 7)])
+@pytest.mark.parametrize("where", ["statistics", "keys", "both"])
+def test_scores_that_are_nan_rank_as_in_the_rows_form(B, T, NB, L, top, K, where):
+    from relation_lm.kernels.relation_select import relation_select_packed, relation_select_packed_rows
+
+    args = [x.clone() for x in select_args(to_cuda(cases.make_inputs(_case(B, T, NB, L, top, K))))]
+    for i in (1, 9):
+        if where != "statistics":
+            args[i][:, 5::37, 5] = float("nan")
+    for i in (3, 10):
+        if where != "keys":
+            args[i].view(B, NB, -1)[:, 2::7] = float("nan")
+    rows = torch.arange(B, dtype=torch.int32).cuda()
+    for t in _positions(T, NB, L):
+        got = relation_select_packed(*args, position_tensor(t), L, top, K, False)
+        ref = relation_select_packed_rows(*args, rows, torch.full_like(rows, t), L, top, K, False)
+        for a, b in zip(got, ref):
+            assert _equal(a, b), t
+    assert_status_clear()
+
+
 def test_strided_queries_and_query_views_off_16_bytes():
     """Queries as columns of one matrix whose rows start anywhere, as a step hands them over."""
     from relation_lm.kernels.relation_select import relation_select_packed
