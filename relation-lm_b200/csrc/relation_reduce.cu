@@ -463,21 +463,31 @@ __global__ void __launch_bounds__(kFewThreads) relation_hidden_few_kernel(const 
     }
 }
 
-// Where it is the faster one (us a launch in a graph, tiled kernel -> this one; K 8, R 128, H 4 d).  With the update: d 256,
-// 1 sequence 6.9 -> 2.5, 16 7.7 -> 6.7, 48 16.4 -> 15.0; d 576, 1 7.2 -> 2.8, 8 7.7 -> 6.2, 48 29.5 -> 26.5; d 768, 1 7.2 -> 3.1,
-// 6 10.6 -> 6.4, 48 39.3 -> 34.7.  Without it the tiled kernel stages a third of the weights: d 256, 1 4.6 -> 2.1,
-// 12 5.3 -> 4.4 (16 5.3 -> 5.7); d 512, 12 7.3 -> 7.0 (16 7.3 -> 8.8); d 768, 8 7.3 -> 6.4 (12 7.3 -> 8.9).
+// Where it is the faster one: sequences times hidden width up to a line that rises with the relation width (a lane holds
+// four of 128 relation columns whatever the width, while the tiled kernel's work falls with it; the partners, one to
+// eight, hardly matter).  us a launch in a graph, tiled kernel -> this one, K 8.  With the update, R 128: d 256, 1 sequence
+// 7.1 -> 2.7, 48 7.8 -> 5.1; H 1024, 32 11.3 -> 9.4; H 2304, 8 7.9 -> 6.4, 48 29.7 -> 26.7; H 3072, 12 11.3 -> 10.6, 48 39.9 -> 34.8.
+// R 96: 32 x 1024 9.7 -> 9.2, 16 x 2304 9.9 -> 10.4; R 64: 24 x 1024 8.0 -> 7.2, 12 x 2304 8.0 -> 8.3; R 32: 12 x 1024
+// 5.4 -> 5.0, 16 x 1024 5.3 -> 5.9; R 16: 48 x 256 5.0 -> 4.9, 32 x 1024 6.3 -> 9.0.  Without it the tiled kernel stages a third
+// of the weights; R 128: 1 x 1024 4.9 -> 2.4, 8 x 3072 7.4 -> 6.5, 12 x 2304 7.4 -> 7.2 (K 1 7.0 -> 7.4); R 64: 4 x 3072
+// 4.4 -> 4.3, 8 x 2304 4.5 -> 5.4; R 16: 4 x 2304 3.6 -> 3.5, 12 x 1024 3.7 -> 4.4.
 bool hidden_few_applicable(const HiddenArgs& a, bool update) {
+    const int64_t columns = a.n_rows * static_cast<int64_t>(a.hdim);
+    const int64_t most = a.rdim == 128 ? (update ? 147456 : 24576) : a.rdim >= 96 ? (update ? 32768 : 12288)
+                         : a.rdim >= 64 ? (update ? 24576 : 12288) : (update ? 12288 : 9216);
     return a.cache_dtype == RLM_F32 && a.weight_dtype == RLM_F32 && !a.row_batch && a.k_out <= 8 && a.rdim <= 128 &&
-           (update ? a.n_rows <= 48 : a.n_rows <= 12 && a.n_rows * static_cast<int64_t>(a.hdim) <= 28800);
+           a.n_rows <= (update ? 48 : 12) && columns <= most;
 }
 
 template <bool kUpdate>
 int launch_hidden_few(const HiddenArgs& a, void* stream) {
     constexpr int kCtaColumns = kFewThreads / 32 * kFewColumns;
     const int gx = (a.hdim + kCtaColumns - 1) / kCtaColumns;
-    int gy = (3 * sm_count() + gx - 1) / gx;             // three CTAs fit an SM; beyond that a CTA takes several sequences
+    // Four CTAs fit an SM with the update's 128 registers; what would not run at once, a CTA takes as further sequences
+    // (us, three CTAs -> four: 24 x 1024 8.9 -> 7.7, 32 x 1024 11.2 -> 9.4; R 128, K 8.  Other sizes within 2 %).
+    int gy = 4 * sm_count() / gx;
     if (gy > a.n_rows) gy = a.n_rows;
+    if (gy < 1) gy = 1;
     launch_kernel(relation_hidden_few_kernel<kUpdate>, dim3(gx, gy), dim3(kFewThreads), 0, stream, a);
     count_launch();
     return check_launch("relation_hidden_few_kernel");

@@ -51,6 +51,9 @@ def _reference(x, t, update):
     (1, 128, 128, 1024, 8), (1, 40, 16, 37, 1), (3, 64, 48, 130, 5), (7, 96, 128, 2304, 8), (2, 32, 64, 64, 4),
     (12, 64, 128, 2304, 8), (33, 64, 128, 256, 8), (48, 32, 128, 3072, 3), (49, 32, 128, 64, 8), (2, 32, 144, 96, 8),
     (2, 32, 128, 96, 9),
+    # both sides of the lines of sequences x hidden width (with the update | without) for narrower relations
+    (12, 32, 96, 1024, 4), (13, 32, 96, 1024, 4), (32, 32, 96, 1024, 2), (33, 32, 96, 1024, 2), (24, 32, 64, 1024, 8), (25, 32, 64, 1024, 8),
+    (9, 32, 32, 1024, 8), (10, 32, 32, 1024, 8), (12, 32, 16, 1024, 1), (13, 32, 16, 1024, 1), (12, 32, 128, 2048, 8), (12, 32, 128, 2052, 8),
 ])
 def test_against_64_bits(B, T, R, H, K, update):
     from relation_lm.kernels.relation_reduce import relation_hidden_cache_update, relation_hidden_cached
