@@ -7,15 +7,16 @@
 // contiguous bytes of one row, and keep kRows x kCols partial sums that are added over the lanes once, at the
 // end, by exchanges that halve the number of sums a lane holds.  The warps of a CTA that share columns split K
 // in steps of 128 and add up through shared memory in a fixed order: results do not depend on timing.  No shared
-// memory is filled first: a weight row is used by one warp, and so is, within a CTA, an x segment.
-// More rows go in passes of sixteen (or eight) over the same columns: on CTAs of their own, or, where there are columns
-// enough, one after the other in a CTA, whose weights then come from L1.
+// memory is filled first: a weight row is used by one warp of a CTA, and so is an x segment.
+// More rows go in passes of sixteen (or eight) over the same columns: one after the other in a CTA, whose weights come
+// from L1 in all but the first, or each on a CTA of its own, whose weights then come from L2.
 //
-// What bounds it: M = 8 B rows of the second relation-MLP layer move M * K * 4 bytes of x into every CTA, which is
-// more than the weights from 16 rows on, though what counts there is how many passes are in flight; the heads and the packed projection are the weights' stream from DRAM (one
-// row, 768 x 16256: 4.1 of 6.5 TB/s).  us a launch in a graph over weights that exceed the L2, cuBLAS (with its split-K
+// What bounds it: the passes of a CTA move kRows * K * 4 bytes of x each, from 16 rows on more than its weights (M = 8 B
+// rows of the second relation-MLP layer), but what counts there is how many passes are in flight; the heads and the packed
+// projection are the weights' stream from DRAM (one row, 768 x 16256: 4.1 of 6.5 TB/s).  us a launch in a graph over weights
+// that exceed the L2, cuBLAS (with its split-K
 // reduction) -> here, and the error against 64 bits: 8 x 3072 x 768 23.6 -> 5.7 (2.3e-7 -> 1.1e-7), 32 x 2048 x 512
-// 18.6 -> 6.0 (3.2e-7 -> 1.0e-7), 64 x 3072 x 768 33.2 -> 20.1, 4 x 512 x 256 4.3 -> 2.3, 2 x 512 x 3072 5.7 -> 2.8,
+// 18.6 -> 6.3 (3.2e-7 -> 1.0e-7), 64 x 3072 x 768 33.2 -> 19.8, 4 x 512 x 256 4.3 -> 2.3, 2 x 512 x 3072 5.7 -> 2.8,
 // 1 x 512 x 16256 17.6 -> 8.4, 8 x 768 x 16256 27.8 -> 22.8.
 // The first step's weights are requested before the dependency wait: parameters, which no kernel of the step writes.
 //
@@ -39,19 +40,19 @@ struct FewRowsArgs {
     int n0, n1;
     int rows, k;
     int k_parts;                                // warps that share columns
-    int row_parts;                              // CTAs that share columns: each takes every row_parts-th pass of rows
 };
 
 // kRows rows at a time, kCols columns per warp.  Fewer rows leave registers for more CTAs on an SM, whose loads are what
 // a stream needs (one row, 512 x 16256: 11.7 us with two CTAs, 8.4 with four).  Under those caps <4, *> and <2, 4> spill
 // 4 to 20 bytes.
-template <int kRows, int kCols>
+// kApart: a pass of kRows rows per CTA (x; y: the columns), else a CTA makes all passes over its columns (x).
+template <int kRows, int kCols, bool kApart>
 __global__ void __launch_bounds__(kFewThreads, kRows <= 2 ? 4 : kRows <= 4 ? 3 : 2) few_rows_projection_kernel(const FewRowsArgs a) {
     constexpr int kSums = kRows * kCols;
     __shared__ float part_s[kFewWarps][kSums];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int groups = kFewWarps / a.k_parts, part = warp % a.k_parts, group = warp / a.k_parts;
-    const int tile = blockIdx.x / a.row_parts * groups * kCols, first_row = blockIdx.x % a.row_parts * kRows, n_all = a.n0 + a.n1;
+    const int tile = (kApart ? blockIdx.y : blockIdx.x) * groups * kCols, n_all = a.n0 + a.n1;
     const int steps = (a.k + kFewStep - 1) / kFewStep;
 
     const float* wrow[kCols];
@@ -69,7 +70,7 @@ __global__ void __launch_bounds__(kFewThreads, kRows <= 2 ? 4 : kRows <= 4 ? 3 :
     griddep_sync();
 
 #pragma unroll 1
-    for (int m0 = first_row; m0 < a.rows; m0 += a.row_parts * kRows) {
+    for (int m0 = kApart ? blockIdx.x * kRows : 0; m0 < a.rows; m0 += kApart ? a.rows : kRows) {
         int xrow[kRows];                        // rows beyond the last repeat it (and are not stored)
 #pragma unroll
         for (int m = 0; m < kRows; ++m) xrow[m] = min(m0 + m, a.rows - 1) * a.x_stride;
@@ -151,14 +152,16 @@ int few_rows_tiles(const FewRowsArgs& a) {
 }
 
 template <int kRows, int kCols>
-int launch_few_rows(const FewRowsArgs& args, void* stream) {
-    FewRowsArgs a = args;
-    const int tiles = few_rows_tiles<kCols>(a);
-    // Passes over rows on CTAs of their own where the columns alone do not fill the SMs (two CTAs each): a pass is a few
-    // dependent loads long, not a stream (us: 32 x 1024 x 256 3.9 -> 3.3, 32 x 2304 x 576 10.2 -> 7.4, 64 x 2304 x 576 17.2 -> 13.5,
-    // 48 x 3072 x 768 19.5 -> 14.7; the same sums in the same order).
-    a.row_parts = tiles <= 2 * sm_count() ? (a.rows + kRows - 1) / kRows : 1;
-    launch_kernel(few_rows_projection_kernel<kRows, kCols>, dim3(tiles * a.row_parts), dim3(kFewThreads), 0, stream, a);
+int launch_few_rows(const FewRowsArgs& a, void* stream) {
+    // Passes over rows on CTAs of their own where that makes fewer waves (two CTAs an SM) than a CTA would make passes: a pass
+    // is a few dependent loads long, not a stream; where the columns fill the SMs, further passes find their weights in L1.
+    // us: 32 x 1024 x 256 3.8 -> 3.3, 32 x 2304 x 576 10.5 -> 7.6, 64 x 2304 x 576 17.6 -> 13.6, 48 x 3072 x 768 19.6 -> 14.6;
+    // 32 x 1536 x 768 9.1 -> 9.8 and 64 x 512 x 2304 11.5 -> 12.9, as many waves as passes, stay in one CTA.  The sums and
+    // their order are the same.
+    const int tiles = few_rows_tiles<kCols>(a), passes = (a.rows + kRows - 1) / kRows, at_once = 2 * sm_count();
+    const bool apart = tiles <= at_once && (tiles * passes + at_once - 1) / at_once < passes;
+    if (apart) launch_kernel(few_rows_projection_kernel<kRows, kCols, (kRows >= 8)>, dim3(passes, tiles), dim3(kFewThreads), 0, stream, a);
+    else launch_kernel(few_rows_projection_kernel<kRows, kCols, false>, dim3(tiles), dim3(kFewThreads), 0, stream, a);
     count_launch();
     return check_launch("few_rows_projection_kernel");
 }
@@ -168,8 +171,8 @@ int dispatch_few_rows(const FewRowsArgs& a, void* stream) {
     if (a.rows == 1) return launch_few_rows<1, kCols>(a, stream);
     if (a.rows == 2) return launch_few_rows<2, kCols>(a, stream);
     if (a.rows <= 4) return launch_few_rows<4, kCols>(a, stream);
-    // Eight rows a pass where all passes then run at once and are long enough to gain by it (us: 16 x 2048 x 512 4.9 -> 4.45,
-    // 16 x 2304 x 576 6.6 -> 5.4; 9 x 1024 x 256 2.4 -> 2.55).
+    // Eight rows a pass where all passes then run at once and are long enough to gain by it (us: 16 x 2048 x 512 5.2 -> 4.7,
+    // 16 x 2304 x 576 6.8 -> 5.6; 9 x 1024 x 256 2.4 -> 2.55).
     const bool eight = a.rows <= 8 || (a.k >= 16 * kFewStep && few_rows_tiles<kCols>(a) * static_cast<int64_t>((a.rows + 7) / 8) <= 2 * sm_count());
     return eight ? launch_few_rows<8, kCols>(a, stream) : launch_few_rows<16, kCols>(a, stream);
 }
