@@ -746,8 +746,9 @@ __device__ __forceinline__ int rank_among(const uint32_t* keys, int n_groups, ui
 // eight warps' bests, add the anchor's partner-query row and do the same for the partners; the top K come from ranking
 // every candidate against all others by the whole CTA.  Half of a cold phase is instruction fetch (a pass of blocks
 // takes 2300 cycles where its arithmetic needs some 900), so both streams run through one copy of the code.
-// In fp32 a lane's eighth of a row is 32 bytes and whole caches fit up to 352 positions: 9.4 -> 6.2 us at one row of 128
-// positions, 10.5 -> 9.1 at 512 (window alone), against select_row.
+// In fp32 a lane's eighth of a row is 32 bytes, and whole caches fit where 512 bytes a position and 1024 a block leave some
+// 2.5 KB of 220 (384 positions in 12 blocks, 344 in 43): 9.4 -> 6.2 us at one row of 128 positions, 10.5 -> 9.1 at 512 (window
+// alone), against select_row.
 // kResident: both key caches of the sequence in shared memory (requested before the dependency wait), else the window
 // there and the picked rows from L2.
 template <int kDt, bool kResident>
@@ -1557,9 +1558,16 @@ int launch(SelectArgs& a, void* stream) {
     const Plan& plan = a.plan;
     const int dtype = a.key_dtype == a.query_dtype && a.stats_dtype == a.query_dtype ? a.query_dtype : kAnyDtype;
     const bool decode = a.mode == kPacked && !a.row_batch && !a.row_position && !a.exclude_list;
-    // (single precision: two such CTAs per SM, three of the general form, which therefore holds more rows at once)
+    // Single precision: two such CTAs per SM, three of the general form, which therefore holds more rows at once; and the
+    // many rounds of choosing short blocks are no shorter here (us with whole caches not staged, general form -> this one:
+    // 512 positions in blocks of 8, top 8 11.3 -> 11.6, top 4 10.4 -> 10.3).
     const bool passes = decode && a.top_blocks <= kDecodeTop && plan.total <= kSmemDynamicLimit - kDecodeStatic &&
-                        (dtype != RLM_F32 || a.n_rows <= 2 * a.sm_count);
+                        (dtype != RLM_F32 || (a.n_rows <= 2 * a.sm_count && (a.resident || a.block_size >= 16 || a.top_blocks <= 4)));
+    // Picked rows are read where they lie: with a buffer for them only one CTA of a wide choice fitted an SM (us, 149 rows of
+    // 352 positions in fp32, eight blocks of 32: 19.0 -> 11.3, 15.1 in the general form).
+    if (passes && !many_rows && !a.resident)
+        a.plan = make_plan(a.n_blocks, a.block_size, a.local_window, a.top_blocks, a.buckets, dtype_size(a.key_dtype),
+                           dtype_size(a.stats_dtype), a.mode, false, 0, false);
     auto kernel = dtype == RLM_BF16 ? select_kernel<RLM_BF16>(many_rows, decode, passes, a.resident)
                   : dtype == RLM_F16 ? select_kernel<RLM_F16>(many_rows, decode, passes, a.resident)
                   : dtype == RLM_F32 ? select_kernel<RLM_F32>(many_rows, decode, passes, a.resident)

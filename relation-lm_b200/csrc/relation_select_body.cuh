@@ -85,10 +85,11 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 // anchor's place once the anchor's first scoring pass has read them: a smaller footprint, so
 // more rows per SM, for launches of many rows.
 // resident_rows > 0: the whole key cache of the sequence (that many rows) takes the place of the
-// local window, and no buffer is kept for remote blocks (see SelectArgs::resident).
+// local window, and no buffer is kept for remote blocks (see SelectArgs::resident).  Nor is one with `remote` = false, for
+// the kernel that reads them where they lie.
 __host__ __device__ inline Plan make_plan(int nb, int bs, int local, int top, int buckets,
                                           int key_size, int stats_size, int mode, bool shared_streams,
-                                          int resident_rows = 0) {
+                                          int resident_rows = 0, bool remote = true) {
     Plan p;
     int off = 0;
     int stats_bytes = nb * kD * stats_size;
@@ -100,7 +101,7 @@ __host__ __device__ inline Plan make_plan(int nb, int bs, int local, int top, in
     p.p_std = shared_streams ? p.a_std : off; off += partner && !shared_streams ? stats_bytes : 0;
     p.a_local = off; off += anchor ? local_bytes : 0;
     p.p_local = shared_streams ? p.a_local : off; off += partner && !shared_streams ? local_bytes : 0;
-    p.remote = off; off += resident_rows > 0 ? 0 : top * bs * kD * key_size;
+    p.remote = off; off += resident_rows > 0 || !remote ? 0 : top * bs * kD * key_size;
     p.queries = off; off += 4 * kD * 4;
     p.params = off; off += align16(8 * buckets * 4);
     p.block_scores = off; off += align16(((nb + 3) & ~3) * 4);

@@ -30,6 +30,13 @@ SHAPES = [
     (2, 1024, 16, 64, 4, 32),     # 320 candidates
     (1, 2048, 16, 40, 4, 8),      # 552 candidates
     (297, 64, 8, 16, 2, 8),       # more rows than two per SM: the general form
+    (2, 384, 12, 32, 2, 8),       # both key caches staged, blocks of 32
+    (2, 416, 13, 32, 2, 8),       # ... a block more: the window
+    (2, 344, 43, 16, 2, 8),       # both staged, blocks of 8
+    (2, 352, 44, 16, 2, 8),       # ... a block more: the window
+    (149, 352, 11, 64, 8, 8),     # two rows an SM, more picked rows than a pass per warp
+    (2, 512, 64, 16, 4, 8),       # the most short blocks this form chooses
+    (2, 512, 64, 16, 5, 8),       # ... and one more: the general form
 ]
 
 
