@@ -1,6 +1,6 @@
 """Single-precision products of several passes of rows, the passes on CTAs of their own or in one CTA: on both sides of
-the rules' lines (columns that fill two CTAs an SM, eight or sixteen rows a pass), against 64-bit products, and each row
-the same bits as alone with seven others."""
+the rules' lines (columns that fill two CTAs an SM, waves against passes, eight or sixteen rows a pass), against 64-bit
+products, and each row the same bits as alone with seven others."""
 from __future__ import annotations
 
 import pytest
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows", [9, 16, 17, 24, 33, 64])
-@pytest.mark.parametrize("d_in,n_out", [(2048, 592), (2044, 600), (1024, 1184), (1024, 1185), (2304, 576), (1920, 40)])
+@pytest.mark.parametrize("d_in,n_out", [(2048, 592), (2044, 600), (1024, 1184), (1024, 1185), (2304, 576), (1920, 40), (1536, 768)])
 def test_passes(rows, d_in, n_out):
     from relation_lm.kernels.packed_projection import few_rows_projection
 
