@@ -230,26 +230,33 @@ Four relation_select_packed_rows(SELECT_PARAMS, const Tensor& row_batch, const T
     return select(SELECT_TENSORS, nullptr, &row_batch, &row_position, local_window, top_blocks, k_out, strict_valid);
 }
 
-Four relation_select_packed_prefill(SELECT_PARAMS, int64_t query_length, int64_t local_window, int64_t top_blocks,
-                                    int64_t k_out, bool strict_valid) {
-    const SelectTensors s = SELECT_TENSORS;
+// `fits`: where to say that the tile's staging exceeds the shared memory (nothing was launched), instead of raising.
+Four select_prefill(const SelectTensors& s, int64_t query_length, int64_t local_window, int64_t top_blocks, int64_t k_out,
+                    bool strict_valid, bool* fits) {
     s.rows();
     const c10::Device device = s.caches();
-    const int64_t n_seq = anchor_keys.size(0), rows = n_seq * query_length;
-    TORCH_CHECK_VALUE(is_shape(anchor_query, {rows, 64}) && is_shape(anchor_router_query, {rows, 64}) &&
-                          is_shape(partner_base, {rows, 128}),
+    const int64_t n_seq = s.anchor_keys.size(0), rows = n_seq * query_length;
+    TORCH_CHECK_VALUE(is_shape(s.anchor_query, {rows, 64}) && is_shape(s.anchor_router_query, {rows, 64}) &&
+                          is_shape(s.partner_base, {rows, 128}),
                       "queries must hold one row per (sequence, position): [B * query_length, width]");
-    check_router_width(anchor_query, anchor_block_mean);
+    check_router_width(s.anchor_query, s.anchor_block_mean);
     const int q = s.query_dtype(), k = s.key_dtype(), st = s.stats_dtype(), p = s.param_dtype();
     Launch launch(device);
     Tensor anchor = empty({rows}, at::kInt, device), anchor_score = empty({rows}, at::kFloat, device);
     Tensor partner = empty({rows, k_out}, at::kInt, device), partner_score = empty({rows, k_out}, at::kFloat, device);
-    check(rlm_relation_select_packed_prefill(
-        SELECT_POINTERS(s), i32(anchor), f32(anchor_score), i32(partner), f32(partner_score), anchor_query.stride(0),
-        anchor_router_query.stride(0), partner_base.stride(0), n_seq, query_length, anchor_keys.size(1),
-        anchor_block_mean.size(1), anchor_bias.size(1), local_window, top_blocks, k_out, strict_valid, q, k, st, p,
-        launch.status, launch.stream));
+    const int rc = rlm_relation_select_packed_prefill(
+        SELECT_POINTERS(s), i32(anchor), f32(anchor_score), i32(partner), f32(partner_score), s.anchor_query.stride(0),
+        s.anchor_router_query.stride(0), s.partner_base.stride(0), n_seq, query_length, s.anchor_keys.size(1),
+        s.anchor_block_mean.size(1), s.anchor_bias.size(1), local_window, top_blocks, k_out, strict_valid, q, k, st, p,
+        launch.status, launch.stream);
+    if (fits) *fits = rc != RLM_ERR_SMEM;
+    if (!fits || *fits) check(rc);
     return {anchor, anchor_score, partner, partner_score};
+}
+
+Four relation_select_packed_prefill(SELECT_PARAMS, int64_t query_length, int64_t local_window, int64_t top_blocks,
+                                    int64_t k_out, bool strict_valid) {
+    return select_prefill(SELECT_TENSORS, query_length, local_window, top_blocks, k_out, strict_valid, nullptr);
 }
 
 // Shared by the two multi-anchor forms: shapes, outputs and the call.  The kernels write the anchors'
@@ -1082,8 +1089,9 @@ std::vector<Tensor> prefill_state(const Tensor& x, const Tensor& norm_weight, co
     return state;
 }
 
-// The layer's output [B, T, d] for residual inputs x and their state.
-Tensor prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps, const Tensor& query_weight,
+// The layer's output [B, T, d] for residual inputs x and their state, and its queries; no output where the selector's tile
+// does not fit: the queries then go on to the selector of rows.
+Two prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps, const Tensor& query_weight,
                      const Tensor& anchor_keys, const Tensor& anchor_mean, const Tensor& anchor_std, const Tensor& anchor_gamma,
                      const Tensor& anchor_bias, const Tensor& partner_anchor_cache, const Tensor& partner_keys,
                      const Tensor& partner_mean, const Tensor& partner_std, const Tensor& partner_gamma, const Tensor& partner_bias,
@@ -1095,14 +1103,17 @@ Tensor prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& n
     Tensor normalized = empty(rows.sizes(), query_weight.scalar_type(), x.device());
     layer_norm_cast(rows, norm_weight, norm_bias, norm_eps, normalized);
     const Tensor q = packed_projection(normalized, query_weight, std::nullopt);
-    const auto [anchor, anchor_score, partner, score] = relation_select_packed_prefill(
-        q.narrow(1, 0, 64), anchor_keys, q.narrow(1, 64, 64), anchor_mean, anchor_std, anchor_gamma, anchor_bias, q.narrow(1, 128, 128),
-        partner_anchor_cache, partner_keys, partner_mean, partner_std, partner_gamma, partner_bias, length, local_window, top_blocks,
-        k_out, strict_valid);
+    const Tensor anchor_query = q.narrow(1, 0, 64), router_query = q.narrow(1, 64, 64), partner_base = q.narrow(1, 128, 128);
+    bool fits = true;
+    const auto [anchor, anchor_score, partner, score] = select_prefill(
+        {anchor_query, anchor_keys, router_query, anchor_mean, anchor_std, anchor_gamma, anchor_bias, partner_base, partner_anchor_cache,
+         partner_keys, partner_mean, partner_std, partner_gamma, partner_bias},
+        length, local_window, top_blocks, k_out, strict_valid, &fits);
+    if (!fits) return {Tensor(), q};
     Tensor out = empty(rows.sizes(), at::kFloat, x.device());
     relation_mlp_rows(out, expanded_cache, operand_cache, anchor, partner, score, std::nullopt, std::nullopt, mix, product_weight,
                       second_weight, second_bias, relation_norm_weight, relation_norm_bias, norm_eps, rows.contiguous(), 1, length, true);
-    return out.view({batch, length, dim});
+    return {out.view({batch, length, dim}), q};
 }
 
 // ------------------------------------------------------------------ what surrounds an operator

@@ -103,23 +103,23 @@ class RoutedPrefillLayer:
         B, T, d = x.shape
         N, K, H = B * T, cfg.k_max, cfg.hidden_dim
         fused, tiled = self.fused_mlp and keep is None, cfg.local_window + cfg.top_blocks * cfg.block_size <= 512
+        q = None
         if fused and tiled and self.tiled_select:
-            try:
-                out = _abi.direct_call(
-                    "prefill_layer", x, w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, w["w_query"], state["anchor_keys"],
-                    state["anchor_mean"], state["anchor_std"], w["anchor_gamma"], w["anchor_bias"], state["partner_anchor_cache"],
-                    state["partner_keys"], state["partner_mean"], state["partner_std"], w["partner_gamma"], w["partner_bias"],
-                    cfg.local_window, cfg.top_blocks, K, cfg.strict_valid, state["expanded_cache"], state["operand_cache"],
-                    w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"])
-                if out is not NotImplemented:
+            made = _abi.direct_call(
+                "prefill_layer", x, w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, w["w_query"], state["anchor_keys"],
+                state["anchor_mean"], state["anchor_std"], w["anchor_gamma"], w["anchor_bias"], state["partner_anchor_cache"],
+                state["partner_keys"], state["partner_mean"], state["partner_std"], w["partner_gamma"], w["partner_bias"],
+                cfg.local_window, cfg.top_blocks, K, cfg.strict_valid, state["expanded_cache"], state["operand_cache"],
+                w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"])
+            if made is not NotImplemented:
+                out, q = made
+                if out is not None:
                     return out
-            except (ValueError, RuntimeError) as error:
-                if "shared memory" not in str(error):       # only "the tile's staging does not fit" falls back
-                    raise
-                self.tiled_select = False
-        normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
-        layer_norm_cast(x.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
-        q = packed_projection(normalized, w["w_query"])
+                self.tiled_select = False                   # the tile's staging does not fit: the queries' rows one by one
+        if q is None:
+            normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
+            layer_norm_cast(x.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
+            q = packed_projection(normalized, w["w_query"])
         select_args = (q[:, 0:64], state["anchor_keys"], q[:, 64:128], state["anchor_mean"], state["anchor_std"],
                        w["anchor_gamma"], w["anchor_bias"], q[:, 128:256], state["partner_anchor_cache"],
                        state["partner_keys"], state["partner_mean"], state["partner_std"], w["partner_gamma"],
