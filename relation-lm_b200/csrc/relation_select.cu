@@ -1383,9 +1383,9 @@ TileShape tile_shape(int n_seq, int q_len, int most_warps, const Smem& smem) {
 // 80.6 -> 68.4, 2 x 640 77.3 -> 67.4, 2 x 1024 of d 768 169 -> 159, 1 x 512 52.5 -> 52.5; with the selector alone launched
 // in the ordinary way 69.7, 66.1, 160, 52.1; of a multi-anchor stack: 2 x 848 of d 256, two slots 123 -> 101, 1 x 2048 of
 // d 512 196 -> 177).  More tiles than SMs share them anyway.
-int tile_smem(int total, int tiles) {
+int tile_smem(int total, int tiles, int warps) {
     constexpr int kMoreThanHalf = 228 * 1024 / 2;
-    return tiles <= sm_count() && total < kMoreThanHalf ? kMoreThanHalf : total;
+    return tiles <= sm_count() && warps <= 16 && total < kMoreThanHalf ? kMoreThanHalf : total;
 }
 
 template <int kDt>
@@ -1465,7 +1465,7 @@ int launch_multi_tile(MultiTileArgs& ta, void* stream) {
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     const int tiles = a.n_seq * ((ta.q_len + ta.tile_queries - 1) / ta.tile_queries);
-    launch_kernel(kernel, dim3(tiles), dim3(32 * warps), tile_smem(total, tiles), stream, ta);
+    launch_kernel(kernel, dim3(tiles), dim3(32 * warps), tile_smem(total, tiles, warps), stream, ta);
     count_launch();
     return check_launch("relation_select_multi_tile_kernel");
 }
@@ -1527,7 +1527,7 @@ int launch_tile(TileArgs& m, void* stream) {
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
     const int tiles = a.n_seq * ((m.q_len + m.tile_queries - 1) / m.tile_queries);
-    launch_kernel(kernel, dim3(tiles), dim3(32 * warps), tile_smem(total, tiles), stream, m);
+    launch_kernel(kernel, dim3(tiles), dim3(32 * warps), tile_smem(total, tiles, warps), stream, m);
     count_launch();
     return check_launch("relation_select_tile_kernel");
 }

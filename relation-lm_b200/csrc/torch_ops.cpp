@@ -1089,9 +1089,9 @@ std::vector<Tensor> prefill_state(const Tensor& x, const Tensor& norm_weight, co
     return state;
 }
 
-// The layer's output [B, T, d] for residual inputs x and their state, and its queries; no output where the selector's tile
-// does not fit: the queries then go on to the selector of rows.
-Two prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps, const Tensor& query_weight,
+// The layer's output [B, T, d] for residual inputs x and their state; where the selector's tile does not fit, none, and the
+// queries, which then go on to the selector of rows.
+std::vector<Tensor> prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm_bias, double norm_eps, const Tensor& query_weight,
                      const Tensor& anchor_keys, const Tensor& anchor_mean, const Tensor& anchor_std, const Tensor& anchor_gamma,
                      const Tensor& anchor_bias, const Tensor& partner_anchor_cache, const Tensor& partner_keys,
                      const Tensor& partner_mean, const Tensor& partner_std, const Tensor& partner_gamma, const Tensor& partner_bias,
@@ -1113,7 +1113,7 @@ Two prefill_layer(const Tensor& x, const Tensor& norm_weight, const Tensor& norm
     Tensor out = empty(rows.sizes(), at::kFloat, x.device());
     relation_mlp_rows(out, expanded_cache, operand_cache, anchor, partner, score, std::nullopt, std::nullopt, mix, product_weight,
                       second_weight, second_bias, relation_norm_weight, relation_norm_bias, norm_eps, rows.contiguous(), 1, length, true);
-    return {out.view({batch, length, dim}), q};
+    return {out.view({batch, length, dim})};
 }
 
 // ------------------------------------------------------------------ what surrounds an operator

@@ -112,10 +112,10 @@ class RoutedPrefillLayer:
                 cfg.local_window, cfg.top_blocks, K, cfg.strict_valid, state["expanded_cache"], state["operand_cache"],
                 w["mix"], w["product_weight"], w["w2"], w["b2"], w["relation_norm_w"], w["relation_norm_b"])
             if made is not NotImplemented:
-                out, q = made
-                if out is not None:
-                    return out
+                if made[0] is not None:
+                    return made[0]
                 self.tiled_select = False                   # the tile's staging does not fit: the queries' rows one by one
+                q = made[1]
         if q is None:
             normalized = torch.empty(N, d, device=self.device, dtype=self.dtype)
             layer_norm_cast(x.view(N, d), w["input_norm_w"], w["input_norm_b"], cfg.norm_eps, normalized)
