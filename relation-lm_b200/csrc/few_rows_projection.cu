@@ -156,10 +156,13 @@ int launch_few_rows(const FewRowsArgs& a, void* stream) {
     // Passes over rows on CTAs of their own where that makes fewer waves (two CTAs an SM) than a CTA would make passes: a pass
     // is a few dependent loads long, not a stream; where the columns fill the SMs, further passes find their weights in L1.
     // us: 32 x 1024 x 256 3.8 -> 3.3, 32 x 2304 x 576 10.5 -> 7.6, 64 x 2304 x 576 17.6 -> 13.6, 48 x 3072 x 768 19.6 -> 14.6;
-    // 32 x 1536 x 768 9.1 -> 9.8 and 64 x 512 x 2304 11.5 -> 12.9, as many waves as passes, stay in one CTA.  The sums and
-    // their order are the same.
+    // 32 x 1536 x 768 9.1 -> 9.8 and 64 x 512 x 2304 11.5 -> 12.9, as many waves as passes, stay in one CTA, except where the
+    // second wave is at most half full and its passes are long and even: 32 x 2048 x 768 10.3 -> 9.8, 24 x 3072 x 768
+    // 13.7 -> 12.4 (but 32 x 2304 x 768 12.6 -> 13.2).  The sums and their order are the same.
     const int tiles = few_rows_tiles<kCols>(a), passes = (a.rows + kRows - 1) / kRows, at_once = 2 * sm_count();
-    const bool apart = tiles <= at_once && (tiles * passes + at_once - 1) / at_once < passes;
+    const bool fewer = (tiles * static_cast<int64_t>(passes) + at_once - 1) / at_once < passes;
+    const bool even = 2 * tiles * static_cast<int64_t>(passes) <= 3 * at_once && a.k >= 16 * kFewStep && a.k % (a.k_parts * kFewStep) == 0;
+    const bool apart = passes > 1 && tiles <= at_once && (fewer || even);
     if (apart) launch_kernel(few_rows_projection_kernel<kRows, kCols, (kRows >= 8)>, dim3(passes, tiles), dim3(kFewThreads), 0, stream, a);
     else launch_kernel(few_rows_projection_kernel<kRows, kCols, false>, dim3(tiles), dim3(kFewThreads), 0, stream, a);
     count_launch();
