@@ -751,7 +751,10 @@ __device__ __forceinline__ int rank_among(const uint32_t* keys, int n_groups, ui
 // alone), against select_row.
 // kResident: both key caches of the sequence in shared memory (requested before the dependency wait), else the window
 // there and the picked rows from L2.
-template <int kDt, bool kResident>
+// kCtaTop: the top K of 257 to 512 candidates by the CTA, as in select_row, not by a warp (fp32, whose scores that are NaN
+// then rank as in launches of more rows).  A build of its own: without the warp's top K the other one's code is the slower,
+// whether a launch comes there or not (us a step of batch 7, d 768, 5 layers 272.8 -> 275.7).
+template <int kDt, bool kResident, bool kCtaTop = false>
 __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_decode_kernel(const SelectArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t best_key_s[kWarps], short_list[64];
@@ -943,7 +946,7 @@ __global__ void __launch_bounds__(kThreads, kResident ? 1 : 2) relation_select_d
         }
         // more partners than candidates
         for (int k = cap + tid; k < K; k += kThreads) { out_pos[k] = t - L + 1; out_score[k] = kNegInf; }
-    } else if (cap4 > 512 || kDt == RLM_F32) {       // (fp32: the position of a score that is NaN, as select_row)
+    } else if (kCtaTop || cap4 > 512) {
         topk_large(cand, cap, K, L, t, bs, sel_s, out_pos, out_score);
     } else if (warp == 0) {
         topk_warp(cand, cap4, K, L, t, bs, bs_shift, sel, short_list, out_pos, out_score);
@@ -1542,10 +1545,9 @@ auto select_kernel(bool many_rows, bool decode, bool passes, bool resident) {
                        : relation_select_kernel<3, kDt, false>;
 }
 
-template <>
-auto select_kernel<RLM_F32>(bool many_rows, bool decode, bool passes, bool resident) {
-    return resident ? relation_select_decode_kernel<RLM_F32, true>
-           : passes && !many_rows ? relation_select_decode_kernel<RLM_F32, false>
+auto select_kernel_fp32(bool many_rows, bool decode, bool passes, bool resident, bool cta_top) {
+    return resident ? (cta_top ? relation_select_decode_kernel<RLM_F32, true, true> : relation_select_decode_kernel<RLM_F32, true>)
+           : passes && !many_rows ? (cta_top ? relation_select_decode_kernel<RLM_F32, false, true> : relation_select_decode_kernel<RLM_F32, false>)
            : decode ? (many_rows ? relation_select_kernel<4, RLM_F32, true> : relation_select_kernel<3, RLM_F32, true>)
                     : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
 }
@@ -1570,7 +1572,7 @@ int launch(SelectArgs& a, void* stream) {
                            dtype_size(a.stats_dtype), a.mode, false, 0, false);
     auto kernel = dtype == RLM_BF16 ? select_kernel<RLM_BF16>(many_rows, decode, passes, a.resident)
                   : dtype == RLM_F16 ? select_kernel<RLM_F16>(many_rows, decode, passes, a.resident)
-                  : dtype == RLM_F32 ? select_kernel<RLM_F32>(many_rows, decode, passes, a.resident)
+                  : dtype == RLM_F32 ? select_kernel_fp32(many_rows, decode, passes, a.resident, a.local_window + a.top_blocks * a.block_size > 256)
                                      : (many_rows ? relation_select_kernel<4, kAnyDtype, false> : relation_select_kernel<3, kAnyDtype, false>);
     int rc = allow_large_smem(reinterpret_cast<const void*>(kernel), kSmemPerCta);
     if (rc != RLM_OK) return rc;
