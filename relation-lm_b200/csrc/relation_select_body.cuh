@@ -252,7 +252,8 @@ __device__ __forceinline__ void score_rows(const unsigned char* rows, int key_dt
 }
 
 // Block scores of the first `n_complete` blocks with the `nw` warps of a group; the other
-// entries of `out` (up to the next multiple of four) are set to -inf.
+// entries of `out` (up to the next multiple of four) are set to -inf.  So is a score that is NaN: such a block is no
+// choice, as in the forms of warp passes, while its key would come before all others or among them.
 template <int kDt>
 __device__ __noinline__ void score_blocks(const unsigned char* mean, const unsigned char* stdv,
                                           int stats_dtype_arg, int nb, int n_complete, int bs, int t,
@@ -296,7 +297,7 @@ __device__ __noinline__ void score_blocks(const unsigned char* mean, const unsig
         e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 4));
         float acc = __fadd_rn(mx, canon_log(e));
         if (j == 0 && live) {
-            bool eligible = !strict || end < ls;
+            bool eligible = (!strict || end < ls) && acc > -1.0e30f;
             out[n] = eligible ? acc : kNegInf;
         }
     }
@@ -354,7 +355,7 @@ __device__ __noinline__ void score_blocks_head(const unsigned char* mean, const 
         e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, 2));       // (e0 + e1) + (e2 + e3)
         const float acc = __fadd_rn(mx, canon_log(e));
         if (head == 0 && live) {
-            const bool eligible = !strict || end < ls;
+            const bool eligible = (!strict || end < ls) && acc > -1.0e30f;
             out[n] = eligible ? acc : kNegInf;
         }
     }
@@ -593,18 +594,14 @@ __device__ __noinline__ void topk_large(float* cand, int cap, int K, int L, int 
 // one pass.  Lane l holds the scores of blocks l, l + 32, ...; each of the `top` rounds takes
 // the best remaining block of the warp (two redux instructions; ties to the lowest index) and
 // hands it to lane `round`, which then requests its own block, after lane 0 has posted the byte
-// count of all of them.  Same result as pick_blocks + issue_remote: a block whose score is NaN is no choice, as in every
-// other form (taken by its key it would come before all others and end the choice).
+// count of all of them.  Same result as pick_blocks + issue_remote (no score is NaN, see score_blocks).
 __device__ __noinline__ void pick_and_issue(const float* scores, int nb, int top, int bs, int ls, int* sel,
                                             const unsigned char* keys, unsigned char* dst, size_t key_row,
                                             size_t seq_keys, uint32_t bar) {
     const int lane = threadIdx.x & 31;
     uint32_t k[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float v = lane + 32 * i < nb ? scores[lane + 32 * i] : kNegInf;
-        k[i] = v > -1.0e30f ? float_key(v) : 0u;
-    }
+    for (int i = 0; i < 4; ++i) k[i] = lane + 32 * i < nb ? float_key(scores[lane + 32 * i]) : 0u;
     int my_block = 0, my_rows = 0;
     for (int r = 0; r < top; ++r) {
         uint32_t bk = 0;
@@ -613,7 +610,7 @@ __device__ __noinline__ void pick_and_issue(const float* scores, int nb, int top
         for (int i = 0; i < 4; ++i)
             if (k[i] > bk) { bk = k[i]; bn = lane + 32 * i; }
         warp_argmax_key(bk, bn);
-        if (bk == 0u) break;                             // no usable block is left
+        if (!(key_float(bk) > -1.0e30f)) break;          // no usable block is left
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (lane + 32 * i == bn) k[i] = 0u;
