@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 3) relation_select_multi_kernel(cons
 // registers (128 per thread, 16 warps per SM), and remote rows had to pass through shared memory to be read that
 // way: 96 cycles of the SM's shared-memory pipe for 32 rows against 39 here.
 // Whole-sequence selection of 8 x 4096 rows (384 candidates, 64 blocks): 466 -> 341 us; 16 x 2048 rows of four slots:
-// 1233 -> 955 us.  Issue slots are 71 % taken now (56 % before).
+// 1233 -> 955 us.  Issue slots 56 -> 71 % taken (69 % since anchor queries stay in 16 bits, below, with 8 % fewer instructions).
 constexpr uint32_t kRow = 2 * kD;
 
 // A row in kDt, and a lane's eighth of it: 16 bytes, in single precision (the decode form alone) 32.
@@ -203,8 +203,8 @@ __device__ __forceinline__ QueryChunk magnitude(const QueryChunk& q) {
 
 // The chunk of a query whose values are kDt's own (the anchor stream's: a partner query is a sum, rounded to fp32), as
 // they lie: the mixed-precision fma takes both factors in 16 bits, widens them exactly and rounds once, the same sums
-// as of widened rows in two thirds of the instructions (16 instead of 24 for two rows' chunks; 0.54 against 0.68 ms for
-// 19 G of them on all SMs).  A multi-anchor pass, us: 16 x 2048 rows of four slots, four layers 11 440 -> 11 270,
+// as of widened rows in two thirds of the instructions (16 instead of 24 for two rows' chunks; 135 -> 124 million
+// for 4 x 4096 rows of a whole-sequence launch, 192 -> 174 us under the profiler).  A multi-anchor pass, us: 16 x 2048 rows of four slots, four layers 11 440 -> 11 270,
 // 3 x 1056 rows of two slots, two layers 260 -> 256.
 template <int kDt>
 struct NarrowChunk { uint32_t v[4]; };
